@@ -315,6 +315,8 @@ __global__ void __launch_bounds__(kBThreads) k_batch_compact(BatchLayout L, Comp
     for (i64 e = L.G - 1; e >= 0 && __ldg(L.item_off + e) == n; --e) out.unique_ptr[e] = total;
     counters[CNT_UNIQUE] = total;
     counters[CNT_NNZ] = L.indices_ptr[L.G];
+    mail_post(out.mail, 0, total, counters);
+    mail_post(out.mail, 1, L.indices_ptr[L.G], counters);
   }
 }
 
@@ -629,10 +631,21 @@ static int read_totals(gsb_ctx* ctx, cudaStream_t stream, i64* unique_total_host
   return GSB_OK;
 }
 
+// The same two totals from the mailbox that the last pass to know them posted to.
+static int mailed_totals(gsb_ctx* ctx, cudaStream_t stream, const Mail& mail, i64* unique_total_host,
+                         i64* edges_total_host) {
+  i64 v[2] = {0, 0};
+  const int st = ctx_mail_result(ctx, stream, mail, 2, v);
+  if (unique_total_host) *unique_total_host = v[0];
+  if (edges_total_host) *edges_total_host = v[1];
+  return st;
+}
+static inline Mail mail_if(gsb_ctx* ctx, bool wanted) { return wanted ? ctx_mail(ctx) : Mail{nullptr, 0}; }
+
 // L carries seeds / seeds_ptr / indices / indices_ptr / G; scratch fields are filled here.  seeds_bound / edges_bound
 // are what the caller sized the outputs for (the exact counts are read on the device).
 static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64 seeds_bound, i64 edges_bound,
-                           i64 num_nodes, int flags, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled) {
+                           i64 num_nodes, int flags, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled, Mail mail) {
   const i64 G = L.G;
   const i64 n_cap = seeds_bound + edges_bound;
   i64* counters = ctx_counters(ctx);
@@ -671,7 +684,7 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
     T.rank_of_item = (uint32_t*)((char*)ws + off_bytes);
     T.seeds_distinct = (flags & GSB_SEEDS_DISTINCT) ? 1 : 0;
     return direct_unique_relabel_launch(ctx, stream, L, T, n_cap, edges_bound, out_unique, out_unique_ptr,
-                                        out_relabeled);
+                                        out_relabeled, mail);
   }
   if (path == 3 || (path == 0 && partition_suits(n_cap, G))) {
     // partitioned form (the default for large calls when the direct-address tables above were not chosen): shared-memory tables per bucket of items, then ranking by bit vectors
@@ -693,7 +706,7 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
     }
     GSB_LAUNCH_OK();
     return partition_unique_relabel(ctx, stream, L, n_cap, bucket_cap, (char*)ws + 3 * off_bytes, false, out_unique,
-                                    out_unique_ptr, out_relabeled);
+                                    out_unique_ptr, out_relabeled, mail);
   }
   if (!L.indices_ptr) return GSB_ERR_INVALID_ARGUMENT;  // the forms below expect both arrays
   const i64 slot_cap = region_size_for(n_cap) + 32 * G + 64;
@@ -730,7 +743,8 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   // compaction that only READS the slots and leaves, for every neighbour, its frontier rank or a reference to the
   // item that came first, then the fix-up pass over a dense 4-byte array: one random table access fewer per first
   // occurrence and about half a random access per neighbour instead of a second probe of the table
-  return direct_unique_relabel_launch(ctx, stream, L, T, n_cap, edges_bound, out_unique, out_unique_ptr, out_relabeled);
+  return direct_unique_relabel_launch(ctx, stream, L, T, n_cap, edges_bound, out_unique, out_unique_ptr, out_relabeled,
+                                      mail);
 }
 
 // One hop of the partitioned form with the per-bucket item counts taken by the sampler itself (fan-outs up to 16): the
@@ -740,7 +754,7 @@ static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64*
                                    i64 num_nodes, const i64* seeds, const i64* seeds_ptr, const i64* batch_ids, i64 G,
                                    i64 S, i64 k, i64 cap, int replace, u64 seed, i64* out_indptr, i64* out_indices,
                                    i64* out_select, i64* out_indices_ptr, i64* out_unique, i64* out_unique_ptr,
-                                   i64* out_relabeled) {
+                                   i64* out_relabeled, Mail mail) {
   i64* counters = ctx_counters(ctx);
   const i64 n_cap = S + cap;
   const size_t off_bytes = ((size_t)(G + 1) * 8 + 255) & ~(size_t)255;
@@ -772,7 +786,7 @@ static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64*
   st = partition_after_sampler(ctx, stream, L, n_cap, bucket_cap, part_ws, out_indptr, S, cap, out_indices_ptr);
   if (st != GSB_OK) return st;
   return partition_unique_relabel(ctx, stream, L, n_cap, bucket_cap, part_ws, true, out_unique, out_unique_ptr,
-                                  out_relabeled);
+                                  out_relabeled, mail);
 }
 
 }  // namespace gsb
@@ -826,11 +840,11 @@ int gsb_batch_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* seeds, 
   L.indices = indices;
   L.indices_ptr = indices_ptr;
   L.G = G;
+  const Mail mail = mail_if(ctx, unique_total_host || edges_total_host);
   int st = relabel_batches(ctx, stream, L, num_seeds, indices_capacity, num_nodes, flags, out_unique, out_unique_ptr,
-                           out_relabeled);
-  if (st != GSB_OK) return st;
-  if (unique_total_host || edges_total_host) return read_totals(ctx, stream, unique_total_host, edges_total_host);
-  return GSB_OK;
+                           out_relabeled, mail);
+  if (st != GSB_OK || !mail.word) return st;
+  return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
 }
 
 int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64_t* indices, int64_t num_nodes,
@@ -852,15 +866,15 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
   GSB_REQUIRE(cap == 0 || (indices && out_indices && out_select && out_relabeled), GSB_ERR_INVALID_ARGUMENT);
   cudaStream_t stream = (cudaStream_t)stream_;
   int st;
+  const Mail mail = mail_if(ctx, unique_total_host || edges_total_host);
   const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
   const bool direct_small = (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes && num_nodes > 0;
   if (k >= 1 && k <= 16 && n_cap > 0 && (path == 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
     st = sage_hop_sampler_counts(ctx, stream, indptr, indices, num_nodes, seeds, seeds_ptr, batch_ids, G, S, k, cap,
                                  replace, (u64)seed, out_indptr, out_indices, out_select, out_indices_ptr, out_unique,
-                                 out_unique_ptr, out_relabeled);
-    if (st != GSB_OK) return st;
-    if (unique_total_host || edges_total_host) return read_totals(ctx, stream, unique_total_host, edges_total_host);
-    return GSB_OK;
+                                 out_unique_ptr, out_relabeled, mail);
+    if (st != GSB_OK || !mail.word) return st;
+    return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
   }
   // the exact seed count is seeds_ptr[G] on the device; S only has to bound it (grids, scratch and capacities)
   st = sample_uniform_launch(ctx, stream, indptr, indices, num_nodes, seeds, S, k, replace, (u64)seed, out_indptr,
@@ -879,10 +893,9 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
   L.indices = out_indices;
   L.indices_ptr = out_indices_ptr;
   L.G = G;
-  st = relabel_batches(ctx, stream, L, S, cap, num_nodes, flags, out_unique, out_unique_ptr, out_relabeled);
-  if (st != GSB_OK) return st;
-  if (unique_total_host || edges_total_host) return read_totals(ctx, stream, unique_total_host, edges_total_host);
-  return GSB_OK;
+  st = relabel_batches(ctx, stream, L, S, cap, num_nodes, flags, out_unique, out_unique_ptr, out_relabeled, mail);
+  if (st != GSB_OK || !mail.word) return st;
+  return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
 }
 
 }  // extern "C"
@@ -947,7 +960,7 @@ static int build_batch_tables(gsb_ctx* ctx, cudaStream_t stream, const i64* seed
     TileState ts;
     st = ctx_tile_state(ctx, tiles, stream, &ts);
     if (st != GSB_OK) return st;
-    CompactOut out{out_unique, out_unique_ptr};
+    CompactOut out{out_unique, out_unique_ptr, Mail{nullptr, 0}};
     ScopedKernelTimer timer(ctx, KID_FIRST_COMPACT, stream);
     k_batch_compact<<<tiles, kBThreads, 0, stream>>>(L, out, counters, ts);
     GSB_LAUNCH_OK();
@@ -981,7 +994,7 @@ int gsb_batch_unique(gsb_ctx* ctx, void* stream_, const int64_t* data, const int
       L.indices = nullptr;
       L.indices_ptr = nullptr;
       L.G = G;
-      st = relabel_batches(ctx, stream, L, n, 0, 0, 0, out_unique, out_unique_ptr, nullptr);
+      st = relabel_batches(ctx, stream, L, n, 0, 0, 0, out_unique, out_unique_ptr, nullptr, Mail{nullptr, 0});
     } else {
       st = build_batch_tables(ctx, stream, data, data_ptr, n, nullptr, nullptr, 0, G, out_unique, out_unique_ptr, &L,
                               0, nullptr);
@@ -1145,7 +1158,8 @@ int unique_relabel_packed(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i
   st = ctx_tile_state(ctx, tiles, stream, &ts);
   if (st != GSB_OK) return st;
   // unique_ptr[0..1] lives in scratch: nobody needs it here
-  CompactOut out{out_unique, L.item_off + 8};
+  const Mail mail = ctx_mail(ctx);
+  CompactOut out{out_unique, L.item_off + 8, mail};
   {
     ScopedKernelTimer timer(ctx, KID_FIRST_COMPACT, stream);
     k_batch_compact<<<tiles, kBThreads, 0, stream>>>(L, out, counters, ts);
@@ -1157,12 +1171,10 @@ int unique_relabel_packed(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i
                                                                                       counters);
   }
   GSB_LAUNCH_OK();
-  const i64* c;
-  st = ctx_fetch_counters(ctx, stream, CNT_ERROR, 4, &c);
-  if (st != GSB_OK) return st;
-  *unique_host = c[CNT_UNIQUE];
-  if (c[CNT_ERROR] != 0) return ctx_check_device_error(ctx, stream);
-  return GSB_OK;
+  i64 unique = 0;
+  st = ctx_mail_result(ctx, stream, mail, 1, &unique);
+  *unique_host = unique;
+  return st;
 }
 
 }  // namespace gsb

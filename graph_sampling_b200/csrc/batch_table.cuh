@@ -161,7 +161,8 @@ constexpr uint32_t kEdgeKeyBit = 0x80000000u;
 // insert -> first-occurrence compaction -> relabel with direct-address tables (defined in direct_relabel.cu).
 // L.item_off must be valid (k_batch_layout); n_cap / e_cap bound the items / edges of the call.
 int direct_unique_relabel_launch(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L, const DirectTables& T,
-                                 i64 n_cap, i64 e_cap, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled);
+                                 i64 n_cap, i64 e_cap, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled,
+                                 Mail mail);
 // Partitioned form of the batched unique + relabel (defined in partition_relabel.cu): shared-memory tables per bucket of
 // items, bit-vector ranking, no fix-up pass.  L carries seeds / seeds_ptr / indices / indices_ptr / G; item_off and
 // region_off (first bucket of every minibatch) must be filled by k_batch_layout; `ws` is scratch of
@@ -172,7 +173,7 @@ i64 partition_bucket_capacity(i64 items_bound, i64 G);
 size_t partition_workspace_bytes(i64 n_cap, i64 bucket_cap);
 uint32_t* partition_bucket_counts(void* ws);
 int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64 n_cap, i64 bucket_cap, void* ws,
-                             bool counted, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled);
+                             bool counted, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled, Mail mail);
 // The one-call hop, after its counting sampler: edge offsets of the minibatches (from the sampled block's offsets),
 // item offsets, bound check, bucket starts — everything partition_unique_relabel(counted = true) expects, one launch.
 int partition_after_sampler(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64 n_cap, i64 bucket_cap, void* ws,
@@ -190,6 +191,7 @@ constexpr int kBucketTarget = 2048;  // mean items per bucket
 struct CompactOut {
   i64* unique;      // all frontiers back to back
   i64* unique_ptr;  // [G + 1]
+  Mail mail;        // slots 0, 1: frontier and edge totals, for a caller that waits for them
 };
 
 // Single-batch unique + relabel through the packed-slot batched kernels (defined in batch_relabel.cu).
@@ -202,6 +204,7 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
                           const i64* seeds, i64 S, i64 k, int replace, u64 seed, i64* out_indptr, i64* out_indices,
                           i64* out_select, i64* out_coo_col, const float* data, const i64* e_ids, float* out_data,
                           i64 capacity, const i64* S_dev = nullptr, const i64* batch_ptr = nullptr,
-                          const i64* batch_ids = nullptr, i64 G = 0, const SamplerCount* count = nullptr);
+                          const i64* batch_ids = nullptr, i64 G = 0, const SamplerCount* count = nullptr,
+                          Mail mail = Mail{nullptr, 0});
 
 }  // namespace gsb

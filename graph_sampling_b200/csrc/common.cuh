@@ -90,17 +90,26 @@ enum KernelId {
   KID_NUM
 };
 
-// Context internals (defined in ctx.cu).
-struct Workspace {
-  void* ptr;
-  size_t bytes;
+// Result word a kernel leaves for the host that waits for it: one 64-bit store into page-locked host memory,
+// [tag : 16 | a device error is recorded : 1 | value : 47].  The host spins on the word, so it has the size a few
+// microseconds after the thread that knows it, without the copy, the stream synchronisation and the launch gap that
+// reading a device counter costs (13 us per wait measured for a 24-byte copy + cudaStreamSynchronize).  word == null:
+// nobody waits.
+struct Mail {
+  u64* word;
+  u64 tag;  // already shifted
 };
+constexpr int kMailSlots = 8;
+constexpr int kMailErrorBit = 47;
+constexpr u64 kMailValueMask = (1ull << kMailErrorBit) - 1;
+
+// Context internals (defined in ctx.cu).
 int ctx_reserve_workspace(gsb_ctx* ctx, size_t bytes, void** out);
 int ctx_tile_state(gsb_ctx* ctx, i64 num_tiles, cudaStream_t stream, TileState* out);
 // Offsets of a per-column result by the counting kernel alone (defined in slice_sample.cu): mode 0 = degrees,
 // 1 = min(degree, k), 2 = k per non-empty column.  The total is left in the context's counters.
 int count_scan_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, i64 num_cols, const i64* seeds, i64 S, i64 k,
-                      int mode, i64* out_indptr);
+                      int mode, i64* out_indptr, Mail mail = Mail{nullptr, 0});
 i64* ctx_counters(gsb_ctx* ctx);
 i64* ctx_pinned(gsb_ctx* ctx);
 int ctx_device(gsb_ctx* ctx);
@@ -115,9 +124,16 @@ i64 ctx_option(gsb_ctx* ctx, int option);
 int ctx_direct_tables(gsb_ctx* ctx, i64 count, i64 num_nodes, cudaStream_t stream, u64** out_table,
                       uint32_t* out_epoch);
 int ctx_check_device_error(gsb_ctx* ctx, cudaStream_t stream);
-// Copies `n` counters starting at `first` to pinned memory, synchronises the stream and returns
-// the pinned pointer.
+// Waits until everything queued on `stream` so far is done and returns the `n` counters starting at `first` (a copy in
+// page-locked memory, written by a one-warp kernel that the host spins on).
 int ctx_fetch_counters(gsb_ctx* ctx, cudaStream_t stream, int first, int n, const i64** out);
+// A fresh mailbox for the call's kernels, and the wait for `n` of its slots.  A slot holds the value its kernel posted;
+// *error tells whether a device error was recorded by then (the caller then takes ctx_check_device_error, which waits
+// for the stream).  Outputs of the posting kernel are complete in stream order, as after any launch.
+Mail ctx_mail(gsb_ctx* ctx);
+int ctx_wait_mail(gsb_ctx* ctx, cudaStream_t stream, const Mail& mail, int n, i64* values, bool* error);
+// The usual end of a call that reports `n` posted values: waits, fills `values`, returns the device error if there is one.
+int ctx_mail_result(gsb_ctx* ctx, cudaStream_t stream, const Mail& mail, int n, i64* values);
 void ctx_count_launches(gsb_ctx* ctx, int n);
 // When profiling is enabled (gsb_profile_enable) these bracket a launch with CUDA events on the
 // launching stream; otherwise they only count the launch.

@@ -2,10 +2,13 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
+#include <chrono>
 #include <new>
 #include <vector>
 
 #include "common.cuh"
+#include "scan.cuh"
 
 struct gsb_ctx {
   int device;
@@ -15,7 +18,9 @@ struct gsb_ctx {
   i64 tile_capacity;
   uint32_t epoch;
   i64* counters;  // device, CNT_NUM entries
-  i64* pinned;    // host pinned, CNT_NUM entries
+  i64* pinned;    // page-locked host memory the device writes: CNT_NUM counters, kMailSlots result words, one ticket
+  u64 mail_tag;   // 1 .. 65535, of the last mailbox handed out
+  u64 ticket;     // of the last counter fetch
   i64 launches;
   char message[512];
   // per-kernel event timing (off by default)
@@ -152,13 +157,86 @@ static int ctx_wait(gsb_ctx* ctx, cudaStream_t stream) {
   return GSB_OK;
 }
 
-int ctx_fetch_counters(gsb_ctx* ctx, cudaStream_t stream, int first, int n, const i64** out) {
-  GSB_CUDA_OK(cudaMemcpyAsync(ctx->pinned + first, ctx->counters + first, sizeof(i64) * (size_t)n,
-                              cudaMemcpyDeviceToHost, stream));
-  {
+// Spins until `*word & mask == want`.  The device normally answers within microseconds; from half a millisecond on the
+// stream's status is asked now and then, so that a failed launch or a stream that finished without writing the word
+// (*answered = false) ends the wait.
+static int ctx_spin(gsb_ctx* ctx, cudaStream_t stream, const volatile u64* word, u64 mask, u64 want, bool* answered) {
+  *answered = true;
+  if (ctx->options[GSB_OPT_BLOCKING_WAIT] != 0) {
     int st = ctx_wait(ctx, stream);
     if (st != GSB_OK) return st;
+    *answered = (*word & mask) == want;
+    return GSB_OK;
   }
+  const auto begin = std::chrono::steady_clock::now();
+  auto next_query = std::chrono::microseconds(500);
+  for (;;) {
+    for (int i = 0; i < 256; ++i) {
+      if ((*word & mask) == want) {
+        std::atomic_thread_fence(std::memory_order_acquire);
+        return GSB_OK;
+      }
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+    }
+    if (std::chrono::steady_clock::now() - begin < next_query) continue;
+    next_query += std::chrono::microseconds(100);
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e == cudaErrorNotReady) continue;
+    GSB_CUDA_OK(e);
+    *answered = (*word & mask) == want;
+    return GSB_OK;
+  }
+}
+
+Mail ctx_mail(gsb_ctx* ctx) {
+  ctx->mail_tag = ctx->mail_tag >= 0xFFFF ? 1 : ctx->mail_tag + 1;
+  return Mail{(u64*)(ctx->pinned + CNT_NUM), ctx->mail_tag << 48};
+}
+
+int ctx_wait_mail(gsb_ctx* ctx, cudaStream_t stream, const Mail& mail, int n, i64* values, bool* error) {
+  *error = false;
+  for (int q = 0; q < n; ++q) {
+    const volatile u64* word = mail.word + q;
+    bool answered;
+    int st = ctx_spin(ctx, stream, word, 0xFFFFull << 48, mail.tag, &answered);
+    if (st != GSB_OK) return st;
+    if (!answered) {  // the stream is done and nothing was posted: only a kernel that gave up does that
+      *error = true;
+      values[q] = 0;
+      continue;
+    }
+    const u64 w = *word;
+    values[q] = (i64)(w & kMailValueMask);
+    *error |= ((w >> kMailErrorBit) & 1ull) != 0;
+  }
+  return GSB_OK;
+}
+
+int ctx_mail_result(gsb_ctx* ctx, cudaStream_t stream, const Mail& mail, int n, i64* values) {
+  bool error;
+  int st = ctx_wait_mail(ctx, stream, mail, n, values, &error);
+  if (st != GSB_OK) return st;
+  return error ? ctx_check_device_error(ctx, stream) : GSB_OK;
+}
+
+// One warp: counters -> page-locked host memory, then the ticket the host spins on.
+__global__ void k_publish_counters(const i64* __restrict__ counters, int first, int n, i64* host, u64 ticket) {
+  for (int q = threadIdx.x; q < n; q += 32) ((volatile i64*)host)[first + q] = ((const volatile i64*)counters)[first + q];
+  __threadfence_system();
+  __syncwarp();
+  if (threadIdx.x == 0) st_volatile_u64((u64*)host + CNT_NUM + kMailSlots, ticket);
+}
+
+int ctx_fetch_counters(gsb_ctx* ctx, cudaStream_t stream, int first, int n, const i64** out) {
+  ctx->ticket += 1;
+  k_publish_counters<<<1, 32, 0, stream>>>(ctx->counters, first, n, ctx->pinned, ctx->ticket);
+  GSB_LAUNCH_OK();
+  bool answered;
+  int st = ctx_spin(ctx, stream, (const volatile u64*)ctx->pinned + CNT_NUM + kMailSlots, ~0ull, ctx->ticket, &answered);
+  if (st != GSB_OK) return st;
+  if (!answered) return GSB_ERR_CUDA;
   *out = ctx->pinned + first;
   return GSB_OK;
 }
@@ -246,8 +324,8 @@ int gsb_ctx_create(int device, gsb_ctx** out_ctx) {
     if ((e = cudaSetDevice(device)) != cudaSuccess) break;
     if ((e = cudaMalloc((void**)&ctx->counters, sizeof(i64) * gsb::CNT_NUM)) != cudaSuccess) break;
     if ((e = cudaMemset(ctx->counters, 0, sizeof(i64) * gsb::CNT_NUM)) != cudaSuccess) break;
-    if ((e = cudaMallocHost((void**)&ctx->pinned, sizeof(i64) * gsb::CNT_NUM)) != cudaSuccess) break;
-    memset(ctx->pinned, 0, sizeof(i64) * gsb::CNT_NUM);
+    if ((e = cudaMallocHost((void**)&ctx->pinned, sizeof(i64) * (gsb::CNT_NUM + gsb::kMailSlots + 1))) != cudaSuccess) break;
+    memset(ctx->pinned, 0, sizeof(i64) * (gsb::CNT_NUM + gsb::kMailSlots + 1));
   } while (0);
   if (e != cudaSuccess) {
     st = gsb::cuda_fail(nullptr, e, __FILE__, __LINE__);

@@ -225,6 +225,8 @@ __global__ void __launch_bounds__(kBThreads, 4) k_direct_compact(BatchLayout L, 
     for (i64 e = L.G - 1; e >= 0 && __ldg(L.item_off + e) == n; --e) out.unique_ptr[e] = total;
     counters[CNT_UNIQUE] = total;
     counters[CNT_NNZ] = L.indices_ptr[L.G];
+    mail_post(out.mail, 0, total, counters);
+    mail_post(out.mail, 1, L.indices_ptr[L.G], counters);
   }
 }
 
@@ -266,7 +268,8 @@ __global__ void __launch_bounds__(kBThreads) k_direct_fixup(BatchLayout L, const
 }
 
 int direct_unique_relabel_launch(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L, const DirectTables& T,
-                                 i64 n_cap, i64 e_cap, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled) {
+                                 i64 n_cap, i64 e_cap, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled,
+                                 Mail mail) {
   i64* counters = ctx_counters(ctx);
   const int wide = kNumSMs * 8;
   const bool hash = T.words == nullptr;  // the regions of L were filled by k_batch_insert; only compaction + fix-up here
@@ -280,7 +283,7 @@ int direct_unique_relabel_launch(gsb_ctx* ctx, cudaStream_t stream, const BatchL
   TileState ts;
   int st = ctx_tile_state(ctx, tiles, stream, &ts);
   if (st != GSB_OK) return st;
-  CompactOut out{out_unique, out_unique_ptr};
+  CompactOut out{out_unique, out_unique_ptr, mail};
   {
     ScopedKernelTimer timer(ctx, KID_FIRST_COMPACT, stream);
     if (hash) k_direct_compact<true><<<tiles, kBThreads, 0, stream>>>(L, T, out, out_relabeled, n_cap, counters, ts);

@@ -588,6 +588,8 @@ __global__ void __launch_bounds__(kPrefixThreads) k_rank_prefix(BatchLayout L, R
     for (i64 e = L.G - 1; e >= 0 && L.item_off[e] == n; --e) out.unique_ptr[e] = all;
     counters[CNT_UNIQUE] = all;
     counters[CNT_NNZ] = L.indices_ptr[L.G];
+    mail_post(out.mail, 0, all, counters);
+    mail_post(out.mail, 1, L.indices_ptr[L.G], counters);
   }
 }
 
@@ -733,7 +735,7 @@ int partition_after_sampler(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i6
 }
 
 int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64 n_cap, i64 bucket_cap, void* ws,
-                             bool counted, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled) {
+                             bool counted, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled, Mail mail) {
   i64* counters = ctx_counters(ctx);
   const PartArrays arrays = carve(L, n_cap, bucket_cap, ws);
   const PartLayout& P = arrays.P;
@@ -776,7 +778,7 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   TileState ts;
   int st = ctx_tile_state(ctx, prefix_tiles, stream, &ts);
   if (st != GSB_OK) return st;
-  CompactOut out{out_unique, out_unique_ptr};
+  CompactOut out{out_unique, out_unique_ptr, mail};
   {
     ScopedKernelTimer timer(ctx, KID_OTHER, stream);
     k_rank_prefix<<<prefix_tiles, kPrefixThreads, 0, stream>>>(L, R, n_cap, out, counters, ts);

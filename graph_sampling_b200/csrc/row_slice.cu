@@ -45,6 +45,7 @@ struct RowFilterParams {
   i64* edge_prefix;     // [E + 1] exclusive prefix of the keep flags (CSC form), may be null
   i64* counters;
   TileState ts;
+  Mail mail;
 };
 
 __global__ void __launch_bounds__(kRowThreads) k_row_filter(RowFilterParams p) {
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(kRowThreads) k_row_filter(RowFilterParams p) {
   if (base + kRowTile >= p.E && threadIdx.x == kRowThreads - 1) {
     if (p.edge_prefix) p.edge_prefix[p.E] = s_base + total;
     p.counters[CNT_NNZ] = s_base + total;
+    mail_post(p.mail, 0, s_base + total, p.counters);
   }
 }
 
@@ -147,6 +149,7 @@ struct ColRowParams {
   float* out_data;
   i64* counters;
   TileState ts;
+  Mail mail;
 };
 
 __global__ void __launch_bounds__(kRowThreads) k_build_batch_row_table(const i64* __restrict__ row_ids, i64 R,
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(kRowThreads) k_col_row_filter(ColRowParams p) 
       }
       if (keep[q]) {
         p.out_indices[out] = value[q];
-        p.out_select[out] = edge[q];
+        if (p.out_select) p.out_select[out] = edge[q];
         if (p.out_data) p.out_data[out] = p.data[p.e_ids ? p.e_ids[edge[q]] : edge[q]];
       }
     }
@@ -307,6 +310,7 @@ __global__ void __launch_bounds__(kRowThreads) k_col_row_filter(ColRowParams p) 
     p.out_indptr[p.S] = total;
     for (i64 e = p.S - 1; e >= 0 && __ldg(p.sub_indptr + e) == p.D; --e) p.out_indptr[e] = total;
     p.counters[CNT_NNZ] = total;
+    mail_post(p.mail, 0, total, p.counters);
   }
 }
 
@@ -345,14 +349,12 @@ static int build_table(gsb_ctx* ctx, cudaStream_t stream, const int64_t* row_ids
   return GSB_OK;
 }
 
-static int finish_count(gsb_ctx* ctx, cudaStream_t stream, int64_t* nnz_host) {
+static int finish_count(gsb_ctx* ctx, cudaStream_t stream, const Mail& mail, int64_t* nnz_host) {
   if (!nnz_host) return GSB_OK;
-  const i64* c;
-  int st = ctx_fetch_counters(ctx, stream, CNT_ERROR, 3, &c);
-  if (st != GSB_OK) return st;
-  *nnz_host = c[CNT_NNZ];
-  if (c[CNT_ERROR] != 0) return ctx_check_device_error(ctx, stream);
-  return GSB_OK;
+  i64 total = 0;
+  const int st = ctx_mail_result(ctx, stream, mail, 1, &total);
+  *nnz_host = total;
+  return st;
 }
 
 extern "C" {
@@ -373,7 +375,8 @@ int gsb_row_slice_csc(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
   TileState ts;
   st = ctx_tile_state(ctx, tiles, stream, &ts);
   if (st != GSB_OK) return st;
-  RowFilterParams p{indices, nullptr, E, table, out_indices, nullptr, out_select, edge_prefix, ctx_counters(ctx), ts};
+  RowFilterParams p{indices, nullptr, E, table, out_indices, nullptr, out_select, edge_prefix, ctx_counters(ctx), ts,
+                    nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0}};
   k_row_filter<<<tiles, kRowThreads, 0, stream>>>(p);
   GSB_LAUNCH_OK();
   const i64 blocks = ((num_cols + 1) * 32 + kRowThreads - 1) / kRowThreads;
@@ -381,7 +384,7 @@ int gsb_row_slice_csc(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
                                                                                  out_indptr, out_coo_col);
   GSB_LAUNCH_OK();
   ctx_count_launches(ctx, 2);
-  return finish_count(ctx, stream, nnz_host);
+  return finish_count(ctx, stream, p.mail, nnz_host);
 }
 
 int gsb_row_slice_coo(gsb_ctx* ctx, void* stream_, const int64_t* coo_row, const int64_t* coo_col, int64_t E,
@@ -399,11 +402,12 @@ int gsb_row_slice_coo(gsb_ctx* ctx, void* stream_, const int64_t* coo_row, const
   TileState ts;
   st = ctx_tile_state(ctx, tiles, stream, &ts);
   if (st != GSB_OK) return st;
-  RowFilterParams p{coo_row, coo_col, E, table, out_row, out_col, out_select, nullptr, ctx_counters(ctx), ts};
+  RowFilterParams p{coo_row, coo_col, E, table, out_row, out_col, out_select, nullptr, ctx_counters(ctx), ts,
+                    nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0}};
   k_row_filter<<<tiles, kRowThreads, 0, stream>>>(p);
   GSB_LAUNCH_OK();
   ctx_count_launches(ctx, 1);
-  return finish_count(ctx, stream, nnz_host);
+  return finish_count(ctx, stream, p.mail, nnz_host);
 }
 
 }  // extern "C"
@@ -444,7 +448,7 @@ int gsb_col_row_slice(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
               GSB_ERR_INVALID_ARGUMENT);
   GSB_REQUIRE((col_ptr == nullptr) == (row_ptr == nullptr) && (!col_ptr || G >= 1), GSB_ERR_INVALID_ARGUMENT);
   GSB_REQUIRE(R == 0 || row_ids, GSB_ERR_INVALID_ARGUMENT);
-  GSB_REQUIRE(D == 0 || (indices && out_indices && out_select), GSB_ERR_INVALID_ARGUMENT);
+  GSB_REQUIRE(D == 0 || (indices && out_indices), GSB_ERR_INVALID_ARGUMENT);
   GSB_REQUIRE(D < ((i64)1 << 40), GSB_ERR_UNSUPPORTED);
   cudaStream_t stream = (cudaStream_t)stream_;
   if (D == 0 || R == 0) {  // nothing can survive
@@ -460,13 +464,14 @@ int gsb_col_row_slice(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
   st = ctx_tile_state(ctx, tiles, stream, &ts);
   if (st != GSB_OK) return st;
   ColRowParams p{indptr, indices, num_cols, column_ids, S, sub_indptr, D, col_ptr, G, encoding_size, table, renumber ? 1 : 0,
-                 out_indptr, out_indices, out_select, data, e_ids, out_data, ctx_counters(ctx), ts};
+                 out_indptr, out_indices, out_select, data, e_ids, out_data, ctx_counters(ctx), ts,
+                 nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0}};
   {
     ScopedKernelTimer timer(ctx, KID_ROW_FILTER, stream);
     k_col_row_filter<<<tiles, kRowThreads, 0, stream>>>(p);
   }
   GSB_LAUNCH_OK();
-  return finish_count(ctx, stream, nnz_host);
+  return finish_count(ctx, stream, p.mail, nnz_host);
 }
 
 int gsb_index_search(gsb_ctx* ctx, void* stream_, const int64_t* origin, int64_t n, const int64_t* keys, int64_t m,

@@ -32,6 +32,16 @@ __device__ __forceinline__ void st_volatile_u64(u64* p, u64 v) {
 
 __device__ __forceinline__ void raise_error(i64* counters, int code, i64 info) {
   if (atomicCAS((u64*)&counters[CNT_ERROR], 0ull, (u64)(i64)code) == 0ull) counters[CNT_ERROR_INFO] = info;
+  __threadfence();  // recorded before anything this thread publishes afterwards (mail_post reads the flag)
+}
+
+// Posts `value` to slot `slot` of a mailbox together with the error flag as it stands.  Called by one thread that knows
+// the final value; errors that can still be raised after that point are found by the next status check, as they are
+// when nobody waits.
+__device__ __forceinline__ void mail_post(const Mail& m, int slot, i64 value, const i64* counters) {
+  if (!m.word) return;
+  const u64 err = ld_volatile_u64((const u64*)counters + CNT_ERROR) != 0ull ? 1ull : 0ull;
+  st_volatile_u64(m.word + slot, m.tag | (err << kMailErrorBit) | ((u64)value & kMailValueMask));
 }
 
 // The two halves of tile_exclusive_prefix, for kernels that have independent work to put between them: a tile first

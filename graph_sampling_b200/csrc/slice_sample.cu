@@ -38,7 +38,8 @@ __device__ __forceinline__ bool column_in_range(i64 col, i64 num_cols, i64* coun
 
 __global__ void __launch_bounds__(kThreads) k_count_scan(const i64* __restrict__ indptr, i64 num_cols,
                                                          const i64* __restrict__ seeds, i64 S, i64 k, int mode,
-                                                         i64* __restrict__ out_indptr, i64* counters, TileState ts) {
+                                                         i64* __restrict__ out_indptr, i64* counters, TileState ts,
+                                                         Mail mail) {
   __shared__ i64 s_scan[33];
   __shared__ i64 s_base;
   const int tile = blockIdx.x;
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(kThreads) k_count_scan(const i64* __restrict__
   if ((i64)(tile + 1) * kThreads >= S && threadIdx.x == 0) {
     out_indptr[S] = tile_base + total;
     counters[CNT_NNZ] = tile_base + total;
+    mail_post(mail, 0, tile_base + total, counters);
   }
 }
 
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(kThreads) k_slice_fill(FillParams p) {
       if (in_pos[r] < 0) continue;
       const i64 pos = tile_base + chunk + r * 32 + lane;
       p.out_indices[pos] = val[r] + (ENCODE ? s_enc[col_of[r]] : 0);
-      p.out_select[pos] = in_pos[r];
+      if (p.out_select) p.out_select[pos] = in_pos[r];
       if (p.out_coo_col) p.out_coo_col[pos] = base + col_of[r];
       if (p.out_data) p.out_data[pos] = p.data[p.e_ids ? p.e_ids[in_pos[r]] : in_pos[r]];
     }
@@ -253,7 +255,7 @@ __global__ void __launch_bounds__(kThreads) k_slice_fill_edges(FillParams p) {
         v += b * p.encoding_size;
       }
       p.out_indices[pos] = v;
-      p.out_select[pos] = in_pos[r];
+      if (p.out_select) p.out_select[pos] = in_pos[r];
       if (p.out_coo_col) p.out_coo_col[pos] = col_of[r];
       if (p.out_data) p.out_data[pos] = p.data[p.e_ids ? p.e_ids[in_pos[r]] : in_pos[r]];
     }
@@ -310,6 +312,7 @@ struct SampleParams {
   // every seed and every sampled id adds one to the count of its bucket.
   uint32_t* bucket_count;
   const i64* bucket_base;  // [G + 1] first bucket of every minibatch
+  Mail mail;               // the edge total, for a caller that waits for it
 };
 
 // Random-stream item of the column at position i of the call.
@@ -320,7 +323,7 @@ __device__ __forceinline__ u64 sample_item(const SampleParams& p, i64 i, i64 bat
 
 __device__ __forceinline__ void emit_pick(const SampleParams& p, i64 out_pos, i64 in_pos, i64 column_pos) {
   p.out_indices[out_pos] = __ldg(p.indices + in_pos);
-  p.out_select[out_pos] = in_pos;
+  if (p.out_select) p.out_select[out_pos] = in_pos;
   if (p.out_coo_col) p.out_coo_col[out_pos] = column_pos;
   if (p.out_data) p.out_data[out_pos] = p.data[p.e_ids ? p.e_ids[in_pos] : in_pos];
 }
@@ -368,10 +371,12 @@ __global__ void __launch_bounds__(kThreads) k_sample_uniform(SampleParams p) {
     p.out_indptr[S] = tile_base + total;
     p.counters[CNT_NNZ] = tile_base + total;
   }
-  if (tile_base + total > p.capacity) {
-    if (tid == 0) raise_error(p.counters, GSB_ERR_CAPACITY, tile_base + total);
-    return;
+  const bool overflow = tile_base + total > p.capacity;  // the prefix only grows: the last tile sees it if any tile does
+  if (tid == 0) {
+    if (overflow) raise_error(p.counters, GSB_ERR_CAPACITY, tile_base + total);
+    if (base + kTileCols >= S) mail_post(p.mail, 0, tile_base + total, p.counters);
   }
+  if (overflow) return;
 
   constexpr int kGroups = kThreads / G;
   const int lane = tid % G;
@@ -411,12 +416,12 @@ __global__ void __launch_bounds__(kThreads) k_sample_uniform(SampleParams p) {
         const i64 m = d - k + j;
         const i64 tj = b + (i64)rand_bounded(p.seed, item, (u64)j, STREAM_UNIFORM, (u64)(m + 1));
         bool dup = false;
-        for (i64 q = lane; q < j; q += G) dup |= (p.out_select[o + q] == tj);
+        for (i64 q = lane; q < j; q += G) dup |= (p.out_indices[o + q] == tj);
         const unsigned any = __ballot_sync(gmask, dup);
-        if (lane == 0) p.out_select[o + j] = any ? (b + m) : tj;
+        if (lane == 0) p.out_indices[o + j] = any ? (b + m) : tj;
         __syncwarp(gmask);
       }
-      for (i64 j = lane; j < k; j += G) emit_pick(p, o + j, p.out_select[o + j], col_pos);
+      for (i64 j = lane; j < k; j += G) emit_pick(p, o + j, p.out_indices[o + j], col_pos);
     }
   }
 }
@@ -474,11 +479,11 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     if (lane >= o) inc += t;
   }
   const i64 total = __shfl_sync(0xffffffffu, inc, 31);
+  const bool too_long = valid && d > 0xFFFFFFFFll;   // positions inside a column are drawn from one 32-bit word
+  if (too_long) raise_error(p.counters, GSB_ERR_UNSUPPORTED, i);
   // The tile's count is published at once; its own prefix is resolved only after the picks are drawn and the gathers
   // issued, so the wait for the predecessors' counts overlaps the k random loads of every lane.
   tile_publish_aggregate(p.ts, (int)tile, total);
-  const bool too_long = valid && d > 0xFFFFFFFFll;   // positions inside a column are drawn from one 32-bit word
-  if (too_long) raise_error(p.counters, GSB_ERR_UNSUPPORTED, i);
   const int n = valid && !too_long ? (int)f : 0;
   // minibatch of the warp's first column by one search; a lane beyond that minibatch's end searches for itself
   i64 bt = 0;
@@ -531,18 +536,19 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     p.out_indptr[0] = 0;
     p.counters[CNT_NNZ] = 0;
   }
-  const bool overflow = prefix + total > p.capacity;
-  if (overflow) {
-    if (lane == 0) raise_error(p.counters, GSB_ERR_CAPACITY, prefix + total);
-    if (!COUNT) return;
+  const bool overflow = prefix + total > p.capacity;  // the prefix only grows: the last tile sees it if any tile does
+  if (lane == 0) {
+    if (overflow) raise_error(p.counters, GSB_ERR_CAPACITY, prefix + total);
+    if (tile * 32 + 32 >= S) mail_post(p.mail, 0, prefix + total, p.counters);
   }
+  if (overflow && !COUNT) return;
   if (!overflow) {
 #pragma unroll
     for (int j = 0; j < KMAX; ++j) {
       if (j < n) {
         const i64 in_pos = b + pick[j];
         p.out_indices[o + j] = val[j];
-        p.out_select[o + j] = in_pos;
+        if (p.out_select) p.out_select[o + j] = in_pos;
         if (p.out_coo_col) p.out_coo_col[o + j] = i;
         if (p.out_data) p.out_data[o + j] = p.data[p.e_ids ? p.e_ids[in_pos] : in_pos];
       }
@@ -601,14 +607,14 @@ __global__ void __launch_bounds__(kThreads) k_sample_one_keepdim(const i64* __re
 // Offsets of a per-column sample (min(degree, k) without replacement, k per non-empty column with) or of the plain
 // slice (mode 0) by the counting kernel alone; the total lands in the context's counters.
 int count_scan_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, i64 num_cols, const i64* seeds, i64 S, i64 k,
-                      int mode, i64* out_indptr) {
+                      int mode, i64* out_indptr, Mail mail) {
   const int grid = grid_for(S, kThreads);
   TileState ts;
   int st = ctx_tile_state(ctx, grid, stream, &ts);
   if (st != GSB_OK) return st;
   {
     ScopedKernelTimer timer(ctx, KID_COUNT_SCAN, stream);
-    k_count_scan<<<grid, kThreads, 0, stream>>>(indptr, num_cols, seeds, S, k, mode, out_indptr, ctx_counters(ctx), ts);
+    k_count_scan<<<grid, kThreads, 0, stream>>>(indptr, num_cols, seeds, S, k, mode, out_indptr, ctx_counters(ctx), ts, mail);
   }
   GSB_LAUNCH_OK();
   return GSB_OK;
@@ -624,7 +630,7 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
                           const i64* seeds, i64 S, i64 k, int replace, u64 seed, i64* out_indptr, i64* out_indices,
                           i64* out_select, i64* out_coo_col, const float* data, const i64* e_ids, float* out_data,
                           i64 capacity, const i64* S_dev, const i64* batch_ptr, const i64* batch_ids, i64 G,
-                          const SamplerCount* count) {
+                          const SamplerCount* count, Mail mail) {
   const bool per_thread = k <= 16;  // small fanouts: one lane per column, one warp per tile of 32 columns
   const int grid = per_thread ? grid_for(S, kTpcThreads) : grid_for(S, kTileCols);
   TileState ts;
@@ -633,7 +639,7 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
   SampleParams p{indptr,     indices,     num_cols, seeds, S,        k,        replace,           seed, out_indptr,
                  out_indices, out_select, out_coo_col, data, e_ids, out_data, capacity, ctx_counters(ctx), ts,
                  S_dev,      batch_ptr,  batch_ptr ? batch_ids : nullptr,
-                 batch_ptr ? G : 0,      nullptr,    nullptr};
+                 batch_ptr ? G : 0,      nullptr,    nullptr, mail};
   if (count && count->bucket_count) {
     if (!per_thread || !batch_ptr || G < 1) return GSB_ERR_INVALID_ARGUMENT;
     p.bucket_count = count->bucket_count;
@@ -675,35 +681,24 @@ int gsb_col_slice_count(gsb_ctx* ctx, void* stream_, const int64_t* indptr, int6
   GSB_ENTER(ctx);
   GSB_REQUIRE(indptr && out_indptr && S >= 0 && num_cols >= 0 && (seeds || S <= num_cols), GSB_ERR_INVALID_ARGUMENT);
   cudaStream_t stream = (cudaStream_t)stream_;
-  const int grid = grid_for(S, kThreads);
-  TileState ts;
-  int st = ctx_tile_state(ctx, grid, stream, &ts);
-  if (st != GSB_OK) return st;
-  {
-    ScopedKernelTimer timer(ctx, KID_COUNT_SCAN, stream);
-    k_count_scan<<<grid, kThreads, 0, stream>>>(indptr, num_cols, seeds, S, 0, COUNT_DEGREE, out_indptr,
-                                                ctx_counters(ctx), ts);
-  }
-  GSB_LAUNCH_OK();
-  if (nnz_host) {
-    const i64* c;
-    st = ctx_fetch_counters(ctx, stream, CNT_ERROR, 3, &c);
-    if (st != GSB_OK) return st;
-    *nnz_host = c[CNT_NNZ];
-    if (c[CNT_ERROR] != 0) return ctx_check_device_error(ctx, stream);
-  }
-  return GSB_OK;
+  const Mail mail = nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0};
+  int st = count_scan_launch(ctx, stream, indptr, num_cols, seeds, S, 0, COUNT_DEGREE, out_indptr, mail);
+  if (st != GSB_OK || !nnz_host) return st;
+  i64 total = 0;
+  st = ctx_mail_result(ctx, stream, mail, 1, &total);
+  *nnz_host = total;
+  return st;
 }
 
 int gsb_col_slice_fill(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64_t* indices, int64_t num_cols,
                        const int64_t* seeds, int64_t S, const int64_t* out_indptr, int64_t D, int64_t* out_indices,
                        int64_t* out_select, int64_t* out_coo_col, const float* data, const int64_t* e_ids,
                        float* out_data) {
-  // out_indices / out_select may be null only when the slice is empty (nothing is written then)
+  // out_indices may be null only when the slice is empty (nothing is written then)
   GSB_ENTER(ctx);
   GSB_REQUIRE(indptr && out_indptr && S >= 0 && num_cols >= 0 && (seeds || S <= num_cols), GSB_ERR_INVALID_ARGUMENT);
   if (S == 0 || D == 0) return GSB_OK;
-  GSB_REQUIRE(indices && out_indices && out_select, GSB_ERR_INVALID_ARGUMENT);
+  GSB_REQUIRE(indices && out_indices, GSB_ERR_INVALID_ARGUMENT);
   FillParams p{indptr, indices, num_cols, seeds, S, out_indptr, out_indices, out_select, out_coo_col, data, e_ids,
                out_data, nullptr, 0, 0, false};
   {
@@ -747,19 +742,17 @@ int gsb_sample_uniform(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const
   GSB_ENTER(ctx);
   GSB_REQUIRE(indptr && out_indptr && S >= 0 && k >= 0 && num_cols >= 0 && (seeds || S <= num_cols),
               GSB_ERR_INVALID_ARGUMENT);
-  GSB_REQUIRE((out_indices && out_select) || capacity == 0, GSB_ERR_INVALID_ARGUMENT);
+  GSB_REQUIRE(out_indices || capacity == 0, GSB_ERR_INVALID_ARGUMENT);
   cudaStream_t stream = (cudaStream_t)stream_;
+  const Mail mail = nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0};
   int st = sample_uniform_launch(ctx, stream, indptr, indices, num_cols, seeds, S, k, replace, (u64)seed, out_indptr,
-                                 out_indices, out_select, out_coo_col, data, e_ids, out_data, capacity);
-  if (st != GSB_OK) return st;
-  if (nnz_host) {
-    const i64* c;
-    st = ctx_fetch_counters(ctx, stream, CNT_ERROR, 3, &c);
-    if (st != GSB_OK) return st;
-    *nnz_host = c[CNT_NNZ];
-    if (c[CNT_ERROR] != 0) return ctx_check_device_error(ctx, stream);
-  }
-  return GSB_OK;
+                                 out_indices, out_select, out_coo_col, data, e_ids, out_data, capacity, nullptr, nullptr,
+                                 nullptr, 0, nullptr, mail);
+  if (st != GSB_OK || !nnz_host) return st;
+  i64 total = 0;
+  st = ctx_mail_result(ctx, stream, mail, 1, &total);
+  *nnz_host = total;
+  return st;
 }
 
 int gsb_sample_one_keepdim(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64_t* indices,

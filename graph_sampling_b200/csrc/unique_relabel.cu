@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kThreads) k_insert(Segments items, Table table
 }
 
 __global__ void __launch_bounds__(kThreads) k_first_compact(Segments items, Table table, i64* __restrict__ out_unique,
-                                                            i64* counters, TileState ts) {
+                                                            i64* counters, TileState ts, Mail mail) {
   __shared__ i64 s_scan[33];
   __shared__ i64 s_base;
   const i64 n = items.start[items.n];
@@ -107,7 +107,10 @@ __global__ void __launch_bounds__(kThreads) k_first_compact(Segments items, Tabl
       ++pos;
     }
   }
-  if (base + kTileItems >= n && threadIdx.x == 0) counters[CNT_UNIQUE] = s_base + total;
+  if (base + kTileItems >= n && threadIdx.x == 0) {
+    counters[CNT_UNIQUE] = s_base + total;
+    mail_post(mail, 0, s_base + total, counters);
+  }
 }
 
 __global__ void __launch_bounds__(kThreads) k_relabel(Segments rel, Table table) {
@@ -204,6 +207,7 @@ extern "C" int gsb_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* co
   st = ctx_tile_state(ctx, tiles, stream, &ts);
   if (st != GSB_OK) return st;
   const int sm_grid = kNumSMs * 8;
+  const Mail mail = unique_host ? ctx_mail(ctx) : Mail{nullptr, 0};
   if (n > 0) {
     ScopedKernelTimer timer(ctx, KID_TABLE_INSERT, stream);
     k_insert<<<min(grid_for(n, kThreads), sm_grid), kThreads, 0, stream>>>(items, table, ctx_counters(ctx));
@@ -211,7 +215,7 @@ extern "C" int gsb_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* co
   GSB_LAUNCH_OK();
   {
     ScopedKernelTimer timer(ctx, KID_FIRST_COMPACT, stream);
-    k_first_compact<<<tiles, kThreads, 0, stream>>>(items, table, out_unique, ctx_counters(ctx), ts);
+    k_first_compact<<<tiles, kThreads, 0, stream>>>(items, table, out_unique, ctx_counters(ctx), ts, mail);
   }
   GSB_LAUNCH_OK();
   if (m > 0) {
@@ -219,14 +223,11 @@ extern "C" int gsb_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* co
     k_relabel<<<min(grid_for(m, kThreads), sm_grid), kThreads, 0, stream>>>(rel, table);
   }
   GSB_LAUNCH_OK();
-  if (unique_host) {
-    const i64* c;
-    st = ctx_fetch_counters(ctx, stream, CNT_ERROR, 4, &c);
-    if (st != GSB_OK) return st;
-    *unique_host = c[CNT_UNIQUE];
-    if (c[CNT_ERROR] != 0) return ctx_check_device_error(ctx, stream);
-  }
-  return GSB_OK;
+  if (!unique_host) return GSB_OK;
+  i64 unique = 0;
+  st = ctx_mail_result(ctx, stream, mail, 1, &unique);
+  *unique_host = unique;
+  return st;
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -332,7 +333,8 @@ extern "C" int gsb_unique_relabel_static(void* stream_, const int64_t* items, in
   TileState ts{sc->tile_words, 1u, sc->counters};
   const int sm_grid = kNumSMs * 8;
   if (n > 0) k_insert<<<min(grid_for(n, kThreads), sm_grid), kThreads, 0, stream>>>(seg_items, table, sc->counters);
-  k_first_compact<<<grid_for(n, kTileItems), kThreads, 0, stream>>>(seg_items, table, out_unique, sc->counters, ts);
+  k_first_compact<<<grid_for(n, kTileItems), kThreads, 0, stream>>>(seg_items, table, out_unique, sc->counters, ts,
+                                                                 Mail{nullptr, 0});
   if (m > 0) k_relabel<<<min(grid_for(m, kThreads), sm_grid), kThreads, 0, stream>>>(seg_rel, table);
   if (cudaGetLastError() != cudaSuccess) return GSB_ERR_CUDA;
   // results stay on the device: [0] = number of distinct ids, [1] = first device-side error code (0 = none)

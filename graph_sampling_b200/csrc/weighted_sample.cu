@@ -49,6 +49,7 @@ struct WeightedParams {
   i64 capacity;
   i64* counters;
   TileState ts;
+  Mail mail;  // the edge total, for a caller that waits for it
 };
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
@@ -64,7 +65,7 @@ __device__ __forceinline__ bool ranks_before(float ka, u32 ia, float kb, u32 ib)
 
 __device__ __forceinline__ void emit_weighted(const WeightedParams& p, i64 out_pos, i64 in_pos, i64 col_pos) {
   p.out_indices[out_pos] = __ldg(p.indices + in_pos);
-  p.out_select[out_pos] = in_pos;
+  if (p.out_select) p.out_select[out_pos] = in_pos;
   if (p.out_coo_col) p.out_coo_col[out_pos] = col_pos;
   if (p.out_data) p.out_data[out_pos] = p.data[p.e_ids ? p.e_ids[in_pos] : in_pos];
 }
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(kWThreads, 6) k_sample_weighted(WeightedParams
     }
     f = p.replace ? (d > 0 ? k : 0) : (d < k ? d : k);
     is_long = !p.replace && d > kLongColumn && d > k;
+    if (is_long && d > (i64)kMaxScanEnd) raise_error(p.counters, GSB_ERR_UNSUPPORTED, d);  // positions are 32-bit here
     s_in[tid] = b;
     s_deg[tid] = d;
   }
@@ -247,10 +249,12 @@ __global__ void __launch_bounds__(kWThreads, 6) k_sample_weighted(WeightedParams
     p.out_indptr[S] = tile_base + total;
     p.counters[CNT_NNZ] = tile_base + total;
   }
-  if (tile_base + total > p.capacity) {
-    if (tid == 0) raise_error(p.counters, GSB_ERR_CAPACITY, tile_base + total);
-    return;
+  const bool overflow = tile_base + total > p.capacity;  // the prefix only grows: the last tile sees it if any tile does
+  if (tid == 0) {
+    if (overflow) raise_error(p.counters, GSB_ERR_CAPACITY, tile_base + total);
+    if (base + kWTileCols >= S) mail_post(p.mail, 0, tile_base + total, p.counters);
   }
+  if (overflow) return;
 
   const int lane = tid & 31, warp = tid >> 5;
   constexpr int kWarps = kWThreads / 32;
@@ -265,10 +269,7 @@ __global__ void __launch_bounds__(kWThreads, 6) k_sample_weighted(WeightedParams
     for (int c = 0; c < ncol; ++c) {
       const i64 d = s_deg[c];
       if (d <= kLongColumn || d <= k) continue;  // uniform across the CTA
-      if (d > (i64)kMaxScanEnd) {                // positions inside a column are 32-bit here
-        if (tid == 0) raise_error(p.counters, GSB_ERR_UNSUPPORTED, d);
-        continue;
-      }
+      if (d > (i64)kMaxScanEnd) continue;
       const i64 b = s_in[c], o = tile_base + s_off[c], col_pos = base + c;
       const i64 chunk = (((d + kWarps - 1) / kWarps) + 31) & ~(i64)31;
       const i64 e_begin = min(d, (i64)warp * chunk), e_end = min(d, (i64)(warp + 1) * chunk);
@@ -467,14 +468,14 @@ extern "C" int gsb_sample_weighted(gsb_ctx* ctx, void* stream_, const int64_t* i
   GSB_ENTER(ctx);
   GSB_REQUIRE(indptr && out_indptr && S >= 0 && k >= 0 && num_cols >= 0 && (seeds || S <= num_cols),
               GSB_ERR_INVALID_ARGUMENT);
-  GSB_REQUIRE((out_indices && out_select) || capacity == 0, GSB_ERR_INVALID_ARGUMENT);
+  GSB_REQUIRE(out_indices || capacity == 0, GSB_ERR_INVALID_ARGUMENT);
   GSB_REQUIRE(replace || k <= kWideMaxK, GSB_ERR_UNSUPPORTED);
   cudaStream_t stream = (cudaStream_t)stream_;
   if (!replace && k > 32) {
     int st = count_scan_launch(ctx, stream, indptr, num_cols, seeds, S, k, /*without replacement*/ 1, out_indptr);
     if (st != GSB_OK) return st;
     WeightedParams p{indptr, indices,    probs, num_cols,      seeds, S,     k,        replace,  (u64)seed,         out_indptr,
-                     out_indices, out_select, out_coo_col, data,  e_ids, out_data, capacity, ctx_counters(ctx), TileState{}};
+                     out_indices, out_select, out_coo_col, data,  e_ids, out_data, capacity, ctx_counters(ctx), TileState{}, Mail{nullptr, 0}};
     if (S > 0) {
       ScopedKernelTimer timer(ctx, KID_SAMPLE_WEIGHTED, stream);
       k_sample_weighted_wide<<<(int)min(S, (i64)kNumSMs * 8), kWideThreads, 0, stream>>>(p);
@@ -495,7 +496,8 @@ extern "C" int gsb_sample_weighted(gsb_ctx* ctx, void* stream_, const int64_t* i
   int st = ctx_tile_state(ctx, grid, stream, &ts);
   if (st != GSB_OK) return st;
   WeightedParams p{indptr, indices,    probs, num_cols,      seeds, S,     k,        replace,  (u64)seed,         out_indptr,
-                   out_indices, out_select, out_coo_col, data,  e_ids, out_data, capacity, ctx_counters(ctx), ts};
+                   out_indices, out_select, out_coo_col, data,  e_ids, out_data, capacity, ctx_counters(ctx), ts,
+                   nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0}};
   {
     ScopedKernelTimer timer(ctx, KID_SAMPLE_WEIGHTED, stream);
     if (narrow)
@@ -504,12 +506,9 @@ extern "C" int gsb_sample_weighted(gsb_ctx* ctx, void* stream_, const int64_t* i
       k_sample_weighted<kWTileColsWide><<<grid, kWThreads, 0, stream>>>(p);
   }
   GSB_LAUNCH_OK();
-  if (nnz_host) {
-    const i64* c;
-    st = ctx_fetch_counters(ctx, stream, CNT_ERROR, 3, &c);
-    if (st != GSB_OK) return st;
-    *nnz_host = c[CNT_NNZ];
-    if (c[CNT_ERROR] != 0) return ctx_check_device_error(ctx, stream);
-  }
-  return GSB_OK;
+  if (!nnz_host) return GSB_OK;
+  i64 total = 0;
+  st = ctx_mail_result(ctx, stream, p.mail, 1, &total);
+  *nnz_host = total;
+  return st;
 }

@@ -13,6 +13,9 @@
  *  - the return value is a status code (0 = GSB_OK); nothing aborts the process (the reference
  *    LOG(FATAL)s: src/cuda/cuda_common.h:15-28);
  *  - inputs are borrowed and never modified; outputs are caller-allocated;
+ *  - out_select of the column slices, the per-column samplers and gsb_col_row_slice is optional (NULL: not written);
+ *  - a call that reports a size to the host returns as soon as the size is known, which may be a little before its last
+ *    kernel has finished: outputs are complete in stream order, as after any launch;
  *  - a gsb_ctx owns scratch memory and device-side counters for ONE stream of work at a time:
  *    calls sharing a context must be ordered on one stream (use one context per stream/thread).
  *    Scratch grows on demand with cudaMalloc the first time a size is seen (this synchronises the

@@ -1,6 +1,7 @@
-"""Builds the sm_100a kernel library (graph_sampling_b200/lib/libgsb200.so) with nvcc.
+"""Builds the sm_100a kernel library (graph_sampling_b200/lib/libgsb200.so) with nvcc, and the extension module that
+graph_sampling_b200.ops calls it through (lib/_gsb_native.so) with g++.
 
-    python -m graph_sampling_b200.build [--force] [--verbose]
+    python -m graph_sampling_b200.build [--force] [--verbose] [--glue]
 
 The library has no torch dependency: it is plain CUDA C++ behind the C ABI of include/gsb200.h.
 nvcc cross-compiles for sm_100a, so this also runs on a machine without a GPU.
@@ -60,30 +61,42 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 GLUE_SRC = os.path.join(CSRC, "glue", "gs_glue.cc")
 GLUE_LIB = os.path.join(LIBDIR, "libgs.so")
+NATIVE_SRC = os.path.join(CSRC, "glue", "gs_native.cc")
+NATIVE_LIB = os.path.join(LIBDIR, "_gsb_native.so")
 
 
-def build_glue(force: bool = False) -> str:
-    """Builds lib/libgs.so: the TorchScript front end (gs_classes.Graph, gs_ops.*) over the C ABI.  Needs the
-    torch headers; links against libgsb200.so (found next to it through $ORIGIN) and torch."""
+def _build_against_torch(src, lib, extra_libs, force):
+    """g++ over the C ABI and the torch headers; links against libgsb200.so (found next to it through $ORIGIN)."""
     build(force=False)
-    deps = [GLUE_SRC, os.path.join(os.path.dirname(PKG), "include", "gsb200.h")]
-    if not force and os.path.exists(GLUE_LIB) and all(os.path.getmtime(GLUE_LIB) >= os.path.getmtime(d) for d in deps):
-        return GLUE_LIB
+    deps = [src, os.path.join(os.path.dirname(PKG), "include", "gsb200.h")]
+    if not force and os.path.exists(lib) and all(os.path.getmtime(lib) >= os.path.getmtime(d) for d in deps):
+        return lib
     import sysconfig
     import torch
     tdir = os.path.dirname(torch.__file__)
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}", "-w",
            "-I", os.path.join(tdir, "include"), "-I", os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
-           "-I", sysconfig.get_paths()["include"], "-I", "/usr/local/cuda/include", GLUE_SRC, "-o", GLUE_LIB,
-           "-L", LIBDIR, "-lgsb200", "-Wl,-rpath,$ORIGIN", "-L", os.path.join(tdir, "lib"), "-ltorch", "-ltorch_cpu",
-           "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath," + os.path.join(tdir, "lib"),
+           "-I", sysconfig.get_paths()["include"], "-I", "/usr/local/cuda/include", src, "-o", lib,
+           "-L", LIBDIR, "-lgsb200", "-Wl,-rpath,$ORIGIN", "-L", os.path.join(tdir, "lib"), *extra_libs, "-ltorch",
+           "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath," + os.path.join(tdir, "lib"),
            "-L", "/usr/local/cuda/lib64", "-lcudart"]
     subprocess.check_call(cmd)
-    return GLUE_LIB
+    return lib
+
+
+def build_glue(force: bool = False) -> str:
+    """Builds lib/libgs.so: the TorchScript front end (gs_classes.Graph, gs_ops.*)."""
+    return _build_against_torch(GLUE_SRC, GLUE_LIB, [], force)
+
+
+def build_native(force: bool = False) -> str:
+    """Builds lib/_gsb_native.so: the extension module behind graph_sampling_b200.ops."""
+    return _build_against_torch(NATIVE_SRC, NATIVE_LIB, ["-ltorch_python"], force)
 
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    print(build_native(force="--force" in sys.argv))
     if "--glue" in sys.argv:
         print(build_glue(force="--force" in sys.argv))

@@ -232,13 +232,10 @@ class Graph:
         id that has no edges is absent from val_ids and yields an empty segment."""
         pos = ops.index_search(val_ids, n_ids)
         present = torch.nonzero(pos >= 0).reshape(-1)
-        r = ops.csc_col_slicing(fmt.indptr, fmt.indices, pos[present].contiguous(), with_coo, data=data, e_ids=e_ids)
+        r = ops.col_slice(fmt.indptr, fmt.indices, pos[present].contiguous(), with_coo, data=data, e_ids=e_ids)
         counts = torch.zeros(n_ids.numel() + 1, dtype=torch.int64, device=n_ids.device)
         counts[present + 1] = r[0][1:] - r[0][:-1]
-        out = [torch.cumsum(counts, 0), present[r[1]] if with_coo else None, r[2], r[3]]
-        if data is not None:
-            out.append(r[4])
-        return out
+        return torch.cumsum(counts, 0), present[r[1]] if with_coo else None, r[2], r[3]
 
     # ---- helpers -----------------------------------------------------------------------------------------
     def _child(self, col_ids, row_ids, num_cols, num_rows):
@@ -285,10 +282,8 @@ class Graph:
                 if self.val_col_ids_ is not None:
                     r = self._compact_col_slicing(self.csc_, self.val_col_ids_, n_ids, with_coo, data, e_ids)
                 else:
-                    r = ops.csc_col_slicing(self.csc_.indptr, self.csc_.indices, n_ids, with_coo, data=data,
-                                            e_ids=e_ids)
-                indptr, coo_col, indices = r[0], r[1], r[2]
-                out_data = r[4] if data is not None else None
+                    r = ops.col_slice(self.csc_.indptr, self.csc_.indices, n_ids, with_coo, data=data, e_ids=e_ids)
+                indptr, coo_col, indices, out_data = r
                 if relabel:
                     frontier, (indices,) = ops.relabel([indices], [indices])
                     new_row_ids, new_num_rows = frontier, frontier.numel()
@@ -323,10 +318,8 @@ class Graph:
                 if self.val_row_ids_ is not None:
                     r = self._compact_col_slicing(self.csr_, self.val_row_ids_, n_ids, with_coo, data, e_ids)
                 else:
-                    r = ops.csc_col_slicing(self.csr_.indptr, self.csr_.indices, n_ids, with_coo, data=data,
-                                            e_ids=e_ids)
-                indptr, coo_row, indices = r[0], r[1], r[2]
-                out_data = r[4] if data is not None else None
+                    r = ops.col_slice(self.csr_.indptr, self.csr_.indices, n_ids, with_coo, data=data, e_ids=e_ids)
+                indptr, coo_row, indices, out_data = r
                 if relabel:
                     frontier, (indices,) = ops.relabel([indices], [indices])
                     new_col_ids, new_num_cols = frontier, frontier.numel()
@@ -393,12 +386,12 @@ class Graph:
         col_ids = self.col_ids_[column_seeds] if self.col_ids_ is not None else column_seeds
         row_ids = self.row_ids_[row_seeds] if self.row_ids_ is not None else row_seeds
         data, e_ids = self._gather_args(self.csc_)
-        r = ops.csc_col_row_slicing(self.csc_.indptr, self.csc_.indices, col_ids, row_ids, data=data, e_ids=e_ids)
+        r = ops.col_row_slice(self.csc_.indptr, self.csc_.indices, col_ids, row_ids, data=data, e_ids=e_ids)
         ret = self._child(col_ids, row_ids, column_seeds.numel(), row_seeds.numel())
         ret.csc_ = CSC(r[0], r[1])
         ret.num_edges_ = r[1].numel()
         if data is not None:
-            ret.data_ = r[3]
+            ret.data_ = r[2]
         return ret
 
     def BatchFusedBidirSlicing(self, column_seeds, col_ptr, row_seeds, row_ptr):
@@ -406,13 +399,13 @@ class Graph:
         self.CreateSparseFormat(_CSC)
         col_ids = self.col_ids_[column_seeds] if self.col_ids_ is not None else column_seeds
         data, e_ids = self._gather_args(self.csc_)
-        r = ops.csc_col_row_slicing(self.csc_.indptr, self.csc_.indices, col_ids, row_seeds, col_ptr, row_ptr,
-                                    self.num_rows_, data=data, e_ids=e_ids)
+        r = ops.col_row_slice(self.csc_.indptr, self.csc_.indices, col_ids, row_seeds, col_ptr, row_ptr,
+                              self.num_rows_, data=data, e_ids=e_ids)
         ret = self._child(col_ids, self.row_ids_, column_seeds.numel(), self.num_rows_)
         ret.csc_ = CSC(r[0], r[1])
         ret.num_edges_ = r[1].numel()
         if data is not None:
-            ret.data_ = r[3]
+            ret.data_ = r[2]
         return ret
 
     def EDivUSum(self, divisor):
@@ -465,13 +458,10 @@ class Graph:
         else:
             _fatal("No implementation!")
         data, e_ids = self._gather_args(fmt)
-        if probs is None:
-            r = ops.csc_col_sampling(fmt.indptr, fmt.indices, fanout, replace, with_coo, seed=seed, data=data,
-                                     e_ids=e_ids)
-        else:
-            r = ops.csc_col_sampling_probs(fmt.indptr, fmt.indices, probs, fanout, replace, with_coo, seed=seed,
-                                           data=data, e_ids=e_ids)
-        indptr, coo_other, indices = r[0], r[1], r[2]
+        if probs is not None and probs.numel() != fmt.indices.numel():
+            raise ValueError("probs must have one entry per edge of the operand")
+        indptr, coo_other, indices, out_data = ops.col_sample(fmt.indptr, fmt.indices, None, fanout, replace, with_coo,
+                                                              probs=probs, seed=seed, data=data, e_ids=e_ids)
         if axis == 0:
             if output_format & _CSC:
                 ret.csc_ = CSC(indptr, indices)
@@ -484,7 +474,7 @@ class Graph:
                 ret.coo_ = COO(coo_other, indices, None, True, False)
         ret.num_edges_ = indices.numel()
         if data is not None:
-            ret.data_ = r[4]
+            ret.data_ = out_data
         return ret
 
     def Sampling(self, axis, fanout, replace, on_format, output_format, seed=None):
@@ -509,10 +499,8 @@ class Graph:
                 safe = select.clamp(min=0)
                 out_data = ops.take(data, ops.take(e_ids, safe) if e_ids is not None else safe)
         else:
-            r = ops.fused_csc_col_slicing_sampling(csc.indptr, csc.indices, column_index, fanout, replace, seed=seed,
-                                                   data=data, e_ids=e_ids)
-            indptr, indices = r[0], r[1]
-            out_data = r[3] if data is not None else None
+            indptr, _, indices, out_data = ops.col_sample(csc.indptr, csc.indices, column_index, fanout, replace, False,
+                                                          seed=seed, data=data, e_ids=e_ids)
         ret.csc_ = CSC(indptr, indices)
         ret.num_edges_ = indices.numel()
         if out_data is not None:

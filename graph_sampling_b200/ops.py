@@ -8,12 +8,34 @@ else raises (the reference instantiates only those types and aborts otherwise).
 """
 import ctypes
 
+import importlib.machinery
+import importlib.util
+import os
+
 import torch
 
 from . import cabi
 from .cabi import GsbError, c_i64, c_i64p, c_int, c_u64, c_vp
 
 _contexts = {}
+_native = None
+
+
+def _load_native():
+    """The extension module that does an operator's host work (csrc/glue/gs_native.cc).  As strict as cabi.load: there
+    is no Python form of these operators to fall back to."""
+    global _native
+    if _native is None:
+        path = os.path.join(os.path.dirname(cabi.LIB_PATH), "_gsb_native.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} not found: run `python -m graph_sampling_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_gsb_native", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_gsb_native", loader))
+        loader.exec_module(module)
+        module.set_error_class(GsbError)
+        _native = module
+    return _native
+
 _seed_state = {"base": 7777, "counter": 0, "auto_advance": True}
 
 
@@ -51,11 +73,13 @@ class Context:
         if st != 0:
             raise GsbError(st, "gsb_ctx_create")
         self.handle = h
+        self.address = h.value          # what the functions of `native` take as their first argument
+        self.native = _load_native()
 
     def close(self):
         if getattr(self, "handle", None):
             self.lib.gsb_ctx_destroy(self.handle)
-            self.handle = None
+            self.handle = self.address = None
 
     def __del__(self):
         try:
@@ -123,6 +147,15 @@ def default_context(device=None):
     return ctx
 
 
+def _context_for(t, ctx=None):
+    """`ctx`, or the default context of the device that holds `t`."""
+    if ctx is not None:
+        return ctx
+    if isinstance(t, torch.Tensor):
+        return _contexts.get(t.get_device()) or default_context(t.device)
+    return default_context()
+
+
 def _stream():
     return c_vp(torch.cuda.current_stream().cuda_stream)
 
@@ -176,65 +209,47 @@ def _empty(n, like, dtype=torch.int64):
 def csc_col_slicing(indptr, indices, column_ids, with_coo=True, data=None, e_ids=None, ctx=None):
     """CSCColSlicingCUDA (src/cuda/slicing.cu:170-182) → (sub_indptr, coo_col | None, sub_indices,
     select_index[, sliced_data]).  `column_ids=None` slices every column."""
-    indptr, indices = _i64(indptr, "indptr"), _i64(indices, "indices")
-    column_ids = _i64(column_ids, "column_ids", allow_none=True)
-    data, e_ids = _f32(data, "data", True), _i64(e_ids, "e_ids", True)
-    ctx = ctx or default_context(indptr.device)
-    lib = ctx.lib
-    S = column_ids.numel() if column_ids is not None else indptr.numel() - 1
-    sub_indptr = _empty(S + 1, indptr)
-    nnz = c_i64(0)
-    num_cols = indptr.numel() - 1
-    ctx.check(lib.gsb_col_slice_count(ctx.handle, _stream(), _p(indptr), c_i64(num_cols), _p(column_ids), c_i64(S),
-                                      _p(sub_indptr), ctypes.byref(nnz)), "gsb_col_slice_count")
-    n = nnz.value
-    sub_indices, select = _empty(n, indptr), _empty(n, indptr)
-    coo_col = _empty(n, indptr) if with_coo else None
-    out_data = _empty(n, indptr, torch.float32) if data is not None else None
-    ctx.check(lib.gsb_col_slice_fill(ctx.handle, _stream(), _p(indptr), _p(indices), c_i64(num_cols), _p(column_ids),
-                                     c_i64(S), _p(sub_indptr), c_i64(n), _p(sub_indices), _p(select), _p(coo_col),
-                                     _p(data), _p(e_ids), _p(out_data)), "gsb_col_slice_fill")
-    if data is not None:
-        return sub_indptr, coo_col, sub_indices, select, out_data
-    return sub_indptr, coo_col, sub_indices, select
+    ctx = _context_for(indptr, ctx)
+    out = ctx.native.col_slicing(ctx.address, indptr, indices, column_ids, with_coo, True, data, e_ids)
+    return out if data is not None else out[:4]
 
 
-def _sample_uniform(indptr, indices, column_ids, fanout, replace, with_coo, seed, data, e_ids, ctx):
-    indptr, indices = _i64(indptr, "indptr"), _i64(indices, "indices")
-    column_ids = _i64(column_ids, "column_ids", allow_none=True)
-    data, e_ids = _f32(data, "data", True), _i64(e_ids, "e_ids", True)
-    ctx = ctx or default_context(indptr.device)
-    S = column_ids.numel() if column_ids is not None else indptr.numel() - 1
-    cap = S * int(fanout)
-    sub_indptr = _empty(S + 1, indptr)
-    sub_indices, select = _empty(cap, indptr), _empty(cap, indptr)
-    coo_col = _empty(cap, indptr) if with_coo else None
-    out_data = _empty(cap, indptr, torch.float32) if data is not None else None
-    nnz = c_i64(0)
-    ctx.check(ctx.lib.gsb_sample_uniform(ctx.handle, _stream(), _p(indptr), _p(indices), c_i64(indptr.numel() - 1),
-                                         _p(column_ids), c_i64(S),
-                                         c_i64(int(fanout)), c_int(int(bool(replace))), c_u64(next_seed(seed)),
-                                         _p(sub_indptr), _p(sub_indices), _p(select), _p(coo_col), _p(data), _p(e_ids),
-                                         _p(out_data), c_i64(cap), ctypes.byref(nnz)), "gsb_sample_uniform")
-    n = nnz.value
-    out = [sub_indptr, coo_col[:n] if with_coo else None, sub_indices[:n], select[:n]]
-    if data is not None:
-        out.append(out_data[:n])
-    return tuple(out)
+def col_slice(indptr, indices, column_ids, with_coo, data=None, e_ids=None, ctx=None):
+    """csc_col_slicing without the edge positions, for callers that need none →
+    (sub_indptr, coo_col | None, sub_indices, sliced_data | None)."""
+    ctx = _context_for(indptr, ctx)
+    out = ctx.native.col_slicing(ctx.address, indptr, indices, column_ids, with_coo, False, data, e_ids)
+    return out[0], out[1], out[2], out[4]
+
+
+def _sample_columns(indptr, indices, probs, column_ids, fanout, replace, with_coo, with_select, seed, data, e_ids, ctx):
+    """(sub_indptr, coo_col | None, sub_indices, select_index | None, sampled data | None)."""
+    ctx = _context_for(indptr, ctx)
+    return ctx.native.col_sampling(ctx.address, indptr, indices, probs, column_ids, int(fanout), replace, with_coo,
+                                   with_select, next_seed(seed), data, e_ids)
+
+
+def col_sample(indptr, indices, column_ids, fanout, replace, with_coo, probs=None, seed=None, data=None, e_ids=None,
+               ctx=None):
+    """Per-column sampling without the edge positions, for callers that need none →
+    (sub_indptr, coo_col | None, sub_indices, sampled data | None)."""
+    out = _sample_columns(indptr, indices, probs, column_ids, fanout, replace, with_coo, False, seed, data, e_ids, ctx)
+    return out[0], out[1], out[2], out[4]
 
 
 def csc_col_sampling(indptr, indices, fanout, replace, with_coo=True, seed=None, data=None, e_ids=None, ctx=None):
     """CSCColSamplingCUDA (src/cuda/sampling.cu:156-167): sample every column of the operand →
     (sub_indptr, coo_col | None, sub_indices, select_index[, data])."""
-    return _sample_uniform(indptr, indices, None, fanout, replace, with_coo, seed, data, e_ids, ctx)
+    out = _sample_columns(indptr, indices, None, None, fanout, replace, with_coo, True, seed, data, e_ids, ctx)
+    return out if data is not None else out[:4]
 
 
 def fused_csc_col_slicing_sampling(indptr, indices, column_ids, fanout, replace, seed=None, data=None, e_ids=None,
                                    ctx=None):
     """FusedCSCColSlicingSamplingCUDA (src/cuda/fusion/slice_sampling.cu:145-151) →
     (sub_indptr, sub_indices, select_index[, data]); select_index points into the ORIGINAL indices."""
-    r = _sample_uniform(indptr, indices, column_ids, fanout, replace, False, seed, data, e_ids, ctx)
-    return (r[0],) + tuple(r[2:])
+    r = _sample_columns(indptr, indices, None, column_ids, fanout, replace, False, True, seed, data, e_ids, ctx)
+    return (r[0],) + r[2:] if data is not None else (r[0], r[2], r[3])
 
 
 def fused_csc_col_slicing_sampling_one_keepdim(indptr, indices, column_ids, seed=None, ctx=None):
@@ -267,21 +282,12 @@ def _len_array(tensors):
 def relabel(mapping_tensors, data_requiring_relabel, ctx=None):
     """RelabelCUDA (src/cuda/unique_reindex.cu:179-199) → (unique_tensor, [relabeled tensors]).
     unique_tensor lists the distinct ids of cat(mapping_tensors) in order of first occurrence."""
-    maps = [_i64(t, "mapping tensor") for t in mapping_tensors]
-    rels = [_i64(t, "tensor to relabel") for t in data_requiring_relabel]
-    if not maps:
+    if not mapping_tensors:
         raise ValueError("at least one mapping tensor is required")
-    if len(maps) > 4 or len(rels) > 4:
+    if len(mapping_tensors) > 4 or len(data_requiring_relabel) > 4:
         raise ValueError("at most 4 mapping tensors and 4 tensors to relabel per call")
-    ctx = ctx or default_context(maps[0].device)
-    n = sum(t.numel() for t in maps)
-    uniq = _empty(n, maps[0])
-    outs = [torch.empty_like(t) for t in rels]
-    nu = c_i64(0)
-    ctx.check(ctx.lib.gsb_unique_relabel(ctx.handle, _stream(), _ptr_array(maps), _len_array(maps), c_int(len(maps)),
-                                         _p(uniq), _ptr_array(rels), _len_array(rels), _ptr_array(outs),
-                                         c_int(len(rels)), ctypes.byref(nu)), "gsb_unique_relabel")
-    return uniq[:nu.value], outs
+    ctx = _context_for(mapping_tensors[0], ctx)
+    return ctx.native.relabel(ctx.address, mapping_tensors, data_requiring_relabel)
 
 
 def tensor_unique(node_ids, ctx=None):
@@ -293,15 +299,9 @@ def fused_random_walk(seeds, walk_length, indices, indptr, seed=None, layout=0, 
     """FusedRandomWalkCUDA (src/cuda/fusion/random_walk.cu:52-68).  layout=0 returns the reference's
     result exactly as it does: step-major memory viewed as [num_seeds, walk_length + 1]; layout=1
     returns a true walker-major [num_seeds, walk_length + 1] trace."""
-    seeds, indptr, indices = _i64(seeds, "seeds"), _i64(indptr, "indptr"), _i64(indices, "indices")
-    ctx = ctx or default_context(indptr.device)
-    W, L = seeds.numel(), int(walk_length)
-    out = _empty(W * (L + 1), indptr)
-    ctx.check(ctx.lib.gsb_random_walk(ctx.handle, _stream(), _p(indptr), _p(indices), c_i64(indptr.numel() - 1),
-                                      _p(seeds), c_i64(W), c_i64(L),
-                                      c_u64(next_seed(seed)), c_int(int(layout)), c_i64(int(walker_offset)), _p(out)),
-              "gsb_random_walk")
-    return out.reshape(W, L + 1)
+    ctx = _context_for(indptr, ctx)
+    return ctx.native.random_walk(ctx.address, indptr, indices, seeds, int(walk_length), next_seed(seed), int(layout),
+                                  int(walker_offset))
 
 
 def fused_metapath_random_walk(seeds, metapath, graphs, seed=None, layout=0, walker_offset=0, ctx=None):
@@ -329,59 +329,28 @@ def csc_col_row_slicing(indptr, indices, column_ids, row_ids, col_ptr=None, row_
     (sub_indptr, sub_indices, select_index[, sliced_data]).  Without col_ptr / row_ptr the kept row ids are
     renumbered to their position in row_ids; with them (the super-batch form) a column of batch b is matched
     against batch b's rows and row ids stay as they are.  select_index points into `indices`."""
-    indptr, indices = _i64(indptr, "indptr"), _i64(indices, "indices")
-    column_ids, row_ids = _i64(column_ids, "column_ids"), _i64(row_ids, "row_ids")
-    col_ptr, row_ptr = _i64(col_ptr, "col_ptr", True), _i64(row_ptr, "row_ptr", True)
-    data, e_ids = _f32(data, "data", True), _i64(e_ids, "e_ids", True)
     if (col_ptr is None) != (row_ptr is None):
         raise ValueError("col_ptr and row_ptr go together")
-    ctx = ctx or default_context(indptr.device)
-    S, R = column_ids.numel(), row_ids.numel()
-    G = 1 if col_ptr is None else col_ptr.numel() - 1
-    slice_indptr = _empty(S + 1, indptr)
-    d = c_i64(0)
-    num_cols = indptr.numel() - 1
-    ctx.check(ctx.lib.gsb_col_slice_count(ctx.handle, _stream(), _p(indptr), c_i64(num_cols), _p(column_ids), c_i64(S),
-                                          _p(slice_indptr), ctypes.byref(d)), "gsb_col_slice_count")
-    D = d.value
-    sub_indptr = _empty(S + 1, indptr)
-    sub_indices, select = _empty(D, indptr), _empty(D, indptr)
-    out_data = _empty(D, indptr, torch.float32) if data is not None else None
-    nnz = c_i64(0)
-    ctx.check(ctx.lib.gsb_col_row_slice(ctx.handle, _stream(), _p(indptr), _p(indices), c_i64(num_cols),
-                                        _p(column_ids), c_i64(S),
-                                        _p(slice_indptr), c_i64(D), _p(row_ids), c_i64(R), _p(col_ptr), _p(row_ptr),
-                                        c_i64(G), c_i64(int(encoding_size)), c_int(1 if col_ptr is None else 0),
-                                        _p(sub_indptr), _p(sub_indices), _p(select), _p(data), _p(e_ids),
-                                        _p(out_data), ctypes.byref(nnz)), "gsb_col_row_slice")
-    n = nnz.value
-    sub_indices, select = sub_indices[:n], select[:n]
-    if out_data is not None:
-        out_data = out_data[:n]
-    if data is not None:
-        return sub_indptr, sub_indices, select, out_data
-    return sub_indptr, sub_indices, select
+    ctx = _context_for(indptr, ctx)
+    out = ctx.native.col_row_slicing(ctx.address, indptr, indices, column_ids, row_ids, col_ptr, row_ptr,
+                                     int(encoding_size), True, data, e_ids)
+    return out if data is not None else out[:3]
+
+
+def col_row_slice(indptr, indices, column_ids, row_ids, col_ptr=None, row_ptr=None, encoding_size=0, data=None,
+                  e_ids=None, ctx=None):
+    """csc_col_row_slicing without the edge positions → (sub_indptr, sub_indices, sliced_data | None)."""
+    ctx = _context_for(indptr, ctx)
+    out = ctx.native.col_row_slicing(ctx.address, indptr, indices, column_ids, row_ids, col_ptr, row_ptr,
+                                     int(encoding_size), False, data, e_ids)
+    return out[0], out[1], out[3]
 
 
 def gather_rows(src, index, ctx=None):
     """out[i] = src[index[i]] for a float32 matrix (or vector) `src` that lives on the GPU or in pinned host memory
     (read in place by the GPU, like IndexSelectCPUFromGPU, src/cuda/index_select_uvm.cu:8-45)."""
-    index = _i64(index, "index")
-    if not (isinstance(src, torch.Tensor) and src.dtype == torch.float32 and src.is_contiguous()):
-        raise TypeError("src must be a contiguous float32 tensor")
-    if not (src.is_cuda or src.is_pinned()):
-        raise TypeError("src must live on the GPU or in pinned host memory")
-    ctx = ctx or default_context(index.device)
-    num_rows = src.shape[0] if src.dim() > 0 else 0
-    row_len = 1
-    for d in src.shape[1:]:
-        row_len *= int(d)
-    out = torch.empty((index.numel(),) + tuple(src.shape[1:]), dtype=torch.float32, device=index.device)
-    if row_len == 0:
-        return out
-    ctx.check(ctx.lib.gsb_gather_rows(ctx.handle, _stream(), c_vp(src.data_ptr()), c_i64(num_rows), c_i64(row_len),
-                                      _p(index), c_i64(index.numel()), _p(out)), "gsb_gather_rows")
-    return out
+    ctx = _context_for(index, ctx)
+    return ctx.native.gather_rows(ctx.address, src, index)
 
 
 index_select_cpu_from_gpu = gather_rows
@@ -427,48 +396,21 @@ def csc_col_sampling_probs(indptr, indices, probs, fanout, replace, with_coo=Tru
     """CSCColSamplingProbsCUDA (src/cuda/sampling_probs.cu:267-282) → (sub_indptr, coo_col | None,
     sub_indices, select_index[, data]).  `probs[j]` pairs with `indices[j]`.  `column_ids` (not in the
     reference) fuses a column slice in front."""
-    indptr, indices, probs = _i64(indptr, "indptr"), _i64(indices, "indices"), _f32(probs, "probs")
-    column_ids = _i64(column_ids, "column_ids", allow_none=True)
-    data, e_ids = _f32(data, "data", True), _i64(e_ids, "e_ids", True)
+    if probs is None:
+        raise TypeError("probs is required")
     if probs.numel() != indices.numel():
         raise ValueError("probs must have one entry per edge of the operand")
-    ctx = ctx or default_context(indptr.device)
-    S = column_ids.numel() if column_ids is not None else indptr.numel() - 1
-    cap = S * int(fanout)
-    sub_indptr = _empty(S + 1, indptr)
-    sub_indices, select = _empty(cap, indptr), _empty(cap, indptr)
-    coo_col = _empty(cap, indptr) if with_coo else None
-    out_data = _empty(cap, indptr, torch.float32) if data is not None else None
-    nnz = c_i64(0)
-    ctx.check(ctx.lib.gsb_sample_weighted(ctx.handle, _stream(), _p(indptr), _p(indices), c_i64(indptr.numel() - 1),
-                                          _p(probs), _p(column_ids),
-                                          c_i64(S), c_i64(int(fanout)), c_int(int(bool(replace))),
-                                          c_u64(next_seed(seed)), _p(sub_indptr), _p(sub_indices), _p(select),
-                                          _p(coo_col), _p(data), _p(e_ids), _p(out_data), c_i64(cap),
-                                          ctypes.byref(nnz)), "gsb_sample_weighted")
-    n = nnz.value
-    out = [sub_indptr, coo_col[:n] if with_coo else None, sub_indices[:n], select[:n]]
-    if data is not None:
-        out.append(out_data[:n])
-    return tuple(out)
+    out = _sample_columns(indptr, indices, probs, column_ids, fanout, replace, with_coo, True, seed, data, e_ids, ctx)
+    return out if data is not None else out[:4]
 
 
 def list_sampling(data, num_picks, replace, probs=None, seed=None, ctx=None):
     """ListSamplingCUDA (src/cuda/list_sampling.cu:76-83) / ListSamplingProbsCUDA
     (src/cuda/list_sampling_probs.cu:185-191) → (selected_data, selected_index)."""
-    data = _i64(data, "data")
-    probs = _f32(probs, "probs", allow_none=True)
     if probs is not None and probs.numel() != data.numel():
         raise ValueError("probs must have one entry per item")
-    ctx = ctx or default_context(data.device)
-    N, k = data.numel(), int(num_picks)
-    cap = max(N if (not replace and N <= k) else k, 1)
-    out_d, out_i = _empty(cap, data), _empty(cap, data)
-    n_out = c_i64(0)
-    ctx.check(ctx.lib.gsb_list_sample(ctx.handle, _stream(), _p(data), _p(probs), c_i64(N), c_i64(k),
-                                      c_int(int(bool(replace))), c_u64(next_seed(seed)), _p(out_d), _p(out_i),
-                                      ctypes.byref(n_out)), "gsb_list_sample")
-    return out_d[:n_out.value], out_i[:n_out.value]
+    ctx = _context_for(data, ctx)
+    return ctx.native.list_sampling(ctx.address, data, int(num_picks), replace, probs, next_seed(seed))
 
 
 SDDMM_OPS = {"add": 0, "sub": 1, "mul": 2, "div": 3, "copy_lhs": 4, "copy_rhs": 5, "dot": 6}
@@ -526,103 +468,65 @@ def sddmm(op, lhs, rhs, out, lhs_target, rhs_target, row, col=None, indptr=None,
     lhs, rhs = _f32(lhs, "lhs", op == "copy_rhs"), _f32(rhs, "rhs", op == "copy_lhs")
     if not (isinstance(out, torch.Tensor) and out.is_cuda and out.dtype == torch.float32 and out.is_contiguous()):
         raise TypeError("out must be a contiguous float32 CUDA tensor")
-    ctx = ctx or default_context(row.device)
+    ctx = _context_for(row, ctx)
     bc = calc_bcast_off(op, lhs if lhs is not None else rhs, rhs if rhs is not None else lhs)
     E = row.numel()
     if out.numel() != E * bc["out_len"]:
         raise ValueError(f"out has {out.numel()} elements, expected {E} x {bc['out_len']}")
     lo = torch.tensor(bc["lhs_off"], dtype=torch.int64, device=row.device) if bc["lhs_off"] is not None else None
     ro = torch.tensor(bc["rhs_off"], dtype=torch.int64, device=row.device) if bc["rhs_off"] is not None else None
-    num_cols = indptr.numel() - 1 if indptr is not None else 0
-    ctx.check(ctx.lib.gsb_sddmm(ctx.handle, _stream(), c_int(SDDMM_OPS[op]), _p(row), _p(col), _p(indptr),
-                                c_i64(num_cols), _p(e_ids), c_i64(E), _p(lhs), _p(rhs), _p(out), c_int(int(lhs_target)),
-                                c_int(int(rhs_target)), c_i64(bc["lhs_len"]), c_i64(bc["rhs_len"]), c_i64(bc["out_len"]),
-                                c_i64(bc["reduce_size"]), _p(lo), _p(ro)), "gsb_sddmm")
+    ctx.native.sddmm(ctx.address, SDDMM_OPS[op], row, col, indptr, e_ids, lhs, rhs, out, int(lhs_target), int(rhs_target),
+                     bc["lhs_len"], bc["rhs_len"], bc["out_len"], bc["reduce_size"], lo, ro)
     return out
 
 
 def csc_sum(indptr, e_ids, data, out, powk, ctx=None):
     """CSCSumCUDA (src/cuda/graph_ops.cu:66-96): out[s] = sum over segment s of data^powk (data=None → ones)."""
-    indptr, e_ids, data = _i64(indptr, "indptr"), _i64(e_ids, "e_ids", True), _f32(data, "data", True)
-    ctx = ctx or default_context(indptr.device)
-    ctx.check(ctx.lib.gsb_segment_sum_csc(ctx.handle, _stream(), _p(indptr), c_i64(indptr.numel() - 1), _p(e_ids),
-                                          _p(data), c_i64(int(powk)), _p(out)), "gsb_segment_sum_csc")
+    ctx = _context_for(indptr, ctx)
+    ctx.native.segment_sum_csc(ctx.address, indptr, e_ids, data, int(powk), out)
     return out
 
 
 def coo_sum(target, e_ids, data, out, powk, ctx=None, targets_in_runs=False):
     """COOSumCUDA (src/cuda/graph_ops.cu:98-125): out[target[e]] += data[e]^powk; `out` must be zeroed.
     targets_in_runs: equal targets are adjacent (the sorted coordinate of a COO) — a hint, not a requirement."""
-    target, e_ids, data = _i64(target, "target"), _i64(e_ids, "e_ids", True), _f32(data, "data", True)
-    ctx = ctx or default_context(target.device)
-    ctx.check(ctx.lib.gsb_segment_sum_coo(ctx.handle, _stream(), _p(target), c_i64(target.numel()), _p(e_ids),
-                                          _p(data), c_i64(int(powk)), c_int(int(bool(targets_in_runs))), _p(out)),
-              "gsb_segment_sum_coo")
+    ctx = _context_for(target, ctx)
+    ctx.native.segment_sum_coo(ctx.address, target, e_ids, data, int(powk), targets_in_runs, out)
     return out
 
 
 def csc_normalize(indptr, e_ids, data, out, ctx=None):
     """CSCNormalizeCUDA (src/cuda/graph_ops.cu:160-188): out[e] = data[e] / (sum of its segment)."""
-    indptr, e_ids, data = _i64(indptr, "indptr"), _i64(e_ids, "e_ids", True), _f32(data, "data")
-    ctx = ctx or default_context(indptr.device)
-    ctx.check(ctx.lib.gsb_segment_normalize_csc(ctx.handle, _stream(), _p(indptr), c_i64(indptr.numel() - 1),
-                                                _p(e_ids), _p(data), _p(out)), "gsb_segment_normalize_csc")
+    ctx = _context_for(indptr, ctx)
+    ctx.native.segment_normalize_csc(ctx.address, indptr, e_ids, data, out)
     return out
 
 
 def csc_row_slicing(indptr, indices, row_ids, with_coo=True, ctx=None):
     """CSCRowSlicingCUDA (src/cuda/slicing.cu:528-539) → (out_indptr, coo_col | None, out_indices,
     select_index); kept row ids are renumbered to their position in row_ids."""
-    indptr, indices, row_ids = _i64(indptr, "indptr"), _i64(indices, "indices"), _i64(row_ids, "row_ids")
-    ctx = ctx or default_context(indptr.device)
-    nc, E = indptr.numel() - 1, indices.numel()
-    out_indptr = _empty(nc + 1, indptr)
-    oi, osel = _empty(E, indptr), _empty(E, indptr)
-    oc = _empty(E, indptr) if with_coo else None
-    nnz = c_i64(0)
-    ctx.check(ctx.lib.gsb_row_slice_csc(ctx.handle, _stream(), _p(indptr), _p(indices), c_i64(nc), c_i64(E),
-                                        _p(row_ids), c_i64(row_ids.numel()), _p(out_indptr), _p(oi), _p(osel), _p(oc),
-                                        ctypes.byref(nnz)), "gsb_row_slice_csc")
-    n = nnz.value
-    return out_indptr, (oc[:n] if with_coo else None), oi[:n], osel[:n]
+    ctx = _context_for(indptr, ctx)
+    return ctx.native.row_slicing_csc(ctx.address, indptr, indices, row_ids, with_coo)
 
 
 def coo_row_slicing(coo_row, coo_col, row_ids, ctx=None):
     """COORowSlicingCUDA (src/cuda/slicing.cu:768-771) → (renumbered_row, col, select_index)."""
-    coo_row, coo_col, row_ids = _i64(coo_row, "coo_row"), _i64(coo_col, "coo_col"), _i64(row_ids, "row_ids")
-    ctx = ctx or default_context(coo_row.device)
-    E = coo_row.numel()
-    o_r, o_c, o_s = _empty(E, coo_row), _empty(E, coo_row), _empty(E, coo_row)
-    nnz = c_i64(0)
-    ctx.check(ctx.lib.gsb_row_slice_coo(ctx.handle, _stream(), _p(coo_row), _p(coo_col), c_i64(E), _p(row_ids),
-                                        c_i64(row_ids.numel()), _p(o_r), _p(o_c), _p(o_s), ctypes.byref(nnz)),
-              "gsb_row_slice_coo")
-    n = nnz.value
-    return o_r[:n], o_c[:n], o_s[:n]
+    ctx = _context_for(coo_row, ctx)
+    return ctx.native.row_slicing_coo(ctx.address, coo_row, coo_col, row_ids)
 
 
 def csc2coo(indptr, indices, ctx=None):
     """CSC2COOCUDA (src/cuda/format_transform.cu:35-46) → (row = indices, col)."""
-    indptr, indices = _i64(indptr, "indptr"), _i64(indices, "indices")
-    ctx = ctx or default_context(indptr.device)
-    col = _empty(indices.numel(), indptr)
-    ctx.check(ctx.lib.gsb_csc2coo(ctx.handle, _stream(), _p(indptr), c_i64(indptr.numel() - 1), _p(col)),
-              "gsb_csc2coo")
-    return indices, col
+    ctx = _context_for(indptr, ctx)
+    indices = _i64(indices, "indices")
+    return indices, ctx.native.csc2coo(ctx.address, indptr, indices.numel())
 
 
 def coo2csc(row, col, num_cols, col_sorted, ctx=None):
     """COO2CSCCUDA (src/cuda/format_transform.cu:135-156) → (indptr, sorted_row, sort_index | None).
     For CSR pass (col, row, num_rows, row_sorted)."""
-    row, col = _i64(row, "row"), _i64(col, "col")
-    ctx = ctx or default_context(row.device)
-    E = row.numel()
-    indptr = _empty(int(num_cols) + 1, row)
-    out_row = _empty(E, row)
-    perm = None if col_sorted else _empty(E, row)
-    ctx.check(ctx.lib.gsb_coo2csc(ctx.handle, _stream(), _p(col), _p(row), c_i64(E), c_i64(int(num_cols)),
-                                  c_int(int(bool(col_sorted))), _p(indptr), _p(out_row), _p(perm)), "gsb_coo2csc")
-    return indptr, out_row, perm
+    ctx = _context_for(row, ctx)
+    return ctx.native.coo2csc(ctx.address, row, col, int(num_cols), col_sorted)
 
 
 # ---- batched ("super-batch") operators --------------------------------------------------------------
@@ -635,33 +539,17 @@ def batch_csr_relabel(seeds, seeds_ptr, indices, indices_ptr, indices_count=None
     count (indices_ptr[-1]); with sync=False the outputs keep their upper-bound length and the exact
     sizes stay on the device.  num_nodes > 0 (every id is below it) allows the direct-address tables;
     seeds_distinct promises that no id repeats among the seeds of a batch."""
-    seeds, seeds_ptr = _i64(seeds, "seeds"), _i64(seeds_ptr, "seeds_ptr")
-    indices, indices_ptr = _i64(indices, "indices"), _i64(indices_ptr, "indices_ptr")
-    ctx = ctx or default_context(seeds.device)
-    G = seeds_ptr.numel() - 1
+    ctx = _context_for(seeds, ctx)
     cap = indices.numel() if indices_count is None else int(indices_count)
-    uniq = _empty(seeds.numel() + cap, seeds)
-    uniq_ptr = _empty(G + 1, seeds)
-    rel = _empty(cap, seeds)
-    nu, ne = c_i64(0), c_i64(0)
-    ctx.check(ctx.lib.gsb_batch_unique_relabel(ctx.handle, _stream(), _p(seeds), _p(seeds_ptr), c_i64(seeds.numel()),
-                                               _p(indices), _p(indices_ptr), c_i64(cap), c_i64(G),
-                                               c_i64(int(num_nodes)), c_int(1 if seeds_distinct else 0), _p(uniq),
-                                               _p(uniq_ptr), _p(rel), ctypes.byref(nu) if sync else None,
-                                               ctypes.byref(ne) if sync else None), "gsb_batch_unique_relabel")
-    if sync:
-        return uniq[:nu.value], uniq_ptr, rel[:ne.value], indices_ptr
+    uniq, uniq_ptr, rel = ctx.native.batch_csr_relabel(ctx.address, seeds, seeds_ptr, indices, indices_ptr, cap, sync,
+                                                       int(num_nodes), seeds_distinct)
     return uniq, uniq_ptr, rel, indices_ptr
 
 
 def batch_edge_offsets(sub_indptr, seeds_ptr, ctx=None):
     """indices_ptr[b] = sub_indptr[seeds_ptr[b]] (what GetBatchCSC derives, examples/graphsage/batching.py:66)."""
-    sub_indptr, seeds_ptr = _i64(sub_indptr, "sub_indptr"), _i64(seeds_ptr, "seeds_ptr")
-    ctx = ctx or default_context(sub_indptr.device)
-    out = _empty(seeds_ptr.numel(), seeds_ptr)
-    ctx.check(ctx.lib.gsb_batch_edge_offsets(ctx.handle, _stream(), _p(sub_indptr), _p(seeds_ptr),
-                                             c_i64(seeds_ptr.numel() - 1), _p(out)), "gsb_batch_edge_offsets")
-    return out
+    ctx = _context_for(sub_indptr, ctx)
+    return ctx.native.batch_edge_offsets(ctx.address, sub_indptr, seeds_ptr)
 
 
 # ---- the rest of the super-batch family (gs_ops registry, src/pybind.cc:65-84) ------------------
@@ -915,17 +803,11 @@ def sage_sample_batches(indptr, indices, seeds, seeds_ptr, fanouts, replace=Fals
     proportion.  The first hop's seed bound is ignored (its seed count is exact).  If a hop meets more seeds or edges
     than hinted, the device records GSB_ERR_CAPACITY (ctx.check_device() raises it) and the caller repeats the call
     without hints; nothing is written out of bounds."""
-    ctx = ctx or default_context(indptr.device)
+    ctx = _context_for(indptr, ctx)
     out = []
     base_seed = next_seed(seed)
-    batch_ids = _i64(batch_ids, "batch_ids", allow_none=True)
     if batch_ids is not None and batch_ids.numel() != seeds_ptr.numel() - 1:
         raise ValueError("batch_ids needs one entry per minibatch")
-    num_nodes = indptr.numel() - 1
-
-    def alloc(name, hop, n):
-        return _empty(n, indptr) if arena is None else arena.get((name, hop), n, indptr)
-
     if size_hints is not None and (sync or len(size_hints) != len(fanouts)):
         raise ValueError("size_hints needs sync=False and one (seed_bound, edge_bound) pair per hop")
     for hop, k in enumerate(fanouts):
@@ -937,29 +819,19 @@ def sage_sample_batches(indptr, indices, seeds, seeds_ptr, fanouts, replace=Fals
                 S = min(S, int(size_hints[hop][0]))
                 seeds = seeds[:S]
             cap = min(S * int(k), int(size_hints[hop][1]))
-        sub_indptr = alloc("sub_indptr", hop, S + 1)
-        sub_indices, select, rel = alloc("indices", hop, cap), alloc("select", hop, cap), alloc("relabeled", hop, cap)
-        indices_ptr, uniq_ptr = alloc("indices_ptr", hop, G + 1), alloc("frontier_ptr", hop, G + 1)
-        uniq = alloc("frontier", hop, S + cap)
-        nu, ne = c_i64(0), c_i64(0)
         flags = 1 if (hop > 0 or seeds_distinct) else 0
-        ctx.check(ctx.lib.gsb_sage_hop(ctx.handle, _stream(), _p(indptr), _p(indices), c_i64(num_nodes), _p(seeds),
-                                       _p(seeds_ptr), _p(batch_ids), c_i64(G), c_i64(S), c_i64(int(k)), c_i64(cap),
-                                       c_int(int(bool(replace))), c_u64((base_seed + hop) & (2**64 - 1)),
-                                       c_int(flags), _p(sub_indptr), _p(sub_indices),
-                                       _p(select), _p(indices_ptr), _p(uniq), _p(uniq_ptr), _p(rel),
-                                       ctypes.byref(nu) if sync else None, ctypes.byref(ne) if sync else None),
-                  "gsb_sage_hop")
-        if sync:
-            E, U = ne.value, nu.value
-            out.append(dict(seeds=seeds, seeds_ptr=seeds_ptr, sub_indptr=sub_indptr, indices=sub_indices[:E],
-                            relabeled=rel[:E], select_index=select[:E], indices_ptr=indices_ptr, frontier=uniq[:U],
-                            frontier_ptr=uniq_ptr))
-            seeds, seeds_ptr = uniq[:U], uniq_ptr
-        else:
-            counts = torch.cat([seeds_ptr[G:], indices_ptr[G:], uniq_ptr[G:]])
-            out.append(dict(seeds=seeds, seeds_ptr=seeds_ptr, sub_indptr=sub_indptr, indices=sub_indices,
-                            relabeled=rel, select_index=select, indices_ptr=indices_ptr, frontier=uniq,
-                            frontier_ptr=uniq_ptr, counts=counts))
-            seeds, seeds_ptr = uniq, uniq_ptr
+        buffers = None
+        if arena is not None:
+            buffers = (arena.get(("sub_indptr", hop), S + 1, indptr), arena.get(("indices", hop), cap, indptr),
+                       arena.get(("select", hop), cap, indptr), arena.get(("relabeled", hop), cap, indptr),
+                       arena.get(("indices_ptr", hop), G + 1, indptr), arena.get(("frontier_ptr", hop), G + 1, indptr),
+                       arena.get(("frontier", hop), S + cap, indptr))
+        sub_indptr, sub_indices, select, rel, indices_ptr, uniq_ptr, uniq = ctx.native.sage_hop(
+            ctx.address, indptr, indices, seeds, seeds_ptr, batch_ids, int(k), cap, replace,
+            (base_seed + hop) & (2**64 - 1), flags, sync, buffers)
+        out.append(dict(seeds=seeds, seeds_ptr=seeds_ptr, sub_indptr=sub_indptr, indices=sub_indices, relabeled=rel,
+                        select_index=select, indices_ptr=indices_ptr, frontier=uniq, frontier_ptr=uniq_ptr))
+        if not sync:
+            out[-1]["counts"] = torch.cat([seeds_ptr[G:], indices_ptr[G:], uniq_ptr[G:]])
+        seeds, seeds_ptr = uniq, uniq_ptr
     return out

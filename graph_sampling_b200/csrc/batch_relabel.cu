@@ -651,6 +651,9 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   i64* counters = ctx_counters(ctx);
   const size_t off_bytes = ((size_t)(G + 1) * 8 + 255) & ~(size_t)255;
   const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
+  if (path == 0 && L.indices_ptr && fused_unique_suits(ctx, n_cap, G))
+    return fused_unique_batched(ctx, stream, L, seeds_bound, edges_bound, nullptr, nullptr, out_unique, out_unique_ptr,
+                                out_relabeled, mail);
   u64* tables = nullptr;
   uint32_t epoch = 0;
   // Automatic choice: direct-address tables only while all tables of the call stay L2-sized.  A minibatch touches
@@ -868,8 +871,9 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
   int st;
   const Mail mail = mail_if(ctx, unique_total_host || edges_total_host);
   const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
+  const bool fused = path == 0 && fused_unique_suits(ctx, n_cap, G);
   const bool direct_small = (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes && num_nodes > 0;
-  if (k >= 1 && k <= 16 && n_cap > 0 && (path == 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
+  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && (path == 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
     st = sage_hop_sampler_counts(ctx, stream, indptr, indices, num_nodes, seeds, seeds_ptr, batch_ids, G, S, k, cap,
                                  replace, (u64)seed, out_indptr, out_indices, out_select, out_indices_ptr, out_unique,
                                  out_unique_ptr, out_relabeled, mail);
@@ -881,6 +885,17 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
                                  out_indices, out_select, nullptr, nullptr, nullptr, nullptr, cap, seeds_ptr + G,
                                  seeds_ptr, batch_ids, G);
   if (st != GSB_OK) return st;
+  if (fused) {
+    BatchLayout F{};
+    F.seeds = seeds;
+    F.seeds_ptr = seeds_ptr;
+    F.indices = out_indices;
+    F.G = G;
+    st = fused_unique_batched(ctx, stream, F, S, cap, out_indptr, out_indices_ptr, out_unique, out_unique_ptr,
+                              out_relabeled, mail);
+    if (st != GSB_OK || !mail.word) return st;
+    return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
+  }
   {
     ScopedKernelTimer timer(ctx, KID_OTHER, stream);
     k_gather_offsets<<<grid_for(G + 1, kBThreads), kBThreads, 0, stream>>>(out_indptr, seeds_ptr, G, S,

@@ -194,6 +194,24 @@ struct CompactOut {
   Mail mail;        // slots 0, 1: frontier and edge totals, for a caller that waits for them
 };
 
+// Single-launch unique + relabel (defined in fused_unique.cu).  Ids below 2^32 - 1; a larger or negative one makes the
+// kernel record GSB_ERR_INDEX_RANGE.  fused_unique_suits: whether a call of n items in G minibatches fits its registers,
+// its table and one resident grid.
+//   single   unique(cat(first, second)) -> out_unique, ranks of `second` -> out_second (may be null), and with col_index
+//            (positions in `first`, one per entry of `second`) the ranks of first[col_index[e]] -> out_col; copies
+//            copy_n words from copy_src to copy_dst along the way.  mail slot 0: distinct ids.
+//   batched  as gsb_batch_unique_relabel; with sub_indptr the edge offsets of the minibatches are sub_indptr[seeds_ptr[b]]
+//            and are written to out_indices_ptr.  mail slots 0, 1: frontier and edge totals.
+constexpr i64 kFusedUniqueMaxItems = 1ll << 21;
+constexpr i64 kFusedUniqueMaxBatches = 1ll << 16;
+bool fused_unique_suits(gsb_ctx* ctx, i64 n, i64 G);
+int fused_unique_single(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64 S, const i64* second, i64 E,
+                        const i64* col_index, i64* out_unique, i64* out_second, i64* out_col, const i64* copy_src,
+                        i64* copy_dst, i64 copy_n, Mail mail);
+int fused_unique_batched(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L, i64 seeds_bound, i64 edges_bound,
+                         const i64* sub_indptr, i64* out_indices_ptr, i64* out_unique, i64* out_unique_ptr,
+                         i64* out_relabeled, Mail mail);
+
 // Single-batch unique + relabel through the packed-slot batched kernels (defined in batch_relabel.cu).
 int unique_relabel_packed(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64 S, const i64* second, i64 E,
                           i64* out_unique, i64* out_relabeled, i64* unique_host);

@@ -17,7 +17,7 @@ struct gsb_ctx {
   u64* tile_words;
   i64 tile_capacity;
   uint32_t epoch;
-  i64* counters;  // device, CNT_NUM entries
+  i64* counters;  // device, CNT_NUM entries and the grid-barrier word
   i64* pinned;    // page-locked host memory the device writes: CNT_NUM counters, kMailSlots result words, one ticket
   u64 mail_tag;   // 1 .. 65535, of the last mailbox handed out
   u64 ticket;     // of the last counter fetch
@@ -36,6 +36,11 @@ struct gsb_ctx {
   u64* direct_tables;
   size_t direct_bytes;
   uint32_t direct_epoch;
+  // table and barrier word of the single-launch unique + relabel (see ctx_epoch_table)
+  u64* epoch_table;
+  i64 epoch_slots;
+  uint32_t table_epoch;
+  u64 barrier_arrivals;  // the barrier word itself is counters[CNT_NUM]
   cudaEvent_t wait_event;  // created on first use when GSB_OPT_BLOCKING_WAIT is set
 };
 
@@ -136,6 +141,36 @@ int ctx_direct_tables(gsb_ctx* ctx, i64 count, i64 num_nodes, cudaStream_t strea
   *out_table = ctx->direct_tables;
   *out_epoch = ctx->direct_epoch;
   return GSB_OK;
+}
+
+int ctx_epoch_table(gsb_ctx* ctx, i64 slots, uint32_t epochs, cudaStream_t stream, u64** table, uint32_t* epoch,
+                    u64** barrier) {
+  if (slots > ctx->epoch_slots) {
+    GSB_CUDA_OK(cudaDeviceSynchronize());
+    if (ctx->epoch_table) GSB_CUDA_OK(cudaFree(ctx->epoch_table));
+    ctx->epoch_table = nullptr;
+    ctx->epoch_slots = 0;
+    i64 cap = 1 << 16;
+    while (cap < slots) cap <<= 1;
+    GSB_CUDA_OK(cudaMalloc((void**)&ctx->epoch_table, sizeof(u64) * (size_t)cap));
+    ctx->epoch_slots = cap;
+    ctx->table_epoch = epochs - 1;  // cleared below
+  }
+  ctx->table_epoch += 1;
+  if (ctx->table_epoch >= epochs) {
+    GSB_CUDA_OK(cudaMemsetAsync(ctx->epoch_table, 0, sizeof(u64) * (size_t)ctx->epoch_slots, stream));
+    ctx->table_epoch = 1;
+  }
+  *table = ctx->epoch_table;
+  *epoch = ctx->table_epoch;
+  *barrier = (u64*)(ctx->counters + CNT_NUM);
+  return GSB_OK;
+}
+
+u64 ctx_barrier_base(gsb_ctx* ctx, u64 arrivals) {
+  const u64 base = ctx->barrier_arrivals;
+  ctx->barrier_arrivals += arrivals;
+  return base;
 }
 
 i64* ctx_counters(gsb_ctx* ctx) { return ctx->counters; }
@@ -322,8 +357,8 @@ int gsb_ctx_create(int device, gsb_ctx** out_ctx) {
   int st = GSB_OK;
   do {
     if ((e = cudaSetDevice(device)) != cudaSuccess) break;
-    if ((e = cudaMalloc((void**)&ctx->counters, sizeof(i64) * gsb::CNT_NUM)) != cudaSuccess) break;
-    if ((e = cudaMemset(ctx->counters, 0, sizeof(i64) * gsb::CNT_NUM)) != cudaSuccess) break;
+    if ((e = cudaMalloc((void**)&ctx->counters, sizeof(i64) * (gsb::CNT_NUM + 1))) != cudaSuccess) break;
+    if ((e = cudaMemset(ctx->counters, 0, sizeof(i64) * (gsb::CNT_NUM + 1))) != cudaSuccess) break;
     if ((e = cudaMallocHost((void**)&ctx->pinned, sizeof(i64) * (gsb::CNT_NUM + gsb::kMailSlots + 1))) != cudaSuccess) break;
     memset(ctx->pinned, 0, sizeof(i64) * (gsb::CNT_NUM + gsb::kMailSlots + 1));
   } while (0);
@@ -352,6 +387,7 @@ int gsb_ctx_destroy(gsb_ctx* ctx) {
   if (ctx->workspace) cudaFree(ctx->workspace);
   if (ctx->tile_words) cudaFree(ctx->tile_words);
   if (ctx->direct_tables) cudaFree(ctx->direct_tables);
+  if (ctx->epoch_table) cudaFree(ctx->epoch_table);
   if (ctx->wait_event) cudaEventDestroy(ctx->wait_event);
   if (ctx->counters) cudaFree(ctx->counters);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);

@@ -1,0 +1,538 @@
+// Unique + relabel of an ordinary call in ONE launch.
+//
+// A minibatch relabelled on its own (or a few of them) is 10^4 to 10^6 items: each pass over them is a few microseconds of
+// work, and the multi-launch forms (batch_relabel.cu, partition_relabel.cu) spend more time between their five to nine
+// launches than in them.  Here the grid is launched cooperatively, small enough to be resident as a whole, the items of a
+// thread stay in registers, and two grid-wide barriers separate the phases:
+//
+//   insert   every item claims a slot of an L2-resident hash table for its id and lowers the slot's position to its own;
+//            a slot is one word, [epoch : 11 | id : 32 | position : 21], and a word of an older epoch counts as empty, so
+//            the table is never cleared between calls (once per 2 047 calls, when the epoch wraps).  Slots come in
+//            buckets of four, one 32-byte sector that is read in one go, three slots per item: the longest chain of
+//            dependent reads of a call sets the pace of its insert, and it is a handful of buckets here where linear
+//            probing over single slots at load 0.5 had chains of fifty (813 000 items: 92 -> 52 us);
+//   ------   barrier
+//   flag     the item whose position the slot kept is the first occurrence of its id: one bit per item and a running
+//            count per 32 items inside the CTA, one total per CTA;
+//   ------   barrier
+//   emit     the rank of any position is its CTA's prefix (a scan of at most a few hundred totals, done by every CTA for
+//            itself) + its word's prefix + the bits below it: the frontier is written at those ranks, and every item to
+//            relabel writes the rank of the first occurrence of its id.
+//
+// BATCHED: the items belong to G minibatches (numbered batch-major, as in batch_table.cuh), each with a region of the
+// table of its own; ranks are then relative to the minibatch's first item.
+//
+// Against the five-launch form, GPU time without its launch gaps: 16 000 items 26 -> 11 us, 813 000 items 86 -> 52 us.
+// What bounds it now: the chain bucket read -> CAS -> CAS of the slowest lane of every warp, item after item.
+#include "batch_table.cuh"
+#include "common.cuh"
+#include "scan.cuh"
+
+namespace gsb {
+
+typedef uint32_t u32;
+
+constexpr int kFuThreads = 512;
+constexpr int kFuWarps = kFuThreads / 32;
+constexpr int kFuPosBits = 21;
+constexpr u64 kFuPosMask = (1ull << kFuPosBits) - 1;
+constexpr u32 kFuEpochs = 1u << (64 - 32 - kFuPosBits);  // epochs 1 .. kFuEpochs - 1
+constexpr u32 kFuNone = 0xFFFFFFFFu;
+constexpr int kFuWindow = 512;  // minibatches whose offsets a CTA keeps in shared memory
+
+struct FusedParams {
+  const i64* first;   // S ids
+  const i64* second;  // E ids, relabelled into out_second (may be null)
+  i64 S, E;           // BATCHED: bounds of the device-side totals
+  i64* out_unique;
+  i64* out_second;
+  const i64* col_index;  // E positions in `first`; out_col receives the rank of the id found there (may be null)
+  i64* out_col;
+  const i64* copy_src;  // an array to copy along the way (may be null)
+  i64* copy_dst;
+  i64 copy_n;
+  // BATCHED
+  const i64* seeds_ptr;    // [G + 1]
+  const i64* indices_ptr;  // [G + 1], or null: the offsets are sub_indptr[seeds_ptr[b]] and are written to out_indices_ptr
+  const i64* sub_indptr;   // [S + 1]
+  i64* out_indices_ptr;
+  i64* out_unique_ptr;  // [G + 1]
+  i64 G;
+  // scratch
+  u64* table;
+  u64 epoch;  // already shifted
+  u64* packed;    // [items / 32 + 1]  first occurrences of the CTA before the word << 32 | bits
+  u32* totals;    // [CTAs]
+  u32* seed_ref;  // [S] first position of every id of `first` (only with col_index)
+  u64* barrier;
+  u64 barrier_base;
+  i64* counters;
+  int max_polls;
+  Mail mail;
+};
+
+__device__ __forceinline__ u64 ld_acquire_u64(const u64* p) {
+  u64 v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Every CTA of the (cooperatively launched, hence resident) grid arrives; the wait is bounded like every other.
+__device__ __forceinline__ void grid_barrier(const FusedParams& p, u64 target) {
+  __syncthreads();
+  if (threadIdx.x == 0) {  // release / acquire, cumulative over what the CTA did before its barrier
+    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(p.barrier) : "memory");
+    int polls = 0;
+    while ((i64)(ld_acquire_u64(p.barrier) - target) < 0) {
+      if (++polls > p.max_polls) {
+        raise_error(p.counters, GSB_ERR_LOOKBACK_TIMEOUT, blockIdx.x);
+        break;
+      }
+      if (polls > 64) __nanosleep(20);
+    }
+  }
+  __syncthreads();
+}
+
+// Buckets of a region: minibatch b, whose items are [begin, next), has the buckets [bucket0(begin, b), bucket0(next, b + 1)),
+// at least 0.75 per item.
+__host__ __device__ __forceinline__ u32 fused_bucket0(u32 begin, u32 b) { return begin - (begin >> 2) + 2 * b; }
+
+__device__ __forceinline__ u32 fused_home(u32 id, u32 size) {
+  u32 x = id * 0x9E3779B1u;
+  x ^= x >> 15;
+  x *= 0x85EBCA6Bu;
+  return __umulhi(x, size);
+}
+
+// Offsets of minibatch b: first seed, first edge.
+__device__ __forceinline__ i64 fused_edges_begin(const FusedParams& p, i64 b, i64 seeds_begin) {
+  return p.indices_ptr ? __ldg(p.indices_ptr + b) : __ldg(p.sub_indptr + max((i64)0, min(seeds_begin, p.S)));
+}
+__device__ __forceinline__ i64 fused_item_off(const FusedParams& p, i64 b) {
+  const i64 s = __ldg(p.seeds_ptr + b);
+  return s + fused_edges_begin(p, b, s);
+}
+
+__device__ __forceinline__ void load_bucket(const u64* table, u32 bucket, u64 (&w)[4]) {
+  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(table + 4ull * bucket);
+  const ulonglong2 a = __ldcg(p), b = __ldcg(p + 1);
+  w[0] = a.x;
+  w[1] = a.y;
+  w[2] = b.x;
+  w[3] = b.y;
+}
+
+// Slot of the bucket that holds mine's id with a position no larger than mine's — found or newly claimed — or kFuNone when
+// the bucket is full of other ids.  An id always takes the first slot that is free, so nobody misses a copy of it.
+__device__ __forceinline__ u32 claim_in_bucket(const FusedParams& p, u32 bucket, const u64 (&word)[4], u64 mine) {
+#pragma unroll
+  for (u32 j = 0; j < 4; ++j) {
+    u64 w = word[j];
+    u64* s = p.table + 4ull * bucket + j;
+    if ((w ^ p.epoch) >> (32 + kFuPosBits)) {  // of an older epoch: free
+      const u64 old = atomicCAS(s, w, mine);
+      if (old == w) return 4 * bucket + j;
+      w = old;  // of this epoch: whoever was first put it there
+    }
+    if (((w ^ mine) >> kFuPosBits) == 0) {
+      if (w > mine) atomicMin(s, mine);
+      return 4 * bucket + j;
+    }
+  }
+  return kFuNone;
+}
+
+template <int R, bool BATCHED>
+__global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_constant__ FusedParams p) {
+  constexpr u32 kItems = kFuThreads * R;  // of a CTA
+  __shared__ u32 s_group[kFuWarps * R];   // counts per 32 items, then their exclusive prefixes
+  __shared__ u32 s_prefix[kFuThreads];    // first occurrences before every CTA
+  __shared__ u32 s_warp[kFuWarps];
+  __shared__ u32 s_off[BATCHED ? kFuWindow + 1 : 1];    // item offsets of the CTA's minibatches
+  __shared__ u32 s_seeds[BATCHED ? kFuWindow + 1 : 1];  // their first seeds
+  __shared__ i64 s_range[2];
+  const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const u32 base = blockIdx.x * kItems;
+  i64 ns = p.S, ne = p.E;
+  if (BATCHED) {
+    ns = __ldg(p.seeds_ptr + p.G);
+    ne = fused_edges_begin(p, p.G, ns);
+    if (ns > p.S || ne > p.E || ns < 0 || ne < 0) {  // every CTA sees the same: nobody waits for anybody
+      if (tid == 0) {
+        raise_error(p.counters, GSB_ERR_CAPACITY, ns > p.S ? ns : ne);
+        atomicAdd(p.barrier, 2ull);
+        if (blockIdx.x == 0) {
+          p.counters[CNT_ABORT] = 1;
+          mail_post(p.mail, 0, 0, p.counters);
+          mail_post(p.mail, 1, ne, p.counters);
+        }
+      }
+      return;
+    }
+    if (blockIdx.x == 0 && tid == 0) p.counters[CNT_ABORT] = 0;
+  }
+  const u32 n = (u32)(ns + ne);
+
+  // ---- the minibatches of the CTA's items
+  i64 b_first = 0, b_count = 1;
+  if (BATCHED && base < n) {
+    const u32 last = min(n, base + kItems) - 1;
+    if (warp < 2) {  // two warp-wide searches side by side: 32 pivots a round
+      const i64 g = warp == 0 ? base : last;
+      i64 lo = 0, end = p.G;
+      while (end - lo > 1) {
+        const i64 step = (end - lo + 31) >> 5, idx = lo + (i64)(lane + 1) * step;
+        const bool le = idx < end && fused_item_off(p, idx) <= g;
+        const i64 hits = __popc(__ballot_sync(0xffffffffu, le));
+        lo += hits * step;
+        end = min(end, lo + step);
+      }
+      if (lane == 0) s_range[warp] = lo;
+    }
+    __syncthreads();
+    b_first = s_range[0];
+    b_count = s_range[1] - b_first + 1;
+    if (b_count <= kFuWindow) {
+      for (u32 j = tid; j <= b_count; j += kFuThreads) {
+        const i64 s = __ldg(p.seeds_ptr + b_first + j);
+        s_seeds[j] = (u32)s;
+        s_off[j] = (u32)(s + fused_edges_begin(p, b_first + j, s));
+      }
+    }
+    __syncthreads();
+  }
+  const bool windowed = b_count <= kFuWindow;
+  // minibatch of item g: its item offset, first seed and the offset of the next one's seeds
+  struct Where {
+    i64 batch;
+    u32 begin, seeds, next_seeds, next_begin;
+    bool ok;  // the offsets are those of a minibatch (they come from the caller): nothing is accessed otherwise
+  };
+  auto where = [&](u32 g) {
+    Where w;
+    if (windowed) {
+      u32 lo = 0, hi = (u32)b_count;
+      while (hi - lo > 1) {
+        const u32 mid = (lo + hi) >> 1;
+        if (s_off[mid] <= g) lo = mid;
+        else hi = mid;
+      }
+      w.batch = b_first + lo;
+      w.begin = s_off[lo];
+      w.seeds = s_seeds[lo];
+      w.next_seeds = s_seeds[lo + 1];
+      w.next_begin = s_off[lo + 1];
+    } else {
+      i64 lo = b_first, hi = b_first + b_count;
+      while (hi - lo > 1) {
+        const i64 mid = (lo + hi) >> 1;
+        if (fused_item_off(p, mid) <= (i64)g) lo = mid;
+        else hi = mid;
+      }
+      w.batch = lo;
+      w.seeds = (u32)__ldg(p.seeds_ptr + lo);
+      w.next_seeds = (u32)__ldg(p.seeds_ptr + lo + 1);
+      w.begin = (u32)fused_item_off(p, lo);
+      w.next_begin = (u32)fused_item_off(p, lo + 1);
+    }
+    w.ok = w.begin <= g && g < w.next_begin && w.next_begin <= n && w.seeds <= w.begin && w.seeds <= w.next_seeds &&
+           w.next_seeds <= (u32)ns && w.next_seeds - w.seeds <= w.next_begin - w.begin;
+    return w;
+  };
+
+  // ---- insert
+  u32 id[R], slot[R], batch0[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const u32 g = base + r * kFuThreads + tid;
+    i64 v = -1;
+    u32 region = 0, size = fused_bucket0(n, 1);
+    batch0[r] = 0;
+    if (g < n) {
+      if (BATCHED) {
+        const Where w = where(g);
+        const u32 lc = g - w.begin, seeds = w.next_seeds - w.seeds;
+        if (w.ok) v = lc < seeds ? __ldg(p.first + w.seeds + lc) : __ldg(p.second + (g - w.next_seeds));
+        region = fused_bucket0(w.begin, (u32)w.batch);
+        size = fused_bucket0(w.next_begin, (u32)w.batch + 1) - region;
+        batch0[r] = w.begin;
+      } else {
+        v = g < (u32)p.S ? __ldg(p.first + g) : __ldg(p.second + (g - (u32)p.S));
+      }
+      if (!valid_id(v)) raise_error(p.counters, GSB_ERR_INDEX_RANGE, g);
+    }
+    id[r] = valid_id(v) ? (u32)v : kFuNone;
+    slot[r] = kFuNone;
+    if (id[r] != kFuNone) slot[r] = region + fused_home(id[r], size);
+  }
+  // the home buckets of up to two items are in flight at once; an insertion is one read and one atomic almost always
+  constexpr int kAhead = R < 2 ? R : 2;
+#pragma unroll
+  for (int r0 = 0; r0 < R; r0 += kAhead) {
+    u64 word[kAhead][4];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+      if (slot[r0 + q] != kFuNone) load_bucket(p.table, slot[r0 + q], word[q]);
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      const int r = r0 + q;
+      if (slot[r] == kFuNone) continue;
+      const u32 g = base + r * kFuThreads + tid;
+      const u64 mine = p.epoch | ((u64)id[r] << kFuPosBits) | (u64)g;
+      u32 bucket = slot[r];
+      u32 at = claim_in_bucket(p, bucket, word[q], mine);
+      if (at == kFuNone) {
+        u32 lo = 0, end = fused_bucket0(n, 1);  // the buckets of the item's region
+        if (BATCHED) {
+          const Where w = where(g);
+          lo = fused_bucket0(w.begin, (u32)w.batch);
+          end = fused_bucket0(w.next_begin, (u32)w.batch + 1);
+        }
+        for (u32 probe = lo; at == kFuNone && probe < end; ++probe) {
+          bucket = bucket + 1 == end ? lo : bucket + 1;
+          u64 more[4];
+          load_bucket(p.table, bucket, more);
+          at = claim_in_bucket(p, bucket, more, mine);
+        }
+        if (at == kFuNone) raise_error(p.counters, GSB_ERR_TABLE_FULL, g);  // more slots than items: cannot happen
+      }
+      slot[r] = at;
+    }
+  }
+  for (i64 j = (i64)blockIdx.x * kFuThreads + tid; j < p.copy_n; j += (i64)gridDim.x * kFuThreads)
+    p.copy_dst[j] = __ldg(p.copy_src + j);
+  grid_barrier(p, p.barrier_base + gridDim.x);
+
+  // ---- flag
+  unsigned bits[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const u32 g = base + r * kFuThreads + tid;
+    u32 ref = kFuNone;
+    if (slot[r] != kFuNone) ref = (u32)(__ldcg(p.table + slot[r]) & kFuPosMask);
+    if (!BATCHED && p.col_index && g < (u32)p.S) p.seed_ref[g] = ref;
+    slot[r] = ref;  // from here on: the first position of the item's id
+    bits[r] = __ballot_sync(0xffffffffu, ref == g);
+    if (lane == 0) s_group[r * kFuWarps + warp] = __popc(bits[r]);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    u32 carry = 0;
+#pragma unroll
+    for (int q = 0; q < kFuWarps * R; q += 32) {
+      const u32 at = q + lane;
+      const u32 c = at < kFuWarps * R ? s_group[at] : 0;
+      u32 inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+      }
+      if (at < kFuWarps * R) s_group[at] = carry + inc - c;
+      carry += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) p.totals[blockIdx.x] = carry;
+  }
+  __syncthreads();
+  if (lane == 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const u32 g = base + r * kFuThreads + warp * 32;
+      if (g < n) p.packed[g >> 5] = ((u64)s_group[r * kFuWarps + warp] << 32) | (u64)bits[r];
+    }
+  }
+  grid_barrier(p, p.barrier_base + 2ull * gridDim.x);
+
+  // ---- emit
+  u32 all;
+  {
+    const u32 t = tid < gridDim.x ? __ldcg(p.totals + tid) : 0;
+    u32 inc = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    u32 before = 0;
+    all = 0;
+#pragma unroll
+    for (int w = 0; w < kFuWarps; ++w) {
+      if (w < (int)warp) before += s_warp[w];
+      all += s_warp[w];
+    }
+    s_prefix[tid] = before + inc - t;
+    __syncthreads();
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    p.counters[CNT_UNIQUE] = all;
+    if (BATCHED) p.counters[CNT_NNZ] = ne;
+    mail_post(p.mail, 0, all, p.counters);
+    if (BATCHED) mail_post(p.mail, 1, ne, p.counters);
+  }
+  auto rank_of = [&](u32 pos) {
+    const u64 w = __ldcg(p.packed + (pos >> 5));
+    return s_prefix[pos / kItems] + (u32)(w >> 32) + __popc((u32)w & ((1u << (pos & 31)) - 1u));
+  };
+  u64 own[R], of_ref[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const u32 g = base + r * kFuThreads + tid;
+    own[r] = 0;
+    of_ref[r] = 0;
+    if (g < n && slot[r] < n) of_ref[r] = __ldcg(p.packed + (slot[r] >> 5));
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const u32 g = base + r * kFuThreads + tid;
+    if (g >= n) continue;
+    i64 rank = -1;
+    const u32 ref = slot[r];
+    if (ref < n) rank = s_prefix[ref / kItems] + (u32)(of_ref[r] >> 32) + __popc((u32)of_ref[r] & ((1u << (ref & 31)) - 1u));
+    if (ref == g) p.out_unique[rank] = (i64)id[r];
+    if (BATCHED) {
+      if (p.out_second) {
+        const Where w = where(g);
+        const u32 lc = g - w.begin;
+        if (w.ok && lc >= w.next_seeds - w.seeds)
+          p.out_second[g - w.next_seeds] = rank < 0 ? -1 : rank - (i64)rank_of(batch0[r]);
+      }
+    } else if (g >= (u32)p.S) {
+      const u32 e = g - (u32)p.S;
+      if (p.out_second) p.out_second[e] = rank;
+      if (p.out_col) {
+        const i64 c = __ldg(p.col_index + e);
+        u32 cref = kFuNone;
+        if ((u64)c < (u64)p.S) cref = __ldcg(p.seed_ref + c);
+        p.out_col[e] = cref < n ? (i64)rank_of(cref) : (i64)-1;
+      }
+    }
+  }
+  if (BATCHED) {
+    for (i64 b = (i64)blockIdx.x * kFuThreads + tid; b <= p.G; b += (i64)gridDim.x * kFuThreads) {
+      const i64 s = __ldg(p.seeds_ptr + b), e = fused_edges_begin(p, b, s);
+      if (p.out_indices_ptr) p.out_indices_ptr[b] = e;
+      p.out_unique_ptr[b] = (u64)(s + e) < (u64)n ? (i64)rank_of((u32)(s + e)) : (i64)all;
+    }
+  }
+}
+
+// ---- host side ------------------------------------------------------------------------------------------------------
+static int items_per_thread(i64 n, int max_ctas) {
+  int r = 1;
+  while (r < 16 && (n + (i64)kFuThreads * r - 1) / ((i64)kFuThreads * r) > max_ctas) r <<= 1;
+  return r;
+}
+
+template <bool BATCHED>
+static const void* fused_kernel(int r) {
+  switch (r) {
+    case 1: return (const void*)k_fused_unique<1, BATCHED>;
+    case 2: return (const void*)k_fused_unique<2, BATCHED>;
+    case 4: return (const void*)k_fused_unique<4, BATCHED>;
+    case 8: return (const void*)k_fused_unique<8, BATCHED>;
+    default: return (const void*)k_fused_unique<16, BATCHED>;
+  }
+}
+
+// CTAs that are resident at once on the current device (0: cooperative launches are not available).
+static int resident_ctas(int device) {
+  static int known[64];
+  if (device < 0 || device >= 64) return 0;
+  if (known[device] == 0) {
+    int coop = 0, sms = 0, a = 0, b = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_fused_unique<16, false>, kFuThreads, 0) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused_unique<16, true>, kFuThreads, 0) != cudaSuccess)
+      (void)cudaGetLastError();
+    const int ctas = min(min(a, b) * sms, kFuThreads);  // one thread per CTA total in the scan
+    known[device] = coop && ctas > 0 ? ctas : -1;
+  }
+  return known[device] > 0 ? known[device] : 0;
+}
+
+bool fused_unique_suits(gsb_ctx* ctx, i64 n, i64 G) {
+  return n > 0 && n <= kFusedUniqueMaxItems && G <= kFusedUniqueMaxBatches &&
+         n <= (i64)resident_ctas(ctx_device(ctx)) * kFuThreads * 16;
+}
+
+template <bool BATCHED>
+static int launch_fused(gsb_ctx* ctx, cudaStream_t stream, FusedParams p, i64 n) {
+  const int r = items_per_thread(n, resident_ctas(ctx_device(ctx)));
+  const int grid = grid_for(n, kFuThreads * r);
+  void* ws;
+  const size_t packed_bytes = ((size_t)n / 32 + 2) * 8;
+  int st = ctx_reserve_workspace(ctx, packed_bytes + sizeof(u32) * (size_t)(kFuThreads + (p.col_index ? p.S : 0)), &ws);
+  if (st != GSB_OK) return st;
+  p.packed = (u64*)ws;
+  p.totals = (u32*)((char*)ws + packed_bytes);
+  p.seed_ref = p.totals + kFuThreads;
+  u32 epoch;
+  st = ctx_epoch_table(ctx, 4 * (i64)fused_bucket0((u32)n, (u32)(BATCHED ? p.G : 1)), kFuEpochs, stream, &p.table, &epoch, &p.barrier);
+  if (st != GSB_OK) return st;
+  p.epoch = (u64)epoch << (32 + kFuPosBits);
+  p.barrier_base = ctx_barrier_base(ctx, 2ull * (u64)grid);
+  p.counters = ctx_counters(ctx);
+  p.max_polls = (int)ctx_option(ctx, GSB_OPT_MAX_POLLS);
+  ScopedKernelTimer timer(ctx, KID_RELABEL, stream);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kFuThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  void* args[] = {&p};
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, fused_kernel<BATCHED>(r), args);
+  if (e != cudaSuccess) {  // nothing ran: the barrier word stands where it stood
+    ctx_barrier_base(ctx, 0ull - 2ull * (u64)grid);
+    return cuda_fail(ctx, e, __FILE__, __LINE__);
+  }
+  return GSB_OK;
+}
+
+int fused_unique_single(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64 S, const i64* second, i64 E,
+                        const i64* col_index, i64* out_unique, i64* out_second, i64* out_col, const i64* copy_src,
+                        i64* copy_dst, i64 copy_n, Mail mail) {
+  FusedParams p{};
+  p.first = first;
+  p.second = second;
+  p.S = S;
+  p.E = E;
+  p.out_unique = out_unique;
+  p.out_second = out_second;
+  p.col_index = out_col ? col_index : nullptr;
+  p.out_col = out_col;
+  p.copy_src = copy_src;
+  p.copy_dst = copy_dst;
+  p.copy_n = copy_src && copy_dst ? copy_n : 0;
+  p.mail = mail;
+  return launch_fused<false>(ctx, stream, p, S + E);
+}
+
+int fused_unique_batched(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L, i64 seeds_bound, i64 edges_bound,
+                         const i64* sub_indptr, i64* out_indices_ptr, i64* out_unique, i64* out_unique_ptr,
+                         i64* out_relabeled, Mail mail) {
+  FusedParams p{};
+  p.first = L.seeds;
+  p.second = L.indices;
+  p.S = seeds_bound;
+  p.E = edges_bound;
+  p.out_unique = out_unique;
+  p.out_second = out_relabeled;
+  p.seeds_ptr = L.seeds_ptr;
+  p.indices_ptr = sub_indptr ? nullptr : L.indices_ptr;
+  p.sub_indptr = sub_indptr;
+  p.out_indices_ptr = sub_indptr ? out_indices_ptr : nullptr;
+  p.out_unique_ptr = out_unique_ptr;
+  p.G = L.G;
+  p.mail = mail;
+  return launch_fused<true>(ctx, stream, p, seeds_bound + edges_bound);
+}
+
+}  // namespace gsb

@@ -301,6 +301,33 @@ FUNCTION(relabel, 3) {
   return tuple_of(wrap(std::move(unique)), list);
 }
 
+// ---- relabelling of a sampled graph: (ctx, col_ids, rows, cols | None, indptr to copy | None)
+//      -> (unique, rows, cols | None, copy | None), or None when gsb_graph_relabel does not serve the call
+FUNCTION(graph_relabel, 5) {
+  gsb_ctx* ctx = context(a[0]);
+  IDS(col_ids, a[1], "col_ids");
+  IDS(rows, a[2], "rows");
+  IDS_OR_NONE(cols, a[3], "cols");
+  IDS_OR_NONE(indptr, a[4], "indptr");
+  const c10::Device dev = device_of(col_ids);
+  const int64_t S = col_ids.numel(), E = rows.numel();
+  if (cols.given() && cols.numel() != E) type_error("cols must have one entry per row id");
+  Tensor unique = empty(S + E, dev), out_rows = empty(E, dev), out_cols, copy;
+  if (cols.given()) out_cols = empty(E, dev);
+  if (indptr.given()) copy = empty(indptr.numel(), dev);
+  int64_t count = 0;
+  int st;
+  {
+    NoGil free;
+    st = gsb_graph_relabel(ctx, stream(), col_ids.ids(), S, rows.ids(), E, cols.ids(), indptr.ids(), mut(copy),
+                           indptr.given() ? indptr.numel() : 0, mut(unique), mut(out_rows), mut(out_cols), &count);
+  }
+  if (st == GSB_ERR_UNSUPPORTED) Py_RETURN_NONE;
+  check(ctx, st, "gsb_graph_relabel");
+  trim(unique, count);
+  return tuple_of(wrap(std::move(unique)), wrap(std::move(out_rows)), wrap(std::move(out_cols)), wrap(std::move(copy)));
+}
+
 // ---- random walk: (ctx, indptr, indices, seeds, length, seed, layout, walker_offset) -> trace [W, L + 1]
 FUNCTION(random_walk, 8) {
   gsb_ctx* ctx = context(a[0]);
@@ -670,7 +697,8 @@ PyObject* set_error_class(PyObject*, PyObject* cls) {
 
 #define ENTRY(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ENTRY(col_slicing),        ENTRY(col_sampling),
-                         ENTRY(relabel),            ENTRY(random_walk),
+                         ENTRY(relabel),            ENTRY(graph_relabel),
+                         ENTRY(random_walk),
                          ENTRY(col_row_slicing),    ENTRY(list_sampling),
                          ENTRY(sddmm),              ENTRY(segment_sum_csc),
                          ENTRY(segment_sum_coo),    ENTRY(segment_normalize_csc),

@@ -176,8 +176,18 @@ extern "C" int gsb_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* co
     if (rel_ok) {
       const i64* first = num_item_arrays == 2 ? item_ptrs_host[0] : nullptr;
       const i64 S = num_item_arrays == 2 ? item_lens_host[0] : 0;
-      st = unique_relabel_packed(ctx, stream, first, S, last, last_len, out_unique,
-                                 num_relabel ? out_relabel_ptrs_host[0] : nullptr, unique_host);
+      i64* out_rel = num_relabel ? out_relabel_ptrs_host[0] : nullptr;
+      if (fused_unique_suits(ctx, n, 1)) {
+        const Mail mail = ctx_mail(ctx);
+        st = fused_unique_single(ctx, stream, first, S, last, last_len, nullptr, out_unique, out_rel, nullptr, nullptr,
+                                 nullptr, 0, mail);
+        if (st != GSB_OK) return st;
+        i64 unique = 0;
+        st = ctx_mail_result(ctx, stream, mail, 1, &unique);
+        *unique_host = unique;
+      } else {
+        st = unique_relabel_packed(ctx, stream, first, S, last, last_len, out_unique, out_rel, unique_host);
+      }
       if (st != GSB_ERR_INDEX_RANGE) return st;
       // an id >= 2^32 - 1 (or a negative one, which the wide path reports again): fall through
     }
@@ -228,6 +238,28 @@ extern "C" int gsb_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* co
   st = ctx_mail_result(ctx, stream, mail, 1, &unique);
   *unique_host = unique;
   return st;
+}
+
+extern "C" int gsb_graph_relabel(gsb_ctx* ctx, void* stream_, const int64_t* col_ids, int64_t S, const int64_t* rows,
+                                 int64_t E, const int64_t* cols, const int64_t* copy_src, int64_t* copy_dst,
+                                 int64_t copy_n, int64_t* out_unique, int64_t* out_rows, int64_t* out_cols,
+                                 int64_t* unique_host) {
+  GSB_ENTER(ctx);
+  GSB_REQUIRE(S >= 0 && E >= 0 && copy_n >= 0 && unique_host, GSB_ERR_INVALID_ARGUMENT);
+  GSB_REQUIRE((S == 0 || col_ids) && (E == 0 || (rows && out_rows)) && (copy_n == 0 || (copy_src && copy_dst)),
+              GSB_ERR_INVALID_ARGUMENT);
+  GSB_REQUIRE((cols == nullptr) == (out_cols == nullptr) || E == 0, GSB_ERR_INVALID_ARGUMENT);
+  GSB_REQUIRE(S + E == 0 || out_unique, GSB_ERR_INVALID_ARGUMENT);
+  if (ctx_option(ctx, GSB_OPT_TABLE_SLOTS) != 0 || !fused_unique_suits(ctx, S + E, 1)) return GSB_ERR_UNSUPPORTED;
+  cudaStream_t stream = (cudaStream_t)stream_;
+  const Mail mail = ctx_mail(ctx);
+  int st = fused_unique_single(ctx, stream, col_ids, S, rows, E, cols, out_unique, out_rows, out_cols, copy_src, copy_dst,
+                               copy_n, mail);
+  if (st != GSB_OK) return st;
+  i64 unique = 0;
+  st = ctx_mail_result(ctx, stream, mail, 1, &unique);
+  *unique_host = unique;
+  return st == GSB_ERR_INDEX_RANGE ? GSB_ERR_UNSUPPORTED : st;  // ids beyond 32 bits: the general form takes them
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -532,15 +532,13 @@ class Graph:
             if self.val_col_ids_ is not None:
                 col_ids = col_ids[self.val_col_ids_]
             row_indices = self.row_ids_[self.csc_.indices] if self.row_ids_ is not None else self.csc_.indices
-            frontier, (relabeled,) = ops.relabel([col_ids, row_indices], [row_indices])
-            return (frontier, frontier.numel(), col_ids.numel(), self.csc_.indptr.clone(), relabeled, self.csc_.e_ids,
-                    "csc")
+            frontier, relabeled, _, indptr = ops.graph_relabel(col_ids, row_indices, indptr=self.csc_.indptr)
+            return frontier, frontier.numel(), col_ids.numel(), indptr, relabeled, self.csc_.e_ids, "csc"
         if self.csr_ is not None or self.coo_ is not None:
             if self.coo_ is None:
                 self.coo_ = self._csc2coo(self.csr_, False)
-            coo_col = col_ids[self.coo_.col]
             coo_row = self.row_ids_[self.coo_.row] if self.row_ids_ is not None else self.coo_.row
-            frontier, (rel_col, rel_row) = ops.relabel([col_ids, coo_row], [coo_col, coo_row])
+            frontier, rel_row, rel_col, _ = ops.graph_relabel(col_ids, coo_row, cols=self.coo_.col)
             return (frontier, frontier.numel(), col_ids.numel(), rel_row, rel_col, self.coo_.e_ids, "coo")
         _fatal("Error in Relabel!")
 

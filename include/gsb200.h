@@ -80,6 +80,7 @@ GSB_API int gsb_check_device_status(gsb_ctx* ctx, void* stream);
  *                               to a power of two) instead of sizing it from the item count — a table that is too
  *                               small reports GSB_ERR_TABLE_FULL; 0 (default) = automatic;
  *  GSB_OPT_RELABEL_PATH         how gsb_sage_hop / gsb_batch_unique_relabel find first occurrences: 0 (default) =
+ *                               one cooperative launch for calls it suits (up to 2^21 items), else
  *                               direct-address tables when all tables of the call are L2-sized (32 MiB), else the
  *                               partitioned form (items bucketed by a hash of their id, one shared-memory table per
  *                               bucket) for calls of at least 2^19 items whose minibatches average at most 2^19
@@ -199,6 +200,18 @@ GSB_API int gsb_unique_relabel(gsb_ctx* ctx, void* stream, const int64_t* const*
                                const int64_t* item_lens_host, int num_item_arrays, int64_t* out_unique,
                                const int64_t* const* relabel_ptrs_host, const int64_t* relabel_lens_host,
                                int64_t* const* out_relabel_ptrs_host, int num_relabel, int64_t* unique_host);
+
+/* What gs::Graph::Relabel does with a sampled graph (src/graph.cc:785-839), in one launch: out_unique =
+ * unique(cat(col_ids, rows)) in first-occurrence order; out_rows[e] = position of rows[e] in it; with `cols` (COO
+ * form: cols[e] = position of edge e's column in col_ids) also out_cols[e] = position of col_ids[cols[e]]; copies
+ * copy_n words from copy_src to copy_dst along the way (the offsets a CSC result hands out).  out_unique holds S + E
+ * entries.  Waits for the number of distinct ids.  GSB_ERR_UNSUPPORTED — nothing usable was written — for calls beyond
+ * 2^21 items or with ids of more than 32 bits, which gsb_unique_relabel serves.
+ */
+GSB_API int gsb_graph_relabel(gsb_ctx* ctx, void* stream, const int64_t* col_ids, int64_t S, const int64_t* rows,
+                              int64_t E, const int64_t* cols, const int64_t* copy_src, int64_t* copy_dst,
+                              int64_t copy_n, int64_t* out_unique, int64_t* out_rows, int64_t* out_cols,
+                              int64_t* unique_host);
 
 /* ---- uniform random walk ----------------------------------------------------------------------
  * Replaces gs::impl::fusion::FusedRandomWalkCUDA / _RandomWalkKernel

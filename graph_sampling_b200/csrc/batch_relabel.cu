@@ -613,10 +613,13 @@ constexpr i64 kDirectAutoBytes = 32ll << 20;
 // the hash regions take five, which a call of a few thousand items (one minibatch relabelled on its own) feels more
 // than the per-item work it saves — about 20 ns per 1 000 items.
 constexpr i64 kPartitionAutoItems = 1ll << 19;
-// ... and a minibatch with more than 256 buckets (above 524 288 items) leaves the fast paths of the partitioning passes
-// (a tile counts and sorts 256 buckets in shared memory), so calls whose AVERAGE minibatch is larger than that keep the
-// hash regions too.
-constexpr i64 kPartitionAutoMaxMinibatch = 256ll * kBucketTarget;
+// ... and a minibatch with more buckets than a tile counts in shared memory (1 024, above 2 097 152 items) leaves the fast
+// paths of the partitioning passes, so calls whose AVERAGE minibatch is larger than that keep the hash regions too.  (With
+// a window of 256 buckets, a call of 500 minibatches of 740 000 items ran on the hash regions: 28.6 ms of the hop.)
+constexpr i64 kPartitionAutoMaxMinibatch = 1024ll * kBucketTarget;
+// The counting sampler flushes its per-bucket counts once per 128 columns: with more than 256 buckets a minibatch that is
+// an atomic for every other item, and the separate counting pass is cheaper.
+constexpr i64 kSamplerCountsMaxMinibatch = 256ll * kBucketTarget;
 static inline bool partition_suits(i64 n_cap, i64 G) {
   return n_cap >= kPartitionAutoItems && n_cap / (G > 0 ? G : 1) <= kPartitionAutoMaxMinibatch;
 }
@@ -873,7 +876,7 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
   const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
   const bool fused = path == 0 && fused_unique_suits(ctx, n_cap, G);
   const bool direct_small = (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes && num_nodes > 0;
-  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && (path == 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
+  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && n_cap / G <= kSamplerCountsMaxMinibatch && (path == 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
     st = sage_hop_sampler_counts(ctx, stream, indptr, indices, num_nodes, seeds, seeds_ptr, batch_ids, G, S, k, cap,
                                  replace, (u64)seed, out_indptr, out_indices, out_select, out_indices_ptr, out_unique,
                                  out_unique_ptr, out_relabeled, mail);

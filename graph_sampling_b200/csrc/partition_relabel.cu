@@ -47,7 +47,10 @@ constexpr int kPartPerThread = 16;
 constexpr int kPartTile = kPartThreads * kPartPerThread;        // items per CTA of the count pass
 constexpr int kScatterPerThread = 8;
 constexpr int kScatterTile = kPartThreads * kScatterPerThread;  // items per CTA of the scatter pass
-constexpr int kWindow = 256;                                    // buckets a tile counts in shared memory
+// Buckets of one minibatch that a tile counts in shared memory: 256 serve minibatches of up to 524 288 items; calls with
+// larger ones take the instantiations of 1 024 (2 097 152 items), whose arrays cost the narrow calls resident CTAs.
+constexpr int kNarrowWindow = 256;
+constexpr int kWideWindow = 1024;
 constexpr u32 kNoBucket = 0xFFFFFFFFu;
 constexpr int kResolveThreads = 256;
 constexpr int kResolvePer = 12;                          // items per thread of a bucket that fits shared memory
@@ -138,6 +141,7 @@ __device__ __forceinline__ Located locate(const BatchLayout& L, i64 g) {
 
 constexpr int kMaxSegments = 8;  // minibatches a tile may touch and still be handled segment by segment
 
+template <int kWindow>
 __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n_bound, i64* counters) {
   __shared__ u32 s_cnt[kWindow];
   if (counters[CNT_ABORT] != 0) return;
@@ -294,6 +298,7 @@ __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const
 
 // A tile's items are first sorted by bucket in shared memory (their rank inside the tile's share of a bucket is what
 // the counting atomic returns), so the copy to global memory writes whole runs of consecutive words.
+template <int kWindow>
 __global__ void __launch_bounds__(kPartThreads) k_part_scatter(PartLayout P, i64 n_bound, i64* counters) {
   __shared__ u64 s_stage[kScatterTile];
   __shared__ uint16_t s_which[kScatterTile];
@@ -301,13 +306,14 @@ __global__ void __launch_bounds__(kPartThreads) k_part_scatter(PartLayout P, i64
   __shared__ u32 s_off[kWindow];
   __shared__ u32 s_base[kWindow];
   __shared__ i64 s_scan[33];
-  static_assert(kWindow == kPartThreads, "one window entry per thread in the scan");
+  constexpr int kPer = kWindow / kPartThreads;  // consecutive window entries per thread in the scan
+  static_assert(kPer * kPartThreads == kWindow, "the threads cover the window");
   if (counters[CNT_ABORT] != 0) return;
   const BatchLayout& L = P.L;
   const i64 n = min(L.item_off[L.G], n_bound);
   const i64 tile_base = (i64)blockIdx.x * kScatterTile;
   if (tile_base >= n) return;
-  s_cnt[threadIdx.x] = 0;
+  for (int i = threadIdx.x; i < kWindow; i += kPartThreads) s_cnt[i] = 0;
   const BatchUniform u = load_batch<false>(L, L.item_off, batch_of_warp(L.item_off, L.G, tile_base));
   const TileBatch t = tile_batch(L, u);
   const u32 lc0 = (u32)(tile_base - u.begin);
@@ -349,12 +355,22 @@ __global__ void __launch_bounds__(kPartThreads) k_part_scatter(PartLayout P, i64
   }
   __syncthreads();
   {
-    const u32 c = s_cnt[threadIdx.x];
+    u32 c[kPer], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      c[j] = s_cnt[threadIdx.x * kPer + j];
+      sum += c[j];
+    }
     i64 total;
-    s_off[threadIdx.x] = (u32)block_exclusive_scan<kPartThreads>((i64)c, s_scan, &total);
-    if (c != 0)
-      s_base[threadIdx.x] = __ldg(P.bucket_start + t.bucket0 + threadIdx.x) +
-                            atomicAdd(P.bucket_cursor + t.bucket0 + threadIdx.x, c);
+    u32 run = (u32)block_exclusive_scan<kPartThreads>((i64)sum, s_scan, &total);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const u32 w = threadIdx.x * kPer + j;
+      s_off[w] = run;
+      run += c[j];
+      if (c[j] != 0)
+        s_base[w] = __ldg(P.bucket_start + t.bucket0 + w) + atomicAdd(P.bucket_cursor + t.bucket0 + w, c[j]);
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -740,6 +756,7 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   const PartArrays arrays = carve(L, n_cap, bucket_cap, ws);
   const PartLayout& P = arrays.P;
   const RankArrays& R = arrays.R;
+  const bool wide = n_cap / L.G > (i64)kNarrowWindow * kBucketTarget * 3 / 4;  // the larger minibatches of a ragged call count
   static bool attr_set[64] = {};
   const int dev = ctx_device(ctx);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
@@ -750,7 +767,8 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
     GSB_CUDA_OK(cudaMemsetAsync(P.bucket_count, 0, sizeof(u32) * (size_t)(bucket_cap + 1), stream));
     {
       ScopedKernelTimer timer(ctx, KID_PART_COUNT, stream);
-      k_part_count<<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
+      if (wide) k_part_count<kWideWindow><<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
+      else k_part_count<kNarrowWindow><<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
     }
     GSB_LAUNCH_OK();
     {
@@ -761,7 +779,8 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   }
   {
     ScopedKernelTimer timer(ctx, KID_PART_SCATTER, stream);
-    k_part_scatter<<<grid_for(n_cap, kScatterTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
+    if (wide) k_part_scatter<kWideWindow><<<grid_for(n_cap, kScatterTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
+    else k_part_scatter<kNarrowWindow><<<grid_for(n_cap, kScatterTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
   }
   GSB_LAUNCH_OK();
   {

@@ -14,7 +14,7 @@
 //             sampler does this counting itself while it holds the ids (slice_sample.cu, COUNT) — the buckets are then
 //             laid out from the bound seeds x (1 + fanout) before it runs — and this pass is not launched;
 //   scan      bucket sizes -> bucket starts (one CTA; in the one-call hop part of k_part_after_sampler);
-//   scatter   tiles of 2 048 items: sorted by bucket in shared memory, a range reserved per bucket with one global
+//   scatter   tiles of 2 048 or 8 192 items: sorted by bucket in shared memory, a range reserved per bucket with one global
 //             atomic, whole runs of (id << 32 | position inside the minibatch) copied out — the order inside a bucket
 //             does not matter, the table keeps the smallest position per id;
 //   resolve   one CTA per bucket: the bucket's items stay in registers; position-min insert into a shared-memory
@@ -45,14 +45,14 @@ typedef uint32_t u32;
 constexpr int kPartThreads = 256;
 constexpr int kPartPerThread = 16;
 constexpr int kPartTile = kPartThreads * kPartPerThread;        // items per CTA of the count pass
-constexpr int kScatterPerThread = 8;
-constexpr int kScatterTile = kPartThreads * kScatterPerThread;  // items per CTA of the scatter pass
+constexpr int scatter_smem(int tile, int window) { return tile * 8 + window * 8; }  // bytes of the scatter pass
 // Buckets of one minibatch that a tile counts in shared memory: 256 serve minibatches of up to 524 288 items; calls with
 // larger ones take the instantiations of 1 024 (2 097 152 items), whose arrays cost the narrow calls resident CTAs.
 constexpr int kNarrowWindow = 256;
 constexpr int kWideWindow = 1024;
 constexpr u32 kNoBucket = 0xFFFFFFFFu;
 constexpr int kResolveThreads = 256;
+constexpr int kResolveAhead = 2;                         // items of a thread whose first probes are in flight together
 constexpr int kResolvePer = 12;                          // items per thread of a bucket that fits shared memory
 constexpr int kBucketSlots = 6144;                       // shared-memory table of a resolve CTA: 48 KB
 constexpr int kBucketSmemItems = kBucketSlots / 2 - 16;  // largest bucket that fits it at two slots per item
@@ -297,30 +297,33 @@ __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const
 }
 
 // A tile's items are first sorted by bucket in shared memory (their rank inside the tile's share of a bucket is what
-// the counting atomic returns), so the copy to global memory writes whole runs of consecutive words.
-template <int kWindow>
-__global__ void __launch_bounds__(kPartThreads) k_part_scatter(PartLayout P, i64 n_bound, i64* counters) {
-  __shared__ u64 s_stage[kScatterTile];
-  __shared__ uint16_t s_which[kScatterTile];
-  __shared__ u32 s_cnt[kWindow];
-  __shared__ u32 s_off[kWindow];
-  __shared__ u32 s_base[kWindow];
+// the counting atomic returned), so the copy to global memory writes whole runs of consecutive words.  The bucket of a
+// staged item is computed from its id again instead of being kept beside it.
+// THREADS x PER items per tile.  Tiles of 2 048 suit minibatches of some ten thousand items (a tile that straddles
+// minibatches takes the per-item path); with hundreds of buckets per minibatch such a tile reserves a range — a global
+// atomic, on a cursor that every other tile of the minibatch wants too — for every five items, so large minibatches take
+// tiles of 8 192.
+template <int WINDOW, int THREADS, int PER>
+__global__ void __launch_bounds__(THREADS) k_part_scatter(PartLayout P, i64 n_bound, i64* counters) {
+  constexpr int kTile = THREADS * PER;
+  constexpr int kPer = WINDOW / THREADS > 0 ? WINDOW / THREADS : 1;  // consecutive window entries per thread in the scan
+  extern __shared__ __align__(16) u64 s_stage[];                     // [kTile] items, then [WINDOW] two arrays
+  u32* s_cnt = reinterpret_cast<u32*>(s_stage + kTile);              // counts, then where the bucket's run starts in the tile
+  u32* s_delta = s_cnt + WINDOW;                                     // where it starts in the bucket array minus that
   __shared__ i64 s_scan[33];
-  constexpr int kPer = kWindow / kPartThreads;  // consecutive window entries per thread in the scan
-  static_assert(kPer * kPartThreads == kWindow, "the threads cover the window");
   if (counters[CNT_ABORT] != 0) return;
   const BatchLayout& L = P.L;
   const i64 n = min(L.item_off[L.G], n_bound);
-  const i64 tile_base = (i64)blockIdx.x * kScatterTile;
+  const i64 tile_base = (i64)blockIdx.x * kTile;
   if (tile_base >= n) return;
-  for (int i = threadIdx.x; i < kWindow; i += kPartThreads) s_cnt[i] = 0;
+  for (int i = threadIdx.x; i < WINDOW; i += THREADS) s_cnt[i] = 0;
   const BatchUniform u = load_batch<false>(L, L.item_off, batch_of_warp(L.item_off, L.G, tile_base));
   const TileBatch t = tile_batch(L, u);
   const u32 lc0 = (u32)(tile_base - u.begin);
-  const u32 here = (u32)min((i64)kScatterTile, n - tile_base);
-  const bool uniform = (u64)lc0 + here <= (u64)t.items && t.parts <= (u32)kWindow;
+  const u32 here = (u32)min((i64)kTile, n - tile_base);
+  const bool uniform = (u64)lc0 + here <= (u64)t.items && t.parts <= (u32)WINDOW;
   if (!uniform) {  // a tile over several minibatches: every item straight to its place
-    for (u32 i = threadIdx.x; i < here; i += kPartThreads) {
+    for (u32 i = threadIdx.x; i < here; i += THREADS) {
       const Located it = locate(L, tile_base + i);
       if (!valid_id(it.node)) {  // never bucketed: marked for the ranking passes
         raise_error(counters, GSB_ERR_INDEX_RANGE, tile_base + i);
@@ -332,60 +335,69 @@ __global__ void __launch_bounds__(kPartThreads) k_part_scatter(PartLayout P, i64
     }
     return;
   }
-  i64 node[kScatterPerThread];
+  i64 node[PER];
 #pragma unroll
-  for (int q = 0; q < kScatterPerThread; ++q) {
-    const u32 i = q * kPartThreads + threadIdx.x;
+  for (int q = 0; q < PER; ++q) {
+    const u32 i = q * THREADS + threadIdx.x;
     node[q] = i < here ? tile_item(t, lc0 + i) : -1;
   }
   __syncthreads();
-  u32 where[kScatterPerThread];  // bucket (inside the minibatch) << 16 | rank inside the tile's share of it
+  u32 id[PER], where[PER];  // where: bucket (inside the minibatch) << 16 | rank inside the tile's share of it
 #pragma unroll
-  for (int q = 0; q < kScatterPerThread; ++q) {
+  for (int q = 0; q < PER; ++q) {
     where[q] = kNoBucket;
+    id[q] = (u32)node[q];
     if (!valid_id(node[q])) {
-      if (q * kPartThreads + threadIdx.x < here) {  // never bucketed: marked for the ranking passes
-        raise_error(counters, GSB_ERR_INDEX_RANGE, tile_base + q * kPartThreads + threadIdx.x);
-        P.ref[tile_base + q * kPartThreads + threadIdx.x] = 0xFFFFFFFFu;
+      if (q * THREADS + threadIdx.x < here) {  // never bucketed: marked for the ranking passes
+        raise_error(counters, GSB_ERR_INDEX_RANGE, tile_base + q * THREADS + threadIdx.x);
+        P.ref[tile_base + q * THREADS + threadIdx.x] = 0xFFFFFFFFu;
       }
       continue;
     }
-    const u32 w = bucket_of_id((u32)node[q], t.parts);
-    where[q] = (w << 16) | atomicAdd(&s_cnt[w], 1u);  // at most 2 048 items per tile: the rank fits 16 bits
+    const u32 w = bucket_of_id(id[q], t.parts);
+    where[q] = (w << 16) | atomicAdd(&s_cnt[w], 1u);  // at most 8 192 items per tile: the rank fits 16 bits
   }
   __syncthreads();
+  u32 staged;
   {
     u32 c[kPer], sum = 0;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
-      c[j] = s_cnt[threadIdx.x * kPer + j];
+      const int w = threadIdx.x * kPer + j;
+      c[j] = w < WINDOW ? s_cnt[w] : 0;
       sum += c[j];
     }
-    i64 total;
-    u32 run = (u32)block_exclusive_scan<kPartThreads>((i64)sum, s_scan, &total);
+    // the reservations are in flight during the scan
+    u32 base[kPer];
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
-      const u32 w = threadIdx.x * kPer + j;
-      s_off[w] = run;
+      const u32 w = t.bucket0 + threadIdx.x * kPer + j;
+      base[j] = 0;
+      if (c[j] != 0) base[j] = __ldg(P.bucket_start + w) + atomicAdd(P.bucket_cursor + w, c[j]);
+    }
+    i64 total;
+    u32 run = (u32)block_exclusive_scan<THREADS>((i64)sum, s_scan, &total);
+    staged = (u32)total;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int w = threadIdx.x * kPer + j;
+      if (w < WINDOW) {
+        s_cnt[w] = run;
+        s_delta[w] = base[j] - run;
+      }
       run += c[j];
-      if (c[j] != 0)
-        s_base[w] = __ldg(P.bucket_start + t.bucket0 + w) + atomicAdd(P.bucket_cursor + t.bucket0 + w, c[j]);
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < kScatterPerThread; ++q) {
+  for (int q = 0; q < PER; ++q) {
     if (where[q] == kNoBucket) continue;
-    const u32 w = where[q] >> 16;
-    const u32 at = s_off[w] + (where[q] & 0xFFFFu);
-    s_stage[at] = ((u64)node[q] << 32) | (u64)(lc0 + q * kPartThreads + threadIdx.x);
-    s_which[at] = (uint16_t)w;
+    s_stage[s_cnt[where[q] >> 16] + (where[q] & 0xFFFFu)] = ((u64)id[q] << 32) | (u64)(lc0 + q * THREADS + threadIdx.x);
   }
   __syncthreads();
-  const u32 staged = s_off[kWindow - 1] + s_cnt[kWindow - 1];
-  for (u32 i = threadIdx.x; i < staged; i += kPartThreads) {
-    const u32 w = s_which[i];
-    P.bucketed[s_base[w] + (i - s_off[w])] = s_stage[i];
+  for (u32 i = threadIdx.x; i < staged; i += THREADS) {
+    const u64 w = s_stage[i];
+    P.bucketed[s_delta[bucket_of_id((u32)(w >> 32), t.parts)] + i] = w;
   }
 }
 
@@ -409,18 +421,12 @@ __device__ __forceinline__ u32 table_insert_min(u64* table, u32 size, u32 h, u64
   return 0;  // cannot happen: the table has more slots than the bucket has items
 }
 
-// Shared-memory table as two 32-bit arrays — ids and smallest positions — so that the probe loop, which the lanes of
-// a warp leave at different times, is a 32-bit load and two compares per step, and both atomics are native 32-bit
-// shared-memory operations.  Returns the slot of the id.
-__device__ __forceinline__ u32 smem_claim_slot(u32* keys, u32 size, u32 h, u32 id) {
-  for (;;) {  // ends: the table has more slots than the bucket has items
-    u32 k = *(volatile u32*)(keys + h);
-    if (k == 0xFFFFFFFFu) k = atomicCAS(keys + h, 0xFFFFFFFFu, id);  // ids are below 2^32 - 1
-    if (k == 0xFFFFFFFFu || k == id) return h;
-    h = h + 1 == size ? 0 : h + 1;
-  }
-}
-
+// Shared-memory table as two 32-bit arrays, ids and smallest positions: the probe loop is a 32-bit load and two compares per
+// step, and both atomics are native 32-bit shared-memory operations.
+// What the kernel waits for (162 M items in 2.29 ms): half of it is the 4-byte scatter of `ref`, one L2 sector per item
+// (1.18 ms with the same words written in bucket order); probing costs a tenth and the position minimum nothing that can be
+// measured.  All twelve items of a thread probing side by side with a compare-and-swap per round was slower (3.8 against
+// 2.4 ms per launch): without the read in front of it every repeat of a frequent id is an atomic on the same word.
 // Measured and not kept: five CTAs per SM instead of four (40 KB tables of 2.5 slots per item, 48 registers): 2.61
 // against 2.62 ms per 1 000 minibatches — the kernel is not short of resident warps.
 __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout P, i64* counters) {
@@ -456,21 +462,40 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
       __syncthreads();
       u32 slot[kResolvePer];
 #pragma unroll
-      for (int q = 0; q < kResolvePer; ++q) {
-        slot[q] = 0;
-        if ((u32)(q * kResolveThreads) >= n) break;  // uniform
-        if (w[q] != kEmptyWord) {
-          const u32 id = (u32)(w[q] >> 32);
-          slot[q] = smem_claim_slot(keys, size, slot_of_id(id, size), id);
-          atomicMin(first + slot[q], (u32)w[q]);
+      for (int q0 = 0; q0 < kResolvePer; q0 += kResolveAhead) {
+        if ((u32)(q0 * kResolveThreads) >= n) break;  // uniform
+        u32 found[kResolveAhead];
+#pragma unroll
+        for (int q = 0; q < kResolveAhead; ++q) {
+          slot[q0 + q] = slot_of_id((u32)(w[q0 + q] >> 32), size);
+          found[q] = *(volatile u32*)(keys + slot[q0 + q]);
+        }
+#pragma unroll
+        for (int q = 0; q < kResolveAhead; ++q)
+          if (found[q] == 0xFFFFFFFFu && w[q0 + q] != kEmptyWord)
+            found[q] = atomicCAS(keys + slot[q0 + q], 0xFFFFFFFFu, (u32)(w[q0 + q] >> 32));  // ids are below 2^32 - 1
+#pragma unroll
+        for (int q = 0; q < kResolveAhead; ++q) {
+          if (w[q0 + q] == kEmptyWord) continue;
+          const u32 id = (u32)(w[q0 + q] >> 32);
+          u32 k = found[q], h = slot[q0 + q];
+          while (k != 0xFFFFFFFFu && k != id) {  // ends: the table has more slots than the bucket has items
+            h = h + 1 == size ? 0 : h + 1;
+            k = *(volatile u32*)(keys + h);
+            if (k == 0xFFFFFFFFu) k = atomicCAS(keys + h, 0xFFFFFFFFu, id);
+          }
+          slot[q0 + q] = h;
+          atomicMin(first + h, (u32)w[q0 + q]);
         }
       }
       __syncthreads();
+      u32 ref_of[kResolvePer];
 #pragma unroll
-      for (int q = 0; q < kResolvePer; ++q) {
-        if ((u32)(q * kResolveThreads) >= n) break;
-        if (w[q] != kEmptyWord) ref[(u32)w[q]] = first[slot[q]];
-      }
+      for (int q = 0; q < kResolvePer; ++q)
+        if ((u32)(q * kResolveThreads) < n) ref_of[q] = first[slot[q]];
+#pragma unroll
+      for (int q = 0; q < kResolvePer; ++q)
+        if ((u32)(q * kResolveThreads) < n && w[q] != kEmptyWord) ref[(u32)w[q]] = ref_of[q];
       continue;
     }
     // oversized bucket (many repeats of a few ids): a table of its own in global memory
@@ -761,6 +786,8 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   const int dev = ctx_device(ctx);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     GSB_CUDA_OK(cudaFuncSetAttribute(k_part_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, kBucketSlots * 8));
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_scatter<kWideWindow, 512, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     scatter_smem(8192, kWideWindow)));
     attr_set[dev] = true;
   }
   if (!counted) {
@@ -779,8 +806,12 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   }
   {
     ScopedKernelTimer timer(ctx, KID_PART_SCATTER, stream);
-    if (wide) k_part_scatter<kWideWindow><<<grid_for(n_cap, kScatterTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
-    else k_part_scatter<kNarrowWindow><<<grid_for(n_cap, kScatterTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
+    if (wide)
+      k_part_scatter<kWideWindow, 512, 16><<<grid_for(n_cap, 8192), 512, scatter_smem(8192, kWideWindow), stream>>>(
+          P, n_cap, counters);
+    else
+      k_part_scatter<kNarrowWindow, 256, 8><<<grid_for(n_cap, 2048), 256, scatter_smem(2048, kNarrowWindow), stream>>>(
+          P, n_cap, counters);
   }
   GSB_LAUNCH_OK();
   {

@@ -7,6 +7,7 @@
 
 typedef int64_t i64;
 typedef unsigned long long u64;
+typedef uint32_t u32;
 
 #define GSB_CUDA_OK(expr)                                 \
   do {                                                    \
@@ -127,10 +128,7 @@ int ctx_check_device_error(gsb_ctx* ctx, cudaStream_t stream);
 // Epoch-tagged hash table of the single-launch unique + relabel (fused_unique.cu): at least `slots` 64-bit words kept by
 // the context, never cleared between calls.  *epoch (1 .. epochs - 1) is new for every call; when the epochs are used up,
 // and when the table grows, it is zeroed.  Bounded by what kFusedUniqueMaxItems needs (64 MB), freed with the context.
-int ctx_epoch_table(gsb_ctx* ctx, i64 slots, uint32_t epochs, cudaStream_t stream, u64** table, uint32_t* epoch,
-                    u64** barrier);
-// The grid-barrier word counts arrivals for ever; returns its value before the coming launch and adds the launch's.
-u64 ctx_barrier_base(gsb_ctx* ctx, u64 arrivals);
+int ctx_epoch_table(gsb_ctx* ctx, i64 slots, uint32_t epochs, cudaStream_t stream, u64** table, uint32_t* epoch);
 // Waits until everything queued on `stream` so far is done and returns the `n` counters starting at `first` (a copy in
 // page-locked memory, written by a one-warp kernel that the host spins on).
 int ctx_fetch_counters(gsb_ctx* ctx, cudaStream_t stream, int first, int n, const i64** out);

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "grid_sync.cuh"
 #include "scan.cuh"
 
 struct gsb_ctx {
@@ -143,8 +144,7 @@ int ctx_direct_tables(gsb_ctx* ctx, i64 count, i64 num_nodes, cudaStream_t strea
   return GSB_OK;
 }
 
-int ctx_epoch_table(gsb_ctx* ctx, i64 slots, uint32_t epochs, cudaStream_t stream, u64** table, uint32_t* epoch,
-                    u64** barrier) {
+int ctx_epoch_table(gsb_ctx* ctx, i64 slots, uint32_t epochs, cudaStream_t stream, u64** table, uint32_t* epoch) {
   if (slots > ctx->epoch_slots) {
     GSB_CUDA_OK(cudaDeviceSynchronize());
     if (ctx->epoch_table) GSB_CUDA_OK(cudaFree(ctx->epoch_table));
@@ -163,14 +163,48 @@ int ctx_epoch_table(gsb_ctx* ctx, i64 slots, uint32_t epochs, cudaStream_t strea
   }
   *table = ctx->epoch_table;
   *epoch = ctx->table_epoch;
-  *barrier = (u64*)(ctx->counters + CNT_NUM);
   return GSB_OK;
 }
 
-u64 ctx_barrier_base(gsb_ctx* ctx, u64 arrivals) {
-  const u64 base = ctx->barrier_arrivals;
-  ctx->barrier_arrivals += arrivals;
-  return base;
+int ctx_resident_ctas(gsb_ctx* ctx, const void* kernel, int threads, size_t smem, int (&known)[64]) {
+  const int device = ctx->device;
+  if (device < 0 || device >= 64) return 0;
+  if (known[device] == 0) {
+    int coop = 0, sms = 0, per_sm = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
+      (void)cudaGetLastError();
+    known[device] = coop && per_sm * sms > 0 ? per_sm * sms : -1;
+  }
+  return known[device] > 0 ? known[device] : 0;
+}
+
+GridSync ctx_grid_sync(gsb_ctx* ctx, int grid, int barriers) {
+  const GridSync g{(u64*)(ctx->counters + CNT_NUM), ctx->barrier_arrivals, ctx->counters,
+                   (int)ctx->options[GSB_OPT_MAX_POLLS]};
+  ctx->barrier_arrivals += (u64)grid * (u64)barriers;
+  return g;
+}
+
+int launch_cooperative(gsb_ctx* ctx, cudaStream_t stream, const void* kernel, int grid, int threads, size_t smem,
+                       void** args, const GridSync& sync) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
+  if (e != cudaSuccess) {
+    ctx->barrier_arrivals = sync.base;  // nothing ran: the barrier word stands where it stood
+    return cuda_fail(ctx, e, __FILE__, __LINE__);
+  }
+  return GSB_OK;
 }
 
 i64* ctx_counters(gsb_ctx* ctx) { return ctx->counters; }

@@ -1,6 +1,7 @@
 // Sparse-format conversion: CSC -> COO (column id per edge) and COO -> CSC / CSR (stable sort by
 // the key coordinate, edge permutation, offsets).
 #include "common.cuh"
+#include "grid_sync.cuh"
 #include "radix_sort.cuh"
 
 namespace gsb {
@@ -67,6 +68,212 @@ __global__ void __launch_bounds__(kFmtThreads) k_gather_i64(const i64* __restric
     dst[e] = src[idx ? idx[e] : e];
 }
 
+// ---- COO -> CSC / CSR in one launch ------------------------------------------------------------------------------
+// Stable counting sort of E edges by key with the offsets over all keys, as one cooperative kernel with a grid barrier
+// between its steps.  The slices that layer-wise sampling converts have 10^4 to 10^6 edges: the radix sort's fifteen
+// launches (count, scan, three passes of three, gather, copies) were 60 us of kernels and as much again between them.
+//
+//   per digit of up to 11 bits (one to three of them):
+//     count    CTA c owns the c-th stretch of the current order, warp w the w-th part of that; 16-bit counts per warp and
+//              digit in shared memory; the CTA's counts go to matrix[digit][c]
+//     scan     a warp per digit turns its row of the matrix into exclusive prefixes, and notes the digit's total
+//     place    every warp walks its part again, 32 items at a time ranked with __match_any_sync, and writes each item to
+//              digit start + CTA prefix + warp prefix + rank: stable, since everything is numbered in order
+//   along the way, the offsets: counts per key (one reduction per edge) during the first scan, totals per CTA of keys
+//   during the first place, offsets written during the next step.
+// An item is (key << 32 | edge).  The last place step writes the permutation and the other coordinate directly.
+constexpr int kConvThreads = 1024;
+constexpr int kConvWarps = kConvThreads / 32;
+constexpr int kConvMaxBins = 2048;
+constexpr i64 kConvMaxEdges = 4ll << 20;  // 28 000 edges per CTA: a warp's count fits 16 bits
+
+struct ConvParams {
+  const i64* key;
+  const i64* other;
+  i64 E, num_keys;
+  int digits, digit_bits;
+  u64* items[2];   // [E] each
+  u32* matrix;     // [bins][CTAs]
+  u32* bin_total;  // [bins]
+  u32* counts;     // [num_keys]
+  u32* key_total;  // [CTAs]
+  i64* out_indptr;
+  i64* out_other;
+  i64* out_perm;
+  i64* counters;
+  GridSync sync;
+};
+
+__global__ void __launch_bounds__(kConvThreads) k_coo2csc(const __grid_constant__ ConvParams p) {
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  uint16_t* s_count = reinterpret_cast<uint16_t*>(s_dyn);  // [warps][bins]
+  __shared__ u32 s_start[kConvMaxBins];                    // where the CTA's items of a digit go
+  __shared__ u32 s_warp[kConvWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ctas = gridDim.x;
+  const int bins = 1 << p.digit_bits;
+  const u32 E = (u32)p.E;
+  const u32 per_cta = (u32)(((p.E + ctas - 1) / ctas + 32 * kConvWarps - 1) / (32 * kConvWarps) * (32 * kConvWarps));
+  const u32 per_warp = per_cta / kConvWarps;
+  const u32 begin = min(E, (u32)blockIdx.x * per_cta + (u32)warp * per_warp), end = min(E, begin + per_warp);
+  const i64 keys_per_cta = (p.num_keys + ctas - 1) / ctas;
+  const i64 key_begin = min(p.num_keys, (i64)blockIdx.x * keys_per_cta), key_end = min(p.num_keys, key_begin + keys_per_cta);
+  const unsigned lt = (1u << lane) - 1u;
+  uint16_t* my_count = s_count + warp * bins;
+  u32 barrier = 0;
+
+  auto load_item = [&](int digit, u32 i) -> u64 {
+    if (digit > 0) return __ldcg(p.items[(digit - 1) & 1] + i);
+    i64 k = __ldg(p.key + i);
+    if ((u64)k >= (u64)p.num_keys) {
+      raise_error(p.counters, GSB_ERR_INDEX_RANGE, i);
+      k = 0;
+    }
+    return ((u64)k << 32) | (u64)i;
+  };
+  // inclusive scan over the CTA of one value per thread, and its total
+  auto block_scan = [&](u32 v, u32* total) -> u32 {
+    u32 inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    __syncthreads();
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    u32 before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kConvWarps; ++w) {
+      const u32 t = s_warp[w];
+      if (w < warp) before += t;
+      all += t;
+    }
+    *total = all;
+    return before + inc;
+  };
+
+  for (i64 k = key_begin + tid; k < key_end; k += kConvThreads) p.counts[k] = 0;
+  for (int digit = 0; digit < p.digits; ++digit) {
+    const int shift = 32 + digit * p.digit_bits;
+    const u32 mask = (u32)bins - 1;
+    // ---- count
+    for (int i = tid; i < kConvWarps * bins / 2; i += kConvThreads) reinterpret_cast<u32*>(s_count)[i] = 0;
+    __syncthreads();
+    for (u32 i0 = begin; i0 < end; i0 += 32) {
+      const u32 i = i0 + lane;
+      const bool valid = i < end;
+      const u32 d = valid ? (u32)(load_item(digit, i) >> shift) & mask : 0xFFFFFFFFu;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      if (valid && (peers & lt) == 0) my_count[d] = (uint16_t)(my_count[d] + __popc(peers));
+      __syncwarp();
+    }
+    __syncthreads();
+    for (int b = tid; b < bins; b += kConvThreads) {
+      u32 run = 0;
+      for (int w = 0; w < kConvWarps; ++w) {  // counts -> prefixes over the warps
+        const u32 c = s_count[w * bins + b];
+        s_count[w * bins + b] = (uint16_t)run;
+        run += c;
+      }
+      p.matrix[(size_t)b * ctas + blockIdx.x] = run;
+    }
+    grid_barrier(p.sync, ++barrier);
+    // ---- scan of the matrix rows; counts per key
+    for (int b = (int)blockIdx.x * kConvWarps + warp; b < bins; b += ctas * kConvWarps) {
+      u32* row = p.matrix + (size_t)b * ctas;
+      u32 carry = 0;
+      for (int c0 = 0; c0 < ctas; c0 += 32) {
+        const int c = c0 + lane;
+        const u32 v = c < ctas ? __ldcg(row + c) : 0;
+        u32 inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += t;
+        }
+        if (c < ctas) row[c] = carry + inc - v;
+        carry += __shfl_sync(0xffffffffu, inc, 31);
+      }
+      if (lane == 0) p.bin_total[b] = carry;
+    }
+    if (digit == 0)
+      for (u32 i = begin + lane; i < end; i += 32) {
+        const i64 k = __ldg(p.key + i);
+        atomicAdd(p.counts + ((u64)k < (u64)p.num_keys ? k : 0), 1u);
+      }
+    grid_barrier(p.sync, ++barrier);
+    // ---- place
+    {
+      const int per = bins > kConvThreads ? bins / kConvThreads : 1;  // consecutive digits per thread: 1 or 2
+      u32 v[2] = {0, 0}, total;
+      for (int j = 0; j < per; ++j)
+        if (tid * per + j < bins) v[j] = __ldcg(p.bin_total + tid * per + j);
+      u32 run = block_scan(v[0] + v[1], &total) - v[0] - v[1];
+      for (int j = 0; j < per; ++j) {
+        const int b = tid * per + j;
+        if (b < bins) s_start[b] = run + __ldcg(p.matrix + (size_t)b * ctas + blockIdx.x);
+        run += v[j];
+      }
+      __syncthreads();
+    }
+    const bool last = digit == p.digits - 1;
+    for (u32 i0 = begin; i0 < end; i0 += 32) {
+      const u32 i = i0 + lane;
+      const bool valid = i < end;
+      const u64 item = valid ? load_item(digit, i) : 0;
+      const u32 d = valid ? (u32)(item >> shift) & mask : 0xFFFFFFFFu;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      u32 base = 0;
+      if (valid) base = my_count[d];
+      __syncwarp();
+      if (valid && (peers & lt) == 0) my_count[d] = (uint16_t)(base + __popc(peers));
+      __syncwarp();
+      if (valid) {
+        const u32 pos = s_start[d] + base + __popc(peers & lt);
+        if (last) {
+          const u32 e = (u32)item;
+          p.out_perm[pos] = (i64)e;
+          p.out_other[pos] = __ldg(p.other + e);
+        } else {
+          p.items[digit & 1][pos] = item;
+        }
+      }
+    }
+    // ---- totals of the CTA's keys (their counts are complete since the last barrier)
+    if (digit == 0) {
+      u32 sum = 0, total;
+      for (i64 k = key_begin + tid; k < key_end; k += kConvThreads) sum += __ldcg(p.counts + k);
+      block_scan(sum, &total);
+      if (tid == 0) p.key_total[blockIdx.x] = total;
+    }
+    if (!last || digit == 0) grid_barrier(p.sync, ++barrier);
+    if (digit == 0) {  // offsets: the CTA's prefix, then its keys, a thread's share of consecutive ones at a time
+      u32 before = 0, total;
+      for (int c = tid; c < (int)blockIdx.x; c += kConvThreads) before += __ldcg(p.key_total + c);
+      block_scan(before, &total);
+      u32 run = total;
+      constexpr int kPer = 4;
+      for (i64 k0 = key_begin; k0 < key_end; k0 += kConvThreads * kPer) {
+        u32 v[kPer], sum = 0, all;
+        const i64 mine = k0 + (i64)tid * kPer;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          v[j] = mine + j < key_end ? __ldcg(p.counts + mine + j) : 0;
+          sum += v[j];
+        }
+        u32 at = run + block_scan(sum, &all) - sum;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          if (mine + j < key_end) p.out_indptr[mine + j] = (i64)at;
+          at += v[j];
+        }
+        run += all;
+      }
+      if (blockIdx.x == 0 && tid == 0) p.out_indptr[p.num_keys] = p.E;
+    }
+  }
+}
+
 }  // namespace gsb
 
 using namespace gsb;
@@ -91,6 +298,63 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
   GSB_REQUIRE(key_sorted || E == 0 || out_perm, GSB_ERR_INVALID_ARGUMENT);
   cudaStream_t stream = (cudaStream_t)stream_;
   const int grid = min(grid_for(E, kFmtThreads), kNumSMs * 8);
+  int bits = 1;
+  while (bits < 63 && (1ll << bits) < num_keys) ++bits;
+  // One cooperative launch while a warp's share of the edges fits its 16-bit counts (and keys fit three digits);
+  // beyond that the passes are long enough for launches of their own.
+  if (!key_sorted && E > 0 && E <= kConvMaxEdges && bits <= 32 && num_keys > 0) {
+    ConvParams p{};
+    p.digits = (bits + 10) / 11;
+    p.digit_bits = max(5, (bits + p.digits - 1) / p.digits);
+    const int bins = 1 << p.digit_bits;
+    const size_t smem = sizeof(uint16_t) * (size_t)kConvWarps * (size_t)bins;
+    static int resident[64];
+    static bool attr_set[64];
+    const int dev = ctx_device(ctx);
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+      GSB_CUDA_OK(cudaFuncSetAttribute(k_coo2csc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(sizeof(uint16_t) * kConvWarps * kConvMaxBins)));
+      attr_set[dev] = true;
+    }
+    const int ctas = min(kNumSMs, ctx_resident_ctas(ctx, (const void*)k_coo2csc, kConvThreads,
+                                                    sizeof(uint16_t) * kConvWarps * kConvMaxBins, resident));
+    // two items per thread at least: fewer CTAs make the barriers and the matrix of a short list cheaper; the offsets of a
+    // long key range want CTAs too
+    const i64 want = max((E + 2 * kConvThreads - 1) / (2 * kConvThreads), num_keys / (16 * kConvThreads));
+    const int conv_grid = (int)max((i64)1, min((i64)ctas, want));
+    if (ctas > 0 && (E + conv_grid - 1) / conv_grid + 32 * kConvWarps <= 65535ll) {
+      auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+      const size_t item_bytes = p.digits > 1 ? al(sizeof(u64) * (size_t)E) : 0;
+      const size_t matrix_bytes = al(sizeof(u32) * (size_t)bins * (size_t)conv_grid);
+      void* ws;
+      int st = ctx_reserve_workspace(ctx, item_bytes * (p.digits > 2 ? 2 : 1) + matrix_bytes + al(sizeof(u32) * (size_t)bins) +
+                                              al(sizeof(u32) * (size_t)num_keys) + 4096, &ws);
+      if (st != GSB_OK) return st;
+      char* at = (char*)ws;
+      p.items[0] = (u64*)at;
+      p.items[1] = (u64*)(at + (p.digits > 2 ? item_bytes : 0));
+      at += item_bytes * (p.digits > 2 ? 2 : 1);
+      p.matrix = (u32*)at;
+      at += matrix_bytes;
+      p.bin_total = (u32*)at;
+      at += al(sizeof(u32) * (size_t)bins);
+      p.key_total = (u32*)at;
+      at += 4096;
+      p.counts = (u32*)at;
+      p.key = key;
+      p.other = other;
+      p.E = E;
+      p.num_keys = num_keys;
+      p.out_indptr = out_indptr;
+      p.out_other = out_other;
+      p.out_perm = out_perm;
+      p.counters = ctx_counters(ctx);
+      p.sync = ctx_grid_sync(ctx, conv_grid, p.digits == 1 ? 3 : 3 * p.digits - 1);
+      ScopedKernelTimer timer(ctx, KID_FORMAT, stream);
+      void* args[] = {&p};
+      return launch_cooperative(ctx, stream, (const void*)k_coo2csc, conv_grid, kConvThreads, smem, args, p.sync);
+    }
+  }
   GSB_CUDA_OK(cudaMemsetAsync(out_indptr, 0, sizeof(i64) * (size_t)(num_keys + 1), stream));
   if (E > 0) {
     k_count_keys<<<grid, kFmtThreads, 0, stream>>>(key, E, num_keys, out_indptr, ctx_counters(ctx));
@@ -104,8 +368,6 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
     GSB_CUDA_OK(cudaMemcpyAsync(out_other, other, sizeof(i64) * (size_t)E, cudaMemcpyDeviceToDevice, stream));
     return GSB_OK;
   }
-  int bits = 1;
-  while (bits < 63 && (1ll << bits) < num_keys) ++bits;
   void* ws;
   const size_t sort_bytes = radix_sort_scratch_bytes(E);
   st = ctx_reserve_workspace(ctx, sort_bytes + sizeof(u64) * (size_t)E + 256, &ws);

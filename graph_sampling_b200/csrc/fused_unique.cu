@@ -26,11 +26,10 @@
 // What bounds it now: the chain bucket read -> CAS -> CAS of the slowest lane of every warp, item after item.
 #include "batch_table.cuh"
 #include "common.cuh"
+#include "grid_sync.cuh"
 #include "scan.cuh"
 
 namespace gsb {
-
-typedef uint32_t u32;
 
 constexpr int kFuThreads = 512;
 constexpr int kFuWarps = kFuThreads / 32;
@@ -64,35 +63,10 @@ struct FusedParams {
   u64* packed;    // [items / 32 + 1]  first occurrences of the CTA before the word << 32 | bits
   u32* totals;    // [CTAs]
   u32* seed_ref;  // [S] first position of every id of `first` (only with col_index)
-  u64* barrier;
-  u64 barrier_base;
+  GridSync sync;
   i64* counters;
-  int max_polls;
   Mail mail;
 };
-
-__device__ __forceinline__ u64 ld_acquire_u64(const u64* p) {
-  u64 v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Every CTA of the (cooperatively launched, hence resident) grid arrives; the wait is bounded like every other.
-__device__ __forceinline__ void grid_barrier(const FusedParams& p, u64 target) {
-  __syncthreads();
-  if (threadIdx.x == 0) {  // release / acquire, cumulative over what the CTA did before its barrier
-    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(p.barrier) : "memory");
-    int polls = 0;
-    while ((i64)(ld_acquire_u64(p.barrier) - target) < 0) {
-      if (++polls > p.max_polls) {
-        raise_error(p.counters, GSB_ERR_LOOKBACK_TIMEOUT, blockIdx.x);
-        break;
-      }
-      if (polls > 64) __nanosleep(20);
-    }
-  }
-  __syncthreads();
-}
 
 // Buckets of a region: minibatch b, whose items are [begin, next), has the buckets [bucket0(begin, b), bucket0(next, b + 1)),
 // at least 0.75 per item.
@@ -159,9 +133,9 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
     ns = __ldg(p.seeds_ptr + p.G);
     ne = fused_edges_begin(p, p.G, ns);
     if (ns > p.S || ne > p.E || ns < 0 || ne < 0) {  // every CTA sees the same: nobody waits for anybody
+      grid_arrive(p.sync, 2);
       if (tid == 0) {
         raise_error(p.counters, GSB_ERR_CAPACITY, ns > p.S ? ns : ne);
-        atomicAdd(p.barrier, 2ull);
         if (blockIdx.x == 0) {
           p.counters[CNT_ABORT] = 1;
           mail_post(p.mail, 0, 0, p.counters);
@@ -302,7 +276,7 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
   }
   for (i64 j = (i64)blockIdx.x * kFuThreads + tid; j < p.copy_n; j += (i64)gridDim.x * kFuThreads)
     p.copy_dst[j] = __ldg(p.copy_src + j);
-  grid_barrier(p, p.barrier_base + gridDim.x);
+  grid_barrier(p.sync, 1);
 
   // ---- flag
   unsigned bits[R];
@@ -342,7 +316,7 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
       if (g < n) p.packed[g >> 5] = ((u64)s_group[r * kFuWarps + warp] << 32) | (u64)bits[r];
     }
   }
-  grid_barrier(p, p.barrier_base + 2ull * gridDim.x);
+  grid_barrier(p.sync, 2);
 
   // ---- emit
   u32 all;
@@ -437,31 +411,21 @@ static const void* fused_kernel(int r) {
   }
 }
 
-// CTAs that are resident at once on the current device (0: cooperative launches are not available).
-static int resident_ctas(int device) {
-  static int known[64];
-  if (device < 0 || device >= 64) return 0;
-  if (known[device] == 0) {
-    int coop = 0, sms = 0, a = 0, b = 0;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_fused_unique<16, false>, kFuThreads, 0) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fused_unique<16, true>, kFuThreads, 0) != cudaSuccess)
-      (void)cudaGetLastError();
-    const int ctas = min(min(a, b) * sms, kFuThreads);  // one thread per CTA total in the scan
-    known[device] = coop && ctas > 0 ? ctas : -1;
-  }
-  return known[device] > 0 ? known[device] : 0;
+static int resident_ctas(gsb_ctx* ctx) {
+  static int single[64], batched[64];
+  const int a = ctx_resident_ctas(ctx, (const void*)k_fused_unique<16, false>, kFuThreads, 0, single);
+  const int b = ctx_resident_ctas(ctx, (const void*)k_fused_unique<16, true>, kFuThreads, 0, batched);
+  return min(min(a, b), kFuThreads);  // one thread per CTA total in the scan
 }
 
 bool fused_unique_suits(gsb_ctx* ctx, i64 n, i64 G) {
   return n > 0 && n <= kFusedUniqueMaxItems && G <= kFusedUniqueMaxBatches &&
-         n <= (i64)resident_ctas(ctx_device(ctx)) * kFuThreads * 16;
+         n <= (i64)resident_ctas(ctx) * kFuThreads * 16;
 }
 
 template <bool BATCHED>
 static int launch_fused(gsb_ctx* ctx, cudaStream_t stream, FusedParams p, i64 n) {
-  const int r = items_per_thread(n, resident_ctas(ctx_device(ctx)));
+  const int r = items_per_thread(n, resident_ctas(ctx));
   const int grid = grid_for(n, kFuThreads * r);
   void* ws;
   const size_t packed_bytes = ((size_t)n / 32 + 2) * 8;
@@ -471,29 +435,14 @@ static int launch_fused(gsb_ctx* ctx, cudaStream_t stream, FusedParams p, i64 n)
   p.totals = (u32*)((char*)ws + packed_bytes);
   p.seed_ref = p.totals + kFuThreads;
   u32 epoch;
-  st = ctx_epoch_table(ctx, 4 * (i64)fused_bucket0((u32)n, (u32)(BATCHED ? p.G : 1)), kFuEpochs, stream, &p.table, &epoch, &p.barrier);
+  st = ctx_epoch_table(ctx, 4 * (i64)fused_bucket0((u32)n, (u32)(BATCHED ? p.G : 1)), kFuEpochs, stream, &p.table, &epoch);
   if (st != GSB_OK) return st;
   p.epoch = (u64)epoch << (32 + kFuPosBits);
-  p.barrier_base = ctx_barrier_base(ctx, 2ull * (u64)grid);
   p.counters = ctx_counters(ctx);
-  p.max_polls = (int)ctx_option(ctx, GSB_OPT_MAX_POLLS);
+  p.sync = ctx_grid_sync(ctx, grid, 2);
   ScopedKernelTimer timer(ctx, KID_RELABEL, stream);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(kFuThreads);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeCooperative;
-  attr.val.cooperative = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
   void* args[] = {&p};
-  const cudaError_t e = cudaLaunchKernelExC(&cfg, fused_kernel<BATCHED>(r), args);
-  if (e != cudaSuccess) {  // nothing ran: the barrier word stands where it stood
-    ctx_barrier_base(ctx, 0ull - 2ull * (u64)grid);
-    return cuda_fail(ctx, e, __FILE__, __LINE__);
-  }
-  return GSB_OK;
+  return launch_cooperative(ctx, stream, fused_kernel<BATCHED>(r), grid, kFuThreads, 0, args, p.sync);
 }
 
 int fused_unique_single(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64 S, const i64* second, i64 E,

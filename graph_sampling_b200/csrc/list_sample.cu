@@ -4,11 +4,12 @@
 // A-Res key log2(u)/w for the weighted case (w <= 0 can never beat a positive weight) — and the k
 // best keys win; ties go to the smaller position; the output is in descending key order, which is
 // what the reference's descending stable sort yields (src/cuda/list_sampling_probs.cu:56-88).
-// Instead of sorting all N keys to take k of them, the k-th best key is found by an 8-pass (one launch each)
-// most-significant-digit radix SELECT over the 64-bit composite (key << 32 | ~position), the k
-// winners are compacted and only they are sorted.  With replacement: k independent draws, uniform
+// Instead of sorting all N keys to take k of them, the k-th best key is found by a most-significant-digit radix SELECT
+// over the 64-bit composite (key << 32 | ~position), and only the k winners are sorted: one cooperative launch up to
+// k = 4 096 (k_list_select), one launch per pass beyond.  With replacement: k independent draws, uniform
 // or by inverse CDF (src/cuda/list_sampling.cu:35-52, list_sampling_probs.cu:28-55).
 #include "common.cuh"
+#include "grid_sync.cuh"
 #include "philox.cuh"
 #include "radix_sort.cuh"
 #include "scan.cuh"
@@ -20,6 +21,160 @@ constexpr int kListPerThread = 4;
 constexpr int kListTile = kListThreads * kListPerThread;
 constexpr int kCdfChunk = 1024;
 
+__device__ __forceinline__ uint32_t orderable_f32(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+__device__ __forceinline__ u64 list_composite(const float* __restrict__ probs, i64 i, u64 seed) {
+  const uint32_t key = probs ? orderable_f32(ares_key(rand_u32(seed, (u64)i, 0, STREAM_LIST_WEIGHTED), __ldg(probs + i)))
+                             : rand_u32(seed, (u64)i, 0, STREAM_LIST);
+  return ((u64)key << 32) | (u64)(0xFFFFFFFFu - (uint32_t)i);
+}
+
+// Sampling without replacement of k <= kSelectMaxK items in one launch: composites -> radix select, 11 bits per pass, a
+// grid barrier per pass, until the selected bin is needed whole (two or three passes unless keys tie) -> the winners are
+// appended in any order -> CTA 0 sorts and emits them.  Layer-wise sampling makes one such call per layer on a list of a
+// million rows; as thirteen launches it was 140 us, most of it between the launches (30 us now).
+constexpr int kSelectThreads = 1024;
+constexpr int kSelectBins = 2048;
+constexpr int kSelectMaxK = 4096;
+constexpr int kSelectPasses = 6;                   // shifts 53, 42, 31, 20, 9 and 0 (the last digit has nine bits)
+constexpr int kSelectBarriers = kSelectPasses + 2;
+
+struct SelectParams {
+  const float* probs;
+  const i64* data;
+  i64 N, k;
+  u64 seed;
+  u64* composite;    // [N]
+  unsigned* hist;    // [kSelectPasses][kSelectBins]
+  unsigned* found;   // [1]
+  u64* winners;      // [kSelectMaxK]
+  i64* out_data;
+  i64* out_index;
+  i64* counters;
+  GridSync sync;
+};
+
+// One entry of a shared-memory histogram per distinct digit of the warp: all zero-weight items share one key, and plain
+// atomics on one address would serialise the CTA.
+__device__ __forceinline__ void select_count(unsigned* s_hist, unsigned digit, bool counts) {
+  const unsigned peers = __match_any_sync(0xffffffffu, counts ? digit : 0xFFFFFFFFu);
+  if (counts && (int)(__ffs(peers) - 1) == (int)(threadIdx.x & 31)) atomicAdd(&s_hist[digit], (unsigned)__popc(peers));
+}
+
+__global__ void __launch_bounds__(kSelectThreads) k_list_select(const __grid_constant__ SelectParams p) {
+  __shared__ __align__(16) u64 s_win[kSelectMaxK];   // the histogram of a pass, later the winners
+  __shared__ unsigned s_warp[kSelectThreads / 32];
+  __shared__ unsigned s_pick[2];                     // bin, items of it that are needed
+  unsigned* s_hist = reinterpret_cast<unsigned*>(s_win);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const i64 stride = (i64)gridDim.x * kSelectThreads;
+  const i64 rounds = (p.N + stride - 1) / stride;
+  for (i64 i = (i64)blockIdx.x * kSelectThreads + tid; i < kSelectPasses * kSelectBins; i += stride) p.hist[i] = 0;
+  if (blockIdx.x == 0 && tid == 0) *p.found = 0;
+  for (int i = tid; i < kSelectBins; i += kSelectThreads) s_hist[i] = 0;
+  __syncthreads();
+  for (i64 r = 0; r < rounds; ++r) {
+    const i64 i = r * stride + (i64)blockIdx.x * kSelectThreads + tid;
+    const bool valid = i < p.N;
+    const u64 c = valid ? list_composite(p.probs, i, p.seed) : 0;
+    if (valid) p.composite[i] = c;
+    select_count(s_hist, (unsigned)(c >> 53), valid);
+  }
+  u32 barrier = 1;
+  grid_barrier(p.sync, barrier);  // the global histograms are clear
+  u64 prefix = 0, mask = 0;
+  unsigned need = (unsigned)p.k;
+  int pass = 0;
+  for (int shift = 53;; ++pass) {
+    const int bits = pass == kSelectPasses - 1 ? 9 : 11;
+    unsigned* hist = p.hist + pass * kSelectBins;
+    for (int i = tid; i < kSelectBins; i += kSelectThreads)
+      if (s_hist[i]) atomicAdd(hist + i, s_hist[i]);
+    grid_barrier(p.sync, ++barrier);
+    // every CTA picks the bin for itself: thread t owns bins 2t, 2t + 1; `above` counts the items in larger bins
+    {
+      const uint2 h = __ldcg(reinterpret_cast<const uint2*>(hist) + tid);
+      unsigned inc = h.x + h.y;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_down_sync(0xffffffffu, inc, o);
+        if (lane + o < 32) inc += t;
+      }
+      if (lane == 0) s_warp[warp] = inc;
+      __syncthreads();
+      unsigned above = inc - h.x - h.y;
+      for (int w = warp + 1; w < kSelectThreads / 32; ++w) above += s_warp[w];
+      if (above < need && above + h.y >= need) {
+        s_pick[0] = 2 * tid + 1;
+        s_pick[1] = need - above;
+      }
+      above += h.y;
+      if (above < need && above + h.x >= need) {
+        s_pick[0] = 2 * tid;
+        s_pick[1] = need - above;
+      }
+      __syncthreads();
+    }
+    const unsigned bin = s_pick[0];
+    need = s_pick[1];
+    prefix |= (u64)bin << shift;
+    mask |= ((1ull << bits) - 1ull) << shift;
+    const bool whole = __ldcg(hist + bin) == need;  // all composites >= prefix are exactly the winners
+    if (whole || pass == kSelectPasses - 1) break;
+    shift = pass == kSelectPasses - 2 ? 0 : shift - 11;
+    const unsigned digit_mask = pass == kSelectPasses - 2 ? 511u : 2047u;
+    for (int i = tid; i < kSelectBins; i += kSelectThreads) s_hist[i] = 0;
+    __syncthreads();
+    for (i64 r = 0; r < rounds; ++r) {
+      const i64 i = r * stride + (i64)blockIdx.x * kSelectThreads + tid;
+      const u64 c = i < p.N ? p.composite[i] : 0;  // written by this very thread
+      select_count(s_hist, (unsigned)(c >> shift) & digit_mask, i < p.N && (c & mask) == prefix);
+    }
+    __syncthreads();
+  }
+  for (i64 i = (i64)blockIdx.x * kSelectThreads + tid; i < p.N; i += stride) {
+    const u64 c = p.composite[i];
+    if (c < prefix) continue;
+    const unsigned at = atomicAdd(p.found, 1u);
+    if (at < (unsigned)p.k) p.winners[at] = c;
+    else raise_error(p.counters, GSB_ERR_CAPACITY, at);  // cannot happen: composites are distinct
+  }
+  if (blockIdx.x != 0) {  // everybody arrives, only CTA 0 waits: it has the rest to itself
+    __syncthreads();
+    __threadfence();
+    grid_arrive(p.sync, 1);
+    return;
+  }
+  grid_barrier(p.sync, ++barrier);
+  grid_arrive(p.sync, (kSelectBarriers - barrier) * gridDim.x);  // the arrivals of the passes that were not needed
+  int n = 1;
+  while (n < (int)p.k) n <<= 1;
+  for (int i = tid; i < n; i += kSelectThreads) s_win[i] = i < (int)p.k ? __ldcg(p.winners + i) : 0ull;  // 0 sorts last
+  __syncthreads();
+  for (int size = 2; size <= n; size <<= 1) {
+    for (int j = size >> 1; j > 0; j >>= 1) {
+      for (int i = tid; i < n / 2; i += kSelectThreads) {
+        const int lo = 2 * i - (i & (j - 1)), hi = lo + j;
+        const bool desc = (lo & size) == 0;
+        const u64 a = s_win[lo], b = s_win[hi];
+        if ((a < b) == desc) {
+          s_win[lo] = b;
+          s_win[hi] = a;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int i = tid; i < (int)p.k; i += kSelectThreads) {
+    const i64 idx = (i64)(0xFFFFFFFFu - (uint32_t)s_win[i]);
+    p.out_index[i] = idx;
+    p.out_data[i] = __ldg(p.data + idx);
+  }
+}
+
 struct SelectState {
   u64 prefix;     // bits decided so far (high digits)
   i64 remaining;  // how many winners must still come from the undecided bin
@@ -28,18 +183,10 @@ struct SelectState {
   unsigned resolved;  // the selected bin is needed entirely: the threshold is final, later passes have nothing to do
 };
 
-__device__ __forceinline__ uint32_t orderable_f32(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
 __global__ void __launch_bounds__(kListThreads) k_list_keys(const float* __restrict__ probs, i64 N, u64 seed,
                                                             u64* __restrict__ composite) {
   for (i64 i = (i64)blockIdx.x * kListThreads + threadIdx.x; i < N; i += (i64)gridDim.x * kListThreads) {
-    uint32_t key;
-    if (probs) key = orderable_f32(ares_key(rand_u32(seed, (u64)i, 0, STREAM_LIST_WEIGHTED), __ldg(probs + i)));
-    else key = rand_u32(seed, (u64)i, 0, STREAM_LIST);
-    composite[i] = ((u64)key << 32) | (u64)(0xFFFFFFFFu - (uint32_t)i);
+    composite[i] = list_composite(probs, i, seed);
   }
 }
 
@@ -142,32 +289,6 @@ __global__ void __launch_bounds__(kListThreads) k_compact_winners(const u64* __r
   }
 }
 
-// Descending bitonic sort of up to 4096 composites in shared memory (one CTA).
-constexpr int kSmallSort = 4096;
-__global__ void __launch_bounds__(1024) k_sort_winners_small(u64* __restrict__ winners, i64 k) {
-  __shared__ u64 s[kSmallSort];
-  int n = 1;
-  while (n < k) n <<= 1;
-  for (int i = threadIdx.x; i < n; i += 1024) s[i] = i < k ? winners[i] : 0ull;  // 0 sorts last (descending)
-  __syncthreads();
-  for (int size = 2; size <= n; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < n / 2; i += 1024) {
-        const int lo = 2 * i - (i & (stride - 1));
-        const int hi = lo + stride;
-        const bool desc = ((lo & size) == 0);
-        const u64 a = s[lo], b = s[hi];
-        if ((a < b) == desc) {
-          s[lo] = b;
-          s[hi] = a;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  for (int i = threadIdx.x; i < k; i += 1024) winners[i] = s[i];
-}
-
 __global__ void __launch_bounds__(kListThreads) k_invert_keys(u64* __restrict__ keys, i64* __restrict__ vals, i64 n) {
   for (i64 i = (i64)blockIdx.x * kListThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kListThreads) {
     keys[i] = ~keys[i];
@@ -175,11 +296,11 @@ __global__ void __launch_bounds__(kListThreads) k_invert_keys(u64* __restrict__ 
   }
 }
 
-__global__ void __launch_bounds__(kListThreads) k_emit_winners(const u64* __restrict__ winners, int inverted, i64 k,
+__global__ void __launch_bounds__(kListThreads) k_emit_winners(const u64* __restrict__ winners, i64 k,
                                                                const i64* __restrict__ data, i64* __restrict__ out_data,
                                                                i64* __restrict__ out_index) {
   for (i64 j = (i64)blockIdx.x * kListThreads + threadIdx.x; j < k; j += (i64)gridDim.x * kListThreads) {
-    const u64 c = inverted ? ~winners[j] : winners[j];
+    const u64 c = ~winners[j];  // k_invert_keys
     const i64 idx = (i64)(0xFFFFFFFFu - (uint32_t)c);
     out_index[j] = idx;
     out_data[j] = data[idx];
@@ -316,10 +437,37 @@ extern "C" int gsb_list_sample(gsb_ctx* ctx, void* stream_, const int64_t* data,
     ctx_count_launches(ctx, 3);
     return GSB_OK;
   }
-  // without replacement: keys -> radix select of the k-th best -> compact winners -> order them
+  static int resident[64];
+  const int ctas = ctx_resident_ctas(ctx, (const void*)k_list_select, kSelectThreads, 0, resident);
+  if (k <= kSelectMaxK && ctas > 0) {
+    const size_t bytes = ((size_t)N * 8 + 255) & ~(size_t)255;
+    void* ws;
+    int st = ctx_reserve_workspace(ctx, bytes + kSelectMaxK * 8 + sizeof(unsigned) * (kSelectPasses * kSelectBins + 64), &ws);
+    if (st != GSB_OK) return st;
+    SelectParams p{};
+    p.probs = probs;
+    p.data = data;
+    p.N = N;
+    p.k = k;
+    p.seed = (u64)seed;
+    p.composite = (u64*)ws;
+    p.winners = (u64*)((char*)ws + bytes);
+    p.hist = (unsigned*)(p.winners + kSelectMaxK);
+    p.found = p.hist + kSelectPasses * kSelectBins;
+    p.out_data = out_data;
+    p.out_index = out_index;
+    p.counters = ctx_counters(ctx);
+    // four items per thread: fewer CTAs make the barriers of a short list cheaper
+    const int grid = (int)min((i64)min(ctas, kNumSMs), (N + 4 * kSelectThreads - 1) / (4 * kSelectThreads));
+    p.sync = ctx_grid_sync(ctx, grid, kSelectBarriers);
+    ScopedKernelTimer timer(ctx, KID_LIST_SAMPLE, stream);
+    void* args[] = {&p};
+    return launch_cooperative(ctx, stream, (const void*)k_list_select, grid, kSelectThreads, 0, args, p.sync);
+  }
+  // many winners: keys -> radix select of the k-th best -> compact winners -> order them, one launch per pass
   const size_t comp_bytes = ((size_t)N * 8 + 255) & ~(size_t)255;
-  const size_t win_bytes = ((size_t)k * 16 + 255) & ~(size_t)255;  // winners + index payload for the big sort
-  const size_t sort_bytes = k > kSmallSort ? radix_sort_scratch_bytes(k) : 0;
+  const size_t win_bytes = ((size_t)k * 16 + 255) & ~(size_t)255;  // winners + index payload for the sort
+  const size_t sort_bytes = radix_sort_scratch_bytes(k);
   void* ws;
   int st = ctx_reserve_workspace(ctx, comp_bytes + win_bytes + sort_bytes + 4096, &ws);
   if (st != GSB_OK) return st;
@@ -354,20 +502,12 @@ extern "C" int gsb_list_sample(gsb_ctx* ctx, void* stream_, const int64_t* data,
   }
   GSB_LAUNCH_OK();
   ctx_count_launches(ctx, 1);
-  int inverted = 0;
-  if (k <= kSmallSort) {
-    ScopedKernelTimer timer(ctx, KID_OTHER, stream);
-    k_sort_winners_small<<<1, 1024, 0, stream>>>(winners, k);
-    GSB_LAUNCH_OK();
-  } else {
-    k_invert_keys<<<min(grid_for(k, kListThreads), wide), kListThreads, 0, stream>>>(winners, win_vals, k);
-    GSB_LAUNCH_OK();
-    st = radix_sort_pairs(ctx, stream, winners, win_vals, k, 0, 64, sort_ws);
-    if (st != GSB_OK) return st;
-    inverted = 1;
-    ctx_count_launches(ctx, 1);
-  }
-  k_emit_winners<<<min(grid_for(k, kListThreads), wide), kListThreads, 0, stream>>>(winners, inverted, k, data,
+  k_invert_keys<<<min(grid_for(k, kListThreads), wide), kListThreads, 0, stream>>>(winners, win_vals, k);
+  GSB_LAUNCH_OK();
+  st = radix_sort_pairs(ctx, stream, winners, win_vals, k, 0, 64, sort_ws);
+  if (st != GSB_OK) return st;
+  ctx_count_launches(ctx, 1);
+  k_emit_winners<<<min(grid_for(k, kListThreads), wide), kListThreads, 0, stream>>>(winners, k, data,
                                                                                     out_data, out_index);
   GSB_LAUNCH_OK();
   ctx_count_launches(ctx, 1);

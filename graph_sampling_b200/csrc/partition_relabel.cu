@@ -40,8 +40,6 @@
 
 namespace gsb {
 
-typedef uint32_t u32;
-
 constexpr int kPartThreads = 256;
 constexpr int kPartPerThread = 16;
 constexpr int kPartTile = kPartThreads * kPartPerThread;        // items per CTA of the count pass

@@ -11,9 +11,9 @@
 namespace gsb {
 
 constexpr int kSegThreads = 256;
-// Segments longer than this are left to k_segment_long_* (one CTA per segment): with power-law degrees a
-// single hub column would otherwise keep one warp busy for hundreds of iterations while the rest of the
-// grid has long finished.
+constexpr int kSegWarps = kSegThreads / 32;
+// Segments longer than this are taken by a whole CTA: with power-law degrees a single hub column would otherwise keep one
+// warp busy for hundreds of iterations while the rest of the grid has long finished.
 constexpr i64 kLongSegment = 2048;
 
 __device__ __forceinline__ float int_pow(float x, i64 powk) {
@@ -23,85 +23,130 @@ __device__ __forceinline__ float int_pow(float x, i64 powk) {
   return r;
 }
 
-// Two kernels sum the segments of a CSC; both are launched and the one whose shape it is not returns at once (the edge
-// total is indptr[num_seg], known on the device only).  Dense: at least four edges per segment on average, one warp
-// per segment.  Sparse: fewer, 32 segments per warp step.
+// Fewer than four edges per segment on average: most segments of a slice's row view are empty.
 __device__ __forceinline__ bool segments_are_sparse(const i64* __restrict__ indptr, i64 num_seg) {
   return __ldg(indptr + num_seg) - __ldg(indptr) < 4 * num_seg;
 }
 
-__global__ void __launch_bounds__(kSegThreads) k_segment_sum_csc_dense(const i64* __restrict__ indptr, i64 num_seg,
-                                                                       const i64* __restrict__ e_ids,
-                                                                       const float* __restrict__ data, i64 powk,
-                                                                       float* __restrict__ out, i64* long_list,
-                                                                       i64* long_count) {
-  if (segments_are_sparse(indptr, num_seg)) return;
-  const int lane = threadIdx.x & 31;
-  const i64 warp_global = ((i64)blockIdx.x * kSegThreads + threadIdx.x) >> 5;
-  const i64 num_warps = ((i64)gridDim.x * kSegThreads) >> 5;
-  for (i64 s = warp_global; s < num_seg; s += num_warps) {
-    const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
-    if (e - b > kLongSegment) {
-      if (lane == 0) long_list[atomicAdd((u64*)long_count, 1ull)] = s;
-      continue;
-    }
-    float acc = 0.f;
-    for (i64 j = b + lane; j < e; j += 32) {
-      const float x = data ? __ldg(data + (e_ids ? __ldg(e_ids + j) : j)) : 1.0f;
-      acc += int_pow(x, powk);
-    }
+// Lane `at` of `width` lanes: its share of f(b) + f(b + 1) + ... + f(e - 1), eight elements requested before the first is
+// added.  (One element per iteration had a warp wait out a memory round trip per 32 edges: 1.46 M edges in 2 048 columns
+// took 41 us to normalise, 8 us now.)
+template <class F>
+__device__ __forceinline__ float strided_sum(i64 b, i64 e, int at, int width, F f) {
+  constexpr int kAhead = 8;
+  float acc = 0.f;
+  i64 j = b + at;
+  for (; j + (kAhead - 1) * (i64)width < e; j += kAhead * (i64)width) {
+    float v[kAhead];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) out[s] = acc;
+    for (int q = 0; q < kAhead; ++q) v[q] = f(j + q * (i64)width);
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) acc += v[q];
   }
+  for (; j < e; j += width) acc += f(j);
+  return acc;
 }
 
-// A warp takes 32 consecutive segments per step: lane i reads the bounds of segment s0 + i (two coalesced loads for
-// the 32 of them).  Segments of at most four edges — on a slice of a large graph almost all of them are empty — are
-// summed by their own lane; the others are summed by the whole warp, one after the other, lanes striding over the
-// edges and a xor tree at the end.  The short form adds in the order the tree would, (v0 + v2) + (v1 + v3), so a
-// segment's sum does not depend on which form took it.  (One warp per segment spent a step, with two dependent
-// loads, on every empty row: 78 us for the 1 M rows of a slice with 25 000 edges.)
-__global__ void __launch_bounds__(kSegThreads) k_segment_sum_csc(const i64* __restrict__ indptr, i64 num_seg,
-                                                                 const i64* __restrict__ e_ids,
-                                                                 const float* __restrict__ data, i64 powk,
-                                                                 float* __restrict__ out, i64* long_list,
-                                                                 i64* long_count) {
-  if (!segments_are_sparse(indptr, num_seg)) return;
-  const int lane = threadIdx.x & 31;
-  const i64 warp_global = ((i64)blockIdx.x * kSegThreads + threadIdx.x) >> 5;
-  const i64 num_warps = ((i64)gridDim.x * kSegThreads) >> 5;
-  auto value = [&](i64 j) { return int_pow(data ? __ldg(data + (e_ids ? __ldg(e_ids + j) : j)) : 1.0f, powk); };
-  for (i64 s0 = warp_global * 32; s0 < num_seg; s0 += num_warps * 32) {
-    const i64 s = s0 + lane;
-    i64 b = 0, e = 0;
-    if (s < num_seg) {
-      b = __ldg(indptr + s);
-      e = __ldg(indptr + s + 1);
+template <class F>
+__device__ __forceinline__ void strided_for(i64 b, i64 e, int at, int width, F f) {
+#pragma unroll 8
+  for (i64 j = b + at; j < e; j += width) f(j);
+}
+
+// NORMALIZE: out[j] = data[j] / (sum of its segment); otherwise out[s] = sum of data^powk over segment s.  One launch:
+// a warp takes one segment per step, or — when segments are sparse — 32 of them: lane i reads the bounds of segment s0 + i
+// (two coalesced loads for the 32), sums it itself if it has at most four edges, and the others are summed by the whole
+// warp one after the other.  (One warp per segment spent a step, with two dependent loads, on every empty row: 78 us for
+// the 1 M rows of a slice with 25 000 edges.)  The short form adds in the order the tree would, (v0 + v2) + (v1 + v3), so
+// a segment's sum does not depend on which form took it.  Long segments are left to the whole CTA at the end of the step.
+template <bool NORMALIZE>
+__global__ void __launch_bounds__(kSegThreads) k_segments(const i64* __restrict__ indptr, i64 num_seg,
+                                                          const i64* __restrict__ e_ids, const float* __restrict__ data,
+                                                          i64 powk, float* __restrict__ out) {
+  __shared__ i64 s_long[kSegThreads];
+  __shared__ int s_num_long;
+  __shared__ float s_part[kSegWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto at = [&](i64 j) { return e_ids ? __ldg(e_ids + j) : j; };
+  auto value = [&](i64 j) {
+    const float x = data ? __ldg(data + at(j)) : 1.0f;
+    return NORMALIZE ? x : int_pow(x, powk);
+  };
+  auto warp_segment = [&](i64 s, i64 b, i64 e) {
+    float acc = strided_sum(b, e, lane, 32, value);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (NORMALIZE) {
+      strided_for(b, e, lane, 32, [&](i64 j) {
+        const i64 q = at(j);
+        out[q] = __ldg(data + q) / acc;
+      });
+    } else if (lane == 0) {
+      out[s] = acc;
     }
-    const i64 len = e - b;
-    // the loads of a short segment are issued now and used after the warp-wide part, which hides their latency
-    const bool is_short = s < num_seg && len <= 4;
-    float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-    if (is_short) {
-      if (len > 0) v0 = value(b);
-      if (len > 1) v1 = value(b + 1);
-      if (len > 2) v2 = value(b + 2);
-      if (len > 3) v3 = value(b + 3);
+  };
+  const bool sparse = !NORMALIZE && segments_are_sparse(indptr, num_seg);
+  const i64 per_cta = sparse ? kSegThreads : kSegWarps;
+  for (i64 first = (i64)blockIdx.x * per_cta; first < num_seg; first += (i64)gridDim.x * per_cta) {
+    if (threadIdx.x == 0) s_num_long = 0;
+    __syncthreads();
+    if (!sparse) {
+      const i64 s = first + warp;
+      if (s < num_seg) {
+        const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
+        if (e - b <= kLongSegment) warp_segment(s, b, e);
+        else if (lane == 0) s_long[atomicAdd(&s_num_long, 1)] = s;
+      }
+    } else {
+      const i64 s0 = first + warp * 32, s = s0 + lane;
+      i64 b = 0, e = 0;
+      if (s < num_seg) {
+        b = __ldg(indptr + s);
+        e = __ldg(indptr + s + 1);
+      }
+      const i64 len = e - b;
+      // the loads of a short segment are issued now and used after the warp-wide part, which hides their latency
+      const bool is_short = s < num_seg && len <= 4;
+      float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
+      if (is_short) {
+        if (len > 0) v0 = value(b);
+        if (len > 1) v1 = value(b + 1);
+        if (len > 2) v2 = value(b + 2);
+        if (len > 3) v3 = value(b + 3);
+      }
+      if (s < num_seg && len > kLongSegment) s_long[atomicAdd(&s_num_long, 1)] = s;
+      unsigned medium = __ballot_sync(0xffffffffu, s < num_seg && len > 4 && len <= kLongSegment);
+      while (medium) {
+        const int src = __ffs(medium) - 1;
+        medium &= medium - 1;
+        warp_segment(s0 + src, __shfl_sync(0xffffffffu, b, src), __shfl_sync(0xffffffffu, e, src));
+      }
+      if (is_short) out[s] = (v0 + v2) + (v1 + v3);
     }
-    if (s < num_seg && len > kLongSegment) long_list[atomicAdd((u64*)long_count, 1ull)] = s;
-    unsigned medium = __ballot_sync(0xffffffffu, s < num_seg && len > 4 && len <= kLongSegment);
-    while (medium) {
-      const int src = __ffs(medium) - 1;
-      medium &= medium - 1;
-      const i64 mb = __shfl_sync(0xffffffffu, b, src), me = __shfl_sync(0xffffffffu, e, src);
-      float acc = 0.f;
-      for (i64 j = mb + lane; j < me; j += 32) acc += value(j);
+    __syncthreads();
+    const int num_long = s_num_long;
+    for (int q = 0; q < num_long; ++q) {
+      const i64 s = s_long[q];
+      const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
+      float acc = strided_sum(b, e, threadIdx.x, kSegThreads, value);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) out[s0 + src] = acc;
+      if (lane == 0) s_part[warp] = acc;
+      __syncthreads();
+      float total = 0.f;
+#pragma unroll
+      for (int w = 0; w < kSegWarps; ++w) total += s_part[w];
+      if (NORMALIZE) {
+        strided_for(b, e, threadIdx.x, kSegThreads, [&](i64 j) {
+          const i64 p = at(j);
+          out[p] = __ldg(data + p) / total;
+        });
+      } else if (threadIdx.x == 0) {
+        out[s] = total;
+      }
+      __syncthreads();
     }
-    if (is_short) out[s] = (v0 + v2) + (v1 + v3);
+    __syncthreads();  // s_long / s_num_long are rewritten by the next step
   }
 }
 
@@ -179,83 +224,8 @@ __global__ void __launch_bounds__(kSegThreads) k_edge_div_u_sum(const i64* __res
   }
 }
 
-// One CTA per long segment (taken from the list the warp kernels filled): strided partial sums, a fixed-order
-// shared-memory reduction (deterministic), then the result / the normalised values.
-template <bool NORMALIZE>
-__global__ void __launch_bounds__(kSegThreads) k_segment_long(const i64* __restrict__ indptr,
-                                                              const i64* __restrict__ e_ids,
-                                                              const float* __restrict__ data, i64 powk,
-                                                              float* __restrict__ out, const i64* __restrict__ long_list,
-                                                              const i64* __restrict__ long_count) {
-  __shared__ float s_part[kSegThreads];
-  const i64 n_long = *long_count;
-  for (i64 q = blockIdx.x; q < n_long; q += gridDim.x) {
-    const i64 s = long_list[q];
-    const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
-    float acc = 0.f;
-    for (i64 j = b + threadIdx.x; j < e; j += kSegThreads) {
-      const float x = data ? __ldg(data + (e_ids ? __ldg(e_ids + j) : j)) : 1.0f;
-      acc += NORMALIZE ? x : int_pow(x, powk);
-    }
-    s_part[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = kSegThreads / 2; w > 0; w >>= 1) {
-      if (threadIdx.x < w) s_part[threadIdx.x] += s_part[threadIdx.x + w];
-      __syncthreads();
-    }
-    const float total = s_part[0];
-    if (NORMALIZE) {
-      for (i64 j = b + threadIdx.x; j < e; j += kSegThreads) {
-        const i64 p = e_ids ? __ldg(e_ids + j) : j;
-        out[p] = __ldg(data + p) / total;
-      }
-    } else if (threadIdx.x == 0) {
-      out[s] = total;
-    }
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(kSegThreads) k_segment_normalize_csc(const i64* __restrict__ indptr, i64 num_seg,
-                                                                       const i64* __restrict__ e_ids,
-                                                                       const float* __restrict__ data,
-                                                                       float* __restrict__ out, i64* long_list,
-                                                                       i64* long_count) {
-  const int lane = threadIdx.x & 31;
-  const i64 warp_global = ((i64)blockIdx.x * kSegThreads + threadIdx.x) >> 5;
-  const i64 num_warps = ((i64)gridDim.x * kSegThreads) >> 5;
-  for (i64 s = warp_global; s < num_seg; s += num_warps) {
-    const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
-    if (e - b > kLongSegment) {
-      if (lane == 0) long_list[atomicAdd((u64*)long_count, 1ull)] = s;
-      continue;
-    }
-    float acc = 0.f;
-    for (i64 j = b + lane; j < e; j += 32) acc += __ldg(data + (e_ids ? __ldg(e_ids + j) : j));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    for (i64 j = b + lane; j < e; j += 32) {
-      const i64 q = e_ids ? __ldg(e_ids + j) : j;
-      out[q] = __ldg(data + q) / acc;
-    }
-  }
-}
-
-static inline int warp_grid(i64 segments) {
-  const i64 blocks = (segments * 32 + kSegThreads - 1) / kSegThreads;
-  return (int)max((i64)1, min(blocks, (i64)kNumSMs * 16));
-}
-
-// Scratch for the list of long segments: [count | ids...] in the context arena, count zeroed on the stream.
-static int long_segment_scratch(gsb_ctx* ctx, cudaStream_t stream, i64 num_seg, i64** list, i64** count) {
-  void* ws;
-  int st = ctx_reserve_workspace(ctx, sizeof(i64) * (size_t)(num_seg + 32), &ws);
-  if (st != GSB_OK) return st;
-  *count = (i64*)ws;
-  *list = (i64*)ws + 32;
-  GSB_CUDA_OK(cudaMemsetAsync(*count, 0, sizeof(i64), stream));
-  return GSB_OK;
-}
+// Grid of k_segments: a CTA per eight segments (a sparse call strides further with the same grid), up to 16 per SM.
+static inline int segments_grid(i64 num_seg) { return min(grid_for(num_seg, kSegWarps), kNumSMs * 16); }
 
 }  // namespace gsb
 
@@ -270,20 +240,9 @@ int gsb_segment_sum_csc(gsb_ctx* ctx, void* stream_, const int64_t* indptr, int6
   if (num_seg == 0) return GSB_OK;
   GSB_REQUIRE(indptr && out, GSB_ERR_INVALID_ARGUMENT);
   cudaStream_t stream = (cudaStream_t)stream_;
-  i64 *long_list, *long_count;
-  int st = long_segment_scratch(ctx, stream, num_seg, &long_list, &long_count);
-  if (st != GSB_OK) return st;
   {
     ScopedKernelTimer timer(ctx, KID_SEGMENT, stream);
-    k_segment_sum_csc_dense<<<warp_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, powk, out,
-                                                                            long_list, long_count);
-    k_segment_sum_csc<<<warp_grid((num_seg + 31) / 32), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, powk,
-                                                                                  out, long_list, long_count);
-  }
-  GSB_LAUNCH_OK();
-  {
-    ScopedKernelTimer timer(ctx, KID_SEGMENT, stream);
-    k_segment_long<false><<<kNumSMs * 2, kSegThreads, 0, stream>>>(indptr, e_ids, data, powk, out, long_list, long_count);
+    k_segments<false><<<segments_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, powk, out);
   }
   GSB_LAUNCH_OK();
   return GSB_OK;
@@ -314,18 +273,9 @@ int gsb_segment_normalize_csc(gsb_ctx* ctx, void* stream_, const int64_t* indptr
   if (num_seg == 0) return GSB_OK;
   GSB_REQUIRE(indptr && data && out, GSB_ERR_INVALID_ARGUMENT);
   cudaStream_t stream = (cudaStream_t)stream_;
-  i64 *long_list, *long_count;
-  int st = long_segment_scratch(ctx, stream, num_seg, &long_list, &long_count);
-  if (st != GSB_OK) return st;
   {
     ScopedKernelTimer timer(ctx, KID_SEGMENT, stream);
-    k_segment_normalize_csc<<<warp_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, out,
-                                                                            long_list, long_count);
-  }
-  GSB_LAUNCH_OK();
-  {
-    ScopedKernelTimer timer(ctx, KID_SEGMENT, stream);
-    k_segment_long<true><<<kNumSMs * 2, kSegThreads, 0, stream>>>(indptr, e_ids, data, 1, out, long_list, long_count);
+    k_segments<true><<<segments_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, 1, out);
   }
   GSB_LAUNCH_OK();
   return GSB_OK;

@@ -22,7 +22,6 @@
 
 namespace gsb {
 
-using u32 = uint32_t;
 constexpr int kWThreads = 256;
 // Columns per CTA.  64 (8 per warp) when the call has many columns; 8 (one per warp) when it has few, so that a call
 // with a few thousand long columns — the later hops of adaptive sampling — still fills the GPU.

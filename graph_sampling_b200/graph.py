@@ -577,7 +577,8 @@ class Graph:
         self.CreateSparseFormat(on_format)
         data = self.data_
         out_size = self.num_cols_ if axis == 0 else self.num_rows_
-        out = torch.zeros(out_size, dtype=torch.float32, device=self._device())
+        accumulates = on_format == _COO   # into zeros; the segment forms write every entry
+        out = (torch.zeros if accumulates else torch.empty)(out_size, dtype=torch.float32, device=self._device())
         if on_format == _COO:
             by_row = (1 - axis) == 0
             target = self.coo_.row if by_row else self.coo_.col
@@ -588,9 +589,9 @@ class Graph:
             if val_ids is None:
                 ops.csc_sum(fmt.indptr, fmt.e_ids, data, out, powk)
             else:  # segment c of a compact form belongs to node val_ids[c] (src/cuda/graph_ops.cu:15-39)
-                compact = torch.zeros(val_ids.numel(), dtype=torch.float32, device=out.device)
+                compact = torch.empty(val_ids.numel(), dtype=torch.float32, device=out.device)
                 ops.csc_sum(fmt.indptr, fmt.e_ids, data, compact, powk)
-                out[val_ids] = compact
+                out.zero_()[val_ids] = compact
         else:
             _fatal("axis should be 0 or 1? on_format and axis do not match?")
         return out
@@ -618,7 +619,8 @@ class Graph:
     def Divide(self, divisor, axis, on_format):
         self.CreateSparseFormat(on_format)
         in_data = self._data_or_ones()
-        out = torch.zeros(self.num_edges_, dtype=torch.float32, device=in_data.device)
+        covered = on_format == _COO and self.coo_.e_ids is None and self.coo_.row.numel() == self.num_edges_
+        out = (torch.empty if covered else torch.zeros)(self.num_edges_, dtype=torch.float32, device=in_data.device)
         if on_format == _COO:
             rhs_target = 0 if (1 - axis) == 0 else 2
             ops.sddmm("div", in_data, divisor, out, 1, rhs_target, self.coo_.row, self.coo_.col,

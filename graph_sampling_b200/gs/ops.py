@@ -38,8 +38,10 @@ def _gsddmm(gidx, op, lhs, rhs, lhs_target="u", rhs_target="v", on_format=_COO):
         rhs, expand_rhs = rhs.unsqueeze(-1), True
     lt, rt = target_mapping[lhs_target], target_mapping[rhs_target]
     n_edges = gidx._CAPI_get_num_edges()
-    out = torch.zeros((n_edges,) + infer_broadcast_shape(op, lhs.shape[1:], rhs.shape[1:]), dtype=lhs.dtype,
-                      device=lhs.device)
+    # without edge ids every edge writes its own row of the result; with them rows may be left out
+    coo = getattr(gidx, "coo_", None) if on_format == _COO else None
+    new = torch.empty if coo is not None and coo.e_ids is None and coo.row.numel() == n_edges else torch.zeros
+    out = new((n_edges,) + infer_broadcast_shape(op, lhs.shape[1:], rhs.shape[1:]), dtype=lhs.dtype, device=lhs.device)
     if n_edges > 0:
         gidx._CAPI_sddmm(op, lhs.contiguous(), rhs.contiguous(), out, lt, rt, on_format)
     if expand_lhs and expand_rhs:

@@ -23,11 +23,6 @@ __device__ __forceinline__ float int_pow(float x, i64 powk) {
   return r;
 }
 
-// Fewer than four edges per segment on average: most segments of a slice's row view are empty.
-__device__ __forceinline__ bool segments_are_sparse(const i64* __restrict__ indptr, i64 num_seg) {
-  return __ldg(indptr + num_seg) - __ldg(indptr) < 4 * num_seg;
-}
-
 // Lane `at` of `width` lanes: its share of f(b) + f(b + 1) + ... + f(e - 1), eight elements requested before the first is
 // added.  (One element per iteration had a warp wait out a memory round trip per 32 edges: 1.46 M edges in 2 048 columns
 // took 41 us to normalise, 8 us now.)
@@ -47,14 +42,30 @@ __device__ __forceinline__ float strided_sum(i64 b, i64 e, int at, int width, F 
   return acc;
 }
 
-template <class F>
-__device__ __forceinline__ void strided_for(i64 b, i64 e, int at, int width, F f) {
-#pragma unroll 8
-  for (i64 j = b + at; j < e; j += width) f(j);
+// out[at(j)] = data[at(j)] / total for the same share, eight at a time as well.
+template <class At>
+__device__ __forceinline__ void strided_divide(i64 b, i64 e, int first, int width, const float* __restrict__ data,
+                                               float* __restrict__ out, float total, At at) {
+  constexpr int kAhead = 8;
+  for (i64 j = b + first; j < e; j += kAhead * (i64)width) {
+    i64 p[kAhead];
+    float v[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+      if (j + q * (i64)width < e) p[q] = at(j + q * (i64)width);
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+      if (j + q * (i64)width < e) v[q] = __ldg(data + p[q]);
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+      if (j + q * (i64)width < e) out[p[q]] = v[q] / total;
+  }
 }
 
 // NORMALIZE: out[j] = data[j] / (sum of its segment); otherwise out[s] = sum of data^powk over segment s.  One launch:
-// a warp takes one segment per step, or — when segments are sparse — 32 of them: lane i reads the bounds of segment s0 + i
+// a CTA takes one segment per step when they are long on average (at least 128 edges: a warp each would leave few warps with
+// everything, and a CTA that meets several hubs does them one after the other), a warp takes one when they are not, or — when
+// most are empty, below four edges on average, as in the row view of a slice — 32 of them: lane i reads the bounds of segment s0 + i
 // (two coalesced loads for the 32), sums it itself if it has at most four edges, and the others are summed by the whole
 // warp one after the other.  (One warp per segment spent a step, with two dependent loads, on every empty row: 78 us for
 // the 1 M rows of a slice with 25 000 edges.)  The short form adds in the order the tree would, (v0 + v2) + (v1 + v3), so
@@ -77,20 +88,24 @@ __global__ void __launch_bounds__(kSegThreads) k_segments(const i64* __restrict_
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (NORMALIZE) {
-      strided_for(b, e, lane, 32, [&](i64 j) {
-        const i64 q = at(j);
-        out[q] = __ldg(data + q) / acc;
-      });
+      strided_divide(b, e, lane, 32, data, out, acc, at);
     } else if (lane == 0) {
       out[s] = acc;
     }
   };
-  const bool sparse = !NORMALIZE && segments_are_sparse(indptr, num_seg);
-  const i64 per_cta = sparse ? kSegThreads : kSegWarps;
+  const i64 mean = (__ldg(indptr + num_seg) - __ldg(indptr)) / num_seg;
+  const bool sparse = !NORMALIZE && mean < 4;
+  const bool dense = mean >= 128;
+  const i64 per_cta = sparse ? kSegThreads : dense ? 1 : kSegWarps;
   for (i64 first = (i64)blockIdx.x * per_cta; first < num_seg; first += (i64)gridDim.x * per_cta) {
     if (threadIdx.x == 0) s_num_long = 0;
     __syncthreads();
-    if (!sparse) {
+    if (dense) {
+      if (threadIdx.x == 0) {
+        s_long[0] = first;
+        s_num_long = 1;
+      }
+    } else if (!sparse) {
       const i64 s = first + warp;
       if (s < num_seg) {
         const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
@@ -137,10 +152,7 @@ __global__ void __launch_bounds__(kSegThreads) k_segments(const i64* __restrict_
 #pragma unroll
       for (int w = 0; w < kSegWarps; ++w) total += s_part[w];
       if (NORMALIZE) {
-        strided_for(b, e, threadIdx.x, kSegThreads, [&](i64 j) {
-          const i64 p = at(j);
-          out[p] = __ldg(data + p) / total;
-        });
+        strided_divide(b, e, threadIdx.x, kSegThreads, data, out, total, at);
       } else if (threadIdx.x == 0) {
         out[s] = total;
       }
@@ -224,8 +236,8 @@ __global__ void __launch_bounds__(kSegThreads) k_edge_div_u_sum(const i64* __res
   }
 }
 
-// Grid of k_segments: a CTA per eight segments (a sparse call strides further with the same grid), up to 16 per SM.
-static inline int segments_grid(i64 num_seg) { return min(grid_for(num_seg, kSegWarps), kNumSMs * 16); }
+// Grid of k_segments, whose step the device chooses: a CTA per segment, up to 16 per SM.
+static inline int segments_grid(i64 num_seg) { return (int)min(num_seg, (i64)kNumSMs * 16); }
 
 }  // namespace gsb
 

@@ -18,7 +18,7 @@
 namespace gsb {
 
 constexpr int kThreads = 256;
-constexpr int kTileCols = 128;  // columns per CTA in the fill / sample kernels
+constexpr int kTileCols = 128;  // columns per CTA of the lane-group sampler
 
 enum CountMode { COUNT_DEGREE = 0, COUNT_WOR = 1, COUNT_WR = 2 };
 
@@ -36,33 +36,53 @@ __device__ __forceinline__ bool column_in_range(i64 col, i64 num_cols, i64* coun
   return false;
 }
 
+// PER consecutive columns per thread: one when the call is small (every column wants a thread of its own, they are all in
+// flight at once), four when it is large, where the number of tiles sets the length of the look-back chain.
+template <int PER>
 __global__ void __launch_bounds__(kThreads) k_count_scan(const i64* __restrict__ indptr, i64 num_cols,
                                                          const i64* __restrict__ seeds, i64 S, i64 k, int mode,
                                                          i64* __restrict__ out_indptr, i64* counters, TileState ts,
                                                          Mail mail) {
   __shared__ i64 s_scan[33];
   __shared__ i64 s_base;
+  constexpr i64 kTile = kThreads * PER;
   const int tile = blockIdx.x;
-  const i64 i = (i64)tile * kThreads + threadIdx.x;
-  if ((i64)tile * kThreads >= S && !(S == 0 && tile == 0)) return;
-  i64 f = 0;
-  if (i < S) {
-    const i64 col = seeds ? seeds[i] : i;
-    if (column_in_range(col, num_cols, counters, i)) {
-      const i64 b = indptr[col];
-      f = column_count(indptr[col + 1] - b, k, mode);
+  const i64 i = (i64)tile * kTile + (i64)threadIdx.x * PER;
+  if ((i64)tile * kTile >= S && !(S == 0 && tile == 0)) return;
+  i64 col[PER], begin[PER], f[PER], sum = 0;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    col[q] = -1;
+    if (i + q < S) {
+      col[q] = seeds ? seeds[i + q] : i + q;
+      if (!column_in_range(col[q], num_cols, counters, i + q)) col[q] = -1;
     }
   }
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    begin[q] = col[q] >= 0 ? __ldg(indptr + col[q]) : 0;
+    f[q] = col[q] >= 0 ? __ldg(indptr + col[q] + 1) : 0;
+  }
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    f[q] = column_count(f[q] - begin[q], k, mode);
+    sum += f[q];
+  }
   i64 total;
-  const i64 excl = block_exclusive_scan<kThreads>(f, s_scan, &total);
+  i64 run = block_exclusive_scan<kThreads>(sum, s_scan, &total);
   if (threadIdx.x < 32) {
     const i64 prefix = tile_exclusive_prefix(ts, tile, total);
     if (threadIdx.x == 0) s_base = prefix;
   }
   __syncthreads();
   const i64 tile_base = s_base;
-  if (i < S) out_indptr[i] = tile_base + excl;
-  if ((i64)(tile + 1) * kThreads >= S && threadIdx.x == 0) {
+  run += tile_base;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    if (i + q < S) out_indptr[i + q] = run;
+    run += f[q];
+  }
+  if ((i64)(tile + 1) * kTile >= S && threadIdx.x == 0) {
     out_indptr[S] = tile_base + total;
     counters[CNT_NNZ] = tile_base + total;
     mail_post(mail, 0, tile_base + total, counters);
@@ -88,97 +108,29 @@ struct FillParams {
   const i64* nid_ptr;
   i64 G;
   i64 encoding_size;
-  bool host_chose;  // the caller knew the edge total and launched only the kernel that suits the shape
+  i64 D;  // edge total, or -1: it is read on the device
 };
+constexpr i64 kFillNoColumn = (i64)1 << 62;
 
-// Which of the two fill kernels copies a slice of S columns with D edges: both are launched and the one whose shape
-// it is not returns at once (the edge total is known on the device only).  Column tiles — offsets and column starts
-// loaded once per column, coalesced — win when there are many short columns; output tiles win when columns are long
-// (D >= 128·S) or too few to give every SM a column tile.
-__host__ __device__ __forceinline__ bool fill_by_output_tiles(i64 S, i64 D) { return D >= 128 * S || S < 148 * kTileCols; }
+// The OUTPUT positions are cut into tiles, whatever columns they belong to, and a CTA copies a tile at a time: a hub column
+// is spread over the grid, and a call with few, long columns fills it as well as one with many short ones.
+//   1. the tile's first and last column, by two warp-wide searches of the offsets (32 pivots a round);
+//   2. the offsets of the tile's columns and what to add to an output position to get the input position, a column per
+//      thread, into shared memory (the two dependent reads seeds -> indptr are made once per column and tile);
+//   3. a warp copies 256 consecutive positions: one binary search in shared memory per lane for the first of its eight, then
+//      the column only walks forward; all reads are requested before anything is written.
+// What bounds it is the chain search -> offsets -> ids against the positions in flight per SM, so registers are spent on
+// resident CTAs: a position keeps the number of its column in the window and nothing else until its id has arrived.
+// 262 144 columns with 13.2 M edges, weights and column ids, whole call: column tiles (a CTA per 128 columns) 177 us; output
+// tiles with the input positions in registers 155 us; this form with 256 threads and 4 / 5 / 6 CTAs per SM 137 / 133 / 153
+// us, with 128 threads and 10 / 12 CTAs 130 / 150 us (fewer registers spill).  Tiles of 256 positions per warp, without any
+// CTA barrier: 167 us, the search is then paid four times as often.
+constexpr int kFillThreads = 128;
+constexpr int kFillPer = 8;
+constexpr int kFillTile = kFillThreads * kFillPer;
+constexpr int kFillWindow = 512;  // columns of a tile held in shared memory at a time
 
-template <bool ENCODE>
-__global__ void __launch_bounds__(kThreads) k_slice_fill(FillParams p) {
-  if (!p.host_chose && fill_by_output_tiles(p.S, __ldg(p.out_indptr + p.S))) return;
-  __shared__ i64 s_in[kTileCols];
-  __shared__ i64 s_off[kTileCols + 1];
-  __shared__ i64 s_enc[ENCODE ? kTileCols : 1];
-  const i64 base = (i64)blockIdx.x * kTileCols;
-  if (base >= p.S) return;
-  const int ncol = (int)min((i64)kTileCols, p.S - base);
-  const int tid = threadIdx.x;
-  if (tid <= ncol) s_off[tid] = p.out_indptr[base + tid];
-  if (tid < ncol) {
-    const i64 col = p.seeds ? p.seeds[base + tid] : base + tid;
-    s_in[tid] = (u64)col < (u64)p.num_cols ? p.indptr[col] : 0;  // a bad id has no output positions (count 0)
-    if (ENCODE) s_enc[tid] = batch_of(p.nid_ptr, p.G, base + tid) * p.encoding_size;
-  }
-  __syncthreads();
-  const i64 tile_base = s_off[0];
-  const i64 tile_sum = s_off[ncol] - tile_base;
-  // A warp copies 256 consecutive output positions at a time (lanes on consecutive positions): the column of the
-  // first one is found by binary search in the shared tile offsets, after that the column index only walks
-  // forward — a hub column is spread over the whole CTA, and no position pays for its own search.
-  constexpr int kChunk = 32 * 8;
-  const int lane = tid & 31, warp = tid >> 5;
-  for (i64 chunk = (i64)warp * kChunk; chunk < tile_sum; chunk += (i64)(kThreads / 32) * kChunk) {
-    int c = 0;
-    {
-      const i64 first = tile_base + chunk;
-      int lo = 0, hi = ncol;  // invariant: s_off[lo] <= first < s_off[hi]
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (s_off[mid] <= first) lo = mid;
-        else hi = mid;
-      }
-      c = lo;
-    }
-    // all eight loads first, then the stores: the compiler may not move a load above a store it cannot prove
-    // independent, and eight dependent DRAM round trips per chunk would set the pace
-    i64 in_pos[8], val[8];
-    int col_of[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const i64 q = chunk + r * 32 + lane;
-      in_pos[r] = -1;
-      if (q < tile_sum) {
-        const i64 pos = tile_base + q;
-        while (s_off[c + 1] <= pos) ++c;  // empty columns are stepped over; pos < s_off[ncol] bounds the walk
-        col_of[r] = c;
-        in_pos[r] = s_in[c] + (pos - s_off[c]);
-        val[r] = __ldg(p.indices + in_pos[r]);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      if (in_pos[r] < 0) continue;
-      const i64 pos = tile_base + chunk + r * 32 + lane;
-      p.out_indices[pos] = val[r] + (ENCODE ? s_enc[col_of[r]] : 0);
-      if (p.out_select) p.out_select[pos] = in_pos[r];
-      if (p.out_coo_col) p.out_coo_col[pos] = base + col_of[r];
-      if (p.out_data) p.out_data[pos] = p.data[p.e_ids ? p.e_ids[in_pos[r]] : in_pos[r]];
-    }
-  }
-}
-
-// Edge-parallel form of the fill: the OUTPUT positions are cut into tiles of 2 048, whatever columns they belong to,
-// and a fixed grid of CTAs walks over the tiles (the edge total is read from out_indptr[S] on the device).  The
-// column-tiled kernel above gives one CTA all the edges of its 128 columns, so a call with few, long columns — the
-// later layers of layer-wise and adaptive sampling, whose seeds are the hubs the previous layer picked — ran on a
-// handful of SMs (1 024 columns with 1.8 M edges: 400 us there, 7 us here).
-constexpr int kFillTile = 2048;  // positions per CTA pass: 8 warps x 256
-
-// largest c in [lo, hi] with off[c] <= pos  (off[lo] <= pos is given)
-__device__ __forceinline__ i64 fill_column_at(const i64* __restrict__ off, i64 lo, i64 hi, i64 pos) {
-  while (lo < hi) {
-    const i64 mid = (lo + hi + 1) >> 1;
-    if (__ldg(off + mid) <= pos) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
-// The same search by a whole warp, 32 pivots per step.  Needs off[0] <= pos < off[S].
+// Largest c with off[c] <= pos, by a whole warp.  Needs off[0] <= pos < off[S].
 __device__ __forceinline__ i64 fill_warp_column_at(const i64* __restrict__ off, i64 S, i64 pos) {
   const int lane = threadIdx.x & 31;
   i64 lo = 0, hi = S;
@@ -195,88 +147,90 @@ __device__ __forceinline__ i64 fill_warp_column_at(const i64* __restrict__ off, 
 }
 
 template <bool ENCODE>
-__global__ void __launch_bounds__(kThreads) k_slice_fill_edges(FillParams p) {
-  __shared__ i64 s_clo, s_chi;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const i64 D = __ldg(p.out_indptr + p.S);
-  if (!p.host_chose && !fill_by_output_tiles(p.S, D)) return;
-  for (i64 tile_base = (i64)blockIdx.x * kFillTile; tile_base < D; tile_base += (i64)gridDim.x * kFillTile) {
-    const i64 tile_end = min(D, tile_base + kFillTile);
-    if (warp < 2) {  // the tile's column range: two warp-wide searches side by side
-      const i64 c = fill_warp_column_at(p.out_indptr, p.S, warp == 0 ? tile_base : tile_end - 1);
-      if (lane == 0) (warp == 0 ? s_clo : s_chi) = c;
+__global__ void __launch_bounds__(kFillThreads, 10) k_slice_fill(FillParams p) {
+  __shared__ i64 s_range[2];
+  __shared__ i64 s_delta[kFillWindow];    // input position of an edge = its output position + this
+  __shared__ int s_off[kFillWindow + 1];  // first output position of a column, relative to the tile
+  __shared__ i64 s_enc[ENCODE ? kFillWindow : 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const i64 D = p.D >= 0 ? p.D : __ldg(p.out_indptr + p.S);
+  for (i64 tile = (i64)blockIdx.x * kFillTile; tile < D; tile += (i64)gridDim.x * kFillTile) {
+    const int here = (int)min((i64)kFillTile, D - tile);
+    if (warp < 2) {
+      const i64 c = fill_warp_column_at(p.out_indptr, p.S, warp == 0 ? tile : tile + here - 1);
+      if (lane == 0) s_range[warp] = c;
     }
     __syncthreads();
-    const i64 clo = s_clo, chi = s_chi;
-    const i64 base = tile_base + (i64)warp * 256;
-    // a warp's 256 positions are consecutive: one search for the first, then the column only walks forward; each
-    // phase (column, start of the column, row id) issues its eight loads per lane before the next one begins
-    i64 c = base < tile_end ? fill_column_at(p.out_indptr, clo, chi, base) : clo;
-    i64 col_of[8], in_pos[8], val[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const i64 pos = base + r * 32 + lane;
-      col_of[r] = -1;
-      if (pos < tile_end) {
-        while (c < chi && __ldg(p.out_indptr + c + 1) <= pos) ++c;
-        col_of[r] = c;
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      if (col_of[r] < 0) continue;
-      const i64 pos = base + r * 32 + lane;
-      const i64 col = p.seeds ? __ldg(p.seeds + col_of[r]) : col_of[r];
-      if ((u64)col >= (u64)p.num_cols) {  // only reachable with offsets that were not counted for these seeds
-        col_of[r] = -1;
-        continue;
-      }
-      in_pos[r] = __ldg(p.indptr + col) + (pos - __ldg(p.out_indptr + col_of[r]));
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      if (col_of[r] >= 0) val[r] = __ldg(p.indices + in_pos[r]);
-    // the batch of a column, for the encoded form: searched once per lane, then it only walks forward
-    i64 b = 0, b_next = 0;
-    if (ENCODE && col_of[0] >= 0) {
-      b = batch_of(p.nid_ptr, p.G, col_of[0]);
-      b_next = __ldg(p.nid_ptr + b + 1);
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      if (col_of[r] < 0) continue;
-      const i64 pos = base + r * 32 + lane;
-      i64 v = val[r];
-      if (ENCODE) {
-        while (col_of[r] >= b_next && b + 1 < p.G) {
-          ++b;
-          b_next = __ldg(p.nid_ptr + b + 1);
+    const i64 c_end = s_range[1] + 1;
+    // one window of columns, unless the tile meets more of them (runs of empty ones)
+    for (i64 c0 = s_range[0]; c0 < c_end; c0 += kFillWindow) {
+      const int cols = (int)min((i64)kFillWindow, c_end - c0);
+      for (int j = tid; j <= cols; j += kFillThreads) {
+        const i64 o = __ldg(p.out_indptr + c0 + j);
+        s_off[j] = (int)max((i64)0, min(o - tile, (i64)here));
+        if (j < cols) {
+          const i64 col = p.seeds ? __ldg(p.seeds + c0 + j) : c0 + j;
+          // a bad id has no output positions unless the offsets were not counted for these seeds: then nothing is read
+          s_delta[j] = (u64)col < (u64)p.num_cols ? __ldg(p.indptr + col) - o + tile : kFillNoColumn;
+          if (ENCODE) s_enc[j] = batch_of(p.nid_ptr, p.G, c0 + j) * p.encoding_size;
         }
-        v += b * p.encoding_size;
       }
-      p.out_indices[pos] = v;
-      if (p.out_select) p.out_select[pos] = in_pos[r];
-      if (p.out_coo_col) p.out_coo_col[pos] = col_of[r];
-      if (p.out_data) p.out_data[pos] = p.data[p.e_ids ? p.e_ids[in_pos[r]] : in_pos[r]];
+      __syncthreads();
+      const int begin = s_off[0], end = s_off[cols];  // the tile's positions that the window covers
+      const int base = warp * (32 * kFillPer) + lane;
+      int c = 0;
+      {
+        const int q = max(base, begin);
+        int hi = cols;
+        while (hi - c > 1) {
+          const int mid = (c + hi) >> 1;
+          if (s_off[mid] <= q) c = mid;
+          else hi = mid;
+        }
+      }
+      int col[kFillPer];
+#pragma unroll
+      for (int r = 0; r < kFillPer; ++r) {
+        const int q = base + r * 32;
+        col[r] = -1;
+        if (q < begin || q >= end) continue;
+        while (s_off[c + 1] <= q) ++c;  // empty columns are stepped over; q < end = s_off[cols] bounds the walk
+        if (s_delta[c] != kFillNoColumn) col[r] = c;
+      }
+      i64 val[kFillPer];
+#pragma unroll
+      for (int r = 0; r < kFillPer; ++r)
+        if (col[r] >= 0) val[r] = __ldg(p.indices + (base + r * 32 + s_delta[col[r]]));
+      float x[kFillPer];
+      if (p.out_data) {
+#pragma unroll
+        for (int r = 0; r < kFillPer; ++r)
+          if (col[r] >= 0) {
+            const i64 in = base + r * 32 + s_delta[col[r]];
+            x[r] = __ldg(p.data + (p.e_ids ? __ldg(p.e_ids + in) : in));
+          }
+      }
+#pragma unroll
+      for (int r = 0; r < kFillPer; ++r) {
+        if (col[r] < 0) continue;
+        const i64 pos = tile + base + r * 32;
+        p.out_indices[pos] = val[r] + (ENCODE ? s_enc[col[r]] : 0);
+        if (p.out_select) p.out_select[pos] = base + r * 32 + s_delta[col[r]];
+        if (p.out_coo_col) p.out_coo_col[pos] = c0 + col[r];
+        if (p.out_data) p.out_data[pos] = x[r];
+      }
+      __syncthreads();  // the shared arrays are rewritten by the next pass
     }
-    __syncthreads();  // s_clo / s_chi are rewritten by the next pass
   }
 }
 
-// One CTA pass covers 2 048 positions; three CTAs per SM (66 registers per thread) hide the searches of one pass behind the copies of another.
-static inline int fill_grid() { return 148 * 3; }
-
-// Launches the copy of a slice: with the edge total known on the host only the kernel that suits the shape, without
-// it both (the one whose shape it is not returns at once).
-// Measured and dropped: the column-tiled copy with 128-bit accesses (a lane owning pairs of consecutive output
-// positions: every store 16 bytes, loads 16 bytes where the column's parity allows) — 0.156 ms against 0.148 ms for the
-// 13.4 M-edge slice of 262,144 columns.  The copy is bound by DRAM behaviour (two thirds of the traffic are stores, ragged
-// column starts), not by instruction count: issue slots are 35 % busy.
+// With the edge total known on the host a CTA per tile (the hardware balances them); without it a grid that fills the chip
+// strides over whatever the device finds.
 template <bool ENCODE>
 static void launch_fill(FillParams p, i64 D, cudaStream_t stream) {
-  p.host_chose = D >= 0;
-  if (D < 0 || !fill_by_output_tiles(p.S, D)) k_slice_fill<ENCODE><<<grid_for(p.S, kTileCols), kThreads, 0, stream>>>(p);
-  if (D < 0 || fill_by_output_tiles(p.S, D)) k_slice_fill_edges<ENCODE><<<fill_grid(), kThreads, 0, stream>>>(p);
+  p.D = D;
+  const int grid = D >= 0 ? min(grid_for(D, kFillTile), 1 << 20) : kNumSMs * 16;
+  k_slice_fill<ENCODE><<<grid, kFillThreads, 0, stream>>>(p);
 }
 
 
@@ -608,13 +562,19 @@ __global__ void __launch_bounds__(kThreads) k_sample_one_keepdim(const i64* __re
 // slice (mode 0) by the counting kernel alone; the total lands in the context's counters.
 int count_scan_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, i64 num_cols, const i64* seeds, i64 S, i64 k,
                       int mode, i64* out_indptr, Mail mail) {
-  const int grid = grid_for(S, kThreads);
+  const bool large = S >= 4ll * kThreads * kNumSMs;  // a full wave of CTAs at four columns per thread
+  const int grid = grid_for(S, large ? 4 * kThreads : kThreads);
   TileState ts;
   int st = ctx_tile_state(ctx, grid, stream, &ts);
   if (st != GSB_OK) return st;
   {
     ScopedKernelTimer timer(ctx, KID_COUNT_SCAN, stream);
-    k_count_scan<<<grid, kThreads, 0, stream>>>(indptr, num_cols, seeds, S, k, mode, out_indptr, ctx_counters(ctx), ts, mail);
+    if (large)
+      k_count_scan<4><<<grid, kThreads, 0, stream>>>(indptr, num_cols, seeds, S, k, mode, out_indptr, ctx_counters(ctx), ts,
+                                                     mail);
+    else
+      k_count_scan<1><<<grid, kThreads, 0, stream>>>(indptr, num_cols, seeds, S, k, mode, out_indptr, ctx_counters(ctx), ts,
+                                                     mail);
   }
   GSB_LAUNCH_OK();
   return GSB_OK;
@@ -700,7 +660,7 @@ int gsb_col_slice_fill(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const
   if (S == 0 || D == 0) return GSB_OK;
   GSB_REQUIRE(indices && out_indices, GSB_ERR_INVALID_ARGUMENT);
   FillParams p{indptr, indices, num_cols, seeds, S, out_indptr, out_indices, out_select, out_coo_col, data, e_ids,
-               out_data, nullptr, 0, 0, false};
+               out_data, nullptr, 0, 0, D};
   {
     ScopedKernelTimer timer(ctx, KID_SLICE_FILL, (cudaStream_t)stream_);
     launch_fill<false>(p, D, (cudaStream_t)stream_);
@@ -725,7 +685,7 @@ int gsb_batch_col_slice_fill(gsb_ctx* ctx, void* stream_, const int64_t* indptr,
   }
   if (S == 0) return GSB_OK;
   FillParams p{indptr, indices, num_cols, seeds, S, out_indptr, out_indices, out_select, out_coo_col, data, e_ids,
-               out_data, nid_ptr, G, encoding_size, false};
+               out_data, nid_ptr, G, encoding_size, -1};
   {
     ScopedKernelTimer timer(ctx, KID_SLICE_FILL, stream);
     if (encoding_size > 0) launch_fill<true>(p, -1, stream);

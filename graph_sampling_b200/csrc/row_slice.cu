@@ -11,6 +11,7 @@
 // (:543-563, 727-771) is the same without offsets.
 #include "batch_table.cuh"
 #include "common.cuh"
+#include "grid_sync.cuh"
 #include "hash_table.cuh"
 #include "radix_sort.cuh"
 #include "scan.cuh"
@@ -22,8 +23,19 @@ constexpr int kRowPerThread = 4;
 constexpr int kRowTile = kRowThreads * kRowPerThread;
 constexpr u64 kMaxFlip = 0x7fffffffffffffffull;  // val = kMaxFlip - position, so atomicMin keeps the LARGEST position
 
+// Membership filter in front of the row table: one bit per hashed id, kept INVERTED (0 = some row id hashes here) so that
+// one 0xFF fill clears table and filter together.  It is small enough for shared memory, and most edges of a slice miss:
+// they never reach the table, whose random 32-byte reads were what the filter kernels waited for.
+struct RowBloom {
+  u32* words;  // null: no filter
+  int shift;   // 64 - log2(bits)
+};
+__device__ __forceinline__ u32 bloom_bit(const RowBloom& b, i64 key) {
+  return (u32)(((u64)key * 0xD6E8FEB86659FD93ull) >> b.shift);
+}
+
 __global__ void __launch_bounds__(kRowThreads) k_build_row_table(const i64* __restrict__ row_ids, i64 R, Table table,
-                                                                 i64* counters) {
+                                                                 RowBloom bloom, i64* counters) {
   for (i64 i = (i64)blockIdx.x * kRowThreads + threadIdx.x; i < R; i += (i64)gridDim.x * kRowThreads) {
     const i64 key = row_ids[i];
     if (key < 0) {
@@ -31,6 +43,10 @@ __global__ void __launch_bounds__(kRowThreads) k_build_row_table(const i64* __re
       continue;
     }
     if (!table_insert_min(table, key, kMaxFlip - (u64)i)) raise_error(counters, GSB_ERR_TABLE_FULL, i);
+    if (bloom.words) {
+      const u32 bit = bloom_bit(bloom, key);
+      atomicAnd(bloom.words + (bit >> 5), ~(1u << (bit & 31)));
+    }
   }
 }
 
@@ -128,6 +144,7 @@ __global__ void __launch_bounds__(kRowThreads) k_row_indptr(const i64* __restric
 // the survivors with ballots + one look-back; the thread that owns the first edge of a column also writes
 // that column's output offset.  (One warp per column was measured 6x slower on a power-law graph: the
 // warp that gets a 17 000-edge column runs 540 dependent rounds while the rest of the grid is idle.)
+constexpr i64 kNoColumn = (i64)1 << 62;
 struct ColRowParams {
   const i64* indptr;
   const i64* indices;
@@ -314,6 +331,220 @@ __global__ void __launch_bounds__(kRowThreads) k_col_row_filter(ColRowParams p) 
   }
 }
 
+// ---- induced subgraph of one node set in one launch -----------------------------------------------------------------
+// The single-batch form of k_col_row_filter as a cooperative kernel: a CTA owns one stretch of the virtual edge list.
+//   filter   tiles of 4 096 positions, columns found as in the slice copy (the tile's columns in shared memory); an edge is
+//            looked up in the table only when the shared-memory filter lets it pass; survivors go to scratch in order, and
+//            every 32 positions leave [survivors of the CTA before them : 32 | bits : 32];
+//   barrier
+//   emit     every CTA scans the CTAs' totals, copies its survivors to their places (and gathers their edge data), and a
+//            share of the columns gets its offset as the rank of the column's first position.
+// 20 000 columns with 6.5 M edges, 20 000 rows: 178 us with a table probe per edge and a look-back chain of 6 400 tiles.
+constexpr int kInThreads = 512;
+constexpr int kInPer = 8;
+constexpr int kInTile = kInThreads * kInPer;
+constexpr int kInWarps = kInThreads / 32;
+constexpr int kInWindow = 512;
+constexpr int kBloomMaxBits = 1 << 19;  // 64 KB: two CTAs per SM
+constexpr i64 kBloomMaxRows = 1 << 18;  // beyond, most edges would pass
+constexpr i64 kInducedMaxEdges = 1 << 27;  // its scratch is 12 bytes per edge
+
+struct InducedParams {
+  ColRowParams c;
+  RowBloom bloom;
+  i64 range;        // positions per CTA, a multiple of kInTile
+  u64* packed;      // [D / 32 + 1]
+  u32* totals;      // [CTAs]
+  u32* kept_row;    // [D] position in row_ids
+  i64* kept_edge;   // [D]
+  GridSync sync;
+};
+
+__global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant__ InducedParams p) {
+  extern __shared__ __align__(16) u32 s_bloom[];
+  __shared__ i64 s_range[2];
+  __shared__ i64 s_delta[kInWindow];
+  __shared__ int s_off[kInWindow + 1];
+  __shared__ u32 s_warp[kInWarps];
+  __shared__ u32 s_prefix[kInThreads];
+  __shared__ i64 s_queue_id[kInWarps][64];            // edges that passed the filter: row id,
+  __shared__ unsigned char s_queue_at[kInWarps][64];  // place among the warp's 256 positions
+  __shared__ u32 s_row[kInWarps][32 * kInPer];        // what the table said
+  const ColRowParams& c = p.c;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const i64 begin = min(c.D, (i64)blockIdx.x * p.range), end = min(c.D, begin + p.range);
+  if (p.bloom.words) {
+    const int quads = (1 << (64 - p.bloom.shift)) / 128;
+    for (int i = tid; i < quads; i += kInThreads)
+      reinterpret_cast<uint4*>(s_bloom)[i] = __ldcg(reinterpret_cast<const uint4*>(p.bloom.words) + i);
+  }
+  u32 kept = 0;  // survivors of the CTA so far
+  for (i64 tile = begin; tile < end; tile += kInTile) {
+    const int here = (int)min((i64)kInTile, end - tile);
+    if (warp < 2) {
+      const i64 col = warp_column_at(c.sub_indptr, c.S, warp == 0 ? tile : tile + here - 1);
+      if (lane == 0) s_range[warp] = col;
+    }
+    __syncthreads();  // (also: the filter is loaded)
+    const i64 c_end = s_range[1] + 1;
+    const int base = warp * (32 * kInPer) + lane;
+    u32 row[kInPer];  // position in row_ids, or kNoRow
+    i64 edge[kInPer];
+    constexpr u32 kNoRow = 0xFFFFFFFFu;
+#pragma unroll
+    for (int r = 0; r < kInPer; ++r) edge[r] = -1;
+    for (i64 c0 = s_range[0]; c0 < c_end; c0 += kInWindow) {
+      const int cols = (int)min((i64)kInWindow, c_end - c0);
+      for (int j = tid; j <= cols; j += kInThreads) {
+        const i64 o = __ldg(c.sub_indptr + c0 + j);
+        s_off[j] = (int)max((i64)0, min(o - tile, (i64)here));
+        if (j < cols) {
+          const i64 col = __ldg(c.seeds + c0 + j);
+          const bool ok = (u64)col < (u64)c.num_cols;  // false only when sub_indptr was not counted for these seeds
+          if (!ok) raise_error(c.counters, GSB_ERR_INDEX_RANGE, c0 + j);
+          s_delta[j] = ok ? __ldg(c.indptr + col) - o + tile : kNoColumn;
+        }
+      }
+      __syncthreads();
+      const int w_begin = s_off[0], w_end = s_off[cols];
+      int at = 0;
+      {
+        const int q = max(base, w_begin);
+        int hi = cols;
+        while (hi - at > 1) {
+          const int mid = (at + hi) >> 1;
+          if (s_off[mid] <= q) at = mid;
+          else hi = mid;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < kInPer; ++r) {
+        const int q = base + r * 32;
+        if (q < w_begin || q >= w_end) continue;
+        while (s_off[at + 1] <= q) ++at;
+        if (s_delta[at] != kNoColumn) edge[r] = q + s_delta[at];
+      }
+      __syncthreads();  // the window is rewritten
+    }
+    i64 id[kInPer];
+#pragma unroll
+    for (int r = 0; r < kInPer; ++r) id[r] = edge[r] >= 0 ? __ldg(c.indices + edge[r]) : -1;
+    // Few edges pass the filter, but nearly every group of 32 has some: looked up where they stand, each group would wait
+    // out a chain of table reads for two or three lanes.  They are queued instead, and looked up 32 at a time.
+    int queued = 0;
+    auto look_up = [&](int count) {
+      __syncwarp();
+      if (lane < count) {
+        const Slot* s = table_find(c.table, s_queue_id[warp][lane]);
+        if (s) s_row[warp][s_queue_at[warp][lane]] = (u32)(kMaxFlip - s->val);
+      }
+      __syncwarp();
+      if (lane + 32 < queued) {  // what lies beyond the 32 moves to the front
+        s_queue_id[warp][lane] = s_queue_id[warp][lane + 32];
+        s_queue_at[warp][lane] = s_queue_at[warp][lane + 32];
+      }
+      queued -= count;
+      __syncwarp();
+    };
+#pragma unroll
+    for (int r = 0; r < kInPer; ++r) s_row[warp][r * 32 + lane] = kNoRow;
+#pragma unroll
+    for (int r = 0; r < kInPer; ++r) {
+      bool pass = id[r] >= 0;
+      if (pass && p.bloom.words) {
+        const u32 bit = bloom_bit(p.bloom, id[r]);
+        pass = ((s_bloom[bit >> 5] >> (bit & 31)) & 1u) == 0u;
+      }
+      const unsigned passing = __ballot_sync(0xffffffffu, pass);
+      if (pass) {
+        const int to = queued + __popc(passing & lt);
+        s_queue_id[warp][to] = id[r];
+        s_queue_at[warp][to] = (unsigned char)(r * 32 + lane);
+      }
+      queued += __popc(passing);
+      if (queued >= 32) look_up(32);
+    }
+    if (queued > 0) look_up(queued);
+#pragma unroll
+    for (int r = 0; r < kInPer; ++r) row[r] = s_row[warp][r * 32 + lane];
+    // ---- ranks: positions of a warp are consecutive, groups of 32
+    unsigned bits[kInPer];
+    u32 warp_total = 0;
+#pragma unroll
+    for (int r = 0; r < kInPer; ++r) {
+      bits[r] = __ballot_sync(0xffffffffu, row[r] != kNoRow);
+      warp_total += __popc(bits[r]);
+    }
+    if (lane == 0) s_warp[warp] = warp_total;
+    __syncthreads();
+    u32 before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kInWarps; ++w) {
+      const u32 t = s_warp[w];
+      if (w < warp) before += t;
+      all += t;
+    }
+    u32 run = kept + before;
+#pragma unroll
+    for (int r = 0; r < kInPer; ++r) {
+      const int q = base + r * 32;
+      if (lane == 0 && q < here) p.packed[(tile + q) >> 5] = ((u64)run << 32) | (u64)bits[r];
+      if (row[r] != kNoRow) {
+        const i64 to = begin + run + __popc(bits[r] & lt);
+        p.kept_row[to] = row[r];
+        p.kept_edge[to] = edge[r];
+      }
+      run += __popc(bits[r]);
+    }
+    kept += all;
+  }
+  if (tid == 0) p.totals[blockIdx.x] = kept;
+  grid_barrier(p.sync, 1);
+  // ---- emit
+  u32 total;
+  {
+    const u32 t = tid < (int)gridDim.x ? __ldcg(p.totals + tid) : 0;
+    u32 inc = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    u32 before = 0;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < kInWarps; ++w) {
+      if (w < warp) before += s_warp[w];
+      total += s_warp[w];
+    }
+    s_prefix[tid] = before + inc - t;
+    __syncthreads();
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    c.counters[CNT_NNZ] = total;
+    mail_post(c.mail, 0, total, c.counters);
+  }
+  const i64 out0 = s_prefix[blockIdx.x];
+  for (u32 j = tid; j < kept; j += kInThreads) {  // written by this very CTA
+    const i64 e = __ldcg(p.kept_edge + begin + j);
+    c.out_indices[out0 + j] = c.renumber ? (i64)__ldcg(p.kept_row + begin + j) : __ldg(c.indices + e);
+    if (c.out_select) c.out_select[out0 + j] = e;
+    if (c.out_data) c.out_data[out0 + j] = __ldg(c.data + (c.e_ids ? __ldg(c.e_ids + e) : e));
+  }
+  for (i64 j = (i64)blockIdx.x * kInThreads + tid; j <= c.S; j += (i64)gridDim.x * kInThreads) {
+    const i64 pos = __ldg(c.sub_indptr + j);
+    i64 rank = total;
+    if (pos < c.D) {
+      const u64 w = __ldcg(p.packed + (pos >> 5));
+      rank = s_prefix[pos / p.range] + (u32)(w >> 32) + __popc((u32)w & ((1u << (pos & 31)) - 1u));
+    }
+    c.out_indptr[j] = rank;
+  }
+}
+
 // ---- index search: position of every key in `origin` (largest position for a repeated id), -1 if absent --
 __global__ void __launch_bounds__(kRowThreads) k_index_search(const i64* __restrict__ keys, i64 M, Table table,
                                                               i64* __restrict__ out) {
@@ -328,21 +559,31 @@ __global__ void __launch_bounds__(kRowThreads) k_index_search(const i64* __restr
 
 using namespace gsb;
 
+// With `bloom` the filter is built too: 24 bits per row id (a miss passes it one time in 25), at most kBloomMaxBits.
 static int build_table(gsb_ctx* ctx, cudaStream_t stream, const int64_t* row_ids, int64_t R, size_t extra_bytes,
-                       Table* table, void** extra) {
+                       Table* table, void** extra, RowBloom* bloom = nullptr) {
   u64 cap;
   table_geometry(R, &cap, &table->shift);
   table->mask = cap - 1;
+  int bits_log2 = 10;
+  while (bloom && (1 << bits_log2) < kBloomMaxBits && ((i64)1 << bits_log2) < 24 * R) ++bits_log2;
+  const size_t bloom_bytes = bloom ? ((size_t)1 << bits_log2) / 8 : 0;
   void* ws;
-  const size_t table_bytes = cap * sizeof(Slot);
+  const size_t table_bytes = cap * sizeof(Slot) + bloom_bytes;
   int st = ctx_reserve_workspace(ctx, table_bytes + extra_bytes + 256, &ws);
   if (st != GSB_OK) return st;
   table->slots = (Slot*)ws;
   *extra = (char*)ws + table_bytes;
+  RowBloom filter{nullptr, 0};
+  if (bloom) {
+    filter.words = (u32*)((char*)ws + cap * sizeof(Slot));
+    filter.shift = 64 - bits_log2;
+    *bloom = filter;
+  }
   GSB_CUDA_OK(cudaMemsetAsync(table->slots, 0xFF, table_bytes, stream));
   if (R > 0) {
     k_build_row_table<<<min(grid_for(R, kRowThreads), kNumSMs * 8), kRowThreads, 0, stream>>>(row_ids, R, *table,
-                                                                                              ctx_counters(ctx));
+                                                                                              filter, ctx_counters(ctx));
     GSB_LAUNCH_OK();
     ctx_count_launches(ctx, 1);
   }
@@ -457,6 +698,44 @@ int gsb_col_row_slice(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
     return GSB_OK;
   }
   Table table;
+  if (!col_ptr && column_ids && D <= kInducedMaxEdges && R < (i64)1 << 31) {
+    static int resident[64];
+    static bool attr_set[64];
+    const int dev = ctx_device(ctx);
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+      GSB_CUDA_OK(cudaFuncSetAttribute(k_induced, cudaFuncAttributeMaxDynamicSharedMemorySize, kBloomMaxBits / 8));
+      attr_set[dev] = true;
+    }
+    const int ctas = min(kInThreads, ctx_resident_ctas(ctx, (const void*)k_induced, kInThreads, kBloomMaxBits / 8, resident));
+    if (ctas > 0) {
+      InducedParams p{};
+      const i64 tiles = (D + kInTile - 1) / kInTile;
+      p.range = ((tiles + ctas - 1) / ctas) * kInTile;
+      const int grid = (int)((D + p.range - 1) / p.range);
+      auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+      const size_t packed_bytes = al(8 * ((size_t)D / 32 + 2)), edge_bytes = al(8 * (size_t)D), row_bytes = al(4 * (size_t)D);
+      void* extra;
+      int st = build_table(ctx, stream, row_ids, R, packed_bytes + edge_bytes + row_bytes + 4 * kInThreads, &table, &extra,
+                           R <= kBloomMaxRows ? &p.bloom : nullptr);
+      if (st != GSB_OK) return st;
+      p.packed = (u64*)extra;
+      p.kept_edge = (i64*)((char*)extra + packed_bytes);
+      p.kept_row = (u32*)((char*)extra + packed_bytes + edge_bytes);
+      p.totals = (u32*)((char*)extra + packed_bytes + edge_bytes + row_bytes);
+      p.c = ColRowParams{indptr, indices, num_cols, column_ids, S, sub_indptr, D, nullptr, G, encoding_size, table,
+                         renumber ? 1 : 0, out_indptr, out_indices, out_select, data, e_ids, out_data, ctx_counters(ctx),
+                         TileState{}, nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0}};
+      p.sync = ctx_grid_sync(ctx, grid, 1);
+      {
+        ScopedKernelTimer timer(ctx, KID_ROW_FILTER, stream);
+        void* args[] = {&p};
+        st = launch_cooperative(ctx, stream, (const void*)k_induced, grid, kInThreads,
+                                p.bloom.words ? ((size_t)1 << (64 - p.bloom.shift)) / 8 : 0, args, p.sync);
+      }
+      if (st != GSB_OK) return st;
+      return finish_count(ctx, stream, p.c.mail, nnz_host);
+    }
+  }
   int st = col_row_table(ctx, stream, row_ids, R, row_ptr, G, encoding_size, &table);
   if (st != GSB_OK) return st;
   const int tiles = grid_for(D, kCrTile);

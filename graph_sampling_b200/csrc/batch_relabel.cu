@@ -624,6 +624,12 @@ static inline bool partition_suits(i64 n_cap, i64 G) {
   return n_cap >= kPartitionAutoItems && n_cap / (G > 0 ? G : 1) <= kPartitionAutoMaxMinibatch;
 }
 
+// Id bound that the batched forms may hold the caller to: where the tables of the call are small, ids beyond num_nodes have
+// always been an error (the direct-address tables below refuse them).
+static inline i64 direct_bound(i64 G, i64 num_nodes) {
+  return num_nodes < 0xFFFFFFFFll && (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes ? num_nodes : 0;
+}
+
 static int read_totals(gsb_ctx* ctx, cudaStream_t stream, i64* unique_total_host, i64* edges_total_host) {
   const i64* c;
   int st = ctx_fetch_counters(ctx, stream, CNT_ERROR, 4, &c);
@@ -656,7 +662,7 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
   if (path == 0 && L.indices_ptr && fused_unique_suits(ctx, n_cap, G))
     return fused_unique_batched(ctx, stream, L, seeds_bound, edges_bound, nullptr, nullptr, out_unique, out_unique_ptr,
-                                out_relabeled, mail);
+                                out_relabeled, direct_bound(G, num_nodes), mail);
   u64* tables = nullptr;
   uint32_t epoch = 0;
   // Automatic choice: direct-address tables only while all tables of the call stay L2-sized.  A minibatch touches
@@ -895,7 +901,7 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
     F.indices = out_indices;
     F.G = G;
     st = fused_unique_batched(ctx, stream, F, S, cap, out_indptr, out_indices_ptr, out_unique, out_unique_ptr,
-                              out_relabeled, mail);
+                              out_relabeled, direct_bound(G, num_nodes), mail);
     if (st != GSB_OK || !mail.word) return st;
     return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
   }

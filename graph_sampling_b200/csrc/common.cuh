@@ -125,10 +125,12 @@ i64 ctx_option(gsb_ctx* ctx, int option);
 int ctx_direct_tables(gsb_ctx* ctx, i64 count, i64 num_nodes, cudaStream_t stream, u64** out_table,
                       uint32_t* out_epoch);
 int ctx_check_device_error(gsb_ctx* ctx, cudaStream_t stream);
-// Epoch-tagged hash table of the single-launch unique + relabel (fused_unique.cu): at least `slots` 64-bit words kept by
-// the context, never cleared between calls.  *epoch (1 .. epochs - 1) is new for every call; when the epochs are used up,
-// and when the table grows, it is zeroed.  Bounded by what kFusedUniqueMaxItems needs (64 MB), freed with the context.
-int ctx_epoch_table(gsb_ctx* ctx, i64 slots, uint32_t epochs, cudaStream_t stream, u64** table, uint32_t* epoch);
+// Epoch-tagged tables of the single-launch unique + relabel (fused_unique.cu): at least `bytes` bytes kept by the context,
+// never cleared between calls.  which = 0: hash table, 1: direct-address table.  *epoch (1 .. epochs - 1) is new for every
+// call; when the epochs are used up, and when the table grows, every byte is set to `fill`.  Bounded by the callers (64 MB
+// each), freed with the context.
+int ctx_epoch_table(gsb_ctx* ctx, int which, size_t bytes, int fill, uint32_t epochs, cudaStream_t stream, void** table,
+                    uint32_t* epoch);
 // Waits until everything queued on `stream` so far is done and returns the `n` counters starting at `first` (a copy in
 // page-locked memory, written by a one-warp kernel that the host spins on).
 int ctx_fetch_counters(gsb_ctx* ctx, cudaStream_t stream, int first, int n, const i64** out);

@@ -37,10 +37,10 @@ struct gsb_ctx {
   u64* direct_tables;
   size_t direct_bytes;
   uint32_t direct_epoch;
-  // table and barrier word of the single-launch unique + relabel (see ctx_epoch_table)
-  u64* epoch_table;
-  i64 epoch_slots;
-  uint32_t table_epoch;
+  // tables of the single-launch unique + relabel (see ctx_epoch_table)
+  void* epoch_table[2];
+  size_t epoch_bytes[2];
+  uint32_t table_epoch[2];
   u64 barrier_arrivals;  // the barrier word itself is counters[CNT_NUM]
   cudaEvent_t wait_event;  // created on first use when GSB_OPT_BLOCKING_WAIT is set
 };
@@ -144,25 +144,26 @@ int ctx_direct_tables(gsb_ctx* ctx, i64 count, i64 num_nodes, cudaStream_t strea
   return GSB_OK;
 }
 
-int ctx_epoch_table(gsb_ctx* ctx, i64 slots, uint32_t epochs, cudaStream_t stream, u64** table, uint32_t* epoch) {
-  if (slots > ctx->epoch_slots) {
+int ctx_epoch_table(gsb_ctx* ctx, int which, size_t bytes, int fill, uint32_t epochs, cudaStream_t stream, void** table,
+                    uint32_t* epoch) {
+  if (bytes > ctx->epoch_bytes[which]) {
     GSB_CUDA_OK(cudaDeviceSynchronize());
-    if (ctx->epoch_table) GSB_CUDA_OK(cudaFree(ctx->epoch_table));
-    ctx->epoch_table = nullptr;
-    ctx->epoch_slots = 0;
-    i64 cap = 1 << 16;
-    while (cap < slots) cap <<= 1;
-    GSB_CUDA_OK(cudaMalloc((void**)&ctx->epoch_table, sizeof(u64) * (size_t)cap));
-    ctx->epoch_slots = cap;
-    ctx->table_epoch = epochs - 1;  // cleared below
+    if (ctx->epoch_table[which]) GSB_CUDA_OK(cudaFree(ctx->epoch_table[which]));
+    ctx->epoch_table[which] = nullptr;
+    ctx->epoch_bytes[which] = 0;
+    size_t cap = 1 << 19;
+    while (cap < bytes) cap <<= 1;
+    GSB_CUDA_OK(cudaMalloc(&ctx->epoch_table[which], cap));
+    ctx->epoch_bytes[which] = cap;
+    ctx->table_epoch[which] = epochs - 1;  // filled below
   }
-  ctx->table_epoch += 1;
-  if (ctx->table_epoch >= epochs) {
-    GSB_CUDA_OK(cudaMemsetAsync(ctx->epoch_table, 0, sizeof(u64) * (size_t)ctx->epoch_slots, stream));
-    ctx->table_epoch = 1;
+  ctx->table_epoch[which] += 1;
+  if (ctx->table_epoch[which] >= epochs) {
+    GSB_CUDA_OK(cudaMemsetAsync(ctx->epoch_table[which], fill, ctx->epoch_bytes[which], stream));
+    ctx->table_epoch[which] = 1;
   }
-  *table = ctx->epoch_table;
-  *epoch = ctx->table_epoch;
+  *table = ctx->epoch_table[which];
+  *epoch = ctx->table_epoch[which];
   return GSB_OK;
 }
 
@@ -421,7 +422,8 @@ int gsb_ctx_destroy(gsb_ctx* ctx) {
   if (ctx->workspace) cudaFree(ctx->workspace);
   if (ctx->tile_words) cudaFree(ctx->tile_words);
   if (ctx->direct_tables) cudaFree(ctx->direct_tables);
-  if (ctx->epoch_table) cudaFree(ctx->epoch_table);
+  for (void* t : ctx->epoch_table)
+    if (t) cudaFree(t);
   if (ctx->wait_event) cudaEventDestroy(ctx->wait_event);
   if (ctx->counters) cudaFree(ctx->counters);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);

@@ -19,11 +19,17 @@
 //            itself) + its word's prefix + the bits below it: the frontier is written at those ranks, and every item to
 //            relabel writes the rank of the first occurrence of its id.
 //
+// DIRECT: when the ids are known to be below a bound and the table of one 4-byte word per id and minibatch stays small, the
+// table is addressed by the id itself, [2047 - epoch : 11 | position : 21], and an insertion is one fire-and-forget
+// reduction: no reads, no chains, no answers to wait for.  An id beyond the bound makes the call report
+// GSB_ERR_INDEX_RANGE, and the caller repeats it with the hash table.
+//
 // BATCHED: the items belong to G minibatches (numbered batch-major, as in batch_table.cuh), each with a region of the
 // table of its own; ranks are then relative to the minibatch's first item.
 //
-// Against the five-launch form, GPU time without its launch gaps: 16 000 items 26 -> 11 us, 813 000 items 86 -> 52 us.
-// What bounds it now: the chain bucket read -> CAS -> CAS of the slowest lane of every warp, item after item.
+// GPU time of a call, five launches (without the gaps between them) / hash table / direct table: 16 000 items
+// 26 / 11 / 7 us, 813 000 items 86 / 51 / 29 us.  What bounds the hash table (813 000 items): bucket reads and
+// compare-and-swaps at the rate of the L2's atomics, 107 G/s each, and the rounds of the slowest lanes behind them.
 #include "batch_table.cuh"
 #include "common.cuh"
 #include "grid_sync.cuh"
@@ -60,6 +66,9 @@ struct FusedParams {
   // scratch
   u64* table;
   u64 epoch;  // already shifted
+  u32* direct;       // DIRECT: [minibatches][id_bound]
+  u32 direct_epoch;  // already inverted and shifted
+  u32 id_bound;
   u64* packed;    // [items / 32 + 1]  first occurrences of the CTA before the word << 32 | bits
   u32* totals;    // [CTAs]
   u32* seed_ref;  // [S] first position of every id of `first` (only with col_index)
@@ -97,27 +106,24 @@ __device__ __forceinline__ void load_bucket(const u64* table, u32 bucket, u64 (&
   w[3] = b.y;
 }
 
-// Slot of the bucket that holds mine's id with a position no larger than mine's — found or newly claimed — or kFuNone when
-// the bucket is full of other ids.  An id always takes the first slot that is free, so nobody misses a copy of it.
-__device__ __forceinline__ u32 claim_in_bucket(const FusedParams& p, u32 bucket, const u64 (&word)[4], u64 mine) {
+// The first slot of a bucket, in the order start, start + 1, ... (mod 4), that is free or holds mine's id; 4 if none does.
+// Starting places differ from id to id: with everybody trying slot 0 first, the ids of a bucket queued up behind each
+// other's compare-and-swaps.
+__device__ __forceinline__ u32 pick_slot(const u64 (&w)[4], u32 start, u64 mine, u64 epoch, u64* word) {
+  u32 best = 4;
 #pragma unroll
   for (u32 j = 0; j < 4; ++j) {
-    u64 w = word[j];
-    u64* s = p.table + 4ull * bucket + j;
-    if ((w ^ p.epoch) >> (32 + kFuPosBits)) {  // of an older epoch: free
-      const u64 old = atomicCAS(s, w, mine);
-      if (old == w) return 4 * bucket + j;
-      w = old;  // of this epoch: whoever was first put it there
-    }
-    if (((w ^ mine) >> kFuPosBits) == 0) {
-      if (w > mine) atomicMin(s, mine);
-      return 4 * bucket + j;
+    const u32 turn = (j - start) & 3u;
+    const bool usable = ((w[j] ^ epoch) >> (32 + kFuPosBits)) != 0 || ((w[j] ^ mine) >> kFuPosBits) == 0;
+    if (usable && turn < best) {
+      best = turn;
+      *word = w[j];
     }
   }
-  return kFuNone;
+  return best == 4 ? 4 : (best + start) & 3u;
 }
 
-template <int R, bool BATCHED>
+template <int R, bool BATCHED, bool DIRECT>
 __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_constant__ FusedParams p) {
   constexpr u32 kItems = kFuThreads * R;  // of a CTA
   __shared__ u32 s_group[kFuWarps * R];   // counts per 32 items, then their exclusive prefixes
@@ -216,6 +222,7 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
   };
 
   // ---- insert
+  auto in_range = [&](i64 v) { return DIRECT ? (u64)v < (u64)p.id_bound : valid_id(v); };
   u32 id[R], slot[R], batch0[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -228,51 +235,87 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
         const Where w = where(g);
         const u32 lc = g - w.begin, seeds = w.next_seeds - w.seeds;
         if (w.ok) v = lc < seeds ? __ldg(p.first + w.seeds + lc) : __ldg(p.second + (g - w.next_seeds));
-        region = fused_bucket0(w.begin, (u32)w.batch);
-        size = fused_bucket0(w.next_begin, (u32)w.batch + 1) - region;
+        region = DIRECT ? (u32)w.batch * p.id_bound : fused_bucket0(w.begin, (u32)w.batch);
+        size = DIRECT ? 0 : fused_bucket0(w.next_begin, (u32)w.batch + 1) - region;
         batch0[r] = w.begin;
       } else {
         v = g < (u32)p.S ? __ldg(p.first + g) : __ldg(p.second + (g - (u32)p.S));
       }
-      if (!valid_id(v)) raise_error(p.counters, GSB_ERR_INDEX_RANGE, g);
+      if (!in_range(v)) raise_error(p.counters, GSB_ERR_INDEX_RANGE, g);
     }
-    id[r] = valid_id(v) ? (u32)v : kFuNone;
+    id[r] = in_range(v) ? (u32)v : kFuNone;
     slot[r] = kFuNone;
-    if (id[r] != kFuNone) slot[r] = region + fused_home(id[r], size);
+    if (id[r] != kFuNone) slot[r] = region + (DIRECT ? id[r] : fused_home(id[r], size));
   }
-  // the home buckets of up to two items are in flight at once; an insertion is one read and one atomic almost always
-  constexpr int kAhead = R < 2 ? R : 2;
+  if (DIRECT) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (slot[r] != kFuNone)
+        asm volatile("red.relaxed.gpu.global.min.u32 [%0], %1;" ::"l"(p.direct + slot[r]),
+                     "r"(p.direct_epoch | (base + r * kFuThreads + tid))
+                     : "memory");
+  } else {
+  // A round reads the buckets of up to four unsettled items, then issues their compare-and-swaps, then looks at the
+  // answers: the two round trips are paid per round, not per item.  An id always takes the first usable slot of its own
+  // order, and slots are never given up, so nobody misses a copy of it.
+  constexpr int kAhead = R < 4 ? R : 4;
 #pragma unroll
   for (int r0 = 0; r0 < R; r0 += kAhead) {
-    u64 word[kAhead][4];
-#pragma unroll
-    for (int q = 0; q < kAhead; ++q)
-      if (slot[r0 + q] != kFuNone) load_bucket(p.table, slot[r0 + q], word[q]);
+    u32 bucket[kAhead], probes = 0;
+    unsigned open = 0;
 #pragma unroll
     for (int q = 0; q < kAhead; ++q) {
-      const int r = r0 + q;
-      if (slot[r] == kFuNone) continue;
-      const u32 g = base + r * kFuThreads + tid;
-      const u64 mine = p.epoch | ((u64)id[r] << kFuPosBits) | (u64)g;
-      u32 bucket = slot[r];
-      u32 at = claim_in_bucket(p, bucket, word[q], mine);
-      if (at == kFuNone) {
-        u32 lo = 0, end = fused_bucket0(n, 1);  // the buckets of the item's region
-        if (BATCHED) {
-          const Where w = where(g);
-          lo = fused_bucket0(w.begin, (u32)w.batch);
-          end = fused_bucket0(w.next_begin, (u32)w.batch + 1);
-        }
-        for (u32 probe = lo; at == kFuNone && probe < end; ++probe) {
-          bucket = bucket + 1 == end ? lo : bucket + 1;
-          u64 more[4];
-          load_bucket(p.table, bucket, more);
-          at = claim_in_bucket(p, bucket, more, mine);
-        }
-        if (at == kFuNone) raise_error(p.counters, GSB_ERR_TABLE_FULL, g);  // more slots than items: cannot happen
-      }
-      slot[r] = at;
+      bucket[q] = slot[r0 + q];
+      if (slot[r0 + q] != kFuNone) open |= 1u << q;
     }
+    while (open) {
+      u64 expect[kAhead], found[kAhead];
+      u32 at[kAhead];
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        at[q] = 4;
+        if (!((open >> q) & 1u)) continue;
+        u64 w[4];
+        load_bucket(p.table, bucket[q], w);
+        const u64 mine = p.epoch | ((u64)id[r0 + q] << kFuPosBits) | (u64)(base + (r0 + q) * kFuThreads + tid);
+        at[q] = pick_slot(w, id[r0 + q] & 3u, mine, p.epoch, &expect[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        found[q] = 0;
+        if (!((open >> q) & 1u) || at[q] == 4) continue;
+        const u64 mine = p.epoch | ((u64)id[r0 + q] << kFuPosBits) | (u64)(base + (r0 + q) * kFuThreads + tid);
+        found[q] = expect[q];
+        if ((expect[q] ^ p.epoch) >> (32 + kFuPosBits)) found[q] = atomicCAS(p.table + 4ull * bucket[q] + at[q], expect[q], mine);
+      }
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        if (!((open >> q) & 1u)) continue;
+        const u32 g = base + (r0 + q) * kFuThreads + tid;
+        const u64 mine = p.epoch | ((u64)id[r0 + q] << kFuPosBits) | (u64)g;
+        if (at[q] == 4) {  // full of other ids: the next bucket of the item's region
+          u32 lo = 0, end = fused_bucket0(n, 1);
+          if (BATCHED) {
+            const Where w = where(g);
+            lo = fused_bucket0(w.begin, (u32)w.batch);
+            end = fused_bucket0(w.next_begin, (u32)w.batch + 1);
+          }
+          bucket[q] = bucket[q] + 1 == end ? lo : bucket[q] + 1;
+          if (++probes > 4 * (end - lo)) {  // more slots than items: cannot happen
+            raise_error(p.counters, GSB_ERR_TABLE_FULL, g);
+            slot[r0 + q] = kFuNone;
+            open &= ~(1u << q);
+          }
+          continue;
+        }
+        const bool claimed = found[q] == expect[q] && ((expect[q] ^ p.epoch) >> (32 + kFuPosBits)) != 0;
+        if (!claimed && ((found[q] ^ mine) >> kFuPosBits) != 0) continue;  // somebody else's id came first: look again
+        if (!claimed && found[q] > mine) atomicMin(p.table + 4ull * bucket[q] + at[q], mine);
+        slot[r0 + q] = 4 * bucket[q] + at[q];
+        open &= ~(1u << q);
+      }
+    }
+  }
   }
   for (i64 j = (i64)blockIdx.x * kFuThreads + tid; j < p.copy_n; j += (i64)gridDim.x * kFuThreads)
     p.copy_dst[j] = __ldg(p.copy_src + j);
@@ -284,7 +327,8 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
   for (int r = 0; r < R; ++r) {
     const u32 g = base + r * kFuThreads + tid;
     u32 ref = kFuNone;
-    if (slot[r] != kFuNone) ref = (u32)(__ldcg(p.table + slot[r]) & kFuPosMask);
+    if (slot[r] != kFuNone)
+      ref = DIRECT ? __ldcg(p.direct + slot[r]) & (u32)kFuPosMask : (u32)(__ldcg(p.table + slot[r]) & kFuPosMask);
     if (!BATCHED && p.col_index && g < (u32)p.S) p.seed_ref[g] = ref;
     slot[r] = ref;  // from here on: the first position of the item's id
     bits[r] = __ballot_sync(0xffffffffu, ref == g);
@@ -400,22 +444,25 @@ static int items_per_thread(i64 n, int max_ctas) {
   return r;
 }
 
-template <bool BATCHED>
+template <bool BATCHED, bool DIRECT>
 static const void* fused_kernel(int r) {
   switch (r) {
-    case 1: return (const void*)k_fused_unique<1, BATCHED>;
-    case 2: return (const void*)k_fused_unique<2, BATCHED>;
-    case 4: return (const void*)k_fused_unique<4, BATCHED>;
-    case 8: return (const void*)k_fused_unique<8, BATCHED>;
-    default: return (const void*)k_fused_unique<16, BATCHED>;
+    case 1: return (const void*)k_fused_unique<1, BATCHED, DIRECT>;
+    case 2: return (const void*)k_fused_unique<2, BATCHED, DIRECT>;
+    case 4: return (const void*)k_fused_unique<4, BATCHED, DIRECT>;
+    case 8: return (const void*)k_fused_unique<8, BATCHED, DIRECT>;
+    default: return (const void*)k_fused_unique<16, BATCHED, DIRECT>;
   }
 }
 
+// All instantiations are compiled for two CTAs per SM; the largest of each kind is asked.
 static int resident_ctas(gsb_ctx* ctx) {
-  static int single[64], batched[64];
-  const int a = ctx_resident_ctas(ctx, (const void*)k_fused_unique<16, false>, kFuThreads, 0, single);
-  const int b = ctx_resident_ctas(ctx, (const void*)k_fused_unique<16, true>, kFuThreads, 0, batched);
-  return min(min(a, b), kFuThreads);  // one thread per CTA total in the scan
+  static int known[4][64];
+  int ctas = kFuThreads;  // one thread per CTA total in the scan
+  ctas = min(ctas, ctx_resident_ctas(ctx, fused_kernel<false, false>(16), kFuThreads, 0, known[0]));
+  ctas = min(ctas, ctx_resident_ctas(ctx, fused_kernel<true, false>(16), kFuThreads, 0, known[1]));
+  ctas = min(ctas, ctx_resident_ctas(ctx, fused_kernel<false, true>(16), kFuThreads, 0, known[2]));
+  return min(ctas, ctx_resident_ctas(ctx, fused_kernel<true, true>(16), kFuThreads, 0, known[3]));
 }
 
 bool fused_unique_suits(gsb_ctx* ctx, i64 n, i64 G) {
@@ -423,10 +470,15 @@ bool fused_unique_suits(gsb_ctx* ctx, i64 n, i64 G) {
          n <= (i64)resident_ctas(ctx) * kFuThreads * 16;
 }
 
+// The direct-address table: 4 bytes per id and minibatch.  Up to 32 MB it lives in L2 beside what the call reads.
+bool fused_unique_direct(i64 G, i64 id_bound) { return id_bound > 0 && (double)G * (double)id_bound * 4.0 <= (double)(32 << 20); }
+
 template <bool BATCHED>
-static int launch_fused(gsb_ctx* ctx, cudaStream_t stream, FusedParams p, i64 n) {
+static int launch_fused(gsb_ctx* ctx, cudaStream_t stream, FusedParams p, i64 n, i64 id_bound) {
   const int r = items_per_thread(n, resident_ctas(ctx));
   const int grid = grid_for(n, kFuThreads * r);
+  const i64 G = BATCHED ? p.G : 1;
+  const bool direct = fused_unique_direct(G, id_bound);
   void* ws;
   const size_t packed_bytes = ((size_t)n / 32 + 2) * 8;
   int st = ctx_reserve_workspace(ctx, packed_bytes + sizeof(u32) * (size_t)(kFuThreads + (p.col_index ? p.S : 0)), &ws);
@@ -434,20 +486,27 @@ static int launch_fused(gsb_ctx* ctx, cudaStream_t stream, FusedParams p, i64 n)
   p.packed = (u64*)ws;
   p.totals = (u32*)((char*)ws + packed_bytes);
   p.seed_ref = p.totals + kFuThreads;
+  void* table;
   u32 epoch;
-  st = ctx_epoch_table(ctx, 4 * (i64)fused_bucket0((u32)n, (u32)(BATCHED ? p.G : 1)), kFuEpochs, stream, &p.table, &epoch);
+  if (direct) st = ctx_epoch_table(ctx, 1, sizeof(u32) * (size_t)(G * id_bound), 0xFF, kFuEpochs, stream, &table, &epoch);
+  else st = ctx_epoch_table(ctx, 0, 32 * (size_t)fused_bucket0((u32)n, (u32)G), 0, kFuEpochs, stream, &table, &epoch);
   if (st != GSB_OK) return st;
+  p.table = (u64*)table;
   p.epoch = (u64)epoch << (32 + kFuPosBits);
+  p.direct = (u32*)table;
+  p.direct_epoch = (kFuEpochs - 1 - epoch) << kFuPosBits;
+  p.id_bound = (u32)id_bound;
   p.counters = ctx_counters(ctx);
   p.sync = ctx_grid_sync(ctx, grid, 2);
   ScopedKernelTimer timer(ctx, KID_RELABEL, stream);
   void* args[] = {&p};
-  return launch_cooperative(ctx, stream, fused_kernel<BATCHED>(r), grid, kFuThreads, 0, args, p.sync);
+  return launch_cooperative(ctx, stream, direct ? fused_kernel<BATCHED, true>(r) : fused_kernel<BATCHED, false>(r), grid,
+                            kFuThreads, 0, args, p.sync);
 }
 
 int fused_unique_single(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64 S, const i64* second, i64 E,
                         const i64* col_index, i64* out_unique, i64* out_second, i64* out_col, const i64* copy_src,
-                        i64* copy_dst, i64 copy_n, Mail mail) {
+                        i64* copy_dst, i64 copy_n, i64 id_bound, Mail mail) {
   FusedParams p{};
   p.first = first;
   p.second = second;
@@ -461,12 +520,12 @@ int fused_unique_single(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64
   p.copy_dst = copy_dst;
   p.copy_n = copy_src && copy_dst ? copy_n : 0;
   p.mail = mail;
-  return launch_fused<false>(ctx, stream, p, S + E);
+  return launch_fused<false>(ctx, stream, p, S + E, id_bound);
 }
 
 int fused_unique_batched(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L, i64 seeds_bound, i64 edges_bound,
                          const i64* sub_indptr, i64* out_indices_ptr, i64* out_unique, i64* out_unique_ptr,
-                         i64* out_relabeled, Mail mail) {
+                         i64* out_relabeled, i64 id_bound, Mail mail) {
   FusedParams p{};
   p.first = L.seeds;
   p.second = L.indices;
@@ -481,7 +540,7 @@ int fused_unique_batched(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L
   p.out_unique_ptr = out_unique_ptr;
   p.G = L.G;
   p.mail = mail;
-  return launch_fused<true>(ctx, stream, p, seeds_bound + edges_bound);
+  return launch_fused<true>(ctx, stream, p, seeds_bound + edges_bound, id_bound);
 }
 
 }  // namespace gsb

@@ -49,16 +49,17 @@ class Graph:
         self.data_ = None
         self.col_ids_, self.row_ids_ = col_ids, row_ids
         self.val_col_ids_ = self.val_row_ids_ = None
+        self._id_bound = 0   # node ids of the loaded graph lie below it (0: unknown); a hint, inherited by its slices
 
     # ---- loading (src/graph.cc:14-60) -------------------------------------------------------------
     def LoadCSC(self, indptr, indices):
         self.csc_ = CSC(indptr, indices)
-        self.num_cols_ = self.num_rows_ = indptr.numel() - 1
+        self.num_cols_ = self.num_rows_ = self._id_bound = indptr.numel() - 1
         self.num_edges_ = indices.numel()
 
     def LoadCSR(self, indptr, indices):
         self.csr_ = CSC(indptr, indices)
-        self.num_cols_ = self.num_rows_ = indptr.numel() - 1
+        self.num_cols_ = self.num_rows_ = self._id_bound = indptr.numel() - 1
         self.num_edges_ = indices.numel()
 
     def LoadCOO(self, row, col):
@@ -239,7 +240,9 @@ class Graph:
 
     # ---- helpers -----------------------------------------------------------------------------------------
     def _child(self, col_ids, row_ids, num_cols, num_rows):
-        return Graph(True, col_ids, row_ids, num_cols, num_rows)
+        ret = Graph(True, col_ids, row_ids, num_cols, num_rows)
+        ret._id_bound = self._id_bound
+        return ret
 
     def _gather_args(self, fmt_struct):
         """(data, e_ids) handed to a kernel so that it emits data_[e_ids?[select_index]] itself."""
@@ -368,6 +371,7 @@ class Graph:
             frontier, (indices,) = ops.relabel([indices], [indices])
             new_row_ids, new_num_rows = frontier, frontier.numel()
         ret = self._child(new_col_ids, new_row_ids, n_ids.numel(), new_num_rows)
+        ret._id_bound = 0    # ids carry their batch number
         ret.num_edges_ = indices.numel()
         if output_format & _CSC:
             ret.csc_ = CSC(indptr, indices)
@@ -524,7 +528,7 @@ class Graph:
             rows = self.row_ids_ if self.row_ids_ is not None else self.coo_.row
         else:
             _fatal("Error in AllValidNode!")
-        return ops.relabel([col_ids, rows], [])[0]
+        return ops.graph_unique(col_ids, rows, id_bound=self._id_bound)
 
     def Relabel(self):
         col_ids = self._require_col_ids()
@@ -532,13 +536,15 @@ class Graph:
             if self.val_col_ids_ is not None:
                 col_ids = col_ids[self.val_col_ids_]
             row_indices = self.row_ids_[self.csc_.indices] if self.row_ids_ is not None else self.csc_.indices
-            frontier, relabeled, _, indptr = ops.graph_relabel(col_ids, row_indices, indptr=self.csc_.indptr)
+            frontier, relabeled, _, indptr = ops.graph_relabel(col_ids, row_indices, indptr=self.csc_.indptr,
+                                                                id_bound=self._id_bound)
             return frontier, frontier.numel(), col_ids.numel(), indptr, relabeled, self.csc_.e_ids, "csc"
         if self.csr_ is not None or self.coo_ is not None:
             if self.coo_ is None:
                 self.coo_ = self._csc2coo(self.csr_, False)
             coo_row = self.row_ids_[self.coo_.row] if self.row_ids_ is not None else self.coo_.row
-            frontier, rel_row, rel_col, _ = ops.graph_relabel(col_ids, coo_row, cols=self.coo_.col)
+            frontier, rel_row, rel_col, _ = ops.graph_relabel(col_ids, coo_row, cols=self.coo_.col,
+                                                               id_bound=self._id_bound)
             return (frontier, frontier.numel(), col_ids.numel(), rel_row, rel_col, self.coo_.e_ids, "coo")
         _fatal("Error in Relabel!")
 
@@ -599,7 +605,7 @@ class Graph:
     def _same_structure_child(self, data):
         ret = Graph(self.is_subgraph_, self.col_ids_, self.row_ids_, self.num_cols_, self.num_rows_)
         ret.csc_, ret.csr_, ret.coo_ = self.csc_, self.csr_, self.coo_
-        ret.num_edges_ = self.num_edges_
+        ret.num_edges_, ret._id_bound = self.num_edges_, self._id_bound
         ret.data_ = data
         ret.val_col_ids_, ret.val_row_ids_ = self.val_col_ids_, self.val_row_ids_
         return ret

@@ -290,13 +290,13 @@ def relabel(mapping_tensors, data_requiring_relabel, ctx=None):
     return ctx.native.relabel(ctx.address, mapping_tensors, data_requiring_relabel)
 
 
-def graph_relabel(col_ids, rows, cols=None, indptr=None, ctx=None):
+def graph_relabel(col_ids, rows, cols=None, indptr=None, ctx=None, id_bound=0):
     """What Graph.Relabel does with a sampled graph (src/graph.cc:785-839) → (unique, relabelled rows, relabelled
     columns | None, copy of indptr | None): the frontier unique(cat(col_ids, rows)), every row id's position in it and,
     for a COO whose edge e lies in column cols[e], the position of col_ids[cols[e]]."""
     ctx = _context_for(col_ids, ctx)
     on_device = indptr is None or indptr.is_cuda
-    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, cols, indptr if on_device else None)
+    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, cols, indptr if on_device else None, True, int(id_bound))
     if out is not None:
         return out if on_device else out[:3] + (indptr.clone(),)
     if cols is None:
@@ -304,6 +304,13 @@ def graph_relabel(col_ids, rows, cols=None, indptr=None, ctx=None):
         return frontier, new_rows, None, indptr.clone() if indptr is not None else None
     frontier, (new_cols, new_rows) = relabel([col_ids, rows], [col_ids[cols], rows], ctx)
     return frontier, new_rows, new_cols, indptr.clone() if indptr is not None else None
+
+
+def graph_unique(col_ids, rows, ctx=None, id_bound=0):
+    """unique(cat(col_ids, rows)) in first-occurrence order; id_bound as in gsb_graph_relabel, a hint."""
+    ctx = _context_for(col_ids, ctx)
+    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, None, None, False, int(id_bound))
+    return out[0] if out is not None else relabel([col_ids, rows], [], ctx)[0]
 
 
 def tensor_unique(node_ids, ctx=None):

@@ -31,7 +31,9 @@ def test_graph_relabel_matches_oracle(ops, oracle, n, spread):
     first, second = ids[:S], ids[S:]
     frontier, (w_rows,) = oracle.unique_relabel([first, second], [second])
     indptr = rng.integers(0, 1 << 40, 77).astype(np.int64)
-    f, rows, cols, copy = ops.graph_relabel(dev(first), dev(second), indptr=dev(indptr))
+    bound = int(ids.max()) + 1 if spread == 3 else 0     # the direct-address table; without a bound the hash table
+    assert np.array_equal(ops.graph_unique(dev(first), dev(second), id_bound=max(1, bound - 1)).cpu().numpy(), frontier)
+    f, rows, cols, copy = ops.graph_relabel(dev(first), dev(second), indptr=dev(indptr), id_bound=bound)
     assert cols is None and np.array_equal(f.cpu().numpy(), frontier)
     assert np.array_equal(rows.cpu().numpy(), w_rows) and np.array_equal(copy.cpu().numpy(), indptr)
     f, (rel,) = ops.relabel([dev(first), dev(second)], [dev(second)])
@@ -39,7 +41,7 @@ def test_graph_relabel_matches_oracle(ops, oracle, n, spread):
     if S > 0:
         at = rng.integers(0, S, n - S).astype(np.int64)
         _, (w_cols,) = oracle.unique_relabel([first, second], [first[at]])
-        f, rows, cols, _ = ops.graph_relabel(dev(first), dev(second), cols=dev(at))
+        f, rows, cols, _ = ops.graph_relabel(dev(first), dev(second), cols=dev(at), id_bound=bound)
         assert np.array_equal(f.cpu().numpy(), frontier)
         assert np.array_equal(rows.cpu().numpy(), w_rows) and np.array_equal(cols.cpu().numpy(), w_cols)
 
@@ -66,6 +68,8 @@ def test_batched_relabel_matches_oracle(ops, oracle, G, mean):
     sp, ep = np.concatenate([[0], np.cumsum(ns)]), np.concatenate([[0], np.cumsum(ne)])
     seeds, edges = rng.integers(0, 3 * mean + 1, sp[-1]), rng.integers(0, 3 * mean + 1, ep[-1])
     f, fp, rel, _ = ops.batch_csr_relabel(dev(seeds), dev(sp), dev(edges), dev(ep))
+    again = ops.batch_csr_relabel(dev(seeds), dev(sp), dev(edges), dev(ep), num_nodes=3 * mean + 1)
+    assert all(torch.equal(a, b) for a, b in zip((f, fp, rel), again))
     f, fp, rel = f.cpu().numpy(), fp.cpu().numpy(), rel.cpu().numpy()
     assert fp[0] == 0 and fp[-1] == len(f) and len(rel) == ep[-1]
     for b in range(G):
@@ -84,5 +88,5 @@ def test_epochs_wrap(ops, oracle):
     want, _ = oracle.unique_relabel([ids], [])
     d = dev(ids)
     for i in range(2100):
-        got = ops.tensor_unique(d)
-    assert np.array_equal(got.cpu().numpy(), want)
+        got, direct = ops.tensor_unique(d), ops.graph_unique(d, d, id_bound=40)
+    assert np.array_equal(got.cpu().numpy(), want) and np.array_equal(direct.cpu().numpy(), want)

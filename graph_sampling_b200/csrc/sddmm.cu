@@ -128,6 +128,77 @@ __global__ void __launch_bounds__(kSddmmThreads) k_sddmm_dot_warp(SddmmParams p)
   }
 }
 
+// The shape of adaptive sampling: one side is the edge's destination, edges come column by column, rows of at most 512
+// floats.  LANES lanes (a warp, or half or a quarter of one for rows of up to 64 or 32 floats) take LANES / 2 or LANES
+// consecutive edges; the destination row stays in their registers for as long as the column lasts, so only source rows are
+// read, AHEAD of them at a time.  What bounds it is HBM with rows in no order; enough rows have to be on their way.  1.2 M edges
+// of 256 floats: a warp per edge with both rows read 305 us (80 registers, a third of the warps resident); four rows ahead
+// and three CTAs per SM 237 us, two rows ahead and five CTAs 196 us (6.3 TB/s), with six CTAs it spills: 239 us.  The products
+// of an edge are added in the same order as in k_sddmm_dot_warp.
+template <int LANES, int QUADS, int AHEAD, int CTAS>
+__global__ void __launch_bounds__(kSddmmThreads, CTAS) k_sddmm_dot_columns(SddmmParams p) {
+  constexpr int CHUNK = LANES > 16 ? 16 : LANES;
+  const int lane = threadIdx.x & (LANES - 1);
+  const unsigned mask = LANES == 32 ? 0xffffffffu : ((1u << (LANES & 31)) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));
+  const bool dst_is_rhs = p.rhs_target == 2;
+  const float* near_rows = dst_is_rhs ? p.rhs : p.lhs;
+  const float* far_rows = dst_is_rhs ? p.lhs : p.rhs;
+  const i64 near_len = dst_is_rhs ? p.rhs_len : p.lhs_len, far_len = dst_is_rhs ? p.lhs_len : p.rhs_len;
+  const int far_target = dst_is_rhs ? p.lhs_target : p.rhs_target;
+  const int n4 = (int)(p.reduce_size >> 2);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const i64 groups = (i64)gridDim.x * (kSddmmThreads / LANES);
+  float4 b[QUADS];
+  i64 held = -1;  // destination whose row is in b
+  for (i64 e0 = ((i64)blockIdx.x * (kSddmmThreads / LANES) + threadIdx.x / LANES) * CHUNK; e0 < p.E; e0 += groups * CHUNK) {
+    const int n = (int)min((i64)CHUNK, p.E - e0);
+    const i64 e = e0 + min(lane, n - 1);
+    const i64 src = __ldg(p.row + e);
+    const i64 dst = p.col ? __ldg(p.col + e) : column_of_edge(p.indptr, p.num_cols, e);
+    const i64 eid = p.e_ids ? __ldg(p.e_ids + e) : e;
+    const i64 far = select_target(far_target, src, eid, dst) * far_len;
+    float mine = 0.f;  // lane u keeps the result of edge e0 + u
+    for (int g = 0; g < n; g += AHEAD) {
+      float4 a[AHEAD][QUADS];
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const float4* r = reinterpret_cast<const float4*>(far_rows + __shfl_sync(mask, far, g + u, LANES));
+#pragma unroll
+        for (int q = 0; q < QUADS; ++q) a[u][q] = q * LANES + lane < n4 ? __ldg(r + q * LANES + lane) : zero;
+      }
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const i64 to = __shfl_sync(mask, dst, g + u, LANES);
+        if (to != held) {  // the same in the edge's lanes
+          held = to;
+          const float4* r = reinterpret_cast<const float4*>(near_rows + held * near_len);
+#pragma unroll
+          for (int q = 0; q < QUADS; ++q) b[q] = q * LANES + lane < n4 ? __ldg(r + q * LANES + lane) : zero;
+        }
+        float acc = 0.f;
+#pragma unroll
+        for (int q = 0; q < QUADS; ++q) {
+          acc = fmaf(a[u][q].x, b[q].x, acc);
+          acc = fmaf(a[u][q].y, b[q].y, acc);
+          acc = fmaf(a[u][q].z, b[q].z, acc);
+          acc = fmaf(a[u][q].w, b[q].w, acc);
+        }
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(mask, acc, o, LANES);
+        if (lane == g + u) mine = acc;
+      }
+    }
+    if (lane < n) p.out[eid] = mine;
+  }
+}
+
+template <int LANES, int QUADS, int AHEAD, int CTAS>
+static void launch_dot_columns(cudaStream_t stream, const SddmmParams& p) {
+  const i64 per_cta = (i64)(kSddmmThreads / LANES) * (LANES > 16 ? 16 : LANES);
+  const int grid = (int)min((i64)kNumSMs * 32, (p.E + per_cta - 1) / per_cta);
+  k_sddmm_dot_columns<LANES, QUADS, AHEAD, CTAS><<<grid, kSddmmThreads, 0, stream>>>(p);
+}
+
 __global__ void __launch_bounds__(kSddmmThreads) k_sddmm_generic(SddmmParams p) {
   const i64 total = p.E * p.out_len;
   for (i64 i = (i64)blockIdx.x * kSddmmThreads + threadIdx.x; i < total; i += (i64)gridDim.x * kSddmmThreads) {
@@ -182,7 +253,15 @@ extern "C" int gsb_sddmm(gsb_ctx* ctx, void* stream_, int op, const int64_t* row
     const bool vec = (reduce_size % 4 == 0) && (lhs_len % 4 == 0) && (rhs_len % 4 == 0) &&
                      (((uintptr_t)lhs | (uintptr_t)rhs) % 16 == 0);
     ScopedKernelTimer timer(ctx, KID_SDDMM_DOT, stream);
-    if (vec) k_sddmm_dot_warp<true><<<grid, kSddmmThreads, 0, stream>>>(p);
+    // one destination side, the other not: the destination row is worth holding (an edge feature on either side has a row
+    // per edge); rows beyond 512 floats would not fit the registers
+    if (vec && (lhs_target == 2) != (rhs_target == 2) && reduce_size <= 512) {
+      if (reduce_size <= 32) launch_dot_columns<8, 1, 4, 5>(stream, p);
+      else if (reduce_size <= 64) launch_dot_columns<16, 1, 4, 5>(stream, p);
+      else if (reduce_size <= 128) launch_dot_columns<32, 1, 4, 5>(stream, p);
+      else if (reduce_size <= 256) launch_dot_columns<32, 2, 2, 5>(stream, p);
+      else launch_dot_columns<32, 4, 2, 3>(stream, p);
+    } else if (vec) k_sddmm_dot_warp<true><<<grid, kSddmmThreads, 0, stream>>>(p);
     else k_sddmm_dot_warp<false><<<grid, kSddmmThreads, 0, stream>>>(p);
   } else {
     const int grid = (int)min((i64)kNumSMs * 16, (E * out_len + kSddmmThreads - 1) / kSddmmThreads);

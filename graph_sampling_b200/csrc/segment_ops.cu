@@ -23,44 +23,54 @@ __device__ __forceinline__ float int_pow(float x, i64 powk) {
   return r;
 }
 
-// Lane `at` of `width` lanes: its share of f(b) + f(b + 1) + ... + f(e - 1), eight elements requested before the first is
-// added.  (One element per iteration had a warp wait out a memory round trip per 32 edges: 1.46 M edges in 2 048 columns
-// took 41 us to normalise, 8 us now.)
-template <class F>
-__device__ __forceinline__ float strided_sum(i64 b, i64 e, int at, int width, F f) {
-  constexpr int kAhead = 8;
-  float acc = 0.f;
-  i64 j = b + at;
-  for (; j + (kAhead - 1) * (i64)width < e; j += kAhead * (i64)width) {
-    float v[kAhead];
-#pragma unroll
-    for (int q = 0; q < kAhead; ++q) v[q] = f(j + q * (i64)width);
-#pragma unroll
-    for (int q = 0; q < kAhead; ++q) acc += v[q];
-  }
-  for (; j < e; j += width) acc += f(j);
-  return acc;
-}
+// One segment by `width` threads, thread `first` of them: loads eight elements before the first is used (with one element per
+// iteration a warp waited out a memory round trip per 32 edges), and keeps them in registers when that is the whole segment,
+// so that a normalisation reads its data once.  1.2 M edges in 2 048 columns: 45 us with a remainder loop of single loads and 80
+// registers a thread (28 % of the warps resident), 12.5 us now.
+constexpr int kSegAhead = 8;
 
-// out[at(j)] = data[at(j)] / total for the same share, eight at a time as well.
-template <class At>
-__device__ __forceinline__ void strided_divide(i64 b, i64 e, int first, int width, const float* __restrict__ data,
-                                               float* __restrict__ out, float total, At at) {
-  constexpr int kAhead = 8;
-  for (i64 j = b + first; j < e; j += kAhead * (i64)width) {
-    i64 p[kAhead];
-    float v[kAhead];
-#pragma unroll
-    for (int q = 0; q < kAhead; ++q)
-      if (j + q * (i64)width < e) p[q] = at(j + q * (i64)width);
-#pragma unroll
-    for (int q = 0; q < kAhead; ++q)
-      if (j + q * (i64)width < e) v[q] = __ldg(data + p[q]);
-#pragma unroll
-    for (int q = 0; q < kAhead; ++q)
-      if (j + q * (i64)width < e) out[p[q]] = v[q] / total;
+template <bool NORMALIZE, bool IDS>
+struct SegmentReader {
+  const i64* e_ids;
+  const float* data;
+  i64 powk;
+  float v[kSegAhead];
+
+  __device__ __forceinline__ float value(i64 j) const {
+    if (NORMALIZE) return __ldg(data + j);
+    return int_pow(data ? __ldg(data + j) : 1.0f, powk);
   }
-}
+  __device__ __forceinline__ void load(i64 b, i64 j, i64 len, int width) {
+    if (IDS) {
+      i64 at[kSegAhead];
+#pragma unroll
+      for (int q = 0; q < kSegAhead; ++q)
+        if (j + q * width < len) at[q] = __ldg(e_ids + b + j + q * width);
+#pragma unroll
+      for (int q = 0; q < kSegAhead; ++q) v[q] = j + q * width < len ? value(at[q]) : 0.f;
+    } else {
+#pragma unroll
+      for (int q = 0; q < kSegAhead; ++q) v[q] = j + q * width < len ? value(b + j + q * width) : 0.f;
+    }
+  }
+  __device__ __forceinline__ float sum(i64 b, i64 len, int first, int width) {
+    float acc = 0.f;
+    for (i64 j = first; j < len; j += kSegAhead * width) {
+      load(b, j, len, width);
+#pragma unroll
+      for (int q = 0; q < kSegAhead; ++q) acc += v[q];
+    }
+    return acc;
+  }
+  __device__ __forceinline__ void divide(i64 b, i64 len, int first, int width, float total, float* __restrict__ out) {
+    for (i64 j = first; j < len; j += kSegAhead * width) {
+      if (len > kSegAhead * width) load(b, j, len, width);  // else they are still in v
+#pragma unroll
+      for (int q = 0; q < kSegAhead; ++q)
+        if (j + q * width < len) out[IDS ? __ldg(e_ids + b + j + q * width) : b + j + q * width] = v[q] / total;
+    }
+  }
+};
 
 // NORMALIZE: out[j] = data[j] / (sum of its segment); otherwise out[s] = sum of data^powk over segment s.  One launch:
 // a CTA takes one segment per step when they are long on average (at least 128 edges: a warp each would leave few warps with
@@ -70,42 +80,49 @@ __device__ __forceinline__ void strided_divide(i64 b, i64 e, int first, int widt
 // warp one after the other.  (One warp per segment spent a step, with two dependent loads, on every empty row: 78 us for
 // the 1 M rows of a slice with 25 000 edges.)  The short form adds in the order the tree would, (v0 + v2) + (v1 + v3), so
 // a segment's sum does not depend on which form took it.  Long segments are left to the whole CTA at the end of the step.
-template <bool NORMALIZE>
-__global__ void __launch_bounds__(kSegThreads) k_segments(const i64* __restrict__ indptr, i64 num_seg,
-                                                          const i64* __restrict__ e_ids, const float* __restrict__ data,
-                                                          i64 powk, float* __restrict__ out) {
+template <bool NORMALIZE, bool IDS>
+__global__ void __launch_bounds__(kSegThreads, IDS ? 3 : 5) k_segments(const i64* __restrict__ indptr, i64 num_seg,
+                                                             const i64* __restrict__ e_ids, const float* __restrict__ data,
+                                                             i64 powk, float* __restrict__ out) {
   __shared__ i64 s_long[kSegThreads];
   __shared__ int s_num_long;
   __shared__ float s_part[kSegWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  auto at = [&](i64 j) { return e_ids ? __ldg(e_ids + j) : j; };
-  auto value = [&](i64 j) {
-    const float x = data ? __ldg(data + at(j)) : 1.0f;
-    return NORMALIZE ? x : int_pow(x, powk);
-  };
+  SegmentReader<NORMALIZE, IDS> reader{e_ids, data, powk};
   auto warp_segment = [&](i64 s, i64 b, i64 e) {
-    float acc = strided_sum(b, e, lane, 32, value);
+    const i64 len = e - b;
+    float acc = reader.sum(b, len, lane, 32);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (NORMALIZE) {
-      strided_divide(b, e, lane, 32, data, out, acc, at);
-    } else if (lane == 0) {
-      out[s] = acc;
-    }
+    if (NORMALIZE) reader.divide(b, len, lane, 32, acc, out);
+    else if (lane == 0) out[s] = acc;
+  };
+  auto cta_segment = [&](i64 s) {
+    const i64 b = __ldg(indptr + s);
+    const i64 len = __ldg(indptr + s + 1) - b;
+    float acc = reader.sum(b, len, threadIdx.x, kSegThreads);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) s_part[warp] = acc;
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int w = 0; w < kSegWarps; ++w) total += s_part[w];
+    if (NORMALIZE) reader.divide(b, len, threadIdx.x, kSegThreads, total, out);
+    else if (threadIdx.x == 0) out[s] = total;
+    __syncthreads();
   };
   const i64 mean = (__ldg(indptr + num_seg) - __ldg(indptr)) / num_seg;
+  if (mean >= 128) {
+    for (i64 s = blockIdx.x; s < num_seg; s += gridDim.x) cta_segment(s);
+    return;
+  }
   const bool sparse = !NORMALIZE && mean < 4;
-  const bool dense = mean >= 128;
-  const i64 per_cta = sparse ? kSegThreads : dense ? 1 : kSegWarps;
+  const i64 per_cta = sparse ? kSegThreads : kSegWarps;
   for (i64 first = (i64)blockIdx.x * per_cta; first < num_seg; first += (i64)gridDim.x * per_cta) {
     if (threadIdx.x == 0) s_num_long = 0;
     __syncthreads();
-    if (dense) {
-      if (threadIdx.x == 0) {
-        s_long[0] = first;
-        s_num_long = 1;
-      }
-    } else if (!sparse) {
+    if (!sparse) {
       const i64 s = first + warp;
       if (s < num_seg) {
         const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
@@ -120,6 +137,7 @@ __global__ void __launch_bounds__(kSegThreads) k_segments(const i64* __restrict_
         e = __ldg(indptr + s + 1);
       }
       const i64 len = e - b;
+      auto value = [&](i64 j) { return reader.value(IDS ? __ldg(e_ids + j) : j); };
       // the loads of a short segment are issued now and used after the warp-wide part, which hides their latency
       const bool is_short = s < num_seg && len <= 4;
       float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
@@ -139,25 +157,7 @@ __global__ void __launch_bounds__(kSegThreads) k_segments(const i64* __restrict_
       if (is_short) out[s] = (v0 + v2) + (v1 + v3);
     }
     __syncthreads();
-    const int num_long = s_num_long;
-    for (int q = 0; q < num_long; ++q) {
-      const i64 s = s_long[q];
-      const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
-      float acc = strided_sum(b, e, threadIdx.x, kSegThreads, value);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) s_part[warp] = acc;
-      __syncthreads();
-      float total = 0.f;
-#pragma unroll
-      for (int w = 0; w < kSegWarps; ++w) total += s_part[w];
-      if (NORMALIZE) {
-        strided_divide(b, e, threadIdx.x, kSegThreads, data, out, total, at);
-      } else if (threadIdx.x == 0) {
-        out[s] = total;
-      }
-      __syncthreads();
-    }
+    for (int q = 0, n = s_num_long; q < n; ++q) cta_segment(s_long[q]);
     __syncthreads();  // s_long / s_num_long are rewritten by the next step
   }
 }
@@ -254,7 +254,8 @@ int gsb_segment_sum_csc(gsb_ctx* ctx, void* stream_, const int64_t* indptr, int6
   cudaStream_t stream = (cudaStream_t)stream_;
   {
     ScopedKernelTimer timer(ctx, KID_SEGMENT, stream);
-    k_segments<false><<<segments_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, powk, out);
+    if (e_ids) k_segments<false, true><<<segments_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, powk, out);
+    else k_segments<false, false><<<segments_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, powk, out);
   }
   GSB_LAUNCH_OK();
   return GSB_OK;
@@ -287,7 +288,8 @@ int gsb_segment_normalize_csc(gsb_ctx* ctx, void* stream_, const int64_t* indptr
   cudaStream_t stream = (cudaStream_t)stream_;
   {
     ScopedKernelTimer timer(ctx, KID_SEGMENT, stream);
-    k_segments<true><<<segments_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, 1, out);
+    if (e_ids) k_segments<true, true><<<segments_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, 1, out);
+    else k_segments<true, false><<<segments_grid(num_seg), kSegThreads, 0, stream>>>(indptr, num_seg, e_ids, data, 1, out);
   }
   GSB_LAUNCH_OK();
   return GSB_OK;

@@ -23,18 +23,17 @@ __device__ __forceinline__ float int_pow(float x, i64 powk) {
   return r;
 }
 
-// One segment by `width` threads, thread `first` of them: loads eight elements before the first is used (with one element per
+// One segment by `width` threads, thread `first` of them: loads kAhead elements before the first is used (with one element per
 // iteration a warp waited out a memory round trip per 32 edges), and keeps them in registers when that is the whole segment,
 // so that a normalisation reads its data once.  1.2 M edges in 2 048 columns: 45 us with a remainder loop of single loads and 80
 // registers a thread (28 % of the warps resident), 12.5 us now.
-constexpr int kSegAhead = 8;
-
 template <bool NORMALIZE, bool IDS>
 struct SegmentReader {
+  static constexpr int kAhead = IDS ? 4 : 8;  // more ids would not fit the registers of five CTAs per SM
   const i64* e_ids;
   const float* data;
   i64 powk;
-  float v[kSegAhead];
+  float v[kAhead];
 
   __device__ __forceinline__ float value(i64 j) const {
     if (NORMALIZE) return __ldg(data + j);
@@ -42,31 +41,35 @@ struct SegmentReader {
   }
   __device__ __forceinline__ void load(i64 b, i64 j, i64 len, int width) {
     if (IDS) {
-      i64 at[kSegAhead];
+      i64 at[kAhead];
 #pragma unroll
-      for (int q = 0; q < kSegAhead; ++q)
+      for (int q = 0; q < kAhead; ++q)
         if (j + q * width < len) at[q] = __ldg(e_ids + b + j + q * width);
 #pragma unroll
-      for (int q = 0; q < kSegAhead; ++q) v[q] = j + q * width < len ? value(at[q]) : 0.f;
+      for (int q = 0; q < kAhead; ++q) v[q] = j + q * width < len ? value(at[q]) : 0.f;
     } else {
 #pragma unroll
-      for (int q = 0; q < kSegAhead; ++q) v[q] = j + q * width < len ? value(b + j + q * width) : 0.f;
+      for (int q = 0; q < kAhead; ++q) v[q] = j + q * width < len ? value(b + j + q * width) : 0.f;
     }
   }
   __device__ __forceinline__ float sum(i64 b, i64 len, int first, int width) {
+    if (len <= width) {  // most of a warp's segments
+      v[0] = first < len ? value(IDS ? __ldg(e_ids + b + first) : b + first) : 0.f;
+      return v[0];
+    }
     float acc = 0.f;
-    for (i64 j = first; j < len; j += kSegAhead * width) {
+    for (i64 j = first; j < len; j += kAhead * width) {
       load(b, j, len, width);
 #pragma unroll
-      for (int q = 0; q < kSegAhead; ++q) acc += v[q];
+      for (int q = 0; q < kAhead; ++q) acc += v[q];
     }
     return acc;
   }
   __device__ __forceinline__ void divide(i64 b, i64 len, int first, int width, float total, float* __restrict__ out) {
-    for (i64 j = first; j < len; j += kSegAhead * width) {
-      if (len > kSegAhead * width) load(b, j, len, width);  // else they are still in v
+    for (i64 j = first; j < len; j += kAhead * width) {
+      if (len > kAhead * width) load(b, j, len, width);  // else they are still in v
 #pragma unroll
-      for (int q = 0; q < kSegAhead; ++q)
+      for (int q = 0; q < kAhead; ++q)
         if (j + q * width < len) out[IDS ? __ldg(e_ids + b + j + q * width) : b + j + q * width] = v[q] / total;
     }
   }
@@ -81,7 +84,7 @@ struct SegmentReader {
 // the 1 M rows of a slice with 25 000 edges.)  The short form adds in the order the tree would, (v0 + v2) + (v1 + v3), so
 // a segment's sum does not depend on which form took it.  Long segments are left to the whole CTA at the end of the step.
 template <bool NORMALIZE, bool IDS>
-__global__ void __launch_bounds__(kSegThreads, IDS ? 3 : 5) k_segments(const i64* __restrict__ indptr, i64 num_seg,
+__global__ void __launch_bounds__(kSegThreads, 5) k_segments(const i64* __restrict__ indptr, i64 num_seg,
                                                              const i64* __restrict__ e_ids, const float* __restrict__ data,
                                                              i64 powk, float* __restrict__ out) {
   __shared__ i64 s_long[kSegThreads];

@@ -19,16 +19,18 @@
 //             does not matter, the table keeps the smallest position per id;
 //   resolve   one CTA per bucket: the bucket's items stay in registers; position-min insert into a shared-memory
 //             table (48 KB: ids and smallest positions as two 32-bit arrays, three slots per item where that fits, two
-//             otherwise), then every item reads the first position of its id from the slot it ended in and
-//             writes it to ref[item] — the only scattered accesses to global memory of the whole sequence, 4 bytes
-//             per item into the minibatch's own window; a bucket with more items than the shared-memory table is sized
+//             otherwise), then every item reads the first position of its id from the slot it ended in; they are
+//             written in the bucket's order; a bucket with more items than the shared-memory table is sized
 //             for (many repeats of a few hub ids, or an unlucky hash) uses a table in global memory of its own
 //             instead, so nothing depends on luck;
-//   rank      bit vector of the first occurrences (ref[item] == own position), prefix counts per 32 items, then one
+//   rank      the first positions brought back into the order of the items, which the scatter pass told where they went (a
+//             tile's share of a bucket is a run, so a CTA that takes the same tile reads whole sectors); bit vector of
+//             the first occurrences (ref[item] == own position), prefix counts per 32 items, then one
 //             pass that writes the frontier and every neighbour's position in it (see "ranking by bit vectors").
 //
-// Every pass over the items is coalesced except the 4-byte scatter of `ref` and the 8-byte rank look-ups, both inside
-// the minibatch's own window.  All of these kernels are bound by instruction issue, not by memory, so their common
+// Every pass over the items is coalesced except the 8-byte rank look-ups inside the minibatch's own window.  (While resolve
+// wrote ref[item] itself, a sector per item, that scatter was two thirds of its time: 8.3 ms for 320 M items of 500 large
+// minibatches, now 2.8 with 0.9 more in the first ranking pass and 0.2 in the scatter pass.)  All of these kernels are bound by instruction issue, not by memory, so their common
 // case — a tile or warp whose items lie in ONE minibatch — runs on 32-bit positions with the minibatch's parameters
 // in registers; a tile that straddles minibatches takes a general path per item (the counting pass handles the part
 // of each minibatch in turn when they are few; doing the same in the scatter pass was measured: 64 instead of 46
@@ -60,10 +62,9 @@ struct PartLayout {
   u32* bucket_count;   // [buckets + 1]
   u32* bucket_start;   // [buckets + 1]
   u32* bucket_cursor;  // [buckets]
-  u32* bucket_item0;   // [buckets]  first item of the bucket's minibatch (what its positions count from); written by
-                       //            the counting pass for every bucket that holds an item
   u64* bucketed;       // [items]   id << 32 | position inside the minibatch, grouped by bucket
-  u32* ref;            // [items]   position inside the minibatch of the first occurrence of the item's id
+  u32* found;          // [items]   in the same order: position inside the minibatch of the first occurrence of the id
+  u32* ref;            // [items]   by item: where it lies in `bucketed`; from k_first_bits on what `found` says there
   u64* spill;          // tables of the buckets that do not fit shared memory: 2 x start + 32 x bucket
 };
 
@@ -155,7 +156,6 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
       const Located it = locate(L, g);
       if (!valid_id(it.node)) continue;  // never bucketed; reported by the scatter pass
       atomicAdd(P.bucket_count + it.bucket, 1u);
-      P.bucket_item0[it.bucket] = (u32)(g - it.lc);
     }
     return;
   }
@@ -172,7 +172,6 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
         if (!valid_id(node)) continue;
         const u32 k = t.bucket0 + bucket_of_id((u32)node, t.parts);
         atomicAdd(P.bucket_count + k, 1u);
-        P.bucket_item0[k] = (u32)u.begin;
       }
       continue;
     }
@@ -191,10 +190,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
       if (valid_id(node[q])) atomicAdd(&s_cnt[bucket_of_id((u32)node[q], t.parts)], 1u);  // the others: scatter pass
     __syncthreads();
     for (u32 i = threadIdx.x; i < t.parts; i += kPartThreads) {
-      if (s_cnt[i] != 0) {
-        atomicAdd(P.bucket_count + t.bucket0 + i, s_cnt[i]);
-        P.bucket_item0[t.bucket0 + i] = (u32)u.begin;  // every tile of the minibatch writes the same value
-      }
+      if (s_cnt[i] != 0) atomicAdd(P.bucket_count + t.bucket0 + i, s_cnt[i]);
     }
   }
 }
@@ -262,8 +258,6 @@ __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const
     const i64 ip = sub_indptr[max((i64)0, min(sp, S))];
     indices_ptr[b] = ip;
     L.item_off[b] = sp + ip;
-    if (b < G && !s_abort)
-      for (i64 k = L.region_off[b]; k < L.region_off[b + 1]; ++k) P.bucket_item0[k] = (u32)(sp + ip);
   }
   if (s_abort) return;
   const i64 buckets = L.region_off[G];
@@ -328,8 +322,9 @@ __global__ void __launch_bounds__(THREADS) k_part_scatter(PartLayout P, i64 n_bo
         P.ref[tile_base + i] = 0xFFFFFFFFu;
         continue;
       }
-      P.bucketed[__ldg(P.bucket_start + it.bucket) + atomicAdd(P.bucket_cursor + it.bucket, 1u)] =
-          ((u64)it.node << 32) | (u64)it.lc;
+      const u32 at = __ldg(P.bucket_start + it.bucket) + atomicAdd(P.bucket_cursor + it.bucket, 1u);
+      P.bucketed[at] = ((u64)it.node << 32) | (u64)it.lc;
+      P.ref[tile_base + i] = at;
     }
     return;
   }
@@ -390,7 +385,9 @@ __global__ void __launch_bounds__(THREADS) k_part_scatter(PartLayout P, i64 n_bo
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
     if (where[q] == kNoBucket) continue;
-    s_stage[s_cnt[where[q] >> 16] + (where[q] & 0xFFFFu)] = ((u64)id[q] << 32) | (u64)(lc0 + q * THREADS + threadIdx.x);
+    const u32 i = q * THREADS + threadIdx.x, staged_at = s_cnt[where[q] >> 16] + (where[q] & 0xFFFFu);
+    s_stage[staged_at] = ((u64)id[q] << 32) | (u64)(lc0 + i);
+    P.ref[tile_base + i] = s_delta[where[q] >> 16] + staged_at;
   }
   __syncthreads();
   for (u32 i = threadIdx.x; i < staged; i += THREADS) {
@@ -421,10 +418,8 @@ __device__ __forceinline__ u32 table_insert_min(u64* table, u32 size, u32 h, u64
 
 // Shared-memory table as two 32-bit arrays, ids and smallest positions: the probe loop is a 32-bit load and two compares per
 // step, and both atomics are native 32-bit shared-memory operations.
-// What the kernel waits for (162 M items in 2.29 ms): half of it is the 4-byte scatter of `ref`, one L2 sector per item
-// (1.18 ms with the same words written in bucket order); probing costs a tenth and the position minimum nothing that can be
-// measured.  All twelve items of a thread probing side by side with a compare-and-swap per round was slower (3.8 against
-// 2.4 ms per launch): without the read in front of it every repeat of a frequent id is an atomic on the same word.
+// Probing costs a tenth of the kernel and the position minimum nothing that can be measured.  All twelve items of a thread probing side by side with a compare-and-swap per round was slower (3.8 against
+// 2.4 ms per launch of an earlier form): without the read in front of it every repeat of a frequent id is an atomic on the same word.
 // Measured and not kept: five CTAs per SM instead of four (40 KB tables of 2.5 slots per item, 48 registers): 2.61
 // against 2.62 ms per 1 000 minibatches — the kernel is not short of resident warps.
 __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout P, i64* counters) {
@@ -437,7 +432,7 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
     const u32 start = P.bucket_start[k];
     const u32 n = P.bucket_start[k + 1] - start;
     if (n == 0) continue;
-    u32* ref = P.ref + P.bucket_item0[k];
+    u32* found = P.found + start;
     const u64* items = P.bucketed + start;
     if (n <= (u32)kBucketSmemItems) {
       // three slots per item where the table allows it: the lanes of a warp leave the probe loop together more often
@@ -462,21 +457,21 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
 #pragma unroll
       for (int q0 = 0; q0 < kResolvePer; q0 += kResolveAhead) {
         if ((u32)(q0 * kResolveThreads) >= n) break;  // uniform
-        u32 found[kResolveAhead];
+        u32 seen[kResolveAhead];
 #pragma unroll
         for (int q = 0; q < kResolveAhead; ++q) {
           slot[q0 + q] = slot_of_id((u32)(w[q0 + q] >> 32), size);
-          found[q] = *(volatile u32*)(keys + slot[q0 + q]);
+          seen[q] = *(volatile u32*)(keys + slot[q0 + q]);
         }
 #pragma unroll
         for (int q = 0; q < kResolveAhead; ++q)
-          if (found[q] == 0xFFFFFFFFu && w[q0 + q] != kEmptyWord)
-            found[q] = atomicCAS(keys + slot[q0 + q], 0xFFFFFFFFu, (u32)(w[q0 + q] >> 32));  // ids are below 2^32 - 1
+          if (seen[q] == 0xFFFFFFFFu && w[q0 + q] != kEmptyWord)
+            seen[q] = atomicCAS(keys + slot[q0 + q], 0xFFFFFFFFu, (u32)(w[q0 + q] >> 32));  // ids are below 2^32 - 1
 #pragma unroll
         for (int q = 0; q < kResolveAhead; ++q) {
           if (w[q0 + q] == kEmptyWord) continue;
           const u32 id = (u32)(w[q0 + q] >> 32);
-          u32 k = found[q], h = slot[q0 + q];
+          u32 k = seen[q], h = slot[q0 + q];
           while (k != 0xFFFFFFFFu && k != id) {  // ends: the table has more slots than the bucket has items
             h = h + 1 == size ? 0 : h + 1;
             k = *(volatile u32*)(keys + h);
@@ -493,7 +488,7 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
         if ((u32)(q * kResolveThreads) < n) ref_of[q] = first[slot[q]];
 #pragma unroll
       for (int q = 0; q < kResolvePer; ++q)
-        if ((u32)(q * kResolveThreads) < n && w[q] != kEmptyWord) ref[(u32)w[q]] = ref_of[q];
+        if ((u32)(q * kResolveThreads) < n && w[q] != kEmptyWord) found[q * kResolveThreads + threadIdx.x] = ref_of[q];
       continue;
     }
     // oversized bucket (many repeats of a few ids): a table of its own in global memory
@@ -520,13 +515,13 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
         if (x == kEmptyWord) break;
         h = h + 1 == size ? 0 : h + 1;
       }
-      ref[(u32)w] = first;
+      found[j] = first;
     }
   }
 }
 
 // ---- ranking by bit vectors -----------------------------------------------------------------------------------------
-// An item is a first occurrence iff ref[item] is its own position.  k_first_bits leaves one bit per item (a 32-bit word
+// An item is a first occurrence iff ref[item] is its own position.  k_first_bits fills ref in and leaves one bit per item (a 32-bit word
 // per 32 consecutive items of the call); k_rank_prefix scans the words' population counts (single pass, look-back over
 // tiles of 2 048 words = 65 536 items, so the chain is a few hundred tiles at most) and packs, per word,
 // [ number of first occurrences before the word : 32 | bits : 32 ].  The frontier rank of ANY item p is then
@@ -536,7 +531,6 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
 // over a rank array.  None of the three kernels waits for anything but the short chain of k_rank_prefix.
 constexpr int kBitsThreads = 256;
 constexpr int kBitsGroups = 8;                                     // 32-item groups per warp
-constexpr int kBitsTile = (kBitsThreads / 32) * kBitsGroups * 32;  // items per CTA
 constexpr int kEmitGroups = 4;
 constexpr int kEmitTile = (kBitsThreads / 32) * kEmitGroups * 32;
 constexpr int kPrefixThreads = 256;
@@ -544,24 +538,33 @@ constexpr int kPrefixPer = 8;
 constexpr int kPrefixTile = kPrefixThreads * kPrefixPer;  // words per CTA
 
 struct RankArrays {
-  const u32* ref;
+  const u32* found;
+  u32* ref;
   u32* bits;    // [ceil(items / 32)]
   u64* packed;  // [ceil(items / 32) + 1]
 };
 
-__global__ void __launch_bounds__(kBitsThreads) k_first_bits(BatchLayout L, RankArrays R, i64 n_bound, i64* counters) {
+__global__ void __launch_bounds__(1024) k_first_bits(BatchLayout L, RankArrays R, i64 n_bound, i64* counters) {
   if (counters[CNT_ABORT] != 0) return;
   const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const i64 n = min(L.item_off[L.G], n_bound);
-  const i64 base = (i64)blockIdx.x * kBitsTile + (i64)warp * (kBitsGroups * 32);
+  const i64 base = (i64)blockIdx.x * (blockDim.x * kBitsGroups) + (i64)warp * (kBitsGroups * 32);
   if (base >= n) return;
   const u32 here = (u32)min((i64)(kBitsGroups * 32), n - base);  // items of this warp
-  const u32* ref = R.ref + base;
+  u32* ref = R.ref + base;
   u32 r[kBitsGroups];
 #pragma unroll
   for (int q = 0; q < kBitsGroups; ++q) {
     const u32 i = q * 32 + lane;
-    r[q] = i < here ? __ldg(ref + i) : 0xFFFFFFFFu;
+    r[q] = i < here ? ref[i] : 0xFFFFFFFFu;  // an id that was never bucketed is marked so, too
+  }
+#pragma unroll
+  for (int q = 0; q < kBitsGroups; ++q)
+    if (r[q] != 0xFFFFFFFFu) r[q] = __ldg(R.found + r[q]);
+#pragma unroll
+  for (int q = 0; q < kBitsGroups; ++q) {
+    const u32 i = q * 32 + lane;
+    if (i < here) ref[i] = r[q];
   }
   const i64 b = batch_of_warp(L.item_off, L.G, base);
   const i64 begin = __ldg(L.item_off + b), next_begin = __ldg(L.item_off + b + 1);
@@ -727,7 +730,7 @@ i64 partition_bucket_capacity(i64 items_bound, i64 G) { return items_bound / kBu
 
 size_t partition_workspace_bytes(i64 n_cap, i64 bucket_cap) {
   const size_t words = (size_t)((n_cap + 31) / 32) + 2;
-  return al256(sizeof(u32) * 4 * (size_t)(bucket_cap + 1)) + al256(8 * (size_t)n_cap) + al256(4 * (size_t)n_cap) +
+  return al256(sizeof(u32) * 3 * (size_t)(bucket_cap + 1)) + al256(8 * (size_t)n_cap) + 2 * al256(4 * (size_t)n_cap) +
          al256(4 * words) + al256(8 * words) + al256(8 * (2 * (size_t)n_cap + 32 * (size_t)bucket_cap + 64));
 }
 
@@ -747,12 +750,14 @@ static PartArrays carve(const BatchLayout& L, i64 n_cap, i64 bucket_cap, void* w
   P.bucket_count = (u32*)at;
   P.bucket_start = P.bucket_count + (bucket_cap + 1);
   P.bucket_cursor = P.bucket_count + 2 * (bucket_cap + 1);
-  P.bucket_item0 = P.bucket_count + 3 * (bucket_cap + 1);
-  at += al256(sizeof(u32) * 4 * (size_t)(bucket_cap + 1));
+  at += al256(sizeof(u32) * 3 * (size_t)(bucket_cap + 1));
   P.bucketed = (u64*)at;
   at += al256(8 * (size_t)n_cap);
+  P.found = (u32*)at;
+  at += al256(4 * (size_t)n_cap);
   P.ref = (u32*)at;
   at += al256(4 * (size_t)n_cap);
+  a.R.found = P.found;
   a.R.ref = P.ref;
   a.R.bits = (u32*)at;
   at += al256(4 * words);
@@ -819,7 +824,9 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   GSB_LAUNCH_OK();
   {
     ScopedKernelTimer timer(ctx, KID_FIRST_BITS, stream);
-    k_first_bits<<<grid_for(n_cap, kBitsTile), kBitsThreads, 0, stream>>>(L, R, n_cap, counters);
+    // a CTA takes the tile that the scatter pass took
+    const int threads = wide ? 1024 : 256;
+    k_first_bits<<<grid_for(n_cap, threads * kBitsGroups), threads, 0, stream>>>(L, R, n_cap, counters);
   }
   GSB_LAUNCH_OK();
   const int prefix_tiles = grid_for((n_cap + 31) / 32, kPrefixTile);

@@ -13,7 +13,7 @@
 //             bucket sizes (one global atomic per CTA and bucket).  In the one-call hop (gsb_sage_hop) the uniform
 //             sampler does this counting itself while it holds the ids (slice_sample.cu, COUNT) — the buckets are then
 //             laid out from the bound seeds x (1 + fanout) before it runs — and this pass is not launched;
-//   scan      bucket sizes -> bucket starts (one CTA; in the one-call hop part of k_part_after_sampler);
+//   scan      bucket sizes -> bucket starts (single pass; in the one-call hop part of k_part_after_sampler);
 //   scatter   tiles of 2 048 or 8 192 items: sorted by bucket in shared memory, a range reserved per bucket with one global
 //             atomic, whole runs of (id << 32 | position inside the minibatch) copied out — the order inside a bucket
 //             does not matter, the table keeps the smallest position per id;
@@ -195,39 +195,44 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
   }
 }
 
-// bucket sizes -> bucket starts, cursors cleared (one CTA of 1 024 threads, 8 buckets per thread and round)
-__global__ void __launch_bounds__(1024) k_part_scan(PartLayout P, i64* counters) {
+// bucket sizes -> bucket starts, cursors cleared: single pass with look-back over tiles of 2 048 buckets (one CTA that walked
+// all buckets took 250 us for the 130 000 of 500 large minibatches)
+constexpr int kScanThreads = 256;
+constexpr int kScanPer = 8;
+constexpr int kScanTile = kScanThreads * kScanPer;
+
+__global__ void __launch_bounds__(kScanThreads) k_part_scan(PartLayout P, i64* counters, TileState ts) {
   __shared__ i64 s_scan[33];
-  __shared__ i64 s_carry;
+  __shared__ i64 s_base;
   if (counters[CNT_ABORT] != 0) return;
   const i64 buckets = P.L.region_off[P.L.G];
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  constexpr int kPer = 8;
-  for (i64 base = 0; base < buckets; base += 1024 * kPer) {
-    const i64 first = base + (i64)threadIdx.x * kPer;
-    u32 c[kPer];
-    i64 sum = 0;
+  const int tile = blockIdx.x;
+  const i64 first = (i64)tile * kScanTile + (i64)threadIdx.x * kScanPer;
+  if ((i64)tile * kScanTile >= buckets && !(buckets == 0 && tile == 0)) return;
+  u32 c[kScanPer];
+  i64 sum = 0;
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      c[j] = first + j < buckets ? P.bucket_count[first + j] : 0u;
-      sum += c[j];
-    }
-    i64 total;
-    i64 run = s_carry + block_exclusive_scan<1024>(sum, s_scan, &total);
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      if (first + j < buckets) {
-        P.bucket_start[first + j] = (u32)run;
-        P.bucket_cursor[first + j] = 0u;
-      }
-      run += c[j];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) s_carry += total;
-    __syncthreads();
+  for (int j = 0; j < kScanPer; ++j) {
+    c[j] = first + j < buckets ? P.bucket_count[first + j] : 0u;
+    sum += c[j];
   }
-  if (threadIdx.x == 0) P.bucket_start[buckets] = (u32)s_carry;
+  i64 total;
+  const i64 excl = block_exclusive_scan<kScanThreads>(sum, s_scan, &total);
+  if (threadIdx.x < 32) {
+    const i64 prefix = tile_exclusive_prefix(ts, tile, total);
+    if (threadIdx.x == 0) s_base = prefix;
+  }
+  __syncthreads();
+  i64 run = s_base + excl;
+#pragma unroll
+  for (int j = 0; j < kScanPer; ++j) {
+    if (first + j < buckets) {
+      P.bucket_start[first + j] = (u32)run;
+      P.bucket_cursor[first + j] = 0u;
+    }
+    run += c[j];
+  }
+  if ((i64)(tile + 1) * kScanTile >= buckets && threadIdx.x == 0) P.bucket_start[buckets] = (u32)(s_base + total);
 }
 
 // The one-call hop, between its sampler and the scatter pass — one CTA does what three small launches did: the edge
@@ -294,9 +299,11 @@ __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const
 // THREADS x PER items per tile.  Tiles of 2 048 suit minibatches of some ten thousand items (a tile that straddles
 // minibatches takes the per-item path); with hundreds of buckets per minibatch such a tile reserves a range — a global
 // atomic, on a cursor that every other tile of the minibatch wants too — for every five items, so large minibatches take
-// tiles of 8 192.
+// tiles of 8 192, two of whose CTAs are resident per SM (with the 83 registers the compiler takes of its own accord one is, and
+// its barriers leave the SM idle: 3.1 against 2.1 ms for 270 M items; 1 024 threads with half the items each 2.8, tiles of
+// 4 096 2.7).
 template <int WINDOW, int THREADS, int PER>
-__global__ void __launch_bounds__(THREADS) k_part_scatter(PartLayout P, i64 n_bound, i64* counters) {
+__global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatter(PartLayout P, i64 n_bound, i64* counters) {
   constexpr int kTile = THREADS * PER;
   constexpr int kPer = WINDOW / THREADS > 0 ? WINDOW / THREADS : 1;  // consecutive window entries per thread in the scan
   extern __shared__ __align__(16) u64 s_stage[];                     // [kTile] items, then [WINDOW] two arrays
@@ -801,9 +808,13 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
       else k_part_count<kNarrowWindow><<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
     }
     GSB_LAUNCH_OK();
+    const int scan_tiles = grid_for(bucket_cap, kScanTile);
+    TileState scan_ts;
+    const int st = ctx_tile_state(ctx, scan_tiles, stream, &scan_ts);
+    if (st != GSB_OK) return st;
     {
       ScopedKernelTimer timer(ctx, KID_OTHER, stream);
-      k_part_scan<<<1, 1024, 0, stream>>>(P, counters);
+      k_part_scan<<<scan_tiles, kScanThreads, 0, stream>>>(P, counters, scan_ts);
     }
     GSB_LAUNCH_OK();
   }

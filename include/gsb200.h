@@ -80,7 +80,8 @@ GSB_API int gsb_check_device_status(gsb_ctx* ctx, void* stream);
  *                               to a power of two) instead of sizing it from the item count — a table that is too
  *                               small reports GSB_ERR_TABLE_FULL; 0 (default) = automatic;
  *  GSB_OPT_RELABEL_PATH         how gsb_sage_hop / gsb_batch_unique_relabel find first occurrences: 0 (default) =
- *                               one cooperative launch for calls it suits (up to 2^21 items), else
+ *                               one cooperative launch for calls it suits (up to 2^21 items, half of that
+ *                               in several minibatches), else
  *                               direct-address tables when all tables of the call are L2-sized (32 MiB), else the
  *                               partitioned form (items bucketed by a hash of their id, one shared-memory table per
  *                               bucket) for calls of at least 2^19 items whose minibatches average at most 2^19

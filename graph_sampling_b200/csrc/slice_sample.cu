@@ -11,6 +11,7 @@
 // whatever its degree (Floyd's k-subset), instead of the reference's O(degree) reservoir pass
 // (src/cuda/fusion/slice_sampling.cu:62-75).
 #include "batch_table.cuh"
+#include "column_walk.cuh"
 #include "common.cuh"
 #include "philox.cuh"
 #include "scan.cuh"
@@ -110,129 +111,77 @@ struct FillParams {
   i64 encoding_size;
   i64 D;  // edge total, or -1: it is read on the device
 };
-constexpr i64 kFillNoColumn = (i64)1 << 62;
 
-// The OUTPUT positions are cut into tiles, whatever columns they belong to, and a CTA copies a tile at a time: a hub column
-// is spread over the grid, and a call with few, long columns fills it as well as one with many short ones.
-//   1. the tile's first and last column, by two warp-wide searches of the offsets (32 pivots a round);
-//   2. the offsets of the tile's columns and what to add to an output position to get the input position, a column per
-//      thread, into shared memory (the two dependent reads seeds -> indptr are made once per column and tile);
-//   3. a warp copies 256 consecutive positions: one binary search in shared memory per lane for the first of its eight, then
-//      the column only walks forward; all reads are requested before anything is written.
-// What bounds it is the chain search -> offsets -> ids against the positions in flight per SM, so registers are spent on
-// resident CTAs: a position keeps the number of its column in the window and nothing else until its id has arrived.
-// 262 144 columns with 13.2 M edges, weights and column ids, whole call: column tiles (a CTA per 128 columns) 177 us; output
-// tiles with the input positions in registers 155 us; this form with 256 threads and 4 / 5 / 6 CTAs per SM 137 / 133 / 153
-// us, with 128 threads and 10 / 12 CTAs 130 / 150 us (fewer registers spill).  Tiles of 256 positions per warp, without any
-// CTA barrier: 167 us, the search is then paid four times as often.
+// The OUTPUT positions are cut into one stretch per warp, whatever columns they belong to: a hub column is spread over the
+// grid, and a call with few, long columns fills it as well as one with many short ones.  A warp finds the columns of 192
+// positions at a time (column_walk.cuh) and requests all their ids and data before it writes any.
+// What bounds it is HBM and the positions in flight per SM, and anything spilled costs more than the resident warps it buys:
+// 262 144 columns with 13.2 M edges, weights and column ids: 92 us with six positions per lane and 8 CTAs per SM; eight
+// positions and 8 / 7 / 9 / 10 CTAs 94 / 99 / 142 / 147, four and 10 CTAs 132.  Tiles of 1 024 positions whose columns a CTA
+// keeps in shared memory, two barriers and two searches each: 105 us, and 16 instead of 5 us for the slices of layer-wise
+// sampling, whose columns are mostly empty.
 constexpr int kFillThreads = 128;
-constexpr int kFillPer = 8;
-constexpr int kFillTile = kFillThreads * kFillPer;
-constexpr int kFillWindow = 512;  // columns of a tile held in shared memory at a time
+constexpr int kFillCtas = 8;
+constexpr int kFillPer = 6;
+constexpr int kFillStretch = 1024;
 
-// Largest c with off[c] <= pos, by a whole warp.  Needs off[0] <= pos < off[S].
-__device__ __forceinline__ i64 fill_warp_column_at(const i64* __restrict__ off, i64 S, i64 pos) {
+template <bool ENCODE, bool EIDS>
+__global__ void __launch_bounds__(kFillThreads, kFillCtas) k_slice_fill(FillParams p) {
   const int lane = threadIdx.x & 31;
-  i64 lo = 0, hi = S;
-  while (hi - lo > 1) {
-    const i64 step = (hi - lo + 31) / 32;
-    const i64 idx = lo + (i64)(lane + 1) * step;
-    const bool le = idx < hi && __ldg(off + idx) <= pos;  // true for a prefix of the lanes
-    const int n = __popc(__ballot_sync(0xffffffffu, le));
-    const i64 new_hi = min(hi, lo + (i64)(n + 1) * step);
-    lo += (i64)n * step;
-    hi = new_hi;
-  }
-  return lo;
-}
-
-template <bool ENCODE>
-__global__ void __launch_bounds__(kFillThreads, 10) k_slice_fill(FillParams p) {
-  __shared__ i64 s_range[2];
-  __shared__ i64 s_delta[kFillWindow];    // input position of an edge = its output position + this
-  __shared__ int s_off[kFillWindow + 1];  // first output position of a column, relative to the tile
-  __shared__ i64 s_enc[ENCODE ? kFillWindow : 1];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const i64 D = p.D >= 0 ? p.D : __ldg(p.out_indptr + p.S);
-  for (i64 tile = (i64)blockIdx.x * kFillTile; tile < D; tile += (i64)gridDim.x * kFillTile) {
-    const int here = (int)min((i64)kFillTile, D - tile);
-    if (warp < 2) {
-      const i64 c = fill_warp_column_at(p.out_indptr, p.S, warp == 0 ? tile : tile + here - 1);
-      if (lane == 0) s_range[warp] = c;
+  const i64 warps = (i64)gridDim.x * (kFillThreads / 32);
+  const i64 per = ((D + warps - 1) / warps + 31) / 32 * 32;
+  const i64 begin = ((i64)blockIdx.x * (kFillThreads / 32) + (threadIdx.x >> 5)) * per;
+  if (begin >= D) return;
+  ColumnWalk walk;
+  walk.off = p.out_indptr;
+  walk.seeds = p.seeds;
+  walk.indptr = p.indptr;
+  walk.S = p.S;
+  walk.num_cols = p.num_cols;
+  walk.counters = nullptr;  // the counting pass reported bad seeds; they have no positions
+  walk.init(begin, (int)min(per, D - begin));
+  for (int at = 0; at < walk.len; at += 32 * kFillPer) {
+    i64 val[kFillPer];
+    float x[kFillPer];
+    i64 add[ENCODE ? kFillPer : 1];
+    unsigned valid = 0;
+#pragma unroll
+    for (int r = 0; r < kFillPer; ++r) {
+      if (at + r * 32 >= walk.len) break;  // uniform
+      i64 column = 0;
+      const i64 in = walk.locate<true>(at + r * 32, &column);
+      if (in < 0) continue;
+      valid |= 1u << r;
+      const i64 pos = begin + at + r * 32 + lane;
+      val[r] = __ldg(p.indices + in);
+      if (EIDS) x[r] = __ldg(p.data + __ldg(p.e_ids + in));
+      else if (p.out_data) x[r] = __ldg(p.data + in);
+      if (p.out_select) p.out_select[pos] = in;
+      if (p.out_coo_col) p.out_coo_col[pos] = column;
+      if (ENCODE) add[r] = batch_of(p.nid_ptr, p.G, column) * p.encoding_size;
     }
-    __syncthreads();
-    const i64 c_end = s_range[1] + 1;
-    // one window of columns, unless the tile meets more of them (runs of empty ones)
-    for (i64 c0 = s_range[0]; c0 < c_end; c0 += kFillWindow) {
-      const int cols = (int)min((i64)kFillWindow, c_end - c0);
-      for (int j = tid; j <= cols; j += kFillThreads) {
-        const i64 o = __ldg(p.out_indptr + c0 + j);
-        s_off[j] = (int)max((i64)0, min(o - tile, (i64)here));
-        if (j < cols) {
-          const i64 col = p.seeds ? __ldg(p.seeds + c0 + j) : c0 + j;
-          // a bad id has no output positions unless the offsets were not counted for these seeds: then nothing is read
-          s_delta[j] = (u64)col < (u64)p.num_cols ? __ldg(p.indptr + col) - o + tile : kFillNoColumn;
-          if (ENCODE) s_enc[j] = batch_of(p.nid_ptr, p.G, c0 + j) * p.encoding_size;
-        }
-      }
-      __syncthreads();
-      const int begin = s_off[0], end = s_off[cols];  // the tile's positions that the window covers
-      const int base = warp * (32 * kFillPer) + lane;
-      int c = 0;
-      {
-        const int q = max(base, begin);
-        int hi = cols;
-        while (hi - c > 1) {
-          const int mid = (c + hi) >> 1;
-          if (s_off[mid] <= q) c = mid;
-          else hi = mid;
-        }
-      }
-      int col[kFillPer];
 #pragma unroll
-      for (int r = 0; r < kFillPer; ++r) {
-        const int q = base + r * 32;
-        col[r] = -1;
-        if (q < begin || q >= end) continue;
-        while (s_off[c + 1] <= q) ++c;  // empty columns are stepped over; q < end = s_off[cols] bounds the walk
-        if (s_delta[c] != kFillNoColumn) col[r] = c;
-      }
-      i64 val[kFillPer];
-#pragma unroll
-      for (int r = 0; r < kFillPer; ++r)
-        if (col[r] >= 0) val[r] = __ldg(p.indices + (base + r * 32 + s_delta[col[r]]));
-      float x[kFillPer];
-      if (p.out_data) {
-#pragma unroll
-        for (int r = 0; r < kFillPer; ++r)
-          if (col[r] >= 0) {
-            const i64 in = base + r * 32 + s_delta[col[r]];
-            x[r] = __ldg(p.data + (p.e_ids ? __ldg(p.e_ids + in) : in));
-          }
-      }
-#pragma unroll
-      for (int r = 0; r < kFillPer; ++r) {
-        if (col[r] < 0) continue;
-        const i64 pos = tile + base + r * 32;
-        p.out_indices[pos] = val[r] + (ENCODE ? s_enc[col[r]] : 0);
-        if (p.out_select) p.out_select[pos] = base + r * 32 + s_delta[col[r]];
-        if (p.out_coo_col) p.out_coo_col[pos] = c0 + col[r];
-        if (p.out_data) p.out_data[pos] = x[r];
-      }
-      __syncthreads();  // the shared arrays are rewritten by the next pass
+    for (int r = 0; r < kFillPer; ++r) {
+      if (!((valid >> r) & 1u)) continue;
+      const i64 pos = begin + at + r * 32 + lane;
+      p.out_indices[pos] = ENCODE ? val[r] + add[r] : val[r];
+      if (EIDS || p.out_data) p.out_data[pos] = x[r];
     }
   }
 }
 
-// With the edge total known on the host a CTA per tile (the hardware balances them); without it a grid that fills the chip
-// strides over whatever the device finds.
+// A grid that fills the chip; smaller when the edge total is known to be small, as a warp takes 32 positions at least, and
+// larger when it is large, so that the hardware can balance stretches of 1 024 positions (2 048: 102, 512: 99 us for the slice
+// above, where the search for a stretch's first column begins to show).
 template <bool ENCODE>
 static void launch_fill(FillParams p, i64 D, cudaStream_t stream) {
   p.D = D;
-  const int grid = D >= 0 ? min(grid_for(D, kFillTile), 1 << 20) : kNumSMs * 16;
-  k_slice_fill<ENCODE><<<grid, kFillThreads, 0, stream>>>(p);
+  const int full = kNumSMs * kFillCtas;
+  const int grid = D >= 0 ? max(min(grid_for(D, kFillThreads), full), grid_for(D, kFillThreads / 32 * kFillStretch)) : full;
+  if (p.out_data && p.e_ids) k_slice_fill<ENCODE, true><<<grid, kFillThreads, 0, stream>>>(p);
+  else k_slice_fill<ENCODE, false><<<grid, kFillThreads, 0, stream>>>(p);
 }
-
 
 // ---- fused count + scan + uniform sampling -------------------------------------------------------
 struct SampleParams {

@@ -1,5 +1,5 @@
-"""The slice copy at the sizes where it can go wrong: tiles of 1 024 positions that end inside, at and between columns,
-columns much longer and much shorter than a tile, more (empty) columns in a tile than its window holds, every optional
+"""The slice copy at the sizes where it can go wrong: stretches that end inside, at and between columns,
+columns much longer and much shorter than a stretch, more (empty) columns in it than its window holds, every optional
 output, and the batched form with encoded ids — against numpy."""
 import numpy as np
 import pytest
@@ -14,7 +14,7 @@ def dev(a):
 
 SHAPES = {"one": [1], "exact": [1024, 1024], "off_by_one": [1023, 1, 1, 1025], "hub": [0, 50_001, 3], "short": [3] * 5000,
           "empty_runs": [2] + [0] * 3000 + [5] + [0] * 700 + [1, 1, 1], "mixed": [7, 0, 900, 0, 0, 2100, 1, 40] * 60,
-          "all_empty": [0] * 70}
+          "all_empty": [0] * 70, "stretches": [7, 0, 900, 0, 0, 2100, 1, 40] * 700, "many": [3, 0, 0, 4] * 200_000}
 
 
 @pytest.mark.parametrize("shape", sorted(SHAPES))

@@ -42,6 +42,9 @@ struct ColumnWalk {
   int next;   // of the column after the window
   i64 delta;  // input position minus relative position
   i64 off1, ptr1, off2, col2;  // the two windows that follow
+  i64 run_in;   // the column of the last position located: what to add to its positions, its number,
+  int run_end;  // and where it ends
+  int run_column;
 
   __device__ __forceinline__ int relative(i64 o) const { return (int)max((i64)0, min(o - begin, (i64)len)); }
   __device__ __forceinline__ void fetch(i64 c, i64& o, i64& col) const {
@@ -62,6 +65,7 @@ struct ColumnWalk {
     const int lane = threadIdx.x & 31;
     begin = first;
     len = length;
+    run_end = 0;
     c0 = warp_column_search(off, S, begin);
     i64 o, col, col1;
     fetch(c0 + lane, o, col);
@@ -85,6 +89,10 @@ struct ColumnWalk {
   template <bool COLUMN>
   __device__ __forceinline__ i64 locate(int at, i64* column) {
     const int lane = threadIdx.x & 31, q = at + lane, end = min(at + 32, len);
+    if (end <= run_end) {  // inside a long column
+      if (COLUMN) *column = c0 + run_column;
+      return q < end && run_in != kNoWalkColumn ? q + run_in : -1;
+    }
     i64 in = -1;
     for (;;) {
       const int rel = start - at;
@@ -104,7 +112,13 @@ struct ColumnWalk {
         in = q + d;
         if (COLUMN) *column = c0 + c;
       }
-      if (end <= next) return in;
+      if (end <= next) {
+        run_column = __shfl_sync(0xffffffffu, max(c, 0), end - 1 - at);
+        run_in = __shfl_sync(0xffffffffu, d, end - 1 - at);
+        run_end = __shfl_sync(0xffffffffu, start, (run_column + 1) & 31);
+        if (run_column == 31) run_end = next;
+        return in;
+      }
       advance();
     }
   }

@@ -10,6 +10,7 @@
 // torch::nonzero and two or three torch index gathers (src/cuda/slicing.cu:416-526); the COO form
 // (:543-563, 727-771) is the same without offsets.
 #include "batch_table.cuh"
+#include "column_walk.cuh"
 #include "common.cuh"
 #include "grid_sync.cuh"
 #include "hash_table.cuh"
@@ -332,19 +333,18 @@ __global__ void __launch_bounds__(kRowThreads) k_col_row_filter(ColRowParams p) 
 }
 
 // ---- induced subgraph of one node set in one launch -----------------------------------------------------------------
-// The single-batch form of k_col_row_filter as a cooperative kernel: a CTA owns one stretch of the virtual edge list.
-//   filter   tiles of 4 096 positions, columns found as in the slice copy (the tile's columns in shared memory); an edge is
-//            looked up in the table only when the shared-memory filter lets it pass; survivors go to scratch in order, and
-//            every 32 positions leave [survivors of the CTA before them : 32 | bits : 32];
+// The single-batch form of k_col_row_filter as a cooperative kernel: a warp owns one stretch of the virtual edge list.
+//   filter   192 positions at a time, columns found without barriers (column_walk.cuh); an edge is looked up in the table only
+//            when the shared-memory filter lets it pass; survivors go to scratch in order, and every 32 positions leave
+//            [survivors of the warp before them : 32 | bits : 32];
 //   barrier
 //   emit     every CTA scans the CTAs' totals, copies its survivors to their places (and gathers their edge data), and a
 //            share of the columns gets its offset as the rank of the column's first position.
-// 20 000 columns with 6.5 M edges, 20 000 rows: 178 us with a table probe per edge and a look-back chain of 6 400 tiles.
+// 20 000 columns with 6.5 M edges, 20 000 rows: 178 us with a table probe per edge and a look-back chain of 6 400 tiles, 84
+// with a stretch per CTA (six tiles of two searches and four barriers each), 64 with one per warp.
 constexpr int kInThreads = 512;
-constexpr int kInPer = 8;
-constexpr int kInTile = kInThreads * kInPer;
+constexpr int kInPer = 6;
 constexpr int kInWarps = kInThreads / 32;
-constexpr int kInWindow = 512;
 constexpr int kBloomMaxBits = 1 << 19;  // 64 KB: two CTAs per SM
 constexpr i64 kBloomMaxRows = 1 << 18;  // beyond, most edges would pass
 constexpr i64 kInducedMaxEdges = 1 << 27;  // its scratch is 12 bytes per edge
@@ -352,9 +352,10 @@ constexpr i64 kInducedMaxEdges = 1 << 27;  // its scratch is 12 bytes per edge
 struct InducedParams {
   ColRowParams c;
   RowBloom bloom;
-  i64 range;        // positions per CTA, a multiple of kInTile
+  i64 range;        // positions per warp, a multiple of 32
   u64* packed;      // [D / 32 + 1]
   u32* totals;      // [CTAs]
+  u32* warp_before;  // [CTAs][kInWarps] survivors of the CTA's warps before this one
   u32* kept_row;    // [D] position in row_ids
   i64* kept_edge;   // [D]
   GridSync sync;
@@ -362,74 +363,40 @@ struct InducedParams {
 
 __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant__ InducedParams p) {
   extern __shared__ __align__(16) u32 s_bloom[];
-  __shared__ i64 s_range[2];
-  __shared__ i64 s_delta[kInWindow];
-  __shared__ int s_off[kInWindow + 1];
   __shared__ u32 s_warp[kInWarps];
   __shared__ u32 s_prefix[kInThreads];
   __shared__ i64 s_queue_id[kInWarps][64];            // edges that passed the filter: row id,
-  __shared__ unsigned char s_queue_at[kInWarps][64];  // place among the warp's 256 positions
+  __shared__ unsigned char s_queue_at[kInWarps][64];  // place among the warp's 192 positions
   __shared__ u32 s_row[kInWarps][32 * kInPer];        // what the table said
   const ColRowParams& c = p.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  const i64 begin = min(c.D, (i64)blockIdx.x * p.range), end = min(c.D, begin + p.range);
+  const i64 begin = min(c.D, ((i64)blockIdx.x * kInWarps + warp) * p.range), end = min(c.D, begin + p.range);
   if (p.bloom.words) {
     const int quads = (1 << (64 - p.bloom.shift)) / 128;
     for (int i = tid; i < quads; i += kInThreads)
       reinterpret_cast<uint4*>(s_bloom)[i] = __ldcg(reinterpret_cast<const uint4*>(p.bloom.words) + i);
   }
-  u32 kept = 0;  // survivors of the CTA so far
-  for (i64 tile = begin; tile < end; tile += kInTile) {
-    const int here = (int)min((i64)kInTile, end - tile);
-    if (warp < 2) {
-      const i64 col = warp_column_at(c.sub_indptr, c.S, warp == 0 ? tile : tile + here - 1);
-      if (lane == 0) s_range[warp] = col;
-    }
-    __syncthreads();  // (also: the filter is loaded)
-    const i64 c_end = s_range[1] + 1;
-    const int base = warp * (32 * kInPer) + lane;
+  ColumnWalk walk;
+  walk.off = c.sub_indptr;
+  walk.seeds = c.seeds;
+  walk.indptr = c.indptr;
+  walk.S = c.S;
+  walk.num_cols = c.num_cols;
+  walk.counters = c.counters;  // a bad seed has positions only when sub_indptr was not counted for these seeds
+  if (begin < end) walk.init(begin, (int)(end - begin));
+  __syncthreads();  // the filter is loaded
+  u32 kept = 0;  // survivors of the warp so far
+  for (i64 at = begin; at < end; at += 32 * kInPer) {
     u32 row[kInPer];  // position in row_ids, or kNoRow
-    i64 edge[kInPer];
+    i64 edge[kInPer], id[kInPer];
     constexpr u32 kNoRow = 0xFFFFFFFFu;
 #pragma unroll
-    for (int r = 0; r < kInPer; ++r) edge[r] = -1;
-    for (i64 c0 = s_range[0]; c0 < c_end; c0 += kInWindow) {
-      const int cols = (int)min((i64)kInWindow, c_end - c0);
-      for (int j = tid; j <= cols; j += kInThreads) {
-        const i64 o = __ldg(c.sub_indptr + c0 + j);
-        s_off[j] = (int)max((i64)0, min(o - tile, (i64)here));
-        if (j < cols) {
-          const i64 col = __ldg(c.seeds + c0 + j);
-          const bool ok = (u64)col < (u64)c.num_cols;  // false only when sub_indptr was not counted for these seeds
-          if (!ok) raise_error(c.counters, GSB_ERR_INDEX_RANGE, c0 + j);
-          s_delta[j] = ok ? __ldg(c.indptr + col) - o + tile : kNoColumn;
-        }
-      }
-      __syncthreads();
-      const int w_begin = s_off[0], w_end = s_off[cols];
-      int at = 0;
-      {
-        const int q = max(base, w_begin);
-        int hi = cols;
-        while (hi - at > 1) {
-          const int mid = (at + hi) >> 1;
-          if (s_off[mid] <= q) at = mid;
-          else hi = mid;
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < kInPer; ++r) {
-        const int q = base + r * 32;
-        if (q < w_begin || q >= w_end) continue;
-        while (s_off[at + 1] <= q) ++at;
-        if (s_delta[at] != kNoColumn) edge[r] = q + s_delta[at];
-      }
-      __syncthreads();  // the window is rewritten
+    for (int r = 0; r < kInPer; ++r) {
+      edge[r] = -1;
+      if (at + r * 32 < end) edge[r] = walk.locate<false>((int)(at - begin) + r * 32, nullptr);  // uniform
+      id[r] = edge[r] >= 0 ? __ldg(c.indices + edge[r]) : -1;
     }
-    i64 id[kInPer];
-#pragma unroll
-    for (int r = 0; r < kInPer; ++r) id[r] = edge[r] >= 0 ? __ldg(c.indices + edge[r]) : -1;
     // Few edges pass the filter, but nearly every group of 32 has some: looked up where they stand, each group would wait
     // out a chain of table reads for two or three lanes.  They are queued instead, and looked up 32 at a time.
     int queued = 0;
@@ -468,38 +435,32 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
     if (queued > 0) look_up(queued);
 #pragma unroll
     for (int r = 0; r < kInPer; ++r) row[r] = s_row[warp][r * 32 + lane];
-    // ---- ranks: positions of a warp are consecutive, groups of 32
-    unsigned bits[kInPer];
-    u32 warp_total = 0;
 #pragma unroll
     for (int r = 0; r < kInPer; ++r) {
-      bits[r] = __ballot_sync(0xffffffffu, row[r] != kNoRow);
-      warp_total += __popc(bits[r]);
-    }
-    if (lane == 0) s_warp[warp] = warp_total;
-    __syncthreads();
-    u32 before = 0, all = 0;
-#pragma unroll
-    for (int w = 0; w < kInWarps; ++w) {
-      const u32 t = s_warp[w];
-      if (w < warp) before += t;
-      all += t;
-    }
-    u32 run = kept + before;
-#pragma unroll
-    for (int r = 0; r < kInPer; ++r) {
-      const int q = base + r * 32;
-      if (lane == 0 && q < here) p.packed[(tile + q) >> 5] = ((u64)run << 32) | (u64)bits[r];
+      const unsigned bits = __ballot_sync(0xffffffffu, row[r] != kNoRow);
+      const i64 q = at + r * 32;
+      if (lane == 0 && q < end) p.packed[q >> 5] = ((u64)kept << 32) | (u64)bits;
       if (row[r] != kNoRow) {
-        const i64 to = begin + run + __popc(bits[r] & lt);
+        const i64 to = begin + kept + __popc(bits & lt);
         p.kept_row[to] = row[r];
         p.kept_edge[to] = edge[r];
       }
-      run += __popc(bits[r]);
+      kept += __popc(bits);
     }
-    kept += all;
   }
-  if (tid == 0) p.totals[blockIdx.x] = kept;
+  u32 cta_before = 0;  // of the CTA's warps before this one
+  if (lane == 0) s_warp[warp] = kept;
+  __syncthreads();
+  {
+    u32 all = 0;
+#pragma unroll
+    for (int w = 0; w < kInWarps; ++w) {
+      if (w < warp) cta_before += s_warp[w];
+      all += s_warp[w];
+    }
+    if (lane == 0) p.warp_before[blockIdx.x * kInWarps + warp] = cta_before;
+    if (tid == 0) p.totals[blockIdx.x] = all;
+  }
   grid_barrier(p.sync, 1);
   // ---- emit
   u32 total;
@@ -527,8 +488,8 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
     c.counters[CNT_NNZ] = total;
     mail_post(c.mail, 0, total, c.counters);
   }
-  const i64 out0 = s_prefix[blockIdx.x];
-  for (u32 j = tid; j < kept; j += kInThreads) {  // written by this very CTA
+  const i64 out0 = s_prefix[blockIdx.x] + cta_before;
+  for (u32 j = lane; j < kept; j += 32) {  // written by this very warp
     const i64 e = __ldcg(p.kept_edge + begin + j);
     c.out_indices[out0 + j] = c.renumber ? (i64)__ldcg(p.kept_row + begin + j) : __ldg(c.indices + e);
     if (c.out_select) c.out_select[out0 + j] = e;
@@ -539,7 +500,9 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
     i64 rank = total;
     if (pos < c.D) {
       const u64 w = __ldcg(p.packed + (pos >> 5));
-      rank = s_prefix[pos / p.range] + (u32)(w >> 32) + __popc((u32)w & ((1u << (pos & 31)) - 1u));
+      const u32 owner = (u32)(pos / p.range);
+      rank = s_prefix[owner / kInWarps] + __ldcg(p.warp_before + owner) + (u32)(w >> 32) +
+             __popc((u32)w & ((1u << (pos & 31)) - 1u));
     }
     c.out_indptr[j] = rank;
   }
@@ -709,19 +672,20 @@ int gsb_col_row_slice(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
     const int ctas = min(kInThreads, ctx_resident_ctas(ctx, (const void*)k_induced, kInThreads, kBloomMaxBits / 8, resident));
     if (ctas > 0) {
       InducedParams p{};
-      const i64 tiles = (D + kInTile - 1) / kInTile;
-      p.range = ((tiles + ctas - 1) / ctas) * kInTile;
-      const int grid = (int)((D + p.range - 1) / p.range);
+      const i64 warps = (i64)ctas * kInWarps;
+      p.range = max((i64)(32 * kInPer), ((D + warps - 1) / warps + 31) / 32 * 32);
+      const int grid = (int)((D + p.range * kInWarps - 1) / (p.range * kInWarps));
       auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
       const size_t packed_bytes = al(8 * ((size_t)D / 32 + 2)), edge_bytes = al(8 * (size_t)D), row_bytes = al(4 * (size_t)D);
       void* extra;
-      int st = build_table(ctx, stream, row_ids, R, packed_bytes + edge_bytes + row_bytes + 4 * kInThreads, &table, &extra,
+      int st = build_table(ctx, stream, row_ids, R, packed_bytes + edge_bytes + row_bytes + 4 * kInThreads * (1 + kInWarps), &table, &extra,
                            R <= kBloomMaxRows ? &p.bloom : nullptr);
       if (st != GSB_OK) return st;
       p.packed = (u64*)extra;
       p.kept_edge = (i64*)((char*)extra + packed_bytes);
       p.kept_row = (u32*)((char*)extra + packed_bytes + edge_bytes);
       p.totals = (u32*)((char*)extra + packed_bytes + edge_bytes + row_bytes);
+      p.warp_before = p.totals + kInThreads;
       p.c = ColRowParams{indptr, indices, num_cols, column_ids, S, sub_indptr, D, nullptr, G, encoding_size, table,
                          renumber ? 1 : 0, out_indptr, out_indices, out_select, data, e_ids, out_data, ctx_counters(ctx),
                          TileState{}, nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0}};

@@ -199,7 +199,8 @@ struct CompactOut {
 // its table and one resident grid.
 //   single   unique(cat(first, second)) -> out_unique, ranks of `second` -> out_second (may be null), and with col_index
 //            (positions in `first`, one per entry of `second`) the ranks of first[col_index[e]] -> out_col; copies
-//            copy_n words from copy_src to copy_dst along the way.  mail slot 0: distinct ids.
+//            copy_n words from copy_src to copy_dst and sets E floats of `ones` (may be null) along the way.  mail slot 0:
+//            distinct ids.
 // id_bound > 0: ids are expected below it, which allows the direct-address table when fused_unique_direct says so; an id
 // beyond it is then reported as GSB_ERR_INDEX_RANGE too.
 //   batched  as gsb_batch_unique_relabel; with sub_indptr the edge offsets of the minibatches are sub_indptr[seeds_ptr[b]]
@@ -210,7 +211,7 @@ bool fused_unique_suits(gsb_ctx* ctx, i64 n, i64 G);
 bool fused_unique_direct(i64 G, i64 id_bound);
 int fused_unique_single(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64 S, const i64* second, i64 E,
                         const i64* col_index, i64* out_unique, i64* out_second, i64* out_col, const i64* copy_src,
-                        i64* copy_dst, i64 copy_n, i64 id_bound, Mail mail);
+                        i64* copy_dst, i64 copy_n, float* ones, i64 id_bound, Mail mail);
 int fused_unique_batched(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L, i64 seeds_bound, i64 edges_bound,
                          const i64* sub_indptr, i64* out_indices_ptr, i64* out_unique, i64* out_unique_ptr,
                          i64* out_relabeled, i64 id_bound, Mail mail);

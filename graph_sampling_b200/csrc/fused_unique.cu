@@ -56,6 +56,8 @@ struct FusedParams {
   const i64* copy_src;  // an array to copy along the way (may be null)
   i64* copy_dst;
   i64 copy_n;
+  float* ones;  // ones_n floats set to 1 along the way
+  i64 ones_n;
   // BATCHED
   const i64* seeds_ptr;    // [G + 1]
   const i64* indices_ptr;  // [G + 1], or null: the offsets are sub_indptr[seeds_ptr[b]] and are written to out_indices_ptr
@@ -319,6 +321,7 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
   }
   for (i64 j = (i64)blockIdx.x * kFuThreads + tid; j < p.copy_n; j += (i64)gridDim.x * kFuThreads)
     p.copy_dst[j] = __ldg(p.copy_src + j);
+  for (i64 j = (i64)blockIdx.x * kFuThreads + tid; j < p.ones_n; j += (i64)gridDim.x * kFuThreads) p.ones[j] = 1.0f;
   grid_barrier(p.sync, 1);
 
   // ---- flag
@@ -510,7 +513,7 @@ static int launch_fused(gsb_ctx* ctx, cudaStream_t stream, FusedParams p, i64 n,
 
 int fused_unique_single(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64 S, const i64* second, i64 E,
                         const i64* col_index, i64* out_unique, i64* out_second, i64* out_col, const i64* copy_src,
-                        i64* copy_dst, i64 copy_n, i64 id_bound, Mail mail) {
+                        i64* copy_dst, i64 copy_n, float* ones, i64 id_bound, Mail mail) {
   FusedParams p{};
   p.first = first;
   p.second = second;
@@ -523,6 +526,8 @@ int fused_unique_single(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i64
   p.copy_src = copy_src;
   p.copy_dst = copy_dst;
   p.copy_n = copy_src && copy_dst ? copy_n : 0;
+  p.ones = ones;
+  p.ones_n = ones ? E : 0;
   p.mail = mail;
   return launch_fused<false>(ctx, stream, p, S + E, id_bound);
 }

@@ -302,8 +302,8 @@ FUNCTION(relabel, 3) {
 }
 
 // ---- relabelling of a sampled graph: (ctx, col_ids, rows, cols | None, indptr to copy | None, relabel, id bound)
-//      -> (unique, rows | None, cols | None, copy | None), or None when gsb_graph_relabel does not serve the call
-FUNCTION(graph_relabel, 7) {
+//      -> (unique, rows | None, cols | None, copy | None, ones | None), or None when gsb_graph_relabel does not serve the call
+FUNCTION(graph_relabel, 8) {
   gsb_ctx* ctx = context(a[0]);
   IDS(col_ids, a[1], "col_ids");
   IDS(rows, a[2], "rows");
@@ -312,7 +312,8 @@ FUNCTION(graph_relabel, 7) {
   const c10::Device dev = device_of(col_ids);
   const int64_t S = col_ids.numel(), E = rows.numel();
   if (cols.given() && cols.numel() != E) type_error("cols must have one entry per row id");
-  Tensor unique = empty(S + E, dev), out_rows, out_cols, copy;
+  Tensor unique = empty(S + E, dev), out_rows, out_cols, copy, ones;
+  if (truth(a[7])) ones = empty(E, dev, at::kFloat);
   if (truth(a[5])) out_rows = empty(E, dev);
   const int64_t bound = integer(a[6]);
   if (cols.given()) out_cols = empty(E, dev);
@@ -322,12 +323,13 @@ FUNCTION(graph_relabel, 7) {
   {
     NoGil free;
     st = gsb_graph_relabel(ctx, stream(), col_ids.ids(), S, rows.ids(), E, cols.ids(), indptr.ids(), mut(copy),
-                           indptr.given() ? indptr.numel() : 0, bound, mut(unique), mut(out_rows), mut(out_cols), &count);
+                           indptr.given() ? indptr.numel() : 0, bound, mut(unique), mut(out_rows), mut(out_cols), mutf(ones), &count);
   }
   if (st == GSB_ERR_UNSUPPORTED) Py_RETURN_NONE;
   check(ctx, st, "gsb_graph_relabel");
   trim(unique, count);
-  return tuple_of(wrap(std::move(unique)), wrap(std::move(out_rows)), wrap(std::move(out_cols)), wrap(std::move(copy)));
+  return tuple_of(wrap(std::move(unique)), wrap(std::move(out_rows)), wrap(std::move(out_cols)), wrap(std::move(copy)),
+                  wrap(std::move(ones)));
 }
 
 // ---- random walk: (ctx, indptr, indices, seeds, length, seed, layout, walker_offset) -> trace [W, L + 1]

@@ -180,7 +180,7 @@ extern "C" int gsb_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* co
       if (fused_unique_suits(ctx, n, 1)) {
         const Mail mail = ctx_mail(ctx);
         st = fused_unique_single(ctx, stream, first, S, last, last_len, nullptr, out_unique, out_rel, nullptr, nullptr,
-                                 nullptr, 0, 0, mail);
+                                 nullptr, 0, nullptr, 0, mail);
         if (st != GSB_OK) return st;
         i64 unique = 0;
         st = ctx_mail_result(ctx, stream, mail, 1, &unique);
@@ -243,7 +243,7 @@ extern "C" int gsb_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* co
 extern "C" int gsb_graph_relabel(gsb_ctx* ctx, void* stream_, const int64_t* col_ids, int64_t S, const int64_t* rows,
                                  int64_t E, const int64_t* cols, const int64_t* copy_src, int64_t* copy_dst,
                                  int64_t copy_n, int64_t id_bound, int64_t* out_unique, int64_t* out_rows,
-                                 int64_t* out_cols, int64_t* unique_host) {
+                                 int64_t* out_cols, float* out_ones, int64_t* unique_host) {
   GSB_ENTER(ctx);
   GSB_REQUIRE(S >= 0 && E >= 0 && copy_n >= 0 && unique_host, GSB_ERR_INVALID_ARGUMENT);
   GSB_REQUIRE((S == 0 || col_ids) && (E == 0 || rows) && (copy_n == 0 || (copy_src && copy_dst)), GSB_ERR_INVALID_ARGUMENT);
@@ -257,7 +257,7 @@ extern "C" int gsb_graph_relabel(gsb_ctx* ctx, void* stream_, const int64_t* col
   for (i64 bound = fused_unique_direct(1, id_bound) ? id_bound : 0; st == GSB_ERR_INDEX_RANGE; bound = 0) {
     const Mail mail = ctx_mail(ctx);
     st = fused_unique_single(ctx, stream, col_ids, S, rows, E, cols, out_unique, out_rows, out_cols, copy_src, copy_dst,
-                             copy_n, bound, mail);
+                             copy_n, out_ones, bound, mail);
     if (st != GSB_OK) return st;
     st = ctx_mail_result(ctx, stream, mail, 1, &unique);
     if (bound == 0) break;

@@ -531,21 +531,35 @@ class Graph:
         return ops.graph_unique(col_ids, rows, id_bound=self._id_bound)
 
     def Relabel(self):
+        return self._relabel(False)[:7]
+
+    def relabel_with_data(self):
+        """Relabel's seven values and the edge data in the order of its edges (src/graph.cc:785-839, 68-90), ones for a graph
+        without data: the two calls of a block in one launch."""
+        out = self._relabel(self.data_ is None)
+        data, e_ids = (out[7] if out[7] is not None else self._data_or_ones()), out[5]
+        return out[:7] + (data[e_ids] if e_ids is not None else data,)
+
+    def _relabel(self, ones):
         col_ids = self._require_col_ids()
         if self.csc_ is not None:
             if self.val_col_ids_ is not None:
                 col_ids = col_ids[self.val_col_ids_]
             row_indices = self.row_ids_[self.csc_.indices] if self.row_ids_ is not None else self.csc_.indices
-            frontier, relabeled, _, indptr = ops.graph_relabel(col_ids, row_indices, indptr=self.csc_.indptr,
-                                                                id_bound=self._id_bound)
-            return frontier, frontier.numel(), col_ids.numel(), indptr, relabeled, self.csc_.e_ids, "csc"
+            ones = ones and self.csc_.e_ids is None and row_indices.numel() == self.num_edges_
+            frontier, relabeled, _, indptr, *data = ops.graph_relabel(col_ids, row_indices, indptr=self.csc_.indptr,
+                                                                       id_bound=self._id_bound, ones=ones)
+            return (frontier, frontier.numel(), col_ids.numel(), indptr, relabeled, self.csc_.e_ids, "csc",
+                    data[0] if data else None)
         if self.csr_ is not None or self.coo_ is not None:
             if self.coo_ is None:
                 self.coo_ = self._csc2coo(self.csr_, False)
             coo_row = self.row_ids_[self.coo_.row] if self.row_ids_ is not None else self.coo_.row
-            frontier, rel_row, rel_col, _ = ops.graph_relabel(col_ids, coo_row, cols=self.coo_.col,
-                                                               id_bound=self._id_bound)
-            return (frontier, frontier.numel(), col_ids.numel(), rel_row, rel_col, self.coo_.e_ids, "coo")
+            ones = ones and self.coo_.e_ids is None and coo_row.numel() == self.num_edges_
+            frontier, rel_row, rel_col, _, *data = ops.graph_relabel(col_ids, coo_row, cols=self.coo_.col,
+                                                                      id_bound=self._id_bound, ones=ones)
+            return (frontier, frontier.numel(), col_ids.numel(), rel_row, rel_col, self.coo_.e_ids, "coo",
+                    data[0] if data else None)
         _fatal("Error in Relabel!")
 
     # ---- RandomWalk (src/graph.cc:646-648) -------------------------------------------------------------------------

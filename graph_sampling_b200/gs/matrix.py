@@ -48,6 +48,9 @@ class Matrix:
         return self._graph._CAPI_get_num_cols()
 
     def to_block(self) -> Block:
+        if type(self._graph) is Graph:  # not under tracing
+            frontier, num_row, num_col, t1, t2, e_ids, fmt, data = self._graph.relabel_with_data()
+            return Block(fmt, t1, t2, num_row, num_col, frontier, e_ids, data)
         frontier, num_row, num_col, t1, t2, e_ids, fmt = self._graph._CAPI_relabel()
         data = self._graph._CAPI_get_data("default")
         if data is not None and e_ids is not None:

@@ -290,15 +290,21 @@ def relabel(mapping_tensors, data_requiring_relabel, ctx=None):
     return ctx.native.relabel(ctx.address, mapping_tensors, data_requiring_relabel)
 
 
-def graph_relabel(col_ids, rows, cols=None, indptr=None, ctx=None, id_bound=0):
+def graph_relabel(col_ids, rows, cols=None, indptr=None, ctx=None, id_bound=0, ones=False):
     """What Graph.Relabel does with a sampled graph (src/graph.cc:785-839) → (unique, relabelled rows, relabelled
     columns | None, copy of indptr | None): the frontier unique(cat(col_ids, rows)), every row id's position in it and,
-    for a COO whose edge e lies in column cols[e], the position of col_ids[cols[e]]."""
+    for a COO whose edge e lies in column cols[e], the position of col_ids[cols[e]].  With `ones` a fifth value: a float 1
+    per edge, the weights of a graph that has none, written by the same launch."""
     ctx = _context_for(col_ids, ctx)
     on_device = indptr is None or indptr.is_cuda
-    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, cols, indptr if on_device else None, True, int(id_bound))
+    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, cols, indptr if on_device else None, True, int(id_bound),
+                                   ones)
     if out is not None:
-        return out if on_device else out[:3] + (indptr.clone(),)
+        out = out if on_device else out[:3] + (indptr.clone(),) + out[4:]
+        return out if ones else out[:4]
+    if ones:
+        return graph_relabel(col_ids, rows, cols, indptr, ctx, id_bound) + (
+            torch.ones(rows.numel(), dtype=torch.float32, device=col_ids.device),)
     if cols is None:
         frontier, (new_rows,) = relabel([col_ids, rows], [rows], ctx)
         return frontier, new_rows, None, indptr.clone() if indptr is not None else None
@@ -309,7 +315,7 @@ def graph_relabel(col_ids, rows, cols=None, indptr=None, ctx=None, id_bound=0):
 def graph_unique(col_ids, rows, ctx=None, id_bound=0):
     """unique(cat(col_ids, rows)) in first-occurrence order; id_bound as in gsb_graph_relabel, a hint."""
     ctx = _context_for(col_ids, ctx)
-    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, None, None, False, int(id_bound))
+    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, None, None, False, int(id_bound), False)
     return out[0] if out is not None else relabel([col_ids, rows], [], ctx)[0]
 
 

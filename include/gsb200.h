@@ -205,7 +205,8 @@ GSB_API int gsb_unique_relabel(gsb_ctx* ctx, void* stream, const int64_t* const*
 /* What gs::Graph::Relabel does with a sampled graph (src/graph.cc:785-839), in one launch: out_unique =
  * unique(cat(col_ids, rows)) in first-occurrence order; out_rows[e] = position of rows[e] in it; with `cols` (COO
  * form: cols[e] = position of edge e's column in col_ids) also out_cols[e] = position of col_ids[cols[e]]; copies
- * copy_n words from copy_src to copy_dst along the way (the offsets a CSC result hands out).  out_unique holds S + E
+ * copy_n words from copy_src to copy_dst along the way (the offsets a CSC result hands out) and sets the E floats of
+ * out_ones, unless it is NULL, to 1 (the edge weights of a graph without any).  out_unique holds S + E
  * entries; out_rows may be NULL when only the distinct ids are wanted.  id_bound > 0 is a hint that ids lie below it (a
  * graph knows its node count): it allows a direct-address table; ids beyond it cost a second launch, nothing else.
  * Waits for the number of distinct ids.  GSB_ERR_UNSUPPORTED — nothing usable was written — for calls beyond
@@ -214,7 +215,7 @@ GSB_API int gsb_unique_relabel(gsb_ctx* ctx, void* stream, const int64_t* const*
 GSB_API int gsb_graph_relabel(gsb_ctx* ctx, void* stream, const int64_t* col_ids, int64_t S, const int64_t* rows,
                               int64_t E, const int64_t* cols, const int64_t* copy_src, int64_t* copy_dst,
                               int64_t copy_n, int64_t id_bound, int64_t* out_unique, int64_t* out_rows,
-                              int64_t* out_cols, int64_t* unique_host);
+                              int64_t* out_cols, float* out_ones, int64_t* unique_host);
 
 /* ---- uniform random walk ----------------------------------------------------------------------
  * Replaces gs::impl::fusion::FusedRandomWalkCUDA / _RandomWalkKernel

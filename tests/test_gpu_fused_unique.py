@@ -33,7 +33,8 @@ def test_graph_relabel_matches_oracle(ops, oracle, n, spread):
     indptr = rng.integers(0, 1 << 40, 77).astype(np.int64)
     bound = int(ids.max()) + 1 if spread == 3 else 0     # the direct-address table; without a bound the hash table
     assert np.array_equal(ops.graph_unique(dev(first), dev(second), id_bound=max(1, bound - 1)).cpu().numpy(), frontier)
-    f, rows, cols, copy = ops.graph_relabel(dev(first), dev(second), indptr=dev(indptr), id_bound=bound)
+    f, rows, cols, copy, ones = ops.graph_relabel(dev(first), dev(second), indptr=dev(indptr), id_bound=bound, ones=True)
+    assert ones.numel() == len(second) and bool((ones == 1.0).all())
     assert cols is None and np.array_equal(f.cpu().numpy(), frontier)
     assert np.array_equal(rows.cpu().numpy(), w_rows) and np.array_equal(copy.cpu().numpy(), indptr)
     f, (rel,) = ops.relabel([dev(first), dev(second)], [dev(second)])
@@ -51,6 +52,7 @@ def test_ids_beyond_32_bits_take_the_general_form(ops, oracle):
     second = np.array([1 << 40, 7, 5], np.int64)
     frontier, (want,) = oracle.unique_relabel([first, second], [second])
     f, rows, _, _ = ops.graph_relabel(dev(first), dev(second))
+    assert ops.graph_relabel(dev(first), dev(second), ones=True)[4].tolist() == [1.0] * len(second)
     assert np.array_equal(f.cpu().numpy(), frontier) and np.array_equal(rows.cpu().numpy(), want)
     with pytest.raises(Exception):
         ops.graph_relabel(dev(np.array([3, -2], np.int64)), dev(second))

@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(kFmtThreads) k_gather_i64(const i64* __restric
 //   per digit of up to 11 bits (one to three of them):
 //     count    CTA c owns the c-th stretch of the current order, warp w the w-th part of that; 16-bit counts per warp and
 //              digit in shared memory; the CTA's counts go to matrix[digit][c]
-//     scan     a warp per digit turns its row of the matrix into exclusive prefixes, and notes the digit's total
+//     scan     a warp per digit (a thread when there are few CTAs: a single one took 10 of its 23 us to walk 1 024 rows a
+//              warp at a time) turns its row of the matrix into exclusive prefixes, and notes the digit's total
 //     place    every warp walks its part again, 32 items at a time ranked with __match_any_sync, and writes each item to
 //              digit start + CTA prefix + warp prefix + rank: stable, since everything is numbered in order
 //   along the way, the offsets: counts per key (one reduction per edge) during the first scan, totals per CTA of keys
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(kFmtThreads) k_gather_i64(const i64* __restric
 constexpr int kConvThreads = 1024;
 constexpr int kConvWarps = kConvThreads / 32;
 constexpr int kConvMaxBins = 2048;
+constexpr int kConvFewCtas = 8;
 constexpr i64 kConvMaxEdges = 4ll << 20;  // 28 000 edges per CTA: a warp's count fits 16 bits
 
 struct ConvParams {
@@ -170,31 +172,51 @@ __global__ void __launch_bounds__(kConvThreads) k_coo2csc(const __grid_constant_
     __syncthreads();
     for (int b = tid; b < bins; b += kConvThreads) {
       u32 run = 0;
-      for (int w = 0; w < kConvWarps; ++w) {  // counts -> prefixes over the warps
-        const u32 c = s_count[w * bins + b];
-        s_count[w * bins + b] = (uint16_t)run;
-        run += c;
+      for (int w0 = 0; w0 < kConvWarps; w0 += 16) {  // counts -> prefixes over the warps
+        u32 c[16];
+#pragma unroll
+        for (int w = 0; w < 16; ++w) c[w] = s_count[(w0 + w) * bins + b];
+#pragma unroll
+        for (int w = 0; w < 16; ++w) {
+          s_count[(w0 + w) * bins + b] = (uint16_t)run;
+          run += c[w];
+        }
       }
       p.matrix[(size_t)b * ctas + blockIdx.x] = run;
     }
     grid_barrier(p.sync, ++barrier);
     // ---- scan of the matrix rows; counts per key
-    for (int b = (int)blockIdx.x * kConvWarps + warp; b < bins; b += ctas * kConvWarps) {
-      u32* row = p.matrix + (size_t)b * ctas;
-      u32 carry = 0;
-      for (int c0 = 0; c0 < ctas; c0 += 32) {
-        const int c = c0 + lane;
-        const u32 v = c < ctas ? __ldcg(row + c) : 0;
-        u32 inc = v;
+    if (ctas <= kConvFewCtas) {  // a row is a few words and there are many rows per warp: a thread per row instead
+      for (int b = (int)blockIdx.x * kConvThreads + tid; b < bins; b += ctas * kConvThreads) {
+        u32* row = p.matrix + (size_t)b * ctas;
+        u32 v[kConvFewCtas], run = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
-          if (lane >= o) inc += t;
+        for (int c = 0; c < kConvFewCtas; ++c) v[c] = c < ctas ? __ldcg(row + c) : 0;
+#pragma unroll
+        for (int c = 0; c < kConvFewCtas; ++c) {
+          if (c < ctas) row[c] = run;
+          run += v[c];
         }
-        if (c < ctas) row[c] = carry + inc - v;
-        carry += __shfl_sync(0xffffffffu, inc, 31);
+        p.bin_total[b] = run;
       }
-      if (lane == 0) p.bin_total[b] = carry;
+    } else {
+      for (int b = (int)blockIdx.x * kConvWarps + warp; b < bins; b += ctas * kConvWarps) {
+        u32* row = p.matrix + (size_t)b * ctas;
+        u32 carry = 0;
+        for (int c0 = 0; c0 < ctas; c0 += 32) {
+          const int c = c0 + lane;
+          const u32 v = c < ctas ? __ldcg(row + c) : 0;
+          u32 inc = v;
+  #pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+          }
+          if (c < ctas) row[c] = carry + inc - v;
+          carry += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) p.bin_total[b] = carry;
+      }
     }
     if (digit == 0)
       for (u32 i = begin + lane; i < end; i += 32) {
@@ -320,7 +342,7 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
                                                     sizeof(uint16_t) * kConvWarps * kConvMaxBins, resident));
     // two items per thread at least: fewer CTAs make the barriers and the matrix of a short list cheaper; the offsets of a
     // long key range want CTAs too
-    const i64 want = max((E + 2 * kConvThreads - 1) / (2 * kConvThreads), num_keys / (16 * kConvThreads));
+    const i64 want = max((E + 2 * kConvThreads - 1) / (2 * kConvThreads), num_keys / (4 * kConvThreads));
     const int conv_grid = (int)max((i64)1, min((i64)ctas, want));
     if (ctas > 0 && (E + conv_grid - 1) / conv_grid + 32 * kConvWarps <= 65535ll) {
       auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };

@@ -446,15 +446,29 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
   }
   if (overflow && !COUNT) return;
   if (!overflow) {
+    // one array after the other, each behind one test (a test of every optional array per pick: 2 265 against 2 138 us for the
+    // last hop of 500 minibatches, 83 against 77 for 61 000 columns of ten picks)
 #pragma unroll
-    for (int j = 0; j < KMAX; ++j) {
-      if (j < n) {
-        const i64 in_pos = b + pick[j];
-        p.out_indices[o + j] = val[j];
-        if (p.out_select) p.out_select[o + j] = in_pos;
-        if (p.out_coo_col) p.out_coo_col[o + j] = i;
-        if (p.out_data) p.out_data[o + j] = p.data[p.e_ids ? p.e_ids[in_pos] : in_pos];
-      }
+    for (int j = 0; j < KMAX; ++j)
+      if (j < n) p.out_indices[o + j] = val[j];
+    if (p.out_data) {
+      float x[KMAX];
+#pragma unroll
+      for (int j = 0; j < KMAX; ++j)
+        if (j < n) x[j] = __ldg(p.data + (p.e_ids ? __ldg(p.e_ids + b + pick[j]) : b + pick[j]));
+#pragma unroll
+      for (int j = 0; j < KMAX; ++j)
+        if (j < n) p.out_data[o + j] = x[j];
+    }
+    if (p.out_select) {
+#pragma unroll
+      for (int j = 0; j < KMAX; ++j)
+        if (j < n) p.out_select[o + j] = b + pick[j];
+    }
+    if (p.out_coo_col) {
+#pragma unroll
+      for (int j = 0; j < KMAX; ++j)
+        if (j < n) p.out_coo_col[o + j] = i;
     }
   }
   if (COUNT) {

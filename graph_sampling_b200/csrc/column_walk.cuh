@@ -13,7 +13,8 @@ namespace gsb {
 
 constexpr i64 kNoWalkColumn = (i64)1 << 62;  // a seed outside the operand: its positions are skipped
 
-// Largest c with off[c] <= pos, by a whole warp.  Needs off[0] <= pos < off[S].
+// Largest c with off[c] <= pos, by a whole warp: 32 pivots per step, so a search over a few hundred thousand columns takes four
+// dependent loads instead of eighteen.  Needs off[0] <= pos < off[S].
 __device__ __forceinline__ i64 warp_column_search(const i64* __restrict__ off, i64 S, i64 pos) {
   const int lane = threadIdx.x & 31;
   i64 lo = 0, hi = S;

@@ -145,7 +145,6 @@ __global__ void __launch_bounds__(kRowThreads) k_row_indptr(const i64* __restric
 // the survivors with ballots + one look-back; the thread that owns the first edge of a column also writes
 // that column's output offset.  (One warp per column was measured 6x slower on a power-law graph: the
 // warp that gets a 17 000-edge column runs 540 dependent rounds while the rest of the grid is idle.)
-constexpr i64 kNoColumn = (i64)1 << 62;
 struct ColRowParams {
   const i64* indptr;
   const i64* indices;
@@ -199,23 +198,6 @@ __device__ __forceinline__ i64 column_at(const i64* __restrict__ sub_indptr, i64
   return lo;
 }
 
-// The same search done by a whole warp: 32 pivots per step, so a search over a few hundred thousand columns takes
-// four dependent loads instead of eighteen.  Needs sub_indptr[0] <= pos < sub_indptr[S].
-__device__ __forceinline__ i64 warp_column_at(const i64* __restrict__ sub_indptr, i64 S, i64 pos) {
-  const int lane = threadIdx.x & 31;
-  i64 lo = 0, hi = S;
-  while (hi - lo > 1) {
-    const i64 step = (hi - lo + 31) / 32;
-    const i64 idx = lo + (i64)(lane + 1) * step;
-    const bool le = idx < hi && __ldg(sub_indptr + idx) <= pos;   // true for a prefix of the lanes
-    const int n = __popc(__ballot_sync(0xffffffffu, le));
-    const i64 new_hi = min(hi, lo + (i64)(n + 1) * step);
-    lo += (i64)n * step;
-    hi = new_hi;
-  }
-  return lo;
-}
-
 __global__ void __launch_bounds__(kRowThreads) k_col_row_filter(ColRowParams p) {
   __shared__ i64 s_warp_total[kRowThreads / 32];
   __shared__ i64 s_base, s_clo, s_chi;
@@ -226,7 +208,7 @@ __global__ void __launch_bounds__(kRowThreads) k_col_row_filter(ColRowParams p) 
   // the tile's column range: two warp-wide searches side by side (one thread doing both binary searches over the
   // global offsets was 36 dependent loads with the rest of the CTA waiting at the barrier — most of the kernel's time)
   if (warp < 2) {
-    const i64 c = warp_column_at(p.sub_indptr, p.S, warp == 0 ? tile_base : tile_end - 1);
+    const i64 c = warp_column_search(p.sub_indptr, p.S, warp == 0 ? tile_base : tile_end - 1);
     if (lane == 0) (warp == 0 ? s_clo : s_chi) = c;
   }
   __syncthreads();

@@ -182,7 +182,7 @@ int ctx_resident_ctas(gsb_ctx* ctx, const void* kernel, int threads, size_t smem
 }
 
 GridSync ctx_grid_sync(gsb_ctx* ctx, int grid, int barriers) {
-  const GridSync g{(u64*)(ctx->counters + CNT_NUM), ctx->barrier_arrivals, ctx->counters,
+  const GridSync g{(u64*)(ctx->counters + CNT_NUM), ctx->barrier_arrivals, (u32)barriers, ctx->counters,
                    (int)ctx->options[GSB_OPT_MAX_POLLS]};
   ctx->barrier_arrivals += (u64)grid * (u64)barriers;
   return g;
@@ -320,6 +320,8 @@ int ctx_check_device_error(gsb_ctx* ctx, cudaStream_t stream) {
     snprintf(ctx->message, sizeof(ctx->message), "device-side error %d (%s), detail %lld", code,
              gsb_status_string(code), (long long)c[1]);
     GSB_CUDA_OK(cudaMemsetAsync(ctx->counters + CNT_ERROR, 0, 2 * sizeof(i64), stream));
+    // the mark of a grid barrier that was given up, the top byte of its word (grid_sync.cuh)
+    GSB_CUDA_OK(cudaMemsetAsync((char*)(ctx->counters + CNT_NUM) + kBarrierCountBits / 8, 0, 1, stream));
     {
       int st2 = ctx_wait(ctx, stream);
       if (st2 != GSB_OK) return st2;

@@ -322,7 +322,22 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
   for (i64 j = (i64)blockIdx.x * kFuThreads + tid; j < p.copy_n; j += (i64)gridDim.x * kFuThreads)
     p.copy_dst[j] = __ldg(p.copy_src + j);
   for (i64 j = (i64)blockIdx.x * kFuThreads + tid; j < p.ones_n; j += (i64)gridDim.x * kFuThreads) p.ones[j] = 1.0f;
-  grid_barrier(p.sync, 1);
+  // The results of a call that was given up, for the super-batch hops that run on without the host: empty frontiers.
+  auto give_up = [&] {
+    if (!BATCHED) return;
+    for (i64 b = (i64)blockIdx.x * kFuThreads + tid; b <= p.G; b += (i64)gridDim.x * kFuThreads) {
+      const i64 e = fused_edges_begin(p, b, __ldg(p.seeds_ptr + b));
+      if (p.out_indices_ptr) p.out_indices_ptr[b] = e;
+      p.out_unique_ptr[b] = 0;
+    }
+    if (p.out_second)
+      for (i64 e = (i64)blockIdx.x * kFuThreads + tid; e < ne; e += (i64)gridDim.x * kFuThreads) p.out_second[e] = -1;
+    if (blockIdx.x == 0 && tid == 0) {
+      p.counters[CNT_UNIQUE] = 0;
+      p.counters[CNT_NNZ] = ne;
+    }
+  };
+  if (!grid_barrier(p.sync, 1)) return give_up();
 
   // ---- flag
   unsigned bits[R];
@@ -363,7 +378,7 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
       if (g < n) p.packed[g >> 5] = ((u64)s_group[r * kFuWarps + warp] << 32) | (u64)bits[r];
     }
   }
-  grid_barrier(p.sync, 2);
+  if (!grid_barrier(p.sync, 2)) return give_up();
 
   // ---- emit
   u32 all;

@@ -3,16 +3,29 @@
 //
 // The barrier word counts arrivals for ever: a launch is told the count it starts from, and every CTA arrives exactly
 // `barriers` times whatever happens, so the word never needs clearing.  The wait is bounded like every other wait of the
-// library (GSB_OPT_MAX_POLLS, then GSB_ERR_LOOKBACK_TIMEOUT).
+// library (GSB_OPT_MAX_POLLS, then GSB_ERR_LOOKBACK_TIMEOUT), and what follows a barrier indexes with what other CTAs wrote
+// before it, so nobody may go on from one that was given up.  All CTAs agree on that: giving up is a compare-and-swap of the
+// word as it was last seen, incomplete, to the same count with a mark on it.  Whoever sees a complete count therefore sees the
+// mark too if there is one, and a count without it means that everybody has arrived.  The mark stays until the error is read
+// (ctx_check_device_error), and cooperative kernels launched in between end at their first barrier.
+//
+// A call that does not wait for its result cannot report the error before its outputs are used, so a kernel that gives up
+// leaves results that are wrong but within range: an empty sample or subgraph, a conversion with all edges in column 0.  Every
+// CTA of the launch comes to that point and writes its own share of them; shares are such that no other CTA writes there
+// before the last barrier.
 #pragma once
 #include "common.cuh"
 #include "scan.cuh"
 
 namespace gsb {
 
+constexpr int kBarrierCountBits = 56;  // arrivals; the top byte is the mark
+constexpr u64 kBarrierGivenUp = 1ull << 63;
+
 struct GridSync {
   u64* word;
   u64 base;
+  u32 barriers;
   i64* counters;
   int max_polls;
 };
@@ -23,27 +36,37 @@ __device__ __forceinline__ u64 ld_acquire_u64(const u64* p) {
   return v;
 }
 
-// Barrier number `index` (1, 2, ...) of the launch.  Release / acquire, cumulative over what the CTA did before it.
-__device__ __forceinline__ void grid_barrier(const GridSync& g, u32 index) {
+// For a CTA that returns early: the arrivals it still owes.
+__device__ __forceinline__ void grid_arrive(const GridSync& g, u32 arrivals) {
+  if (threadIdx.x == 0) atomicAdd(g.word, (u64)arrivals);
+}
+
+// Barrier number `index` (1, 2, ...) of the launch.  Release / acquire, cumulative over what the CTA did before it.  False, in
+// every thread, when this barrier or (while the CTA was looking) a later one was given up: the CTA has made the arrivals of its
+// later barriers then and has to return without using anything that another CTA was to write.
+[[nodiscard]] __device__ __forceinline__ bool grid_barrier(const GridSync& g, u32 index) {
+  bool ok = true;
   __syncthreads();
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(g.word) : "memory");
     const u64 target = g.base + (u64)index * gridDim.x;
     int polls = 0;
-    while ((i64)(ld_acquire_u64(g.word) - target) < 0) {
-      if (++polls > g.max_polls) {
-        raise_error(g.counters, GSB_ERR_LOOKBACK_TIMEOUT, blockIdx.x);
-        break;
+    for (;;) {
+      const u64 seen = ld_acquire_u64(g.word);
+      ok = seen < kBarrierGivenUp;
+      if (!ok || (i64)((seen - target) << (64 - kBarrierCountBits)) >= 0) break;
+      if (++polls > g.max_polls) {  // fails only when somebody arrived meanwhile: at most as often as there are CTAs
+        ok = atomicCAS(g.word, seen, seen | kBarrierGivenUp) != seen;
+        if (!ok) break;
       }
       if (polls > 64) __nanosleep(20);
     }
+    if (!ok) {
+      raise_error(g.counters, GSB_ERR_LOOKBACK_TIMEOUT, blockIdx.x);
+      grid_arrive(g, g.barriers - index);
+    }
   }
-  __syncthreads();
-}
-
-// For a CTA that returns early: the arrivals it still owes.
-__device__ __forceinline__ void grid_arrive(const GridSync& g, u32 arrivals) {
-  if (threadIdx.x == 0) atomicAdd(g.word, (u64)arrivals);
+  return __syncthreads_and(ok);
 }
 
 // CTAs of a kernel that are resident at once on the context's device (0: cooperative launches are not available).  The

@@ -83,8 +83,16 @@ __global__ void __launch_bounds__(kSelectThreads) k_list_select(const __grid_con
     if (valid) p.composite[i] = c;
     select_count(s_hist, (unsigned)(c >> 53), valid);
   }
+  // The result of a call that was given up: the first k items.
+  auto give_up = [&] {
+    if (blockIdx.x != 0) return;
+    for (int i = tid; i < (int)p.k; i += kSelectThreads) {
+      p.out_index[i] = i;
+      p.out_data[i] = __ldg(p.data + i);
+    }
+  };
   u32 barrier = 1;
-  grid_barrier(p.sync, barrier);  // the global histograms are clear
+  if (!grid_barrier(p.sync, barrier)) return give_up();  // the global histograms are clear
   u64 prefix = 0, mask = 0;
   unsigned need = (unsigned)p.k;
   int pass = 0;
@@ -93,7 +101,7 @@ __global__ void __launch_bounds__(kSelectThreads) k_list_select(const __grid_con
     unsigned* hist = p.hist + pass * kSelectBins;
     for (int i = tid; i < kSelectBins; i += kSelectThreads)
       if (s_hist[i]) atomicAdd(hist + i, s_hist[i]);
-    grid_barrier(p.sync, ++barrier);
+    if (!grid_barrier(p.sync, ++barrier)) return give_up();
     // every CTA picks the bin for itself: thread t owns bins 2t, 2t + 1; `above` counts the items in larger bins
     {
       const uint2 h = __ldcg(reinterpret_cast<const uint2*>(hist) + tid);
@@ -148,8 +156,10 @@ __global__ void __launch_bounds__(kSelectThreads) k_list_select(const __grid_con
     grid_arrive(p.sync, 1);
     return;
   }
-  grid_barrier(p.sync, ++barrier);
-  grid_arrive(p.sync, (kSelectBarriers - barrier) * gridDim.x);  // the arrivals of the passes that were not needed
+  const bool complete = grid_barrier(p.sync, ++barrier);
+  // the arrivals of the passes that were not needed (its own are made when the barrier was given up)
+  grid_arrive(p.sync, (kSelectBarriers - barrier) * (gridDim.x - (complete ? 0 : 1)));
+  if (!complete) return give_up();
   int n = 1;
   while (n < (int)p.k) n <<= 1;
   for (int i = tid; i < n; i += kSelectThreads) s_win[i] = i < (int)p.k ? __ldcg(p.winners + i) : 0ull;  // 0 sorts last

@@ -443,7 +443,11 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
     if (lane == 0) p.warp_before[blockIdx.x * kInWarps + warp] = cta_before;
     if (tid == 0) p.totals[blockIdx.x] = all;
   }
-  grid_barrier(p.sync, 1);
+  if (!grid_barrier(p.sync, 1)) {  // given up: an empty subgraph
+    for (i64 j = (i64)blockIdx.x * kInThreads + tid; j <= c.S; j += (i64)gridDim.x * kInThreads) c.out_indptr[j] = 0;
+    if (blockIdx.x == 0 && tid == 0) c.counters[CNT_NNZ] = 0;
+    return;
+  }
   // ---- emit
   u32 total;
   {

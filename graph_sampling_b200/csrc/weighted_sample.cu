@@ -73,7 +73,6 @@ __device__ __forceinline__ bool ranks_before(float ka, u32 ia, float kb, u32 ib)
 }
 
 __device__ __forceinline__ void emit_weighted(const WeightedParams& p, i64 out_pos, i64 in_pos, i64 col_pos) {
-  if ((u64)out_pos >= (u64)p.capacity) return;  // only after a barrier gave up waiting
   p.out_indices[out_pos] = __ldg(p.indices + in_pos);
   if (p.out_select) p.out_select[out_pos] = in_pos;
   if (p.out_coo_col) p.out_coo_col[out_pos] = col_pos;
@@ -390,23 +389,12 @@ __device__ __forceinline__ int kind_of(const WeightedParams& p, i64 d) {
   return d <= kSlice ? KIND_SCAN : KIND_HUGE;
 }
 
-// The lists are read and written within their bounds even if a barrier gave up waiting (the call then ends with an error, but
-// with counts that not every CTA has written).
-__device__ __forceinline__ void list_put(const WeightedParams& p, u64 at, i64 column) {
-  if (at < (u64)p.S) p.lists[at] = column;
-}
-
-__device__ __forceinline__ i64 list_get(const WeightedParams& p, i64 at) {
-  const i64 column = (u64)at < (u64)p.S ? __ldcg(p.lists + at) : -1;
-  return (u64)column < (u64)p.S ? column : -1;
-}
-
 // Warp-collective: a unit of copies (columns no longer than the fan-out) or sorts, as many columns as fit a warp.
 __device__ __forceinline__ void short_columns(const WeightedParams& p, int kind, i64 list, i64 first, i64 count, u64* s_order) {
   const int lanes = kind == KIND_SORT128 ? 32 : kind == KIND_SORT64 ? 16 : 8;
   const int lane = lane_id(), g = lane & (lanes - 1);
   const i64 at = first + lane / lanes;
-  const i64 c = at < count ? list_get(p, list + at) : -1;
+  const i64 c = at < count ? __ldcg(p.lists + list + at) : -1;
   i64 o = 0;
   Column column{0, 0};
   if (c >= 0) {
@@ -428,14 +416,12 @@ __device__ __forceinline__ void scan_column(const WeightedParams& p, i64 c, bool
     c = __ldcg(&p.slices[unit].column);
     index = __ldcg(&p.slices[unit].index);
     first = __ldcg(&p.slices[unit].first);
-    if ((u64)c >= (u64)p.S || first > unit) return;
   }
   const Column column = column_of(p, c, false);
   const i64 o = __ldcg(p.out_indptr + c);
   u32 e_begin = 0, e_end = (u32)column.d;
   if (sliced) {
     slices = (unsigned)((column.d + slice - 1) / slice);
-    if (first + slices > kMaxSlices) return;
     e_begin = (u32)(index * slice);
     e_end = (u32)min(column.d, (i64)(index + 1) * slice);
   }
@@ -631,7 +617,12 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
     for (int w = 0; w < kWarps; ++w) sum += s_part[w][tid][0];
     p.partial[(i64)blockIdx.x * NUM_SUMS + tid] = (i64)sum;
   }
-  grid_barrier(p.sync, 1);
+  // The result of a call that was given up: an empty sample.
+  auto give_up = [&] {
+    for (i64 c = lo + tid; c < hi; c += kWThreads) p.out_indptr[c] = 0;
+    if (blockIdx.x == 0 && tid == 0) p.out_indptr[S] = p.counters[CNT_NNZ] = 0;
+  };
+  if (!grid_barrier(p.sync, 1)) return give_up();
 
   // every CTA adds up what comes before it and the totals
   static_assert(NUM_SUMS == 8, "eight threads take one CTA's sums");
@@ -670,8 +661,10 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
   if (blockIdx.x == 0 && tid == 0) {
     p.out_indptr[S] = edges;
     p.counters[CNT_NNZ] = edges;
-    if (overflow) raise_error(p.counters, GSB_ERR_CAPACITY, edges);
-    mail_post(p.mail, 0, edges, p.counters);
+    if (overflow) {
+      raise_error(p.counters, GSB_ERR_CAPACITY, edges);
+      mail_post(p.mail, 0, edges, p.counters);
+    }
   }
   // slices so long that there is room for them: no more than kMaxSlices / 2 columns are longer than one, and what is left over
   // of each adds one more at most
@@ -701,11 +694,11 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
       unsigned at = 0;
       if (lane == 0) at = atomicAdd(&s_listed[v], (unsigned)__popc(who));
       at = __shfl_sync(0xffffffffu, at, 0);
-      if (kind == v) list_put(p, s_at[v] + at + __popc(who & ((1u << lane) - 1u)), c);
+      if (kind == v) p.lists[s_at[v] + at + __popc(who & ((1u << lane) - 1u))] = c;
     }
     if (kind == KIND_HUGE) {
       if (WIDE || p.replace || d <= slice) {
-        list_put(p, atomicAdd(p.queue + QUEUE_HUGE, 1ull), c);  // the first region
+        p.lists[atomicAdd(p.queue + QUEUE_HUGE, 1ull)] = c;  // the first region
       } else {
         const unsigned slices = (unsigned)((d + slice - 1) / slice);
         const u64 first = atomicAdd(p.queue + QUEUE_SLICES, (u64)slices);
@@ -721,17 +714,17 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
     grid_arrive(p.sync, 1);
     return;
   }
-  grid_barrier(p.sync, 2);
+  if (!grid_barrier(p.sync, 2)) return give_up();
+  if (blockIdx.x == 0 && tid == 0) mail_post(p.mail, 0, edges, p.counters);  // nothing can go wrong from here on
 
   // Every CTA does each gridDim-th unit of work, the long ones first, and its warps take them as they become free: a counter
   // for the whole grid is what the grid would wait for (one word takes about one atomic per nanosecond).
-  const i64 slices = min((i64)__ldcg(p.queue + QUEUE_SLICES), (i64)kMaxSlices);
-  const i64 huge = min((i64)__ldcg(p.queue + QUEUE_HUGE), S);
-  const i64 scans = min((i64)s_total[KIND_SCAN], S), scan_list = (i64)s_total[KIND_HUGE];
+  const i64 slices = min((i64)__ldcg(p.queue + QUEUE_SLICES), (i64)kMaxSlices), huge = (i64)__ldcg(p.queue + QUEUE_HUGE);
+  const i64 scans = (i64)s_total[KIND_SCAN], scan_list = (i64)s_total[KIND_HUGE];
   const i64 heavy = slices + huge + scans;
   auto heavy_column = [&](i64 unit) {
     unit -= slices;
-    return list_get(p, unit < huge ? unit : scan_list + unit - huge);
+    return __ldcg(p.lists + (unit < huge ? unit : scan_list + unit - huge));
   };
   i64 first = blockIdx.x;  // of the CTA's units
   if (WIDE) {
@@ -741,8 +734,7 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
       __syncthreads();
       const i64 unit = s_unit;
       if (unit >= heavy) break;
-      const i64 c = heavy_column(unit);
-      if (c >= 0) select_wide(p, s_wide, c);
+      select_wide(p, s_wide, heavy_column(unit));
       __syncthreads();
     }
     first += heavy;
@@ -754,7 +746,6 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
     if (!WIDE && unit < heavy) {
       const bool sliced = unit < slices;
       const i64 c = sliced ? 0 : heavy_column(unit);
-      if (c < 0) continue;
       if (p.replace) {
         const Column column = column_of(p, c, false);
         draw_with_replacement(p, column.b, column.d, __ldcg(p.out_indptr + c), c, reinterpret_cast<float*>(s_order[warp]));
@@ -769,7 +760,7 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
 #pragma unroll 1
     for (; kind < NUM_KINDS; ++kind) {
       const int columns = kind == KIND_SORT128 ? 1 : kind == KIND_SORT64 ? 2 : 4;  // in a unit
-      const i64 count = min((i64)s_total[kind], S), units = (count + columns - 1) / columns;
+      const i64 count = (i64)s_total[kind], units = (count + columns - 1) / columns;
       if (unit < units) {
         short_columns(p, kind, list, unit * columns, count, s_order[warp]);
         break;

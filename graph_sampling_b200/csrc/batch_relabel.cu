@@ -28,12 +28,12 @@ namespace gsb {
 // One CTA: per-batch item offsets and / or table regions (exclusive scan over the G region sizes).
 // bound_k < 0: regions sized from the batches' actual item counts (needs indices_ptr); bound_k >= 0: regions sized
 // from the upper bound seeds * (1 + bound_k), which is known before sampling.
-// what & 1: write region_off; what & 2: write item_off (indices_ptr is valid); what & 4: keep an abort that an earlier
-// launch of the same call set; what & 8: region_off receives the first BUCKET of every minibatch instead of a table
+// what & 1: write region_off; what & 2: write item_off (indices_ptr is valid); what & 8: region_off receives the first BUCKET of every minibatch instead of a table
 // region (partition_relabel.cu; slot_capacity then bounds the bucket count); what & 32: bucket_count, the array of
 // per-bucket item counts that the counting sampler will add to, is cleared (slot_capacity + 1 words).
 // seeds_bound / edges_bound: what the caller sized grids, scratch and outputs for.  Device-side totals above them
-// record GSB_ERR_CAPACITY and set CNT_ABORT, which makes the kernels that follow in the call return at once.
+// record GSB_ERR_CAPACITY and set CNT_ABORT, which makes the kernels that follow in the call return at once; a look-back
+// that was given up since the last error was read sets it too, as the sizes here may be its results.
 __global__ void __launch_bounds__(kBThreads) k_batch_layout(BatchLayout L, i64* counters, i64 bound_k, int what,
                                                             i64 seeds_bound, i64 edges_bound,
                                                             uint32_t* bucket_count = nullptr) {
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(kBThreads) k_batch_layout(BatchLayout L, i64* 
     s_carry = 0;
     const i64 ns = L.seeds_ptr[L.G], ne = (what & 2) ? L.indices_ptr[L.G] : 0;
     const bool over = ns > seeds_bound || ne > edges_bound || ns < 0 || ne < 0;
-    if (!(what & 4) || over) counters[CNT_ABORT] = over ? 1 : 0;
+    counters[CNT_ABORT] = over || counters[CNT_LOST] != 0 ? 1 : 0;
     if (over) raise_error(counters, GSB_ERR_CAPACITY, ns > seeds_bound ? ns : ne);
   }
   __syncthreads();
@@ -405,7 +405,8 @@ __global__ void __launch_bounds__(kBThreads) k_split_indptr(const i64* __restric
 
 // Batch number of every frontier entry (the `key` output of BatchUnique).
 __global__ void __launch_bounds__(kBThreads) k_unique_keys(const i64* __restrict__ unique_ptr, i64 G,
-                                                           i64* __restrict__ out_key) {
+                                                           i64* __restrict__ out_key, const i64* counters) {
+  if (counters[CNT_ABORT] != 0) return;
   for_each_item_with_batch(unique_ptr, G, unique_ptr[G], [&](i64 i, i64 b) { out_key[i] = b; });
 }
 
@@ -427,6 +428,7 @@ __global__ void __launch_bounds__(kBThreads) k_batch_filter(BatchLayout L, Filte
                                                             TileState ts) {
   __shared__ i64 s_warp_total[kBThreads / 32];
   __shared__ i64 s_base;
+  if (counters[CNT_ABORT] != 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tile = blockIdx.x;
   const i64 tile_base = (i64)tile * kBTile;
@@ -571,7 +573,7 @@ __global__ void __launch_bounds__(kBThreads) k_sorted_unique_compact(const u64* 
     const i64 i = base + q * 32 + lane;
     if (i < end && first[q]) {
       const i64 pos = warp_pos + rank[q];
-      const i64 b = (i64)(key[q] >> 32);
+      const i64 b = min((i64)(key[q] >> 32), G - 1);  // larger only where the sort was given up (CNT_LOST)
       out_unique[pos] = (i64)(key[q] & 0xFFFFFFFFull);
       if (out_key) out_key[pos] = b;
       const i64 pb = i > 0 ? (i64)(prev[q] >> 32) : -1;
@@ -580,7 +582,7 @@ __global__ void __launch_bounds__(kBThreads) k_sorted_unique_compact(const u64* 
   }
   if (tile_base + kBTile >= n && threadIdx.x == 0) {
     const i64 total = s_base + tile_total;
-    const i64 last = n > 0 ? (i64)(keys[n - 1] >> 32) : -1;
+    const i64 last = n > 0 ? min((i64)(keys[n - 1] >> 32), G - 1) : -1;
     for (i64 e = last + 1; e <= G; ++e) out_ptr[e] = total;
     counters[CNT_UNIQUE] = total;
   }
@@ -1026,7 +1028,7 @@ int gsb_batch_unique(gsb_ctx* ctx, void* stream_, const int64_t* data, const int
     if (st != GSB_OK) return st;
     if (out_unique_key && n > 0) {
       ScopedKernelTimer timer(ctx, KID_OTHER, stream);
-      k_unique_keys<<<grid, kBThreads, 0, stream>>>(out_unique_ptr, G, out_unique_key);
+      k_unique_keys<<<grid, kBThreads, 0, stream>>>(out_unique_ptr, G, out_unique_key, ctx_counters(ctx));
       GSB_LAUNCH_OK();
     }
     return unique_total_host ? read_totals(ctx, stream, unique_total_host, nullptr) : GSB_OK;

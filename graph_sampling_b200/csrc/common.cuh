@@ -44,6 +44,7 @@ enum CounterSlot {
   CNT_EPOCH = 6,       // device-side epoch base (pipeline mode)
   CNT_ABORT = 7,       // set by the layout kernel of a super-batch call whose device-side sizes exceed the caller's
                        // bounds: the kernels that follow return at once instead of writing past their buffers
+  CNT_LOST = 8,        // set, with CNT_ABORT, by a look-back that was given up; stays until the error is read
   CNT_NUM = 64
 };
 

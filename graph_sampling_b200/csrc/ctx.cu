@@ -320,6 +320,7 @@ int ctx_check_device_error(gsb_ctx* ctx, cudaStream_t stream) {
     snprintf(ctx->message, sizeof(ctx->message), "device-side error %d (%s), detail %lld", code,
              gsb_status_string(code), (long long)c[1]);
     GSB_CUDA_OK(cudaMemsetAsync(ctx->counters + CNT_ERROR, 0, 2 * sizeof(i64), stream));
+    GSB_CUDA_OK(cudaMemsetAsync(ctx->counters + CNT_LOST, 0, sizeof(i64), stream));
     // the mark of a grid barrier that was given up, the top byte of its word (grid_sync.cuh)
     GSB_CUDA_OK(cudaMemsetAsync((char*)(ctx->counters + CNT_NUM) + kBarrierCountBits / 8, 0, 1, stream));
     {

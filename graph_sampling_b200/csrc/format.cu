@@ -62,10 +62,18 @@ __global__ void __launch_bounds__(kFmtThreads) k_make_sort_input(const i64* __re
   }
 }
 
-__global__ void __launch_bounds__(kFmtThreads) k_gather_i64(const i64* __restrict__ src, const i64* __restrict__ idx,
-                                                            i64 n, i64* __restrict__ dst) {
-  for (i64 e = (i64)blockIdx.x * kFmtThreads + threadIdx.x; e < n; e += (i64)gridDim.x * kFmtThreads)
-    dst[e] = src[idx ? idx[e] : e];
+// The other coordinate in key order (perm null: the edges are in that order as they are).  Where a scan was given up the result is
+// what k_coo2csc leaves in that case: all edges, in the order of the list, in column 0.
+__global__ void __launch_bounds__(kFmtThreads) k_conversion_end(const i64* __restrict__ other, i64* perm, i64 E, i64 num_keys,
+                                                                i64* __restrict__ out_indptr, i64* __restrict__ out_other,
+                                                                const i64* counters) {
+  const i64 first = (i64)blockIdx.x * kFmtThreads + threadIdx.x, step = (i64)gridDim.x * kFmtThreads;
+  const bool lost = counters[CNT_LOST] != 0;
+  if (lost) {
+    for (i64 e = first; e < E && perm; e += step) perm[e] = e;
+    for (i64 k = first; k <= num_keys; k += step) out_indptr[k] = k == 0 ? 0 : E;
+  }
+  for (i64 e = first; e < E; e += step) out_other[e] = other[perm && !lost ? perm[e] : e];
 }
 
 // ---- COO -> CSC / CSR in one launch ------------------------------------------------------------------------------
@@ -397,7 +405,9 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
   if (st != GSB_OK) return st;
   if (E == 0) return GSB_OK;
   if (key_sorted) {
-    GSB_CUDA_OK(cudaMemcpyAsync(out_other, other, sizeof(i64) * (size_t)E, cudaMemcpyDeviceToDevice, stream));
+    k_conversion_end<<<grid, kFmtThreads, 0, stream>>>(other, nullptr, E, num_keys, out_indptr, out_other, ctx_counters(ctx));
+    GSB_LAUNCH_OK();
+    ctx_count_launches(ctx, 1);
     return GSB_OK;
   }
   void* ws;
@@ -409,7 +419,7 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
   GSB_LAUNCH_OK();
   st = radix_sort_pairs(ctx, stream, keys, out_perm, E, 0, bits, ws);
   if (st != GSB_OK) return st;
-  k_gather_i64<<<grid, kFmtThreads, 0, stream>>>(other, out_perm, E, out_other);
+  k_conversion_end<<<grid, kFmtThreads, 0, stream>>>(other, out_perm, E, num_keys, out_indptr, out_other, ctx_counters(ctx));
   GSB_LAUNCH_OK();
   ctx_count_launches(ctx, 2);
   return GSB_OK;

@@ -308,10 +308,11 @@ __global__ void __launch_bounds__(kListThreads) k_invert_keys(u64* __restrict__ 
 
 __global__ void __launch_bounds__(kListThreads) k_emit_winners(const u64* __restrict__ winners, i64 k,
                                                                const i64* __restrict__ data, i64* __restrict__ out_data,
-                                                               i64* __restrict__ out_index) {
+                                                               i64* __restrict__ out_index, const i64* counters) {
+  const bool lost = counters[CNT_LOST] != 0;  // then the first k items, as k_list_select leaves them
   for (i64 j = (i64)blockIdx.x * kListThreads + threadIdx.x; j < k; j += (i64)gridDim.x * kListThreads) {
     const u64 c = ~winners[j];  // k_invert_keys
-    const i64 idx = (i64)(0xFFFFFFFFu - (uint32_t)c);
+    const i64 idx = lost ? j : (i64)(0xFFFFFFFFu - (uint32_t)c);
     out_index[j] = idx;
     out_data[j] = data[idx];
   }
@@ -518,7 +519,8 @@ extern "C" int gsb_list_sample(gsb_ctx* ctx, void* stream_, const int64_t* data,
   if (st != GSB_OK) return st;
   ctx_count_launches(ctx, 1);
   k_emit_winners<<<min(grid_for(k, kListThreads), wide), kListThreads, 0, stream>>>(winners, k, data,
-                                                                                    out_data, out_index);
+                                                                                    out_data, out_index,
+                                                                                    ctx_counters(ctx));
   GSB_LAUNCH_OK();
   ctx_count_launches(ctx, 1);
   return GSB_OK;

@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const u64* __res
                                                                const i64* __restrict__ vals_in,
                                                                u64* __restrict__ keys_out, i64* __restrict__ vals_out,
                                                                i64 n, int shift, const i64* __restrict__ hist,
-                                                               int num_tiles) {
+                                                               int num_tiles, const i64* counters) {
+  if (counters[CNT_LOST] != 0) return;
   constexpr int kWarps = kSortThreads / 32;
   constexpr int kRounds = kSortItemsPerThread;  // each warp owns kRounds * 32 consecutive items
   __shared__ unsigned s_warp_count[kWarps][kRadix];
@@ -213,6 +214,7 @@ int radix_sort_pairs(gsb_ctx* ctx, cudaStream_t stream, u64* keys, i64* vals, i6
   u64* keys_tmp = (u64*)scratch;
   i64* vals_tmp = (i64*)(keys_tmp + n);
   i64* hist = vals_tmp + n;
+  const i64* counters = ctx_counters(ctx);
   u64* kin = keys;
   i64* vin = vals;
   u64* kout = keys_tmp;
@@ -222,8 +224,8 @@ int radix_sort_pairs(gsb_ctx* ctx, cudaStream_t stream, u64* keys, i64* vals, i6
     GSB_LAUNCH_OK();
     int st = exclusive_scan_i64(ctx, stream, hist, (i64)kRadix * tiles);
     if (st != GSB_OK) return st;
-    if (vals) k_radix_scatter<true><<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, shift, hist, tiles);
-    else k_radix_scatter<false><<<tiles, kSortThreads, 0, stream>>>(kin, nullptr, kout, nullptr, n, shift, hist, tiles);
+    if (vals) k_radix_scatter<true><<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, shift, hist, tiles, counters);
+    else k_radix_scatter<false><<<tiles, kSortThreads, 0, stream>>>(kin, nullptr, kout, nullptr, n, shift, hist, tiles, counters);
     GSB_LAUNCH_OK();
     ctx_count_launches(ctx, 2);
     u64* tk = kin; kin = kout; kout = tk;

@@ -8,9 +8,12 @@
 // sequence (src/cuda/slicing.cu:133-147, src/cuda/utils.h:17-28).
 //
 // Tiles are numbered by blockIdx.x and rely on CTAs being dispatched in index order, as every
-// single-pass scan does.  The wait on a predecessor is bounded: after TileState::max_polls polls the CTA
-// records GSB_ERR_LOOKBACK_TIMEOUT in the context's error counter and continues with prefix 0, so
-// a lost predecessor can never hang the GPU.
+// single-pass scan does.  The wait on a predecessor is bounded, so a lost predecessor can never hang the GPU: after
+// TileState::max_polls polls the CTA marks the words it still waits for as lost (a compare-and-swap, so a word that was
+// published meanwhile is used after all), records GSB_ERR_LOOKBACK_TIMEOUT and continues with prefix 0.  Words are published
+// with a maximum, which a mark beats, so every tile behind a lost one finds it lost: the last tile, which knows the total and
+// posts it to the host, can't take a sum for complete that another tile has given up on.  The kernels that follow see
+// CNT_ABORT and CNT_LOST and do not use such a scan.
 #pragma once
 #include "common.cuh"
 
@@ -18,6 +21,13 @@ namespace gsb {
 
 __device__ __forceinline__ u64 tile_word(uint32_t epoch, uint32_t flag, i64 value) {
   return ((u64)(epoch & kEpochMask) << 42) | ((u64)flag << 40) | ((u64)value & kValueMask);
+}
+
+constexpr uint32_t kTileLost = 3;
+
+// A word of an older epoch is smaller, and so is an aggregate (1) than an inclusive prefix (2) and both than a mark (3).
+__device__ __forceinline__ void tile_post(const TileState& ts, int tile, u64 word) {
+  asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;" ::"l"(ts.words + tile), "l"(word) : "memory");
 }
 
 __device__ __forceinline__ u64 ld_volatile_u64(const u64* p) {
@@ -48,20 +58,21 @@ __device__ __forceinline__ void mail_post(const Mail& m, int slot, i64 value, co
 // PUBLISHES its aggregate (its successors can then add it up without waiting for this tile's own prefix), issues
 // whatever loads it can, and only then RESOLVES its prefix — the wait for the predecessors overlaps those loads.
 __device__ __forceinline__ void tile_publish_aggregate(const TileState& ts, int tile, i64 aggregate) {
-  if ((threadIdx.x & 31) == 0) st_volatile_u64(&ts.words[tile], tile_word(ts.epoch, tile == 0 ? 2 : 1, aggregate));
+  if ((threadIdx.x & 31) == 0) tile_post(ts, tile, tile_word(ts.epoch, tile == 0 ? 2 : 1, aggregate));
 }
 
-__device__ __forceinline__ i64 tile_resolve_prefix(const TileState& ts, int tile, i64 aggregate);
+__device__ __forceinline__ i64 tile_resolve_prefix(const TileState& ts, int tile, i64 aggregate, bool* lost = nullptr);
 
 // Called by all 32 lanes of warp 0 of the CTA that owns `tile`.  Returns the sum of the
-// aggregates of tiles [0, tile) and publishes this tile's inclusive prefix.
-__device__ __forceinline__ i64 tile_exclusive_prefix(const TileState& ts, int tile, i64 aggregate) {
+// aggregates of tiles [0, tile) and publishes this tile's inclusive prefix.  *lost: a wait was given up, the prefix is 0.
+__device__ __forceinline__ i64 tile_exclusive_prefix(const TileState& ts, int tile, i64 aggregate, bool* lost = nullptr) {
   tile_publish_aggregate(ts, tile, aggregate);
-  return tile_resolve_prefix(ts, tile, aggregate);
+  return tile_resolve_prefix(ts, tile, aggregate, lost);
 }
 
-__device__ __forceinline__ i64 tile_resolve_prefix(const TileState& ts, int tile, i64 aggregate) {
+__device__ __forceinline__ i64 tile_resolve_prefix(const TileState& ts, int tile, i64 aggregate, bool* lost) {
   const int lane = threadIdx.x & 31;
+  if (lost) *lost = false;
   if (tile == 0) return 0;
   i64 exclusive = 0;
   int idx = tile - 1;  // nearest predecessor examined by lane 0
@@ -75,14 +86,22 @@ __device__ __forceinline__ i64 tile_resolve_prefix(const TileState& ts, int tile
       if (my >= 0) w = ld_volatile_u64(&ts.words[my]);
       ready = ((uint32_t)(w >> 42) == ep) && (((w >> 40) & 3ull) != 0ull);
       if (__all_sync(0xffffffffu, ready)) break;
-      if (++polls > ts.max_polls) {
-        if (lane == 0) raise_error(ts.counters, GSB_ERR_LOOKBACK_TIMEOUT, tile);
-        if (!ready) w = tile_word(ep, 2, 0);
-        break;
+      if (++polls > ts.max_polls && !ready) {  // at most as often as the word changes: three times
+        const u64 mark = tile_word(ep, kTileLost, 0);
+        if (atomicCAS(&ts.words[my], w, mark) == w) w = mark;
       }
       __nanosleep(20);
     } while (true);
     const uint32_t flag = (uint32_t)((w >> 40) & 3ull);
+    if (__any_sync(0xffffffffu, flag == kTileLost)) {  // no tile behind a lost one has an inclusive prefix
+      if (lane == 0) {
+        raise_error(ts.counters, GSB_ERR_LOOKBACK_TIMEOUT, tile);
+        ts.counters[CNT_ABORT] = ts.counters[CNT_LOST] = 1;
+        tile_post(ts, tile, tile_word(ep, kTileLost, 0));
+      }
+      if (lost) *lost = true;
+      return 0;
+    }
     const i64 val = (i64)(w & kValueMask);
     const uint32_t full = __ballot_sync(0xffffffffu, flag == 2u);
     if (full) {
@@ -99,7 +118,7 @@ __device__ __forceinline__ i64 tile_resolve_prefix(const TileState& ts, int tile
     exclusive += contrib;
     idx -= 32;
   }
-  if (lane == 0) st_volatile_u64(&ts.words[tile], tile_word(ts.epoch, 2, exclusive + aggregate));
+  if (lane == 0) tile_post(ts, tile, tile_word(ts.epoch, 2, exclusive + aggregate));
   return exclusive;
 }
 

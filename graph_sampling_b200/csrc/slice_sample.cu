@@ -72,11 +72,17 @@ __global__ void __launch_bounds__(kThreads) k_count_scan(const i64* __restrict__
   i64 total;
   i64 run = block_exclusive_scan<kThreads>(sum, s_scan, &total);
   if (threadIdx.x < 32) {
-    const i64 prefix = tile_exclusive_prefix(ts, tile, total);
-    if (threadIdx.x == 0) s_base = prefix;
+    bool lost;
+    const i64 prefix = tile_exclusive_prefix(ts, tile, total, &lost);
+    if (threadIdx.x == 0) s_base = lost ? -1 : prefix;
   }
   __syncthreads();
-  const i64 tile_base = s_base;
+  i64 tile_base = s_base;
+  if (tile_base < 0) {  // given up, and so is every tile behind it: no edges from here on
+    tile_base = total = run = 0;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) f[q] = 0;
+  }
   run += tile_base;
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
@@ -264,11 +270,20 @@ __global__ void __launch_bounds__(kThreads) k_sample_uniform(SampleParams p) {
   const i64 excl = block_exclusive_scan<kThreads>(f, s_scan, &total);
   if (tid < kTileCols) s_off[tid] = excl;
   if (tid < 32) {
-    const i64 prefix = tile_exclusive_prefix(p.ts, tile, total);
-    if (tid == 0) s_base = prefix;
+    bool lost;
+    const i64 prefix = tile_exclusive_prefix(p.ts, tile, total, &lost);
+    if (tid == 0) s_base = lost ? -1 : prefix;
   }
   __syncthreads();
   const i64 tile_base = s_base;
+  if (tile_base < 0) {  // given up, and so is every tile behind it: no edges from here on
+    if (tid < ncol) p.out_indptr[base + tid] = 0;
+    if (base + kTileCols >= S && tid == 0) {
+      p.out_indptr[S] = p.counters[CNT_NNZ] = 0;
+      mail_post(p.mail, 0, 0, p.counters);
+    }
+    return;
+  }
   if (tid < ncol) p.out_indptr[base + tid] = tile_base + excl;
   if (base + kTileCols >= S && tid == 0) {
     p.out_indptr[S] = tile_base + total;
@@ -434,21 +449,22 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     for (int j = 0; j < KMAX; ++j)
       if (j < n) x[j] = __ldg(p.data + b + pick[j]);
   }
-  const i64 prefix = __shfl_sync(0xffffffffu, tile_resolve_prefix(p.ts, (int)tile, total), 0);
+  bool lost;
+  const i64 prefix = __shfl_sync(0xffffffffu, tile_resolve_prefix(p.ts, (int)tile, total, &lost), 0);
   const i64 o = prefix + inc - f;
   if (valid) {
-    p.out_indptr[i] = o;
+    p.out_indptr[i] = lost ? 0 : o;  // given up, and so is every tile behind it: no edges from here on
     if (i == S - 1) {
-      p.out_indptr[S] = o + f;
-      p.counters[CNT_NNZ] = o + f;
+      p.out_indptr[S] = lost ? 0 : o + f;
+      p.counters[CNT_NNZ] = lost ? 0 : o + f;
     }
   } else if (S == 0 && lane == 0) {
     p.out_indptr[0] = 0;
     p.counters[CNT_NNZ] = 0;
   }
-  const bool overflow = prefix + total > p.capacity;  // the prefix only grows: the last tile sees it if any tile does
+  const bool overflow = lost || prefix + total > p.capacity;  // the prefix only grows: the last tile sees it if any tile does
   if (lane == 0) {
-    if (overflow) raise_error(p.counters, GSB_ERR_CAPACITY, prefix + total);
+    if (overflow) raise_error(p.counters, GSB_ERR_CAPACITY, prefix + total);  // (behind the error of a wait that was given up)
     if (tile * 32 + 32 >= S) mail_post(p.mail, 0, prefix + total, p.counters);
   }
   if (overflow && !COUNT) return;

@@ -77,9 +77,10 @@ GSB_API int gsb_check_device_status(gsb_ctx* ctx, void* stream);
  *  GSB_OPT_MAX_POLLS            polls of one look-back window before a scan gives up waiting for a predecessor
  *                               tile, and of a grid barrier before a cooperative kernel gives up waiting for its
  *                               other CTAs, and records GSB_ERR_LOOKBACK_TIMEOUT (default 2^22; polls sleep 20 ns).
- *                               A cooperative kernel that gives up returns without its result (an empty sample or
- *                               subgraph, a conversion with all edges in column 0, the first k items of a list), and
- *                               so do those that follow it until the error is read;
+ *                               A call that reports a size returns that error itself.  Until the error is read, what
+ *                               the call and those that build on it leave behind is within range but not the result
+ *                               (no edges from some column on, an empty subgraph, a conversion with all edges in
+ *                               column 0, the first k items of a list, batched outputs not written);
  *  GSB_OPT_TABLE_SLOTS          > 0: gsb_unique_relabel builds its hash table with this many slots (rounded down
  *                               to a power of two) instead of sizing it from the item count — a table that is too
  *                               small reports GSB_ERR_TABLE_FULL; 0 (default) = automatic;

@@ -1,6 +1,7 @@
-"""Cooperative kernels whose grid barrier runs out of polls (GSB_OPT_MAX_POLLS = 1, so that the first CTAs to arrive give up):
-the call reports it, what it leaves behind lies within its buffers and is a result that later kernels can read, and the
-context works as before once the error is read.  A call that gets through all the same has to be right."""
+"""Grid barriers of the cooperative kernels and look-back chains of the scans that run out of polls (GSB_OPT_MAX_POLLS = 1, so
+that the first CTAs to wait give up): the call reports it, what it leaves behind lies within its buffers and is a result that
+later kernels can read, and the context works as before once the error is read.  A call that gets through all the same has to
+be right: a wait that was given up anywhere in the call must not go unnoticed."""
 import ctypes
 
 import numpy as np
@@ -34,15 +35,21 @@ def same(a, b):
     return np.array_equal(a, b) if a is not None else b is None
 
 
-def run_out(ops, call, left_behind=None):
-    """Calls until the barrier has run out a few times, then again with the usual limit."""
+def pinned(a):
+    """Read in place from host memory: what the CTAs wait for arrives one CTA after the other."""
+    return torch.from_numpy(np.ascontiguousarray(a)).pin_memory()
+
+
+def run_out(ops, call, left_behind=None, tries=200, certain=True):
+    """Calls until a wait has run out a few times, then again with the usual limit.  certain=False: the CTAs arrive so close to
+    each other that no wait may run out, whatever the limit."""
     from graph_sampling_b200.cabi import GsbError
     ctx = ops.Context()
     want = as_numpy(call(ctx))
     ctx.check_device()
     usual, expired = ctx.get_option("max_polls"), 0
     ctx.set_option("max_polls", 1)
-    for _ in range(200):
+    for _ in range(tries):
         got = None
         try:
             got = as_numpy(call(ctx))
@@ -56,7 +63,7 @@ def run_out(ops, call, left_behind=None):
                 break
         else:
             assert same(got, want)
-    assert expired > 0
+    assert expired > 0 or not certain
     ctx.set_option("max_polls", usual)
     for _ in range(2):
         assert same(as_numpy(call(ctx)), want)
@@ -132,8 +139,7 @@ def test_batched_relabel(ops, num_nodes):
 def test_weighted_sampling(ops, hub_graph, k, replace):
     indptr, indices = (dev(a) for a in hub_graph)
     probs = torch.rand(indices.numel(), generator=torch.Generator("cuda").manual_seed(4), device="cuda") + 0.01
-    # read in place from host memory: the CTAs' columns arrive one after the other
-    columns = torch.from_numpy(np.random.default_rng(k).integers(0, len(hub_graph[0]) - 1, 400_000)).pin_memory()
+    columns = pinned(np.random.default_rng(k).integers(0, len(hub_graph[0]) - 1, 400_000))
     run_out(ops, lambda ctx: ops.csc_col_sampling_probs(indptr, indices, probs, k, replace, seed=8, column_ids=columns, ctx=ctx))
 
 
@@ -156,3 +162,104 @@ def test_induced_subgraph(ops):
 
     run_out(ops, call)
     run_out(ops, lambda ctx: call(ctx, wait=False), lambda got: np.testing.assert_array_equal(got[0], 0))
+
+
+# ---- look-back chains ------------------------------------------------------------------------------------------------------
+def test_slice_offsets(ops):
+    indptr, _ = graph(100_000, 2_000_000, 6)
+    for S in (20_000, 700_000):   # one and four columns per thread
+        columns = pinned(np.random.default_rng(S).integers(0, 100_000, S))
+
+        def call(ctx, wait=True):
+            out, nnz = torch.full((S + 1 + PAD,), -7, dtype=torch.int64, device="cuda"), ctypes.c_int64(0)
+            ctx.check(ctx.lib.gsb_col_slice_count(ctx.handle, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream),
+                                                  indptr.data_ptr(), 100_000, columns.data_ptr(), S, out.data_ptr(),
+                                                  ctypes.byref(nnz) if wait else None), "gsb_col_slice_count")
+            assert bool((out[S + 1:] == -7).all())
+            return out[:S + 1], nnz.value
+
+        def left_behind(got):   # offsets up to some column, no edges from there on
+            offsets = got[0]
+            kept = int(np.argmax(np.diff(offsets) < 0)) + 1
+            assert np.all(offsets[kept:] == 0) and np.all(np.diff(offsets[:kept]) >= 0)
+
+        run_out(ops, call)
+        run_out(ops, lambda ctx: call(ctx, wait=False), left_behind)
+
+
+@pytest.mark.parametrize("k", [5, 16, 25])
+def test_uniform_sampling(ops, k):
+    indptr, indices = graph(100_000, 2_000_000, 6)
+    columns = pinned(np.random.default_rng(k).integers(0, 100_000, 300_000))
+    run_out(ops, lambda ctx: ops.fused_csc_col_slicing_sampling(indptr, indices, columns, k, False, seed=3, ctx=ctx))
+
+
+@pytest.mark.parametrize("sort", [False, True])
+def test_batched_unique(ops, sort):
+    rng = np.random.default_rng(9)
+    ptr = np.arange(41) * 20_000
+    data, d_ptr = dev(rng.integers(0, 50_000, ptr[-1])), dev(ptr)
+    run_out(ops, lambda ctx: ops.batch_unique(data, d_ptr, sort=sort, ctx=ctx), tries=50, certain=False)
+
+
+@pytest.mark.parametrize("path", [1, 2, 3])
+def test_batched_relabel_forms(ops, path):
+    rng = np.random.default_rng(7)
+    sp, ep = np.arange(41) * 500, np.arange(41) * 12_000
+    seeds, edges = dev(rng.integers(0, 50_000, sp[-1])), dev(rng.integers(0, 50_000, ep[-1]))
+    d_sp, d_ep = dev(sp), dev(ep)
+
+    def call(ctx):
+        ctx.set_option("relabel_path", path)
+        return ops.batch_csr_relabel(seeds, d_sp, edges, d_ep, ctx=ctx, num_nodes=50_000)[:3]
+
+    run_out(ops, call, tries=50, certain=False)
+
+
+@pytest.mark.parametrize("path", [0, 1, 3])
+def test_queued_hops(ops, path):
+    """Three hops without a wait in between: whichever scan is given up, the hops behind it write nothing out of bounds."""
+    indptr, indices = graph(100_000, 2_000_000, 5)
+    seeds, ptr = pinned(np.arange(16_000)), dev(np.arange(17) * 1000)
+
+    def call(ctx):
+        ctx.set_option("relabel_path", path)
+        hops = ops.sage_sample_batches(indptr, indices, seeds, ptr, [5, 5, 3], seed=2, ctx=ctx, sync=False)
+        return [h["frontier_ptr"] for h in hops]
+
+    run_out(ops, call)
+
+
+def test_row_slices(ops):
+    indptr, indices = graph(100_000, 2_000_000, 6)
+    rows = dev(np.random.default_rng(2).permutation(100_000)[:30_000])
+    run_out(ops, lambda ctx: ops.csc_row_slicing(indptr, indices, rows, ctx=ctx), tries=50, certain=False)
+    cols = ops.csc2coo(indptr, indices)[1]
+    run_out(ops, lambda ctx: ops.coo_row_slicing(pinned(indices.cpu().numpy()), cols, rows, ctx=ctx), tries=50)
+
+
+@pytest.mark.parametrize("presorted", [False, True])
+def test_conversion_in_several_launches(ops, presorted):
+    E, keys = (4 << 20) + 77, 300_000
+    rng = np.random.default_rng(E)
+    key, other = rng.integers(0, keys, E), dev(rng.integers(0, 1 << 40, E))
+    key = dev(np.sort(key) if presorted else key)
+    everything = other.cpu().numpy()
+
+    def left_behind(got):
+        indptr, rows, perm = got
+        assert indptr[0] == 0 and np.all(indptr[1:] == E) and np.array_equal(rows, everything)
+        assert perm is None or np.array_equal(perm, np.arange(E))
+
+    run_out(ops, lambda ctx: ops.coo2csc(other, key, keys, presorted, ctx=ctx), left_behind, tries=20, certain=False)
+
+
+def test_long_list_sample(ops):
+    N, k = 1_000_000, 20_000
+    rng = np.random.default_rng(k)
+    data, probs = dev(rng.permutation(N)), dev(rng.random(N, dtype=np.float32))
+
+    def left_behind(got):
+        assert np.array_equal(got[1], np.arange(k)) and np.array_equal(got[0], data[:k].cpu().numpy())
+
+    run_out(ops, lambda ctx: ops.list_sampling(data, k, False, probs, seed=3, ctx=ctx), left_behind, tries=50, certain=False)

@@ -262,6 +262,11 @@ static int ctx_spin(gsb_ctx* ctx, cudaStream_t stream, const volatile u64* word,
 
 Mail ctx_mail(gsb_ctx* ctx) {
   ctx->mail_tag = ctx->mail_tag >= 0xFFFF ? 1 : ctx->mail_tag + 1;
+  // Tags repeat after 65 535 mailboxes, and a slot that few calls post still holds what the last of them left there: a word
+  // with the tag of this mailbox must not be there yet.  (Who posted to the slots before has been waited for, or its call
+  // failed within the last few mailboxes: its tag is another one.)
+  volatile u64* slots = (volatile u64*)(ctx->pinned + CNT_NUM);
+  for (int q = 0; q < kMailSlots; ++q) slots[q] = 0;
   return Mail{(u64*)(ctx->pinned + CNT_NUM), ctx->mail_tag << 48};
 }
 

@@ -83,6 +83,20 @@ def test_batched_relabel_matches_oracle(ops, oracle, G, mean):
         assert np.array_equal(f[fp[b]:fp[b + 1]], want) and np.array_equal(rel[ep[b]:ep[b + 1]], w_rel)
 
 
+def test_mailbox_tags_wrap(ops):
+    """The sizes of a call reach the host in words tagged with one of 65 535 numbers.  A batched call leaves two of them, the
+    others one: the second must not be taken from the batched call that had the same number before."""
+    ctx, few = ops.Context(), dev(np.arange(32) % 7)
+    ptr = dev(np.array([0, 8, 16]))
+    calls = [(edges, dev(np.array([0, 400, edges])), dev(np.arange(edges) % 50)) for edges in range(1000, 1005)]
+    torch.cuda.synchronize()
+    for edges, iptr, ids in calls:
+        _, _, rel, _ = ops.batch_csr_relabel(few[:16], ptr, ids, iptr, ctx=ctx)
+        assert rel.numel() == edges
+        for _ in range(65_534):
+            ops.tensor_unique(few, ctx=ctx)
+
+
 def test_epochs_wrap(ops, oracle):
     """2 047 calls use up the epochs of the table; results stay right across the wrap."""
     rng = np.random.default_rng(1)

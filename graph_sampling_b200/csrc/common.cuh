@@ -143,6 +143,7 @@ int ctx_wait_mail(gsb_ctx* ctx, cudaStream_t stream, const Mail& mail, int n, i6
 // The usual end of a call that reports `n` posted values: waits, fills `values`, returns the device error if there is one.
 int ctx_mail_result(gsb_ctx* ctx, cudaStream_t stream, const Mail& mail, int n, i64* values);
 void ctx_count_launches(gsb_ctx* ctx, int n);
+void ctx_count_id_bound_refusal(gsb_ctx* ctx);
 // When profiling is enabled (gsb_profile_enable) these bracket a launch with CUDA events on the
 // launching stream; otherwise they only count the launch.
 void ctx_prof_begin(gsb_ctx* ctx, int kid, cudaStream_t stream);

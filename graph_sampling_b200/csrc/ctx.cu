@@ -23,6 +23,7 @@ struct gsb_ctx {
   u64 mail_tag;   // 1 .. 65535, of the last mailbox handed out
   u64 ticket;     // of the last counter fetch
   i64 launches;
+  i64 id_bound_refusals;
   char message[512];
   // per-kernel event timing (off by default)
   bool profiling;
@@ -338,6 +339,7 @@ int ctx_check_device_error(gsb_ctx* ctx, cudaStream_t stream) {
 }
 
 void ctx_count_launches(gsb_ctx* ctx, int n) { ctx->launches += n; }
+void ctx_count_id_bound_refusal(gsb_ctx* ctx) { ctx->id_bound_refusals += 1; }
 
 void ctx_prof_begin(gsb_ctx* ctx, int kid, cudaStream_t stream) {
   ctx->launches += 1;
@@ -501,6 +503,8 @@ int gsb_ctx_get_option(gsb_ctx* ctx, int option, int64_t* value_host) {
 }
 
 int64_t gsb_launch_count(gsb_ctx* ctx) { return ctx ? ctx->launches : 0; }
+
+int64_t gsb_id_bound_refusals(gsb_ctx* ctx) { return ctx ? ctx->id_bound_refusals : 0; }
 
 int gsb_read_counts(gsb_ctx* ctx, void* stream, int64_t* nnz_host, int64_t* unique_host) {
   GSB_ENTER(ctx);

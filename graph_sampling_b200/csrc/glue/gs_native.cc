@@ -302,7 +302,8 @@ FUNCTION(relabel, 3) {
 }
 
 // ---- relabelling of a sampled graph: (ctx, col_ids, rows, cols | None, indptr to copy | None, relabel, id bound)
-//      -> (unique, rows | None, cols | None, copy | None, ones | None), or None when gsb_graph_relabel does not serve the call
+//      -> (unique, rows | None, cols | None, copy | None, ones | None, whether the bound was refused), or that alone when
+//      gsb_graph_relabel does not serve the call
 FUNCTION(graph_relabel, 8) {
   gsb_ctx* ctx = context(a[0]);
   IDS(col_ids, a[1], "col_ids");
@@ -320,16 +321,18 @@ FUNCTION(graph_relabel, 8) {
   if (indptr.given()) copy = empty(indptr.numel(), dev);
   int64_t count = 0;
   int st;
+  const int64_t refusals = gsb_id_bound_refusals(ctx);
   {
     NoGil free;
     st = gsb_graph_relabel(ctx, stream(), col_ids.ids(), S, rows.ids(), E, cols.ids(), indptr.ids(), mut(copy),
                            indptr.given() ? indptr.numel() : 0, bound, mut(unique), mut(out_rows), mut(out_cols), mutf(ones), &count);
   }
-  if (st == GSB_ERR_UNSUPPORTED) Py_RETURN_NONE;
+  const long refused = gsb_id_bound_refusals(ctx) != refusals;
+  if (st == GSB_ERR_UNSUPPORTED) return PyBool_FromLong(refused);
   check(ctx, st, "gsb_graph_relabel");
   trim(unique, count);
   return tuple_of(wrap(std::move(unique)), wrap(std::move(out_rows)), wrap(std::move(out_cols)), wrap(std::move(copy)),
-                  wrap(std::move(ones)));
+                  wrap(std::move(ones)), PyBool_FromLong(refused));
 }
 
 // ---- random walk: (ctx, indptr, indices, seeds, length, seed, layout, walker_offset) -> trace [W, L + 1]

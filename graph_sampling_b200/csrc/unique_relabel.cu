@@ -261,6 +261,7 @@ extern "C" int gsb_graph_relabel(gsb_ctx* ctx, void* stream_, const int64_t* col
     if (st != GSB_OK) return st;
     st = ctx_mail_result(ctx, stream, mail, 1, &unique);
     if (bound == 0) break;
+    if (st == GSB_ERR_INDEX_RANGE) ctx_count_id_bound_refusal(ctx);
   }
   *unique_host = unique;
   return st == GSB_ERR_INDEX_RANGE ? GSB_ERR_UNSUPPORTED : st;  // ids beyond 32 bits: the general form takes them

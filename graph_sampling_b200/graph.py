@@ -37,6 +37,9 @@ class COO:
         self.row_sorted, self.col_sorted = row_sorted, col_sorted
 
 
+_NO_BOUND = ops.IdBound()
+
+
 def _fatal(msg):
     raise RuntimeError(msg)
 
@@ -49,17 +52,19 @@ class Graph:
         self.data_ = None
         self.col_ids_, self.row_ids_ = col_ids, row_ids
         self.val_col_ids_ = self.val_row_ids_ = None
-        self._id_bound = 0   # node ids of the loaded graph lie below it (0: unknown); a hint, inherited by its slices
+        self._id_bound = _NO_BOUND   # that of the loaded graph, shared with its slices
 
     # ---- loading (src/graph.cc:14-60) -------------------------------------------------------------
     def LoadCSC(self, indptr, indices):
         self.csc_ = CSC(indptr, indices)
-        self.num_cols_ = self.num_rows_ = self._id_bound = indptr.numel() - 1
+        self.num_cols_ = self.num_rows_ = indptr.numel() - 1
+        self._id_bound = ops.IdBound(self.num_cols_)
         self.num_edges_ = indices.numel()
 
     def LoadCSR(self, indptr, indices):
         self.csr_ = CSC(indptr, indices)
-        self.num_cols_ = self.num_rows_ = self._id_bound = indptr.numel() - 1
+        self.num_cols_ = self.num_rows_ = indptr.numel() - 1
+        self._id_bound = ops.IdBound(self.num_cols_)
         self.num_edges_ = indices.numel()
 
     def LoadCOO(self, row, col):
@@ -371,7 +376,7 @@ class Graph:
             frontier, (indices,) = ops.relabel([indices], [indices])
             new_row_ids, new_num_rows = frontier, frontier.numel()
         ret = self._child(new_col_ids, new_row_ids, n_ids.numel(), new_num_rows)
-        ret._id_bound = 0    # ids carry their batch number
+        ret._id_bound = _NO_BOUND    # ids carry their batch number
         ret.num_edges_ = indices.numel()
         if output_format & _CSC:
             ret.csc_ = CSC(indptr, indices)

@@ -290,18 +290,32 @@ def relabel(mapping_tensors, data_requiring_relabel, ctx=None):
     return ctx.native.relabel(ctx.address, mapping_tensors, data_requiring_relabel)
 
 
+class IdBound:
+    """Number that the node ids of a loaded graph lie below (0: not known), shared by the graph and all that is sliced from it.
+    The number of columns, which is the number of nodes only where rows and columns are numbered alike: the first call that
+    meets an id beyond it withdraws it for all of them, as each such call is launched twice."""
+    __slots__ = ("value",)
+
+    def __init__(self, value=0):
+        self.value = int(value)
+
+
 def graph_relabel(col_ids, rows, cols=None, indptr=None, ctx=None, id_bound=0, ones=False):
     """What Graph.Relabel does with a sampled graph (src/graph.cc:785-839) → (unique, relabelled rows, relabelled
     columns | None, copy of indptr | None): the frontier unique(cat(col_ids, rows)), every row id's position in it and,
     for a COO whose edge e lies in column cols[e], the position of col_ids[cols[e]].  With `ones` a fifth value: a float 1
-    per edge, the weights of a graph that has none, written by the same launch."""
+    per edge, the weights of a graph that has none, written by the same launch.  id_bound: a number or an IdBound, a hint."""
     ctx = _context_for(col_ids, ctx)
     on_device = indptr is None or indptr.is_cuda
-    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, cols, indptr if on_device else None, True, int(id_bound),
-                                   ones)
-    if out is not None:
+    shared = type(id_bound) is IdBound
+    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, cols, indptr if on_device else None, True,
+                                   id_bound.value if shared else int(id_bound), ones)
+    served = type(out) is tuple
+    if shared and (out[5] if served else out):
+        id_bound.value = 0
+    if served:
         out = out if on_device else out[:3] + (indptr.clone(),) + out[4:]
-        return out if ones else out[:4]
+        return out[:5] if ones else out[:4]
     if ones:
         return graph_relabel(col_ids, rows, cols, indptr, ctx, id_bound) + (
             torch.ones(rows.numel(), dtype=torch.float32, device=col_ids.device),)
@@ -313,10 +327,15 @@ def graph_relabel(col_ids, rows, cols=None, indptr=None, ctx=None, id_bound=0, o
 
 
 def graph_unique(col_ids, rows, ctx=None, id_bound=0):
-    """unique(cat(col_ids, rows)) in first-occurrence order; id_bound as in gsb_graph_relabel, a hint."""
+    """unique(cat(col_ids, rows)) in first-occurrence order; id_bound as in graph_relabel."""
     ctx = _context_for(col_ids, ctx)
-    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, None, None, False, int(id_bound), False)
-    return out[0] if out is not None else relabel([col_ids, rows], [], ctx)[0]
+    shared = type(id_bound) is IdBound
+    out = ctx.native.graph_relabel(ctx.address, col_ids, rows, None, None, False, id_bound.value if shared else int(id_bound),
+                                   False)
+    served = type(out) is tuple
+    if shared and (out[5] if served else out):
+        id_bound.value = 0
+    return out[0] if served else relabel([col_ids, rows], [], ctx)[0]
 
 
 def tensor_unique(node_ids, ctx=None):

@@ -213,7 +213,8 @@ GSB_API int gsb_unique_relabel(gsb_ctx* ctx, void* stream, const int64_t* const*
  * copy_n words from copy_src to copy_dst along the way (the offsets a CSC result hands out) and sets the E floats of
  * out_ones, unless it is NULL, to 1 (the edge weights of a graph without any).  out_unique holds S + E
  * entries; out_rows may be NULL when only the distinct ids are wanted.  id_bound > 0 is a hint that ids lie below it (a
- * graph knows its node count): it allows a direct-address table; ids beyond it cost a second launch, nothing else.
+ * graph knows its node count): it allows a direct-address table; ids beyond it cost a second launch, nothing else.  A
+ * caller that passes the same bound to every call withdraws it when gsb_id_bound_refusals has grown.
  * Waits for the number of distinct ids.  GSB_ERR_UNSUPPORTED — nothing usable was written — for calls beyond
  * 2^21 items or with ids of more than 32 bits, which gsb_unique_relabel serves.
  */
@@ -221,6 +222,8 @@ GSB_API int gsb_graph_relabel(gsb_ctx* ctx, void* stream, const int64_t* col_ids
                               int64_t E, const int64_t* cols, const int64_t* copy_src, int64_t* copy_dst,
                               int64_t copy_n, int64_t id_bound, int64_t* out_unique, int64_t* out_rows,
                               int64_t* out_cols, float* out_ones, int64_t* unique_host);
+/* Calls of gsb_graph_relabel through this context so far that met an id beyond their id_bound. */
+GSB_API int64_t gsb_id_bound_refusals(gsb_ctx* ctx);
 
 /* ---- uniform random walk ----------------------------------------------------------------------
  * Replaces gs::impl::fusion::FusedRandomWalkCUDA / _RandomWalkKernel

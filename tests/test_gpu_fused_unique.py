@@ -60,6 +60,29 @@ def test_ids_beyond_32_bits_take_the_general_form(ops, oracle):
     assert f.cpu().tolist() == [3, 7, 5]
 
 
+def test_a_bound_that_does_not_hold_is_withdrawn(ops, oracle):
+    """Ids of a rectangular graph lie beyond its number of columns: the first slice that meets one pays a second launch, the
+    others, and later slices of the same graph, do not."""
+    import graph_sampling_b200.gs as gs
+    rng = np.random.default_rng(3)
+    indptr, indices = np.arange(1001) * 20, rng.integers(0, 5000, 20_000)
+    graph = gs.Matrix().load_csc(dev(indptr), dev(indices))
+    launches = ops.default_context().launch_count
+    taken, slices = [], [graph[:, dev(np.arange(i, i + 100))] for i in range(3)]
+    for i, sub in enumerate(slices):
+        seeds, e = np.arange(i, i + 100), indices[i * 20:(i + 100) * 20]
+        want, (want_rows,) = oracle.unique_relabel([seeds, e], [e])
+        before = launches()
+        frontier, _, _, rows, _, _, fmt = sub._graph._CAPI_relabel()
+        taken.append(launches() - before)
+        assert fmt == "coo" and np.array_equal(frontier.cpu().numpy(), want) and np.array_equal(rows.cpu().numpy(), want_rows)
+        assert np.array_equal(sub._graph._CAPI_all_valid_node().cpu().numpy(), want)
+    assert taken == [2, 1, 1]
+    square = gs.Matrix().load_csc(dev(indptr), dev(indices % 1000))   # another graph's bound is its own
+    square[:, dev(np.arange(100))]._graph._CAPI_relabel()
+    assert square._graph._id_bound.value == 1000 and graph._graph._id_bound.value == 0
+
+
 @pytest.mark.parametrize("G,mean", [(1, 700), (2, 1), (7, 90_000), (40, 3000), (1500, 4), (3000, 300)])
 def test_batched_relabel_matches_oracle(ops, oracle, G, mean):
     rng = np.random.default_rng(G * 31 + mean)

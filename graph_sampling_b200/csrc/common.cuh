@@ -113,7 +113,6 @@ int ctx_tile_state(gsb_ctx* ctx, i64 num_tiles, cudaStream_t stream, TileState* 
 int count_scan_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, i64 num_cols, const i64* seeds, i64 S, i64 k,
                       int mode, i64* out_indptr, Mail mail = Mail{nullptr, 0});
 i64* ctx_counters(gsb_ctx* ctx);
-i64* ctx_pinned(gsb_ctx* ctx);
 int ctx_device(gsb_ctx* ctx);
 // GSB_OK when `ctx` is usable from the calling thread: non-null and created on the CUDA device that is current.
 // Every entry point starts with it, so a context is never driven from another device's stream by mistake.

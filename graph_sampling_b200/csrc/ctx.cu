@@ -210,7 +210,6 @@ int launch_cooperative(gsb_ctx* ctx, cudaStream_t stream, const void* kernel, in
 }
 
 i64* ctx_counters(gsb_ctx* ctx) { return ctx->counters; }
-i64* ctx_pinned(gsb_ctx* ctx) { return ctx->pinned; }
 int ctx_device(gsb_ctx* ctx) { return ctx->device; }
 
 // Waits for `stream`.  By default with cudaStreamSynchronize (the calling thread may spin); with

@@ -167,8 +167,8 @@ int direct_unique_relabel_launch(gsb_ctx* ctx, cudaStream_t stream, const BatchL
 // items, bit-vector ranking, no fix-up pass.  L carries seeds / seeds_ptr / indices / indices_ptr / G; item_off and
 // region_off (first bucket of every minibatch) must be filled by k_batch_layout; `ws` is scratch of
 // partition_workspace_bytes(n_cap, bucket_cap) bytes and begins with the per-bucket item counts.  counted = true: the
-// counts, bucket starts and the first item of every bucket's minibatch are already there (the sampler of the same hop
-// counted, partition_after_sampler did the rest) and the counting and scan passes are skipped.
+// counts and bucket starts are already there (the sampler of the same hop counted, partition_after_sampler did the
+// rest) and the counting and scan passes are skipped.
 i64 partition_bucket_capacity(i64 items_bound, i64 G);
 size_t partition_workspace_bytes(i64 n_cap, i64 bucket_cap);
 uint32_t* partition_bucket_counts(void* ws);

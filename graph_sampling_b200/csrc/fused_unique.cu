@@ -30,6 +30,8 @@
 // GPU time of a call, five launches (without the gaps between them) / hash table / direct table: 16 000 items
 // 26 / 11 / 7 us, 813 000 items 86 / 51 / 29 us.  What bounds the hash table (813 000 items): bucket reads and
 // compare-and-swaps at the rate of the L2's atomics, 107 G/s each, and the rounds of the slowest lanes behind them.
+// Two CTAs per SM leave 64 registers a thread: eight and sixteen items per thread partly live in local memory (70 to 660
+// bytes loaded and stored per thread).
 #include "batch_table.cuh"
 #include "common.cuh"
 #include "grid_sync.cuh"

@@ -237,8 +237,7 @@ __global__ void __launch_bounds__(kScanThreads) k_part_scan(PartLayout P, i64* c
 
 // The one-call hop, between its sampler and the scatter pass — one CTA does what three small launches did: the edge
 // offset of every minibatch (the sampled block's offset at the minibatch's first seed), the item offsets, the abort
-// check against the caller's bounds, the first item of every bucket's minibatch, and the scan of the bucket sizes that
-// the sampler counted.
+// check against the caller's bounds, and the scan of the bucket sizes that the sampler counted.
 __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const i64* __restrict__ sub_indptr, i64 S,
                                                              i64 edges_bound, i64* indices_ptr, i64* counters) {
   __shared__ i64 s_scan[33];
@@ -299,9 +298,9 @@ __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const
 // THREADS x PER items per tile.  Tiles of 2 048 suit minibatches of some ten thousand items (a tile that straddles
 // minibatches takes the per-item path); with hundreds of buckets per minibatch such a tile reserves a range — a global
 // atomic, on a cursor that every other tile of the minibatch wants too — for every five items, so large minibatches take
-// tiles of 8 192, two of whose CTAs are resident per SM (with the 83 registers the compiler takes of its own accord one is, and
-// its barriers leave the SM idle: 3.1 against 2.1 ms for 270 M items; 1 024 threads with half the items each 2.8, tiles of
-// 4 096 2.7).
+// tiles of 8 192, two of whose CTAs are resident per SM.  That costs 300 bytes of spilled registers a thread (with the 83
+// registers the compiler takes of its own accord one CTA is resident, and its barriers leave the SM idle: 3.1 against 2.1 ms for
+// 270 M items; 1 024 threads with half the items each 2.8, tiles of 4 096 2.7).
 template <int WINDOW, int THREADS, int PER>
 __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatter(PartLayout P, i64 n_bound, i64* counters) {
   constexpr int kTile = THREADS * PER;

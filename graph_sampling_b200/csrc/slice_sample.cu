@@ -1,15 +1,13 @@
 // Column slicing and uniform per-column sampling (plain and fused with slicing).
 //
 // Data layout: the graph is CSC in HBM (int64 indptr[n+1], int64 indices[nnz]); a call works on a
-// list of S seed columns.  Columns are grouped into tiles of kTileCols consecutive seeds, one CTA
-// per tile.  A CTA (1) stages the tile's (start, degree, count) triples in shared memory with one
-// coalesced read of the seed list and one gathered read of the indptr pairs, (2) scans the counts
-// in shared memory and obtains the tile's output offset by decoupled look-back, (3) produces the
-// outputs.  Slicing copies by OUTPUT position (each thread finds its column by binary search in
-// the shared offsets), so hub columns are spread over the whole CTA; sampling gives each column a
-// group of G lanes, G = smallest power of two >= fanout, and needs O(fanout) draws per column
-// whatever its degree (Floyd's k-subset), instead of the reference's O(degree) reservoir pass
-// (src/cuda/fusion/slice_sampling.cu:62-75).
+// list of S seed columns.  Slicing is a counting pass (degrees and their scan by decoupled look-back)
+// and a copy by OUTPUT position, a stretch of positions per warp (column_walk.cuh), so hub columns are
+// spread over the grid.  Sampling is one launch: counts, their scan and the picks.  Fan-outs up to 16
+// give each column a lane and each warp a tile of 32 columns; larger ones group columns into tiles of
+// kTileCols per CTA, whose (start, degree, count) triples are staged in shared memory, and give each
+// column a group of 32 lanes.  Either needs O(fanout) draws per column whatever its degree (Floyd's
+// k-subset), instead of the reference's O(degree) reservoir pass (src/cuda/fusion/slice_sampling.cu:62-75).
 #include "batch_table.cuh"
 #include "column_walk.cuh"
 #include "common.cuh"
@@ -121,7 +119,8 @@ struct FillParams {
 // The OUTPUT positions are cut into one stretch per warp, whatever columns they belong to: a hub column is spread over the
 // grid, and a call with few, long columns fills it as well as one with many short ones.  A warp finds the columns of 192
 // positions at a time (column_walk.cuh) and requests all their ids and data before it writes any.
-// What bounds it is HBM and the positions in flight per SM, and anything spilled costs more than the resident warps it buys:
+// What bounds it is HBM and the positions in flight per SM against the registers they take (64 at 8 CTAs per SM; the forms with
+// edge ids or batch numbers spill 4 to 36 bytes there):
 // 262 144 columns with 13.2 M edges, weights and column ids: 92 us with six positions per lane and 8 CTAs per SM; eight
 // positions and 8 / 7 / 9 / 10 CTAs 94 / 99 / 142 / 147, four and 10 CTAs 132.  Tiles of 1 024 positions whose columns a CTA
 // keeps in shared memory, two barriers and two searches each: 105 us, and 16 instead of 5 us for the slices of layer-wise

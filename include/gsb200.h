@@ -89,17 +89,18 @@ GSB_API int gsb_check_device_status(gsb_ctx* ctx, void* stream);
  *                               in several minibatches), else
  *                               direct-address tables when all tables of the call are L2-sized (32 MiB), else the
  *                               partitioned form (items bucketed by a hash of their id, one shared-memory table per
- *                               bucket) for calls of at least 2^19 items whose minibatches average at most 2^19
+ *                               bucket) for calls of at least 2^19 items whose minibatches average at most 2^21
  *                               items, and hash-table regions otherwise;
  *                               1 = hash-table regions in global memory, one per minibatch;
  *                               2 = direct-address tables (GSB_ERR_OUT_OF_MEMORY when they do not fit);
  *                               3 = the partitioned form.  Results are identical;
  *  GSB_OPT_DIRECT_TABLE_BUDGET  bytes the direct-address tables (8 bytes x num_nodes x minibatches per call) may
  *                               take, default 6 GiB;
- *  GSB_OPT_BLOCKING_WAIT        1: calls that wait for their stream (the ones with a *_host result) sleep on an event
- *                               created with cudaEventBlockingSync instead of calling cudaStreamSynchronize, which
- *                               may spin — for hosts that drive several streams from several threads, or several
- *                               processes per machine; default 0. */
+ *  GSB_OPT_BLOCKING_WAIT        1: calls that wait for a result (the ones with a *_host argument) sleep until their
+ *                               stream is done, on an event created with cudaEventBlockingSync, instead of spinning
+ *                               on the word in page-locked memory that the kernel leaves the result in — for hosts
+ *                               that drive several streams from several threads, or several processes per machine;
+ *                               default 0. */
 enum gsb_option {
   GSB_OPT_MAX_POLLS = 0,
   GSB_OPT_TABLE_SLOTS = 1,

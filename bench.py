@@ -22,8 +22,8 @@ Prints ONE JSON line (rank 0):
   roofline    per-kernel CUDA-event times from a separate untimed step; algorithmic bytes over the measured HBM peak;
   secondary   short legs of the other configurations (2-hop small graph, layer-wise, random walk, adaptive).
 `--impl reference` times the reference's own implementation of the same steps: its CUDA library compiled unmodified
-for sm_100 (oracle/_ref/libgs_ref.so) if it is present, because the reference has no CPU path; otherwise the CPU
-restatement on the host cores.
+for sm_100 (oracle/_ref/libgs_ref.so).  The reference has no CPU path, so without that library the arm is reported as
+unavailable.
 """
 import argparse
 import json
@@ -671,87 +671,86 @@ def dropin_torchscript(torch, args, device, indptr, indices, pinned, lib_path=No
 def run_reference(args):
     """Reference arm.  The reference implements this path in CUDA only (every dispatcher aborts off-GPU), so its own
     implementation — its sources compiled unmodified for sm_100 — is timed on the GPU through its TorchScript classes
-    with its own loops, on the same steps; if the compiled library is absent the CPU restatement is timed on the host
-    cores instead."""
+    with its own loops, on the same steps.  Where that library is absent there is nothing to time: the CPU restatement
+    (`cpu_baseline` of the other arm) is this repository's own code."""
     rank, world, local = dist_env()
     if rank != 0:
         return
     import torch
     lib = os.path.join(ROOT, "oracle", "_ref", "libgs_ref.so")
+    if not os.path.exists(lib):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libgs_ref.so is not built: the reference's "
+                                                              "sources are not mounted (oracle/build_ref.sh)"}))
+        return
     torch.cuda.set_device(local)
     device = torch.device("cuda", local)
     indptr, indices, batches, _, info, gen_s = make_inputs(args, device, 1, 0)
     base = {"metric": METRIC, "unit": UNIT, "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int64", "data": "synthetic",
             "impl": "reference", "config": workload_config(args, info)}
-    if os.path.exists(lib):
-        pinned = batches.pin_memory()
-        sampler = ClockSampler(physical_gpu_index(local))
-        sampler.start()
-        torch.classes.load_library(lib)
-        G = torch.classes.gs_classes.Graph(False)
-        G._CAPI_LoadCSC(indptr, indices)
-        ptr_cache = {}
+    pinned = batches.pin_memory()
+    sampler = ClockSampler(physical_gpu_index(local))
+    sampler.start()
+    torch.classes.load_library(lib)
+    G = torch.classes.gs_classes.Graph(False)
+    G._CAPI_LoadCSC(indptr, indices)
+    ptr_cache = {}
 
-        def call(sb, first, step_no, lane=0):
-            g, s0 = sb.shape
-            ptr = ptr_cache.get(g)
-            if ptr is None:
-                ptr = ptr_cache[g] = torch.arange(g + 1, dtype=torch.int64, device=device) * s0
-            return superbatch_torchscript(torch, G, sb.reshape(-1), ptr)
+    def call(sb, first, step_no, lane=0):
+        g, s0 = sb.shape
+        ptr = ptr_cache.get(g)
+        if ptr is None:
+            ptr = ptr_cache[g] = torch.arange(g + 1, dtype=torch.int64, device=device) * s0
+        return superbatch_torchscript(torch, G, sb.reshape(-1), ptr)
 
-        # its super-batch loop at this run's group size and at the 256-ish size its examples use: one trial step
-        # each, the faster one is measured in full
-        trial = {}
-        for group in sorted({args.group, 250, 125}):
-            st = Stepper(torch, call, pinned, group, device)
-            sec, e = timed_steps(torch, st, 1, 1, lambda: None, float, min_seconds=0.0, min_repeats=1, max_repeats=1)
-            trial[group] = e / sec[0]
-        group = max(trial, key=trial.get)
+    # its super-batch loop at this run's group size and at the 256-ish size its examples use: one trial step
+    # each, the faster one is measured in full
+    trial = {}
+    for group in sorted({args.group, 250, 125}):
         st = Stepper(torch, call, pinned, group, device)
-        seconds, edges = timed_steps(torch, st, args.warmup, args.steps, lambda: None, float, min_seconds=0.5,
-                                     min_repeats=1, max_repeats=3)
-        sec_med = median(seconds)
-        batched = edges / sec_med
-        # its per-minibatch Graph loop on a bounded sample
-        n = min(pinned.shape[0], 500)
-        for b in range(5):
-            sage_batch_api(G, pinned[b].to(device, non_blocking=True), "_CAPI_FusedColumnwiseSlicingSampling", "_CAPI_Relabel")
-        torch.cuda.synchronize()
-        ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        ev0.record()
-        pb_edges = 0
-        for b in range(n):
-            e, _ = sage_batch_api(G, pinned[b].to(device, non_blocking=True), "_CAPI_FusedColumnwiseSlicingSampling",
-                                  "_CAPI_Relabel")
-            pb_edges += e
-        ev1.record()
-        torch.cuda.synchronize()
-        pb_sec = ev0.elapsed_time(ev1) / 1e3
-        per_batch = pb_edges / pb_sec
-        clocks = sampler.stop()
-        if batched >= per_batch:
-            v, ms_step = batched, sec_med / args.steps * 1e3
-        else:
-            v, ms_step = per_batch, pb_sec / n * args.batches_per_step * 1e3
-        base["arm"] = {"reference_paths": {"per_batch_graph_api_edges_per_s": per_batch,
-                                           "super_batch_edges_per_s": batched, "super_batch_group": group,
-                                           "super_batch_trials_edges_per_s": trial,
-                                           "reported": "super-batch" if batched >= per_batch else "per-batch"},
-                       "graph_gen_seconds": gen_s, "repeats": len(seconds)}
-        base.update({"value": v, "ms_per_step": ms_step, "clocks": clocks,
-                     "cpu_baseline": {"value": v, "unit": UNIT, "cores": 0, "kind": "reference",
-                                      "sample": "the reference has no CPU path; this is its own CUDA library "
-                                                "(unmodified sources compiled for sm_100) on the same GPU, "
-                                                f"{args.steps} steps of {args.batches_per_step} minibatches"},
-                     "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}})
-        if args.secondary:
-            del pinned
-            base["secondary"] = secondary_workloads(args, "reference", device, indptr, indices)
+        sec, e = timed_steps(torch, st, 1, 1, lambda: None, float, min_seconds=0.0, min_repeats=1, max_repeats=1)
+        trial[group] = e / sec[0]
+    group = max(trial, key=trial.get)
+    st = Stepper(torch, call, pinned, group, device)
+    seconds, edges = timed_steps(torch, st, args.warmup, args.steps, lambda: None, float, min_seconds=0.5,
+                                 min_repeats=1, max_repeats=3)
+    sec_med = median(seconds)
+    batched = edges / sec_med
+    # its per-minibatch Graph loop on a bounded sample
+    n = min(pinned.shape[0], 500)
+    for b in range(5):
+        sage_batch_api(G, pinned[b].to(device, non_blocking=True), "_CAPI_FusedColumnwiseSlicingSampling", "_CAPI_Relabel")
+    torch.cuda.synchronize()
+    ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    ev0.record()
+    pb_edges = 0
+    for b in range(n):
+        e, _ = sage_batch_api(G, pinned[b].to(device, non_blocking=True), "_CAPI_FusedColumnwiseSlicingSampling",
+                              "_CAPI_Relabel")
+        pb_edges += e
+    ev1.record()
+    torch.cuda.synchronize()
+    pb_sec = ev0.elapsed_time(ev1) / 1e3
+    per_batch = pb_edges / pb_sec
+    clocks = sampler.stop()
+    if batched >= per_batch:
+        v, ms_step = batched, sec_med / args.steps * 1e3
     else:
-        cpu = cpu_baseline(indptr, indices, batches, limit_s=60.0)
-        base.update({"value": cpu["value"], "ms_per_step": None, "cpu_baseline": cpu,
-                     "e2e": {"value": cpu["value"], "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}})
+        v, ms_step = per_batch, pb_sec / n * args.batches_per_step * 1e3
+    base["arm"] = {"reference_paths": {"per_batch_graph_api_edges_per_s": per_batch,
+                                       "super_batch_edges_per_s": batched, "super_batch_group": group,
+                                       "super_batch_trials_edges_per_s": trial,
+                                       "reported": "super-batch" if batched >= per_batch else "per-batch"},
+                   "graph_gen_seconds": gen_s, "repeats": len(seconds)}
+    base.update({"value": v, "ms_per_step": ms_step, "clocks": clocks,
+                 "cpu_baseline": {"value": v, "unit": UNIT, "cores": 0, "kind": "reference",
+                                  "sample": "the reference has no CPU path; this is its own CUDA library "
+                                            "(unmodified sources compiled for sm_100) on the same GPU, "
+                                            f"{args.steps} steps of {args.batches_per_step} minibatches"},
+                 "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}})
+    if args.secondary:
+        del pinned
+        base["secondary"] = secondary_workloads(args, "reference", device, indptr, indices)
     print(json.dumps(base))
 
 
@@ -1185,7 +1184,8 @@ def run_kernels(args):
     x = torch.randn(n, F, generator=g, device=device)
     xd = x[seeds]
     out = torch.zeros(D, 1, device=device)
-    timed("SDDMM dot, F = 256", lambda: ops.sddmm("dot", x, xd, out, 0, 2, sub_row, sub_col), D * (4 * F + 20) + S * 4 * F)
+    timed("SDDMM dot, F = 256", lambda: ops.sddmm("dot", x, xd, out, 0, 2, sub_row, sub_col), D * (4 * F + 20) + S * 4 * F,
+          note="a row per edge is counted; rows that several edges share come from L2, so this can exceed the copy bandwidth")
     w = torch.rand(D, generator=g, device=device)
     o1 = torch.zeros(S, device=device)
     timed("segment sum of squares (CSC)", lambda: ops.csc_sum(sub_indptr, None, w, o1, 2), 12 * D + 4 * S)
@@ -1205,7 +1205,7 @@ def run_kernels(args):
     lp[torch.rand(1_000_000, generator=g, device=device) < 0.5] = 0
     ld = torch.arange(1_000_000, device=device)
     timed("list sampling, 512 of 1 M weighted", lambda: ops.list_sampling(ld, 512, False, probs=lp), 12 * 1_000_000 + 16 * 512,
-          note="12 launches; bound by host launch time")
+          note="one cooperative launch; grid barriers")
     # ---- feature load, induced subgraph, metapath walk, super-batch operators --------------------------------
     fr = torch.randint(0, n, (1_000_000,), generator=g, device=device)
     timed("feature rows gather, F = 256 (1 M rows)", lambda: ops.gather_rows(x, fr), fr.numel() * (8 + 8 * F))

@@ -401,7 +401,7 @@ int gsb_batch_list_sample(gsb_ctx* ctx, void* stream_, const float* probs, int64
   // of the workspace (which a larger reservation would move) is copied nowhere: the candidate arrays come first
   const size_t pair_bytes = ((size_t)N * 8 + 255) & ~(size_t)255;
   void* ws;
-  int st = ctx_reserve_workspace(ctx, 2 * pair_bytes + radix_sort_scratch_bytes(N) + fixed, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, 2 * pair_bytes + radix_sort_scratch_bytes(N) + fixed, &ws);
   if (st != GSB_OK) return st;
   u64* cand_keys = (u64*)ws;
   i64* cand_vals = (i64*)((char*)ws + pair_bytes);

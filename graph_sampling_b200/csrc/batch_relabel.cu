@@ -680,7 +680,7 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   void* ws;
   if (tables) {
     const size_t rank_bytes = ((size_t)n_cap * 4 + 255) & ~(size_t)255;
-    int st = ctx_reserve_workspace(ctx, off_bytes + rank_bytes, &ws);
+    int st = ctx_reserve_workspace(ctx, stream, off_bytes + rank_bytes, &ws);
     if (st != GSB_OK) return st;
     L.item_off = (i64*)ws;
     L.region_off = nullptr;
@@ -703,7 +703,7 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   if (path == 3 || (path == 0 && partition_suits(n_cap, G))) {
     // partitioned form (the default for large calls when the direct-address tables above were not chosen): shared-memory tables per bucket of items, then ranking by bit vectors
     const i64 bucket_cap = partition_bucket_capacity(n_cap, G);
-    int st = ctx_reserve_workspace(ctx, 3 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
+    int st = ctx_reserve_workspace(ctx, stream, 3 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
     if (st != GSB_OK) return st;
     L.item_off = (i64*)ws;
     L.region_off = (i64*)((char*)ws + off_bytes);
@@ -726,7 +726,7 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   const i64 slot_cap = region_size_for(n_cap) + 32 * G + 64;
   const size_t slots_bytes = ((size_t)slot_cap * 8 + 255) & ~(size_t)255;
   const size_t rank_bytes = ((size_t)n_cap * 4 + 255) & ~(size_t)255;
-  int st = ctx_reserve_workspace(ctx, slots_bytes + 2 * off_bytes + rank_bytes, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, slots_bytes + 2 * off_bytes + rank_bytes, &ws);
   if (st != GSB_OK) return st;
   L.slots = (u64*)ws;
   L.item_off = (i64*)((char*)ws + slots_bytes);
@@ -774,7 +774,7 @@ static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64*
   const size_t off_bytes = ((size_t)(G + 1) * 8 + 255) & ~(size_t)255;
   const i64 bucket_cap = partition_bucket_capacity(S * (1 + k), G);
   void* ws;
-  int st = ctx_reserve_workspace(ctx, 2 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
+  int st = ctx_reserve_workspace(ctx, stream, 2 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
   if (st != GSB_OK) return st;
   void* part_ws = (char*)ws + 2 * off_bytes;
   BatchLayout L;
@@ -943,7 +943,7 @@ static int build_batch_tables(gsb_ctx* ctx, cudaStream_t stream, const i64* seed
   const size_t slots_bytes = ((size_t)slot_cap * 8 + 255) & ~(size_t)255;
   const size_t off_bytes = ((size_t)(G + 1) * 8 + 255) & ~(size_t)255;
   void* ws;
-  int st = ctx_reserve_workspace(ctx, slots_bytes + 3 * off_bytes + 256 + extra_bytes, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, slots_bytes + 3 * off_bytes + 256 + extra_bytes, &ws);
   if (st != GSB_OK) return st;
   BatchLayout L;
   L.seeds = seeds;
@@ -1037,7 +1037,7 @@ int gsb_batch_unique(gsb_ctx* ctx, void* stream_, const int64_t* data, const int
   // first copy of every key (the reference segment-sorts and runs unique-by-key: src/cuda/batch_unique.cu:215-260)
   const size_t key_bytes = ((size_t)n * 8 + 255) & ~(size_t)255;
   void* ws;
-  int st = ctx_reserve_workspace(ctx, key_bytes + radix_sort_scratch_bytes(n) + 256, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, key_bytes + radix_sort_scratch_bytes(n) + 256, &ws);
   if (st != GSB_OK) return st;
   u64* keys = (u64*)ws;
   void* sort_ws = (char*)ws + key_bytes;
@@ -1148,7 +1148,7 @@ int unique_relabel_packed(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i
   const i64 region = region_size_for(n_cap);
   const i64 slot_cap = region + 64;
   const size_t slots_bytes = ((size_t)slot_cap * 8 + 255) & ~(size_t)255;
-  int st = ctx_reserve_workspace(ctx, slots_bytes + 4 * 256, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, slots_bytes + 4 * 256, &ws);
   if (st != GSB_OK) return st;
   BatchLayout L;
   L.seeds = first;

@@ -42,6 +42,8 @@ struct gsb_ctx {
   void* epoch_table[2];
   size_t epoch_bytes[2];
   uint32_t table_epoch[2];
+  cudaStream_t stream;   // of the last call that used scratch
+  bool stream_known;
   u64 barrier_arrivals;  // the barrier word itself is counters[CNT_NUM]
   cudaEvent_t wait_event;  // created on first use when GSB_OPT_BLOCKING_WAIT is set
 };
@@ -53,7 +55,19 @@ int cuda_fail(gsb_ctx* ctx, cudaError_t e, const char* file, int line) {
   return e == cudaErrorMemoryAllocation ? GSB_ERR_OUT_OF_MEMORY : GSB_ERR_CUDA;
 }
 
-int ctx_reserve_workspace(gsb_ctx* ctx, size_t bytes, void** out) {
+// Scratch, look-back words and tables hold one call's work at a time.  A call returns as soon as the size it reports is known,
+// while its last kernel may still use them, so the next call must come behind it in stream order.  Where it comes on another
+// stream the host waits for the device: not for the stream of the call before, which may have been destroyed since.
+static int ctx_on_stream(gsb_ctx* ctx, cudaStream_t stream) {
+  if (ctx->stream_known && ctx->stream != stream) GSB_CUDA_OK(cudaDeviceSynchronize());
+  ctx->stream = stream;
+  ctx->stream_known = true;
+  return GSB_OK;
+}
+
+int ctx_reserve_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, void** out) {
+  const int st = ctx_on_stream(ctx, stream);
+  if (st != GSB_OK) return st;
   if (bytes > ctx->workspace_bytes) {
     // Growing synchronises the device; it only happens the first time a size is seen.
     GSB_CUDA_OK(cudaDeviceSynchronize());
@@ -75,6 +89,8 @@ int ctx_reserve_workspace(gsb_ctx* ctx, size_t bytes, void** out) {
 }
 
 int ctx_tile_state(gsb_ctx* ctx, i64 num_tiles, cudaStream_t stream, TileState* out) {
+  const int st = ctx_on_stream(ctx, stream);
+  if (st != GSB_OK) return st;
   if (num_tiles > ctx->tile_capacity) {
     GSB_CUDA_OK(cudaDeviceSynchronize());
     if (ctx->tile_words) GSB_CUDA_OK(cudaFree(ctx->tile_words));
@@ -119,6 +135,8 @@ int ctx_direct_tables(gsb_ctx* ctx, i64 count, i64 num_nodes, cudaStream_t strea
   *out_epoch = 0;
   if (count <= 0 || num_nodes <= 0) return GSB_OK;
   if ((double)count * (double)num_nodes * 8.0 > (double)ctx->options[GSB_OPT_DIRECT_TABLE_BUDGET]) return GSB_OK;
+  const int st = ctx_on_stream(ctx, stream);
+  if (st != GSB_OK) return st;
   const size_t bytes = (size_t)count * (size_t)num_nodes * sizeof(u64);
   if (bytes > ctx->direct_bytes) {
     // Growing synchronises the device; it only happens the first time a (batches x nodes) size is seen.

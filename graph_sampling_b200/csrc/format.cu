@@ -367,7 +367,7 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
       const size_t item_bytes = p.digits > 1 ? al(sizeof(u64) * (size_t)E) : 0;
       const size_t matrix_bytes = al(sizeof(u32) * (size_t)bins * (size_t)conv_grid);
       void* ws;
-      int st = ctx_reserve_workspace(ctx, item_bytes * (p.digits > 2 ? 2 : 1) + matrix_bytes + al(sizeof(u32) * (size_t)bins) +
+      int st = ctx_reserve_workspace(ctx, stream, item_bytes * (p.digits > 2 ? 2 : 1) + matrix_bytes + al(sizeof(u32) * (size_t)bins) +
                                               al(sizeof(u32) * (size_t)num_keys) + 4096, &ws);
       if (st != GSB_OK) return st;
       char* at = (char*)ws;
@@ -412,7 +412,7 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
   }
   void* ws;
   const size_t sort_bytes = radix_sort_scratch_bytes(E);
-  st = ctx_reserve_workspace(ctx, sort_bytes + sizeof(u64) * (size_t)E + 256, &ws);
+  st = ctx_reserve_workspace(ctx, stream, sort_bytes + sizeof(u64) * (size_t)E + 256, &ws);
   if (st != GSB_OK) return st;
   u64* keys = (u64*)((char*)ws + sort_bytes);
   k_make_sort_input<<<grid, kFmtThreads, 0, stream>>>(key, E, keys, out_perm);

@@ -505,7 +505,7 @@ static int launch_fused(gsb_ctx* ctx, cudaStream_t stream, FusedParams p, i64 n,
   const bool direct = fused_unique_direct(G, id_bound);
   void* ws;
   const size_t packed_bytes = ((size_t)n / 32 + 2) * 8;
-  int st = ctx_reserve_workspace(ctx, packed_bytes + sizeof(u32) * (size_t)(kFuThreads + (p.col_index ? p.S : 0)), &ws);
+  int st = ctx_reserve_workspace(ctx, stream, packed_bytes + sizeof(u32) * (size_t)(kFuThreads + (p.col_index ? p.S : 0)), &ws);
   if (st != GSB_OK) return st;
   p.packed = (u64*)ws;
   p.totals = (u32*)((char*)ws + packed_bytes);

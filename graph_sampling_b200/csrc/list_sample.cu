@@ -435,7 +435,7 @@ extern "C" int gsb_list_sample(gsb_ctx* ctx, void* stream_, const int64_t* data,
   if (replace) {
     const i64 chunks = (N + kCdfChunk - 1) / kCdfChunk;
     void* ws;
-    int st = ctx_reserve_workspace(ctx, sizeof(double) * (size_t)(chunks + 1), &ws);
+    int st = ctx_reserve_workspace(ctx, stream, sizeof(double) * (size_t)(chunks + 1), &ws);
     if (st != GSB_OK) return st;
     double* chunk_pre = (double*)ws;
     k_cdf_chunk_sums<<<(int)chunks, kListThreads, 0, stream>>>(probs, N, chunk_pre);
@@ -453,7 +453,7 @@ extern "C" int gsb_list_sample(gsb_ctx* ctx, void* stream_, const int64_t* data,
   if (k <= kSelectMaxK && ctas > 0) {
     const size_t bytes = ((size_t)N * 8 + 255) & ~(size_t)255;
     void* ws;
-    int st = ctx_reserve_workspace(ctx, bytes + kSelectMaxK * 8 + sizeof(unsigned) * (kSelectPasses * kSelectBins + 64), &ws);
+    int st = ctx_reserve_workspace(ctx, stream, bytes + kSelectMaxK * 8 + sizeof(unsigned) * (kSelectPasses * kSelectBins + 64), &ws);
     if (st != GSB_OK) return st;
     SelectParams p{};
     p.probs = probs;
@@ -480,7 +480,7 @@ extern "C" int gsb_list_sample(gsb_ctx* ctx, void* stream_, const int64_t* data,
   const size_t win_bytes = ((size_t)k * 16 + 255) & ~(size_t)255;  // winners + index payload for the sort
   const size_t sort_bytes = radix_sort_scratch_bytes(k);
   void* ws;
-  int st = ctx_reserve_workspace(ctx, comp_bytes + win_bytes + sort_bytes + 4096, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, comp_bytes + win_bytes + sort_bytes + 4096, &ws);
   if (st != GSB_OK) return st;
   u64* composite = (u64*)ws;
   u64* winners = (u64*)((char*)ws + comp_bytes);

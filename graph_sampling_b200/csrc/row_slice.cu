@@ -519,7 +519,7 @@ static int build_table(gsb_ctx* ctx, cudaStream_t stream, const int64_t* row_ids
   const size_t bloom_bytes = bloom ? ((size_t)1 << bits_log2) / 8 : 0;
   void* ws;
   const size_t table_bytes = cap * sizeof(Slot) + bloom_bytes;
-  int st = ctx_reserve_workspace(ctx, table_bytes + extra_bytes + 256, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, table_bytes + extra_bytes + 256, &ws);
   if (st != GSB_OK) return st;
   table->slots = (Slot*)ws;
   *extra = (char*)ws + table_bytes;
@@ -611,7 +611,7 @@ static int col_row_table(gsb_ctx* ctx, cudaStream_t stream, const int64_t* row_i
   table->mask = cap - 1;
   void* ws;
   const size_t table_bytes = cap * sizeof(Slot);
-  int st = ctx_reserve_workspace(ctx, table_bytes + 256, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, table_bytes + 256, &ws);
   if (st != GSB_OK) return st;
   table->slots = (Slot*)ws;
   GSB_CUDA_OK(cudaMemsetAsync(table->slots, 0xFF, table_bytes, stream));

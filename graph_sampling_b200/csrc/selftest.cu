@@ -100,7 +100,7 @@ extern "C" int gsb_selftest_table_atomics(gsb_ctx* ctx, void* stream_, int where
   if (cluster_size > 8) GSB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   const uint32_t global_slots = 4u << 20;  // 32 MB: stays in L2
   void* ws;
-  int st = ctx_reserve_workspace(ctx, (size_t)global_slots * 8 + 256, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, (size_t)global_slots * 8 + 256, &ws);
   if (st != GSB_OK) return st;
   u64* table = (u64*)ws;
   u64* sink = table + global_slots;

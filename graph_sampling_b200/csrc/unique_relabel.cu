@@ -204,7 +204,7 @@ extern "C" int gsb_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* co
   }
   table.mask = cap - 1;
   void* ws;
-  st = ctx_reserve_workspace(ctx, cap * sizeof(Slot), &ws);
+  st = ctx_reserve_workspace(ctx, stream, cap * sizeof(Slot), &ws);
   if (st != GSB_OK) return st;
   table.slots = (Slot*)ws;
   {

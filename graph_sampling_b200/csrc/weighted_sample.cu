@@ -804,7 +804,7 @@ extern "C" int gsb_sample_weighted(gsb_ctx* ctx, void* stream_, const int64_t* i
   size_t total_bytes = 0;
   for (size_t n : sizes) total_bytes += n;
   void* ws;
-  int st = ctx_reserve_workspace(ctx, total_bytes, &ws);
+  int st = ctx_reserve_workspace(ctx, stream, total_bytes, &ws);
   if (st != GSB_OK) return st;
   at[0] = (char*)ws;
   for (int i = 1; i < 7; ++i) at[i] = at[i - 1] + sizes[i - 1];

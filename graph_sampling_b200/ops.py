@@ -59,8 +59,9 @@ def next_seed(seed=None):
 
 
 class Context:
-    """Owns one gsb_ctx (scratch arena, counters).  Calls through one Context must be ordered on
-    one stream; create one Context per stream for concurrent work."""
+    """Owns one gsb_ctx (scratch arena, counters).  Calls through one Context come one after the other: on another stream
+    than the last one's a call that uses scratch first waits for the device.  Create one Context per stream for concurrent
+    work."""
 
     def __init__(self, device=None):
         if not torch.cuda.is_available():

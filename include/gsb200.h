@@ -9,7 +9,8 @@
  *  - ids and offsets are int64, weights / features / edge data are float (the only instantiation
  *    of the reference: src/cuda/slicing.cu:176, src/cuda/sampling_probs.cu:274);
  *  - `stream` is a cudaStream_t passed as void*; work is enqueued on it and the call returns
- *    without waiting, except where a size has to be reported to the host (documented per call);
+ *    without waiting, except where a size has to be reported to the host (documented per call;
+ *    "waits for" a size or count means just that);
  *  - the return value is a status code (0 = GSB_OK); nothing aborts the process (the reference
  *    LOG(FATAL)s: src/cuda/cuda_common.h:15-28);
  *  - inputs are borrowed and never modified; outputs are caller-allocated;
@@ -17,7 +18,10 @@
  *  - a call that reports a size to the host returns as soon as the size is known, which may be a little before its last
  *    kernel has finished: outputs are complete in stream order, as after any launch;
  *  - a gsb_ctx owns scratch memory and device-side counters for ONE stream of work at a time:
- *    calls sharing a context must be ordered on one stream (use one context per stream/thread).
+ *    calls sharing a context must be ordered on one stream (use one context per stream/thread).  A call of the
+ *    context's thread on another stream than the last one's is ordered behind it by waiting for the whole device;
+ *    calls through a context are not for capture into a CUDA graph (scratch may move, and a launch carries numbers
+ *    that the next one may not repeat): gsb_unique_relabel_static is;
  *    Scratch grows on demand with cudaMalloc the first time a size is seen (this synchronises the
  *    device once); steady-state calls allocate nothing;
  *  - a context belongs to the CUDA device it was created on: every entry point checks that this device is
@@ -25,7 +29,7 @@
  *  - seed / column / walker ids are checked against `num_cols` (the number of columns of the operand,
  *    indptr has num_cols + 1 entries) on the device: an id outside [0, num_cols) counts as an empty column
  *    (or ends a walk with -1), its offsets are never read, and GSB_ERR_INDEX_RANGE is recorded in the context
- *    (returned by the same call when it waits for the stream, else by gsb_check_device_status).  The reference
+ *    (returned by the same call when it waits for a size, else by gsb_check_device_status).  The reference
  *    reads indptr[id] unchecked (src/cuda/slicing.cu:133-141, src/cuda/fusion/random_walk.cu:19-36);
  *  - there is no CPU fallback: without a CUDA device gsb_ctx_create fails.
  */
@@ -149,7 +153,7 @@ GSB_API int gsb_profile_read(gsb_ctx* ctx, int kid, double* total_ms, int64_t* l
  * (src/cuda/slicing.cu:100-182; dispatcher gs::CSCColSlicing, src/graph_ops.cc:141-154).
  *
  * gsb_col_slice_count: out_indptr[i] = sum of the degrees of seeds[0..i) (S+1 entries), computed
- *   by one kernel; waits for the stream and returns the total in *nnz_host.  seeds == NULL means
+ *   by one kernel; waits for the total and returns it in *nnz_host.  seeds == NULL means
  *   "every column 0..S-1" (S <= num_cols).
  * gsb_col_slice_fill: for each seed column copies its index segment in order:
  *   out_indices = GLOBAL row ids, out_select = position in `indices`, out_coo_col (optional) =
@@ -200,7 +204,7 @@ GSB_API int gsb_sample_one_keepdim(gsb_ctx* ctx, void* stream, const int64_t* in
  * them).  out_unique receives the distinct ids in order of first occurrence (capacity = total
  * items).  If num_relabel > 0 the concatenation of relabel_ptrs is mapped to positions in
  * out_unique and written to the matching out_relabel_ptrs (-1 for an id that is not among the
- * items).  Ids must be >= 0.  Waits for the stream when unique_host != NULL.
+ * items).  Ids must be >= 0.  Waits for the number of distinct ids when unique_host != NULL.
  */
 #define GSB_MAX_SEGMENTS 4
 GSB_API int gsb_unique_relabel(gsb_ctx* ctx, void* stream, const int64_t* const* item_ptrs_host,
@@ -345,7 +349,7 @@ GSB_API int gsb_coo2csc(gsb_ctx* ctx, void* stream, const int64_t* key, const in
  * batch's frontier.  seeds_ptr / indices_ptr / out_unique_ptr are DEVICE arrays of G + 1 entries; the
  * number of edges is read from indices_ptr[G] on the device, so the call can follow a sampling call
  * without a host round trip; `indices_capacity` is an upper bound on it used to size scratch and grids.
- * Ids must be below 2^32 - 1 and num_seeds + indices_capacity below 2^30.  Waits for the stream only if
+ * Ids must be below 2^32 - 1 and num_seeds + indices_capacity below 2^30.  Waits for its totals only if
  * a *_host pointer is given.
  * num_nodes > 0 promises that every id is in [0, num_nodes): first occurrences are then found in direct-address
  * tables (one 8-byte word per node and minibatch, kept by the context and never cleared; see GSB_OPT_RELABEL_PATH /
@@ -411,7 +415,7 @@ GSB_API int gsb_edge_div_u_sum(gsb_ctx* ctx, void* stream, const int64_t* coo_ro
  * gs::impl::IndexSelectCPUFromGPU (src/cuda/index_select_uvm.cu:8-45; row_len = 1 there).  src: device memory or
  * page-locked host memory (pageable host memory returns GSB_ERR_INVALID_ARGUMENT); index, out: device memory.
  * An index outside [0, num_rows) leaves its output row untouched and records GSB_ERR_INDEX_RANGE, which the next
- * call that waits for the stream (or gsb_check_device_status) reports. */
+ * call that waits for a size (or gsb_check_device_status) reports. */
 GSB_API int gsb_gather_rows(gsb_ctx* ctx, void* stream, const float* src, int64_t num_rows, int64_t row_len,
                             const int64_t* index, int64_t n, float* out);
 
@@ -431,7 +435,7 @@ GSB_API int gsb_metapath_random_walk(gsb_ctx* ctx, void* stream, const int64_t* 
 
 /* ---- the rest of the super-batch family (gs_ops registry, src/pybind.cc:65-84) ---------------------------
  * Ids of G minibatches travel in one array plus a DEVICE offset array of G + 1 entries.  All sizes the
- * caller passes are exact unless called "capacity".  Calls wait for the stream only where a *_host pointer
+ * caller passes are exact unless called "capacity".  Calls wait for their sizes only where a *_host pointer
  * is given.
  *
  * gsb_batch_encode / gsb_batch_decode / gsb_get_batch_offsets replace gs::impl::BatchEncodeCUDA,
@@ -530,7 +534,7 @@ GSB_API int gsb_batch_list_sample(gsb_ctx* ctx, void* stream, const float* probs
  * caller knows from earlier calls of the same shape rather than the worst case S' * (1 + k'): grids, scratch and clears
  * then follow the real sizes.  If the device meets more seeds or edges than stated, GSB_ERR_CAPACITY is recorded, the
  * passes that follow do nothing, and the caller repeats the call with the worst-case bounds.
- * Ids below 2^32 - 1; S * (1 + k) below 2^30.  Waits for the stream only if a *_host pointer is given.
+ * Ids below 2^32 - 1; S * (1 + k) below 2^30.  Waits for its totals only if a *_host pointer is given.
  */
 GSB_API int gsb_sage_hop(gsb_ctx* ctx, void* stream, const int64_t* indptr, const int64_t* indices,
                          int64_t num_nodes, const int64_t* seeds, const int64_t* seeds_ptr, const int64_t* batch_ids,

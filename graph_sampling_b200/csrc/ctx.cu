@@ -279,12 +279,13 @@ static int ctx_spin(gsb_ctx* ctx, cudaStream_t stream, const volatile u64* word,
 }
 
 Mail ctx_mail(gsb_ctx* ctx) {
-  ctx->mail_tag = ctx->mail_tag >= 0xFFFF ? 1 : ctx->mail_tag + 1;
-  // Tags repeat after 65 535 mailboxes, and a slot that few calls post still holds what the last of them left there: a word
-  // with the tag of this mailbox must not be there yet.  (Who posted to the slots before has been waited for, or its call
-  // failed within the last few mailboxes: its tag is another one.)
-  volatile u64* slots = (volatile u64*)(ctx->pinned + CNT_NUM);
-  for (int q = 0; q < kMailSlots; ++q) slots[q] = 0;
+  if (++ctx->mail_tag > 0xFFFF) {
+    // The tags start over, and a slot that few calls post may still hold what one of them left there under a tag that comes
+    // again: no word is older than its round of tags.
+    volatile u64* slots = (volatile u64*)(ctx->pinned + CNT_NUM);
+    for (int q = 0; q < kMailSlots; ++q) slots[q] = 0;
+    ctx->mail_tag = 1;
+  }
   return Mail{(u64*)(ctx->pinned + CNT_NUM), ctx->mail_tag << 48};
 }
 

@@ -164,12 +164,12 @@ __global__ void __launch_bounds__(kConvThreads) k_coo2csc(const __grid_constant_
 
   // The result of a call that was given up: all edges, in the order of the list, in column 0.
   auto give_up = [&] {
-    for (u32 i = begin + lane; i < end; i += 32) {
-      p.out_perm[i] = (i64)i;
+    grid_share(p.E, [&](i64 i) {
+      p.out_perm[i] = i;
       p.out_other[i] = __ldg(p.other + i);
-    }
-    for (i64 k = key_begin + tid; k < key_end; k += kConvThreads) p.out_indptr[k] = k == 0 ? 0 : p.E;
-    if (blockIdx.x == 0 && tid == 0) p.out_indptr[p.num_keys] = p.E;
+    });
+    grid_share(p.num_keys, [&](i64 k) { p.out_indptr[k] = k == 0 ? 0 : p.E; });  // the CTA's keys
+    if (blockIdx.x == 0) p.out_indptr[p.num_keys] = p.E;
   };
 
   for (i64 k = key_begin + tid; k < key_end; k += kConvThreads) p.counts[k] = 0;
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kConvThreads) k_coo2csc(const __grid_constant_
       }
       p.matrix[(size_t)b * ctas + blockIdx.x] = run;
     }
-    if (!grid_barrier(p.sync, ++barrier)) return give_up();
+    grid_barrier(p.sync, ++barrier, give_up);
     // ---- scan of the matrix rows; counts per key
     if (ctas <= kConvFewCtas) {  // a row is a few words and there are many rows per warp: a thread per row instead
       for (int b = (int)blockIdx.x * kConvThreads + tid; b < bins; b += ctas * kConvThreads) {
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kConvThreads) k_coo2csc(const __grid_constant_
         const i64 k = __ldg(p.key + i);
         atomicAdd(p.counts + ((u64)k < (u64)p.num_keys ? k : 0), 1u);
       }
-    if (!grid_barrier(p.sync, ++barrier)) return give_up();
+    grid_barrier(p.sync, ++barrier, give_up);
     // ---- place
     {
       const int per = bins > kConvThreads ? bins / kConvThreads : 1;  // consecutive digits per thread: 1 or 2
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kConvThreads) k_coo2csc(const __grid_constant_
       block_scan(sum, &total);
       if (tid == 0) p.key_total[blockIdx.x] = total;
     }
-    if ((!last || digit == 0) && !grid_barrier(p.sync, ++barrier)) return give_up();
+    if (!last || digit == 0) grid_barrier(p.sync, ++barrier, give_up);
     if (digit == 0) {  // offsets: the CTA's prefix, then its keys, a thread's share of consecutive ones at a time
       u32 before = 0, total;
       for (int c = tid; c < (int)blockIdx.x; c += kConvThreads) before += __ldcg(p.key_total + c);

@@ -327,19 +327,17 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
   // The results of a call that was given up, for the super-batch hops that run on without the host: empty frontiers.
   auto give_up = [&] {
     if (!BATCHED) return;
-    for (i64 b = (i64)blockIdx.x * kFuThreads + tid; b <= p.G; b += (i64)gridDim.x * kFuThreads) {
-      const i64 e = fused_edges_begin(p, b, __ldg(p.seeds_ptr + b));
-      if (p.out_indices_ptr) p.out_indices_ptr[b] = e;
+    grid_share(p.G + 1, [&](i64 b) {
+      if (p.out_indices_ptr) p.out_indices_ptr[b] = fused_edges_begin(p, b, __ldg(p.seeds_ptr + b));
       p.out_unique_ptr[b] = 0;
-    }
-    if (p.out_second)
-      for (i64 e = (i64)blockIdx.x * kFuThreads + tid; e < ne; e += (i64)gridDim.x * kFuThreads) p.out_second[e] = -1;
-    if (blockIdx.x == 0 && tid == 0) {
+    });
+    grid_share(p.out_second ? ne : 0, [&](i64 e) { p.out_second[e] = -1; });
+    if (blockIdx.x == 0) {
       p.counters[CNT_UNIQUE] = 0;
       p.counters[CNT_NNZ] = ne;
     }
   };
-  if (!grid_barrier(p.sync, 1)) return give_up();
+  grid_barrier(p.sync, 1, give_up);
 
   // ---- flag
   unsigned bits[R];
@@ -380,7 +378,7 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
       if (g < n) p.packed[g >> 5] = ((u64)s_group[r * kFuWarps + warp] << 32) | (u64)bits[r];
     }
   }
-  if (!grid_barrier(p.sync, 2)) return give_up();
+  grid_barrier(p.sync, 2, give_up);
 
   // ---- emit
   u32 all;

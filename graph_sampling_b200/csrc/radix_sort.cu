@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const u64* __res
                                                                u64* __restrict__ keys_out, i64* __restrict__ vals_out,
                                                                i64 n, int shift, const i64* __restrict__ hist,
                                                                int num_tiles, const i64* counters) {
-  if (counters[CNT_LOST] != 0) return;
+  const bool lost = counters[CNT_LOST] != 0;
   constexpr int kWarps = kSortThreads / 32;
   constexpr int kRounds = kSortItemsPerThread;  // each warp owns kRounds * 32 consecutive items
   __shared__ unsigned s_warp_count[kWarps][kRadix];
@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const u64* __res
     }
   }
   __syncthreads();
+  if (lost) return;  // asked for at the top, where nothing waits for the answer
   for (int j = threadIdx.x; j < tile_items; j += kSortThreads) {
     const u64 k = s_keys[j];
     const unsigned digit = (unsigned)(k >> shift) & 0xFFu;

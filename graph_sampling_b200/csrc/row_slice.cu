@@ -443,11 +443,10 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
     if (lane == 0) p.warp_before[blockIdx.x * kInWarps + warp] = cta_before;
     if (tid == 0) p.totals[blockIdx.x] = all;
   }
-  if (!grid_barrier(p.sync, 1)) {  // given up: an empty subgraph
-    for (i64 j = (i64)blockIdx.x * kInThreads + tid; j <= c.S; j += (i64)gridDim.x * kInThreads) c.out_indptr[j] = 0;
-    if (blockIdx.x == 0 && tid == 0) c.counters[CNT_NNZ] = 0;
-    return;
-  }
+  grid_barrier(p.sync, 1, [&] {  // given up: an empty subgraph
+    grid_share(c.S + 1, [&](i64 j) { c.out_indptr[j] = 0; });
+    if (blockIdx.x == 0) c.counters[CNT_NNZ] = 0;
+  });
   // ---- emit
   u32 total;
   {

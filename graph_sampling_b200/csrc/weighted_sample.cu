@@ -619,10 +619,10 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
   }
   // The result of a call that was given up: an empty sample.
   auto give_up = [&] {
-    for (i64 c = lo + tid; c < hi; c += kWThreads) p.out_indptr[c] = 0;
-    if (blockIdx.x == 0 && tid == 0) p.out_indptr[S] = p.counters[CNT_NNZ] = 0;
+    grid_share(p.S, [&](i64 c) { p.out_indptr[c] = 0; });  // the CTA's columns
+    if (blockIdx.x == 0) p.out_indptr[p.S] = p.counters[CNT_NNZ] = 0;
   };
-  if (!grid_barrier(p.sync, 1)) return give_up();
+  grid_barrier(p.sync, 1, give_up);
 
   // every CTA adds up what comes before it and the totals
   static_assert(NUM_SUMS == 8, "eight threads take one CTA's sums");
@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(kWThreads, 4) k_sample_weighted(WeightedParams
     grid_arrive(p.sync, 1);
     return;
   }
-  if (!grid_barrier(p.sync, 2)) return give_up();
+  grid_barrier(p.sync, 2, give_up);
   if (blockIdx.x == 0 && tid == 0) mail_post(p.mail, 0, edges, p.counters);  // nothing can go wrong from here on
 
   // Every CTA does each gridDim-th unit of work, the long ones first, and its warps take them as they become free: a counter

@@ -6,6 +6,8 @@
 // multiplication, i.e. exact integer powers (the reference's __powf is an approximation and is NaN
 // for negative bases).  The COO form accumulates with float atomics into a zero-initialised dense
 // vector, like the reference's _SegmentSumCOOKernel (:44-64); its summation order is not fixed.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace gsb {
@@ -22,6 +24,11 @@ __device__ __forceinline__ float int_pow(float x, i64 powk) {
   for (i64 i = 0; i < powk; ++i) r *= x;
   return r;
 }
+
+constexpr i64 kSegSteps = 8192;  // warps get several segments a step when there are more than this many steps
+// edges from which on a warp keeps several loads ahead within one segment
+template <bool NORMALIZE>
+constexpr int kSegMany = NORMALIZE ? 128 : 192;
 
 // One segment by `width` threads, thread `first` of them: loads kAhead elements before the first is used (with one element per
 // iteration a warp waited out a memory round trip per 32 edges), and keeps them in registers when that is the whole segment,
@@ -75,20 +82,27 @@ struct SegmentReader {
   }
 };
 
-// NORMALIZE: out[j] = data[j] / (sum of its segment); otherwise out[s] = sum of data^powk over segment s.  One launch:
-// a CTA takes one segment per step when they are long on average (at least 128 edges: a warp each would leave few warps with
-// everything, and a CTA that meets several hubs does them one after the other), a warp takes one when they are not, or — when
-// most are empty, below four edges on average, as in the row view of a slice — 32 of them: lane i reads the bounds of segment s0 + i
-// (two coalesced loads for the 32), sums it itself if it has at most four edges, and the others are summed by the whole
-// warp one after the other.  (One warp per segment spent a step, with two dependent loads, on every empty row: 78 us for
-// the 1 M rows of a slice with 25 000 edges.)  The short form adds in the order the tree would, (v0 + v2) + (v1 + v3), so
-// a segment's sum does not depend on which form took it.  Long segments are left to the whole CTA at the end of the step.
+// NORMALIZE: out[j] = data[j] / (sum of its segment); otherwise out[s] = sum of data^powk over segment s.  One launch, three forms:
+//   a CTA per segment where they average at least 128 edges (a warp each would leave few warps with everything, and a CTA that
+//   meets several hubs does them one after the other);
+//   a warp for several segments: up to 16 consecutive ones a step, whose bounds are one load that is asked for a step ahead, two
+//   of them side by side, and those with many edges afterwards, one by one with more loads ahead.  Few segments get a warp each;
+//   sums of segments that average less than four edges, as in the row view of a slice: 32 a step, lane i reads the bounds of
+//   segment s0 + i, sums it itself if it has at most four edges, and the others are summed by the whole warp one after the other.
+//   (One warp per segment spent a step, with two dependent loads, on every empty row: 78 us for the 1 M rows of a slice with
+//   25 000 edges.)  The short form adds in the order the tree would, (v0 + v2) + (v1 + v3), so a segment's sum does not depend
+//   on which form took it.
+// Segments too long for a warp are set aside for the whole CTA, when its warps are done with the others.
+// What bounds the second form is instruction issue and the warps in flight, and the registers are cut to what that takes (7, 7, 6
+// and 4 CTAs per SM; fewer spilled bytes and fewer warps are slower, sums of a million segments 147 us at six).  A million segments
+// of 30 edges: sum 129 us with a warp per segment in a kernel of its own, 353 with barriers around every eight segments, 119 now;
+// normalised 187, 273, 137.  262 144 of 51: sum 46, 78, 39 us; normalised 63, 74, 64; by edge ids 98, 159, 100.
 template <bool NORMALIZE, bool IDS>
-__global__ void __launch_bounds__(kSegThreads, 5) k_segments(const i64* __restrict__ indptr, i64 num_seg,
+__global__ void __launch_bounds__(kSegThreads, !NORMALIZE ? 7 : IDS ? 4 : 6) k_segments(const i64* __restrict__ indptr, i64 num_seg,
                                                              const i64* __restrict__ e_ids, const float* __restrict__ data,
                                                              i64 powk, float* __restrict__ out) {
   __shared__ i64 s_long[kSegThreads];
-  __shared__ int s_num_long;
+  __shared__ int s_num_long;  // long segments met by the CTA's warps
   __shared__ float s_part[kSegWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   SegmentReader<NORMALIZE, IDS> reader{e_ids, data, powk};
@@ -121,19 +135,94 @@ __global__ void __launch_bounds__(kSegThreads, 5) k_segments(const i64* __restri
     return;
   }
   const bool sparse = !NORMALIZE && mean < 4;
-  const i64 per_cta = sparse ? kSegThreads : kSegWarps;
-  for (i64 first = (i64)blockIdx.x * per_cta; first < num_seg; first += (i64)gridDim.x * per_cta) {
-    if (threadIdx.x == 0) s_num_long = 0;
-    __syncthreads();
-    if (!sparse) {
-      const i64 s = first + warp;
-      if (s < num_seg) {
+  if (threadIdx.x == 0) s_num_long = 0;
+  __syncthreads();
+  auto set_aside = [&](i64 s) {
+    const int at = atomicAdd(&s_num_long, 1);
+    if (at < kSegThreads) s_long[at] = s;
+  };
+  const i64 first = (i64)blockIdx.x * kSegWarps + warp, warps = (i64)gridDim.x * kSegWarps;
+  int per = sparse ? 32 : 1;  // consecutive segments per warp and step: their bounds are one load, asked for a step ahead
+  if (!sparse) {
+    while (per < 16 && num_seg >= 2ll * per * kSegSteps) per *= 2;
+    if (per == 1) {
+      for (i64 s = first; s < num_seg; s += warps) {
         const i64 b = __ldg(indptr + s), e = __ldg(indptr + s + 1);
         if (e - b <= kLongSegment) warp_segment(s, b, e);
-        else if (lane == 0) s_long[atomicAdd(&s_num_long, 1)] = s;
+        else if (lane == 0) set_aside(s);
       }
-    } else {
-      const i64 s0 = first + warp * 32, s = s0 + lane;
+    }
+    auto bounds = [&](i64 s0) { return lane <= per && s0 < num_seg ? __ldg(indptr + min(s0 + lane, num_seg)) : 0; };
+    i64 ahead = bounds(first * per);
+    for (i64 s0 = first * per; per > 1 && s0 < num_seg; s0 += warps * per) {
+      const i64 base = __shfl_sync(0xffffffffu, ahead, 0);
+      const int start = (int)min(ahead - base, (i64)1 << 30);  // of the lane's segment, relative to the first one's
+      ahead = bounds(s0 + warps * per);
+      const int count = (int)min((i64)per, num_seg - s0);
+      if (__shfl_sync(0xffffffffu, start, count) == 1 << 30) {  // not in 32 bits
+        if (lane < count) set_aside(s0 + lane);
+        continue;
+      }
+      const i64* ids = IDS ? e_ids + base : nullptr;
+      const float* from = data && !IDS ? data + base : data;
+      using Place = typename std::conditional<IDS, i64, int>::type;
+      auto place = [&](int i) -> Place { return IDS ? (Place)__ldg(ids + i) : (Place)i; };
+      auto value_at = [&](Place at) {
+        const float x = NORMALIZE || data ? __ldg(from + at) : 1.0f;
+        return NORMALIZE ? x : int_pow(x, powk);
+      };
+      unsigned many = 0;  // segments that are worth more loads ahead
+      for (int j = 0; j < count; j += 2) {  // two side by side: their loads and their trees overlap
+        int b[2], len[2];
+        Place at[2];
+        float v[2], acc[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int k = min(j + u, count);
+          b[u] = __shfl_sync(0xffffffffu, start, k);
+          len[u] = __shfl_sync(0xffffffffu, start, min(k + 1, count)) - b[u];
+          if (len[u] > kSegMany<NORMALIZE>) {
+            many |= 1u << k;
+            len[u] = -1;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) at[u] = lane < len[u] ? place(b[u] + lane) : 0;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) acc[u] = v[u] = lane < len[u] ? value_at(at[u]) : 0.f;
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          for (int i = 32 + lane; i < len[u]; i += 32) acc[u] += value_at(place(b[u] + i));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (NORMALIZE) {
+            float* to = IDS ? out : out + base;
+            if (lane < len[u]) to[at[u]] = v[u] / acc[u];
+            for (int i = 32 + lane; i < len[u]; i += 32) {
+              const Place k = place(b[u] + i);
+              to[k] = value_at(k) / acc[u];
+            }
+          } else if (lane == u && len[u] >= 0 && j + u < count) {
+            out[s0 + j + u] = acc[u];
+          }
+        }
+      }
+      while (many) {
+        const int k = __ffs(many) - 1;
+        many &= many - 1;
+        const int b = __shfl_sync(0xffffffffu, start, k), e = __shfl_sync(0xffffffffu, start, k + 1);
+        if (e - b <= kLongSegment) warp_segment(s0 + k, base + b, base + e);
+        else if (lane == 0) set_aside(s0 + k);
+      }
+    }
+  } else {
+    for (i64 s0 = first * 32; s0 < num_seg; s0 += warps * 32) {
+      const i64 s = s0 + lane;
       i64 b = 0, e = 0;
       if (s < num_seg) {
         b = __ldg(indptr + s);
@@ -150,8 +239,8 @@ __global__ void __launch_bounds__(kSegThreads, 5) k_segments(const i64* __restri
         if (len > 2) v2 = value(b + 2);
         if (len > 3) v3 = value(b + 3);
       }
-      if (s < num_seg && len > kLongSegment) s_long[atomicAdd(&s_num_long, 1)] = s;
-      unsigned medium = __ballot_sync(0xffffffffu, s < num_seg && len > 4 && len <= kLongSegment);
+      if (len > kLongSegment) set_aside(s);
+      unsigned medium = __ballot_sync(0xffffffffu, len > 4 && len <= kLongSegment);
       while (medium) {
         const int src = __ffs(medium) - 1;
         medium &= medium - 1;
@@ -159,9 +248,20 @@ __global__ void __launch_bounds__(kSegThreads, 5) k_segments(const i64* __restri
       }
       if (is_short) out[s] = (v0 + v2) + (v1 + v3);
     }
-    __syncthreads();
-    for (int q = 0, n = s_num_long; q < n; ++q) cta_segment(s_long[q]);
-    __syncthreads();  // s_long / s_num_long are rewritten by the next step
+  }
+  __syncthreads();
+  const int num_long = s_num_long;
+  if (num_long <= kSegThreads) {
+    for (int q = 0; q < num_long; ++q) cta_segment(s_long[q]);
+    return;
+  }
+  for (i64 s0 = first - warp; s0 * per < num_seg; s0 += warps) {  // more than the list holds: the CTA's segments once more
+    for (i64 step = s0 * per; step < min(num_seg, (s0 + kSegWarps) * per); step += per) {
+      const i64 end = min(num_seg, step + per);
+      const bool wide = !sparse && __ldg(indptr + end) - __ldg(indptr + step) >= (i64)1 << 30;
+      for (i64 s = step; s < end; ++s)
+        if (wide || __ldg(indptr + s + 1) - __ldg(indptr + s) > kLongSegment) cta_segment(s);
+    }
   }
 }
 

@@ -87,3 +87,43 @@ def test_segments_long_short_and_empty(ops, lengths, permuted):
     norm = torch.empty(len(data), device="cuda")
     got = ops.csc_normalize(dev(indptr), d_ids, dev(data), norm).cpu().numpy()
     assert np.allclose(got[e_ids] if permuted else got, v / total[seg], rtol=1e-5, atol=0)
+
+
+def test_segments_share_warps(ops):
+    """Several segments per warp and step: ragged ones, empty ones, hubs between them, and more segments too long for a warp
+    in one CTA than its list holds."""
+    rng = np.random.default_rng(8)
+    ragged = rng.integers(0, 300, 40_001) * (rng.random(40_001) < 0.5)
+    ragged[[0, 17, 40_000]] = [2049, 5000, 40_000]
+    short = rng.integers(0, 12, 300_000)
+    crowded = np.zeros(700_000, np.int64)   # a CTA's segments lie 303 104 (normalised) and 606 208 (summed) apart
+    for at in (0, 303_104, 606_208):
+        crowded[at:at + 256] = 2049
+    for lengths in (ragged, short, crowded):
+        indptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+        E = int(indptr[-1])
+        data, seg = (rng.random(E) + 0.01).astype(np.float32), np.repeat(np.arange(len(lengths)), lengths)
+        for e_ids in (None, rng.permutation(E)):
+            v = data if e_ids is None else data[e_ids]
+            total = np.bincount(seg, v.astype(np.float64), len(lengths))
+            d_ids, out = None if e_ids is None else dev(e_ids), torch.full((len(lengths),), -1.0, device="cuda")
+            got = ops.csc_sum(dev(indptr), d_ids, dev(data), out, 1).cpu().numpy()
+            assert np.allclose(got, total, rtol=1e-5, atol=0)
+            norm = torch.full((E,), -1.0, device="cuda")
+            got = ops.csc_normalize(dev(indptr), d_ids, dev(data), norm).cpu().numpy()
+            assert np.allclose(got if e_ids is None else got[e_ids], v / total[seg], rtol=1e-5, atol=0)
+
+
+def test_segments_beyond_32_bits_of_edges(ops):
+    """Offsets within a warp's segments are 32-bit; a step that spans more edges is left to whole CTAs.  Sums of ones, which need
+    no data: one segment of 2^30 + 5 edges and one of 2^31 among short ones."""
+    import ctypes
+    n = 30_000_000
+    lengths = torch.full((n,), 3, dtype=torch.int64, device="cuda")
+    lengths[12_345], lengths[20_000_001] = (1 << 30) + 5, 1 << 31
+    indptr = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    torch.cumsum(lengths, 0, out=indptr[1:])
+    out, ctx = torch.full((n,), -1.0, device="cuda"), ops.default_context()
+    ctx.check(ctx.lib.gsb_segment_sum_csc(ctx.handle, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream),
+                                          indptr.data_ptr(), n, None, None, 1, out.data_ptr()), "gsb_segment_sum_csc")
+    assert torch.allclose(out.double(), lengths.double(), rtol=1e-6, atol=0)

@@ -10,6 +10,8 @@
 // floats: 184 us with two rows per group, half the grid apart, and half the CTAs; 145 us now, where reading alone takes 93
 // and writing alone 65.  Copying the rows through shared memory with bulk copies gave 150 to 158, cutting the output into
 // tiles of equal bytes 190.
+#include <type_traits>
+
 #include "common.cuh"
 #include "scan.cuh"
 
@@ -59,19 +61,32 @@ static void launch_rows(cudaStream_t stream, const void* src, i64 num_rows, i64 
                                                                       counters);
 }
 
+// Lanes per row and rows at a time by the units of a row.  A power of two of lanes leaves some of them idle; where half as many
+// lanes take the row in no more steps than three quarters of the whole would (5 and 6 units, 9 to 12, 17 to 24, 33 to 48), they
+// are the better choice, with two rows: a million rows of 17 floats 63 us against 76, of 33 floats 92 against 108, of 42 floats 93
+// against 103, of 160 floats 218 against 251; equal at 24 and 48 floats, and above the three quarters the whole group is ahead (100
+// floats 146 against 152).  Rows of several steps are runs of memory by themselves, two at a time are better than four (63 floats
+// 156 and 172 us, 300 000 rows of 602 floats 289 and 306, 1 000 rows of 512 floats 5.5 and 8.2) except for 64 units (322 against
+// 325) and for odd rows above 4 KB (1 433 floats, 300 000 rows: 925 and 898).
 template <typename Unit>
 static void launch_gather(cudaStream_t stream, const void* src, i64 num_rows, i64 units, const i64* index, i64 n, void* out,
                           i64* counters) {
-  if (units == 1) launch_rows<Unit, 1, 2>(stream, src, num_rows, units, index, n, out, counters);
-  else if (units == 2) launch_rows<Unit, 2, 4>(stream, src, num_rows, units, index, n, out, counters);
-  else if (units <= 4) launch_rows<Unit, 4, 4>(stream, src, num_rows, units, index, n, out, counters);
-  else if (units <= 8) launch_rows<Unit, 8, 4>(stream, src, num_rows, units, index, n, out, counters);
-  else if (units <= 16) launch_rows<Unit, 16, 4>(stream, src, num_rows, units, index, n, out, counters);
-  else if (units <= 64) launch_rows<Unit, 32, 4>(stream, src, num_rows, units, index, n, out, counters);
-  // long rows are runs of memory by themselves: two rows at a time and four, 300 000 rows of 602 floats 289 and 306 us, of 130
-  // floats 72 and 78, 1 000 rows of 512 floats 5.5 and 8.2; only rows of an odd number of floats above 4 KB are the other way
-  // (1 433: 925 and 898)
-  else launch_rows<Unit, 32, 2>(stream, src, num_rows, units, index, n, out, counters);
+  auto go = [&](auto lanes, auto rows) {
+    launch_rows<Unit, decltype(lanes)::value, decltype(rows)::value>(stream, src, num_rows, units, index, n, out, counters);
+  };
+  using std::integral_constant;
+  const integral_constant<int, 2> two{};
+  const integral_constant<int, 4> four{};
+  if (units == 1) go(integral_constant<int, 1>{}, two);
+  else if (units == 2) go(two, four);
+  else if (units <= 4) go(four, four);
+  else if (units <= 6 || (units == 7 && sizeof(Unit) < 16)) go(four, two);
+  else if (units <= 8) go(integral_constant<int, 8>{}, four);
+  else if (units <= 12) go(integral_constant<int, 8>{}, two);
+  else if (units <= 16) go(integral_constant<int, 16>{}, four);
+  else if (units <= 24 || (units > 32 && units <= 48)) go(integral_constant<int, 16>{}, two);
+  else if (units <= 32 || units == 64) go(integral_constant<int, 32>{}, four);
+  else go(integral_constant<int, 32>{}, two);
 }
 
 }  // namespace gsb

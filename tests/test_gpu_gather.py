@@ -27,6 +27,16 @@ def test_gather_rows_matches_torch_index(ops, F, pinned):
     assert ops.gather_rows(s, idx[:0].cuda()).shape == (0, F)
 
 
+@pytest.mark.parametrize("units", [2, 5, 6, 7, 8, 9, 12, 13, 17, 24, 25, 33, 48, 49, 63, 64, 65, 96])
+@pytest.mark.parametrize("width", [1, 2, 4])
+def test_gather_rows_at_the_edges_of_the_lane_groups(ops, units, width):
+    g = torch.Generator("cuda").manual_seed(units)
+    src = torch.randn(3000, units * width, generator=g, device="cuda")
+    for n in (1, 7, 4097):
+        idx = torch.randint(0, 3000, (n,), generator=g, device="cuda")
+        assert torch.equal(ops.gather_rows(src, idx), src[idx])
+
+
 def test_gather_vector_misaligned_and_errors(ops):
     from graph_sampling_b200.cabi import GsbError
     src = torch.arange(1000, dtype=torch.float32).cuda()

@@ -52,8 +52,8 @@ UNIT = "edges/s"
 # proportion to the units a launch processes, so a full launch's traffic is this ratio times its algorithmic bytes.
 TRAFFIC_OVER_ALGORITHMIC = {"sample_uniform": 4.2, "table_insert": 4.1, "first_compact": 3.2, "relabel": 1.04,
                             # partitioned form (profiles/k_part_*_sage3hop_group64.md, k_rank_emit_sage3hop_group64.md)
-                            "partition_count": 1.04, "partition_scatter": 0.81, "bucket_resolve": 0.88,
-                            "first_bits": 1.0}
+                            "partition_count": 1.04, "partition_scatter": 0.83, "bucket_resolve": 0.84,
+                            "first_bits": 0.81}
 # the same with direct-address tables (profiles/k_direct_insert_sage3hop_group64.md)
 TRAFFIC_OVER_ALGORITHMIC_DIRECT = {"sample_uniform": 4.2, "table_insert": 9.1}
 
@@ -518,9 +518,9 @@ def run_ours(args):
         "first_compact": sum(8 * (s_ + e_) + 8 * u_ for s_, e_, u_ in hop_shapes) / n_launch,
         "relabel": sum(16 * e_ for s_, e_, _ in hop_shapes) / n_launch,
         "partition_count": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
-        "partition_scatter": sum(16 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
+        "partition_scatter": sum(20 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
         "bucket_resolve": sum(12 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
-        "first_bits": sum(4 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
+        "first_bits": sum(12 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
         "rank_emit": sum(4 * (s_ + e_) + 16 * u_ + 8 * e_ for s_, e_, u_ in hop_shapes) / n_launch,
     }
     # which form of unique + relabel ran is read off the kernels that were launched

@@ -123,6 +123,52 @@ struct ColumnWalk {
       advance();
     }
   }
+
+  // The other way through the stretch, for columns of some length: pieces of up to 32 positions of ONE column, N of them at a
+  // time, so that locating costs a dozen instructions per piece whatever the columns are.  f(at, edge): the lane's position in the
+  // N pieces, and the input position (negative: none).  Called by all lanes, behind init(); pieces come in ascending order.
+  template <int N, class F>
+  __device__ __forceinline__ void for_pieces(F f) {
+    static_assert(32 % N == 0, "a warp holds 32 pieces");
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+      int stop = __shfl_down_sync(0xffffffffu, start, 1);
+      if (lane == 31) stop = next;
+      const int mine = stop > start && delta != kNoWalkColumn ? (stop - start + 31) >> 5 : 0;
+      int upto = mine;  // pieces of the window's columns up to the lane's
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += t;
+      }
+      const int total = __shfl_sync(0xffffffffu, upto, 31);
+      for (int base = 0; base < total; base += 32) {
+        // piece base + lane: the first column with more pieces up to it than that
+        int c = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(0xffffffffu, upto, c + step - 1) <= base + lane) c += step;
+        const int rank = base + lane - (__shfl_sync(0xffffffffu, upto, c) - __shfl_sync(0xffffffffu, mine, c));
+        const int first = __shfl_sync(0xffffffffu, start, c) + rank * 32;
+        const int end = __shfl_sync(0xffffffffu, stop, c);
+        const i64 in = __shfl_sync(0xffffffffu, delta, c) + first;
+        const int count = base + lane < total ? min(end - first, 32) : 0;
+        for (int piece = 0; piece < min(32, total - base); piece += N) {
+          int at[N];
+          i64 edge[N];
+#pragma unroll
+          for (int r = 0; r < N; ++r) {
+            at[r] = __shfl_sync(0xffffffffu, first, piece + r) + lane;
+            edge[r] = __shfl_sync(0xffffffffu, in, piece + r) + lane;
+            if (lane >= __shfl_sync(0xffffffffu, count, piece + r)) edge[r] = -1;
+          }
+          f(at, edge);
+        }
+      }
+      if (next >= len) return;
+      advance();
+    }
+  }
 };
 
 }  // namespace gsb

@@ -29,11 +29,10 @@ constexpr u64 kMaxFlip = 0x7fffffffffffffffull;  // val = kMaxFlip - position, s
 // they never reach the table, whose random 32-byte reads were what the filter kernels waited for.
 struct RowBloom {
   u32* words;  // null: no filter
-  int shift;   // 64 - log2(bits)
+  int shift;   // 32 - log2(bits)
 };
-__device__ __forceinline__ u32 bloom_bit(const RowBloom& b, i64 key) {
-  return (u32)(((u64)key * 0xD6E8FEB86659FD93ull) >> b.shift);
-}
+// Of the id's low half: a filter may take two ids for one, and the 64-bit product was six instructions more per edge.
+__device__ __forceinline__ u32 bloom_bit(const RowBloom& b, i64 key) { return ((u32)key * 0x9E3779B1u) >> b.shift; }
 
 __global__ void __launch_bounds__(kRowThreads) k_build_row_table(const i64* __restrict__ row_ids, i64 R, Table table,
                                                                  RowBloom bloom, i64* counters) {
@@ -316,46 +315,73 @@ __global__ void __launch_bounds__(kRowThreads) k_col_row_filter(ColRowParams p) 
 
 // ---- induced subgraph of one node set in one launch -----------------------------------------------------------------
 // The single-batch form of k_col_row_filter as a cooperative kernel: a warp owns one stretch of the virtual edge list.
-//   filter   192 positions at a time, columns found without barriers (column_walk.cuh); an edge is looked up in the table only
-//            when the shared-memory filter lets it pass; survivors go to scratch in order, and every 32 positions leave
-//            [survivors of the warp before them : 32 | bits : 32];
+//   filter   128 positions at a time, columns found without barriers (column_walk.cuh); an edge is looked up in the table only
+//            when the shared-memory filter lets it pass; survivors go to scratch in order, with their positions;
 //   barrier
 //   emit     every CTA scans the CTAs' totals, copies its survivors to their places (and gathers their edge data), and a
-//            share of the columns gets its offset as the rank of the column's first position.
-// 20 000 columns with 6.5 M edges, 20 000 rows: 178 us with a table probe per edge and a look-back chain of 6 400 tiles, 84
-// with a stretch per CTA (six tiles of two searches and four barriers each), 64 with one per warp.
+//            share of the columns finds its offset by a binary search among the survivors of the warp that had the column's
+//            first position (seven reads in the case below, instead of a word per 32 positions that all groups have to leave).
+// Bounded by instruction issue, then by the reads a warp waits for.  20 000 columns with 7.1 M edges, 20 000 rows: 178 us with a
+// table probe per edge and a look-back chain of 6 400 tiles, 84 with a stretch per CTA (six tiles of two searches and four
+// barriers each), 67 with one per warp, 51 with pieces of columns, one read per table slot and the edge data on their way to L2
+// before the barrier.  One column after the other, 128 positions a step, has fewer instructions (20 M for 24 M), but a warp
+// whose columns are short takes 80 such steps: half the warps were done after 25 us, the last after 43.
 constexpr int kInThreads = 512;
-constexpr int kInPer = 6;
+constexpr int kInPer = 4;
+constexpr u32 kInQueue = 128;  // edges of a warp that wait for their look-up: 31 left over and 64 more at most
 constexpr int kInWarps = kInThreads / 32;
 constexpr int kBloomMaxBits = 1 << 19;  // 64 KB: two CTAs per SM
 constexpr i64 kBloomMaxRows = 1 << 18;  // beyond, most edges would pass
-constexpr i64 kInducedMaxEdges = 1 << 27;  // its scratch is 12 bytes per edge
+// Edges per column from which pieces of columns are the faster way: 4 M edges, 20 000 rows, positions against pieces: columns of 4
+// 106 / 149 us for the call, 12 92 / 95, 16 86.5 / 85.9, 24 87 / 81, 64 69 / 65; a heavy tail of mean 16 78 / 83, of mean 32 75 / 72.
+constexpr i64 kInPieces = 20;
+constexpr i64 kInducedMaxEdges = 1 << 27;  // its scratch is 16 bytes per edge
 
 struct InducedParams {
   ColRowParams c;
   RowBloom bloom;
-  i64 range;        // positions per warp, a multiple of 32
-  u64* packed;      // [D / 32 + 1]
+  i64 range;        // positions per warp
   u32* totals;      // [CTAs]
   u32* warp_before;  // [CTAs][kInWarps] survivors of the CTA's warps before this one
+  u32* warp_kept;   // [CTAs][kInWarps] survivors of the warp
   u32* kept_row;    // [D] position in row_ids
+  u32* kept_at;     // [D] position in the warp's stretch, ascending
   i64* kept_edge;   // [D]
   GridSync sync;
 };
 
+// Position in row_ids of a row id of the table, or kNoRow.
+constexpr u32 kNoRow = 0xFFFFFFFFu;
+__device__ __forceinline__ u32 find_row(const Table& t, i64 id) {
+  const u32 mask = (u32)t.mask;
+  u32 h = (u32)table_home(t, id);
+  for (u32 left = mask;; --left) {
+    const longlong2 slot = __ldg(reinterpret_cast<const longlong2*>(t.slots) + h);
+    if (slot.x == id) return (u32)(kMaxFlip - (u64)slot.y);
+    if (slot.x == kEmptyKey || left == 0) return kNoRow;
+    h = (h + 1) & mask;
+  }
+}
+
+// PIECES: the columns are long enough to be taken in pieces of their own.
+template <bool PIECES>
 __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant__ InducedParams p) {
   extern __shared__ __align__(16) u32 s_bloom[];
   __shared__ u32 s_warp[kInWarps];
   __shared__ u32 s_prefix[kInThreads];
-  __shared__ i64 s_queue_id[kInWarps][64];            // edges that passed the filter: row id,
-  __shared__ unsigned char s_queue_at[kInWarps][64];  // place among the warp's 192 positions
-  __shared__ u32 s_row[kInWarps][32 * kInPer];        // what the table said
+  struct Passed {  // an edge that passed the filter
+    i64 edge;      // position in the operand
+    u32 id;        // low half of its row id
+    u32 at;        // position in the stretch; kWide: the id has a high half, which is read again
+  };
+  constexpr u32 kWide = 0x80000000u;
+  __shared__ __align__(16) Passed s_queue[kInWarps][kInQueue];
   const ColRowParams& c = p.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
   const i64 begin = min(c.D, ((i64)blockIdx.x * kInWarps + warp) * p.range), end = min(c.D, begin + p.range);
   if (p.bloom.words) {
-    const int quads = (1 << (64 - p.bloom.shift)) / 128;
+    const int quads = (1 << (32 - p.bloom.shift)) / 128;
     for (int i = tid; i < quads; i += kInThreads)
       reinterpret_cast<uint4*>(s_bloom)[i] = __ldcg(reinterpret_cast<const uint4*>(p.bloom.words) + i);
   }
@@ -369,67 +395,72 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
   if (begin < end) walk.init(begin, (int)(end - begin));
   __syncthreads();  // the filter is loaded
   u32 kept = 0;  // survivors of the warp so far
-  for (i64 at = begin; at < end; at += 32 * kInPer) {
-    u32 row[kInPer];  // position in row_ids, or kNoRow
-    i64 edge[kInPer], id[kInPer];
-    constexpr u32 kNoRow = 0xFFFFFFFFu;
-#pragma unroll
-    for (int r = 0; r < kInPer; ++r) {
-      edge[r] = -1;
-      if (at + r * 32 < end) edge[r] = walk.locate<false>((int)(at - begin) + r * 32, nullptr);  // uniform
-      id[r] = edge[r] >= 0 ? __ldg(c.indices + edge[r]) : -1;
+  u32 head = 0, tail = 0;
+  // Few edges pass the filter, but nearly every group of 32 has some: looked up where they stand, each group would wait out a
+  // chain of table reads for two or three lanes.  They are queued instead, and looked up 32 at a time; the queue has the order
+  // of the edges, so the survivors leave it in theirs.
+  auto look_up = [&] {
+    __syncwarp();
+    u32 row = kNoRow;
+    Passed e;
+    if (lane < (int)(tail - head)) {
+      e = s_queue[warp][(head + lane) % kInQueue];
+      row = find_row(c.table, e.at & kWide ? __ldg(c.indices + e.edge) : (i64)e.id);
     }
-    // Few edges pass the filter, but nearly every group of 32 has some: looked up where they stand, each group would wait
-    // out a chain of table reads for two or three lanes.  They are queued instead, and looked up 32 at a time.
-    int queued = 0;
-    auto look_up = [&](int count) {
-      __syncwarp();
-      if (lane < count) {
-        const Slot* s = table_find(c.table, s_queue_id[warp][lane]);
-        if (s) s_row[warp][s_queue_at[warp][lane]] = (u32)(kMaxFlip - s->val);
-      }
-      __syncwarp();
-      if (lane + 32 < queued) {  // what lies beyond the 32 moves to the front
-        s_queue_id[warp][lane] = s_queue_id[warp][lane + 32];
-        s_queue_at[warp][lane] = s_queue_at[warp][lane + 32];
-      }
-      queued -= count;
-      __syncwarp();
-    };
+    const unsigned bits = __ballot_sync(0xffffffffu, row != kNoRow);
+    if (row != kNoRow) {
+      const i64 to = begin + kept + __popc(bits & lt);
+      p.kept_row[to] = row;
+      p.kept_edge[to] = e.edge;
+      p.kept_at[to] = e.at & ~kWide;
+      // random reads that the DRAM serves 43 G of a second: they come while the filter leaves it idle
+      if (c.out_data) asm volatile("prefetch.global.L2 [%0];" ::"l"(c.e_ids ? (const void*)(c.e_ids + e.edge) : c.data + e.edge));
+    }
+    kept += __popc(bits);
+    head += min(32u, tail - head);
+    __syncwarp();
+  };
+  auto test = [&](const int (&at)[kInPer], const i64 (&edge)[kInPer]) {
+    i64 id[kInPer];
 #pragma unroll
-    for (int r = 0; r < kInPer; ++r) s_row[warp][r * 32 + lane] = kNoRow;
+    for (int r = 0; r < kInPer; ++r) id[r] = edge[r] >= 0 ? __ldg(c.indices + edge[r]) : -1;
 #pragma unroll
     for (int r = 0; r < kInPer; ++r) {
       bool pass = id[r] >= 0;
-      if (pass && p.bloom.words) {
+      if (p.bloom.words) {  // (what lies in the filter's place for no id is read and not used)
         const u32 bit = bloom_bit(p.bloom, id[r]);
-        pass = ((s_bloom[bit >> 5] >> (bit & 31)) & 1u) == 0u;
+        pass = pass && ((s_bloom[bit >> 5] >> (bit & 31u)) & 1u) == 0u;
       }
       const unsigned passing = __ballot_sync(0xffffffffu, pass);
       if (pass) {
-        const int to = queued + __popc(passing & lt);
-        s_queue_id[warp][to] = id[r];
-        s_queue_at[warp][to] = (unsigned char)(r * 32 + lane);
+        Passed e;
+        e.edge = edge[r];
+        e.id = (u32)id[r];
+        e.at = (u32)at[r] | ((u64)id[r] >> 32 ? kWide : 0u);
+        s_queue[warp][(tail + __popc(passing & lt)) % kInQueue] = e;
       }
-      queued += __popc(passing);
-      if (queued >= 32) look_up(32);
+      tail += __popc(passing);
+      if (r % 2 == 1)
+        while (tail - head >= 32) look_up();
     }
-    if (queued > 0) look_up(queued);
+  };
+  if (begin < end) {
+    if (PIECES) {
+      walk.for_pieces<kInPer>(test);
+    } else {
+      for (int first = 0; first < walk.len; first += 32 * kInPer) {
+        int at[kInPer];
+        i64 edge[kInPer];
 #pragma unroll
-    for (int r = 0; r < kInPer; ++r) row[r] = s_row[warp][r * 32 + lane];
-#pragma unroll
-    for (int r = 0; r < kInPer; ++r) {
-      const unsigned bits = __ballot_sync(0xffffffffu, row[r] != kNoRow);
-      const i64 q = at + r * 32;
-      if (lane == 0 && q < end) p.packed[q >> 5] = ((u64)kept << 32) | (u64)bits;
-      if (row[r] != kNoRow) {
-        const i64 to = begin + kept + __popc(bits & lt);
-        p.kept_row[to] = row[r];
-        p.kept_edge[to] = edge[r];
+        for (int r = 0; r < kInPer; ++r) {
+          at[r] = first + r * 32 + lane;
+          edge[r] = first + r * 32 < walk.len ? walk.locate<false>(first + r * 32, nullptr) : -1;  // uniform
+        }
+        test(at, edge);
       }
-      kept += __popc(bits);
     }
   }
+  while (tail != head) look_up();
   u32 cta_before = 0;  // of the CTA's warps before this one
   if (lane == 0) s_warp[warp] = kept;
   __syncthreads();
@@ -440,7 +471,10 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
       if (w < warp) cta_before += s_warp[w];
       all += s_warp[w];
     }
-    if (lane == 0) p.warp_before[blockIdx.x * kInWarps + warp] = cta_before;
+    if (lane == 0) {
+      p.warp_before[blockIdx.x * kInWarps + warp] = cta_before;
+      p.warp_kept[blockIdx.x * kInWarps + warp] = kept;
+    }
     if (tid == 0) p.totals[blockIdx.x] = all;
   }
   grid_barrier(p.sync, 1, [&] {  // given up: an empty subgraph
@@ -474,20 +508,45 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
     mail_post(c.mail, 0, total, c.counters);
   }
   const i64 out0 = s_prefix[blockIdx.x] + cta_before;
-  for (u32 j = lane; j < kept; j += 32) {  // written by this very warp
-    const i64 e = __ldcg(p.kept_edge + begin + j);
-    c.out_indices[out0 + j] = c.renumber ? (i64)__ldcg(p.kept_row + begin + j) : __ldg(c.indices + e);
-    if (c.out_select) c.out_select[out0 + j] = e;
-    if (c.out_data) c.out_data[out0 + j] = __ldg(c.data + (c.e_ids ? __ldg(c.e_ids + e) : e));
+  constexpr int kAhead = 4;  // survivors of a lane whose reads are in flight together
+  for (u32 j0 = lane; j0 < kept; j0 += 32 * kAhead) {  // written by this very warp
+    i64 e[kAhead], value[kAhead];
+    float x[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      const u32 j = j0 + q * 32;
+      e[q] = j < kept ? __ldcg(p.kept_edge + begin + j) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+      if (e[q] >= 0) value[q] = c.renumber ? (i64)__ldcg(p.kept_row + begin + j0 + q * 32) : __ldg(c.indices + e[q]);
+    if (c.out_data) {
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q)
+        if (e[q] >= 0) x[q] = __ldg(c.data + (c.e_ids ? __ldg(c.e_ids + e[q]) : e[q]));
+    }
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      if (e[q] < 0) continue;
+      const i64 to = out0 + j0 + q * 32;
+      c.out_indices[to] = value[q];
+      if (c.out_select) c.out_select[to] = e[q];
+      if (c.out_data) c.out_data[to] = x[q];
+    }
   }
   for (i64 j = (i64)blockIdx.x * kInThreads + tid; j <= c.S; j += (i64)gridDim.x * kInThreads) {
     const i64 pos = __ldg(c.sub_indptr + j);
     i64 rank = total;
     if (pos < c.D) {
-      const u64 w = __ldcg(p.packed + (pos >> 5));
-      const u32 owner = (u32)(pos / p.range);
-      rank = s_prefix[owner / kInWarps] + __ldcg(p.warp_before + owner) + (u32)(w >> 32) +
-             __popc((u32)w & ((1u << (pos & 31)) - 1u));
+      const u32 owner = (u32)(pos / p.range), at = (u32)(pos - (i64)owner * p.range);
+      const u32* list = p.kept_at + (i64)owner * p.range;
+      u32 lo = 0, hi = __ldcg(p.warp_kept + owner);  // survivors before the column: the first that lies at or behind it
+      while (lo < hi) {
+        const u32 mid = (lo + hi) >> 1;
+        if (__ldcg(list + mid) < at) lo = mid + 1;
+        else hi = mid;
+      }
+      rank = s_prefix[owner / kInWarps] + __ldcg(p.warp_before + owner) + lo;
     }
     c.out_indptr[j] = rank;
   }
@@ -525,7 +584,7 @@ static int build_table(gsb_ctx* ctx, cudaStream_t stream, const int64_t* row_ids
   RowBloom filter{nullptr, 0};
   if (bloom) {
     filter.words = (u32*)((char*)ws + cap * sizeof(Slot));
-    filter.shift = 64 - bits_log2;
+    filter.shift = 32 - bits_log2;
     *bloom = filter;
   }
   GSB_CUDA_OK(cudaMemsetAsync(table->slots, 0xFF, table_bytes, stream));
@@ -647,30 +706,34 @@ int gsb_col_row_slice(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
   }
   Table table;
   if (!col_ptr && column_ids && D <= kInducedMaxEdges && R < (i64)1 << 31) {
-    static int resident[64];
+    static int resident[2][64];
     static bool attr_set[64];
     const int dev = ctx_device(ctx);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-      GSB_CUDA_OK(cudaFuncSetAttribute(k_induced, cudaFuncAttributeMaxDynamicSharedMemorySize, kBloomMaxBits / 8));
+      GSB_CUDA_OK(cudaFuncSetAttribute(k_induced<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBloomMaxBits / 8));
+      GSB_CUDA_OK(cudaFuncSetAttribute(k_induced<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBloomMaxBits / 8));
       attr_set[dev] = true;
     }
-    const int ctas = min(kInThreads, ctx_resident_ctas(ctx, (const void*)k_induced, kInThreads, kBloomMaxBits / 8, resident));
+    const bool pieces = D >= kInPieces * S;
+    const void* kernel = pieces ? (const void*)k_induced<true> : (const void*)k_induced<false>;
+    const int ctas = min(kInThreads, ctx_resident_ctas(ctx, kernel, kInThreads, kBloomMaxBits / 8, resident[pieces]));
     if (ctas > 0) {
       InducedParams p{};
       const i64 warps = (i64)ctas * kInWarps;
       p.range = max((i64)(32 * kInPer), ((D + warps - 1) / warps + 31) / 32 * 32);
       const int grid = (int)((D + p.range * kInWarps - 1) / (p.range * kInWarps));
       auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-      const size_t packed_bytes = al(8 * ((size_t)D / 32 + 2)), edge_bytes = al(8 * (size_t)D), row_bytes = al(4 * (size_t)D);
+      const size_t edge_bytes = al(8 * (size_t)D), row_bytes = al(4 * (size_t)D);
       void* extra;
-      int st = build_table(ctx, stream, row_ids, R, packed_bytes + edge_bytes + row_bytes + 4 * kInThreads * (1 + kInWarps), &table, &extra,
+      int st = build_table(ctx, stream, row_ids, R, edge_bytes + 2 * row_bytes + 4 * kInThreads * (1 + 2 * kInWarps), &table, &extra,
                            R <= kBloomMaxRows ? &p.bloom : nullptr);
       if (st != GSB_OK) return st;
-      p.packed = (u64*)extra;
-      p.kept_edge = (i64*)((char*)extra + packed_bytes);
-      p.kept_row = (u32*)((char*)extra + packed_bytes + edge_bytes);
-      p.totals = (u32*)((char*)extra + packed_bytes + edge_bytes + row_bytes);
+      p.kept_edge = (i64*)extra;
+      p.kept_row = (u32*)((char*)extra + edge_bytes);
+      p.kept_at = (u32*)((char*)extra + edge_bytes + row_bytes);
+      p.totals = (u32*)((char*)extra + edge_bytes + 2 * row_bytes);
       p.warp_before = p.totals + kInThreads;
+      p.warp_kept = p.warp_before + kInThreads * kInWarps;
       p.c = ColRowParams{indptr, indices, num_cols, column_ids, S, sub_indptr, D, nullptr, G, encoding_size, table,
                          renumber ? 1 : 0, out_indptr, out_indices, out_select, data, e_ids, out_data, ctx_counters(ctx),
                          TileState{}, nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0}};
@@ -678,8 +741,8 @@ int gsb_col_row_slice(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
       {
         ScopedKernelTimer timer(ctx, KID_ROW_FILTER, stream);
         void* args[] = {&p};
-        st = launch_cooperative(ctx, stream, (const void*)k_induced, grid, kInThreads,
-                                p.bloom.words ? ((size_t)1 << (64 - p.bloom.shift)) / 8 : 0, args, p.sync);
+        st = launch_cooperative(ctx, stream, kernel, grid, kInThreads,
+                                p.bloom.words ? ((size_t)1 << (32 - p.bloom.shift)) / 8 : 0, args, p.sync);
       }
       if (st != GSB_OK) return st;
       return finish_count(ctx, stream, p.c.mail, nnz_host);

@@ -30,13 +30,13 @@ namespace gsb {
 // from the upper bound seeds * (1 + bound_k), which is known before sampling.
 // what & 1: write region_off; what & 2: write item_off (indices_ptr is valid); what & 8: region_off receives the first BUCKET of every minibatch instead of a table
 // region (partition_relabel.cu; slot_capacity then bounds the bucket count); what & 32: bucket_count, the array of
-// per-bucket item counts that the counting sampler will add to, is cleared (slot_capacity + 1 words).
+// per-bucket item counts that the counting sampler will add to, is cleared (slot_capacity + 1 words).  bucket_parts > 0: so many buckets in every minibatch.
 // seeds_bound / edges_bound: what the caller sized grids, scratch and outputs for.  Device-side totals above them
 // record GSB_ERR_CAPACITY and set CNT_ABORT, which makes the kernels that follow in the call return at once; a look-back
 // that was given up since the last error was read sets it too, as the sizes here may be its results.
 __global__ void __launch_bounds__(kBThreads) k_batch_layout(BatchLayout L, i64* counters, i64 bound_k, int what,
                                                             i64 seeds_bound, i64 edges_bound,
-                                                            uint32_t* bucket_count = nullptr) {
+                                                            uint32_t* bucket_count = nullptr, i64 bucket_parts = 0) {
   __shared__ i64 s_scan[33];
   __shared__ i64 s_carry;
   if (threadIdx.x == 0) {
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kBThreads) k_batch_layout(BatchLayout L, i64* 
       if (what & 2) L.item_off[b] = L.seeds_ptr[b] + L.indices_ptr[b];
       const i64 items = bound_k >= 0 ? (L.seeds_ptr[b + 1] - L.seeds_ptr[b]) * (1 + bound_k)
                                      : L.seeds_ptr[b + 1] + L.indices_ptr[b + 1] - L.seeds_ptr[b] - L.indices_ptr[b];
-      size = (what & 8) ? (items + kBucketTarget - 1) / kBucketTarget : region_size_for(items);
+      size = !(what & 8) ? region_size_for(items) : bucket_parts > 0 ? bucket_parts : (items + kBucketTarget - 1) / kBucketTarget;
     }
     i64 total;
     const i64 excl = block_exclusive_scan<kBThreads>(size, s_scan, &total);
@@ -620,7 +620,8 @@ constexpr i64 kPartitionAutoItems = 1ll << 19;
 // a window of 256 buckets, a call of 500 minibatches of 740 000 items ran on the hash regions: 28.6 ms of the hop.)
 constexpr i64 kPartitionAutoMaxMinibatch = 1024ll * kBucketTarget;
 // The counting sampler flushes its per-bucket counts once per 128 columns: with more than 256 buckets a minibatch that is
-// an atomic for every other item, and the separate counting pass is cheaper.
+// an atomic for every other item, and the separate counting pass is cheaper (and with 151 ranges, too: sampling 8.2 -> 9.3 ms
+// against 0.67 for the pass, last hop of 500 minibatches of 813 000 items).
 constexpr i64 kSamplerCountsMaxMinibatch = 256ll * kBucketTarget;
 static inline bool partition_suits(i64 n_cap, i64 G) {
   return n_cap >= kPartitionAutoItems && n_cap / (G > 0 ? G : 1) <= kPartitionAutoMaxMinibatch;
@@ -700,9 +701,10 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
     return direct_unique_relabel_launch(ctx, stream, L, T, n_cap, edges_bound, out_unique, out_unique_ptr,
                                         out_relabeled, mail);
   }
-  if (path == 3 || (path == 0 && partition_suits(n_cap, G))) {
+  if (path >= 3 || (path == 0 && partition_suits(n_cap, G))) {
     // partitioned form (the default for large calls when the direct-address tables above were not chosen): shared-memory tables per bucket of items, then ranking by bit vectors
-    const i64 bucket_cap = partition_bucket_capacity(n_cap, G);
+    const i64 parts = path == 3 ? 0 : partition_range_parts(num_nodes, n_cap / G, G, path == 4);
+    const i64 bucket_cap = partition_bucket_capacity(n_cap, G, parts);
     int st = ctx_reserve_workspace(ctx, stream, 3 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
     if (st != GSB_OK) return st;
     L.item_off = (i64*)ws;
@@ -716,10 +718,10 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
     }
     {
       ScopedKernelTimer timer(ctx, KID_OTHER, stream);
-      k_batch_layout<<<1, kBThreads, 0, stream>>>(L, counters, -1, 1 | 2 | 8, seeds_bound, edges_bound);
+      k_batch_layout<<<1, kBThreads, 0, stream>>>(L, counters, -1, 1 | 2 | 8, seeds_bound, edges_bound, nullptr, parts);
     }
     GSB_LAUNCH_OK();
-    return partition_unique_relabel(ctx, stream, L, n_cap, bucket_cap, (char*)ws + 3 * off_bytes, false, out_unique,
+    return partition_unique_relabel(ctx, stream, L, n_cap, bucket_cap, (char*)ws + 3 * off_bytes, parts, false, out_unique,
                                     out_unique_ptr, out_relabeled, mail);
   }
   if (!L.indices_ptr) return GSB_ERR_INVALID_ARGUMENT;  // the forms below expect both arrays
@@ -766,13 +768,13 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
 // and every id it samples to its bucket's count while it holds them, and the counting pass over the items is not run.
 static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, const i64* indices,
                                    i64 num_nodes, const i64* seeds, const i64* seeds_ptr, const i64* batch_ids, i64 G,
-                                   i64 S, i64 k, i64 cap, int replace, u64 seed, i64* out_indptr, i64* out_indices,
+                                   i64 S, i64 k, i64 cap, i64 parts, int replace, u64 seed, i64* out_indptr, i64* out_indices,
                                    i64* out_select, i64* out_indices_ptr, i64* out_unique, i64* out_unique_ptr,
                                    i64* out_relabeled, Mail mail) {
   i64* counters = ctx_counters(ctx);
   const i64 n_cap = S + cap;
   const size_t off_bytes = ((size_t)(G + 1) * 8 + 255) & ~(size_t)255;
-  const i64 bucket_cap = partition_bucket_capacity(S * (1 + k), G);
+  const i64 bucket_cap = partition_bucket_capacity(S * (1 + k), G, parts);
   void* ws;
   int st = ctx_reserve_workspace(ctx, stream, 2 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
   if (st != GSB_OK) return st;
@@ -789,17 +791,17 @@ static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64*
   L.slot_capacity = bucket_cap;
   {
     ScopedKernelTimer timer(ctx, KID_OTHER, stream);
-    k_batch_layout<<<1, kBThreads, 0, stream>>>(L, counters, k, 1 | 8 | 32, S, cap, partition_bucket_counts(part_ws));
+    k_batch_layout<<<1, kBThreads, 0, stream>>>(L, counters, k, 1 | 8 | 32, S, cap, partition_bucket_counts(part_ws), parts);
   }
   GSB_LAUNCH_OK();
-  const SamplerCount count{partition_bucket_counts(part_ws), L.region_off};
+  const SamplerCount count{partition_bucket_counts(part_ws), L.region_off, parts > 0};
   st = sample_uniform_launch(ctx, stream, indptr, indices, num_nodes, seeds, S, k, replace, seed, out_indptr,
                              out_indices, out_select, nullptr, nullptr, nullptr, nullptr, cap, seeds_ptr + G,
                              seeds_ptr, batch_ids, G, &count);
   if (st != GSB_OK) return st;
   st = partition_after_sampler(ctx, stream, L, n_cap, bucket_cap, part_ws, out_indptr, S, cap, out_indices_ptr);
   if (st != GSB_OK) return st;
-  return partition_unique_relabel(ctx, stream, L, n_cap, bucket_cap, part_ws, true, out_unique, out_unique_ptr,
+  return partition_unique_relabel(ctx, stream, L, n_cap, bucket_cap, part_ws, parts, true, out_unique, out_unique_ptr,
                                   out_relabeled, mail);
 }
 
@@ -884,9 +886,11 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
   const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
   const bool fused = path == 0 && fused_unique_suits(ctx, n_cap, G);
   const bool direct_small = (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes && num_nodes > 0;
-  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && n_cap / G <= kSamplerCountsMaxMinibatch && (path == 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
+  const i64 parts = path == 3 || n_cap == 0 ? 0 : partition_range_parts(num_nodes, n_cap / G, G, path == 4);
+  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && n_cap / G <= kSamplerCountsMaxMinibatch &&
+      (path >= 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
     st = sage_hop_sampler_counts(ctx, stream, indptr, indices, num_nodes, seeds, seeds_ptr, batch_ids, G, S, k, cap,
-                                 replace, (u64)seed, out_indptr, out_indices, out_select, out_indices_ptr, out_unique,
+                                 parts, replace, (u64)seed, out_indptr, out_indices, out_select, out_indices_ptr, out_unique,
                                  out_unique_ptr, out_relabeled, mail);
     if (st != GSB_OK || !mail.word) return st;
     return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
@@ -1013,7 +1017,7 @@ int gsb_batch_unique(gsb_ctx* ctx, void* stream_, const int64_t* data, const int
     BatchLayout L;
     int st;
     const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
-    if (path == 3 || (path == 0 && partition_suits(n, G))) {
+    if (path >= 3 || (path == 0 && partition_suits(n, G))) {
       // large calls: the partitioned form of unique + relabel with no second array (first-occurrence order as well)
       L.seeds = data;
       L.seeds_ptr = data_ptr;

@@ -23,6 +23,7 @@
 //             written in the bucket's order; a bucket with more items than the shared-memory table is sized
 //             for (many repeats of a few hub ids, or an unlucky hash) uses a table in global memory of its own
 //             instead, so nothing depends on luck;
+//             With a bound on the ids, buckets can be ranges of them instead: see k_part_resolve_ranges;
 //   rank      the first positions brought back into the order of the items, which the scatter pass told where they went (a
 //             tile's share of a bucket is a run, so a CTA that takes the same tile reads whole sectors); bit vector of
 //             the first occurrences (ref[item] == own position), prefix counts per 32 items, then one
@@ -66,6 +67,7 @@ struct PartLayout {
   u32* found;          // [items]   in the same order: position inside the minibatch of the first occurrence of the id
   u32* ref;            // [items]   by item: where it lies in `bucketed`; from k_first_bits on what `found` says there
   u64* spill;          // tables of the buckets that do not fit shared memory: 2 x start + 32 x bucket
+  u32 range_parts;     // buckets per minibatch when they are ranges of ids, 0: buckets by hash
 };
 
 // Slot inside a bucket's table: a constant other than bucket_of_id's and one xor-shift round, so the ids of one
@@ -128,13 +130,13 @@ struct Located {
   u32 lc;      // position inside its minibatch (seeds first)
   u32 bucket;  // global bucket number
 };
-__device__ __forceinline__ Located locate(const BatchLayout& L, i64 g) {
+__device__ __forceinline__ Located locate(const BatchLayout& L, i64 g, int ranges) {
   const BatchUniform v = load_batch<false>(L, L.item_off, batch_of(L.item_off, L.G, g));
   const TileBatch t = tile_batch(L, v);
   Located r;
   r.lc = (u32)(g - v.begin);
   r.node = tile_item(t, r.lc);
-  r.bucket = t.bucket0 + bucket_of_id((u32)r.node, t.parts);
+  r.bucket = t.bucket0 + bucket_of_id((u32)r.node, t.parts, ranges);
   return r;
 }
 
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
   const i64 b_last = batch_of_warp(L.item_off, L.G, tile_end - 1);
   if (b_last - b_first >= kMaxSegments) {  // a tile over many small minibatches: every item on its own
     for (i64 g = tile_base + threadIdx.x; g < tile_end; g += kPartThreads) {
-      const Located it = locate(L, g);
+      const Located it = locate(L, g, P.range_parts);
       if (!valid_id(it.node)) continue;  // never bucketed; reported by the scatter pass
       atomicAdd(P.bucket_count + it.bucket, 1u);
     }
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
       for (u32 i = threadIdx.x; i < here; i += kPartThreads) {
         const i64 node = tile_item(t, lc0 + i);
         if (!valid_id(node)) continue;
-        const u32 k = t.bucket0 + bucket_of_id((u32)node, t.parts);
+        const u32 k = t.bucket0 + bucket_of_id((u32)node, t.parts, P.range_parts);
         atomicAdd(P.bucket_count + k, 1u);
       }
       continue;
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kPartPerThread; ++q)
-      if (valid_id(node[q])) atomicAdd(&s_cnt[bucket_of_id((u32)node[q], t.parts)], 1u);  // the others: scatter pass
+      if (valid_id(node[q])) atomicAdd(&s_cnt[bucket_of_id((u32)node[q], t.parts, P.range_parts)], 1u);  // the others: scatter pass
     __syncthreads();
     for (u32 i = threadIdx.x; i < t.parts; i += kPartThreads) {
       if (s_cnt[i] != 0) atomicAdd(P.bucket_count + t.bucket0 + i, s_cnt[i]);
@@ -200,6 +202,8 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
 constexpr int kScanThreads = 256;
 constexpr int kScanPer = 8;
 constexpr int kScanTile = kScanThreads * kScanPer;
+// Up to here the one CTA that runs between sampler and scatter pass scans the buckets too (43 000 took it 58 us; k_part_scan 9).
+constexpr i64 kScanAlongBuckets = 8192;
 
 __global__ void __launch_bounds__(kScanThreads) k_part_scan(PartLayout P, i64* counters, TileState ts) {
   __shared__ i64 s_scan[33];
@@ -239,7 +243,7 @@ __global__ void __launch_bounds__(kScanThreads) k_part_scan(PartLayout P, i64* c
 // offset of every minibatch (the sampled block's offset at the minibatch's first seed), the item offsets, the abort
 // check against the caller's bounds, and the scan of the bucket sizes that the sampler counted.
 __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const i64* __restrict__ sub_indptr, i64 S,
-                                                             i64 edges_bound, i64* indices_ptr, i64* counters) {
+                                                             i64 edges_bound, i64* indices_ptr, int scan, i64* counters) {
   __shared__ i64 s_scan[33];
   __shared__ i64 s_carry;
   __shared__ int s_abort;
@@ -263,7 +267,7 @@ __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const
     indices_ptr[b] = ip;
     L.item_off[b] = sp + ip;
   }
-  if (s_abort) return;
+  if (s_abort || !scan) return;
   const i64 buckets = L.region_off[G];
   constexpr int kPer = 8;
   for (i64 base = 0; base < buckets; base += 1024 * kPer) {
@@ -322,7 +326,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatte
   const bool uniform = (u64)lc0 + here <= (u64)t.items && t.parts <= (u32)WINDOW;
   if (!uniform) {  // a tile over several minibatches: every item straight to its place
     for (u32 i = threadIdx.x; i < here; i += THREADS) {
-      const Located it = locate(L, tile_base + i);
+      const Located it = locate(L, tile_base + i, P.range_parts);
       if (!valid_id(it.node)) {  // never bucketed: marked for the ranking passes
         raise_error(counters, GSB_ERR_INDEX_RANGE, tile_base + i);
         P.ref[tile_base + i] = 0xFFFFFFFFu;
@@ -353,7 +357,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatte
       }
       continue;
     }
-    const u32 w = bucket_of_id(id[q], t.parts);
+    const u32 w = bucket_of_id(id[q], t.parts, P.range_parts);
     where[q] = (w << 16) | atomicAdd(&s_cnt[w], 1u);  // at most 8 192 items per tile: the rank fits 16 bits
   }
   __syncthreads();
@@ -398,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatte
   __syncthreads();
   for (u32 i = threadIdx.x; i < staged; i += THREADS) {
     const u64 w = s_stage[i];
-    P.bucketed[s_delta[bucket_of_id((u32)(w >> 32), t.parts)] + i] = w;
+    P.bucketed[s_delta[bucket_of_id((u32)(w >> 32), t.parts, P.range_parts)] + i] = w;
   }
 }
 
@@ -420,6 +424,34 @@ __device__ __forceinline__ u32 table_insert_min(u64* table, u32 size, u32 h, u64
     h = h + 1 == size ? 0 : h + 1;
   }
   return 0;  // cannot happen: the table has more slots than the bucket has items
+}
+
+// A bucket that does not fit shared memory: a table of its own in global memory, by a whole CTA.
+__device__ __noinline__ void resolve_in_memory(const u64* items, u32 n, u64* table, u32* found) {
+  const u32 size = 2 * n + 32;
+  __syncthreads();
+  for (u32 i = threadIdx.x; i < size; i += blockDim.x) table[i] = kEmptyWord;
+  __syncthreads();
+  for (u32 j = threadIdx.x; j < n; j += blockDim.x) {
+    const u64 w = __ldg(items + j);
+    table_insert_min(table, size, slot_of_id((u32)(w >> 32), size), w);
+  }
+  __syncthreads();
+  for (u32 j = threadIdx.x; j < n; j += blockDim.x) {
+    const u64 w = __ldg(items + j);
+    const u32 id = (u32)(w >> 32);
+    u32 h = slot_of_id(id, size), first = 0xFFFFFFFFu;
+    for (u32 probe = 0; probe < size; ++probe) {
+      const u64 x = __ldcg(table + h);
+      if ((u32)(x >> 32) == id) {
+        first = (u32)x;
+        break;
+      }
+      if (x == kEmptyWord) break;
+      h = h + 1 == size ? 0 : h + 1;
+    }
+    found[j] = first;
+  }
 }
 
 // Shared-memory table as two 32-bit arrays, ids and smallest positions: the probe loop is a 32-bit load and two compares per
@@ -497,32 +529,59 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
         if ((u32)(q * kResolveThreads) < n && w[q] != kEmptyWord) found[q * kResolveThreads + threadIdx.x] = ref_of[q];
       continue;
     }
-    // oversized bucket (many repeats of a few ids): a table of its own in global memory
-    const u32 size = 2 * n + 32;
-    u64* table = P.spill + 2 * (u64)start + 32 * (u64)k;
+    resolve_in_memory(items, n, P.spill + 2 * (u64)start + 32 * (u64)k, found);  // many repeats of a few ids
+  }
+}
+
+// Buckets that are ranges of 2^kRangeShift ids: the table is addressed by the low bits of the id, so an item is one reduction and
+// one read in shared memory, without ids to compare and without probes.  Between HBM (12 bytes an item; half of the copy
+// bandwidth) and the latency of a bucket's load, clear, reduce and read, of which an SM has three in flight: 500 M items of 500
+// minibatches in three hops 2.82 -> 1.57 ms, the scatter pass, whose runs are longer, 2.64 -> 2.47.
+constexpr int kRangeThreads = 512;
+constexpr int kRangePer = 12;  // items of a thread that stay in registers
+constexpr int kRangeSlots = 1 << kRangeShift;
+
+__global__ void __launch_bounds__(kRangeThreads, 3) k_part_resolve_ranges(PartLayout P, i64* counters) {
+  extern __shared__ __align__(16) u32 s_first[];  // [kRangeSlots] smallest position of every id
+  if (counters[CNT_ABORT] != 0) return;
+  const u32 buckets = (u32)P.L.region_off[P.L.G];
+  for (u32 k = blockIdx.x; k < buckets; k += gridDim.x) {
+    const u32 start = P.bucket_start[k], n = P.bucket_start[k + 1] - start;
+    if (n == 0) continue;
+    if (k % P.range_parts == P.range_parts - 1) {  // ids beyond the bound
+      resolve_in_memory(P.bucketed + start, n, P.spill + 2 * (u64)start + 32 * (u64)k, P.found + start);
+      continue;
+    }
+    const u64* items = P.bucketed + start;
+    u32* found = P.found + start;
+    if (k + gridDim.x < buckets) {  // the next bucket's items on their way to L2
+      const u32 at = P.bucket_start[k + gridDim.x], end = P.bucket_start[k + gridDim.x + 1];
+      for (u32 i = at + threadIdx.x * 16; i < end; i += kRangeThreads * 16)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(P.bucketed + i));
+    }
+    u64 w[kRangePer];  // their loads are in flight while the table is cleared
+#pragma unroll
+    for (int q = 0; q < kRangePer; ++q) {
+      const u32 j = q * kRangeThreads + threadIdx.x;
+      w[q] = j < n ? __ldg(items + j) : kEmptyWord;
+    }
+    __syncthreads();  // the previous bucket's look-ups are done
+    const uint4 e = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+    for (u32 i = threadIdx.x; i < kRangeSlots / 4; i += kRangeThreads) reinterpret_cast<uint4*>(s_first)[i] = e;
     __syncthreads();
-    for (u32 i = threadIdx.x; i < size; i += kResolveThreads) table[i] = kEmptyWord;
-    __syncthreads();
-    for (u32 j = threadIdx.x; j < n; j += kResolveThreads) {
-      const u64 w = __ldg(items + j);
-      table_insert_min(table, size, slot_of_id((u32)(w >> 32), size), w);
+    auto slot = [&](u64 item) { return s_first + ((u32)(item >> 32) & (kRangeSlots - 1)); };
+#pragma unroll
+    for (int q = 0; q < kRangePer; ++q)
+      if (w[q] != kEmptyWord) atomicMin(slot(w[q]), (u32)w[q]);
+    for (u32 j = kRangePer * kRangeThreads + threadIdx.x; j < n; j += kRangeThreads) {
+      const u64 item = __ldg(items + j);
+      atomicMin(slot(item), (u32)item);
     }
     __syncthreads();
-    for (u32 j = threadIdx.x; j < n; j += kResolveThreads) {
-      const u64 w = __ldg(items + j);
-      const u32 id = (u32)(w >> 32);
-      u32 h = slot_of_id(id, size), first = 0xFFFFFFFFu;
-      for (u32 probe = 0; probe < size; ++probe) {
-        const u64 x = __ldcg(table + h);
-        if ((u32)(x >> 32) == id) {
-          first = (u32)x;
-          break;
-        }
-        if (x == kEmptyWord) break;
-        h = h + 1 == size ? 0 : h + 1;
-      }
-      found[j] = first;
-    }
+#pragma unroll
+    for (int q = 0; q < kRangePer; ++q)
+      if (w[q] != kEmptyWord) found[q * kRangeThreads + threadIdx.x] = *slot(w[q]);
+    for (u32 j = kRangePer * kRangeThreads + threadIdx.x; j < n; j += kRangeThreads) found[j] = *slot(__ldg(items + j));
   }
 }
 
@@ -732,7 +791,17 @@ __global__ void __launch_bounds__(kBitsThreads) k_rank_emit(BatchLayout L, RankA
 // ---- host sequence ----------------------------------------------------------------------------------------------------
 static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-i64 partition_bucket_capacity(i64 items_bound, i64 G) { return items_bound / kBucketTarget + G + 1; }
+// Where ranges are ahead of hashed buckets (whole call, 60 M items): of 789 items 1 583 against 1 472 us, of 1 500 1 356 / 1 448, of
+// 5 000 1 164 / 1 331, of 12 700 1 278 / 1 304, of 20 000 1 298 / 1 231 (most of them lie in no register then).  And there have to
+// be several rounds of them: 6 M items in 3 020 ranges took 206 us against 200.
+i64 partition_range_parts(i64 num_nodes, i64 items_per_minibatch, i64 G, bool forced) {
+  const i64 parts = ((num_nodes + kRangeSlots - 1) >> kRangeShift) + 1;
+  if (num_nodes <= 0 || parts > kNarrowWindow) return 0;
+  const bool suits = items_per_minibatch >= 1400 * parts && items_per_minibatch <= 12288 * parts && G * parts >= 4096;
+  return forced || suits ? parts : 0;
+}
+
+i64 partition_bucket_capacity(i64 items_bound, i64 G, i64 parts) { return parts > 0 ? G * parts : items_bound / kBucketTarget + G + 1; }
 
 size_t partition_workspace_bytes(i64 n_cap, i64 bucket_cap) {
   const size_t words = (size_t)((n_cap + 31) / 32) + 2;
@@ -778,16 +847,18 @@ int partition_after_sampler(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i6
   const PartArrays a = carve(L, n_cap, bucket_cap, ws);
   {
     ScopedKernelTimer timer(ctx, KID_OTHER, stream);
-    k_part_after_sampler<<<1, 1024, 0, stream>>>(a.P, sub_indptr, S, edges_bound, out_indices_ptr, ctx_counters(ctx));
+    k_part_after_sampler<<<1, 1024, 0, stream>>>(a.P, sub_indptr, S, edges_bound, out_indices_ptr,
+                                                 bucket_cap <= kScanAlongBuckets, ctx_counters(ctx));
   }
   GSB_LAUNCH_OK();
   return GSB_OK;
 }
 
 int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64 n_cap, i64 bucket_cap, void* ws,
-                             bool counted, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled, Mail mail) {
+                             i64 parts, bool counted, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled, Mail mail) {
   i64* counters = ctx_counters(ctx);
-  const PartArrays arrays = carve(L, n_cap, bucket_cap, ws);
+  PartArrays arrays = carve(L, n_cap, bucket_cap, ws);
+  arrays.P.range_parts = (u32)parts;
   const PartLayout& P = arrays.P;
   const RankArrays& R = arrays.R;
   const bool wide = n_cap / L.G > (i64)kNarrowWindow * kBucketTarget * 3 / 4;  // the larger minibatches of a ragged call count
@@ -797,16 +868,21 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
     GSB_CUDA_OK(cudaFuncSetAttribute(k_part_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, kBucketSlots * 8));
     GSB_CUDA_OK(cudaFuncSetAttribute(k_part_scatter<kWideWindow, 512, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      scatter_smem(8192, kWideWindow)));
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_resolve_ranges, cudaFuncAttributeMaxDynamicSharedMemorySize, kRangeSlots * 4));
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_scatter<kNarrowWindow, 512, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     scatter_smem(8192, kNarrowWindow)));
     attr_set[dev] = true;
   }
   if (!counted) {
     GSB_CUDA_OK(cudaMemsetAsync(P.bucket_count, 0, sizeof(u32) * (size_t)(bucket_cap + 1), stream));
     {
       ScopedKernelTimer timer(ctx, KID_PART_COUNT, stream);
-      if (wide) k_part_count<kWideWindow><<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
+      if (wide && parts == 0) k_part_count<kWideWindow><<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
       else k_part_count<kNarrowWindow><<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
     }
     GSB_LAUNCH_OK();
+  }
+  if (!counted || bucket_cap > kScanAlongBuckets) {
     const int scan_tiles = grid_for(bucket_cap, kScanTile);
     TileState scan_ts;
     const int st = ctx_tile_state(ctx, scan_tiles, stream, &scan_ts);
@@ -819,7 +895,10 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   }
   {
     ScopedKernelTimer timer(ctx, KID_PART_SCATTER, stream);
-    if (wide)
+    if (wide && parts > 0)
+      k_part_scatter<kNarrowWindow, 512, 16><<<grid_for(n_cap, 8192), 512, scatter_smem(8192, kNarrowWindow), stream>>>(
+          P, n_cap, counters);
+    else if (wide)
       k_part_scatter<kWideWindow, 512, 16><<<grid_for(n_cap, 8192), 512, scatter_smem(8192, kWideWindow), stream>>>(
           P, n_cap, counters);
     else
@@ -829,7 +908,10 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   GSB_LAUNCH_OK();
   {
     ScopedKernelTimer timer(ctx, KID_PART_RESOLVE, stream);
-    k_part_resolve<<<(int)min(bucket_cap, (i64)kNumSMs * 4 * 4), kResolveThreads, kBucketSlots * 8, stream>>>(P, counters);
+    if (parts > 0)
+      k_part_resolve_ranges<<<(int)min(bucket_cap, (i64)kNumSMs * 3 * 4), kRangeThreads, kRangeSlots * 4, stream>>>(P, counters);
+    else
+      k_part_resolve<<<(int)min(bucket_cap, (i64)kNumSMs * 4 * 4), kResolveThreads, kBucketSlots * 8, stream>>>(P, counters);
   }
   GSB_LAUNCH_OK();
   {

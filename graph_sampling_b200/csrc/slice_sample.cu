@@ -220,6 +220,7 @@ struct SampleParams {
   // every seed and every sampled id adds one to the count of its bucket.
   uint32_t* bucket_count;
   const i64* bucket_base;  // [G + 1] first bucket of every minibatch
+  int bucket_ranges;       // buckets are ranges of ids
   Mail mail;               // the edge total, for a caller that waits for it
 };
 
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
       const i64 win = b0 - s_win0;  // >= 0: minibatches follow the CTA's first one
       auto count_id = [&](i64 id) {
         if (id < 0 || id >= 0xFFFFFFFFll) return;  // never bucketed; reported by the pass that scatters the items
-        const i64 w = win + bucket_of_id((uint32_t)id, parts);
+        const i64 w = win + bucket_of_id((uint32_t)id, parts, p.bucket_ranges);
         if (w < kCountWindow) atomicAdd(&s_cnt[w], 1u);
         else atomicAdd(p.bucket_count + s_win0 + w, 1u);
       };
@@ -596,11 +597,12 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
   SampleParams p{indptr,     indices,     num_cols, seeds, S,        k,        replace,           seed, out_indptr,
                  out_indices, out_select, out_coo_col, data, e_ids, out_data, capacity, ctx_counters(ctx), ts,
                  S_dev,      batch_ptr,  batch_ptr ? batch_ids : nullptr,
-                 batch_ptr ? G : 0,      nullptr,    nullptr, mail};
+                 batch_ptr ? G : 0,      nullptr,    nullptr, 0, mail};
   if (count && count->bucket_count) {
     if (!per_thread || !batch_ptr || G < 1) return GSB_ERR_INVALID_ARGUMENT;
     p.bucket_count = count->bucket_count;
     p.bucket_base = count->bucket_base;
+    p.bucket_ranges = count->ranges;
   }
   {
     ScopedKernelTimer timer(ctx, KID_SAMPLE_UNIFORM, stream);

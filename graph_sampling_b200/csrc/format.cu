@@ -76,6 +76,237 @@ __global__ void __launch_bounds__(kFmtThreads) k_conversion_end(const i64* __res
   for (i64 e = first; e < E; e += step) out_other[e] = other[perm && !lost ? perm[e] : e];
 }
 
+// Lanes that hold the same value of up to 2^bits, among the lanes where `valid` holds.  A ballot per bit: __match_any_sync takes
+// its time once per DISTINCT value, 0.5 us for 32 of them.
+__device__ __forceinline__ unsigned same_digit(u32 d, int bits, bool valid) {
+  unsigned peers = __ballot_sync(0xffffffffu, valid);
+  for (int b = 0; b < bits; ++b) {
+    const bool one = (d >> b) & 1u;
+    const unsigned ones = __ballot_sync(0xffffffffu, one);
+    peers &= one ? ones : ~ones;
+  }
+  return peers;
+}
+
+// ---- COO -> CSC / CSR of a short list, without a barrier ----------------------------------------------------------------
+// The keys of up to 26 624 edges are read from L2 by EVERY CTA (213 KB at most; 6 us for the 25 000 edges of a layer-wise
+// minibatch), which needs nothing from the others then: a CTA owns a range of keys, counts the edges with smaller keys (where
+// its output starts) and keeps, in order, those of its range; counts per key, their scan (the offsets) and the stable placing, a
+// warp per part of the range, happen in shared memory.  A CTA with many edges, whose keys may well be the same, sorts them by two
+// digits instead, every warp a part of them.  The cooperative form below, with five grid barriers and 65 536 counters to clear
+// and sum up per CTA and digit, takes 42 us for 25 000 edges over a million keys and 17 us for 700 over a thousand, this 16.4 and
+// 8.9 (calls in a row); 37 when the keys crowd at one end of their range, as those of a power law do whose ids are sorted by
+// degree, and 29 % of the edges are one CTA's.
+constexpr int kShortThreads = 1024;
+constexpr int kShortWarps = kShortThreads / 32;
+constexpr int kKeysAhead = 12;  // keys, and placed edges, of a thread on their way
+constexpr int kShortAhead = 8;
+// At this many edges the two forms are equal where the keys crowd as those of a power law whose ids are sorted by degree; with keys
+// spread evenly this form takes 16.7 us at 32 700 edges, the other 35 to 42.
+constexpr i64 kShortMaxEdges = 26624;
+constexpr u32 kShortHeavy = 1024;  // edges of a CTA from which every warp places a part of them
+constexpr int kShortDigitBits = 7;
+constexpr i64 kShortMaxKeys = 8192;  // of a CTA
+constexpr size_t short_smem(i64 E, i64 keys) { return 4 * (size_t)keys + 4 * (size_t)((E + 1) & ~1ll); }
+
+__global__ void __launch_bounds__(kShortThreads, 1) k_coo2csc_short(const i64* __restrict__ key, const i64* __restrict__ other,
+                                                                   u32 E, i64 num_keys, u32 keys_per_cta,
+                                                                   i64* __restrict__ out_indptr, i64* __restrict__ out_other,
+                                                                   i64* __restrict__ out_perm,
+                                                                   uint16_t* __restrict__ scratch, i64* counters) {
+  extern __shared__ __align__(16) u32 s_start[];  // [keys] counts, then where the next edge of the key goes
+  uint16_t* s_rel = reinterpret_cast<uint16_t*>(s_start + keys_per_cta);  // [E] key relative to the range, or kOutside
+  uint16_t* s_list = s_rel + ((E + 1) & ~1u);                             // [E] the edges of the range, in order
+  __shared__ u32 s_warp[2][kShortWarps];
+  constexpr u32 kOutside = 0xFFFFu;
+  const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
+  const i64 key_begin = (i64)blockIdx.x * keys_per_cta;
+  const u32 keys = (u32)max((i64)0, min((i64)keys_per_cta, num_keys - key_begin));
+  const u32 per_warp = (E + kShortThreads - 1) / kShortThreads * 32;
+  const u32 begin = min(E, warp * per_warp), end = min(E, begin + per_warp);
+  for (u32 k = tid; k < keys; k += kShortThreads) s_start[k] = 0;
+  __syncthreads();
+  u32 below = 0, inside = 0;  // of the lane's edges
+  for (u32 i0 = begin + lane; i0 < end; i0 += 32 * kKeysAhead) {
+    i64 k[kKeysAhead];
+#pragma unroll
+    for (int q = 0; q < kKeysAhead; ++q) k[q] = i0 + 32 * q < end ? __ldg(key + i0 + 32 * q) : num_keys;
+#pragma unroll
+    for (int q = 0; q < kKeysAhead; ++q) {
+      const u32 i = i0 + 32 * q;
+      if (i >= end) break;
+      if ((u64)k[q] >= (u64)num_keys) {
+        if (blockIdx.x == 0) raise_error(counters, GSB_ERR_INDEX_RANGE, i);
+        k[q] = 0;
+      }
+      const i64 rel = k[q] - key_begin;
+      const bool in = (u64)rel < (u64)keys;
+      s_rel[i] = in ? (uint16_t)rel : (uint16_t)kOutside;
+      if (in) atomicAdd(s_start + rel, 1u);
+      inside += in;
+      below += rel < 0;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    inside += __shfl_xor_sync(0xffffffffu, inside, o);
+    below += __shfl_xor_sync(0xffffffffu, below, o);
+  }
+  if (lane == 0) {
+    s_warp[0][warp] = inside;
+    s_warp[1][warp] = below;
+  }
+  __syncthreads();
+  u32 at = 0, total = 0;
+  below = 0;
+#pragma unroll
+  for (u32 w = 0; w < kShortWarps; ++w) {
+    if (w < warp) at += s_warp[0][w];
+    total += s_warp[0][w];
+    below += s_warp[1][w];
+  }
+  if (inside > 0)  // (the whole warp's)
+    for (u32 i0 = begin; i0 < end; i0 += 32) {
+      const bool in = i0 + lane < end && s_rel[i0 + lane] != kOutside;
+      const unsigned bits = __ballot_sync(0xffffffffu, in);
+      if (in) s_list[at + __popc(bits & lt)] = (uint16_t)(i0 + lane);
+      at += __popc(bits);
+    }
+  // offsets: a stretch of keys per thread, eight at most
+  {
+    constexpr u32 kPer = kShortMaxKeys / kShortThreads;
+    const u32 per = (keys + kShortThreads - 1) / kShortThreads, first = tid * per;
+    u32 v[kPer], sum = 0;
+#pragma unroll
+    for (u32 j = 0; j < kPer; ++j) {
+      v[j] = j < per && first + j < keys ? s_start[first + j] : 0;
+      sum += v[j];
+    }
+    u32 inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    __syncthreads();  // s_warp has been read
+    if (lane == 31) s_warp[0][warp] = inc;
+    __syncthreads();
+    u32 run = inc - sum;
+#pragma unroll
+    for (u32 w = 0; w < kShortWarps; ++w)
+      if (w < warp) run += s_warp[0][w];
+#pragma unroll
+    for (u32 j = 0; j < kPer; ++j) {
+      if (j < per && first + j < keys) s_start[first + j] = run;
+      run += v[j];
+    }
+    __syncthreads();
+    for (u32 k = tid; k < keys; k += kShortThreads) out_indptr[key_begin + k] = (i64)(below + s_start[k]);
+    if (blockIdx.x == 0 && tid == 0) out_indptr[num_keys] = (i64)E;
+    __syncthreads();
+  }
+  // the edges in their new order, placed by the two ways below; the outputs follow from it in one go (a warp that wrote them while
+  // placing waited for a random read every 32 edges)
+  constexpr u32 kDigits = 1u << kShortDigitBits;
+  __shared__ uint16_t s_digit[kShortWarps][kDigits];  // of a warp's part, then where its next edge of the digit goes
+  __shared__ u32 s_digit_start[kDigits];
+  static_assert(kShortWarps * kDigits >= kShortHeavy, "the order of a light CTA takes the place of the digits");
+  uint16_t* order = &s_digit[0][0];
+  if (total >= kShortHeavy) {  // a stable counting sort by one or two digits of the key
+    const u32 share = (total + kShortThreads - 1) / kShortThreads * 32;
+    const u32 lo = min(total, warp * share), hi = min(total, lo + share);
+    const int key_bits = keys > 1 ? 32 - __clz(keys - 1) : 0, passes = key_bits > kShortDigitBits ? 2 : 1;
+    uint16_t* second = 2 * total <= E ? s_list + total : scratch + below;
+    for (int pass = 0; pass < passes; ++pass) {
+      const uint16_t* list = pass == 0 ? s_list : second;
+      order = pass == 0 ? second : s_list;
+      const int bits = pass == 0 ? min(key_bits, kShortDigitBits) : key_bits - kShortDigitBits;
+      auto digit_of = [&](u32 e) { return ((u32)s_rel[e] >> (pass * kShortDigitBits)) & (kDigits - 1); };
+      for (u32 d = lane; d < kDigits; d += 32) s_digit[warp][d] = 0;
+      __syncwarp();
+#pragma unroll 4
+      for (u32 j0 = lo; j0 < hi; j0 += 32) {
+        const bool valid = j0 + lane < hi;
+        const u32 d = valid ? digit_of(list[j0 + lane]) : 0;
+        const unsigned peers = same_digit(d, bits, valid);
+        if (valid && (peers & lt) == 0) s_digit[warp][d] += (uint16_t)__popc(peers);
+        __syncwarp();
+      }
+      __syncthreads();
+      if (tid < kDigits) {
+        u32 run = 0;
+        for (u32 w = 0; w < kShortWarps; ++w) {
+          const u32 c = s_digit[w][tid];
+          s_digit[w][tid] = (uint16_t)run;
+          run += c;
+        }
+        s_digit_start[tid] = run;
+      }
+      __syncthreads();
+      if (warp == 0) {
+        u32 carry = 0;
+        for (u32 d0 = 0; d0 < kDigits; d0 += 32) {
+          const u32 c = s_digit_start[d0 + lane];
+          u32 inc = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+          }
+          s_digit_start[d0 + lane] = carry + inc - c;
+          carry += __shfl_sync(0xffffffffu, inc, 31);
+        }
+      }
+      __syncthreads();
+      for (u32 j0 = lo; j0 < hi; j0 += 32) {
+        const bool valid = j0 + lane < hi;
+        const u32 e = valid ? list[j0 + lane] : 0, d = valid ? digit_of(e) : 0;
+        const unsigned peers = same_digit(d, bits, valid);
+        u32 pos = 0;
+        if (valid) pos = s_digit[warp][d];
+        __syncwarp();
+        if (valid && (peers & lt) == 0) s_digit[warp][d] = (uint16_t)(pos + __popc(peers));
+        __syncwarp();
+        if (valid) order[pos + s_digit_start[d] + __popc(peers & lt)] = (uint16_t)e;
+      }
+      __syncthreads();  // the other list is complete
+    }
+  } else {  // a warp takes the edges of its part of the range, in order
+    const u32 part = (keys + kShortWarps - 1) / kShortWarps, part_begin = warp * part;
+    const u32 part_keys = min(part, keys - min(keys, part_begin));
+    for (u32 j0 = 0; j0 < total && part_keys > 0; j0 += 32) {
+      const u32 e = j0 + lane < total ? s_list[j0 + lane] : 0;
+      const u32 rel = s_rel[e];
+      const bool mine = j0 + lane < total && rel - part_begin < part_keys;
+      if (!__any_sync(0xffffffffu, mine)) continue;
+      const unsigned peers = __match_any_sync(0xffffffffu, mine ? rel : kOutside);
+      u32 pos = 0;
+      if (mine) pos = s_start[rel];
+      __syncwarp();
+      if (mine && (peers & lt) == 0) s_start[rel] = pos + __popc(peers);
+      __syncwarp();
+      if (mine) order[pos + __popc(peers & lt)] = (uint16_t)e;
+    }
+    __syncthreads();
+  }
+  for (u32 j0 = tid; j0 < total; j0 += kShortThreads * kShortAhead) {
+    u32 e[kShortAhead];
+    i64 o[kShortAhead];
+#pragma unroll
+    for (int q = 0; q < kShortAhead; ++q) e[q] = j0 + q * kShortThreads < total ? order[j0 + q * kShortThreads] : 0;
+#pragma unroll
+    for (int q = 0; q < kShortAhead; ++q)
+      if (j0 + q * kShortThreads < total) o[q] = __ldg(other + e[q]);
+#pragma unroll
+    for (int q = 0; q < kShortAhead; ++q) {
+      const u32 j = j0 + q * kShortThreads;
+      if (j >= total) break;
+      out_perm[below + j] = (i64)e[q];
+      out_other[below + j] = o[q];
+    }
+  }
+}
+
 // ---- COO -> CSC / CSR in one launch ------------------------------------------------------------------------------
 // Stable counting sort of E edges by key with the offsets over all keys, as one cooperative kernel with a grid barrier
 // between its steps.  The slices that layer-wise sampling converts have 10^4 to 10^6 edges: the radix sort's fifteen
@@ -86,7 +317,7 @@ __global__ void __launch_bounds__(kFmtThreads) k_conversion_end(const i64* __res
 //              digit in shared memory; the CTA's counts go to matrix[digit][c]
 //     scan     a warp per digit (a thread when there are few CTAs: a single one took 10 of its 23 us to walk 1 024 rows a
 //              warp at a time) turns its row of the matrix into exclusive prefixes, and notes the digit's total
-//     place    every warp walks its part again, 32 items at a time ranked with __match_any_sync, and writes each item to
+//     place    every warp walks its part again, 32 items at a time ranked by ballots, and writes each item to
 //              digit start + CTA prefix + warp prefix + rank: stable, since everything is numbered in order
 //   along the way, the offsets: counts per key (one reduction per edge) during the first scan, totals per CTA of keys
 //   during the first place, offsets written during the next step.
@@ -182,8 +413,8 @@ __global__ void __launch_bounds__(kConvThreads) k_coo2csc(const __grid_constant_
     for (u32 i0 = begin; i0 < end; i0 += 32) {
       const u32 i = i0 + lane;
       const bool valid = i < end;
-      const u32 d = valid ? (u32)(load_item(digit, i) >> shift) & mask : 0xFFFFFFFFu;
-      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const u32 d = valid ? (u32)(load_item(digit, i) >> shift) & mask : 0;
+      const unsigned peers = same_digit(d, p.digit_bits, valid);
       if (valid && (peers & lt) == 0) my_count[d] = (uint16_t)(my_count[d] + __popc(peers));
       __syncwarp();
     }
@@ -261,8 +492,8 @@ __global__ void __launch_bounds__(kConvThreads) k_coo2csc(const __grid_constant_
       const u32 i = i0 + lane;
       const bool valid = i < end;
       const u64 item = valid ? load_item(digit, i) : 0;
-      const u32 d = valid ? (u32)(item >> shift) & mask : 0xFFFFFFFFu;
-      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const u32 d = valid ? (u32)(item >> shift) & mask : 0;
+      const unsigned peers = same_digit(d, p.digit_bits, valid);
       u32 base = 0;
       if (valid) base = my_count[d];
       __syncwarp();
@@ -340,6 +571,24 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
   const int grid = min(grid_for(E, kFmtThreads), kNumSMs * 8);
   int bits = 1;
   while (bits < 63 && (1ll << bits) < num_keys) ++bits;
+  if (!key_sorted && E > 0 && E <= kShortMaxEdges && num_keys > 0 && num_keys <= kShortMaxKeys * kNumSMs) {
+    static bool attr_set[64];
+    const int dev = ctx_device(ctx);
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+      GSB_CUDA_OK(cudaFuncSetAttribute(k_coo2csc_short, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)short_smem(kShortMaxEdges, kShortMaxKeys)));
+      attr_set[dev] = true;
+    }
+    const u32 keys_per_cta = (u32)((num_keys + kNumSMs - 1) / kNumSMs);
+    void* scratch;
+    const int st = ctx_reserve_workspace(ctx, stream, sizeof(uint16_t) * (size_t)E, &scratch);
+    if (st != GSB_OK) return st;
+    ScopedKernelTimer timer(ctx, KID_FORMAT, stream);
+    k_coo2csc_short<<<grid_for(num_keys, (int)keys_per_cta), kShortThreads, short_smem(E, keys_per_cta), stream>>>(
+        key, other, (u32)E, num_keys, keys_per_cta, out_indptr, out_other, out_perm, (uint16_t*)scratch, ctx_counters(ctx));
+    GSB_LAUNCH_OK();
+    return GSB_OK;
+  }
   // One cooperative launch while a warp's share of the edges fits its 16-bit counts (and keys fit three digits);
   // beyond that the passes are long enough for launches of their own.
   if (!key_sorted && E > 0 && E <= kConvMaxEdges && bits <= 32 && num_keys > 0) {

@@ -53,12 +53,18 @@ __device__ __forceinline__ void grid_share(i64 n, F f) {
 // runs `give_up`, and the CTA ends here.  It ends by an instruction, and one thread does the work where it waits anyway: with a
 // branch to code for all threads, or to the end of the kernel, the compiler keeps more alive across the barrier (36 spilled bytes
 // in the weighted sampler, 10 000 columns with replacement 217 -> 259 us).
-template <class F>
-__device__ __forceinline__ void grid_barrier(const GridSync& g, u32 index, F give_up) {
-  bool ok = true;
+//
+// grid_barrier_arrive and grid_barrier_wait are its halves, for work in between that needs nothing from other CTAs; a CTA waits
+// before it arrives at the next barrier.
+__device__ __forceinline__ void grid_barrier_arrive(const GridSync& g) {
   __syncthreads();
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(g.word) : "memory");
+}
+
+template <class F>
+__device__ __forceinline__ void grid_barrier_wait(const GridSync& g, u32 index, F give_up) {
+  bool ok = true;
   if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(g.word) : "memory");
     const u64 target = g.base + (u64)index * gridDim.x;
     int polls = 0;
     for (;;) {
@@ -78,6 +84,12 @@ __device__ __forceinline__ void grid_barrier(const GridSync& g, u32 index, F giv
     }
   }
   if (!__syncthreads_and(ok)) asm volatile("exit;");
+}
+
+template <class F>
+__device__ __forceinline__ void grid_barrier(const GridSync& g, u32 index, F give_up) {
+  grid_barrier_arrive(g);
+  grid_barrier_wait(g, index, give_up);
 }
 
 // CTAs of a kernel that are resident at once on the context's device (0: cooperative launches are not available).  The

@@ -26,16 +26,25 @@ __device__ __forceinline__ uint32_t orderable_f32(float f) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+__device__ __forceinline__ uint32_t weighted_key(float w, i64 i, u64 seed) {
+  if (!(w > 0.0f)) return orderable_f32(ares_key(0, w));  // whatever the draw: most rows of a layer's list have no weight
+  return orderable_f32(ares_key(rand_u32(seed, (u64)i, 0, STREAM_LIST_WEIGHTED), w));
+}
+
+__device__ __forceinline__ u64 composite_of(uint32_t key, i64 i) { return ((u64)key << 32) | (u64)(0xFFFFFFFFu - (uint32_t)i); }
+
 __device__ __forceinline__ u64 list_composite(const float* __restrict__ probs, i64 i, u64 seed) {
-  const uint32_t key = probs ? orderable_f32(ares_key(rand_u32(seed, (u64)i, 0, STREAM_LIST_WEIGHTED), __ldg(probs + i)))
-                             : rand_u32(seed, (u64)i, 0, STREAM_LIST);
-  return ((u64)key << 32) | (u64)(0xFFFFFFFFu - (uint32_t)i);
+  return composite_of(probs ? weighted_key(__ldg(probs + i), i, seed) : rand_u32(seed, (u64)i, 0, STREAM_LIST), i);
 }
 
 // Sampling without replacement of k <= kSelectMaxK items in one launch: composites -> radix select, 11 bits per pass, a
 // grid barrier per pass, until the selected bin is needed whole (two or three passes unless keys tie) -> the winners are
-// appended in any order -> CTA 0 sorts and emits them.  Layer-wise sampling makes one such call per layer on a list of a
-// million rows; as thirteen launches it was 140 us, most of it between the launches (30 us now).
+// appended in any order -> every warp counts, for one of them after the other, the winners that rank before it, and puts it there
+// (with few CTAs for many winners CTA 0 sorts them).  Layer-wise sampling makes one such call per layer on a list of a
+// million rows; as thirteen launches it was 140 us, most of it between the launches; with composites read again in every pass
+// and a sort in one CTA 31 us for 512 of a million, of which four were a re-reading each and six the sort; 22 now (4 096 of a
+// million 70 -> 29).  Its grid barriers, four to eight of them, bound it.
+// KEPT: a thread's keys, up to eight, stay in its registers.
 constexpr int kSelectThreads = 1024;
 constexpr int kSelectBins = 2048;
 constexpr int kSelectMaxK = 4096;
@@ -57,16 +66,31 @@ struct SelectParams {
   GridSync sync;
 };
 
-// One entry of a shared-memory histogram per distinct digit of the warp: all zero-weight items share one key, and plain
-// atomics on one address would serialise the CTA.
+// Adds the warp's digits to a shared-memory histogram: the lanes that share the first one's digit, and then those that share the
+// first of the others', add once (all zero-weight items share one key, and plain atomics on one address would serialise the
+// CTA); the rest add one by one (__match_any_sync, which gathers all of them, takes 0.5 us for 32 distinct digits).
 __device__ __forceinline__ void select_count(unsigned* s_hist, unsigned digit, bool counts) {
-  const unsigned peers = __match_any_sync(0xffffffffu, counts ? digit : 0xFFFFFFFFu);
-  if (counts && (int)(__ffs(peers) - 1) == (int)(threadIdx.x & 31)) atomicAdd(&s_hist[digit], (unsigned)__popc(peers));
+  unsigned rest = __ballot_sync(0xffffffffu, counts);
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    if (rest == 0) return;
+    const int first = __ffs(rest) - 1;
+    const unsigned same = __ballot_sync(0xffffffffu, digit == __shfl_sync(0xffffffffu, digit, first)) & rest;
+    if ((int)(threadIdx.x & 31) == first) atomicAdd(&s_hist[digit], (unsigned)__popc(same));
+    rest &= ~same;
+  }
+  if ((rest >> (threadIdx.x & 31)) & 1u) atomicAdd(&s_hist[digit], 1u);
 }
+
+constexpr int kSelectKept = 8;
+// Winners per CTA up to which all CTAs rank them: a rank is k comparisons by a warp (4 096 winners on 22 CTAs about 16 us, 512 on
+// three 2), the sort of one CTA 35 us for 4 096 and 6.5 for 512.
+constexpr i64 kSelectRanked = 192;
 
 // (two CTAs per SM are never launched: the bound is for 32 registers, with 45 the passes over ten million items take 170 us
 // instead of 160)
-__global__ void __launch_bounds__(kSelectThreads, 2) k_list_select(const __grid_constant__ SelectParams p) {
+template <bool KEPT>
+__global__ void __launch_bounds__(kSelectThreads, KEPT ? 1 : 2) k_list_select(const __grid_constant__ SelectParams p) {
   __shared__ __align__(16) u64 s_win[kSelectMaxK];   // the histogram of a pass, later the winners
   __shared__ unsigned s_warp[kSelectThreads / 32];
   __shared__ unsigned s_pick[2];                     // bin, items of it that are needed
@@ -77,14 +101,44 @@ __global__ void __launch_bounds__(kSelectThreads, 2) k_list_select(const __grid_
   for (i64 i = (i64)blockIdx.x * kSelectThreads + tid; i < kSelectPasses * kSelectBins; i += stride) p.hist[i] = 0;
   if (blockIdx.x == 0 && tid == 0) *p.found = 0;
   for (int i = tid; i < kSelectBins; i += kSelectThreads) s_hist[i] = 0;
-  __syncthreads();
-  for (i64 r = 0; r < rounds; ++r) {
-    const i64 i = r * stride + (i64)blockIdx.x * kSelectThreads + tid;
-    const bool valid = i < p.N;
-    const u64 c = valid ? list_composite(p.probs, i, p.seed) : 0;
-    if (valid) p.composite[i] = c;
-    select_count(s_hist, (unsigned)(c >> 53), valid);
+  grid_barrier_arrive(p.sync);
+  const i64 own = (i64)blockIdx.x * kSelectThreads + tid;  // the thread's items: own, own + stride, ...
+  uint32_t key[KEPT ? kSelectKept : 1];
+  if (KEPT) {
+    float w[kSelectKept];
+#pragma unroll
+    for (int r = 0; r < kSelectKept; ++r) w[r] = p.probs && own + r * stride < p.N ? __ldg(p.probs + own + r * stride) : 0.0f;
+#pragma unroll
+    for (int r = 0; r < kSelectKept; ++r) {
+      const i64 i = own + r * stride;
+      key[r] = 0;
+      if (i < p.N) key[r] = p.probs ? weighted_key(w[r], i, p.seed) : rand_u32(p.seed, (u64)i, 0, STREAM_LIST);
+    }
+#pragma unroll
+    for (int r = 0; r < kSelectKept; ++r)
+      if (r < rounds) select_count(s_hist, key[r] >> 21, own + r * stride < p.N);
+  } else {
+    for (i64 r = 0; r < rounds; ++r) {
+      const i64 i = r * stride + own;
+      const bool valid = i < p.N;
+      const u64 c = valid ? list_composite(p.probs, i, p.seed) : 0;
+      if (valid) p.composite[i] = c;
+      select_count(s_hist, (unsigned)(c >> 53), valid);
+    }
   }
+  // f(item's composite, whether there is an item) for the thread's items, in all lanes
+  auto for_composites = [&](auto f) {
+    if (KEPT) {
+#pragma unroll
+      for (int r = 0; r < kSelectKept; ++r)
+        if (r < rounds) f(composite_of(key[r], own + r * stride), own + r * stride < p.N);
+    } else {
+      for (i64 r = 0; r < rounds; ++r) {
+        const i64 i = r * stride + own;
+        f(i < p.N ? p.composite[i] : 0ull, i < p.N);  // written by this very thread
+      }
+    }
+  };
   // The result of a call that was given up: the first k items.
   auto give_up = [&] {
     for (i64 i = 0; blockIdx.x == 0 && i < p.k; ++i) {
@@ -93,7 +147,7 @@ __global__ void __launch_bounds__(kSelectThreads, 2) k_list_select(const __grid_
     }
   };
   u32 barrier = 1;
-  grid_barrier(p.sync, barrier, give_up);  // the global histograms are clear
+  grid_barrier_wait(p.sync, barrier, give_up);  // the global histograms are clear
   u64 prefix = 0, mask = 0;
   unsigned need = (unsigned)p.k;
   int pass = 0;
@@ -137,23 +191,40 @@ __global__ void __launch_bounds__(kSelectThreads, 2) k_list_select(const __grid_
     const unsigned digit_mask = pass == kSelectPasses - 2 ? 511u : 2047u;
     for (int i = tid; i < kSelectBins; i += kSelectThreads) s_hist[i] = 0;
     __syncthreads();
-    for (i64 r = 0; r < rounds; ++r) {
-      const i64 i = r * stride + (i64)blockIdx.x * kSelectThreads + tid;
-      const u64 c = i < p.N ? p.composite[i] : 0;  // written by this very thread
-      select_count(s_hist, (unsigned)(c >> shift) & digit_mask, i < p.N && (c & mask) == prefix);
-    }
+    for_composites([&](u64 c, bool item) {
+      select_count(s_hist, (unsigned)(c >> shift) & digit_mask, item && (c & mask) == prefix);
+    });
     __syncthreads();
   }
-  for (i64 i = (i64)blockIdx.x * kSelectThreads + tid; i < p.N; i += stride) {
-    const u64 c = p.composite[i];
-    if (c < prefix) continue;
+  for_composites([&](u64 c, bool item) {
+    if (!item || c < prefix) return;
     const unsigned at = atomicAdd(p.found, 1u);
     if (at < (unsigned)p.k) p.winners[at] = c;
     else raise_error(p.counters, GSB_ERR_CAPACITY, at);  // cannot happen: composites are distinct
-  }
-  // everybody arrives, also for the passes that were not needed, and only CTA 0 waits: it has the rest to itself
+  });
+  // everybody arrives, also for the passes that were not needed
   const u32 unused = kSelectBarriers - 1 - barrier;
-  if (blockIdx.x != 0) {
+  if (p.k <= (i64)gridDim.x * kSelectRanked) {
+    grid_arrive(p.sync, unused);
+    grid_barrier(p.sync, kSelectBarriers, give_up);
+    const int k = (int)p.k;
+    for (int i = tid; i < k; i += kSelectThreads) s_win[i] = __ldcg(p.winners + i);
+    __syncthreads();
+    const int warps = (int)gridDim.x * (kSelectThreads / 32);
+    for (int j = (int)blockIdx.x * (kSelectThreads / 32) + warp; j < k; j += warps) {
+      const u64 c = s_win[j];
+      unsigned before = 0;
+      for (int i = lane; i < k; i += 32) before += s_win[i] > c;
+      before = __reduce_add_sync(0xffffffffu, before);
+      if (lane == 0) {
+        const i64 idx = (i64)(0xFFFFFFFFu - (uint32_t)c);
+        p.out_index[before] = idx;
+        p.out_data[before] = __ldg(p.data + idx);
+      }
+    }
+    return;
+  }
+  if (blockIdx.x != 0) {  // only CTA 0 waits: it has the rest to itself
     __syncthreads();
     __threadfence();
     grid_arrive(p.sync, unused + 1);
@@ -449,8 +520,9 @@ extern "C" int gsb_list_sample(gsb_ctx* ctx, void* stream_, const int64_t* data,
     ctx_count_launches(ctx, 3);
     return GSB_OK;
   }
-  static int resident[64];
-  const int ctas = ctx_resident_ctas(ctx, (const void*)k_list_select, kSelectThreads, 0, resident);
+  static int resident[2][64];
+  const int ctas = min(ctx_resident_ctas(ctx, (const void*)k_list_select<false>, kSelectThreads, 0, resident[0]),
+                       ctx_resident_ctas(ctx, (const void*)k_list_select<true>, kSelectThreads, 0, resident[1]));
   if (k <= kSelectMaxK && ctas > 0) {
     const size_t bytes = ((size_t)N * 8 + 255) & ~(size_t)255;
     void* ws;
@@ -474,7 +546,9 @@ extern "C" int gsb_list_sample(gsb_ctx* ctx, void* stream_, const int64_t* data,
     p.sync = ctx_grid_sync(ctx, grid, kSelectBarriers);
     ScopedKernelTimer timer(ctx, KID_LIST_SAMPLE, stream);
     void* args[] = {&p};
-    return launch_cooperative(ctx, stream, (const void*)k_list_select, grid, kSelectThreads, 0, args, p.sync);
+    const bool kept = N <= (i64)grid * kSelectThreads * kSelectKept;
+    return launch_cooperative(ctx, stream, kept ? (const void*)k_list_select<true> : (const void*)k_list_select<false>, grid,
+                              kSelectThreads, 0, args, p.sync);
   }
   // many winners: keys -> radix select of the k-th best -> compact winners -> order them, one launch per pass
   const size_t comp_bytes = ((size_t)N * 8 + 255) & ~(size_t)255;

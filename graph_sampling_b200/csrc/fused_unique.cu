@@ -477,21 +477,16 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
 }
 
 // ---- host side ------------------------------------------------------------------------------------------------------
-// Items per thread: what leaves the busiest SM with the fewest.  With powers of two alone 813 000 items were eight a thread for 199
-// CTAs, two on every third SM and one on the others: 29.1 us, with six a thread 21.4.
+// Items per thread: the fewest whose CTAs are resident together.  A finer list than powers of two leaves fewer SMs with one CTA
+// where others have two: 700 000 items, direct / hash table, five a thread 24.3 / 48.1 us, eight 27.9 / 55.6; 340 000, three
+// 20.6 / 36.0, four 21.7 / 38.7.  Fewer CTAs of more items are never ahead, not even where that evens out the SMs: 200 000 items of 20
+// minibatches, two a thread 25.1, three 27.4.
 constexpr int kFuItems[] = {1, 2, 3, 4, 5, 6, 8, 12, 16};
 
 static int items_per_thread(i64 n, int max_ctas) {
-  int best = 16;
-  i64 least = (i64)1 << 40;
-  for (int r : kFuItems) {
-    const i64 ctas = (n + (i64)kFuThreads * r - 1) / ((i64)kFuThreads * r), load = (ctas + kNumSMs - 1) / kNumSMs * r;
-    if (ctas <= max_ctas && load < least) {
-      best = r;
-      least = load;
-    }
-  }
-  return best;
+  for (int r : kFuItems)
+    if (n <= (i64)max_ctas * kFuThreads * r) return r;
+  return 16;
 }
 
 template <bool BATCHED, bool DIRECT>

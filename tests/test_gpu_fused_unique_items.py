@@ -5,7 +5,7 @@ import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
-WAVE = 148 * 512
+WAVE = 148 * 512   # items of one CTA per SM at one item per thread; two are resident
 
 
 def dev(a):

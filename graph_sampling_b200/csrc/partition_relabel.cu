@@ -792,12 +792,13 @@ __global__ void __launch_bounds__(kBitsThreads) k_rank_emit(BatchLayout L, RankA
 static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Where ranges are ahead of hashed buckets (whole call, 60 M items): of 789 items 1 583 against 1 472 us, of 1 500 1 356 / 1 448, of
-// 5 000 1 164 / 1 331, of 12 700 1 278 / 1 304, of 20 000 1 298 / 1 231 (most of them lie in no register then).  And there have to
-// be several rounds of them: 6 M items in 3 020 ranges took 206 us against 200.
+// 5 000 1 164 / 1 331, of 12 700 1 278 / 1 304, of 20 000 1 298 / 1 231 (most of them lie in no register then).  And they have to
+// fill the SMs: three hops with 816 ranges 596 -> 581 us, 1 700 600 -> 545, 2 500 743 -> 688; with 400 ranges, and ids that crowd in
+// a few of them, a call of 6 M items took 229 us against 187.
 i64 partition_range_parts(i64 num_nodes, i64 items_per_minibatch, i64 G, bool forced) {
   const i64 parts = ((num_nodes + kRangeSlots - 1) >> kRangeShift) + 1;
   if (num_nodes <= 0 || parts > kNarrowWindow) return 0;
-  const bool suits = items_per_minibatch >= 1400 * parts && items_per_minibatch <= 12288 * parts && G * parts >= 4096;
+  const bool suits = items_per_minibatch >= 1400 * parts && items_per_minibatch <= 12288 * parts && G * parts >= 512;
   return forced || suits ? parts : 0;
 }
 

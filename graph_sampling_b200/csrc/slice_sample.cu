@@ -197,6 +197,7 @@ struct SampleParams {
   i64 S;
   i64 k;
   int replace;
+  int bucket_ranges;  // of bucket_count below: buckets are ranges of ids (here it costs no room: eight bytes more 0.3 us a launch)
   u64 seed;
   i64* out_indptr;
   i64* out_indices;
@@ -220,7 +221,6 @@ struct SampleParams {
   // every seed and every sampled id adds one to the count of its bucket.
   uint32_t* bucket_count;
   const i64* bucket_base;  // [G + 1] first bucket of every minibatch
-  int bucket_ranges;       // buckets are ranges of ids
   Mail mail;               // the edge total, for a caller that waits for it
 };
 
@@ -594,10 +594,10 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
   TileState ts;
   int st = ctx_tile_state(ctx, per_thread ? (S + 31) / 32 + 1 : grid, stream, &ts);
   if (st != GSB_OK) return st;
-  SampleParams p{indptr,     indices,     num_cols, seeds, S,        k,        replace,           seed, out_indptr,
+  SampleParams p{indptr,     indices,     num_cols, seeds, S,        k,        replace, 0,        seed, out_indptr,
                  out_indices, out_select, out_coo_col, data, e_ids, out_data, capacity, ctx_counters(ctx), ts,
                  S_dev,      batch_ptr,  batch_ptr ? batch_ids : nullptr,
-                 batch_ptr ? G : 0,      nullptr,    nullptr, 0, mail};
+                 batch_ptr ? G : 0,      nullptr,    nullptr, mail};
   if (count && count->bucket_count) {
     if (!per_thread || !batch_ptr || G < 1) return GSB_ERR_INVALID_ARGUMENT;
     p.bucket_count = count->bucket_count;

@@ -89,221 +89,231 @@ __device__ __forceinline__ unsigned same_digit(u32 d, int bits, bool valid) {
 }
 
 // ---- COO -> CSC / CSR of a short list, without a barrier ----------------------------------------------------------------
-// The keys of up to 26 624 edges are read from L2 by EVERY CTA (213 KB at most; 6 us for the 25 000 edges of a layer-wise
-// minibatch), which needs nothing from the others then: a CTA owns a range of keys, counts the edges with smaller keys (where
-// its output starts) and keeps, in order, those of its range; counts per key, their scan (the offsets) and the stable placing, a
-// warp per part of the range, happen in shared memory.  A CTA with many edges, whose keys may well be the same, sorts them by two
-// digits instead, every warp a part of them.  The cooperative form below, with five grid barriers and 65 536 counters to clear
-// and sum up per CTA and digit, takes 42 us for 25 000 edges over a million keys and 17 us for 700 over a thousand, this 16.4 and
-// 8.9 (calls in a row); 37 when the keys crowd at one end of their range, as those of a power law do whose ids are sorted by
-// degree, and 29 % of the edges are one CTA's.
+// The keys of up to 26 624 edges are read from L2 by EVERY CTA (213 KB at most) and stay in its registers, so it needs nothing from
+// the others.  Each counts the edges of up to 8 192 bins of neighbouring keys, and from the counts' prefix sums all of them derive the
+// same shares: a bin costs E units and an edge as many as there are bins, a share is an equal part of that line, and so holds at
+// most two CTA's worth of edges and of keys however the keys crowd.  A bin may span several shares; its edges are then dealt out
+// by their number within the bin, and a CTA that has not the first of them counts, per key, those that others place before its own.
+// Counts per key of the share's bins, their scan (the offsets), and a rank per edge among the few hundred of the share: all in
+// shared memory.
+// Bound by instruction issue, of which reading and counting all keys is the most.  us a call, calls in a row, the cooperative form
+// below / a fixed range of keys per CTA, which sorts its edges / this: 25 000 edges over 200 000 keys evenly 33.3 / 14.9 / 17.3, by
+// a power law numbered by degree 33.2 / 26.4 / 19.3, all within 1 351 neighbouring keys 32.7 / 92.7 / 23.0, all of one key
+// 45.7 / 72.3 / 23.0; over a million keys evenly 41.4 / 15.7 / 18.8, as the sixth power of an even spread 42.1 / 47.7 / 25.0; 700
+// edges over a thousand keys 17.0 / 8.9 / 8.8; 26 600 over a thousand, the case with the least to win, 24.9 .. 39.1 / 14.8 .. 47.5 /
+// 17.7 .. 25.1.
 constexpr int kShortThreads = 1024;
 constexpr int kShortWarps = kShortThreads / 32;
-constexpr int kKeysAhead = 12;  // keys, and placed edges, of a thread on their way
-constexpr int kShortAhead = 8;
-// At this many edges the two forms are equal where the keys crowd as those of a power law whose ids are sorted by degree; with keys
-// spread evenly this form takes 16.7 us at 32 700 edges, the other 35 to 42.
-constexpr i64 kShortMaxEdges = 26624;
-constexpr u32 kShortHeavy = 1024;  // edges of a CTA from which every warp places a part of them
-constexpr int kShortDigitBits = 7;
-constexpr i64 kShortMaxKeys = 8192;  // of a CTA
-constexpr size_t short_smem(i64 E, i64 keys) { return 4 * (size_t)keys + 4 * (size_t)((E + 1) & ~1ll); }
+constexpr int kShortPer = 26;   // keys of a thread
+constexpr int kKeysAhead = 9;   // of them on their way
+constexpr i64 kShortMaxEdges = (i64)kShortPer * kShortThreads;  // more keys of a thread would not stay in its 64 registers
+constexpr int kShortBins = 8192;
+constexpr int kShortBinsPer = kShortBins / kShortThreads;
+// The keys of a share, 55 296 then, have a word of shared memory each (222 KB) and a number of 16 bits.  Up to there this is far
+// ahead: 26 600 edges over four million keys 67 .. 82 us / 23 .. 31.
+constexpr i64 kShortMaxKeys = 4'000'000;
+
+struct ShortShape {
+  u32 grid;
+  int shift;   // a bin is 2^shift keys
+  u32 bins;
+  u32 keys;    // of the bins of a share, at most
+  u32 edges;   // of a share, at most
+};
+// A share is at most 2 x E x bins / grid + 1 units long: the bins that start in it, two more that begin before and at its end.
+static ShortShape short_shape(i64 E, i64 num_keys) {
+  ShortShape s;
+  s.grid = kNumSMs;
+  s.shift = 0;
+  while (((num_keys - 1) >> s.shift) + 1 > kShortBins) ++s.shift;
+  s.bins = (u32)(((num_keys - 1) >> s.shift) + 1);
+  s.keys = min(s.bins, 2 * s.bins / s.grid + 3) << s.shift;
+  s.edges = 2 * (u32)E / s.grid + 2;
+  return s;
+}
+static size_t short_smem(const ShortShape& s) { return 4 * ((size_t)max((u32)kShortBins, s.keys) + ((size_t)1 << s.shift) + s.edges + 7); }
+
+// Exclusive prefix of `mine` over the CTA's threads.
+__device__ __forceinline__ u32 short_scan(u32 mine, u32* s_warp) {
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  u32 inc = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  __syncthreads();  // s_warp may be in use
+  if (lane == 31) s_warp[warp] = inc;
+  __syncthreads();
+  return __reduce_add_sync(0xffffffffu, lane < warp ? s_warp[lane] : 0u) + inc - mine;
+}
 
 __global__ void __launch_bounds__(kShortThreads, 1) k_coo2csc_short(const i64* __restrict__ key, const i64* __restrict__ other,
-                                                                   u32 E, i64 num_keys, u32 keys_per_cta,
+                                                                   u32 E, i64 num_keys, const __grid_constant__ ShortShape shape,
                                                                    i64* __restrict__ out_indptr, i64* __restrict__ out_other,
-                                                                   i64* __restrict__ out_perm,
-                                                                   uint16_t* __restrict__ scratch, i64* counters) {
-  extern __shared__ __align__(16) u32 s_start[];  // [keys] counts, then where the next edge of the key goes
-  uint16_t* s_rel = reinterpret_cast<uint16_t*>(s_start + keys_per_cta);  // [E] key relative to the range, or kOutside
-  uint16_t* s_list = s_rel + ((E + 1) & ~1u);                             // [E] the edges of the range, in order
-  __shared__ u32 s_warp[2][kShortWarps];
-  constexpr u32 kOutside = 0xFFFFu;
+                                                                   i64* __restrict__ out_perm, i64* counters) {
+  extern __shared__ __align__(16) u32 s_start[];  // [bins] edges per bin; later [keys] edges per key, then where the key's begin
+  u32* s_mine = s_start + max((u32)kShortBins, (shape.keys + 3) & ~3u);  // [edges] key within the share : 16 | edge : 16, in order
+  u32* s_before = s_mine + ((shape.edges + 3) & ~3u);  // [2^shift] per key of the first bin: edges that other CTAs place first
+  __shared__ u32 s_warp[3][kShortWarps];
+  __shared__ u32 s_share[6];
   const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
-  const i64 key_begin = (i64)blockIdx.x * keys_per_cta;
-  const u32 keys = (u32)max((i64)0, min((i64)keys_per_cta, num_keys - key_begin));
+  const int shift = shape.shift;
   const u32 per_warp = (E + kShortThreads - 1) / kShortThreads * 32;
   const u32 begin = min(E, warp * per_warp), end = min(E, begin + per_warp);
-  for (u32 k = tid; k < keys; k += kShortThreads) s_start[k] = 0;
+  const u64 line = 2ull * E * shape.bins;
+  const u32 from = (u32)(line * blockIdx.x / gridDim.x), to = (u32)(line * (blockIdx.x + 1) / gridDim.x);
+  for (u32 k = tid; k < kShortBins / 4; k += kShortThreads) reinterpret_cast<uint4*>(s_start)[k] = make_uint4(0, 0, 0, 0);
+  for (u32 k = tid; k < (1u << shift); k += kShortThreads) s_before[k] = 0;
   __syncthreads();
-  u32 below = 0, inside = 0;  // of the lane's edges
-  for (u32 i0 = begin + lane; i0 < end; i0 += 32 * kKeysAhead) {
+  constexpr u32 kNoKey = 0xFFFFFFFFu;
+  u32 mine[kShortPer];  // the lane's keys, of every 32 edges of the warp one
+#pragma unroll
+  for (int q0 = 0; q0 < kShortPer; q0 += kKeysAhead) {
     i64 k[kKeysAhead];
 #pragma unroll
-    for (int q = 0; q < kKeysAhead; ++q) k[q] = i0 + 32 * q < end ? __ldg(key + i0 + 32 * q) : num_keys;
+    for (int q = 0; q < kKeysAhead; ++q) {
+      const u32 i = begin + 32 * (q0 + q) + lane;
+      k[q] = q0 + q < kShortPer && i < end ? __ldg(key + i) : 0;
+    }
 #pragma unroll
     for (int q = 0; q < kKeysAhead; ++q) {
-      const u32 i = i0 + 32 * q;
-      if (i >= end) break;
+      if (q0 + q >= kShortPer) break;
+      const u32 i = begin + 32 * (q0 + q) + lane;
+      mine[q0 + q] = kNoKey;
+      if (i >= end) continue;
       if ((u64)k[q] >= (u64)num_keys) {
         if (blockIdx.x == 0) raise_error(counters, GSB_ERR_INDEX_RANGE, i);
         k[q] = 0;
       }
-      const i64 rel = k[q] - key_begin;
-      const bool in = (u64)rel < (u64)keys;
-      s_rel[i] = in ? (uint16_t)rel : (uint16_t)kOutside;
-      if (in) atomicAdd(s_start + rel, 1u);
-      inside += in;
-      below += rel < 0;
+      mine[q0 + q] = (u32)k[q];
+      atomicAdd(s_start + (mine[q0 + q] >> shift), 1u);
     }
   }
+  if (blockIdx.x == 0 && tid == 0) out_indptr[num_keys] = (i64)E;
+  if (from == to) return;
+  __syncthreads();
+  // ---- the share: bins first .. last, of the first the edges from `skip` on, of the last those up to `stop`
+  {
+    u32 count[kShortBinsPer], sum = 0;
+    const u32 bin0 = tid * kShortBinsPer;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    inside += __shfl_xor_sync(0xffffffffu, inside, o);
-    below += __shfl_xor_sync(0xffffffffu, below, o);
-  }
-  if (lane == 0) {
-    s_warp[0][warp] = inside;
-    s_warp[1][warp] = below;
+    for (int j = 0; j < kShortBinsPer; j += 4) {
+      const uint4 four = reinterpret_cast<const uint4*>(s_start + bin0)[j / 4];
+      count[j] = four.x, count[j + 1] = four.y, count[j + 2] = four.z, count[j + 3] = four.w;
+      sum += four.x + four.y + four.z + four.w;
+    }
+    u32 edges = short_scan(sum, s_warp[0]);
+#pragma unroll
+    for (int j = 0; j < kShortBinsPer; ++j) {
+      const u32 bin = bin0 + j;
+      if (bin >= shape.bins) break;
+      const u32 at = bin * E + edges * shape.bins, its = at + E, next = its + count[j] * shape.bins;
+      if (at <= from && from < next) {
+        s_share[0] = bin;
+        s_share[1] = edges;  // with smaller keys
+        s_share[2] = from <= its ? 0 : (from - its + shape.bins - 1) / shape.bins;
+        s_share[3] = at == from;  // the offsets of its keys are the CTA's to write
+      }
+      if (at < to && to <= next) {
+        s_share[4] = bin;
+        s_share[5] = to <= its ? 0 : (to - its + shape.bins - 1) / shape.bins;
+      }
+      edges += count[j];
+    }
   }
   __syncthreads();
-  u32 at = 0, total = 0;
-  below = 0;
+  const u32 first = s_share[0], below = s_share[1], skip = s_share[2], last = s_share[4], stop = s_share[5];
+  const u32 key_begin = first << shift, keys = min((u32)num_keys, (last + 1) << shift) - key_begin;
+  for (u32 k = tid; k < keys; k += kShortThreads) s_start[k] = 0;
+  __syncthreads();
+  // ---- count the keys of the share's bins; edges of the warp in the first and in the last bin, and between them
+  u32 in_first = 0, in_last = 0, between = 0;
 #pragma unroll
-  for (u32 w = 0; w < kShortWarps; ++w) {
-    if (w < warp) at += s_warp[0][w];
-    total += s_warp[0][w];
-    below += s_warp[1][w];
+  for (int q = 0; q < kShortPer; ++q) {
+    if (begin + 32 * q >= end) break;  // uniform
+    const u32 rel = mine[q] - key_begin;  // (no key: beyond all)
+    const bool in = rel < keys;
+    if (!__any_sync(0xffffffffu, in)) continue;
+    if (in) atomicAdd(s_start + rel, 1u);
+    const u32 bin = mine[q] >> shift;
+    in_first += in && bin == first;
+    in_last += in && bin == last && last != first;
+    between += in && bin != last && bin != first;
   }
-  if (inside > 0)  // (the whole warp's)
-    for (u32 i0 = begin; i0 < end; i0 += 32) {
-      const bool in = i0 + lane < end && s_rel[i0 + lane] != kOutside;
-      const unsigned bits = __ballot_sync(0xffffffffu, in);
-      if (in) s_list[at + __popc(bits & lt)] = (uint16_t)(i0 + lane);
-      at += __popc(bits);
-    }
-  // offsets: a stretch of keys per thread, eight at most
-  {
-    constexpr u32 kPer = kShortMaxKeys / kShortThreads;
-    const u32 per = (keys + kShortThreads - 1) / kShortThreads, first = tid * per;
-    u32 v[kPer], sum = 0;
-#pragma unroll
-    for (u32 j = 0; j < kPer; ++j) {
-      v[j] = j < per && first + j < keys ? s_start[first + j] : 0;
-      sum += v[j];
-    }
-    u32 inc = sum;
+  in_first = __reduce_add_sync(0xffffffffu, in_first);
+  in_last = __reduce_add_sync(0xffffffffu, in_last);
+  between = __reduce_add_sync(0xffffffffu, between);
+  if (lane == 0) {
+    s_warp[0][warp] = in_first;
+    s_warp[1][warp] = in_last;
+    s_warp[2][warp] = between;
+  }
+  __syncthreads();
+  // which of the first (last) bin's edges the CTA places: number skip and up, below `stop` (of the last)
+  const u32 first_stop = first == last ? stop : 0xFFFFFFFFu;
+  auto overlap = [](u32 a0, u32 a1, u32 b0, u32 b1) { return min(a1, b1) > max(a0, b0) ? min(a1, b1) - max(a0, b0) : 0u; };
+  u32 at, total, number_first, number_last;
+  {  // a warp per lane
+    u32 f = s_warp[0][lane], l = s_warp[1][lane];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += t;
+      const u32 tf = __shfl_up_sync(0xffffffffu, f, o), tl = __shfl_up_sync(0xffffffffu, l, o);
+      if (lane >= o) f += tf, l += tl;
     }
-    __syncthreads();  // s_warp has been read
-    if (lane == 31) s_warp[0][warp] = inc;
-    __syncthreads();
-    u32 run = inc - sum;
-#pragma unroll
-    for (u32 w = 0; w < kShortWarps; ++w)
-      if (w < warp) run += s_warp[0][w];
-#pragma unroll
-    for (u32 j = 0; j < kPer; ++j) {
-      if (j < per && first + j < keys) s_start[first + j] = run;
-      run += v[j];
-    }
-    __syncthreads();
-    for (u32 k = tid; k < keys; k += kShortThreads) out_indptr[key_begin + k] = (i64)(below + s_start[k]);
-    if (blockIdx.x == 0 && tid == 0) out_indptr[num_keys] = (i64)E;
-    __syncthreads();
+    const u32 places = s_warp[2][lane] + overlap(f - s_warp[0][lane], f, skip, first_stop) + overlap(l - s_warp[1][lane], l, 0, stop);
+    total = __reduce_add_sync(0xffffffffu, places);
+    at = __reduce_add_sync(0xffffffffu, lane < warp ? places : 0u);
+    number_first = __shfl_sync(0xffffffffu, f, warp) - in_first;
+    number_last = __shfl_sync(0xffffffffu, l, warp) - in_last;
   }
-  // the edges in their new order, placed by the two ways below; the outputs follow from it in one go (a warp that wrote them while
-  // placing waited for a random read every 32 edges)
-  constexpr u32 kDigits = 1u << kShortDigitBits;
-  __shared__ uint16_t s_digit[kShortWarps][kDigits];  // of a warp's part, then where its next edge of the digit goes
-  __shared__ u32 s_digit_start[kDigits];
-  static_assert(kShortWarps * kDigits >= kShortHeavy, "the order of a light CTA takes the place of the digits");
-  uint16_t* order = &s_digit[0][0];
-  if (total >= kShortHeavy) {  // a stable counting sort by one or two digits of the key
-    const u32 share = (total + kShortThreads - 1) / kShortThreads * 32;
-    const u32 lo = min(total, warp * share), hi = min(total, lo + share);
-    const int key_bits = keys > 1 ? 32 - __clz(keys - 1) : 0, passes = key_bits > kShortDigitBits ? 2 : 1;
-    uint16_t* second = 2 * total <= E ? s_list + total : scratch + below;
-    for (int pass = 0; pass < passes; ++pass) {
-      const uint16_t* list = pass == 0 ? s_list : second;
-      order = pass == 0 ? second : s_list;
-      const int bits = pass == 0 ? min(key_bits, kShortDigitBits) : key_bits - kShortDigitBits;
-      auto digit_of = [&](u32 e) { return ((u32)s_rel[e] >> (pass * kShortDigitBits)) & (kDigits - 1); };
-      for (u32 d = lane; d < kDigits; d += 32) s_digit[warp][d] = 0;
-      __syncwarp();
-#pragma unroll 4
-      for (u32 j0 = lo; j0 < hi; j0 += 32) {
-        const bool valid = j0 + lane < hi;
-        const u32 d = valid ? digit_of(list[j0 + lane]) : 0;
-        const unsigned peers = same_digit(d, bits, valid);
-        if (valid && (peers & lt) == 0) s_digit[warp][d] += (uint16_t)__popc(peers);
-        __syncwarp();
-      }
-      __syncthreads();
-      if (tid < kDigits) {
-        u32 run = 0;
-        for (u32 w = 0; w < kShortWarps; ++w) {
-          const u32 c = s_digit[w][tid];
-          s_digit[w][tid] = (uint16_t)run;
-          run += c;
-        }
-        s_digit_start[tid] = run;
-      }
-      __syncthreads();
-      if (warp == 0) {
-        u32 carry = 0;
-        for (u32 d0 = 0; d0 < kDigits; d0 += 32) {
-          const u32 c = s_digit_start[d0 + lane];
-          u32 inc = c;
+  // ---- the share's edges, in order
+  if (in_first + in_last + between > 0) {
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-          }
-          s_digit_start[d0 + lane] = carry + inc - c;
-          carry += __shfl_sync(0xffffffffu, inc, 31);
-        }
-      }
-      __syncthreads();
-      for (u32 j0 = lo; j0 < hi; j0 += 32) {
-        const bool valid = j0 + lane < hi;
-        const u32 e = valid ? list[j0 + lane] : 0, d = valid ? digit_of(e) : 0;
-        const unsigned peers = same_digit(d, bits, valid);
-        u32 pos = 0;
-        if (valid) pos = s_digit[warp][d];
-        __syncwarp();
-        if (valid && (peers & lt) == 0) s_digit[warp][d] = (uint16_t)(pos + __popc(peers));
-        __syncwarp();
-        if (valid) order[pos + s_digit_start[d] + __popc(peers & lt)] = (uint16_t)e;
-      }
-      __syncthreads();  // the other list is complete
+    for (int q = 0; q < kShortPer; ++q) {
+      if (begin + 32 * q >= end) break;
+      const u32 rel = mine[q] - key_begin, bin = mine[q] >> shift;
+      const bool in = rel < keys, of_first = in && bin == first, of_last = in && bin == last && last != first;
+      if (!__any_sync(0xffffffffu, in)) continue;
+      const unsigned firsts = __ballot_sync(0xffffffffu, of_first), lasts = __ballot_sync(0xffffffffu, of_last);
+      const u32 number = of_first ? number_first + __popc(firsts & lt) : number_last + __popc(lasts & lt);
+      const bool take = in && (of_first ? number >= skip && number < first_stop : of_last ? number < stop : true);
+      if (of_first && number < skip) atomicAdd(s_before + rel, 1u);
+      const unsigned taken = __ballot_sync(0xffffffffu, take);
+      if (take) s_mine[at + __popc(taken & lt)] = (rel << 16) | (begin + 32 * q + lane);
+      at += __popc(taken);
+      number_first += __popc(firsts);
+      number_last += __popc(lasts);
     }
-  } else {  // a warp takes the edges of its part of the range, in order
-    const u32 part = (keys + kShortWarps - 1) / kShortWarps, part_begin = warp * part;
-    const u32 part_keys = min(part, keys - min(keys, part_begin));
-    for (u32 j0 = 0; j0 < total && part_keys > 0; j0 += 32) {
-      const u32 e = j0 + lane < total ? s_list[j0 + lane] : 0;
-      const u32 rel = s_rel[e];
-      const bool mine = j0 + lane < total && rel - part_begin < part_keys;
-      if (!__any_sync(0xffffffffu, mine)) continue;
-      const unsigned peers = __match_any_sync(0xffffffffu, mine ? rel : kOutside);
-      u32 pos = 0;
-      if (mine) pos = s_start[rel];
-      __syncwarp();
-      if (mine && (peers & lt) == 0) s_start[rel] = pos + __popc(peers);
-      __syncwarp();
-      if (mine) order[pos + __popc(peers & lt)] = (uint16_t)e;
+  }
+  if (tid < (-total & 3u)) s_mine[total + tid] = 0xFFFFFFFFu;
+  // ---- offsets: a stretch of keys per thread, an odd number of them (each lane another bank)
+  {
+    const u32 per = ((keys + kShortThreads - 1) / kShortThreads) | 1u, k0 = min(keys, tid * per), k1 = min(keys, k0 + per);
+    u32 sum = 0;
+    for (u32 k = k0; k < k1; ++k) sum += s_start[k];
+    u32 run = short_scan(sum, s_warp[0]);
+    for (u32 k = k0; k < k1; ++k) {
+      const u32 c = s_start[k];
+      s_start[k] = run;
+      run += c;
     }
     __syncthreads();
+    const u32 own = s_share[3] ? 0 : 1u << shift;  // the first bin's keys may be another CTA's to write
+    for (u32 k = own + tid; k < keys; k += kShortThreads) out_indptr[key_begin + k] = (i64)(below + s_start[k]);
   }
-  for (u32 j0 = tid; j0 < total; j0 += kShortThreads * kShortAhead) {
-    u32 e[kShortAhead];
-    i64 o[kShortAhead];
-#pragma unroll
-    for (int q = 0; q < kShortAhead; ++q) e[q] = j0 + q * kShortThreads < total ? order[j0 + q * kShortThreads] : 0;
-#pragma unroll
-    for (int q = 0; q < kShortAhead; ++q)
-      if (j0 + q * kShortThreads < total) o[q] = __ldg(other + e[q]);
-#pragma unroll
-    for (int q = 0; q < kShortAhead; ++q) {
-      const u32 j = j0 + q * kShortThreads;
-      if (j >= total) break;
-      out_perm[below + j] = (i64)e[q];
-      out_other[below + j] = o[q];
+  // ---- every edge behind those of its key that come before it
+  for (u32 j = tid; j < total; j += kShortThreads) {
+    const u32 me = s_mine[j], rel = me >> 16, e = me & 0xFFFFu;
+    const i64 value = __ldg(other + e);
+    u32 pos = below + s_start[rel] + (rel < (1u << shift) ? s_before[rel] : 0u);
+    // the key's earlier edges lie between (key, 0) and this one (and so none of them is one of what lies behind the list)
+    for (u32 i = 0; i < j; i += 4) {
+      const uint4 four = *reinterpret_cast<const uint4*>(s_mine + i);
+      pos += (four.x - (rel << 16) < e) + (four.y - (rel << 16) < e) + (four.z - (rel << 16) < e) + (four.w - (rel << 16) < e);
     }
+    out_perm[pos] = (i64)e;
+    out_other[pos] = value;
   }
 }
 
@@ -571,21 +581,18 @@ int gsb_coo2csc(gsb_ctx* ctx, void* stream_, const int64_t* key, const int64_t* 
   const int grid = min(grid_for(E, kFmtThreads), kNumSMs * 8);
   int bits = 1;
   while (bits < 63 && (1ll << bits) < num_keys) ++bits;
-  if (!key_sorted && E > 0 && E <= kShortMaxEdges && num_keys > 0 && num_keys <= kShortMaxKeys * kNumSMs) {
+  if (!key_sorted && E > 0 && E <= kShortMaxEdges && num_keys > 0 && num_keys <= kShortMaxKeys) {
     static bool attr_set[64];
     const int dev = ctx_device(ctx);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
       GSB_CUDA_OK(cudaFuncSetAttribute(k_coo2csc_short, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)short_smem(kShortMaxEdges, kShortMaxKeys)));
+                                       (int)short_smem(short_shape(kShortMaxEdges, kShortMaxKeys))));
       attr_set[dev] = true;
     }
-    const u32 keys_per_cta = (u32)((num_keys + kNumSMs - 1) / kNumSMs);
-    void* scratch;
-    const int st = ctx_reserve_workspace(ctx, stream, sizeof(uint16_t) * (size_t)E, &scratch);
-    if (st != GSB_OK) return st;
+    const ShortShape shape = short_shape(E, num_keys);
     ScopedKernelTimer timer(ctx, KID_FORMAT, stream);
-    k_coo2csc_short<<<grid_for(num_keys, (int)keys_per_cta), kShortThreads, short_smem(E, keys_per_cta), stream>>>(
-        key, other, (u32)E, num_keys, keys_per_cta, out_indptr, out_other, out_perm, (uint16_t*)scratch, ctx_counters(ctx));
+    k_coo2csc_short<<<(int)shape.grid, kShortThreads, short_smem(shape), stream>>>(key, other, (u32)E, num_keys, shape, out_indptr,
+                                                                                  out_other, out_perm, ctx_counters(ctx));
     GSB_LAUNCH_OK();
     return GSB_OK;
   }

@@ -620,7 +620,7 @@ constexpr i64 kPartitionAutoItems = 1ll << 19;
 // a window of 256 buckets, a call of 500 minibatches of 740 000 items ran on the hash regions: 28.6 ms of the hop.)
 constexpr i64 kPartitionAutoMaxMinibatch = 1024ll * kBucketTarget;
 // The counting sampler flushes its per-bucket counts once per 128 columns: with more than 256 buckets a minibatch that is
-// an atomic for every other item, and the separate counting pass is cheaper (and with 151 ranges, too: sampling 8.2 -> 9.3 ms
+// an atomic for every other item, and the separate counting pass is cheaper (and with 151 buckets, too: sampling 8.2 -> 9.3 ms
 // against 0.67 for the pass, last hop of 500 minibatches of 813 000 items).
 constexpr i64 kSamplerCountsMaxMinibatch = 256ll * kBucketTarget;
 static inline bool partition_suits(i64 n_cap, i64 G) {
@@ -703,7 +703,7 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   }
   if (path >= 3 || (path == 0 && partition_suits(n_cap, G))) {
     // partitioned form (the default for large calls when the direct-address tables above were not chosen): shared-memory tables per bucket of items, then ranking by bit vectors
-    const i64 parts = path == 3 ? 0 : partition_range_parts(num_nodes, n_cap / G, G, path == 4);
+    const i64 parts = path == 3 ? 0 : partition_class_parts(num_nodes, n_cap / G, path == 4);
     const i64 bucket_cap = partition_bucket_capacity(n_cap, G, parts);
     int st = ctx_reserve_workspace(ctx, stream, 3 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
     if (st != GSB_OK) return st;
@@ -794,7 +794,7 @@ static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64*
     k_batch_layout<<<1, kBThreads, 0, stream>>>(L, counters, k, 1 | 8 | 32, S, cap, partition_bucket_counts(part_ws), parts);
   }
   GSB_LAUNCH_OK();
-  const SamplerCount count{partition_bucket_counts(part_ws), L.region_off, parts > 0};
+  const SamplerCount count{partition_bucket_counts(part_ws), L.region_off, class_magic(parts)};
   st = sample_uniform_launch(ctx, stream, indptr, indices, num_nodes, seeds, S, k, replace, seed, out_indptr,
                              out_indices, out_select, nullptr, nullptr, nullptr, nullptr, cap, seeds_ptr + G,
                              seeds_ptr, batch_ids, G, &count);
@@ -886,7 +886,7 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
   const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
   const bool fused = path == 0 && fused_unique_suits(ctx, n_cap, G);
   const bool direct_small = (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes && num_nodes > 0;
-  const i64 parts = path == 3 || n_cap == 0 ? 0 : partition_range_parts(num_nodes, n_cap / G, G, path == 4);
+  const i64 parts = path == 3 || n_cap == 0 ? 0 : partition_class_parts(num_nodes, n_cap / G, path == 4);
   if (!fused && k >= 1 && k <= 16 && n_cap > 0 && n_cap / G <= kSamplerCountsMaxMinibatch &&
       (path >= 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
     st = sage_hop_sampler_counts(ctx, stream, indptr, indices, num_nodes, seeds, seeds_ptr, batch_ids, G, S, k, cap,

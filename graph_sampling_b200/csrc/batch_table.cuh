@@ -169,10 +169,14 @@ int direct_unique_relabel_launch(gsb_ctx* ctx, cudaStream_t stream, const BatchL
 // partition_workspace_bytes(n_cap, bucket_cap) bytes and begins with the per-bucket item counts.  counted = true: the
 // counts and bucket starts are already there (the sampler of the same hop counted, partition_after_sampler did the
 // rest) and the counting and scan passes are skipped.
-// parts > 0: buckets are ranges of 2^kRangeShift ids, parts of them per minibatch (partition_range_parts), the last of which takes
-// the ids from the bound on; parts = 0: buckets by a hash of the id.
-constexpr int kRangeShift = 14;
-i64 partition_range_parts(i64 num_nodes, i64 items_per_minibatch, i64 G, bool forced);
+// parts > 0: buckets are the parts - 1 classes of ids with the same remainder by that number (partition_class_parts), and one more
+// that takes the ids from the bound on; parts = 0: buckets by a hash of the id.
+constexpr uint32_t kClassSlots = 1u << 14;  // ids of a class at most, a word of shared memory each
+i64 partition_class_parts(i64 num_nodes, i64 items_per_minibatch, bool forced);
+// m = ceil(2^32 / classes): __umulhi(id, m) is the quotient for every id below kClassSlots x classes, because there
+// id x (m x classes - 2^32) < id x classes < 2^32, which is what may be added to the remainder without reaching the next quotient; the
+// error is upwards, so an id from there on gives kClassSlots at least.
+inline uint32_t class_magic(i64 parts) { return parts > 0 ? (uint32_t)((((u64)1 << 32) + (u64)parts - 2) / (u64)(parts - 1)) : 0u; }
 i64 partition_bucket_capacity(i64 items_bound, i64 G, i64 parts);
 size_t partition_workspace_bytes(i64 n_cap, i64 bucket_cap);
 uint32_t* partition_bucket_counts(void* ws);
@@ -182,17 +186,23 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
 // item offsets, bound check, bucket starts — everything partition_unique_relabel(counted = true) expects, one launch.
 int partition_after_sampler(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64 n_cap, i64 bucket_cap, void* ws,
                             const i64* sub_indptr, i64 S, i64 edges_bound, i64* out_indices_ptr);
-// Bucket of an id among the `parts` buckets of its minibatch: its range (the last bucket takes all ids beyond), or Fibonacci
-// hashing (the high bits of id x odd constant), scaled to the bucket count by a multiply-high.  Ids are below 2^32 - 1
+// Bucket of an id among the `parts` buckets of its minibatch: its class (magic != 0; the last bucket takes all ids beyond), or
+// Fibonacci hashing (the high bits of id x odd constant), scaled to the bucket count by a multiply-high.  Ids are below 2^32 - 1
 // wherever this is used.
-__device__ __forceinline__ uint32_t bucket_of_id(uint32_t id, uint32_t parts, int ranges) {
-  return ranges ? min(id >> kRangeShift, parts - 1) : __umulhi(id * 0x9E3779B1u, parts);
+template <bool CLASSES>
+__device__ __forceinline__ uint32_t bucket_of_id(uint32_t id, uint32_t parts, uint32_t magic) {
+  if (!CLASSES) return __umulhi(id * 0x9E3779B1u, parts);
+  const uint32_t q = __umulhi(id, magic);
+  return q < kClassSlots ? id - q * (parts - 1) : parts - 1;
+}
+__device__ __forceinline__ uint32_t bucket_of_id(uint32_t id, uint32_t parts, uint32_t magic) {
+  return magic != 0 ? bucket_of_id<true>(id, parts, magic) : bucket_of_id<false>(id, parts, 0);
 }
 // What the uniform sampler needs to count, per bucket, the seeds and the ids it samples (fan-outs up to 16).
 struct SamplerCount {
   uint32_t* bucket_count;  // [buckets]
   const i64* bucket_base;  // [G + 1] first bucket of every minibatch
-  int ranges;              // buckets are ranges of ids
+  uint32_t magic;          // of the classes of ids that are the buckets, 0: hashed
 };
 constexpr int kBucketTarget = 2048;  // mean items per bucket
 

@@ -23,7 +23,7 @@
 //             written in the bucket's order; a bucket with more items than the shared-memory table is sized
 //             for (many repeats of a few hub ids, or an unlucky hash) uses a table in global memory of its own
 //             instead, so nothing depends on luck;
-//             With a bound on the ids, buckets can be ranges of them instead: see k_part_resolve_ranges;
+//             With a bound on the ids, buckets can be classes of them instead: see k_part_resolve_classes;
 //   rank      the first positions brought back into the order of the items, which the scatter pass told where they went (a
 //             tile's share of a bucket is a run, so a CTA that takes the same tile reads whole sectors); bit vector of
 //             the first occurrences (ref[item] == own position), prefix counts per 32 items, then one
@@ -67,7 +67,8 @@ struct PartLayout {
   u32* found;          // [items]   in the same order: position inside the minibatch of the first occurrence of the id
   u32* ref;            // [items]   by item: where it lies in `bucketed`; from k_first_bits on what `found` says there
   u64* spill;          // tables of the buckets that do not fit shared memory: 2 x start + 32 x bucket
-  u32 range_parts;     // buckets per minibatch when they are ranges of ids, 0: buckets by hash
+  u32 class_parts;     // buckets per minibatch when they are classes of ids (and one for those beyond), 0: buckets by hash
+  u32 class_magic;     // see bucket_of_id
 };
 
 // Slot inside a bucket's table: a constant other than bucket_of_id's and one xor-shift round, so the ids of one
@@ -130,19 +131,19 @@ struct Located {
   u32 lc;      // position inside its minibatch (seeds first)
   u32 bucket;  // global bucket number
 };
-__device__ __forceinline__ Located locate(const BatchLayout& L, i64 g, int ranges) {
+__device__ __forceinline__ Located locate(const BatchLayout& L, i64 g, u32 magic) {
   const BatchUniform v = load_batch<false>(L, L.item_off, batch_of(L.item_off, L.G, g));
   const TileBatch t = tile_batch(L, v);
   Located r;
   r.lc = (u32)(g - v.begin);
   r.node = tile_item(t, r.lc);
-  r.bucket = t.bucket0 + bucket_of_id((u32)r.node, t.parts, ranges);
+  r.bucket = t.bucket0 + bucket_of_id((u32)r.node, t.parts, magic);
   return r;
 }
 
 constexpr int kMaxSegments = 8;  // minibatches a tile may touch and still be handled segment by segment
 
-template <int kWindow>
+template <int kWindow, bool CLASSES>
 __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n_bound, i64* counters) {
   __shared__ u32 s_cnt[kWindow];
   if (counters[CNT_ABORT] != 0) return;
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
   const i64 b_last = batch_of_warp(L.item_off, L.G, tile_end - 1);
   if (b_last - b_first >= kMaxSegments) {  // a tile over many small minibatches: every item on its own
     for (i64 g = tile_base + threadIdx.x; g < tile_end; g += kPartThreads) {
-      const Located it = locate(L, g, P.range_parts);
+      const Located it = locate(L, g, P.class_magic);
       if (!valid_id(it.node)) continue;  // never bucketed; reported by the scatter pass
       atomicAdd(P.bucket_count + it.bucket, 1u);
     }
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
       for (u32 i = threadIdx.x; i < here; i += kPartThreads) {
         const i64 node = tile_item(t, lc0 + i);
         if (!valid_id(node)) continue;
-        const u32 k = t.bucket0 + bucket_of_id((u32)node, t.parts, P.range_parts);
+        const u32 k = t.bucket0 + bucket_of_id<CLASSES>((u32)node, t.parts, P.class_magic);
         atomicAdd(P.bucket_count + k, 1u);
       }
       continue;
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(PartLayout P, i64 n
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kPartPerThread; ++q)
-      if (valid_id(node[q])) atomicAdd(&s_cnt[bucket_of_id((u32)node[q], t.parts, P.range_parts)], 1u);  // the others: scatter pass
+      if (valid_id(node[q])) atomicAdd(&s_cnt[bucket_of_id<CLASSES>((u32)node[q], t.parts, P.class_magic)], 1u);  // the others: scatter pass
     __syncthreads();
     for (u32 i = threadIdx.x; i < t.parts; i += kPartThreads) {
       if (s_cnt[i] != 0) atomicAdd(P.bucket_count + t.bucket0 + i, s_cnt[i]);
@@ -302,10 +303,10 @@ __global__ void __launch_bounds__(1024) k_part_after_sampler(PartLayout P, const
 // THREADS x PER items per tile.  Tiles of 2 048 suit minibatches of some ten thousand items (a tile that straddles
 // minibatches takes the per-item path); with hundreds of buckets per minibatch such a tile reserves a range — a global
 // atomic, on a cursor that every other tile of the minibatch wants too — for every five items, so large minibatches take
-// tiles of 8 192, two of whose CTAs are resident per SM.  That costs 300 bytes of spilled registers a thread (with the 83
+// tiles of 8 192, two of whose CTAs are resident per SM.  That costs 68 bytes of spilled registers a thread (with the 83
 // registers the compiler takes of its own accord one CTA is resident, and its barriers leave the SM idle: 3.1 against 2.1 ms for
 // 270 M items; 1 024 threads with half the items each 2.8, tiles of 4 096 2.7).
-template <int WINDOW, int THREADS, int PER>
+template <int WINDOW, int THREADS, int PER, bool CLASSES>
 __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatter(PartLayout P, i64 n_bound, i64* counters) {
   constexpr int kTile = THREADS * PER;
   constexpr int kPer = WINDOW / THREADS > 0 ? WINDOW / THREADS : 1;  // consecutive window entries per thread in the scan
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatte
   const bool uniform = (u64)lc0 + here <= (u64)t.items && t.parts <= (u32)WINDOW;
   if (!uniform) {  // a tile over several minibatches: every item straight to its place
     for (u32 i = threadIdx.x; i < here; i += THREADS) {
-      const Located it = locate(L, tile_base + i, P.range_parts);
+      const Located it = locate(L, tile_base + i, P.class_magic);
       if (!valid_id(it.node)) {  // never bucketed: marked for the ranking passes
         raise_error(counters, GSB_ERR_INDEX_RANGE, tile_base + i);
         P.ref[tile_base + i] = 0xFFFFFFFFu;
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatte
       }
       continue;
     }
-    const u32 w = bucket_of_id(id[q], t.parts, P.range_parts);
+    const u32 w = bucket_of_id<CLASSES>(id[q], t.parts, P.class_magic);
     where[q] = (w << 16) | atomicAdd(&s_cnt[w], 1u);  // at most 8 192 items per tile: the rank fits 16 bits
   }
   __syncthreads();
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) k_part_scatte
   __syncthreads();
   for (u32 i = threadIdx.x; i < staged; i += THREADS) {
     const u64 w = s_stage[i];
-    P.bucketed[s_delta[bucket_of_id((u32)(w >> 32), t.parts, P.range_parts)] + i] = w;
+    P.bucketed[s_delta[bucket_of_id<CLASSES>((u32)(w >> 32), t.parts, P.class_magic)] + i] = w;
   }
 }
 
@@ -533,22 +534,25 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
   }
 }
 
-// Buckets that are ranges of 2^kRangeShift ids: the table is addressed by the low bits of the id, so an item is one reduction and
-// one read in shared memory, without ids to compare and without probes.  Between HBM (12 bytes an item; half of the copy
-// bandwidth) and the latency of a bucket's load, clear, reduce and read, of which an SM has three in flight: 500 M items of 500
-// minibatches in three hops 2.82 -> 1.57 ms, the scatter pass, whose runs are longer, 2.64 -> 2.47.
-constexpr int kRangeThreads = 512;
-constexpr int kRangePer = 12;  // items of a thread that stay in registers
-constexpr int kRangeSlots = 1 << kRangeShift;
+// Buckets that are classes of ids, those with the same remainder by a prime: the table is addressed by the quotient, so an item is
+// one reduction and one read in shared memory, without ids to compare and without probes.  Classes and not ranges of neighbouring
+// ids, because a graph numbered by degree, or as a crawler met it, has most neighbours in a few ranges, and the CTA with such a range
+// kept the others waiting: 6 M items of 7 minibatches over 2.45 M nodes by a power law, whole call, hashed buckets 196 us, ranges 343
+// numbered by degree and 164 scattered, classes 166 either way.
+// Between HBM (12 bytes an item; half of the copy bandwidth) and the latency of a bucket's load, clear, reduce and read, of which an
+// SM has three in flight: 500 M items of 500 minibatches in three hops, hashed / classes: this pass 2.82 / 1.51 ms, the scatter
+// pass, whose runs are longer, 2.64 / 2.46, counting 0.67 / 0.73.
+constexpr int kClassThreads = 512;
+constexpr int kClassPer = 12;  // items of a thread that stay in registers
 
-__global__ void __launch_bounds__(kRangeThreads, 3) k_part_resolve_ranges(PartLayout P, i64* counters) {
-  extern __shared__ __align__(16) u32 s_first[];  // [kRangeSlots] smallest position of every id
+__global__ void __launch_bounds__(kClassThreads, 3) k_part_resolve_classes(PartLayout P, i64* counters) {
+  extern __shared__ __align__(16) u32 s_first[];  // [kClassSlots] smallest position of every id
   if (counters[CNT_ABORT] != 0) return;
   const u32 buckets = (u32)P.L.region_off[P.L.G];
   for (u32 k = blockIdx.x; k < buckets; k += gridDim.x) {
     const u32 start = P.bucket_start[k], n = P.bucket_start[k + 1] - start;
     if (n == 0) continue;
-    if (k % P.range_parts == P.range_parts - 1) {  // ids beyond the bound
+    if (k % P.class_parts == P.class_parts - 1) {  // ids beyond the bound
       resolve_in_memory(P.bucketed + start, n, P.spill + 2 * (u64)start + 32 * (u64)k, P.found + start);
       continue;
     }
@@ -556,32 +560,32 @@ __global__ void __launch_bounds__(kRangeThreads, 3) k_part_resolve_ranges(PartLa
     u32* found = P.found + start;
     if (k + gridDim.x < buckets) {  // the next bucket's items on their way to L2
       const u32 at = P.bucket_start[k + gridDim.x], end = P.bucket_start[k + gridDim.x + 1];
-      for (u32 i = at + threadIdx.x * 16; i < end; i += kRangeThreads * 16)
+      for (u32 i = at + threadIdx.x * 16; i < end; i += kClassThreads * 16)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(P.bucketed + i));
     }
-    u64 w[kRangePer];  // their loads are in flight while the table is cleared
+    u64 w[kClassPer];  // their loads are in flight while the table is cleared
 #pragma unroll
-    for (int q = 0; q < kRangePer; ++q) {
-      const u32 j = q * kRangeThreads + threadIdx.x;
+    for (int q = 0; q < kClassPer; ++q) {
+      const u32 j = q * kClassThreads + threadIdx.x;
       w[q] = j < n ? __ldg(items + j) : kEmptyWord;
     }
     __syncthreads();  // the previous bucket's look-ups are done
     const uint4 e = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-    for (u32 i = threadIdx.x; i < kRangeSlots / 4; i += kRangeThreads) reinterpret_cast<uint4*>(s_first)[i] = e;
+    for (u32 i = threadIdx.x; i < kClassSlots / 4; i += kClassThreads) reinterpret_cast<uint4*>(s_first)[i] = e;
     __syncthreads();
-    auto slot = [&](u64 item) { return s_first + ((u32)(item >> 32) & (kRangeSlots - 1)); };
+    auto slot = [&](u64 item) { return s_first + __umulhi((u32)(item >> 32), P.class_magic); };
 #pragma unroll
-    for (int q = 0; q < kRangePer; ++q)
+    for (int q = 0; q < kClassPer; ++q)
       if (w[q] != kEmptyWord) atomicMin(slot(w[q]), (u32)w[q]);
-    for (u32 j = kRangePer * kRangeThreads + threadIdx.x; j < n; j += kRangeThreads) {
+    for (u32 j = kClassPer * kClassThreads + threadIdx.x; j < n; j += kClassThreads) {
       const u64 item = __ldg(items + j);
       atomicMin(slot(item), (u32)item);
     }
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < kRangePer; ++q)
-      if (w[q] != kEmptyWord) found[q * kRangeThreads + threadIdx.x] = *slot(w[q]);
-    for (u32 j = kRangePer * kRangeThreads + threadIdx.x; j < n; j += kRangeThreads) found[j] = *slot(__ldg(items + j));
+    for (int q = 0; q < kClassPer; ++q)
+      if (w[q] != kEmptyWord) found[q * kClassThreads + threadIdx.x] = *slot(w[q]);
+    for (u32 j = kClassPer * kClassThreads + threadIdx.x; j < n; j += kClassThreads) found[j] = *slot(__ldg(items + j));
   }
 }
 
@@ -791,15 +795,21 @@ __global__ void __launch_bounds__(kBitsThreads) k_rank_emit(BatchLayout L, RankA
 // ---- host sequence ----------------------------------------------------------------------------------------------------
 static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// Where ranges are ahead of hashed buckets (whole call, 60 M items): of 789 items 1 583 against 1 472 us, of 1 500 1 356 / 1 448, of
-// 5 000 1 164 / 1 331, of 12 700 1 278 / 1 304, of 20 000 1 298 / 1 231 (most of them lie in no register then).  And they have to
-// fill the SMs: three hops with 816 ranges 596 -> 581 us, 1 700 600 -> 545, 2 500 743 -> 688; with 400 ranges, and ids that crowd in
-// a few of them, a call of 6 M items took 229 us against 187.
-i64 partition_range_parts(i64 num_nodes, i64 items_per_minibatch, i64 G, bool forced) {
-  const i64 parts = ((num_nodes + kRangeSlots - 1) >> kRangeShift) + 1;
-  if (num_nodes <= 0 || parts > kNarrowWindow) return 0;
-  const bool suits = items_per_minibatch >= 1400 * parts && items_per_minibatch <= 12288 * parts && G * parts >= 512;
-  return forced || suits ? parts : 0;
+// Where classes are ahead of hashed buckets, us of a whole call hashed / classes.  40 M items over 2.45 M nodes, ids scattered evenly (in
+// brackets: all of them within 16 384 neighbours, which suits hashing best): 1 000 items a class 929 / 954 (784 / 923), 1 400 917 / 880
+// (772 / 847), 2 000 909 / 821 (771 / 786), 3 000 905 / 780 (771 / 738), 12 200 900 / 772 (785 / 714); numbered by degree, or crowding
+// as squares and fourth powers, 909 / 821, 953 / 825 and 982 / 831 at 2 000.  (Fewer than a hundred buckets in all would be no faster,
+// 1.2 M items in 60 of them 84 / 86, but a call with less than 256 has small tables that are addressed by the id.)
+i64 partition_class_parts(i64 num_nodes, i64 items_per_minibatch, bool forced) {
+  if (num_nodes <= 0 || num_nodes > (i64)(kNarrowWindow - 1) * kClassSlots) return 0;
+  const i64 needed = max((i64)11, (num_nodes + kClassSlots - 1) / kClassSlots);
+  // A prime from 11 on, so that ids that are multiples of something do not crowd in a few classes (multiples of ten in five of them:
+  // 92 us hashed, 149 us); 252 to 255, behind the last prime of that size, as they are.
+  i64 classes = needed;
+  for (i64 d = 2; d * d <= classes && needed <= 251; ++d)
+    if (classes % d == 0) ++classes, d = 1;
+  const i64 parts = classes + 1;
+  return forced || items_per_minibatch >= 2000 * parts ? parts : 0;
 }
 
 i64 partition_bucket_capacity(i64 items_bound, i64 G, i64 parts) { return parts > 0 ? G * parts : items_bound / kBucketTarget + G + 1; }
@@ -859,7 +869,8 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
                              i64 parts, bool counted, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled, Mail mail) {
   i64* counters = ctx_counters(ctx);
   PartArrays arrays = carve(L, n_cap, bucket_cap, ws);
-  arrays.P.range_parts = (u32)parts;
+  arrays.P.class_parts = (u32)parts;
+  arrays.P.class_magic = class_magic(parts);
   const PartLayout& P = arrays.P;
   const RankArrays& R = arrays.R;
   const bool wide = n_cap / L.G > (i64)kNarrowWindow * kBucketTarget * 3 / 4;  // the larger minibatches of a ragged call count
@@ -867,10 +878,10 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   const int dev = ctx_device(ctx);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     GSB_CUDA_OK(cudaFuncSetAttribute(k_part_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, kBucketSlots * 8));
-    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_scatter<kWideWindow, 512, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_scatter<kWideWindow, 512, 16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      scatter_smem(8192, kWideWindow)));
-    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_resolve_ranges, cudaFuncAttributeMaxDynamicSharedMemorySize, kRangeSlots * 4));
-    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_scatter<kNarrowWindow, 512, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_resolve_classes, cudaFuncAttributeMaxDynamicSharedMemorySize, kClassSlots * 4));
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_part_scatter<kNarrowWindow, 512, 16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      scatter_smem(8192, kNarrowWindow)));
     attr_set[dev] = true;
   }
@@ -878,8 +889,10 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
     GSB_CUDA_OK(cudaMemsetAsync(P.bucket_count, 0, sizeof(u32) * (size_t)(bucket_cap + 1), stream));
     {
       ScopedKernelTimer timer(ctx, KID_PART_COUNT, stream);
-      if (wide && parts == 0) k_part_count<kWideWindow><<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
-      else k_part_count<kNarrowWindow><<<grid_for(n_cap, kPartTile), kPartThreads, 0, stream>>>(P, n_cap, counters);
+      const int grid = grid_for(n_cap, kPartTile);
+      if (parts > 0) k_part_count<kNarrowWindow, true><<<grid, kPartThreads, 0, stream>>>(P, n_cap, counters);
+      else if (wide) k_part_count<kWideWindow, false><<<grid, kPartThreads, 0, stream>>>(P, n_cap, counters);
+      else k_part_count<kNarrowWindow, false><<<grid, kPartThreads, 0, stream>>>(P, n_cap, counters);
     }
     GSB_LAUNCH_OK();
   }
@@ -897,20 +910,23 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
   {
     ScopedKernelTimer timer(ctx, KID_PART_SCATTER, stream);
     if (wide && parts > 0)
-      k_part_scatter<kNarrowWindow, 512, 16><<<grid_for(n_cap, 8192), 512, scatter_smem(8192, kNarrowWindow), stream>>>(
+      k_part_scatter<kNarrowWindow, 512, 16, true><<<grid_for(n_cap, 8192), 512, scatter_smem(8192, kNarrowWindow), stream>>>(
           P, n_cap, counters);
     else if (wide)
-      k_part_scatter<kWideWindow, 512, 16><<<grid_for(n_cap, 8192), 512, scatter_smem(8192, kWideWindow), stream>>>(
+      k_part_scatter<kWideWindow, 512, 16, false><<<grid_for(n_cap, 8192), 512, scatter_smem(8192, kWideWindow), stream>>>(
+          P, n_cap, counters);
+    else if (parts > 0)
+      k_part_scatter<kNarrowWindow, 256, 8, true><<<grid_for(n_cap, 2048), 256, scatter_smem(2048, kNarrowWindow), stream>>>(
           P, n_cap, counters);
     else
-      k_part_scatter<kNarrowWindow, 256, 8><<<grid_for(n_cap, 2048), 256, scatter_smem(2048, kNarrowWindow), stream>>>(
+      k_part_scatter<kNarrowWindow, 256, 8, false><<<grid_for(n_cap, 2048), 256, scatter_smem(2048, kNarrowWindow), stream>>>(
           P, n_cap, counters);
   }
   GSB_LAUNCH_OK();
   {
     ScopedKernelTimer timer(ctx, KID_PART_RESOLVE, stream);
     if (parts > 0)
-      k_part_resolve_ranges<<<(int)min(bucket_cap, (i64)kNumSMs * 3 * 4), kRangeThreads, kRangeSlots * 4, stream>>>(P, counters);
+      k_part_resolve_classes<<<(int)min(bucket_cap, (i64)kNumSMs * 3 * 4), kClassThreads, kClassSlots * 4, stream>>>(P, counters);
     else
       k_part_resolve<<<(int)min(bucket_cap, (i64)kNumSMs * 4 * 4), kResolveThreads, kBucketSlots * 8, stream>>>(P, counters);
   }

@@ -197,7 +197,7 @@ struct SampleParams {
   i64 S;
   i64 k;
   int replace;
-  int bucket_ranges;  // of bucket_count below: buckets are ranges of ids (here it costs no room: eight bytes more 0.3 us a launch)
+  uint32_t bucket_magic;  // of bucket_count below: see bucket_of_id (here it costs no room: eight bytes more 0.3 us a launch)
   u64 seed;
   i64* out_indptr;
   i64* out_indices;
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
       const i64 win = b0 - s_win0;  // >= 0: minibatches follow the CTA's first one
       auto count_id = [&](i64 id) {
         if (id < 0 || id >= 0xFFFFFFFFll) return;  // never bucketed; reported by the pass that scatters the items
-        const i64 w = win + bucket_of_id((uint32_t)id, parts, p.bucket_ranges);
+        const i64 w = win + bucket_of_id((uint32_t)id, parts, p.bucket_magic);
         if (w < kCountWindow) atomicAdd(&s_cnt[w], 1u);
         else atomicAdd(p.bucket_count + s_win0 + w, 1u);
       };
@@ -602,7 +602,7 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
     if (!per_thread || !batch_ptr || G < 1) return GSB_ERR_INVALID_ARGUMENT;
     p.bucket_count = count->bucket_count;
     p.bucket_base = count->bucket_base;
-    p.bucket_ranges = count->ranges;
+    p.bucket_magic = count->magic;
   }
   {
     ScopedKernelTimer timer(ctx, KID_SAMPLE_UNIFORM, stream);

@@ -1,7 +1,7 @@
-"""The partitioned unique + relabel with buckets that are ranges of 16 384 ids: one range and many, ids on both sides of a range's
-end and of the bound (those beyond it take a bucket of their own), buckets larger than a thread's registers hold, thousands of
-repeats of one id, minibatches that are empty, tiny or large enough for the larger tiles — against the oracle; and the one-call
-hop, whose sampler counts the ranges."""
+"""The partitioned unique + relabel with buckets that are classes of up to 16 384 ids: few classes and many, ids at multiples of
+16 384 and on both sides of the bound (those beyond it take a bucket of their own), buckets larger than a thread's registers hold,
+thousands of repeats of one id, minibatches that are empty, tiny or large enough for the larger tiles — against the oracle; and the one-call
+hop, whose sampler counts the classes."""
 import numpy as np
 import pytest
 import torch

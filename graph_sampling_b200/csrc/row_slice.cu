@@ -335,7 +335,8 @@ constexpr i64 kBloomMaxRows = 1 << 18;  // beyond, most edges would pass
 // Edges per column from which pieces of columns are the faster way: 4 M edges, 20 000 rows, positions against pieces: columns of 4
 // 106 / 149 us for the call, 12 92 / 95, 16 86.5 / 85.9, 24 87 / 81, 64 69 / 65; a heavy tail of mean 16 78 / 83, of mean 32 75 / 72.
 constexpr i64 kInPieces = 20;
-constexpr i64 kInducedMaxEdges = 1 << 27;  // its scratch is 16 bytes per edge
+constexpr i64 kInducedMaxEdges = 1 << 27;  // its scratch is 12 bytes per edge
+constexpr int kInAtBits = 16;              // of a position in a warp's stretch (28 400 at most with two CTAs on each SM)
 
 struct InducedParams {
   ColRowParams c;
@@ -344,9 +345,9 @@ struct InducedParams {
   u32* totals;      // [CTAs]
   u32* warp_before;  // [CTAs][kInWarps] survivors of the CTA's warps before this one
   u32* warp_kept;   // [CTAs][kInWarps] survivors of the warp
+  u32* kept_at;     // [D] position in the warp's stretch : 16 | high part of the position in the operand : 16, ascending
+  u32* kept_edge;   // [D] its low part
   u32* kept_row;    // [D] position in row_ids
-  u32* kept_at;     // [D] position in the warp's stretch, ascending
-  i64* kept_edge;   // [D]
   GridSync sync;
 };
 
@@ -411,8 +412,8 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
     if (row != kNoRow) {
       const i64 to = begin + kept + __popc(bits & lt);
       p.kept_row[to] = row;
-      p.kept_edge[to] = e.edge;
-      p.kept_at[to] = e.at & ~kWide;
+      p.kept_edge[to] = (u32)e.edge;
+      p.kept_at[to] = (e.at << kInAtBits) | (u32)((u64)e.edge >> 32);  // (which shifts kWide out)
       // random reads that the DRAM serves 43 G of a second: they come while the filter leaves it idle
       if (c.out_data) asm volatile("prefetch.global.L2 [%0];" ::"l"(c.e_ids ? (const void*)(c.e_ids + e.edge) : c.data + e.edge));
     }
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
 #pragma unroll
     for (int q = 0; q < kAhead; ++q) {
       const u32 j = j0 + q * 32;
-      e[q] = j < kept ? __ldcg(p.kept_edge + begin + j) : -1;
+      e[q] = j < kept ? (i64)(((u64)(__ldcg(p.kept_at + begin + j) & 0xFFFFu) << 32) | __ldcg(p.kept_edge + begin + j)) : -1;
     }
 #pragma unroll
     for (int q = 0; q < kAhead; ++q)
@@ -543,7 +544,7 @@ __global__ void __launch_bounds__(kInThreads, 2) k_induced(const __grid_constant
       u32 lo = 0, hi = __ldcg(p.warp_kept + owner);  // survivors before the column: the first that lies at or behind it
       while (lo < hi) {
         const u32 mid = (lo + hi) >> 1;
-        if (__ldcg(list + mid) < at) lo = mid + 1;
+        if (__ldcg(list + mid) < at << kInAtBits) lo = mid + 1;
         else hi = mid;
       }
       rank = s_prefix[owner / kInWarps] + __ldcg(p.warp_before + owner) + lo;
@@ -717,21 +718,22 @@ int gsb_col_row_slice(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const 
     const bool pieces = D >= kInPieces * S;
     const void* kernel = pieces ? (const void*)k_induced<true> : (const void*)k_induced<false>;
     const int ctas = min(kInThreads, ctx_resident_ctas(ctx, kernel, kInThreads, kBloomMaxBits / 8, resident[pieces]));
-    if (ctas > 0) {
+    const i64 warps = (i64)ctas * kInWarps;
+    const i64 range = ctas > 0 ? max((i64)(32 * kInPer), ((D + warps - 1) / warps + 31) / 32 * 32) : 0;
+    if (ctas > 0 && range <= 1 << kInAtBits) {
       InducedParams p{};
-      const i64 warps = (i64)ctas * kInWarps;
-      p.range = max((i64)(32 * kInPer), ((D + warps - 1) / warps + 31) / 32 * 32);
+      p.range = range;
       const int grid = (int)((D + p.range * kInWarps - 1) / (p.range * kInWarps));
       auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-      const size_t edge_bytes = al(8 * (size_t)D), row_bytes = al(4 * (size_t)D);
+      const size_t part_bytes = al(4 * (size_t)D);
       void* extra;
-      int st = build_table(ctx, stream, row_ids, R, edge_bytes + 2 * row_bytes + 4 * kInThreads * (1 + 2 * kInWarps), &table, &extra,
+      int st = build_table(ctx, stream, row_ids, R, 3 * part_bytes + 4 * kInThreads * (1 + 2 * kInWarps), &table, &extra,
                            R <= kBloomMaxRows ? &p.bloom : nullptr);
       if (st != GSB_OK) return st;
-      p.kept_edge = (i64*)extra;
-      p.kept_row = (u32*)((char*)extra + edge_bytes);
-      p.kept_at = (u32*)((char*)extra + edge_bytes + row_bytes);
-      p.totals = (u32*)((char*)extra + edge_bytes + 2 * row_bytes);
+      p.kept_at = (u32*)extra;
+      p.kept_edge = (u32*)((char*)extra + part_bytes);
+      p.kept_row = (u32*)((char*)extra + 2 * part_bytes);
+      p.totals = (u32*)((char*)extra + 3 * part_bytes);
       p.warp_before = p.totals + kInThreads;
       p.warp_kept = p.warp_before + kInThreads * kInWarps;
       p.c = ColRowParams{indptr, indices, num_cols, column_ids, S, sub_indptr, D, nullptr, G, encoding_size, table,

@@ -115,7 +115,9 @@ def test_list_sampling(ops, k):
 def test_unique_and_relabel(ops, n, bound):
     ids = dev(np.random.default_rng(n).integers(0, 500_000, n))
     first, second = ids[:n // 3].contiguous(), ids[n // 3:].contiguous()
-    run_out(ops, lambda ctx: ops.graph_relabel(first, second, ctx=ctx, id_bound=bound))
+    # with a table addressed by the id the 200 CTAs of the small call are done with a few reductions each, and a wait is given up
+    # only between two arrivals
+    run_out(ops, lambda ctx: ops.graph_relabel(first, second, ctx=ctx, id_bound=bound), certain=n > 200_000 or bound == 0)
 
 
 @pytest.mark.parametrize("num_nodes", [0, 50_000])

@@ -540,8 +540,8 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_part_resolve(PartLayout 
 // kept the others waiting: 6 M items of 7 minibatches over 2.45 M nodes by a power law, whole call, hashed buckets 196 us, ranges 343
 // numbered by degree and 164 scattered, classes 166 either way.
 // Between HBM (12 bytes an item; half of the copy bandwidth) and the latency of a bucket's load, clear, reduce and read, of which an
-// SM has three in flight: 500 M items of 500 minibatches in three hops, hashed / classes: this pass 2.82 / 1.51 ms, the scatter
-// pass, whose runs are longer, 2.64 / 2.46, counting 0.67 / 0.73.
+// SM has three in flight: 500 M items of 500 minibatches in three hops, hashed / classes: this pass 2.82 / 1.50 ms, the scatter
+// pass, whose runs are longer, 2.64 / 2.45, counting 0.67 / 0.72.
 constexpr int kClassThreads = 512;
 constexpr int kClassPer = 12;  // items of a thread that stay in registers
 
@@ -573,19 +573,22 @@ __global__ void __launch_bounds__(kClassThreads, 3) k_part_resolve_classes(PartL
     const uint4 e = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
     for (u32 i = threadIdx.x; i < kClassSlots / 4; i += kClassThreads) reinterpret_cast<uint4*>(s_first)[i] = e;
     __syncthreads();
-    auto slot = [&](u64 item) { return s_first + __umulhi((u32)(item >> 32), P.class_magic); };
+    auto slot = [&](u64 item) { return __umulhi((u32)(item >> 32), P.class_magic); };
+    u32 at[kClassPer];
 #pragma unroll
-    for (int q = 0; q < kClassPer; ++q)
-      if (w[q] != kEmptyWord) atomicMin(slot(w[q]), (u32)w[q]);
+    for (int q = 0; q < kClassPer; ++q) {
+      at[q] = slot(w[q]);  // (beyond the table where there is no item)
+      if (at[q] < kClassSlots) atomicMin(s_first + at[q], (u32)w[q]);
+    }
     for (u32 j = kClassPer * kClassThreads + threadIdx.x; j < n; j += kClassThreads) {
       const u64 item = __ldg(items + j);
-      atomicMin(slot(item), (u32)item);
+      atomicMin(s_first + slot(item), (u32)item);
     }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kClassPer; ++q)
-      if (w[q] != kEmptyWord) found[q * kClassThreads + threadIdx.x] = *slot(w[q]);
-    for (u32 j = kClassPer * kClassThreads + threadIdx.x; j < n; j += kClassThreads) found[j] = *slot(__ldg(items + j));
+      if (at[q] < kClassSlots) found[q * kClassThreads + threadIdx.x] = s_first[at[q]];
+    for (u32 j = kClassPer * kClassThreads + threadIdx.x; j < n; j += kClassThreads) found[j] = s_first[slot(__ldg(items + j))];
   }
 }
 
@@ -797,9 +800,10 @@ static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Where classes are ahead of hashed buckets, us of a whole call hashed / classes.  40 M items over 2.45 M nodes, ids scattered evenly (in
 // brackets: all of them within 16 384 neighbours, which suits hashing best): 1 000 items a class 929 / 954 (784 / 923), 1 400 917 / 880
-// (772 / 847), 2 000 909 / 821 (771 / 786), 3 000 905 / 780 (771 / 738), 12 200 900 / 772 (785 / 714); numbered by degree, or crowding
-// as squares and fourth powers, 909 / 821, 953 / 825 and 982 / 831 at 2 000.  (Fewer than a hundred buckets in all would be no faster,
-// 1.2 M items in 60 of them 84 / 86, but a call with less than 256 has small tables that are addressed by the id.)
+// (772 / 847), 1 600 910 / 854 (763 / 816), 2 000 909 / 821 (771 / 786), 3 000 905 / 780 (771 / 738), 12 200 900 / 772 (785 / 714);
+// numbered by degree, or crowding as squares and fourth powers, 909 / 851, 950 / 853 and 971 / 859 at 1 600.  (Fewer than a hundred
+// buckets in all would be no faster, 1.2 M items in 60 of them 84 / 86, but a call with less than 256 has small tables that are
+// addressed by the id.)
 i64 partition_class_parts(i64 num_nodes, i64 items_per_minibatch, bool forced) {
   if (num_nodes <= 0 || num_nodes > (i64)(kNarrowWindow - 1) * kClassSlots) return 0;
   const i64 needed = max((i64)11, (num_nodes + kClassSlots - 1) / kClassSlots);
@@ -809,7 +813,7 @@ i64 partition_class_parts(i64 num_nodes, i64 items_per_minibatch, bool forced) {
   for (i64 d = 2; d * d <= classes && needed <= 251; ++d)
     if (classes % d == 0) ++classes, d = 1;
   const i64 parts = classes + 1;
-  return forced || items_per_minibatch >= 2000 * parts ? parts : 0;
+  return forced || items_per_minibatch >= 1600 * parts ? parts : 0;
 }
 
 i64 partition_bucket_capacity(i64 items_bound, i64 G, i64 parts) { return parts > 0 ? G * parts : items_bound / kBucketTarget + G + 1; }

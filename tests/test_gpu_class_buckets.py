@@ -50,11 +50,12 @@ def test_crowded_ids(oracle, nodes, kind):
     check(oracle, got, seeds, sp, edges, ep)
 
 
-# 12 buckets a minibatch up to 180 224 nodes, 20 from 294 913 on; more than 2^20 items, below that a call is one launch, and tables
+# 12 buckets a minibatch up to 180 224 nodes; more than 2^20 items, below that a call is one launch, and tables
 # of 32 MB at least with 8 bytes per id, below that they are addressed by the id
 @pytest.mark.parametrize("nodes,G,items", [
-    (180_224, 60, 23_999), (180_224, 60, 24_000), (294_912, 60, 40_000),      # 2 000 items a bucket, just below too; 19 buckets
-    (180_225, 60, 28_000), (4_177_920, 3, 520_000), (4_177_921, 3, 520_000)])  # 13 classes; the most nodes and one more
+    (180_224, 60, 19_199), (180_224, 60, 19_200), (294_912, 60, 32_000),       # 1 600 items a bucket, just below too; 19 classes
+    (180_225, 60, 22_400), (4_177_920, 3, 409_599), (4_177_920, 3, 409_600),   # 13 classes; the most nodes
+    (4_177_921, 3, 520_000)])                                                 # and one more
 def test_automatic_choice_at_its_bounds(oracle, nodes, G, items):
     from graph_sampling_b200 import ops
     ctx = ops.Context()

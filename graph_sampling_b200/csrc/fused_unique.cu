@@ -28,10 +28,10 @@
 // table of its own; ranks are then relative to the minibatch's first item.
 //
 // GPU time of a call, five launches (without the gaps between them) / hash table / direct table: 16 000 items
-// 26 / 11 / 7 us, 813 000 items 86 / 51 / 29 us.  What bounds the hash table (813 000 items): bucket reads and
+// 26 / 11 / 7 us, 813 000 items 86 / 49 / 26 us.  What bounds the hash table (813 000 items): bucket reads and
 // compare-and-swaps at the rate of the L2's atomics, 107 G/s each, and the rounds of the slowest lanes behind them.
-// Two CTAs per SM leave 64 registers a thread: eight and sixteen items per thread partly live in local memory (70 to 660
-// bytes loaded and stored per thread).
+// Two CTAs per SM leave 64 registers a thread: five and six items per thread partly live in local memory in some forms (up to 84
+// bytes stored per thread), eight, twelve and sixteen in all (76 to 616).
 #include "batch_table.cuh"
 #include "common.cuh"
 #include "grid_sync.cuh"
@@ -479,8 +479,10 @@ __global__ void __launch_bounds__(kFuThreads, 2) k_fused_unique(const __grid_con
 // ---- host side ------------------------------------------------------------------------------------------------------
 // Items per thread: the fewest whose CTAs are resident together.  A finer list than powers of two leaves fewer SMs with one CTA
 // where others have two: 700 000 items, direct / hash table, five a thread 24.3 / 48.1 us, eight 27.9 / 55.6; 340 000, three
-// 20.6 / 36.0, four 21.7 / 38.7.  Fewer CTAs of more items are never ahead, not even where that evens out the SMs: 200 000 items of 20
-// minibatches, two a thread 25.1, three 27.4.
+// 20.6 / 36.0, four 21.7 / 38.7.  With the hash table fewer CTAs of more items are never ahead, not even where that evens out the SMs:
+// 200 000 items, two a thread 30.6, three 32.6, of 20 minibatches 25.1 and 27.4.  With the direct table they sometimes are, by less
+// than a microsecond (200 000 items 19.1 and 18.4, 120 000 with one and two 17.7 and 17.3, but 260 000 with two and three 18.9
+// and 20.8), and the rule is the same for both.
 constexpr int kFuItems[] = {1, 2, 3, 4, 5, 6, 8, 12, 16};
 
 static int items_per_thread(i64 n, int max_ctas) {

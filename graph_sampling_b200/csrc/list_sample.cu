@@ -82,6 +82,9 @@ __device__ __forceinline__ void select_count(unsigned* s_hist, unsigned digit, b
   if ((rest >> (threadIdx.x & 31)) & 1u) atomicAdd(&s_hist[digit], 1u);
 }
 
+// A thread's keys in registers: 148 CTAs keep the lists of up to 1 212 416 items.  The line lies behind the million rows that layer-wise
+// sampling was timed on (22.8 us for 512 of them); beyond it composites go through memory (1 250 000 items 35.2 us, three million 46.7),
+// and more keys a thread have not been tried.
 constexpr int kSelectKept = 8;
 // Winners per CTA up to which all CTAs rank them: a rank is k comparisons by a warp (4 096 winners on 22 CTAs about 16 us, 512 on
 // three 2), the sort of one CTA 35 us for 4 096 and 6.5 for 512.

@@ -9,7 +9,8 @@
 // Few walkers (FEW) are bound by latency, and a warp takes a step when the slowest of its walkers' reads is back.  So they are
 // spread over all warps that can be resident, down to one walker per warp, and the next four draws are made while a walker waits
 // for its node: 40 steps of 256 .. 4 096 walkers over a 1 GB graph, caches flushed, 69.6 -> 47.1 us (one walker alone: 43 - 45),
-// 16 384 walkers 75.8 -> 59.5, 32 768 79.9 -> 69.6.
+// 16 384 walkers 75.8 -> 59.5, 32 768 79.9 -> 69.6.  Walker-major walks, whose rows a warp stages for its 32
+// walkers together, are not spread, nor has it been tried (80 steps of 1 024 walkers 133 us, step-major 84; of 65 536 184 and 181).
 //
 // Per step the walker does two dependent gathers (the indptr pair of the current node, then one
 // entry of indices) and one trace store.  Step-major stores (layout 0, the reference's memory

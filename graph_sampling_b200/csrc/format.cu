@@ -92,8 +92,9 @@ __device__ __forceinline__ unsigned same_digit(u32 d, int bits, bool valid) {
 // The keys of up to 26 624 edges are read from L2 by EVERY CTA (213 KB at most) and stay in its registers, so it needs nothing from
 // the others.  Each counts the edges of up to 8 192 bins of neighbouring keys, and from the counts' prefix sums all of them derive the
 // same shares: a bin costs E units and an edge as many as there are bins, a share is an equal part of that line, and so holds at
-// most two CTA's worth of edges and of keys however the keys crowd.  A bin may span several shares; its edges are then dealt out
-// by their number within the bin, and a CTA that has not the first of them counts, per key, those that others place before its own.
+// most twice an equal part of the edges and of the bins, however the keys crowd.  A bin may span several shares; its edges are then
+// dealt out by their number within the bin, and a CTA that has not the first of them counts, per key, those that others place before
+// its own.
 // Counts per key of the share's bins, their scan (the offsets), and a rank per edge among the few hundred of the share: all in
 // shared memory.
 // Bound by instruction issue, of which reading and counting all keys is the most.  us a call, calls in a row, the cooperative form

@@ -621,7 +621,8 @@ constexpr i64 kPartitionAutoItems = 1ll << 19;
 constexpr i64 kPartitionAutoMaxMinibatch = 1024ll * kBucketTarget;
 // The counting sampler flushes its per-bucket counts once per 128 columns: with more than 256 buckets a minibatch that is
 // an atomic for every other item, and the separate counting pass is cheaper (and with 151 buckets, too: sampling 8.2 -> 9.3 ms
-// against 0.67 for the pass, last hop of 500 minibatches of 813 000 items).
+// against 0.67 for the pass, last hop of 500 minibatches of 813 000 items).  Sampled by windows and with classes of ids for buckets
+// the counts of such a hop are flushed once per 512 columns by a pass that is bound by memory: 0.92 -> 1.32 ms, and no counting pass.
 constexpr i64 kSamplerCountsMaxMinibatch = 256ll * kBucketTarget;
 static inline bool partition_suits(i64 n_cap, i64 G) {
   return n_cap >= kPartitionAutoItems && n_cap / (G > 0 ? G : 1) <= kPartitionAutoMaxMinibatch;
@@ -770,13 +771,18 @@ static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64*
                                    i64 num_nodes, const i64* seeds, const i64* seeds_ptr, const i64* batch_ids, i64 G,
                                    i64 S, i64 k, i64 cap, i64 parts, int replace, u64 seed, i64* out_indptr, i64* out_indices,
                                    i64* out_select, i64* out_indices_ptr, i64* out_unique, i64* out_unique_ptr,
-                                   i64* out_relabeled, Mail mail) {
+                                   i64* out_relabeled, i64 num_edges, Mail mail) {
   i64* counters = ctx_counters(ctx);
   const i64 n_cap = S + cap;
   const size_t off_bytes = ((size_t)(G + 1) * 8 + 255) & ~(size_t)255;
   const i64 bucket_cap = partition_bucket_capacity(S * (1 + k), G, parts);
+  // the sampler's scratch lies where the passes after it keep theirs, behind the counts that it leaves them
+  const size_t bytes = 2 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap);
+  const size_t behind = 2 * off_bytes + partition_count_bytes(bucket_cap);
   void* ws;
-  int st = ctx_reserve_workspace(ctx, stream, 2 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
+  bool windows = window_sample_suits(ctx, S, k, num_edges) &&
+                 ctx_try_workspace(ctx, stream, max(bytes, behind + window_sample_bytes(ctx, S, k, num_edges)), &ws);
+  int st = windows ? GSB_OK : ctx_reserve_workspace(ctx, stream, bytes, &ws);
   if (st != GSB_OK) return st;
   void* part_ws = (char*)ws + 2 * off_bytes;
   BatchLayout L;
@@ -794,10 +800,11 @@ static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64*
     k_batch_layout<<<1, kBThreads, 0, stream>>>(L, counters, k, 1 | 8 | 32, S, cap, partition_bucket_counts(part_ws), parts);
   }
   GSB_LAUNCH_OK();
-  const SamplerCount count{partition_bucket_counts(part_ws), L.region_off, class_magic(parts)};
+  const SamplerCount count{partition_bucket_counts(part_ws), L.region_off, class_magic(parts),
+                           windows ? (char*)ws + behind : nullptr};
   st = sample_uniform_launch(ctx, stream, indptr, indices, num_nodes, seeds, S, k, replace, seed, out_indptr,
                              out_indices, out_select, nullptr, nullptr, nullptr, nullptr, cap, seeds_ptr + G,
-                             seeds_ptr, batch_ids, G, &count);
+                             seeds_ptr, batch_ids, G, &count, Mail{nullptr, 0}, windows ? num_edges : 0);
   if (st != GSB_OK) return st;
   st = partition_after_sampler(ctx, stream, L, n_cap, bucket_cap, part_ws, out_indptr, S, cap, out_indices_ptr);
   if (st != GSB_OK) return st;
@@ -863,12 +870,12 @@ int gsb_batch_unique_relabel(gsb_ctx* ctx, void* stream_, const int64_t* seeds, 
   return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
 }
 
-int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64_t* indices, int64_t num_nodes,
-                 const int64_t* seeds, const int64_t* seeds_ptr, const int64_t* batch_ids, int64_t G, int64_t S,
-                 int64_t k, int64_t edge_capacity, int replace, uint64_t seed, int flags, int64_t* out_indptr,
-                 int64_t* out_indices,
-                 int64_t* out_select, int64_t* out_indices_ptr, int64_t* out_unique, int64_t* out_unique_ptr,
-                 int64_t* out_relabeled, int64_t* unique_total_host, int64_t* edges_total_host) {
+int gsb_sage_hop_sized(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64_t* indices, int64_t num_nodes,
+                       int64_t num_edges, const int64_t* seeds, const int64_t* seeds_ptr, const int64_t* batch_ids, int64_t G,
+                       int64_t S, int64_t k, int64_t edge_capacity, int replace, uint64_t seed, int flags,
+                       int64_t* out_indptr, int64_t* out_indices, int64_t* out_select, int64_t* out_indices_ptr,
+                       int64_t* out_unique, int64_t* out_unique_ptr, int64_t* out_relabeled, int64_t* unique_total_host,
+                       int64_t* edges_total_host) {
   GSB_ENTER(ctx);
   GSB_REQUIRE(indptr && seeds_ptr && out_indptr && out_indices_ptr && out_unique_ptr && G >= 1 && S >= 0 && k >= 0 &&
                   num_nodes >= 0,
@@ -887,18 +894,19 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
   const bool fused = path == 0 && fused_unique_suits(ctx, n_cap, G);
   const bool direct_small = (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes && num_nodes > 0;
   const i64 parts = path == 3 || n_cap == 0 ? 0 : partition_class_parts(num_nodes, n_cap / G, path == 4);
-  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && n_cap / G <= kSamplerCountsMaxMinibatch &&
+  const bool counts = n_cap / G <= kSamplerCountsMaxMinibatch || (parts > 0 && window_sample_suits(ctx, S, k, num_edges));
+  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && counts &&
       (path >= 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
     st = sage_hop_sampler_counts(ctx, stream, indptr, indices, num_nodes, seeds, seeds_ptr, batch_ids, G, S, k, cap,
                                  parts, replace, (u64)seed, out_indptr, out_indices, out_select, out_indices_ptr, out_unique,
-                                 out_unique_ptr, out_relabeled, mail);
+                                 out_unique_ptr, out_relabeled, num_edges, mail);
     if (st != GSB_OK || !mail.word) return st;
     return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
   }
   // the exact seed count is seeds_ptr[G] on the device; S only has to bound it (grids, scratch and capacities)
   st = sample_uniform_launch(ctx, stream, indptr, indices, num_nodes, seeds, S, k, replace, (u64)seed, out_indptr,
                                  out_indices, out_select, nullptr, nullptr, nullptr, nullptr, cap, seeds_ptr + G,
-                                 seeds_ptr, batch_ids, G);
+                                 seeds_ptr, batch_ids, G, nullptr, Mail{nullptr, 0}, num_edges);
   if (st != GSB_OK) return st;
   if (fused) {
     BatchLayout F{};
@@ -926,6 +934,16 @@ int gsb_sage_hop(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64
   st = relabel_batches(ctx, stream, L, S, cap, num_nodes, flags, out_unique, out_unique_ptr, out_relabeled, mail);
   if (st != GSB_OK || !mail.word) return st;
   return mailed_totals(ctx, stream, mail, unique_total_host, edges_total_host);
+}
+
+int gsb_sage_hop(gsb_ctx* ctx, void* stream, const int64_t* indptr, const int64_t* indices, int64_t num_nodes,
+                 const int64_t* seeds, const int64_t* seeds_ptr, const int64_t* batch_ids, int64_t G, int64_t S,
+                 int64_t k, int64_t edge_capacity, int replace, uint64_t seed, int flags, int64_t* out_indptr,
+                 int64_t* out_indices, int64_t* out_select, int64_t* out_indices_ptr, int64_t* out_unique,
+                 int64_t* out_unique_ptr, int64_t* out_relabeled, int64_t* unique_total_host, int64_t* edges_total_host) {
+  return gsb_sage_hop_sized(ctx, stream, indptr, indices, num_nodes, 0, seeds, seeds_ptr, batch_ids, G, S, k, edge_capacity,
+                            replace, seed, flags, out_indptr, out_indices, out_select, out_indices_ptr, out_unique,
+                            out_unique_ptr, out_relabeled, unique_total_host, edges_total_host);
 }
 
 }  // extern "C"

@@ -180,6 +180,7 @@ inline uint32_t class_magic(i64 parts) { return parts > 0 ? (uint32_t)((((u64)1 
 i64 partition_bucket_capacity(i64 items_bound, i64 G, i64 parts);
 size_t partition_workspace_bytes(i64 n_cap, i64 bucket_cap);
 uint32_t* partition_bucket_counts(void* ws);
+size_t partition_count_bytes(i64 bucket_cap);  // what the counts, starts and cursors of the buckets take of it, at its head
 int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64 n_cap, i64 bucket_cap, void* ws,
                              i64 parts, bool counted, i64* out_unique, i64* out_unique_ptr, i64* out_relabeled, Mail mail);
 // The one-call hop, after its counting sampler: edge offsets of the minibatches (from the sampled block's offsets),
@@ -203,7 +204,12 @@ struct SamplerCount {
   uint32_t* bucket_count;  // [buckets]
   const i64* bucket_base;  // [G + 1] first bucket of every minibatch
   uint32_t magic;          // of the classes of ids that are the buckets, 0: hashed
+  void* scratch;           // of window_sample_bytes, or null: the call does not sample by windows
 };
+// Sampling by windows of the edges (defined in window_sample.cu): whether S columns of k picks out of a graph of num_edges take it,
+// and the scratch it needs then.
+bool window_sample_suits(gsb_ctx* ctx, i64 S, i64 k, i64 num_edges);
+size_t window_sample_bytes(gsb_ctx* ctx, i64 S, i64 k, i64 num_edges);
 constexpr int kBucketTarget = 2048;  // mean items per bucket
 
 struct CompactOut {
@@ -239,12 +245,13 @@ int unique_relabel_packed(gsb_ctx* ctx, cudaStream_t stream, const i64* first, i
                           i64* out_unique, i64* out_relabeled, i64* unique_host);
 
 // Uniform sampler shared by gsb_sample_uniform and the batched hop (defined in slice_sample.cu).  With S_dev the
-// exact seed count is read on the device and S is an upper bound that sizes the grid.
+// exact seed count is read on the device and S is an upper bound that sizes the grid.  num_edges: entries of `indices`, 0: not
+// known (a large call is then sampled in one pass whatever the graph).
 int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, const i64* indices, i64 num_cols,
                           const i64* seeds, i64 S, i64 k, int replace, u64 seed, i64* out_indptr, i64* out_indices,
                           i64* out_select, i64* out_coo_col, const float* data, const i64* e_ids, float* out_data,
                           i64 capacity, const i64* S_dev = nullptr, const i64* batch_ptr = nullptr,
                           const i64* batch_ids = nullptr, i64 G = 0, const SamplerCount* count = nullptr,
-                          Mail mail = Mail{nullptr, 0});
+                          Mail mail = Mail{nullptr, 0}, i64 num_edges = 0);
 
 }  // namespace gsb

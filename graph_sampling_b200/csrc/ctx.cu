@@ -88,6 +88,21 @@ int ctx_reserve_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, void*
   return GSB_OK;
 }
 
+bool ctx_try_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, void** out) {
+  if (bytes > ctx->workspace_bytes) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    size_t room = 0, total = 0;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+        cudaMemGetInfo(&room, &total) != cudaSuccess || bytes > room + ctx->workspace_bytes) {
+      (void)cudaGetLastError();
+      return false;
+    }
+  }
+  if (ctx_reserve_workspace(ctx, stream, bytes, out) == GSB_OK) return true;
+  (void)cudaGetLastError();
+  return false;
+}
+
 int ctx_tile_state(gsb_ctx* ctx, i64 num_tiles, cudaStream_t stream, TileState* out) {
   const int st = ctx_on_stream(ctx, stream);
   if (st != GSB_OK) return st;
@@ -505,6 +520,9 @@ int gsb_ctx_set_option(gsb_ctx* ctx, int option, int64_t value) {
       break;
     case GSB_OPT_BLOCKING_WAIT:
       if (value < 0 || value > 1) return GSB_ERR_INVALID_ARGUMENT;
+      break;
+    case GSB_OPT_SAMPLE_PATH:
+      if (value < 0 || value > 2) return GSB_ERR_INVALID_ARGUMENT;
       break;
     case GSB_OPT_DIRECT_TABLE_BUDGET:
       if (value < 0) return GSB_ERR_INVALID_ARGUMENT;

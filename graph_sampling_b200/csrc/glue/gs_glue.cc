@@ -173,11 +173,11 @@ static Sliced Sample(const CSC& g, const Tensor* seeds, int64_t fanout, bool rep
                               out_d.defined() && cap ? out_d.data_ptr<float>() : nullptr, cap, &nnz),
           "gsb_sample_weighted");
   } else {
-    Check(gsb_sample_uniform(Ctx(), Stream(), IP(g.indptr), IP(g.indices), g.indptr.numel() - 1,
-                             seeds ? IP(s) : nullptr, S, fanout, replace,
-                             NextSeed(), MP(r.indptr), MP(r.indices), MP(r.select),
-                             with_coo ? MP(r.coo_other) : nullptr, FP(d), IP(e),
-                             out_d.defined() && cap ? out_d.data_ptr<float>() : nullptr, cap, &nnz),
+    Check(gsb_sample_uniform_sized(Ctx(), Stream(), IP(g.indptr), IP(g.indices), g.indptr.numel() - 1,
+                                   g.indices.is_cuda() ? g.indices.numel() : 0, seeds ? IP(s) : nullptr, S, fanout, replace,
+                                   NextSeed(), MP(r.indptr), MP(r.indices), MP(r.select),
+                                   with_coo ? MP(r.coo_other) : nullptr, FP(d), IP(e),
+                                   out_d.defined() && cap ? out_d.data_ptr<float>() : nullptr, cap, &nnz),
           "gsb_sample_uniform");
   }
   r.indices = r.indices.narrow(0, 0, nnz);

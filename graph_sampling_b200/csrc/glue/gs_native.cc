@@ -105,6 +105,8 @@ void* stream() { return static_cast<void*>(c10::cuda::getCurrentCUDAStream().str
 c10::Device device_of(const Arg& a) {
   return a.t->is_cuda() ? a.t->device() : c10::Device(c10::kCUDA, c10::cuda::current_device());
 }
+// Entries of an array in device memory; 0 for one that is read from the host.
+int64_t device_entries(const Arg& a) { return a.t->is_cuda() ? a.numel() : 0; }
 Tensor empty(int64_t n, c10::Device dev, at::ScalarType dtype = at::kLong) {
   return at::detail::empty_cuda({n}, dtype, dev, c10::nullopt);
 }
@@ -241,9 +243,10 @@ FUNCTION(col_sampling, 12) {
                                              cols.ids(), S, fanout, replace, seed, mut(sub_indptr), mut(sub_indices),
                                              mut(select), mut(coo_col), data.floats(), e_ids.ids(), mutf(out_data), cap,
                                              &nnz)
-                       : gsb_sample_uniform(ctx, stream(), indptr.ids(), indices.ids(), num_cols, cols.ids(), S, fanout,
-                                            replace, seed, mut(sub_indptr), mut(sub_indices), mut(select), mut(coo_col),
-                                            data.floats(), e_ids.ids(), mutf(out_data), cap, &nnz);
+                       : gsb_sample_uniform_sized(ctx, stream(), indptr.ids(), indices.ids(), num_cols,
+                                                  device_entries(indices), cols.ids(), S, fanout, replace, seed,
+                                                  mut(sub_indptr), mut(sub_indices), mut(select), mut(coo_col),
+                                                  data.floats(), e_ids.ids(), mutf(out_data), cap, &nnz);
   }
   check(ctx, st, probs.given() ? "gsb_sample_weighted" : "gsb_sample_uniform");
   trim(sub_indices, nnz);
@@ -683,9 +686,10 @@ FUNCTION(sage_hop, 13) {
   int st;
   {
     NoGil free;
-    st = gsb_sage_hop(ctx, stream(), indptr.ids(), indices.ids(), indptr.numel() - 1, seeds.ids(), seeds_ptr.ids(),
-                      batch_ids.ids(), G, S, k, cap, replace, seed, flags, mut(out[0]), mut(out[1]), mut(out[2]),
-                      mut(out[4]), mut(out[6]), mut(out[5]), mut(out[3]), sync ? &nu : nullptr, sync ? &ne : nullptr);
+    st = gsb_sage_hop_sized(ctx, stream(), indptr.ids(), indices.ids(), indptr.numel() - 1, device_entries(indices),
+                            seeds.ids(), seeds_ptr.ids(), batch_ids.ids(), G, S, k, cap, replace, seed, flags, mut(out[0]),
+                            mut(out[1]), mut(out[2]), mut(out[4]), mut(out[6]), mut(out[5]), mut(out[3]),
+                            sync ? &nu : nullptr, sync ? &ne : nullptr);
   }
   check(ctx, st, "gsb_sage_hop");
   if (sync) {

@@ -818,9 +818,11 @@ i64 partition_class_parts(i64 num_nodes, i64 items_per_minibatch, bool forced) {
 
 i64 partition_bucket_capacity(i64 items_bound, i64 G, i64 parts) { return parts > 0 ? G * parts : items_bound / kBucketTarget + G + 1; }
 
+size_t partition_count_bytes(i64 bucket_cap) { return al256(sizeof(u32) * 3 * (size_t)(bucket_cap + 1)); }
+
 size_t partition_workspace_bytes(i64 n_cap, i64 bucket_cap) {
   const size_t words = (size_t)((n_cap + 31) / 32) + 2;
-  return al256(sizeof(u32) * 3 * (size_t)(bucket_cap + 1)) + al256(8 * (size_t)n_cap) + 2 * al256(4 * (size_t)n_cap) +
+  return partition_count_bytes(bucket_cap) + al256(8 * (size_t)n_cap) + 2 * al256(4 * (size_t)n_cap) +
          al256(4 * words) + al256(8 * words) + al256(8 * (2 * (size_t)n_cap + 32 * (size_t)bucket_cap + 64));
 }
 
@@ -840,7 +842,7 @@ static PartArrays carve(const BatchLayout& L, i64 n_cap, i64 bucket_cap, void* w
   P.bucket_count = (u32*)at;
   P.bucket_start = P.bucket_count + (bucket_cap + 1);
   P.bucket_cursor = P.bucket_count + 2 * (bucket_cap + 1);
-  at += al256(sizeof(u32) * 3 * (size_t)(bucket_cap + 1));
+  at += partition_count_bytes(bucket_cap);
   P.bucketed = (u64*)at;
   at += al256(8 * (size_t)n_cap);
   P.found = (u32*)at;

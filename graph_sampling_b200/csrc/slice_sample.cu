@@ -8,33 +8,15 @@
 // kTileCols per CTA, whose (start, degree, count) triples are staged in shared memory, and give each
 // column a group of 32 lanes.  Either needs O(fanout) draws per column whatever its degree (Floyd's
 // k-subset), instead of the reference's O(degree) reservoir pass (src/cuda/fusion/slice_sampling.cu:62-75).
-#include "batch_table.cuh"
 #include "column_walk.cuh"
-#include "common.cuh"
-#include "philox.cuh"
-#include "scan.cuh"
+#include "uniform_sample.cuh"
 
 namespace gsb {
 
 constexpr int kThreads = 256;
 constexpr int kTileCols = 128;  // columns per CTA of the lane-group sampler
 
-enum CountMode { COUNT_DEGREE = 0, COUNT_WOR = 1, COUNT_WR = 2 };
-
-__device__ __forceinline__ i64 column_count(i64 d, i64 k, int mode) {
-  if (mode == COUNT_DEGREE) return d;
-  if (mode == COUNT_WOR) return d < k ? d : k;
-  return d > 0 ? k : 0;
-}
-
 // ---- count + scan only (one column per thread) -------------------------------------------------
-// A seed outside [0, num_cols) counts as an empty column: its offsets are never read, GSB_ERR_INDEX_RANGE is recorded.
-__device__ __forceinline__ bool column_in_range(i64 col, i64 num_cols, i64* counters, i64 where) {
-  if ((u64)col < (u64)num_cols) return true;
-  raise_error(counters, GSB_ERR_INDEX_RANGE, where);
-  return false;
-}
-
 // PER consecutive columns per thread: one when the call is small (every column wants a thread of its own, they are all in
 // flight at once), four when it is large, where the number of tiles sets the length of the look-back chain.
 template <int PER>
@@ -189,47 +171,6 @@ static void launch_fill(FillParams p, i64 D, cudaStream_t stream) {
 }
 
 // ---- fused count + scan + uniform sampling -------------------------------------------------------
-struct SampleParams {
-  const i64* indptr;
-  const i64* indices;
-  i64 num_cols;
-  const i64* seeds;
-  i64 S;
-  i64 k;
-  int replace;
-  uint32_t bucket_magic;  // of bucket_count below: see bucket_of_id (here it costs no room: eight bytes more 0.3 us a launch)
-  u64 seed;
-  i64* out_indptr;
-  i64* out_indices;
-  i64* out_select;
-  i64* out_coo_col;
-  const float* data;
-  const i64* e_ids;
-  float* out_data;
-  i64 capacity;
-  i64* counters;
-  TileState ts;
-  const i64* S_dev;  // when set, the exact seed count lives on the device and S above is only an upper bound
-  // Minibatch form (G > 0): the seeds of minibatch j are seeds[batch_ptr[j] .. batch_ptr[j+1]) and the draws of its
-  // column number c are keyed by (batch_ids[j], c) instead of the column's position in the call, so a minibatch
-  // receives the same sample whichever call, group or GPU processes it.
-  // batch_ptr / G alone (batch_ids null) only tell the kernel which minibatch a column belongs to.
-  const i64* batch_ptr;
-  const i64* batch_ids;
-  i64 G;
-  // Per-bucket item counts of the partitioned unique + relabel that follows (thread-per-column kernels only), or null:
-  // every seed and every sampled id adds one to the count of its bucket.
-  uint32_t* bucket_count;
-  const i64* bucket_base;  // [G + 1] first bucket of every minibatch
-  Mail mail;               // the edge total, for a caller that waits for it
-};
-
-// Random-stream item of the column at position i of the call.
-__device__ __forceinline__ u64 sample_item(const SampleParams& p, i64 i, i64 batch) {
-  if (!p.batch_ids) return (u64)i;
-  return ((u64)__ldg(p.batch_ids + batch) << 32) | (u64)(uint32_t)(i - __ldg(p.batch_ptr + batch));
-}
-
 __device__ __forceinline__ void emit_pick(const SampleParams& p, i64 out_pos, i64 in_pos, i64 column_pos) {
   p.out_indices[out_pos] = __ldg(p.indices + in_pos);
   if (p.out_select) p.out_select[out_pos] = in_pos;
@@ -411,34 +352,7 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     if (i >= __ldg(p.batch_ptr + bt + 1)) bt = batch_of(p.batch_ptr, p.G, i);
   }
   uint32_t pick[KMAX];
-  if (n > 0) {
-    if (p.replace || d > k) {
-      const u64 item = sample_item(p, i, bt);
-      U32x4 blk;
-#pragma unroll
-      for (int j = 0; j < KMAX; ++j) {
-        if (j < k) {
-          if ((j & 3) == 0) blk = rand_block(p.seed, item, (u64)(j >> 2), STREAM_UNIFORM);
-          const uint32_t word =
-              (j & 3) == 0 ? blk.v[0] : (j & 3) == 1 ? blk.v[1] : (j & 3) == 2 ? blk.v[2] : blk.v[3];
-          if (p.replace) {
-            pick[j] = (uint32_t)bounded_from_word(word, (u64)d);
-          } else {
-            const uint32_t m = (uint32_t)(d - k + j);
-            const uint32_t t = (uint32_t)bounded_from_word(word, (u64)m + 1);
-            bool dup = false;
-#pragma unroll
-            for (int q = 0; q < KMAX; ++q)
-              if (q < j) dup |= (pick[q] == t);
-            pick[j] = dup ? m : t;
-          }
-        }
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < KMAX; ++j) pick[j] = (uint32_t)j;
-    }
-  }
+  if (n > 0) draw_picks<KMAX>(p, i, bt, d, pick);
   i64 val[KMAX];
 #pragma unroll
   for (int j = 0; j < KMAX; ++j)
@@ -588,7 +502,7 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
                           const i64* seeds, i64 S, i64 k, int replace, u64 seed, i64* out_indptr, i64* out_indices,
                           i64* out_select, i64* out_coo_col, const float* data, const i64* e_ids, float* out_data,
                           i64 capacity, const i64* S_dev, const i64* batch_ptr, const i64* batch_ids, i64 G,
-                          const SamplerCount* count, Mail mail) {
+                          const SamplerCount* count, Mail mail, i64 num_edges) {
   const bool per_thread = k <= 16;  // small fanouts: one lane per column, one warp per tile of 32 columns
   const int grid = per_thread ? grid_for(S, kTpcThreads) : grid_for(S, kTileCols);
   TileState ts;
@@ -603,6 +517,11 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
     p.bucket_count = count->bucket_count;
     p.bucket_base = count->bucket_base;
     p.bucket_magic = count->magic;
+  }
+  if (out_select && !out_coo_col && !out_data && window_sample_suits(ctx, S, k, num_edges)) {
+    void* ws = count ? count->scratch : nullptr;
+    if (!ws && !ctx_try_workspace(ctx, stream, window_sample_bytes(ctx, S, k, num_edges), &ws)) ws = nullptr;
+    if (ws) return window_sample_launch(ctx, stream, p, num_edges, ws);
   }
   {
     ScopedKernelTimer timer(ctx, KID_SAMPLE_UNIFORM, stream);
@@ -688,10 +607,11 @@ int gsb_batch_col_slice_fill(gsb_ctx* ctx, void* stream_, const int64_t* indptr,
   return GSB_OK;
 }
 
-int gsb_sample_uniform(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64_t* indices, int64_t num_cols,
-                       const int64_t* seeds, int64_t S, int64_t k, int replace, uint64_t seed, int64_t* out_indptr,
-                       int64_t* out_indices, int64_t* out_select, int64_t* out_coo_col, const float* data,
-                       const int64_t* e_ids, float* out_data, int64_t capacity, int64_t* nnz_host) {
+int gsb_sample_uniform_sized(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64_t* indices, int64_t num_cols,
+                             int64_t num_edges, const int64_t* seeds, int64_t S, int64_t k, int replace, uint64_t seed,
+                             int64_t* out_indptr, int64_t* out_indices, int64_t* out_select, int64_t* out_coo_col,
+                             const float* data, const int64_t* e_ids, float* out_data, int64_t capacity,
+                             int64_t* nnz_host) {
   GSB_ENTER(ctx);
   GSB_REQUIRE(indptr && out_indptr && S >= 0 && k >= 0 && num_cols >= 0 && (seeds || S <= num_cols),
               GSB_ERR_INVALID_ARGUMENT);
@@ -700,12 +620,20 @@ int gsb_sample_uniform(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const
   const Mail mail = nnz_host ? ctx_mail(ctx) : Mail{nullptr, 0};
   int st = sample_uniform_launch(ctx, stream, indptr, indices, num_cols, seeds, S, k, replace, (u64)seed, out_indptr,
                                  out_indices, out_select, out_coo_col, data, e_ids, out_data, capacity, nullptr, nullptr,
-                                 nullptr, 0, nullptr, mail);
+                                 nullptr, 0, nullptr, mail, num_edges);
   if (st != GSB_OK || !nnz_host) return st;
   i64 total = 0;
   st = ctx_mail_result(ctx, stream, mail, 1, &total);
   *nnz_host = total;
   return st;
+}
+
+int gsb_sample_uniform(gsb_ctx* ctx, void* stream, const int64_t* indptr, const int64_t* indices, int64_t num_cols,
+                       const int64_t* seeds, int64_t S, int64_t k, int replace, uint64_t seed, int64_t* out_indptr,
+                       int64_t* out_indices, int64_t* out_select, int64_t* out_coo_col, const float* data,
+                       const int64_t* e_ids, float* out_data, int64_t capacity, int64_t* nnz_host) {
+  return gsb_sample_uniform_sized(ctx, stream, indptr, indices, num_cols, 0, seeds, S, k, replace, seed, out_indptr,
+                                  out_indices, out_select, out_coo_col, data, e_ids, out_data, capacity, nnz_host);
 }
 
 int gsb_sample_one_keepdim(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const int64_t* indices,

@@ -107,14 +107,19 @@ GSB_API int gsb_check_device_status(gsb_ctx* ctx, void* stream);
  *                               stream is done, on an event created with cudaEventBlockingSync, instead of spinning
  *                               on the word in page-locked memory that the kernel leaves the result in — for hosts
  *                               that drive several streams from several threads, or several processes per machine;
- *                               default 0. */
+ *                               default 0;
+ *  GSB_OPT_SAMPLE_PATH          how uniform samples of up to 16 picks per column are taken where the number of edges is
+ *                               known: 0 (default) = in one pass, or by windows of the edges where a call reads a graph
+ *                               beyond L2 often enough; 1 = in one pass; 2 = by windows (of 1/64 of the edges and more,
+ *                               for tests).  Results are identical. */
 enum gsb_option {
   GSB_OPT_MAX_POLLS = 0,
   GSB_OPT_TABLE_SLOTS = 1,
   GSB_OPT_RELABEL_PATH = 2,
   GSB_OPT_DIRECT_TABLE_BUDGET = 3,
   GSB_OPT_BLOCKING_WAIT = 4,
-  GSB_OPT_NUM = 5
+  GSB_OPT_SAMPLE_PATH = 5,
+  GSB_OPT_NUM = 6
 };
 GSB_API int gsb_ctx_set_option(gsb_ctx* ctx, int option, int64_t value);
 GSB_API int gsb_ctx_get_option(gsb_ctx* ctx, int option, int64_t* value_host);
@@ -192,6 +197,13 @@ GSB_API int gsb_sample_uniform(gsb_ctx* ctx, void* stream, const int64_t* indptr
                                int64_t* out_indptr, int64_t* out_indices, int64_t* out_select, int64_t* out_coo_col,
                                const float* data, const int64_t* e_ids, float* out_data, int64_t capacity,
                                int64_t* nnz_host);
+/* The same for a caller that knows the number of entries of `indices` (num_edges; 0: not known, or not in device memory): a call
+ * that reads a large graph many times over then reads it in windows that L2 holds, with scratch of about 4 * S * k bytes. */
+GSB_API int gsb_sample_uniform_sized(gsb_ctx* ctx, void* stream, const int64_t* indptr, const int64_t* indices,
+                                     int64_t num_cols, int64_t num_edges, const int64_t* seeds, int64_t S, int64_t k,
+                                     int replace, uint64_t seed, int64_t* out_indptr, int64_t* out_indices,
+                                     int64_t* out_select, int64_t* out_coo_col, const float* data, const int64_t* e_ids,
+                                     float* out_data, int64_t capacity, int64_t* nnz_host);
 
 /* Keep-dimension walk step: exactly one draw per seed, -1 / -1 for an isolated seed.  Replaces
  * gs::impl::fusion::FusedCSCColSlicingSamplingOneKeepDimCUDA (src/cuda/fusion/slice_sampling.cu:156-200). */
@@ -545,6 +557,14 @@ GSB_API int gsb_sage_hop(gsb_ctx* ctx, void* stream, const int64_t* indptr, cons
                          int64_t* out_indptr, int64_t* out_indices, int64_t* out_select, int64_t* out_indices_ptr, int64_t* out_unique,
                          int64_t* out_unique_ptr, int64_t* out_relabeled, int64_t* unique_total_host,
                          int64_t* edges_total_host);
+/* The same with the number of entries of `indices` (see gsb_sample_uniform_sized). */
+GSB_API int gsb_sage_hop_sized(gsb_ctx* ctx, void* stream, const int64_t* indptr, const int64_t* indices,
+                               int64_t num_nodes, int64_t num_edges, const int64_t* seeds, const int64_t* seeds_ptr,
+                               const int64_t* batch_ids, int64_t G, int64_t S, int64_t k, int64_t edge_capacity,
+                               int replace, uint64_t seed, int flags, int64_t* out_indptr, int64_t* out_indices,
+                               int64_t* out_select, int64_t* out_indices_ptr, int64_t* out_unique,
+                               int64_t* out_unique_ptr, int64_t* out_relabeled, int64_t* unique_total_host,
+                               int64_t* edges_total_host);
 
 /* ---- unique + relabel without any allocation ----------------------------------------------------------
  * No counterpart in the reference.  For callers that must not allocate device memory while they

@@ -287,11 +287,16 @@ __global__ void __launch_bounds__(kThreads) k_sample_uniform(SampleParams p) {
 
 
 // ---- thread-per-column sampler for small fanouts --------------------------------------------------
-// One lane owns one column: it draws all k picks itself (Floyd's k-subset in registers, one Philox
-// block per four picks), issues the k gathers back to back and then stores.  A warp is a tile of 32
-// columns: counts are scanned with shuffles and the tile prefix comes from the same look-back chain,
-// so the kernel has no CTA-wide barrier at all and every lane keeps k independent loads in flight.
+// One lane owns one column: it draws all k picks itself (Floyd's k-subset in registers, one Philox block per four picks).  A
+// warp is a tile of 32 columns: counts are scanned with shuffles and the tile prefix comes from the same look-back chain, so
+// the kernel has no CTA-wide barrier at all.  The picks then change hands through shared memory: lane e % 32 reads and writes
+// pick e of the tile, with k independent loads in flight.  The picks of a column are so asked for by neighbouring lanes at
+// the same time: those in one line are one request, and lines that lie in one DRAM page arrive together, which DRAM serves
+// faster than as many anywhere (with every lane reading its own column's picks one after the other, 600 000 columns out of
+// 122 M edges, 5 / 10 / 15 picks 82 / 139 / 188 us, now 73 / 102 / 129; with data 117 / 211 / 300, now 107 / 155 / 194).
 constexpr int kTpcThreads = 128;
+constexpr int kOwnerShift = 56;
+constexpr i64 kOwnerMask = (1ll << kOwnerShift) - 1;
 constexpr int kCountWindow = 256;  // buckets a CTA of the counting sampler keeps in shared memory
 
 // COUNT: the kernel also counts, per bucket of the partitioned unique + relabel, the seeds and sampled ids of its
@@ -302,6 +307,7 @@ template <int KMAX, bool COUNT, bool DATA>
 __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams p) {
   __shared__ uint32_t s_cnt[COUNT ? kCountWindow : 1];
   __shared__ i64 s_win0;
+  __shared__ i64 s_picks[kTpcThreads / 32][32 * KMAX];
   const int lane = threadIdx.x & 31;
   const i64 tile = (i64)blockIdx.x * (kTpcThreads / 32) + (threadIdx.x >> 5);
   const i64 S = p.S_dev ? min(p.S, __ldg(p.S_dev)) : p.S;
@@ -328,7 +334,7 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     col = p.seeds ? __ldg(p.seeds + i) : i;
     if (column_in_range(col, p.num_cols, p.counters, i)) {
       b = __ldg(p.indptr + col);
-      d = __ldg(p.indptr + col + 1) - b;
+      d = max(__ldg(p.indptr + col + 1) - b, (i64)0);
     }
     f = column_count(d, k, p.replace ? COUNT_WR : COUNT_WOR);
   }
@@ -351,17 +357,26 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     bt = batch_of(p.batch_ptr, p.G, tile * 32);
     if (i >= __ldg(p.batch_ptr + bt + 1)) bt = batch_of(p.batch_ptr, p.G, i);
   }
-  uint32_t pick[KMAX];
-  if (n > 0) draw_picks<KMAX>(p, i, bt, d, pick);
-  i64 val[KMAX];
-#pragma unroll
-  for (int j = 0; j < KMAX; ++j)
-    if (j < n) val[j] = __ldg(p.indices + b + pick[j]);
-  float x[DATA ? KMAX : 1];
-  if (DATA) {
+  // The picks in the order of the output, where they lie in `indices` and which lane's column they are: lane e % 32 reads pick e,
+  // so that the picks of a column are read together and everything is written in whole lines.
+  i64* s_where = s_picks[threadIdx.x >> 5];
+  {
+    uint32_t pick[KMAX];
+    if (n > 0) draw_picks<KMAX>(p, i, bt, d, pick);
+    i64* to = s_where + (inc - f);
 #pragma unroll
     for (int j = 0; j < KMAX; ++j)
-      if (j < n) x[j] = __ldg(p.data + b + pick[j]);
+      if (j < f) to[j] = n > 0 ? (i64)lane << kOwnerShift | (b + pick[j]) : -1;
+  }
+  __syncwarp();
+  i64 val[KMAX];
+  float x[DATA ? KMAX : 1];
+#pragma unroll
+  for (int r = 0; r < KMAX; ++r) {
+    const int e = r * 32 + lane;
+    const i64 w = e < (int)total ? s_where[e] : -1;
+    val[r] = w >= 0 ? __ldg(p.indices + (w & kOwnerMask)) : -1;
+    if (DATA) x[r] = w >= 0 ? __ldg(p.data + (w & kOwnerMask)) : 0.f;
   }
   bool lost;
   const i64 prefix = __shfl_sync(0xffffffffu, tile_resolve_prefix(p.ts, (int)tile, total, &lost), 0);
@@ -383,52 +398,66 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
   }
   if (overflow && !COUNT) return;
   if (!overflow) {
-    // one array after the other, each behind one test (a test of every optional array per pick: 2 265 against 2 138 us for the
-    // last hop of 500 minibatches, 83 against 77 for 61 000 columns of ten picks)
+    // one array after the other, each behind one test
+    const int have = (int)total;
 #pragma unroll
-    for (int j = 0; j < KMAX; ++j)
-      if (j < n) p.out_indices[o + j] = val[j];
+    for (int r = 0; r < KMAX; ++r)
+      if (r * 32 + lane < have) p.out_indices[prefix + r * 32 + lane] = val[r];
     if (DATA) {
 #pragma unroll
-      for (int j = 0; j < KMAX; ++j)
-        if (j < n) p.out_data[o + j] = x[j];
+      for (int r = 0; r < KMAX; ++r)
+        if (r * 32 + lane < have) p.out_data[prefix + r * 32 + lane] = x[r];
     } else if (p.out_data) {
       float y[KMAX];
 #pragma unroll
-      for (int j = 0; j < KMAX; ++j)
-        if (j < n) y[j] = __ldg(p.data + (p.e_ids ? __ldg(p.e_ids + b + pick[j]) : b + pick[j]));
+      for (int r = 0; r < KMAX; ++r) {
+        const i64 w = r * 32 + lane < have ? s_where[r * 32 + lane] : -1;
+        y[r] = w >= 0 ? __ldg(p.data + (p.e_ids ? __ldg(p.e_ids + (w & kOwnerMask)) : w & kOwnerMask)) : 0.f;
+      }
 #pragma unroll
-      for (int j = 0; j < KMAX; ++j)
-        if (j < n) p.out_data[o + j] = y[j];
+      for (int r = 0; r < KMAX; ++r)
+        if (r * 32 + lane < have) p.out_data[prefix + r * 32 + lane] = y[r];
     }
     if (p.out_select) {
 #pragma unroll
-      for (int j = 0; j < KMAX; ++j)
-        if (j < n) p.out_select[o + j] = b + pick[j];
+      for (int r = 0; r < KMAX; ++r)
+        if (r * 32 + lane < have) p.out_select[prefix + r * 32 + lane] = s_where[r * 32 + lane] & kOwnerMask;
     }
     if (p.out_coo_col) {
 #pragma unroll
-      for (int j = 0; j < KMAX; ++j)
-        if (j < n) p.out_coo_col[o + j] = i;
+      for (int r = 0; r < KMAX; ++r)
+        if (r * 32 + lane < have) p.out_coo_col[prefix + r * 32 + lane] = tile * 32 + (s_where[r * 32 + lane] >> kOwnerShift & 31);
     }
   }
   if (COUNT) {
     // a call whose device-side sizes exceed the caller's bounds was flagged by the layout kernel: its bucket layout
     // may not fit the count array, so nothing is counted (the passes that would use the counts return at once)
-    if (valid && !overflow && p.counters[CNT_ABORT] == 0) {
-      const i64 b0 = __ldg(p.bucket_base + bt);
-      const uint32_t parts = (uint32_t)(__ldg(p.bucket_base + bt + 1) - b0);
-      const i64 win = b0 - s_win0;  // >= 0: minibatches follow the CTA's first one
-      auto count_id = [&](i64 id) {
+    if (!overflow && p.counters[CNT_ABORT] == 0) {  // uniform in the warp
+      const i64 b0 = valid ? __ldg(p.bucket_base + bt) : 0;
+      const int win = (int)(b0 - s_win0);  // >= 0: minibatches follow the CTA's first one
+      const uint32_t parts = valid ? (uint32_t)(__ldg(p.bucket_base + bt + 1) - b0) : 0;
+      auto count_id = [&](i64 id, int first, uint32_t buckets) {
         if (id < 0 || id >= 0xFFFFFFFFll) return;  // never bucketed; reported by the pass that scatters the items
-        const i64 w = win + bucket_of_id((uint32_t)id, parts, p.bucket_magic);
+        const int w = first + (int)bucket_of_id((uint32_t)id, buckets, p.bucket_magic);
         if (w < kCountWindow) atomicAdd(&s_cnt[w], 1u);
         else atomicAdd(p.bucket_count + s_win0 + w, 1u);
       };
-      count_id(col);
+      if (valid) count_id(col, win, parts);
+      const int win_first = __shfl_sync(0xffffffffu, win, 0);
+      const uint32_t parts_first = __shfl_sync(0xffffffffu, parts, 0);
+      if (__all_sync(0xffffffffu, !valid || win == win_first)) {
 #pragma unroll
-      for (int j = 0; j < KMAX; ++j)
-        if (j < n) count_id(val[j]);
+        for (int r = 0; r < KMAX; ++r)
+          if (r * 32 + lane < (int)total) count_id(val[r], win_first, parts_first);
+      } else {
+        for (int e0 = 0; e0 < (int)total; e0 += 32) {  // several minibatches: each pick's lane knows its own
+          const i64 w = e0 + lane < (int)total ? s_where[e0 + lane] : -1;
+          const int owner = (int)(w >> kOwnerShift) & 31;
+          const int first = __shfl_sync(0xffffffffu, win, owner);
+          const uint32_t buckets = __shfl_sync(0xffffffffu, parts, owner);
+          if (w >= 0) count_id(__ldg(p.indices + (w & kOwnerMask)), first, buckets);
+        }
+      }
     }
     __syncthreads();
     for (int t = threadIdx.x; t < kCountWindow; t += kTpcThreads)
@@ -489,12 +518,12 @@ static void launch_sample(const SampleParams& p, int grid, cudaStream_t stream) 
   k_sample_uniform<G><<<grid, kThreads, 0, stream>>>(p);
 }
 
-// Data gathers that go out early shorten a call that waits for latency (1 024 columns of 15 picks 16.4 -> 9.1 us, 15 000 of ten
-// 18.7 -> 13.8) and cost resident warps in one that is bound by DRAM (110 000 columns of ten 42 -> 53): up to 256 lanes per SM.
+// Data in edge order is gathered with the ids: 40 000 columns of ten picks out of 12 M edges 28.4 -> 24.0 us, 600 000 of fifteen
+// 130 -> 112, and out of 122 M, where DRAM is the bound, the same (two million columns of five 304 -> 306).
 template <int KMAX>
 static void launch_tpc(const SampleParams& p, int grid, cudaStream_t stream) {
   if (p.bucket_count) k_sample_uniform_tpc<KMAX, true, false><<<grid, kTpcThreads, 0, stream>>>(p);
-  else if (p.out_data && !p.e_ids && p.S <= kNumSMs * 256) k_sample_uniform_tpc<KMAX, false, true><<<grid, kTpcThreads, 0, stream>>>(p);
+  else if (p.out_data && !p.e_ids) k_sample_uniform_tpc<KMAX, false, true><<<grid, kTpcThreads, 0, stream>>>(p);
   else k_sample_uniform_tpc<KMAX, false, false><<<grid, kTpcThreads, 0, stream>>>(p);
 }
 
@@ -525,12 +554,10 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
   }
   {
     ScopedKernelTimer timer(ctx, KID_SAMPLE_UNIFORM, stream);
-    // the register count follows the unrolled pick array (48 / 48 / 56 / 64 / 80 registers); the usual fan-outs 5 and
-    // 10 get instantiations of their own, which removes the spilled words of <8> and <16> for them.  Measured effect on
-    // the 3-hop benchmark: none (6.45 against 6.47 ms per 1 000 minibatches) — the kernel runs at the rate at which
-    // DRAM serves random 64-byte accesses, not at the limit of its resident lanes.  Gathers through
-    // ld.global.nc.L2::64B (with or without L1::no_allocate) instead of __ldg, to keep the L2 from fetching more than
-    // one 64-byte line per gather: no change either (6.85 / 6.87 against 6.76 ms with the same run-time switch).
+    // the register count follows the unrolled pick array (40 / 46 / 48 / 56 / 64 registers); the usual fan-outs 5 and
+    // 10 get instantiations of their own.  A large call runs at the rate at which DRAM serves random 64-byte accesses, not at
+    // the limit of its resident lanes: gathers through ld.global.nc.L2::64B (with or without L1::no_allocate) instead of
+    // __ldg, to keep the L2 from fetching more than one 64-byte line per gather, changed nothing.
     if (k <= 4) launch_tpc<4>(p, grid, stream);
     else if (k <= 5) launch_tpc<5>(p, grid, stream);
     else if (k <= 8) launch_tpc<8>(p, grid, stream);

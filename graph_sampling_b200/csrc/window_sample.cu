@@ -2,7 +2,7 @@
 //
 // The last hops of a super-batch visit the columns of a graph tens of times, in an order that has nothing to do with where they
 // lie, and the thread-per-column sampler (slice_sample.cu) fetches a 64-byte line from DRAM for nearly every pick, which DRAM
-// serves at 50 G/s.  The edges are therefore cut into WINDOWS of 64 MB, and three passes take the place of one:
+// serves at 50 to 75 G/s.  The edges are therefore cut into WINDOWS of 64 MB, and three passes take the place of one:
 //
 //   draw   tiles of 512 columns in the order of the call: counts, their scan (look-back), the picks and their positions
 //          (out_select); the positions also leave, as 32-bit words, for the tile's own stretch of scratch, sorted by window;
@@ -289,17 +289,19 @@ static int window_shift(gsb_ctx* ctx, i64 num_edges) {
 static i64 window_count(gsb_ctx* ctx, i64 num_edges) { return ((num_edges - 1) >> window_shift(ctx, num_edges)) + 1; }
 
 // One pass / by windows in us, 5 and 10 and 15 picks a column, popular columns, by edges and picks per edge:
-//   20 M edges    1: 273 / 262, 244 / 280, 231 / 257    2: 525 / 455, 464 / 446, 437 / 452
-//   31 M          1: 436 / 387, 391 / 399, 400 / 406    2: 846 / 687, 757 / 680, 773 / 684
-//   60 M          0.25: 268 / 249, 246 / 257, 248 / 262    0.5: 513 / 399, 453 / 408, 466 / 419
-//   122.5 M       0.125: 328 / 276, 300 / 276, 292 / 274    0.5: 1235 / 766, 1069 / 739, 1009 / 736
-//   400 M         0.125: 1135 / 826, 994 / 757, 937 / 732    1: 8860 / 5211, 7674 / 4461, 7109 / 4383
-// The smaller the graph, the more of one pass comes out of L2, and the more often a line has to be asked for before the passes in
-// whole lines cost less; below an eighth of the edges a window's lines are hardly met twice.
+//   20 M edges    1: 262 / 270, 190 / 287, 173 / 257        2: 510 / 454, 344 / 446, 311 / 451
+//   31 M          0.5: 229 / 239, 172 / 249, 156 / 253      1: 443 / 386, 322 / 397, 290 / 405    2: 872 / 687, 622 / 680, 558 / 685
+//   60 M          0.25: 258 / 249, 203 / 257, 186 / 263     0.5: 496 / 400, 386 / 408, 348 / 417   1: 970 / 700, 751 / 689, 671 / 688
+//   122.5 M       0.125: 284 / 277, 228 / 275, 207 / 272    0.25: 544 / 444, 433 / 434, 390 / 440  0.5: 1066 / 767, 846 / 739, 755 / 735
+//   400 M         0.125: 973 / 827, 755 / 755, 667 / 729    0.25: 1922 / 1480, 1487 / 1306, 1307 / 1267
+// The smaller the graph, the more of one pass comes out of L2, and the more picks a column has, the fewer lines they touch in one
+// pass; below so many picks per edge a window's lines are hardly met twice.
 bool window_sample_suits(gsb_ctx* ctx, i64 S, i64 k, i64 num_edges) {
   const i64 path = ctx_option(ctx, GSB_OPT_SAMPLE_PATH);
   if (k < 1 || k > 16 || num_edges < 1 || path == 1 || num_edges > ((i64)kMaxWindows << kWindowShift)) return false;
-  return path == 2 || (S * k >= num_edges / 8 && (double)(S * k) * (double)num_edges >= 2e15);
+  if (path == 2) return true;
+  const double part = 5e6 * (double)(max(k, (i64)5) - 1) / (double)num_edges, picks = (double)(S * k) / (double)num_edges;
+  return num_edges >= (16 << 20) && picks >= (double)k / 64 && picks * picks >= part * part * part;
 }
 
 static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }

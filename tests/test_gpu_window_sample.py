@@ -109,18 +109,18 @@ def test_too_small_a_buffer_is_reported(graph):
 
 
 def test_automatic_choice(oracle):
-    """20 M edges, 100 M picks: just below the rule and just above, the same results."""
+    """20 M edges, 67.5 M picks: just below the rule and just above, the same results."""
     from graph_sampling_b200 import ops
     gen = torch.Generator(device="cuda")
     gen.manual_seed(1)
     indptr = torch.arange(1_000_001, device="cuda") * 20
     indices = torch.randint(0, 1_000_000, (20_000_000,), generator=gen, device="cuda")
-    for S in (9_999_999, 10_000_000):
+    for S in (6_749_900, 6_750_100):
         seeds = torch.randint(0, 1_000_000, (S,), generator=gen, device="cuda")
         plain, auto = ops.Context(), ops.Context()
         plain.set_option("sample_path", 1)
         launches = auto.launch_count()
         got = ops.fused_csc_col_slicing_sampling(indptr, indices, seeds, 10, False, seed=2, ctx=auto)
-        assert auto.launch_count() - launches == (1 if S < 10_000_000 else 3)
+        assert auto.launch_count() - launches == (1 if S < 6_750_000 else 3)
         want = ops.fused_csc_col_slicing_sampling(indptr, indices, seeds, 10, False, seed=2, ctx=plain)
         assert all(torch.equal(a, b) for a, b in zip(got, want))

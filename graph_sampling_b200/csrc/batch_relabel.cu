@@ -31,6 +31,7 @@ namespace gsb {
 // what & 1: write region_off; what & 2: write item_off (indices_ptr is valid); what & 8: region_off receives the first BUCKET of every minibatch instead of a table
 // region (partition_relabel.cu; slot_capacity then bounds the bucket count); what & 32: bucket_count, the array of
 // per-bucket item counts that the counting sampler will add to, is cleared (slot_capacity + 1 words).  bucket_parts > 0: so many buckets in every minibatch.
+// what & 16: region_off numbers the tiles of class_relabel.cu.
 // seeds_bound / edges_bound: what the caller sized grids, scratch and outputs for.  Device-side totals above them
 // record GSB_ERR_CAPACITY and set CNT_ABORT, which makes the kernels that follow in the call return at once; a look-back
 // that was given up since the last error was read sets it too, as the sizes here may be its results.
@@ -54,7 +55,10 @@ __global__ void __launch_bounds__(kBThreads) k_batch_layout(BatchLayout L, i64* 
       if (what & 2) L.item_off[b] = L.seeds_ptr[b] + L.indices_ptr[b];
       const i64 items = bound_k >= 0 ? (L.seeds_ptr[b + 1] - L.seeds_ptr[b]) * (1 + bound_k)
                                      : L.seeds_ptr[b + 1] + L.indices_ptr[b + 1] - L.seeds_ptr[b] - L.indices_ptr[b];
-      size = !(what & 8) ? region_size_for(items) : bucket_parts > 0 ? bucket_parts : (items + kBucketTarget - 1) / kBucketTarget;
+      size = what & 16          ? (items + kClassTile - 1) / kClassTile
+             : !(what & 8)      ? region_size_for(items)
+             : bucket_parts > 0 ? bucket_parts
+                                : (items + kBucketTarget - 1) / kBucketTarget;
     }
     i64 total;
     const i64 excl = block_exclusive_scan<kBThreads>(size, s_scan, &total);
@@ -621,8 +625,7 @@ constexpr i64 kPartitionAutoItems = 1ll << 19;
 constexpr i64 kPartitionAutoMaxMinibatch = 1024ll * kBucketTarget;
 // The counting sampler flushes its per-bucket counts once per 128 columns: with more than 256 buckets a minibatch that is
 // an atomic for every other item, and the separate counting pass is cheaper (and with 151 buckets, too: sampling 8.2 -> 9.3 ms
-// against 0.67 for the pass, last hop of 500 minibatches of 813 000 items).  Sampled by windows and with classes of ids for buckets
-// the counts of such a hop are flushed once per 512 columns by a pass that is bound by memory: 0.92 -> 1.32 ms, and no counting pass.
+// against 0.67 for the pass, last hop of 500 minibatches of 813 000 items).
 constexpr i64 kSamplerCountsMaxMinibatch = 256ll * kBucketTarget;
 static inline bool partition_suits(i64 n_cap, i64 G) {
   return n_cap >= kPartitionAutoItems && n_cap / (G > 0 ? G : 1) <= kPartitionAutoMaxMinibatch;
@@ -704,14 +707,16 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   }
   if (path >= 3 || (path == 0 && partition_suits(n_cap, G))) {
     // partitioned form (the default for large calls when the direct-address tables above were not chosen): shared-memory tables per bucket of items, then ranking by bit vectors
-    const i64 parts = path == 3 ? 0 : partition_class_parts(num_nodes, n_cap / G, path == 4);
+    const i64 parts = path == 3 ? 0 : partition_class_parts(num_nodes, n_cap / G, path >= 4);
+    const bool tiled = path != 4 && class_tiled(n_cap, G, parts, path == 5);
     const i64 bucket_cap = partition_bucket_capacity(n_cap, G, parts);
-    int st = ctx_reserve_workspace(ctx, stream, 3 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap), &ws);
+    const size_t bytes = tiled ? class_workspace_bytes(n_cap, G, parts) : partition_workspace_bytes(n_cap, bucket_cap);
+    int st = ctx_reserve_workspace(ctx, stream, 3 * off_bytes + bytes, &ws);
     if (st != GSB_OK) return st;
     L.item_off = (i64*)ws;
     L.region_off = (i64*)((char*)ws + off_bytes);
     L.slots = nullptr;
-    L.slot_capacity = bucket_cap;
+    L.slot_capacity = tiled ? class_tiles(n_cap, G) : bucket_cap;
     if (!L.indices_ptr) {  // one array only (batched unique): every minibatch has zero neighbours
       i64* zeros = (i64*)((char*)ws + 2 * off_bytes);
       GSB_CUDA_OK(cudaMemsetAsync(zeros, 0, off_bytes, stream));
@@ -719,9 +724,12 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
     }
     {
       ScopedKernelTimer timer(ctx, KID_OTHER, stream);
-      k_batch_layout<<<1, kBThreads, 0, stream>>>(L, counters, -1, 1 | 2 | 8, seeds_bound, edges_bound, nullptr, parts);
+      k_batch_layout<<<1, kBThreads, 0, stream>>>(L, counters, -1, 1 | 2 | (tiled ? 16 : 8), seeds_bound, edges_bound, nullptr, parts);
     }
     GSB_LAUNCH_OK();
+    if (tiled)
+      return class_unique_relabel(ctx, stream, L, n_cap, (char*)ws + 3 * off_bytes, parts, out_unique, out_unique_ptr, out_relabeled,
+                                  mail);
     return partition_unique_relabel(ctx, stream, L, n_cap, bucket_cap, (char*)ws + 3 * off_bytes, parts, false, out_unique,
                                     out_unique_ptr, out_relabeled, mail);
   }
@@ -893,9 +901,9 @@ int gsb_sage_hop_sized(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const
   const i64 path = ctx_option(ctx, GSB_OPT_RELABEL_PATH);
   const bool fused = path == 0 && fused_unique_suits(ctx, n_cap, G);
   const bool direct_small = (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes && num_nodes > 0;
-  const i64 parts = path == 3 || n_cap == 0 ? 0 : partition_class_parts(num_nodes, n_cap / G, path == 4);
-  const bool counts = n_cap / G <= kSamplerCountsMaxMinibatch || (parts > 0 && window_sample_suits(ctx, S, k, num_edges));
-  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && counts &&
+  const i64 parts = path == 3 || n_cap == 0 ? 0 : partition_class_parts(num_nodes, n_cap / G, path >= 4);
+  const bool tiled = path != 4 && n_cap > 0 && class_tiled(n_cap, G, parts, path == 5);  // which need no counts
+  if (!fused && k >= 1 && k <= 16 && n_cap > 0 && !tiled && n_cap / G <= kSamplerCountsMaxMinibatch &&
       (path >= 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
     st = sage_hop_sampler_counts(ctx, stream, indptr, indices, num_nodes, seeds, seeds_ptr, batch_ids, G, S, k, cap,
                                  parts, replace, (u64)seed, out_indptr, out_indices, out_select, out_indices_ptr, out_unique,

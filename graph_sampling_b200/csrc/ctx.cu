@@ -516,7 +516,7 @@ int gsb_ctx_set_option(gsb_ctx* ctx, int option, int64_t value) {
       if (value < 0) return GSB_ERR_INVALID_ARGUMENT;
       break;
     case GSB_OPT_RELABEL_PATH:
-      if (value < 0 || value > 4) return GSB_ERR_INVALID_ARGUMENT;
+      if (value < 0 || value > 5) return GSB_ERR_INVALID_ARGUMENT;
       break;
     case GSB_OPT_BLOCKING_WAIT:
       if (value < 0 || value > 1) return GSB_ERR_INVALID_ARGUMENT;

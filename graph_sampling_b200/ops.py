@@ -99,7 +99,8 @@ class Context:
                "sample_path": 5}
 
     def set_option(self, name, value):
-        """gsb_ctx_set_option by name: max_polls, table_slots, relabel_path (0 auto, 1 hash regions, 2 direct-address tables, 3 partitioned, 4 partitioned by classes of ids),
+        """gsb_ctx_set_option by name: max_polls, table_slots, relabel_path (0 auto, 1 hash regions, 2 direct-address tables, 3 partitioned, 4 partitioned by classes of ids, 5 the same
+        in tiles),
         direct_table_budget (bytes), blocking_wait (0 / 1), sample_path (0 auto, 1 one pass, 2 by windows of the edges)."""
         self.check(self.lib.gsb_ctx_set_option(self.handle, c_int(self.OPTIONS[name]), c_i64(int(value))),
                    "gsb_ctx_set_option")

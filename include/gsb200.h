@@ -99,7 +99,8 @@ GSB_API int gsb_check_device_status(gsb_ctx* ctx, void* stream);
  *                               2 = direct-address tables (GSB_ERR_OUT_OF_MEMORY when they do not fit);
  *                               3 = the partitioned form; 4 = the same with buckets that are classes of ids, those with
  *                               the same remainder, where num_nodes > 0 allows it (up to 4 177 920; 0 chooses them for
- *                               large calls).
+ *                               large calls); 5 = the same in tiles that sort themselves (0 chooses them for large
+ *                               minibatches).
  *                               Results are identical;
  *  GSB_OPT_DIRECT_TABLE_BUDGET  bytes the direct-address tables (8 bytes x num_nodes x minibatches per call) may
  *                               take, default 6 GiB;

@@ -293,10 +293,10 @@ __global__ void __launch_bounds__(kThreads) k_sample_uniform(SampleParams p) {
 // pick e of the tile, with k independent loads in flight.  The picks of a column are so asked for by neighbouring lanes at
 // the same time: those in one line are one request, and lines that lie in one DRAM page arrive together, which DRAM serves
 // faster than as many anywhere (with every lane reading its own column's picks one after the other, 600 000 columns out of
-// 122 M edges, 5 / 10 / 15 picks 82 / 139 / 188 us, now 73 / 102 / 129; with data 117 / 211 / 300, now 107 / 155 / 194).
+// 122 M edges, 5 / 10 / 15 picks 82 / 140 / 189 us, now 73 / 101 / 127; with data 117 / 211 / 299, now 108 / 156 / 197; 1 024
+// columns out of caches 4.8 / 5.6 / 6.7, now 4.6 / 5.1 / 5.6: what a call of a few columns takes is the instructions that every
+// SM has to read first).
 constexpr int kTpcThreads = 128;
-constexpr int kOwnerShift = 56;
-constexpr i64 kOwnerMask = (1ll << kOwnerShift) - 1;
 constexpr int kCountWindow = 256;  // buckets a CTA of the counting sampler keeps in shared memory
 
 // COUNT: the kernel also counts, per bucket of the partitioned unique + relabel, the seeds and sampled ids of its
@@ -335,6 +335,10 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     if (column_in_range(col, p.num_cols, p.counters, i)) {
       b = __ldg(p.indptr + col);
       d = max(__ldg(p.indptr + col + 1) - b, (i64)0);
+      if (d > 0xFFFFFFFFll) {  // positions inside a column are drawn from one 32-bit word
+        raise_error(p.counters, GSB_ERR_UNSUPPORTED, i);
+        d = 0;
+      }
     }
     f = column_count(d, k, p.replace ? COUNT_WR : COUNT_WOR);
   }
@@ -345,39 +349,38 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     if (lane >= o) inc += t;
   }
   const i64 total = __shfl_sync(0xffffffffu, inc, 31);
-  const bool too_long = valid && d > 0xFFFFFFFFll;   // positions inside a column are drawn from one 32-bit word
-  if (too_long) raise_error(p.counters, GSB_ERR_UNSUPPORTED, i);
   // The tile's count is published at once; its own prefix is resolved only after the picks are drawn and the gathers
   // issued, so the wait for the predecessors' counts overlaps the k random loads of every lane.
   tile_publish_aggregate(p.ts, (int)tile, total);
-  const int n = valid && !too_long ? (int)f : 0;
+  const int n = (int)f;
   // minibatch of the warp's first column by one search; a lane beyond that minibatch's end searches for itself
   i64 bt = 0;
   if (p.batch_ptr && valid) {
     bt = batch_of(p.batch_ptr, p.G, tile * 32);
     if (i >= __ldg(p.batch_ptr + bt + 1)) bt = batch_of(p.batch_ptr, p.G, i);
   }
-  // The picks in the order of the output, where they lie in `indices` and which lane's column they are: lane e % 32 reads pick e,
-  // so that the picks of a column are read together and everything is written in whole lines.
+  // The picks in the order of the output, where they lie in `indices`: lane e % 32 reads pick e, so that the picks of a column are
+  // read together and everything is written in whole lines.
   i64* s_where = s_picks[threadIdx.x >> 5];
+  i64* s_own = s_where + (int)(inc - f);  // the lane's own picks
+  const int have = (int)total;
   {
     uint32_t pick[KMAX];
     if (n > 0) draw_picks<KMAX>(p, i, bt, d, pick);
-    i64* to = s_where + (inc - f);
 #pragma unroll
     for (int j = 0; j < KMAX; ++j)
-      if (j < f) to[j] = n > 0 ? (i64)lane << kOwnerShift | (b + pick[j]) : -1;
+      if (j < n) s_own[j] = b + pick[j];
   }
   __syncwarp();
   i64 val[KMAX];
   float x[DATA ? KMAX : 1];
 #pragma unroll
-  for (int r = 0; r < KMAX; ++r) {
-    const int e = r * 32 + lane;
-    const i64 w = e < (int)total ? s_where[e] : -1;
-    val[r] = w >= 0 ? __ldg(p.indices + (w & kOwnerMask)) : -1;
-    if (DATA) x[r] = w >= 0 ? __ldg(p.data + (w & kOwnerMask)) : 0.f;
-  }
+  for (int r = 0; r < KMAX; ++r)
+    if (r * 32 + lane < have) {
+      const i64 w = s_where[r * 32 + lane];
+      val[r] = __ldg(p.indices + w);
+      if (DATA) x[r] = __ldg(p.data + w);
+    }
   bool lost;
   const i64 prefix = __shfl_sync(0xffffffffu, tile_resolve_prefix(p.ts, (int)tile, total, &lost), 0);
   const i64 o = prefix + inc - f;
@@ -399,7 +402,6 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
   if (overflow && !COUNT) return;
   if (!overflow) {
     // one array after the other, each behind one test
-    const int have = (int)total;
 #pragma unroll
     for (int r = 0; r < KMAX; ++r)
       if (r * 32 + lane < have) p.out_indices[prefix + r * 32 + lane] = val[r];
@@ -410,10 +412,8 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     } else if (p.out_data) {
       float y[KMAX];
 #pragma unroll
-      for (int r = 0; r < KMAX; ++r) {
-        const i64 w = r * 32 + lane < have ? s_where[r * 32 + lane] : -1;
-        y[r] = w >= 0 ? __ldg(p.data + (p.e_ids ? __ldg(p.e_ids + (w & kOwnerMask)) : w & kOwnerMask)) : 0.f;
-      }
+      for (int r = 0; r < KMAX; ++r)
+        if (r * 32 + lane < have) y[r] = __ldg(p.data + __ldg(p.e_ids + s_where[r * 32 + lane]));
 #pragma unroll
       for (int r = 0; r < KMAX; ++r)
         if (r * 32 + lane < have) p.out_data[prefix + r * 32 + lane] = y[r];
@@ -421,12 +421,13 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
     if (p.out_select) {
 #pragma unroll
       for (int r = 0; r < KMAX; ++r)
-        if (r * 32 + lane < have) p.out_select[prefix + r * 32 + lane] = s_where[r * 32 + lane] & kOwnerMask;
+        if (r * 32 + lane < have) p.out_select[prefix + r * 32 + lane] = s_where[r * 32 + lane];
     }
-    if (p.out_coo_col) {
-#pragma unroll
-      for (int r = 0; r < KMAX; ++r)
-        if (r * 32 + lane < have) p.out_coo_col[prefix + r * 32 + lane] = tile * 32 + (s_where[r * 32 + lane] >> kOwnerShift & 31);
+    if (!COUNT && p.out_coo_col) {
+      __syncwarp();
+      for (int j = 0; j < n; ++j) s_own[j] = i;
+      __syncwarp();
+      for (int e = lane; e < have; e += 32) p.out_coo_col[prefix + e] = s_where[e];
     }
   }
   if (COUNT) {
@@ -448,15 +449,9 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
       if (__all_sync(0xffffffffu, !valid || win == win_first)) {
 #pragma unroll
         for (int r = 0; r < KMAX; ++r)
-          if (r * 32 + lane < (int)total) count_id(val[r], win_first, parts_first);
-      } else {
-        for (int e0 = 0; e0 < (int)total; e0 += 32) {  // several minibatches: each pick's lane knows its own
-          const i64 w = e0 + lane < (int)total ? s_where[e0 + lane] : -1;
-          const int owner = (int)(w >> kOwnerShift) & 31;
-          const int first = __shfl_sync(0xffffffffu, win, owner);
-          const uint32_t buckets = __shfl_sync(0xffffffffu, parts, owner);
-          if (w >= 0) count_id(__ldg(p.indices + (w & kOwnerMask)), first, buckets);
-        }
+          if (r * 32 + lane < have) count_id(val[r], win_first, parts_first);
+      } else {  // several minibatches: every lane counts its own column's picks
+        for (int j = 0; j < n; ++j) count_id(__ldg(p.indices + s_own[j]), win, parts);
       }
     }
     __syncthreads();
@@ -554,7 +549,7 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
   }
   {
     ScopedKernelTimer timer(ctx, KID_SAMPLE_UNIFORM, stream);
-    // the register count follows the unrolled pick array (40 / 46 / 48 / 56 / 64 registers); the usual fan-outs 5 and
+    // the register count follows the unrolled pick array (56 / 52 / 64 / 72 / 96 registers); the usual fan-outs 5 and
     // 10 get instantiations of their own.  A large call runs at the rate at which DRAM serves random 64-byte accesses, not at
     // the limit of its resident lanes: gathers through ld.global.nc.L2::64B (with or without L1::no_allocate) instead of
     // __ldg, to keep the L2 from fetching more than one 64-byte line per gather, changed nothing.

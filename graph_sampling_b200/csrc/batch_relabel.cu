@@ -707,8 +707,8 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   }
   if (path >= 3 || (path == 0 && partition_suits(n_cap, G))) {
     // partitioned form (the default for large calls when the direct-address tables above were not chosen): shared-memory tables per bucket of items, then ranking by bit vectors
-    const i64 parts = path == 3 ? 0 : partition_class_parts(num_nodes, n_cap / G, path >= 4);
-    const bool tiled = path != 4 && class_tiled(n_cap, G, parts, path == 5);
+    const bool tiled = class_tiled(path, num_nodes, n_cap, G);
+    const i64 parts = path == 3 ? 0 : partition_class_parts(num_nodes, n_cap / G, tiled || path >= 4);
     const i64 bucket_cap = partition_bucket_capacity(n_cap, G, parts);
     const size_t bytes = tiled ? class_workspace_bytes(n_cap, G, parts) : partition_workspace_bytes(n_cap, bucket_cap);
     int st = ctx_reserve_workspace(ctx, stream, 3 * off_bytes + bytes, &ws);
@@ -902,7 +902,7 @@ int gsb_sage_hop_sized(gsb_ctx* ctx, void* stream_, const int64_t* indptr, const
   const bool fused = path == 0 && fused_unique_suits(ctx, n_cap, G);
   const bool direct_small = (double)G * (double)num_nodes * 8.0 <= (double)kDirectAutoBytes && num_nodes > 0;
   const i64 parts = path == 3 || n_cap == 0 ? 0 : partition_class_parts(num_nodes, n_cap / G, path >= 4);
-  const bool tiled = path != 4 && n_cap > 0 && class_tiled(n_cap, G, parts, path == 5);  // which need no counts
+  const bool tiled = n_cap > 0 && class_tiled(path, num_nodes, n_cap, G);  // which needs no counts
   if (!fused && k >= 1 && k <= 16 && n_cap > 0 && !tiled && n_cap / G <= kSamplerCountsMaxMinibatch &&
       (path >= 3 || (path == 0 && !direct_small && partition_suits(n_cap, G)))) {
     st = sage_hop_sampler_counts(ctx, stream, indptr, indices, num_nodes, seeds, seeds_ptr, batch_ids, G, S, k, cap,

@@ -187,12 +187,12 @@ int partition_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i
 // item offsets, bound check, bucket starts — everything partition_unique_relabel(counted = true) expects, one launch.
 int partition_after_sampler(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64 n_cap, i64 bucket_cap, void* ws,
                             const i64* sub_indptr, i64 S, i64 edges_bound, i64* out_indices_ptr);
-// Classes of ids where minibatches have a dozen tiles and more of kClassTile items: the tiles sort themselves (defined in
-// class_relabel.cu).  class_tiled: whether a call takes that form, for `parts` of partition_class_parts.  L.item_off and L.region_off
-// (first tile of every minibatch; class_tiles bounds the tiles) must be filled by k_batch_layout; `ws` is scratch of
+// Classes of ids where minibatches have some tiles of kClassTile items: the tiles sort themselves (defined in
+// class_relabel.cu).  class_tiled: whether a call takes that form, by the option GSB_OPT_RELABEL_PATH and its sizes.  L.item_off and
+// L.region_off (first tile of every minibatch; class_tiles bounds the tiles) must be filled by k_batch_layout; `ws` is scratch of
 // class_workspace_bytes.
 constexpr int kClassTile = 1 << 14;
-bool class_tiled(i64 items, i64 G, i64 parts, bool forced);
+bool class_tiled(i64 path, i64 num_nodes, i64 items, i64 G);
 i64 class_tiles(i64 n_cap, i64 G);
 size_t class_workspace_bytes(i64 n_cap, i64 G, i64 parts);
 int class_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L, i64 n_cap, void* ws, i64 parts, i64* out_unique,

@@ -1,4 +1,4 @@
-// Batched unique + relabel by classes of ids (see k_part_resolve_classes), for minibatches of some hundred thousand items.
+// Batched unique + relabel by classes of ids (see k_part_resolve_classes), for minibatches of a hundred thousand items and more.
 //
 // An item is the quotient of its id and its number in a tile of 16 384 items of one minibatch: one 32-bit word, half of what the
 // partitioned form moves.  A tile sorts its own stretch by class, so nothing is counted before and nothing reserved across tiles:
@@ -14,8 +14,8 @@
 // Items are numbered by tile throughout, so every minibatch begins at a tile, with bit words of its own.
 //
 // 500 minibatches of 813 000 items over 2.45 M nodes, ms, partitioned form / this: count 0.73 / none, scatter 1.94 / 1.45 (instruction
-// issue and shared memory; tiles of 8 192 1.34), resolve 0.88 / 1.21 (latency of the runs; 1.52 out of tiles of 8 192, whose runs are
-// shorter), bits 1.12 / 0.72, emit 2.20 / 1.95 (HBM).
+// issue and shared memory; tiles of 8 192 1.34), resolve 0.88 / 0.86 (1.52 out of tiles of 8 192, whose runs are shorter), bits
+// 1.12 / 0.72, emit 2.20 / 1.95 (HBM).
 #include "batch_table.cuh"
 #include "common.cuh"
 #include "scan.cuh"
@@ -51,6 +51,7 @@ struct ClassLayout {
   u64* packed;      // [tiles][kTileWords], and one: first items before the word : 32 | bits : 32
   u64* spill;       // tables of the ids beyond the bound: 2 x kClassTile x first tile + 32 x minibatch
   u32 parts, magic;
+  u32 chunks, chunk_magic;  // pieces that the runs of a class are dealt out in, and the factor that divides by them
 };
 
 // Minibatch of a tile, searched by a whole warp: 32 pivots a round.
@@ -255,109 +256,146 @@ __device__ __noinline__ void resolve_beyond(const ClassLayout& C, i64 b, u32 til
   __syncthreads();
 }
 
-constexpr int kSlots = kClassTile / 4096;  // loads of a warp for a run
-constexpr int kKeptTiles = 16 / kSlots;    // tiles of a warp whose runs stay in registers, up to 32 x kSlots words each
+// A bucket of a minibatch whose positions take more than 20 bits (see below), by a whole CTA with a table that it clears and leaves
+// as it is.
+__device__ __noinline__ void resolve_wide(const ClassLayout& C, u32 tile0, u32 tiles, u32 c, u32* s_first) {
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto each = [&](auto f) {  // f(word, position of the tile)
+    for (u32 t = warp; t < tiles; t += kClassThreads / 32) {
+      const uint16_t* start = C.start + ((size_t)(tile0 + t) * (C.parts + 1) + c);
+      u32* words = C.words + (size_t)(tile0 + t) * kClassTile;
+      for (u32 j = start[0] + lane; j < start[1]; j += 32) f(words + j, t * kClassTile);
+    }
+  };
+  __syncthreads();  // the previous bucket's look-ups are done
+  for (u32 i = threadIdx.x; i < kClassSlots; i += kClassThreads) s_first[i] = kNoFirst;
+  __syncthreads();
+  each([&](u32* word, u32 before) { atomicMin(s_first + (*word >> kNumberBits), before + (*word & kNumberMask)); });
+  __syncthreads();
+  each([&](u32* word, u32) { *word = s_first[*word >> kNumberBits]; });
+}
 
-__global__ void __launch_bounds__(kClassThreads, 3) k_class_resolve(const __grid_constant__ ClassLayout C, i64* counters) {
+constexpr int kSlots = kClassTile / 4096;  // loads of a warp for a run
+constexpr int kPositionBits = 20;
+constexpr u32 kFirstEpoch = (1u << (32 - kPositionBits)) - 1;
+constexpr u32 kEpochTiles = ((1u << kPositionBits) - 1) / kClassTile;
+constexpr int kKept = 4;  // pieces of a warp that stay in registers
+constexpr u32 kMaxChunks = 8;  // no more than 32 pieces to a warp
+static_assert(kEpochTiles * kMaxChunks <= 32 * kClassThreads / 32, "a lane to each");
+
+// CUT: the runs are long enough to be cut into pieces.
+// Two CTAs per SM, with registers for the pieces and the look-ahead: 843 us for 500 minibatches of 813 000 items; three, which spill 76
+// bytes a thread, 1 088; clearing the table for every bucket 1 200.
+template <bool CUT>
+__global__ void __launch_bounds__(kClassThreads, 2) k_class_resolve(const __grid_constant__ ClassLayout C, i64* counters) {
   extern __shared__ __align__(16) u32 s_first[];  // [kClassSlots] smallest position of every id
   if (counters[CNT_ABORT] != 0) return;
   constexpr u32 kWarps = kClassThreads / 32;
-  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = C.parts + 1;
-  const u32 buckets = (u32)(C.L.G * C.parts);
-  // The warp's tiles of a bucket's minibatch are number `warp` and every kWarps-th from there on; lane m knows the run of its number m.
-  constexpr u32 kChunk = 32 * kSlots;
-  struct Share {
-    u32 tile0, tile_end, begin, end;
-  };
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, parts = C.parts, G = (u32)C.L.G;
+  // The runs of a bucket are cut into `chunks` pieces each, all but the last of 32 kSlots words, and the warp's are number `warp` and
+  // every kWarps-th from there on; lane m knows number m.  kBeyond: the bucket is that of the ids beyond the bound.
+  constexpr u32 kBeyond = 1u << 31;
+  const u32 buckets = G * parts, magic = 0xFFFFFFFFu / parts + 1;
+  const u32 chunks = CUT ? C.chunks : 1;
+  const u32 piece = warp + lane * kWarps, own_tile = CUT ? __umulhi(piece, C.chunk_magic) : piece;
+  const u32 own_first = (piece - own_tile * chunks) * (32 * kSlots);  // word of the run, and whether the piece is the run's last
+  const bool own_last = !CUT || piece + 1 == (own_tile + 1) * chunks;
+  u32 next_tile0 = 0, next_tiles = 0;
+  u32 next_begin = 0, next_end = 0;  // put together where they are used: in here that would wait for them
   auto look_ahead = [&](u32 k) {
-    Share s{0, 0, 0, 0};
-    if (k >= buckets) return s;
-    const u32 b = k / C.parts, c = k - b * C.parts;
-    s.tile0 = (u32)__ldg(C.L.region_off + b);
-    s.tile_end = (u32)__ldg(C.L.region_off + b + 1);
-    if (c != C.parts - 1 && s.tile0 + warp + lane * kWarps < s.tile_end) {
-      const uint16_t* start = C.start + (i64)(s.tile0 + warp + lane * kWarps) * row + c;
-      s.begin = __ldg(start);
-      s.end = __ldg(start + 1);
+    if (k >= buckets) return;
+    u32 b = __umulhi(k, magic);  // k / parts, or one more
+    u32 c = k - b * parts;
+    if (c >= parts) --b, c += parts;
+    next_tile0 = (u32)__ldg(C.L.region_off + b);
+    next_tiles = (u32)__ldg(C.L.region_off + b + 1) - next_tile0;
+    next_begin = next_end = 0;
+    if (own_tile < next_tiles) {
+      const uint16_t* start = C.start + ((size_t)(next_tile0 + own_tile) * (parts + 1) + c);
+      next_begin = __ldg(start);
+      next_end = __ldg(start + 1);
     }
-    return s;
+    if (c == parts - 1) next_tiles |= kBeyond;
   };
-  Share next = look_ahead(blockIdx.x);
+  look_ahead(blockIdx.x);
+  // A table word is [epoch : 12 | position : 20]: every bucket takes a smaller epoch than the one before, so that its positions beat
+  // what that left behind and the table is not cleared in between.
+  u32 epoch = 0;
   for (u32 k = blockIdx.x; k < buckets; k += gridDim.x) {
-    const Share now = next;
-    if (now.tile0 == now.tile_end || k % C.parts == C.parts - 1) {
-      if (now.tile0 != now.tile_end)
-        resolve_beyond(C, k / C.parts, now.tile_end, C.spill + 2ull * kClassTile * now.tile0 + 32ull * (k / C.parts));
-      next = look_ahead(k + gridDim.x);
+    const u32 tile0 = next_tile0, all = next_tiles;
+    const u32 from_word = min(next_begin + own_first, next_end);
+    const u32 run = from_word | (own_last ? next_end : min(from_word + 32 * kSlots, next_end)) << 16;  // [end : 16 | begin : 16]
+    if (all == 0 || all >= kBeyond) {
+      if (all > kBeyond) resolve_beyond(C, k / parts, tile0 + all - kBeyond, C.spill + 2ull * kClassTile * tile0 + 32ull * (k / parts));
+      look_ahead(k + gridDim.x);
       continue;
     }
-    const u32 all = now.tile_end - now.tile0, tiles = warp >= all ? 0 : (all - warp + kWarps - 1) / kWarps;
-    u32* words = C.words + (i64)(now.tile0 + warp) * kClassTile + lane;
-    const u32 run_begin = now.begin, run_end = now.end;
-    u32 w[kSlots * kKeptTiles];  // their loads are in flight while the table is cleared
+    if (all > kEpochTiles) {
+      resolve_wide(C, tile0, all, k % parts, s_first);
+      epoch = 0;
+      look_ahead(k + gridDim.x);
+      continue;
+    }
+    const u32 pieces = all * chunks > warp ? (all * chunks - warp + kWarps - 1) / kWarps : 0;
+    u32* words = C.words + ((size_t)tile0 * kClassTile + lane);
+    u32 w[kSlots * kKept], at[kKept];  // their loads are in flight while the next runs are looked up
 #pragma unroll
-    for (int m = 0; m < kKeptTiles; ++m) {
+    for (int m = 0; m < kKept; ++m) {
 #pragma unroll
       for (int h = 0; h < kSlots; ++h) w[kSlots * m + h] = kNoFirst;
-      if (m >= tiles) continue;  // uniform
-      const u32 begin = __shfl_sync(0xffffffffu, run_begin, m), n = __shfl_sync(0xffffffffu, run_end, m) - begin;
-      const u32* run = words + (size_t)m * (kWarps * kClassTile) + begin;
+      if (m >= pieces) continue;  // uniform
+      const u32 r = __shfl_sync(0xffffffffu, run, m), begin = r & 0xFFFFu, n = (r >> 16) - begin;
+      at[m] = (CUT ? __shfl_sync(0xffffffffu, own_tile, m) : warp + m * kWarps) * kClassTile;
+      const u32* from = words + (at[m] + begin);
 #pragma unroll
       for (int h = 0; h < kSlots; ++h)
-        if (lane + 32 * h < n) w[kSlots * m + h] = run[32 * h];
+        if (lane + 32 * h < n) w[kSlots * m + h] = from[32 * h];
     }
-    // what does not stay: f(word, its position minus its number) for the rest of long runs and the tiles behind
-    const bool more = tiles > kKeptTiles || __any_sync(0xffffffffu, run_end - run_begin > kChunk);
+    // what does not stay: f(word, position of the tile) for the rest of long runs and the pieces behind
+    const bool more = pieces > kKept || __any_sync(0xffffffffu, (run >> 16) - (run & 0xFFFFu) > 32 * kSlots);
     auto rest = [&](auto f) {
-      for (u32 m = 0; m < tiles; ++m) {  // uniform
-        u32 begin, end;
-        if (m < 32) {
-          begin = __shfl_sync(0xffffffffu, run_begin, m);
-          end = __shfl_sync(0xffffffffu, run_end, m);
-        } else {
-          const uint16_t* start = C.start + (i64)(now.tile0 + warp + m * kWarps) * row + k % C.parts;
-          begin = __ldg(start);
-          end = __ldg(start + 1);
-        }
-        u32* run = words + (size_t)m * (kWarps * kClassTile);
-        for (u32 j = begin + (m < kKeptTiles ? kChunk : 0); j < end; j += kChunk) {
-#pragma unroll
-          for (int h = 0; h < kSlots; ++h)
-            if (j + 32 * h + lane < end) f(run + j + 32 * h, (warp + m * kWarps) * kClassTile);
-        }
+#pragma unroll 1
+      for (u32 m = 0; m < pieces; ++m) {  // uniform
+        const u32 r = __shfl_sync(0xffffffffu, run, m), tile = __shfl_sync(0xffffffffu, own_tile, m) * kClassTile;
+#pragma unroll 1
+        for (u32 j = (r & 0xFFFFu) + (m < kKept ? 32 * kSlots : 0); j + lane < r >> 16; j += 32) f(words + (tile + j), tile);
       }
     };
-    next = look_ahead(k + gridDim.x);
+    look_ahead(k + gridDim.x);
     __syncthreads();  // the previous bucket's look-ups are done
-    const uint4 e = make_uint4(kNoFirst, kNoFirst, kNoFirst, kNoFirst);
-    for (u32 i = threadIdx.x; i < kClassSlots / 4; i += kClassThreads) reinterpret_cast<uint4*>(s_first)[i] = e;
-    __syncthreads();
+    if (epoch == 0) {
+      const uint4 e = make_uint4(kNoFirst, kNoFirst, kNoFirst, kNoFirst);
+      for (u32 i = threadIdx.x; i < kClassSlots / 4; i += kClassThreads) reinterpret_cast<uint4*>(s_first)[i] = e;
+      epoch = kFirstEpoch + 1;
+      __syncthreads();
+    }
+    --epoch;
+    const u32 tag = epoch << kPositionBits;
+    constexpr u32 kMask = (1u << kPositionBits) - 1;
 #pragma unroll
-    for (int m = 0; m < kKeptTiles; ++m) {
-      if (m >= tiles) continue;
+    for (int m = 0; m < kKept; ++m) {
+      if (m >= pieces) continue;
 #pragma unroll
       for (int h = 0; h < kSlots; ++h) {
         const u32 x = w[kSlots * m + h];
-        if (x != kNoFirst) atomicMin(s_first + (x >> kNumberBits), (warp + m * kWarps) * kClassTile + (x & kNumberMask));
+        if (x != kNoFirst) atomicMin(s_first + (x >> kNumberBits), tag + at[m] + (x & kNumberMask));
       }
     }
-    if (next.begin < next.end) {  // the next bucket's words on their way to L2
-      const u32* run = C.words + (i64)(next.tile0 + warp + lane * kWarps) * kClassTile;
-      const u32 last = next.end - 1;
-      for (u32 j = next.begin; j < next.end + 31; j += 32)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(run + min(j, last)));
+    if (more) rest([&](u32* word, u32 before) { atomicMin(s_first + (*word >> kNumberBits), tag + before + (*word & kNumberMask)); });
+    if (own_last && next_begin < next_end) {  // the next bucket's words on their way to L2
+      const u32* from = C.words + (size_t)(next_tile0 + own_tile) * kClassTile;
+      for (u32 j = next_begin; j < next_end + 31; j += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(from + min(j, next_end - 1)));
     }
-    if (more) rest([&](u32* word, u32 before) { atomicMin(s_first + (*word >> kNumberBits), before + (*word & kNumberMask)); });
     __syncthreads();
 #pragma unroll
-    for (int m = 0; m < kKeptTiles; ++m) {
-      if (m >= tiles) continue;
-      u32* run = words + (size_t)m * (kWarps * kClassTile) + __shfl_sync(0xffffffffu, run_begin, m);
+    for (int m = 0; m < kKept; ++m) {
+      if (m >= pieces) continue;
+      u32* to = words + (at[m] + (__shfl_sync(0xffffffffu, run, m) & 0xFFFFu));
 #pragma unroll
       for (int h = 0; h < kSlots; ++h)
-        if (w[kSlots * m + h] != kNoFirst) run[32 * h] = s_first[w[kSlots * m + h] >> kNumberBits];
+        if (w[kSlots * m + h] != kNoFirst) to[32 * h] = s_first[w[kSlots * m + h] >> kNumberBits] & kMask;
     }
-    if (more) rest([&](u32* word, u32) { *word = s_first[*word >> kNumberBits]; });
+    if (more) rest([&](u32* word, u32) { *word = s_first[*word >> kNumberBits] & kMask; });
   }
 }
 
@@ -503,13 +541,23 @@ __global__ void __launch_bounds__(kEmitThreads) k_class_emit(ClassLayout C, Comp
 // ---- host ---------------------------------------------------------------------------------------------------------------
 static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// From some fifteen tiles a minibatch on, as many as a CTA of the resolve pass has warps.  us of a whole call, the partitioned form with
-// classes / this: 40 M items over 2.45 M nodes in minibatches of 152 000 943 / 960, 243 000 842 / 811, 289 000 819 / 720, 760 000
-// 741 / 613; 6 M items 152 000 189 / 202, 243 000 169 / 176, 289 000 169 / 161, 760 000 145 / 132; over 500 000 nodes in minibatches
-// of 160 000 741 / 781 and 152 / 165.
-bool class_tiled(i64 items, i64 G, i64 parts, bool forced) {
+// us of a whole call, hashed buckets / the partitioned form with classes / this (ids scattered evenly; in brackets: by a power law
+// numbered by degree), by nodes and items of a minibatch:
+//   40 M items, 2.45 M nodes    76 000 974 / 1187 / 954 (998 / 1189 / 1023)    106 400 973 / 1045 / 821 (978 / 1046 / 878)
+//                               243 200 960 / 845 / 665 (967 / 848 / 692)      760 000 943 / 740 / 572 (1022 / 757 / 602)
+//               1 M nodes       34 000 1005 / 1214 / 1114 (965 / 1216 / 1187)  47 600 969 / 1045 / 910 (1059 / 1049 / 966)
+//                               108 800 949 / 840 / 700 (958 / 845 / 730)      340 000 934 / 736 / 587 (974 / 743 / 629)
+//               700 000         30 800 1008 / 1080 / 949 (969 / 1082 / 1006)   70 400 953 / 843 / 738 (963 / 847 / 783)
+//               500 000         38 400 986 / 919 / 831 (1017 / 923 / 989)      51 200 951 / 825 / 764 (961 / 830 / 882)
+//               180 000         19 200 1018 / 910 / 1402                       60 000 934 / 762 / 957
+//   1.4 M items, 2.45 M nodes   136 800 92 / 87 / 76 (126 / 88 / 81)           760 000 (one) 74 / 59 / 67 (172 / 72 / 81)
+// With few classes a tile's run is longer than the pieces it is cut into; with few tiles SMs are left idle.
+bool class_tiled(i64 path, i64 num_nodes, i64 items, i64 G) {
+  const i64 parts = path == 0 || path == 5 ? partition_class_parts(num_nodes, items / G, true) : 0;
   if (parts <= 0 || parts > kMaxParts || G > items / (kClassTile / 2) + 4096) return false;
-  return forced || items / G >= 16 * kClassTile;
+  if (path == 5) return true;
+  const i64 minibatch = items / G;
+  return parts >= 40 && minibatch >= max(700 * parts, (i64)36'000) && (items >= 4'000'000 || minibatch < 1600 * parts);
 }
 
 i64 class_tiles(i64 n_cap, i64 G) { return n_cap / kClassTile + G; }
@@ -528,6 +576,8 @@ int class_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L
   C.L = L;
   C.parts = (u32)parts;
   C.magic = class_magic(parts);
+  C.chunks = (u32)min((i64)kMaxChunks, (kClassTile / (parts - 1) + 12 + 32 * kSlots - 1) / (32 * kSlots));  // most runs of the mean's size fit
+  C.chunk_magic = 0xFFFFFFFFu / C.chunks + 1;
   char* at = (char*)ws;
   auto take = [&](size_t bytes) {
     char* p = at;
@@ -545,7 +595,8 @@ int class_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L
   static bool attr_set[64] = {};
   const int dev = ctx_device(ctx);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    GSB_CUDA_OK(cudaFuncSetAttribute(k_class_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, kClassSlots * 4));
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_class_resolve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClassSlots * 4));
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_class_resolve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClassSlots * 4));
     GSB_CUDA_OK(cudaFuncSetAttribute(k_class_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kClassTile));
     GSB_CUDA_OK(cudaFuncSetAttribute(k_class_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kClassTile));
     attr_set[dev] = true;
@@ -557,7 +608,9 @@ int class_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L
   GSB_LAUNCH_OK();
   {
     ScopedKernelTimer timer(ctx, KID_PART_RESOLVE, stream);
-    k_class_resolve<<<(int)min(L.G * parts, (i64)kNumSMs * 3 * 4), kClassThreads, kClassSlots * 4, stream>>>(C, counters);
+    const int grid = (int)min(L.G * parts, (i64)kNumSMs * 2);
+    if (C.chunks > 1) k_class_resolve<true><<<grid, kClassThreads, kClassSlots * 4, stream>>>(C, counters);
+    else k_class_resolve<false><<<grid, kClassThreads, kClassSlots * 4, stream>>>(C, counters);
   }
   GSB_LAUNCH_OK();
   {

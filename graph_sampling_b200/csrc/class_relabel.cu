@@ -15,7 +15,7 @@
 //
 // 500 minibatches of 813 000 items over 2.45 M nodes, ms, partitioned form / this: count 0.73 / none, scatter 1.94 / 1.45 (instruction
 // issue and shared memory; tiles of 8 192 1.34), resolve 0.88 / 0.86 (1.52 out of tiles of 8 192, whose runs are shorter), bits
-// 1.12 / 0.72, emit 2.20 / 1.95 (HBM).
+// 1.12 / 0.72, emit 2.20 / 1.78 (HBM).
 #include "batch_table.cuh"
 #include "common.cuh"
 #include "scan.cuh"
@@ -492,6 +492,9 @@ constexpr int kEmitItems = kEmitThreads * kEmitGroups;
 
 __device__ __forceinline__ u32 rank_in(u64 w, u32 bit) { return (u32)(w >> 32) + __popc((u32)w & ((1u << bit) - 1u)); }
 
+// The outputs are stored as what nobody reads soon: they are most of the traffic, and what the pass looks up stays in L2 (400 M items
+// 1.95 -> 1.78 ms; in k_rank_emit 7.2 M 44.5 -> 41.4 us; the sampling passes, the row copy and the other passes here are no faster
+// with it).  Two / eight groups a warp 2.16 / 2.93 ms, six CTAs an SM 2.35.
 __global__ void __launch_bounds__(kEmitThreads) k_class_emit(ClassLayout C, CompactOut out, i64* __restrict__ out_relabeled,
                                                              i64* counters) {
   if (counters[CNT_ABORT] != 0) return;
@@ -528,9 +531,9 @@ __global__ void __launch_bounds__(kEmitThreads) k_class_emit(ClassLayout C, Comp
     const u32 i = first + q * 32;
     if (i >= items) continue;
     const u32 pos = rank_in(own[q], lane);
-    if (r[q] == i) out.unique[pos] = node[q];
+    if (r[q] == i) __stcs(out.unique + pos, node[q]);
     // an id outside the accepted range has no word and its ref says so
-    if (i >= ns && rel) rel[i] = r[q] < items ? (i64)(rank_in(of_first[q], r[q] & 31u) - front) : (i64)-1;
+    if (i >= ns && rel) __stcs(rel + i, r[q] < items ? (i64)(rank_in(of_first[q], r[q] & 31u) - front) : (i64)-1);
   }
   if (first == 0) {  // the frontier of the minibatch starts here; empty minibatches before it start here too
     out.unique_ptr[t.batch] = front;

@@ -759,7 +759,7 @@ __global__ void __launch_bounds__(kBitsThreads) k_rank_emit(BatchLayout L, RankA
       const u32 lc = lc0 + q * 32;
       if (q * 32 + lane >= here) continue;
       const u32 pos = rank_in_word(own[q], lane);
-      if (r[q] == lc) out.unique[pos] = node[q];
+      if (r[q] == lc) __stcs(out.unique + pos, node[q]);  // (see k_class_emit)
       if (lc == 0) {  // the frontier of the minibatch starts here; empty minibatches before it start here too
         out.unique_ptr[u.batch] = pos;
         for (i64 e = u.batch - 1; e >= 0 && __ldg(L.item_off + e) == u.begin; --e) out.unique_ptr[e] = pos;
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(kBitsThreads) k_rank_emit(BatchLayout L, RankA
       // an id outside the accepted range was never bucketed and its ref says so; any value that is not a position of
       // this minibatch is treated alike, so no look-up can leave the rank array
       if (lc >= ns && rel)
-        rel[lc] = r[q] < items ? (i64)(rank_in_word(wref[q], (r[q] + shift) & 31u) - front) : (i64)-1;
+        __stcs(rel + lc, r[q] < items ? (i64)(rank_in_word(wref[q], (r[q] + shift) & 31u) - front) : (i64)-1);
     }
     return;
   }

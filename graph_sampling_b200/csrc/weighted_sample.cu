@@ -4,7 +4,8 @@
 // log2(u) / w (a monotone transform of the reference's u^(1/w), src/cuda/sampling_probs.cu:70-72)
 // from the Philox word keyed by (seed, column position, edge position); the k largest keys win.
 // A column of at most 128 edges is sorted: four edges per lane, so that 8, 16 or 32 lanes hold a column and a warp takes four,
-// two or one of them at a time through a register sorting network.  In a longer column the warp keeps the running top-k as
+// two or one of them at a time: through a register sorting network, or, where k is small beside the lanes, behind a bound that few
+// edges reach.  In a longer column the warp keeps the running top-k as
 // a sorted list, one entry per lane (k <= 32, the reference's own limit: sampling_probs.cu:32).  A new key enters the list
 // only if it beats the current k-th entry, which after the first few dozen edges is rare, so a hub column costs one key
 // evaluation per edge plus O(k log(deg/k)) list insertions.  Ties rank the smaller edge position first; the output is in
@@ -19,7 +20,7 @@
 // work from the lists, the longest first.  What bounds the sampler is latency — a column is three dependent reads, a draw, a
 // sort or a scan, a gather — so what counts is that no warp waits for another one's columns.  With a tile of columns per CTA
 // a CTA lived as long as its slowest column and hubs were scanned one after the other: 65 537 columns of 50 edges, fan-out
-// 16: 112 us, 2 048 hub columns with 1.2 M edges 82 us; now 68 and 43 us.
+// 16: 112 us, 2 048 hub columns with 1.2 M edges 82 us; now 64 and 42 us.
 #include "common.cuh"
 #include "philox.cuh"
 #include "grid_sync.cuh"
@@ -159,8 +160,13 @@ __device__ __forceinline__ float4 four_weights(const float* probs, u32 e, u32 en
 // Edges e_begin .. min(e_end, e_begin + 4 lanes) - 1 of one column, in descending order, by `lanes` lanes (8, 16 or 32: a warp
 // does 32 / lanes columns in step): lane g holds the composites (order-preserving image of the key : 32 | ~position : 32) of
 // edges 4g .. 4g+3 and a bitonic network — steps below 4 inside a lane, the others by exchange — orders them.  Leaves the
-// composites in `s_order`, which is the warp's: position 4 lanes x group + rank; 0, which ranks last, where there is no edge.
-__device__ __noinline__ void sort_edges(u64 seed, const float* probs, i64 col_pos, u32 e_begin, u32 e_end, u32 lanes,
+// composites in `s_order`, which is the warp's: position 4 lanes x group + rank, the first k of them at least; 0, which ranks last,
+// where there is no edge.
+// Where k is no more than half the lanes the k best are nearly always among few: the k-th largest of the lanes' own best keys is a
+// bound that k entries reach, and what reaches it (20 of 128 for k = 16) is ranked by counting, one entry per lane.  With a larger k
+// more entries than lanes would reach it, so the network stays; it also stays for the group of columns of which one has that many.
+// 300 000 columns of 50 edges, network / bound: k = 2 241 / 196 us, 5 247 / 213, 10 257 / 234, 16 253 / 237.
+__device__ __noinline__ void sort_edges(u64 seed, const float* probs, i64 col_pos, u32 e_begin, u32 e_end, u32 lanes, u32 k,
                                         u64* s_order) {
   const u32 g = (u32)lane_id() & (lanes - 1), e = e_begin + 4 * g;
   u64 c0 = 0, c1 = 0, c2 = 0, c3 = 0;
@@ -170,6 +176,42 @@ __device__ __noinline__ void sort_edges(u64 seed, const float* probs, i64 col_po
     if (e + 1 < e_end) c1 = ((u64)sortable_key(key.y) << 32) | (u64)~(e + 1);
     if (e + 2 < e_end) c2 = ((u64)sortable_key(key.z) << 32) | (u64)~(e + 2);
     if (e + 3 < e_end) c3 = ((u64)sortable_key(key.w) << 32) | (u64)~(e + 3);
+  }
+  if (2 * k <= lanes) {
+    const unsigned group = lanes == 32 ? 0xffffffffu : ((1u << lanes) - 1u) << (lane_id() - g), lt = (1u << lane_id()) - 1u;
+    u32 bound = (u32)(max(max(c0, c1), max(c2, c3)) >> 32);
+#pragma unroll 1
+    for (u32 size = 2; size <= lanes; size <<= 1) {
+#pragma unroll 1
+      for (u32 step = size >> 1; step > 0; step >>= 1) {
+        const u32 other = __shfl_xor_sync(0xffffffffu, bound, step);
+        bound = ((g & step) == 0) == ((g & size) == 0) ? max(bound, other) : min(bound, other);
+      }
+    }
+    bound = __shfl_sync(0xffffffffu, bound, k - 1, lanes);
+    auto reaches = [&](u64 c) { return c != 0 && (u32)(c >> 32) >= bound; };
+    const unsigned b0 = __ballot_sync(0xffffffffu, reaches(c0)) & group, b1 = __ballot_sync(0xffffffffu, reaches(c1)) & group,
+                   b2 = __ballot_sync(0xffffffffu, reaches(c2)) & group, b3 = __ballot_sync(0xffffffffu, reaches(c3)) & group;
+    const u32 n0 = __popc(b0), n1 = n0 + __popc(b1), n2 = n1 + __popc(b2), n = n2 + __popc(b3);
+    if (__all_sync(0xffffffffu, n <= lanes)) {
+      u64* s_group = s_order + 4 * (lane_id() - g);
+      __syncwarp();  // the last readers of s_order are done
+      if (reaches(c0)) s_group[__popc(b0 & lt)] = c0;
+      if (reaches(c1)) s_group[n0 + __popc(b1 & lt)] = c1;
+      if (reaches(c2)) s_group[n1 + __popc(b2 & lt)] = c2;
+      if (reaches(c3)) s_group[n2 + __popc(b3 & lt)] = c3;
+      if (g >= n) s_group[g] = 0;
+      __syncwarp();
+      const u64 own = s_group[g];
+      const u32 most = __reduce_max_sync(0xffffffffu, n);
+      u32 rank = 0;
+#pragma unroll 4
+      for (u32 j = 0; j < most; ++j) rank += s_group[j] > own;  // (most <= lanes)
+      __syncwarp();
+      if (g < n) s_group[rank] = own;
+      __syncwarp();
+      return;
+    }
   }
   auto order = [](u64& x, u64& y, bool descending) {
     const bool swap = (x < y) == descending;
@@ -226,7 +268,7 @@ __device__ __noinline__ ListEntry topk_scan(u64 seed, const float* probs, i64 co
   const u32 lane = (u32)lane_id();
   const unsigned kmask = k >= 32 ? 0xffffffffu : ((1u << k) - 1u);
   float4 ahead = four_weights(probs, e_begin + 128 + 4 * lane, e_end);
-  sort_edges(seed, probs, col_pos, e_begin, e_end, 32, s_order);
+  sort_edges(seed, probs, col_pos, e_begin, e_end, 32, (u32)k, s_order);
   const u64 own = (int)lane < k ? s_order[lane] : 0;
   float my_key = own ? key_of_sortable((u32)(own >> 32)) : neg_inf;
   u32 my_idx = own ? ~(u32)own : kNoIdx;
@@ -401,7 +443,7 @@ __device__ __forceinline__ void short_columns(const WeightedParams& p, int kind,
     column = column_of(p, c, false);
     o = __ldcg(p.out_indptr + c);
   }
-  if (kind != KIND_COPY) sort_edges(p.seed, p.probs + column.b, c, 0, (u32)column.d, lanes, s_order);
+  if (kind != KIND_COPY) sort_edges(p.seed, p.probs + column.b, c, 0, (u32)column.d, lanes, (u32)p.k, s_order);
   const u64* order = s_order + 4 * (lane - g);
 #pragma unroll 1
   for (i64 j = g; j < min(p.k, column.d); j += lanes)

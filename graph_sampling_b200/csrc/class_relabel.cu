@@ -13,7 +13,7 @@
 //
 // Items are numbered by tile throughout, so every minibatch begins at a tile, with bit words of its own.
 //
-// 500 minibatches of 813 000 items over 2.45 M nodes, ms, partitioned form / this: count 0.73 / none, scatter 1.94 / 1.45 (instruction
+// 500 minibatches of 813 000 items over 2.45 M nodes, ms, partitioned form / this: count 0.73 / none, scatter 1.94 / 1.29 (instruction
 // issue and shared memory; tiles of 8 192 1.34), resolve 0.88 / 0.86 (1.52 out of tiles of 8 192, whose runs are shorter), bits
 // 1.12 / 0.72, emit 2.20 / 1.78 (HBM).
 #include "batch_table.cuh"
@@ -25,6 +25,7 @@ namespace gsb {
 constexpr int kTileThreads = 512;
 constexpr u32 kClassThreads = 512;
 constexpr int kTilePer = kClassTile / kTileThreads;
+constexpr int kScatterBytes = 6 * kClassTile;  // a word and a rank per item
 constexpr int kNumberBits = 14;  // of an item in its tile
 constexpr u32 kNumberMask = (1u << kNumberBits) - 1;
 static_assert(kClassTile == 1 << kNumberBits && (u64)kClassSlots * kClassTile < (1ull << 32), "quotient and number share a word");
@@ -92,7 +93,9 @@ __device__ __forceinline__ i64 item_id(const BatchLayout& L, const TileOwner& t,
   return __ldg(i < t.num_seeds ? L.seeds + t.seeds + i : L.indices + t.edges + i);
 }
 
-// The ids are read twice, the second time out of L2, so that a thread keeps 16 bits of each of its 32 items and not 64.
+// A thread keeps its 32 ids in registers between counting and placing, the next eight always on their way, and their ranks in shared
+// memory.  Ranks in registers and ids read again (out of L2) took 1.45 ms for 407 M items and 0.38 for 82 M; this 1.29 and 0.31.  Without the second
+// set of eight 1.36 and 0.33; 16 at once 1.35, four and four 1.35, 1 024 threads 1.36 and 0.31.
 __global__ void __launch_bounds__(kTileThreads, 2) k_class_scatter(ClassLayout C, i64* counters) {
   extern __shared__ __align__(16) u32 s_words[];
   __shared__ u32 s_cnt[kMaxParts];
@@ -132,17 +135,21 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_class_scatter(ClassLayout C
     return q < kClassSlots ? Split{id - q * (C.parts - 1), q} : Split{C.parts - 1, 0};  // beyond the bound: looked up again
   };
   __syncthreads();
-  u32 rank[kTilePer / 2];  // inside the tile's share of the class, two to a word
+  constexpr u32 kNoId = 0xFFFFFFFFu;
+  uint16_t* s_rank = reinterpret_cast<uint16_t*>(s_words + kClassTile) + tid;  // by item: its rank in the tile's share of the class
+  u32 ids[kTilePer];
+  i64 node[2][kAhead];
+  load(0, node[0]);
 #pragma unroll
   for (int q0 = 0; q0 < kTilePer; q0 += kAhead) {
-    i64 node[kAhead];
-    load(q0, node);
+    i64(&now)[kAhead] = node[q0 / kAhead % 2];
+    if (q0 + kAhead < kTilePer) load(q0 + kAhead, node[(q0 / kAhead + 1) % 2]);
 #pragma unroll
     for (int q = 0; q < kAhead; ++q) {
       u32 own = 0;
-      if (valid_id(node[q])) own = atomicAdd(&s_cnt[split((u32)node[q]).c], 1u);
-      if (q % 2 == 0) rank[(q0 + q) / 2] = own;
-      else rank[(q0 + q) / 2] |= own << 16;
+      ids[q0 + q] = valid_id(now[q]) ? (u32)now[q] : kNoId;
+      if (valid_id(now[q])) own = atomicAdd(&s_cnt[split((u32)now[q]).c], 1u);
+      s_rank[(q0 + q) * kTileThreads] = (uint16_t)own;
     }
   }
   __syncthreads();
@@ -170,24 +177,18 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_class_scatter(ClassLayout C
   }
   __syncthreads();
 #pragma unroll
-  for (int q0 = 0; q0 < kTilePer; q0 += kAhead) {
-    if (q0 * kTileThreads >= here) break;  // uniform
-    i64 node[kAhead];
-    load(q0, node);
-#pragma unroll
-    for (int q = 0; q < kAhead; ++q) {
-      const u32 i = (q0 + q) * kTileThreads + tid;
-      if (i >= here) break;
-      u32 to = kNoPlace;
-      if (valid_id(node[q])) {
-        const Split s = split((u32)node[q]);
-        to = s_cnt[s.c] + (rank[(q0 + q) / 2] >> 16 * (q % 2) & 0xFFFFu);
-        s_words[to] = s.quotient << kNumberBits | i;
-      } else {
-        raise_error(counters, GSB_ERR_INDEX_RANGE, (i64)first + i);
-      }
-      place[(q0 + q) * kTileThreads] = (uint16_t)to;
+  for (int q = 0; q < kTilePer; ++q) {
+    const u32 i = q * kTileThreads + tid;
+    if (i >= here) break;
+    u32 to = kNoPlace;
+    if (ids[q] != kNoId) {
+      const Split s = split(ids[q]);
+      to = s_cnt[s.c] + s_rank[q * kTileThreads];
+      s_words[to] = s.quotient << kNumberBits | i;
+    } else {
+      raise_error(counters, GSB_ERR_INDEX_RANGE, (i64)first + i);
     }
+    place[q * kTileThreads] = (uint16_t)to;
   }
   __syncthreads();
   uint4* out = reinterpret_cast<uint4*>(C.words + tile * kClassTile);
@@ -600,13 +601,13 @@ int class_unique_relabel(gsb_ctx* ctx, cudaStream_t stream, const BatchLayout& L
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     GSB_CUDA_OK(cudaFuncSetAttribute(k_class_resolve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClassSlots * 4));
     GSB_CUDA_OK(cudaFuncSetAttribute(k_class_resolve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClassSlots * 4));
-    GSB_CUDA_OK(cudaFuncSetAttribute(k_class_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kClassTile));
+    GSB_CUDA_OK(cudaFuncSetAttribute(k_class_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterBytes));
     GSB_CUDA_OK(cudaFuncSetAttribute(k_class_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kClassTile));
     attr_set[dev] = true;
   }
   {
     ScopedKernelTimer timer(ctx, KID_PART_SCATTER, stream);
-    k_class_scatter<<<(int)tiles, kTileThreads, 4 * kClassTile, stream>>>(C, counters);
+    k_class_scatter<<<(int)tiles, kTileThreads, kScatterBytes, stream>>>(C, counters);
   }
   GSB_LAUNCH_OK();
   {

@@ -48,14 +48,15 @@ UNIT = "edges/s"
 
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) divided by algorithmic bytes, from one ncu capture per
-# kernel on hop 3 of a 64-minibatch call of this workload (profiles/k_*_sage3hop_group64.md).  Traffic grows in
-# proportion to the units a launch processes, so a full launch's traffic is this ratio times its algorithmic bytes.
-TRAFFIC_OVER_ALGORITHMIC = {"sample_uniform": 4.2, "table_insert": 4.1, "first_compact": 3.2, "relabel": 1.04,
-                            # partitioned form (profiles/k_part_*_sage3hop_group64.md, k_rank_emit_sage3hop_group64.md)
-                            "partition_count": 1.04, "partition_scatter": 0.83, "bucket_resolve": 0.84,
-                            "first_bits": 0.81}
+# kernel on the last hop: a 50-minibatch call (sampling by windows, the relabel in class tiles:
+# profiles/kernels_of_the_measured_cases.md), or a 64-minibatch call for the forms that --relabel-path asks for
+# (profiles/k_*_sage3hop_group64.md).  Apart from sampling's, whose windows read the graph once per call whatever the
+# call's size, traffic grows in proportion to the units a launch processes.
+TRAFFIC_OVER_ALGORITHMIC = {"sample_uniform": 2.1, "table_insert": 4.1, "first_compact": 3.2, "relabel": 1.04,
+                            "partition_count": 1.04, "partition_scatter": 0.92, "bucket_resolve": 0.82,
+                            "first_bits": 0.89, "rank_emit": 1.09}
 # the same with direct-address tables (profiles/k_direct_insert_sage3hop_group64.md)
-TRAFFIC_OVER_ALGORITHMIC_DIRECT = {"sample_uniform": 4.2, "table_insert": 9.1}
+TRAFFIC_OVER_ALGORITHMIC_DIRECT = {"sample_uniform": 2.1, "table_insert": 9.1}
 
 
 def parse():
@@ -503,25 +504,25 @@ def run_ours(args):
         peak, peak_src = float(json.load(open(peaks_path))["hbm_gbs"]), "measured"
     else:
         peak, peak_src = 6650.0, "fallback"
-    # Algorithmic bytes per launch of each hot kernel, from the shapes of the profiled calls: (S, E, U) per hop.
-    # sample: 32 B per seed column (seed id, indptr pair, output offset) + 24 B per sampled edge (8 read, 16 written);
+    # Algorithmic bytes of each hot kernel over the profiled step, from the shapes of its calls: (S, E, U) per hop.
+    # sample: 32 B per seed column (seed id, indptr pair, output offset) + 24 B per sampled edge (8 read, 16 written),
+    # in one launch per hop or, by windows, three;
     # unique + relabel, hash-region / direct-table forms: three passes over N = S + E items: insert reads 8 N;
     # first-occurrence compaction reads 8 N and writes 8 U; relabel reads 8 E and writes 8 E (table traffic is overhead,
-    # not counted).  Partitioned form: count reads 8 N; scatter reads 8 N and writes 8 N; the per-bucket resolve reads
-    # 8 N and writes 4 N; the bit pass reads 4 N; the emit pass reads 4 N and the 8 U ids of the first occurrences and
-    # writes 8 U + 8 E.
+    # not counted).  By class tiles: scatter reads 8 N and writes 4 N words and 2 N places; resolve reads and writes 4 N;
+    # the bit pass reads 6 N and writes 4 N; the emit pass reads 4 N and the 8 U ids of the first occurrences and writes
+    # 8 U + 8 E.  (The partitioned form, which smaller hops take, moves 20 N, 12 N and 12 N in the first three.)
     hop_shapes = [h for call in shapes for h in call]
-    n_launch = max(1, len(hop_shapes))
     alg = {
-        "sample_uniform": sum(32 * s_ + 8 + 24 * e_ for s_, e_, _ in hop_shapes) / n_launch,
-        "table_insert": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
-        "first_compact": sum(8 * (s_ + e_) + 8 * u_ for s_, e_, u_ in hop_shapes) / n_launch,
-        "relabel": sum(16 * e_ for s_, e_, _ in hop_shapes) / n_launch,
-        "partition_count": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
-        "partition_scatter": sum(20 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
-        "bucket_resolve": sum(12 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
-        "first_bits": sum(12 * (s_ + e_) for s_, e_, _ in hop_shapes) / n_launch,
-        "rank_emit": sum(4 * (s_ + e_) + 16 * u_ + 8 * e_ for s_, e_, u_ in hop_shapes) / n_launch,
+        "sample_uniform": sum(32 * s_ + 8 + 24 * e_ for s_, e_, _ in hop_shapes),
+        "table_insert": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes),
+        "first_compact": sum(8 * (s_ + e_) + 8 * u_ for s_, e_, u_ in hop_shapes),
+        "relabel": sum(16 * e_ for s_, e_, _ in hop_shapes),
+        "partition_count": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes),
+        "partition_scatter": sum(14 * (s_ + e_) for s_, e_, _ in hop_shapes),
+        "bucket_resolve": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes),
+        "first_bits": sum(10 * (s_ + e_) for s_, e_, _ in hop_shapes),
+        "rank_emit": sum(4 * (s_ + e_) + 16 * u_ + 8 * e_ for s_, e_, u_ in hop_shapes),
     }
     # which form of unique + relabel ran is read off the kernels that were launched
     launched = {name for name, (ms, n) in prof.items() if n}
@@ -529,12 +530,12 @@ def run_ours(args):
     direct = form == "direct"
     form_text = {"partition": "shared-memory tables per bucket of items (partitioned form)",
                  "hash": "hash-table regions in global memory", "direct": "direct-address tables"}[form]
-    kernel_names = {"sample_uniform": "k_sample_uniform_tpc (fused count + scan + uniform sample)",
+    kernel_names = {"sample_uniform": "k_window_draw / read / emit, k_sample_uniform_tpc (fused count + scan + uniform sample)",
                     "partition_count": "k_part_count (items per bucket)",
-                    "partition_scatter": "k_part_scatter (items grouped by bucket)",
-                    "bucket_resolve": "k_part_resolve (first position per id in a shared-memory table per bucket)",
-                    "first_bits": "k_first_bits (bit vector of first occurrences)",
-                    "rank_emit": "k_rank_emit (frontier and relabelled ids from the rank bit vector)",
+                    "partition_scatter": "k_class_scatter, k_part_scatter (items grouped by class or bucket)",
+                    "bucket_resolve": "k_class_resolve, k_part_resolve (first position per id in a shared-memory table)",
+                    "first_bits": "k_class_bits, k_first_bits (bit vector of first occurrences)",
+                    "rank_emit": "k_class_emit, k_rank_emit (frontier and relabelled ids from the rank bit vector)",
                     "table_insert": "k_direct_insert (atomicMin into per-minibatch direct-address tables)" if direct
                     else "k_batch_insert (position-min hash insert)",
                     "first_compact": "k_direct_compact (first-occurrence test + scan + compaction)" if direct
@@ -547,19 +548,20 @@ def run_ours(args):
         if name in alg and n:
             avg_s = ms / 1e3 / n
             entry["avg_launch_us"] = round(avg_s * 1e6, 2)
-            entry["bytes_per_launch"] = round(alg[name])
-            entry["achieved_gbs"] = round(alg[name] / avg_s / 1e9, 2)
-            entry["frac"] = round(alg[name] / avg_s / 1e9 / peak, 5)
+            per_launch = alg[name] / n
+            entry["bytes_per_launch"] = round(per_launch)
+            entry["achieved_gbs"] = round(per_launch / avg_s / 1e9, 2)
+            entry["frac"] = round(per_launch / avg_s / 1e9 / peak, 5)
             ratio = (TRAFFIC_OVER_ALGORITHMIC_DIRECT if direct else TRAFFIC_OVER_ALGORITHMIC).get(name)
             if ratio is not None:
-                entry["traffic"] = round(alg[name] * ratio)
+                entry["traffic"] = round(per_launch * ratio)
         per_kernel[name] = entry
     top = max((k for k in per_kernel if k in alg), key=lambda k: per_kernel[k]["ms"], default=None)
     if top is not None:
         t = per_kernel[top]
         roofline = {"bound": "hbm", "kernel": kernel_names[top], "achieved": t["achieved_gbs"], "peak": peak,
                     "peak_source": peak_src, "unit": "GB/s", "frac": t["frac"], "traffic": t.get("traffic"),
-                    "traffic_source": "ncu capture of one launch on a 64-minibatch call, scaled by algorithmic bytes",
+                    "traffic_source": "ncu captures of launches on a smaller call, scaled by algorithmic bytes",
                     "bytes_per_launch": t["bytes_per_launch"], "avg_launch_us": t["avg_launch_us"],
                     "share_of_device_time": t["share"],
                     "measured": "CUDA events around every launch of one untimed step", "kernels": per_kernel}

@@ -547,14 +547,14 @@ static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // us of a whole call, hashed buckets / the partitioned form with classes / this (ids scattered evenly; in brackets: by a power law
 // numbered by degree), by nodes and items of a minibatch:
-//   40 M items, 2.45 M nodes    76 000 974 / 1187 / 954 (998 / 1189 / 1023)    106 400 973 / 1045 / 821 (978 / 1046 / 878)
-//                               243 200 960 / 845 / 665 (967 / 848 / 692)      760 000 943 / 740 / 572 (1022 / 757 / 602)
-//               1 M nodes       34 000 1005 / 1214 / 1114 (965 / 1216 / 1187)  47 600 969 / 1045 / 910 (1059 / 1049 / 966)
-//                               108 800 949 / 840 / 700 (958 / 845 / 730)      340 000 934 / 736 / 587 (974 / 743 / 629)
-//               700 000         30 800 1008 / 1080 / 949 (969 / 1082 / 1006)   70 400 953 / 843 / 738 (963 / 847 / 783)
-//               500 000         38 400 986 / 919 / 831 (1017 / 923 / 989)      51 200 951 / 825 / 764 (961 / 830 / 882)
-//               180 000         19 200 1018 / 910 / 1402                       60 000 934 / 762 / 957
-//   1.4 M items, 2.45 M nodes   136 800 92 / 87 / 76 (126 / 88 / 81)           760 000 (one) 74 / 59 / 67 (172 / 72 / 81)
+//   40 M items, 2.45 M nodes    76 000 959 / 1173 / 892 (977 / 1172 / 962)    106 400 960 / 1029 / 768 (962 / 1032 / 825)
+//                               243 200 945 / 828 / 617 (950 / 830 / 643)      760 000 929 / 730 / 526 (999 / 740 / 562)
+//               1 M nodes       34 000 992 / 1196 / 1034 (951 / 1198 / 1106)   47 600 958 / 1033 / 843 (1044 / 1033 / 899)
+//                               108 800 934 / 827 / 643 (941 / 827 / 673)      340 000 916 / 721 / 539 (952 / 727 / 582)
+//               700 000         30 800 992 / 1063 / 869 (955 / 1067 / 930)     70 400 938 / 826 / 674 (941 / 829 / 719)
+//               500 000         38 400 970 / 900 / 756 (994 / 902 / 913)       51 200 936 / 811 / 697 (942 / 812 / 815)
+//               180 000         19 200 996 / 888 / 1291 (943 / 883 / 1420)     60 000 916 / 746 / 893 (929 / 750 / 1004)
+//   1.4 M items, 2.45 M nodes   136 800 91 / 86 / 67 (129 / 89 / 72)           760 000 (one) 73 / 60 / 58 (171 / 73 / 71)
 // With few classes a tile's run is longer than the pieces it is cut into; with few tiles SMs are left idle.
 bool class_tiled(i64 path, i64 num_nodes, i64 items, i64 G) {
   const i64 parts = path == 0 || path == 5 ? partition_class_parts(num_nodes, items / G, true) : 0;

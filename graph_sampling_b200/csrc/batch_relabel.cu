@@ -787,10 +787,12 @@ static int sage_hop_sampler_counts(gsb_ctx* ctx, cudaStream_t stream, const i64*
   // the sampler's scratch lies where the passes after it keep theirs, behind the counts that it leaves them
   const size_t bytes = 2 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap);
   const size_t behind = 2 * off_bytes + partition_count_bytes(bucket_cap);
+  const bool windows_suit = window_sample_suits(ctx, S, k, num_edges);
+  const size_t with_windows = windows_suit ? behind + window_sample_bytes(ctx, S, k, num_edges) : 0;
   void* ws;
-  bool windows = window_sample_suits(ctx, S, k, num_edges) &&
-                 ctx_try_workspace(ctx, stream, max(bytes, behind + window_sample_bytes(ctx, S, k, num_edges)), &ws);
-  int st = windows ? GSB_OK : ctx_reserve_workspace(ctx, stream, bytes, &ws);
+  bool windows = windows_suit;
+  if (with_windows > bytes) windows = ctx_try_workspace(ctx, stream, with_windows, bytes, &ws);
+  int st = windows && with_windows > bytes ? GSB_OK : ctx_reserve_workspace(ctx, stream, bytes, &ws);
   if (st != GSB_OK) return st;
   void* part_ws = (char*)ws + 2 * off_bytes;
   BatchLayout L;

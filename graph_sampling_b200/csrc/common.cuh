@@ -109,9 +109,11 @@ constexpr u64 kMailValueMask = (1ull << kMailErrorBit) - 1;
 // Scratch of the call that is about to queue work on `stream`.  It is the same memory for every call, which is why they are
 // ordered on one stream; a call on another stream than the last one's waits here until the device is done with that.
 int ctx_reserve_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, void** out);
-// The same for scratch that a call can do without: false, and nothing is left of the attempt, when it cannot be had (out of memory,
-// or it would have to grow while `stream` is captured).
-bool ctx_try_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, void** out);
+// The same for scratch that a call can do without: false, and the scratch of before is still there, when it would have to grow
+// and cannot (out of memory, `stream` is captured), or when what it takes beyond the `needed` bytes (<= bytes) that the call has
+// to have anyway is more than an eighth of the memory left beside those: what grows here stays with the context, and the
+// caller's own allocations come after it.  It grows to `bytes`, not to a quarter more.
+bool ctx_try_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, size_t needed, void** out);
 int ctx_tile_state(gsb_ctx* ctx, i64 num_tiles, cudaStream_t stream, TileState* out);
 // Offsets of a per-column result by the counting kernel alone (defined in slice_sample.cu): mode 0 = degrees,
 // 1 = min(degree, k), 2 = k per non-empty column.  The total is left in the context's counters.

@@ -15,6 +15,8 @@ struct gsb_ctx {
   int device;
   void* workspace;
   size_t workspace_bytes;
+  size_t refused_bytes;  // scratch that ctx_try_workspace could not have last time, 0: none
+  i64 refused_calls;
   u64* tile_words;
   i64 tile_capacity;
   uint32_t epoch;
@@ -88,19 +90,37 @@ int ctx_reserve_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, void*
   return GSB_OK;
 }
 
-bool ctx_try_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, void** out) {
+// Asking for the free memory takes 0.1 to 0.4 ms: a size that was refused is asked for again by every 64th call that wants it.
+constexpr i64 kRefusedCalls = 64;
+
+bool ctx_try_workspace(gsb_ctx* ctx, cudaStream_t stream, size_t bytes, size_t needed, void** out) {
+  if (ctx_on_stream(ctx, stream) != GSB_OK) return false;
   if (bytes > ctx->workspace_bytes) {
+    bytes = (bytes + 255) & ~(size_t)255;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+    if (ctx->refused_bytes != 0 && bytes >= ctx->refused_bytes && ++ctx->refused_calls % kRefusedCalls != 0) return false;
     size_t room = 0, total = 0;
-    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
-        cudaMemGetInfo(&room, &total) != cudaSuccess || bytes > room + ctx->workspace_bytes) {
+    void* grown = nullptr;
+    bool fits = cudaMemGetInfo(&room, &total) == cudaSuccess;
+    const size_t kept = room + ctx->workspace_bytes;  // what there is for the scratch: growth gives the present one back
+    fits = fits && kept >= needed && bytes - needed <= (kept - needed) / 8;
+    // the new scratch is there before the old one goes: an attempt that fails leaves everything as it was
+    if (!fits || cudaMalloc(&grown, bytes) != cudaSuccess) {
       (void)cudaGetLastError();
+      ctx->refused_bytes = bytes;
       return false;
     }
+    ctx->refused_bytes = 0;
+    if (cudaDeviceSynchronize() != cudaSuccess || (ctx->workspace && cudaFree(ctx->workspace) != cudaSuccess)) {
+      (void)cudaFree(grown);
+      return false;
+    }
+    ctx->workspace = grown;
+    ctx->workspace_bytes = bytes;
   }
-  if (ctx_reserve_workspace(ctx, stream, bytes, out) == GSB_OK) return true;
-  (void)cudaGetLastError();
-  return false;
+  *out = ctx->workspace;
+  return true;
 }
 
 int ctx_tile_state(gsb_ctx* ctx, i64 num_tiles, cudaStream_t stream, TileState* out) {

@@ -544,7 +544,7 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
   }
   if (out_select && !out_coo_col && !out_data && window_sample_suits(ctx, S, k, num_edges)) {
     void* ws = count ? count->scratch : nullptr;
-    if (!ws && !ctx_try_workspace(ctx, stream, window_sample_bytes(ctx, S, k, num_edges), &ws)) ws = nullptr;
+    if (!ws && !ctx_try_workspace(ctx, stream, window_sample_bytes(ctx, S, k, num_edges), 0, &ws)) ws = nullptr;
     if (ws) return window_sample_launch(ctx, stream, p, num_edges, ws);
   }
   {

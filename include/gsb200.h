@@ -199,7 +199,8 @@ GSB_API int gsb_sample_uniform(gsb_ctx* ctx, void* stream, const int64_t* indptr
                                const float* data, const int64_t* e_ids, float* out_data, int64_t capacity,
                                int64_t* nnz_host);
 /* The same for a caller that knows the number of entries of `indices` (num_edges; 0: not known, or not in device memory): a call
- * that reads a large graph many times over then reads it in windows that L2 holds, with scratch of about 4 * S * k bytes. */
+ * that reads a large graph many times over then reads it in windows that L2 holds, with scratch of about 4 * S * k bytes that
+ * the context keeps, unless that is more than an eighth of the free memory: then, as without num_edges, in one pass. */
 GSB_API int gsb_sample_uniform_sized(gsb_ctx* ctx, void* stream, const int64_t* indptr, const int64_t* indices,
                                      int64_t num_cols, int64_t num_edges, const int64_t* seeds, int64_t S, int64_t k,
                                      int replace, uint64_t seed, int64_t* out_indptr, int64_t* out_indices,

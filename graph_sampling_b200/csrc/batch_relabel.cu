@@ -707,12 +707,20 @@ static int relabel_batches(gsb_ctx* ctx, cudaStream_t stream, BatchLayout L, i64
   }
   if (path >= 3 || (path == 0 && partition_suits(n_cap, G))) {
     // partitioned form (the default for large calls when the direct-address tables above were not chosen): shared-memory tables per bucket of items, then ranking by bit vectors
-    const bool tiled = class_tiled(path, num_nodes, n_cap, G);
-    const i64 parts = path == 3 ? 0 : partition_class_parts(num_nodes, n_cap / G, tiled || path >= 4);
+    i64 parts = path == 3 ? 0 : partition_class_parts(num_nodes, n_cap / G, path >= 4);
     const i64 bucket_cap = partition_bucket_capacity(n_cap, G, parts);
-    const size_t bytes = tiled ? class_workspace_bytes(n_cap, G, parts) : partition_workspace_bytes(n_cap, bucket_cap);
-    int st = ctx_reserve_workspace(ctx, stream, 3 * off_bytes + bytes, &ws);
-    if (st != GSB_OK) return st;
+    const size_t bytes = 3 * off_bytes + partition_workspace_bytes(n_cap, bucket_cap);
+    // minibatches that fill their tiles badly take more in tiles (38 bytes an item instead of 33 at 36 000 items): the buckets
+    // where that cannot be had
+    bool tiled = class_tiled(path, num_nodes, n_cap, G);
+    const i64 tiled_parts = tiled ? partition_class_parts(num_nodes, n_cap / G, true) : 0;
+    const size_t tiled_bytes = tiled ? 3 * off_bytes + class_workspace_bytes(n_cap, G, tiled_parts) : 0;
+    if (tiled_bytes > bytes) tiled = ctx_try_workspace(ctx, stream, tiled_bytes, bytes, &ws);
+    if (!tiled || tiled_bytes <= bytes) {
+      int st = ctx_reserve_workspace(ctx, stream, tiled ? tiled_bytes : bytes, &ws);
+      if (st != GSB_OK) return st;
+    }
+    if (tiled) parts = tiled_parts;
     L.item_off = (i64*)ws;
     L.region_off = (i64*)((char*)ws + off_bytes);
     L.slots = nullptr;

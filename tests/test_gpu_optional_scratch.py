@@ -57,3 +57,27 @@ def test_windows_leave_the_memory_to_the_caller():
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     assert free - torch.cuda.mem_get_info()[0] <= S * (4 * k + 3) + 4 * MB
+
+
+def test_class_tiles_step_back():
+    from graph_sampling_b200 import ops
+    rng = np.random.default_rng(5)
+    G, nodes = 2000, 200_000                  # 16.4 M items in half-filled tiles: 1.3 GB of scratch, 0.54 in buckets
+    sp, ep = np.arange(G + 1) * 1000, np.arange(G + 1) * 7200
+    dev = [torch.from_numpy(a).cuda() for a in (rng.integers(0, nodes, sp[-1]), sp, rng.integers(0, nodes, ep[-1]), ep)]
+
+    def call(ctx, path):
+        ctx.set_option("relabel_path", path)
+        before = ctx.launch_count()
+        got = ops.batch_csr_relabel(*dev, num_nodes=nodes, ctx=ctx)[:3]
+        return got, ctx.launch_count() - before
+
+    want, in_buckets = call(ops.Context(), 4)
+    want = [t.cpu() for t in want]
+    ctx = ops.Context()
+    with Filled(1250 * MB):
+        got, launches = call(ctx, 5)
+        assert launches == in_buckets and all(torch.equal(a.cpu(), b) for a, b in zip(got, want))
+        del got
+    got, launches = [call(ctx, 5) for _ in range(64)][-1]
+    assert launches < in_buckets and all(torch.equal(a.cpu(), b) for a, b in zip(got, want))

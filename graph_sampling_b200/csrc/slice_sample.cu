@@ -432,8 +432,9 @@ __global__ void __launch_bounds__(kTpcThreads) k_sample_uniform_tpc(SampleParams
   }
   if (COUNT) {
     // a call whose device-side sizes exceed the caller's bounds was flagged by the layout kernel: its bucket layout
-    // may not fit the count array, so nothing is counted (the passes that would use the counts return at once)
-    if (!overflow && p.counters[CNT_ABORT] == 0) {  // uniform in the warp
+    // may not fit the count array, so nothing is counted (the passes that would use the counts return at once).  A look-back that is
+    // given up elsewhere sets the flag at any time: the warp decides as one, what follows needs all its lanes.
+    if (__all_sync(0xffffffffu, !overflow && p.counters[CNT_ABORT] == 0)) {
       const i64 b0 = valid ? __ldg(p.bucket_base + bt) : 0;
       const int win = (int)(b0 - s_win0);  // >= 0: minibatches follow the CTA's first one
       const uint32_t parts = valid ? (uint32_t)(__ldg(p.bucket_base + bt + 1) - b0) : 0;

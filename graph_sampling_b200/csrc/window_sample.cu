@@ -288,41 +288,35 @@ static int window_shift(gsb_ctx* ctx, i64 num_edges) {
 }
 static i64 window_count(gsb_ctx* ctx, i64 num_edges) { return ((num_edges - 1) >> window_shift(ctx, num_edges)) + 1; }
 
-// Windows / one pass, the time of a whole call as a ratio, columns met by popularity, 24 | 50 edges a column on average, by edges, picks
-// a column and picks per edge:
-//                   1 pick          5 picks         6 picks         8 picks         10 picks        15 picks        16 picks
-//   17 M   1        0.76 | 0.76     0.98 | 0.95     1.08 | 1.05     1.19 | 1.27     1.17 | 1.13     1.31 | 1.17     1.41 | 1.36
-//          4        0.74 | 0.74     0.92 | 0.91     1.04 | 1.02     1.17 | 1.24     1.11 | 1.06     1.23 | 1.13     1.33 | 1.34
-//   33 M   1                        0.98 | 0.93     1.08 | 1.01                     1.09 | 0.99
-//          4                        0.92 | 0.87     1.01 | 0.95                     1.00 | 0.91
-//   34 M   0.25                     1.01 | 0.97     1.11 | 1.06                     1.23 | 1.14
-//          1                        0.84 | 0.81     0.97 | 0.91                     1.02 | 0.94
-//   60 M   0.25     0.96 | 0.98     0.99 | 0.93     1.08 | 1.01     1.17 | 1.16     1.13 | 1.01     1.25 | 1.14     1.39 | 1.38
-//          1        0.92 | 0.93     0.86 | 0.80     0.96 | 0.88     1.03 | 1.02     0.97 | 0.87     1.08 | 0.95     1.21 | 1.18
-//   122 M  0.06     1.02 | 1.03     1.11 | 1.10     1.20 | 1.18     1.32 | 1.34     1.30 | 1.22     1.46 | 1.33     1.54 | 1.55
-//          0.25     0.96 | 0.97     0.90 | 0.84     0.99 | 0.92     1.05 | 1.05     1.02 | 0.93     1.13 | 1.02     1.28 | 1.27
-//          1        0.92 | 0.93     0.79 | 0.73     0.88 | 0.81     0.94 | 0.94     0.88 | 0.80     1.00 | 0.89     1.13 | 1.11
-//   400 M  0.06     0.94 | 0.93     1.01 | 0.97     1.12 | 1.07     1.20 | 1.24     1.21 | 1.13     1.29 | 1.22     1.44 | 1.46
-//          0.25     0.95 | 0.94     0.83 | 0.76     0.91 | 0.85     0.98 | 0.99     0.96 | 0.87     1.06 | 0.97     1.20 | 1.21
-// (5 picks at 1 per edge in us, windows / one pass: 17 M 207 / 216, 60 M 754 / 938, 122 M 1540 / 2104.)  Up to four windows hardly ever
-// pay with more than five picks: most of one pass comes out of L2 or finds a column's picks in few lines.  The more picks, the more
-// columns it takes before a window's lines are met often enough: with more than five a bound on the columns fits better than one on
-// the picks.  Eight, twelve and sixteen picks lie in the same shared-memory banks column after column, 12 and more leave few CTAs per
-// SM.  From 20 to 33 M edges windows with 6 to 11 picks are as good as one pass from about 3.4 picks per edge on (0.85 to 1.07 of
-// its time, graphs of 20 M edges up to 1.12).  Where all columns have the same chance one pass gains more from columns that are read
-// whole, and windows take 0.91 to 1.15 of its time with 5 picks, 1.1 to 1.3 with 10 and up to 1.48 with 8 and 12.  Frontiers of super-batches lie between the two (10 picks, 31 M edges, 300 minibatches:
-// 1.12 | 1.01 at 1.2 | 1.4 per edge; 60 M 1.02 | 0.89 at 0.7 | 1.1).  S may be a bound on the columns, which is all that the host knows.
+// Windows / one pass, time of a call, the columns being the frontiers of 500 minibatches of 1 024 seeds after a hop of 15 (3 M columns
+// out of an R-MAT graph with 50 edges a column | 6 M, power-law degrees, 24 edges | 7 M, 50 edges), by edges and picks a column:
+//             2 picks         5 picks         6 picks         8 picks         10 picks        12 picks        15 picks        16 picks
+//   17 M      0.90|0.87|0.86  0.96|0.96|0.94  0.99|1.07|1.05  1.05|1.19|1.27  0.96|1.15|1.10  0.99|1.16|1.18  1.03|1.26|1.17  1.14|1.32|1.34
+//   20 M      0.94|0.91|0.90  0.95|0.97|0.94  0.97|1.08|1.03  1.03|1.18|1.24  0.92|1.13|1.06  0.95|1.16|1.12  0.98|1.24|1.14  1.11|1.32|1.32
+//   25 M      1.01|0.96|0.96  0.93|0.98|0.93  0.95|1.08|1.02  0.98|1.18|1.21  0.87|1.10|1.01  0.89|1.15|1.08  0.91|1.22|1.09  1.06|1.31|1.31
+//   31 M      1.10|1.04|1.04  0.92|1.00|0.94  0.94|1.10|1.02  0.95|1.17|1.18  0.84|1.09|0.97  0.85|1.13|1.08  0.86|1.18|1.06  1.01|1.29|1.28
+//   40 M      0.97|0.91|0.91  0.83|0.88|0.81  0.86|0.98|0.90  0.86|1.06|1.07  0.77|1.01|0.91  0.80|1.08|1.01  0.81|1.13|1.00  0.97|1.24|1.24
+//   60 M      1.09|1.03|1.02  0.85|0.92|0.85  0.87|1.00|0.91  0.86|1.07|1.04  0.76|1.00|0.88  0.79|1.10|1.01  0.77|1.10|0.96  0.92|1.21|1.20
+//   124 M     1.11|1.05|0.95  0.88|0.92|0.78  0.90|0.99|0.84  0.88|1.03|0.97  0.78|0.98|0.82  0.82|1.09|0.95  0.77|1.06|0.90  0.90|1.18|1.16
+// 250 and 100 minibatches (half and a fifth of the columns) at 124 M edges: 5 picks 1.02|1.01|0.92 and -|1.16|1.10, 10 picks 0.94|1.06|0.92
+// and 1.18|1.27|1.12; 10 picks at 31 M 0.89|1.14|1.02 and 1.08|1.25|1.08.
+// What windows save depends on how often a window's lines are met, which the rule has the picks for, and on how the columns lie, which
+// it doesn't know: it stands where the two kinds of graphs lose about the same (2 % on average of the better form, up to 1.35 before for
+// calls that stayed in one pass).  Up to four windows one pass comes out of L2 for the most part, and the smaller the graph the more
+// picks it takes; a step of 15 % lies between four windows and five.  8, 12 and 16 picks a column lie in the same banks of shared
+// memory column after column, and more than 10 leave fewer CTAs an SM.  Columns that all have the same chance are read whole more
+// often and gain least (10 picks 1.1 to 1.4): first hops, which have few picks.  S may be a bound on the columns, which is all that the
+// host knows.
 bool window_sample_suits(gsb_ctx* ctx, i64 S, i64 k, i64 num_edges) {
   const i64 path = ctx_option(ctx, GSB_OPT_SAMPLE_PATH);
   if (k < 1 || k > 16 || num_edges < 1 || path == 1 || num_edges > ((i64)kMaxWindows << kWindowShift)) return false;
   if (path == 2) return true;
   if (num_edges < (16 << 20) || k == 16) return false;
   const i64 picks = S * k;
-  const bool few = num_edges <= ((i64)4 << kWindowShift);
+  const bool few = num_edges <= ((i64)4 << kWindowShift), wide = k == 8 || k >= 12;
   if (k <= 5) return picks >= (few ? num_edges : max((i64)12'000'000, num_edges * max(k, (i64)4) / 64));
-  const bool wide = k == 8 || k >= 12;
-  if (few) return !wide && num_edges >= 20'000'000 && 8 * picks >= 27 * num_edges;
-  return S >= max((i64)4'000'000, num_edges / 50) * (wide ? 2 : 1);
+  if (few) return !wide && num_edges >= 20'000'000 && picks >= 127'500'000 - 3 * num_edges;
+  return picks >= max((i64)(wide ? 40'000'000 : 20'000'000), num_edges * k / 64);
 }
 
 static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }

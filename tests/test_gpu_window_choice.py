@@ -18,12 +18,12 @@ def graph(edges):
 
 @pytest.mark.parametrize("edges,k,columns,windows", [
     (31_000_000, 5, 6_199_000, False), (31_000_000, 5, 6_200_000, True),       # up to four windows: a pick per edge,
-    (31_000_000, 10, 6_200_000, False),                                        # with more picks more of them,
-    (31_000_000, 10, 10_462_000, False), (31_000_000, 10, 10_463_000, True),
+    (31_000_000, 10, 3_449_000, False), (31_000_000, 10, 3_450_000, True),     # with more picks by the edges,
+    (19_000_000, 10, 16_000_000, False),
     (31_000_000, 8, 15_500_000, False), (31_000_000, 12, 12_000_000, False),   # and never with so many
     (34_000_000, 5, 2_399_000, False), (34_000_000, 5, 2_400_000, True),       # five windows
-    (34_000_000, 10, 3_999_000, False), (34_000_000, 10, 4_000_000, True),
-    (34_000_000, 8, 7_999_000, False), (34_000_000, 8, 8_000_000, True),
+    (34_000_000, 10, 1_999_000, False), (34_000_000, 10, 2_000_000, True),
+    (34_000_000, 8, 4_999_000, False), (34_000_000, 8, 5_000_000, True),
     (34_000_000, 16, 8_500_000, False)])
 def test_lines_of_the_rule(edges, k, columns, windows):
     from graph_sampling_b200 import ops

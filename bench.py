@@ -47,16 +47,37 @@ METRIC = "sampled_edges_per_second"
 UNIT = "edges/s"
 
 
-# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) divided by algorithmic bytes, from one ncu capture per
-# kernel on the last hop: a 50-minibatch call (sampling by windows, the relabel in class tiles:
-# profiles/kernels_of_the_measured_cases.md), or a 64-minibatch call for the forms that --relabel-path asks for
-# (profiles/k_*_sage3hop_group64.md).  Apart from sampling's, whose windows read the graph once per call whatever the
-# call's size, traffic grows in proportion to the units a launch processes.
-TRAFFIC_OVER_ALGORITHMIC = {"sample_uniform": 2.1, "table_insert": 4.1, "first_compact": 3.2, "relabel": 1.04,
-                            "partition_count": 1.04, "partition_scatter": 0.92, "bucket_resolve": 0.82,
-                            "first_bits": 0.89, "rank_emit": 1.09}
-# the same with direct-address tables (profiles/k_direct_insert_sage3hop_group64.md)
-TRAFFIC_OVER_ALGORITHMIC_DIRECT = {"sample_uniform": 2.1, "table_insert": 9.1}
+# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) divided by algorithmic bytes, from ncu.  The class tiles: last hop of
+# a 500-minibatch call (profiles/kernels_of_the_measured_cases.md).  The forms that --relabel-path asks for: last hop of a 64-minibatch
+# call (profiles/k_*_sage3hop_group64.md); their traffic grows in proportion to the units a launch processes.
+TRAFFIC_OVER_ALGORITHMIC = {"table_insert": 4.1, "first_compact": 3.2, "relabel": 1.04, "partition_count": 1.04,
+                            "partition_scatter": 0.83, "bucket_resolve": 0.84, "first_bits": 0.81}
+TRAFFIC_OVER_ALGORITHMIC_TILES = {"partition_scatter": 0.99, "bucket_resolve": 0.99, "first_bits": 1.00, "rank_emit": 1.15}
+# direct-address tables (profiles/k_direct_insert_sage3hop_group64.md)
+TRAFFIC_OVER_ALGORITHMIC_DIRECT = {"table_insert": 9.1}
+# A hop sampled by windows reads what the graph has of them, whatever its size: bytes per edge of the graph, per column and per pick.
+# Fits captures of 6.8, 27.1 and 67.7 M columns of five picks and 7.8 M of ten (2.14, 6.86, 16.30, 3.92 GB) within 1 %.
+WINDOW_TRAFFIC = (4.6, 37, 39)
+# The first hop in one pass, 512 000 columns that all have the same chance.  Later hops in one pass meet popular columns and scatter
+# their reads over more lines the fewer they are (4 to 6 times the algorithmic bytes): no figure is given for those.
+FIRST_HOP_TRAFFIC = 1.5
+
+
+def in_class_tiles(nodes, items, minibatches):
+    """Whether unique + relabel takes class tiles by itself, far enough from the line (class_tiled in csrc/class_relabel.cu)."""
+    classes, each = -(-nodes // 16_384) + 1, items // max(1, minibatches)
+    return 40 <= classes <= 256 and each >= max(700 * classes, 36_000) and (items >= 4_000_000 or each < 1600 * classes)
+
+
+def sampling_traffic(shapes, launches, edges):
+    """DRAM bytes of sampling (columns, picks, _) hop by hop, call by call, with so many launches in all: three launches are a hop by
+    windows.  None unless those are all hops but the first of every call."""
+    hops = sum(len(call) for call in shapes)
+    if launches != hops + 2 * (hops - len(shapes)):
+        return None
+    per_edge, per_column, per_pick = WINDOW_TRAFFIC
+    return sum(FIRST_HOP_TRAFFIC * (32 * s + 24 * e) if hop == 0 else per_edge * edges + per_column * s + per_pick * e
+               for call in shapes for hop, (s, e, _) in enumerate(call))
 
 
 def parse():
@@ -509,21 +530,27 @@ def run_ours(args):
     # in one launch per hop or, by windows, three;
     # unique + relabel, hash-region / direct-table forms: three passes over N = S + E items: insert reads 8 N;
     # first-occurrence compaction reads 8 N and writes 8 U; relabel reads 8 E and writes 8 E (table traffic is overhead,
-    # not counted).  By class tiles: scatter reads 8 N and writes 4 N words and 2 N places; resolve reads and writes 4 N;
-    # the bit pass reads 6 N and writes 4 N; the emit pass reads 4 N and the 8 U ids of the first occurrences and writes
-    # 8 U + 8 E.  (The partitioned form, which smaller hops take, moves 20 N, 12 N and 12 N in the first three.)
+    # not counted).  Partitioned form: count reads 8 N; scatter reads 8 N, writes 8 N and 4 N; the resolve reads 8 N and
+    # writes 4 N; the bit pass reads 4 N and 4 N and writes 4 N; the emit pass reads 4 N and the 8 U ids of the first
+    # occurrences and writes 8 U + 8 E.  In class tiles the scatter reads 8 N and writes 4 N words and 2 N places, the
+    # resolve reads and writes 4 N, the bit pass reads 6 N and writes 4 N.
     hop_shapes = [h for call in shapes for h in call]
+    sizes_of_calls = [min(group, batches.shape[0] - first) for first in firsts]
+    by_itself = args.relabel_path in (None, "auto")
+    tiles = [by_itself and in_class_tiles(indptr.numel() - 1, s_ + e_, g) for call, g in zip(shapes, sizes_of_calls)
+             for s_, e_, _ in call]
     alg = {
         "sample_uniform": sum(32 * s_ + 8 + 24 * e_ for s_, e_, _ in hop_shapes),
         "table_insert": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes),
         "first_compact": sum(8 * (s_ + e_) + 8 * u_ for s_, e_, u_ in hop_shapes),
         "relabel": sum(16 * e_ for s_, e_, _ in hop_shapes),
         "partition_count": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes),
-        "partition_scatter": sum(14 * (s_ + e_) for s_, e_, _ in hop_shapes),
-        "bucket_resolve": sum(8 * (s_ + e_) for s_, e_, _ in hop_shapes),
-        "first_bits": sum(10 * (s_ + e_) for s_, e_, _ in hop_shapes),
+        "partition_scatter": sum((14 if t else 20) * (s_ + e_) for (s_, e_, _), t in zip(hop_shapes, tiles)),
+        "bucket_resolve": sum((8 if t else 12) * (s_ + e_) for (s_, e_, _), t in zip(hop_shapes, tiles)),
+        "first_bits": sum((10 if t else 12) * (s_ + e_) for (s_, e_, _), t in zip(hop_shapes, tiles)),
         "rank_emit": sum(4 * (s_ + e_) + 16 * u_ + 8 * e_ for s_, e_, u_ in hop_shapes),
     }
+    traffic = {"sample_uniform": sampling_traffic(shapes, prof["sample_uniform"][1], indices.numel())}
     # which form of unique + relabel ran is read off the kernels that were launched
     launched = {name for name, (ms, n) in prof.items() if n}
     form = "partition" if "bucket_resolve" in launched else "hash" if "table_clear" in launched else "direct"
@@ -553,7 +580,11 @@ def run_ours(args):
             entry["achieved_gbs"] = round(per_launch / avg_s / 1e9, 2)
             entry["frac"] = round(per_launch / avg_s / 1e9 / peak, 5)
             ratio = (TRAFFIC_OVER_ALGORITHMIC_DIRECT if direct else TRAFFIC_OVER_ALGORITHMIC).get(name)
-            if ratio is not None:
+            if any(tiles):  # the hops in tiles have nearly all of the bytes
+                ratio = TRAFFIC_OVER_ALGORITHMIC_TILES.get(name, ratio)
+            if traffic.get(name) is not None:
+                entry["traffic"] = round(traffic[name] / n)
+            elif ratio is not None:
                 entry["traffic"] = round(per_launch * ratio)
         per_kernel[name] = entry
     top = max((k for k in per_kernel if k in alg), key=lambda k: per_kernel[k]["ms"], default=None)
@@ -561,7 +592,8 @@ def run_ours(args):
         t = per_kernel[top]
         roofline = {"bound": "hbm", "kernel": kernel_names[top], "achieved": t["achieved_gbs"], "peak": peak,
                     "peak_source": peak_src, "unit": "GB/s", "frac": t["frac"], "traffic": t.get("traffic"),
-                    "traffic_source": "ncu captures of launches on a smaller call, scaled by algorithmic bytes",
+                    "traffic_source": "ncu captures: sampling by windows as bytes per graph edge, column and pick, the rest "
+                                      "scaled by algorithmic bytes; null where nothing like it was captured",
                     "bytes_per_launch": t["bytes_per_launch"], "avg_launch_us": t["avg_launch_us"],
                     "share_of_device_time": t["share"],
                     "measured": "CUDA events around every launch of one untimed step", "kernels": per_kernel}

@@ -1,4 +1,4 @@
-// Batched unique + relabel by classes of ids (see k_part_resolve_classes), for minibatches of a hundred thousand items and more.
+// Batched unique + relabel by classes of ids (see k_part_resolve_classes), for minibatches of 36 000 items and more.
 //
 // An item is the quotient of its id and its number in a tile of 16 384 items of one minibatch: one 32-bit word, half of what the
 // partitioned form moves.  A tile sorts its own stretch by class, so nothing is counted before and nothing reserved across tiles:
@@ -555,7 +555,10 @@ static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 //               500 000         38 400 970 / 900 / 756 (994 / 902 / 913)       51 200 936 / 811 / 697 (942 / 812 / 815)
 //               180 000         19 200 996 / 888 / 1291 (943 / 883 / 1420)     60 000 916 / 746 / 893 (929 / 750 / 1004)
 //   1.4 M items, 2.45 M nodes   136 800 91 / 86 / 67 (129 / 89 / 72)           760 000 (one) 73 / 60 / 58 (171 / 73 / 71)
-// With few classes a tile's run is longer than the pieces it is cut into; with few tiles SMs are left idle.
+// With few classes a tile's run is longer than the pieces it is cut into; with few tiles SMs are left idle.  Few large minibatches gain
+// or lose by how their ids crowd, partitioned with classes / this, evenly and (as fourth powers): 700 000 nodes, 4.1 M items in 6
+// 121 / 97 (134 / 152), 8 M in 8 194 / 184 (218 / 261), in 24 189 / 154 (197 / 180); 2.45 M nodes, 4.1 M in 2 113 / 110 (142 / 158), in 4
+// 118 / 86 (131 / 113).
 bool class_tiled(i64 path, i64 num_nodes, i64 items, i64 G) {
   const i64 parts = path == 0 || path == 5 ? partition_class_parts(num_nodes, items / G, true) : 0;
   if (parts <= 0 || parts > kMaxParts || G > items / (kClassTile / 2) + 4096) return false;

@@ -72,8 +72,9 @@ __device__ __forceinline__ i64 tile_exclusive_prefix(const TileState& ts, int ti
 
 // Groups of 32 predecessors that a look-back reads at a time, nearest first.  While nobody has an inclusive prefix yet a tile can
 // only add up what it reads, and with n words read per step the first n k^2 / 2 tiles are done after k steps: the last of 4 219
-// tiles (135 000 sampled columns) after eight round trips to L2, with one group after sixteen (27.9 -> 25.8 us for the sampler);
-// with eight and sixteen groups the reads themselves get in the way (28.5, 32.5).
+// tiles (135 000 sampled columns) after eight round trips to L2, with one group after sixteen (24.3 -> 22.6 us for the sampler).
+// With eight groups it takes 21.3 to 22.8 from run to run, but the 117 000 tiles of 60 M columns by windows are 0.5 % slower; with
+// sixteen the reads themselves get in the way (28.2, and 6.5 %).
 constexpr int kLookGroups = 4;
 
 __device__ __forceinline__ i64 tile_resolve_prefix(const TileState& ts, int tile, i64 aggregate, bool* lost) {

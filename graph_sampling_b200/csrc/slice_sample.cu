@@ -550,7 +550,7 @@ int sample_uniform_launch(gsb_ctx* ctx, cudaStream_t stream, const i64* indptr, 
   }
   {
     ScopedKernelTimer timer(ctx, KID_SAMPLE_UNIFORM, stream);
-    // the register count follows the unrolled pick array (56 / 52 / 64 / 72 / 96 registers); the usual fan-outs 5 and
+    // the register count follows the unrolled pick array (64 / 64 / 72 / 80 / 94 registers, with data up to 126); the usual fan-outs 5 and
     // 10 get instantiations of their own.  A large call runs at the rate at which DRAM serves random 64-byte accesses, not at
     // the limit of its resident lanes: gathers through ld.global.nc.L2::64B (with or without L1::no_allocate) instead of
     // __ldg, to keep the L2 from fetching more than one 64-byte line per gather, changed nothing.

@@ -13,8 +13,10 @@
 // A tile's stretch is its own, so nothing has to be counted across tiles; every pick costs 8 more bytes written and 8 more read,
 // in whole lines.  67 M columns of 5 picks and 8.2 M of 10 out of 124 M edges (the last hops of 500 minibatches), ms: one pass 6.30
 // and 1.63 (with the counts of buckets), draw 1.41 and 0.31 (instruction issue, barriers), read 1.25 and 0.33 (random reads at
-// 264 G/s), emit 0.92 and 0.31 (HBM), 1.32 with the counts of the larger one.
-// Tiles of 1 024 columns: read 1.22, draw 1.57, emit 1.04; of 512 with windows of 32 / 128 MB: read 1.35 / 2.17.
+// 264 G/s), emit 0.92 and 0.31 (5.2 TB/s of real traffic), 1.32 with the counts of the larger one.
+// Tiles of 1 024 columns: read 1.22, draw 1.57, emit 1.04; of 512 with windows of 32 / 128 MB: read 1.35 / 2.17.  The emit pass spills a
+// few words at its eight CTAs an SM (64 bytes stored, 56 loaded a thread); with seven a call of 60 M columns takes the
+// same 3.21 ms, with six 3.26.
 #include "uniform_sample.cuh"
 
 namespace gsb {
